@@ -295,17 +295,29 @@ __global__ void __launch_bounds__(128) channel_delta_prepare_kernel(
 
 // ---- mLSTM: q * D^-1/2, k, v to fp32 and the capped log gates -----------------------------
 // proj row: [q: H*D | k: H*D | v: H*E | ...]; gates: fp32 [rows][2H] = [input | forget] logits.
+// kept (or null): fp32 [requests][H*D + H] receives what the requests' states hold of n and m as the step
+// begins: every block of a head in the recurrence reads them and one of them writes the new ones, so
+// they cannot be read where they are written (blocks that start late would find the new ones).
 template <typename T>
 __global__ void mlstm_prepare_kernel(const T* __restrict__ proj, int proj_stride,
                                      const float* __restrict__ gates, int gates_stride,
                                      const float* __restrict__ bias_i,
                                      const float* __restrict__ bias_f, float cap, float* __restrict__ qkv,
                                      float* __restrict__ log_keep, float* __restrict__ log_in,
-                                     int n_heads, int key_dim, int value_dim) {
+                                     int n_heads, int key_dim, int value_dim, float* __restrict__ kept,
+                                     const int* __restrict__ req_state_slot, unsigned char* state,
+                                     long slot_stride, long n_off, long m_off, int n_requests) {
     cb_pdl_trigger();
     cb_pdl_wait();
     const int t = blockIdx.x;
     const int nq = n_heads * key_dim, C = 2 * nq + n_heads * value_dim;
+    if (kept != nullptr && t < n_requests) {      // a request brings one row at least
+        const float* N = state_at(state, slot_stride, req_state_slot[t], n_off);
+        const float* M = state_at(state, slot_stride, req_state_slot[t], m_off);
+        float* to = kept + (size_t)t * (nq + n_heads);
+        for (int c = threadIdx.x; c < nq; c += blockDim.x) to[c] = N[c];
+        for (int h = threadIdx.x; h < n_heads; h += blockDim.x) to[nq + h] = M[h];
+    }
     const float q_scale = 1.0f / sqrtf((float)key_dim);
     const T* src = proj + (size_t)t * proj_stride;
     float* dst = qkv + (size_t)t * C;
@@ -382,8 +394,8 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     const int* __restrict__ req_row_start, const int* __restrict__ req_state_slot,
     unsigned char* state, long slot_stride, long s_off, long n_off, long m_off,
     float* __restrict__ out, int n_heads, int n_qk_heads, int D, int E, int w_off,
-    const float* __restrict__ per_head) {
-    // w_off: wkv's and channel delta's decay vectors in the rows of qkv (one of D per head); per_head: wkv's bonus
+    const float* __restrict__ per_head, const float* __restrict__ kept) {
+    // kept: the mLSTM's n and m as the step begins, [requests][H*D + H]; w_off: wkv's and channel delta's decay vectors in the rows of qkv (one of D per head); per_head: wkv's bonus
     // u [H][D], the state-space rule's skip [H]
     cb_pdl_trigger();
     cb_pdl_wait();
@@ -404,6 +416,7 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     float* S = state_at(state, slot_stride, slot, s_off) + (size_t)head * D * E;
     float* N = RULE == RULE_MLSTM ? state_at(state, slot_stride, slot, n_off) + (size_t)head * D : nullptr;
     float* M = RULE == RULE_MLSTM ? state_at(state, slot_stride, slot, m_off) + head : nullptr;
+    const float* kept_n = RULE == RULE_MLSTM ? kept + (size_t)r * (n_heads * D + n_heads) : nullptr;
     // the padding of the staged rows and the columns beyond E stay zero
     for (int i = threadIdx.x; i < 2 * BUF; i += blockDim.x) stage[i] = 0.f;
     float s[P], n[P];
@@ -412,11 +425,11 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     for (int i = 0; i < P; ++i) {
         const int d = part * P + i;
         s[i] = (live && d < D) ? S[(size_t)d * E + col] : 0.f;
-        n[i] = (RULE == RULE_MLSTM && d < D) ? N[d] : 0.f;
+        n[i] = (RULE == RULE_MLSTM && d < D) ? kept_n[(size_t)head * D + d] : 0.f;
         if (RULE == RULE_WKV) n[i] = d < D ? per_head[(size_t)head * D + d] : 0.f;      // the bonus u
     }
     const float skip = RULE == RULE_SSD ? per_head[head] : 0.f;
-    if (RULE == RULE_MLSTM) m = *M;
+    if (RULE == RULE_MLSTM) m = kept_n[(size_t)n_heads * D + head];
     __syncthreads();
     // 16-byte copies if every row of q and k starts on a 16-byte boundary
     const bool vec = ((C | q_off | k_off | D | (VECTOR ? w_off : 0)) & 3) == 0;
@@ -812,7 +825,7 @@ int launch_memory_as(const float* qkv, int C, int q_off, int k_off, int v_off, c
                      const float* sc1, const int* req_row_start, const int* req_state_slot,
                      unsigned char* state, long slot_stride, long s_off, long n_off, long m_off, float* out,
                      int n_requests, int n_heads, int n_qk_heads, int D, int E, int w_off,
-                     const float* per_head, cudaStream_t s) {
+                     const float* per_head, const float* kept, cudaStream_t s) {
     constexpr int COLS = THREADS / LANES, PAD = P == 4 ? 8 : 4, NVEC = VECTOR_DECAY<RULE> ? 3 : 2;
     const dim3 grid(n_requests, n_heads, (E + COLS - 1) / COLS), block(THREADS);
     const size_t smem = 2 * (size_t)(CHUNK * (NVEC * LANES * (P + PAD) + COLS) + 2 * CHUNK) * sizeof(float);
@@ -827,7 +840,7 @@ int launch_memory_as(const float* qkv, int C, int q_off, int k_off, int v_off, c
     }
     cb_launch(matrix_memory_kernel<P, LANES, RULE>, grid, block, smem, s, qkv, C, q_off, k_off, v_off, sc0,
               sc1, req_row_start, req_state_slot, state, slot_stride, s_off, n_off, m_off, out, n_heads,
-              n_qk_heads, D, E, w_off, per_head);
+              n_qk_heads, D, E, w_off, per_head, kept);
     return cb_last_error();
 }
 
@@ -840,12 +853,12 @@ int launch_memory(const float* qkv, int C, int q_off, int k_off, int v_off, cons
                   const float* sc1, const int* req_row_start, const int* req_state_slot,
                   unsigned char* state, long slot_stride, long s_off, long n_off, long m_off, float* out,
                   int n_requests, int n_heads, int n_qk_heads, int D, int E, int w_off,
-                  const float* per_head, cudaStream_t s) {
+                  const float* per_head, const float* kept, cudaStream_t s) {
 #define CB_MEM(PP, LL)                                                                              \
     return launch_memory_as<PP, LL, RULE>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start,     \
                                           req_state_slot, state, slot_stride, s_off, n_off, m_off,  \
                                           out, n_requests, n_heads, n_qk_heads, D, E, w_off,        \
-                                          per_head, s)
+                                          per_head, kept, s)
     if (D <= 32) CB_MEM(4, 8);
     if (D <= 64) CB_MEM(8, 8);
     if (D <= 128) CB_MEM(16, 8);
@@ -937,18 +950,21 @@ CB_EXPORT int cb_conv_tail_update(const void* proj, int proj_stride, int dtype, 
 CB_EXPORT int cb_mlstm_prepare(const void* proj, int proj_stride, int dtype, const float* gates,
                                int gates_stride, const float* bias_i, const float* bias_f, float cap, float* qkv,
                                float* log_keep, float* log_in, int n_rows, int n_heads, int key_dim,
-                               int value_dim, void* stream) {
+                               int value_dim, float* kept, const int* req_state_slot, void* state,
+                               long slot_stride, long n_off, long m_off, int n_requests, void* stream) {
     if (n_rows <= 0) return 0;
     const int C = n_heads * (2 * key_dim + value_dim);
     const dim3 grid(n_rows), block(C <= 512 ? 128 : (C >= 4096 ? 1024 : (C / 4 + 31) / 32 * 32));
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == CB_F32)
         cb_launch(mlstm_prepare_kernel<float>, grid, block, 0, s, (const float*)proj, proj_stride,
-                  gates, gates_stride, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads, key_dim, value_dim);
+                  gates, gates_stride, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads, key_dim, value_dim,
+                  kept, req_state_slot, (unsigned char*)state, slot_stride, n_off, m_off, n_requests);
     else
         cb_launch(mlstm_prepare_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)proj,
                   proj_stride, gates, gates_stride, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads,
-                  key_dim, value_dim);
+                  key_dim, value_dim, kept, req_state_slot, (unsigned char*)state, slot_stride, n_off, m_off,
+                  n_requests);
     return cb_last_error();
 }
 
@@ -975,7 +991,7 @@ CB_EXPORT int cb_retention_prepare(const void* proj, int proj_stride, int dtype,
     return cb_last_error();
 }
 
-// rule 0: the delta rule (sc0 decay, sc1 beta); rule 1: mLSTM (sc0 log keep, sc1 log in);
+// rule 0: the delta rule (sc0 decay, sc1 beta); rule 1: mLSTM (sc0 log keep, sc1 log in, kept);
 // rule 2: wkv (decay vectors at w_off in the rows, per_head the bonus [H][D]);
 // rule 3: state space (sc0 decay, sc1 step size, per_head the skip [H]);
 // rule 4: channel delta (decay vectors at w_off, one of D per head; sc1 beta).
@@ -984,17 +1000,18 @@ CB_EXPORT int cb_matrix_memory(int rule, const float* qkv, int C, int q_off, int
                                const int* req_state_slot, void* state, long slot_stride, long s_off,
                                long n_off, long m_off, float* out, int n_requests, int n_heads,
                                int n_qk_heads, int key_dim, int value_dim, int w_off,
-                               const float* per_head, void* stream) {
+                               const float* per_head, const float* kept, void* stream) {
     if (n_requests <= 0) return 0;
     if (n_heads % n_qk_heads != 0) return CB_ERR_UNSUPPORTED;
     if ((rule == RULE_WKV || rule == RULE_SSD) && per_head == nullptr) return CB_ERR_UNSUPPORTED;
+    if (rule == RULE_MLSTM && kept == nullptr) return CB_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
 #define CB_RULE(RR)                                                                                  \
     if (rule == RR)                                                                                  \
         return launch_memory<RR>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start,               \
                                  req_state_slot, (unsigned char*)state, slot_stride, s_off, n_off,   \
                                  m_off, out, n_requests, n_heads, n_qk_heads, key_dim, value_dim,    \
-                                 w_off, per_head, s)
+                                 w_off, per_head, kept, s)
     CB_RULE(RULE_DELTA);
     CB_RULE(RULE_MLSTM);
     CB_RULE(RULE_WKV);

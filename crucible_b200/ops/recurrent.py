@@ -72,13 +72,22 @@ def conv_tail_update(proj, taps, channels, ctx, state, tail_off) -> None:
 
 
 def mlstm_prepare(proj, gates, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads, key_dim,
-                  value_dim) -> None:
-    _need_cuda(proj, gates, bias_i, bias_f, qkv, log_keep, log_in)
+                  value_dim, ctx=None, state=None, n_off=0, m_off=0, kept=None) -> None:
+    """`kept` (with `ctx`, `state` and the offsets of n and m in it): float32 [requests, H*D + H] that
+    receives the requests' n and m as the step begins, for `matrix_memory`."""
+    _need_cuda(proj, gates, bias_i, bias_f, qkv, log_keep, log_in, state, kept)
+    sp, stride = _state_args(state) if kept is not None else (_ptr(None), _c_long(0))
+    if kept is not None and (kept.dtype != torch.float32 or not kept.is_contiguous()
+                             or tuple(kept.shape) != (ctx.n_requests, n_heads * (key_dim + 1))
+                             or proj.shape[0] < ctx.n_requests):
+        raise KernelError("mlstm_prepare: kept is float32 [requests, H*D + H]")
     lib = build.load("recurrent")
     _check(lib.cb_mlstm_prepare(
         _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(gates), _c_int(gates.stride(0)), _ptr(bias_i),
         _ptr(bias_f), _c_float(cap), _ptr(qkv), _ptr(log_keep), _ptr(log_in), _c_int(proj.shape[0]),
-        _c_int(n_heads), _c_int(key_dim), _c_int(value_dim), _stream()), "mlstm_prepare")
+        _c_int(n_heads), _c_int(key_dim), _c_int(value_dim), _ptr(kept),
+        _ptr(ctx.req_state_slot if kept is not None else None), sp, stride, _c_long(n_off), _c_long(m_off),
+        _c_int(ctx.n_requests if kept is not None else 0), _stream()), "mlstm_prepare")
 
 
 def retention_prepare(proj, freq, rotary_dim: int, split_halves: bool, ctx, head_decay, k_scale: float,
@@ -106,11 +115,16 @@ def retention_prepare(proj, freq, rotary_dim: int, split_halves: bool, ctx, head
 
 
 def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n_off, m_off, out,
-                  n_heads, n_qk_heads, key_dim, value_dim, w_off=0, per_head=None) -> None:
+                  n_heads, n_qk_heads, key_dim, value_dim, w_off=0, per_head=None, kept=None) -> None:
     """Walks every request's tokens in order through its heads' matrices (see the kernel).
     `w_off`: where the wkv and channel rules' decay vectors (one a head) lie in the rows of `qkv`; `per_head`: float32
-    constants, the wkv rule's bonus [heads, key_dim] or the state-space rule's skip [heads]."""
-    _need_cuda(qkv, sc0, sc1, state, out, per_head)
+    constants, the wkv rule's bonus [heads, key_dim] or the state-space rule's skip [heads]; `kept`: the
+    mLSTM's n and m as `mlstm_prepare` left them (None: they are copied here)."""
+    _need_cuda(qkv, sc0, sc1, state, out, per_head, kept)
+    if rule == MLSTM and kept is None:
+        nd, slots = n_heads * key_dim, ctx.req_state_slot.long()
+        kept = torch.cat([state[:, n_off:n_off + 4 * nd][slots].contiguous().view(torch.float32),
+                          state[:, m_off:m_off + 4 * n_heads][slots].contiguous().view(torch.float32)], 1)
     if per_head is not None and (per_head.dtype != torch.float32 or not per_head.is_contiguous()):
         raise KernelError("matrix_memory: the per-head constants are contiguous float32")
     if qkv.dtype != torch.float32 or out.dtype != torch.float32 or not qkv.is_contiguous():
@@ -122,7 +136,7 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         _ptr(sc0), _ptr(sc1), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride,
         _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(ctx.n_requests),
         _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim), _c_int(w_off),
-        _ptr(per_head), _stream()), "matrix_memory")
+        _ptr(per_head), _ptr(kept), _stream()), "matrix_memory")
 
 
 def head_norm_gate(o, gain, gain_per_head, gate, out, gate_kind, n_heads, value_dim, eps,

@@ -234,10 +234,12 @@ class MLSTM(BranchMixer):
         log_keep = ctx.scratch("mlstm.keep", (t, H), torch.float32)
         log_in = ctx.scratch("mlstm.in", (t, H), torch.float32)
         o = ctx.scratch("mlstm.o", (t, H * E), torch.float32)
+        kept = ctx.scratch("mlstm.kept", (ctx.n_requests, H * D + H), torch.float32)
+        n_off, m_off = self.s_bytes, self.s_bytes + self.n_bytes
         kernels.mlstm_prepare(proj, gates, self.bias_i, self.bias_f, self.cap, qkv, log_keep, log_in,
-                              H, D, E)
+                              H, D, E, ctx=ctx, state=state, n_off=n_off, m_off=m_off, kept=kept)
         kernels.matrix_memory(kernels.MLSTM, qkv, 0, H * D, 2 * H * D, log_keep, log_in, ctx, state, 0,
-                              self.s_bytes, self.s_bytes + self.n_bytes, o, H, H, D, E)
+                              n_off, m_off, o, H, H, D, E, kept=kept)
         kernels.head_norm_gate(o, self.gain, True, proj[:, C:C + H * E], act, kernels.GATE_SIGMOID, H, E,
                                self.eps, out_scale)
 

@@ -314,3 +314,25 @@ def test_mlstm_in_portions(dtype, H, D, E):
         ref[:, h] = plain.matrix_memory(q[:, h], kk[:, h], v[:, h], log_in[:, h], log_keep[:, h])
     ref = plain.rms_unit(ref, 1e-5).reshape(n, H * E) * gain.double() * torch.sigmoid(p[:, C:])
     assert rel(out, ref) < TOL[dtype]
+
+
+def test_mlstm_reads_its_normaliser_before_any_block_writes_it():
+    """More blocks than the GPU holds at once: the late blocks of a head still start from the n and m of
+    the step before, although the block that writes the new ones is long done.  One token for each of 40
+    requests, 16 heads of 128, in 32 bits against float64."""
+    from crucible_b200.config.model_config import MixerSpec
+    from crucible_b200.parts import MIXERS
+    from test_futepel_kernels_gpu import Steps, _bind, _binding
+    R, H, D, width = 40, 16, 128, 64
+    part = MIXERS.build("mlstm", MixerSpec(kind="mlstm", width=width, n_heads=H, n_kv_heads=H, head_dim=D,
+                                           extra=(("gate_cap", 15.0), ("norm_eps", 1e-5))))
+    w = _bind(part, torch.float32, 3, std=0.125)
+    steps = Steps(torch.float32, part.state_bytes(), None, 8, R, 64)
+    binding = _binding(part)
+    h = torch.randn(R, 4, width)
+    for t in range(4):
+        got = torch.zeros(R, width, device=DEV)
+        part.forward(steps.ctx([(r, 1) for r in range(R)], binding), h[:, t].contiguous().to(DEV), got, binding)
+    cfg = {"heads": H, "dim": D, "vdim": D, "gate_cap": 15.0}
+    ref = torch.stack([plain.mlstm(h[r].double(), w, cfg, 1e-5)[-1] for r in range(R)])
+    assert rel(got, ref) < TOL[torch.float32]

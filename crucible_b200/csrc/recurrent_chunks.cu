@@ -13,14 +13,18 @@
 //       (1 + N) u = beta (v - (G k) S0), so  u = U - W S0  with  (1 + N) [U | W] = beta [v | G k],
 //       and  o_t = (G_t q_t - (A W)_t) . S0 + (A U)_t.
 //
-// Products of decays are taken as products (a decay may be 0), never as quotients of running products.
+// Products of decays are taken as products (a decay may be 0), never as quotients of running products; no
+// sum runs over a later token's values, not even times zero (a later NaN stays later).
 //
 // chunk_local_kernel: everything of a chunk that does not need S0, all chunks and heads side by side; the
 // two triangular systems are one column a thread, its 32 values in registers.
 // chunk_walk_kernel: a block owns 16 (or 8) columns of a head's S and walks the chunks in order: per
 // chunk two products on fp32 FMA (rows of Q, and W, over S; k^T over u), the next chunk's operands on
-// their way by asynchronous copies.  Bound by the fp32 pipe: its 2 or 3 multiply-adds per entry of S and
-// token are what the token-by-token walk does too.
+// their way by asynchronous copies.  Its 2 or 3 multiply-adds per entry of S and token are what the
+// token-by-token walk does too; sums run over neighbouring pairs (one instruction for two).
+//
+// Measured at 2,048 tokens of 16 heads of 128 (token by token -> in chunks): delta 503 -> 258 us, channel
+// delta 551 -> 325, mLSTM 590 -> 260, state space 410 -> 201; 64 tokens: 18 -> 21 us, 512: 128 -> 69.
 //
 // The result differs from the token-by-token walk by rounding, and with the way a prompt is cut: the
 // bfloat16 engine's prompts alone take this path; decoded tokens and the float32 engine keep the walk.
@@ -32,8 +36,8 @@ namespace {
 constexpr int RULE_DELTA = 0, RULE_MLSTM = 1, RULE_WKV = 2, RULE_SSD = 3, RULE_CHANNEL = 4;
 template <int RULE> constexpr bool VECTOR_DECAY = RULE == RULE_WKV || RULE == RULE_CHANNEL;
 template <int RULE> constexpr bool IS_DELTA = RULE == RULE_DELTA || RULE == RULE_CHANNEL;
-// rules whose queries' rows over S0 are rows of their own (else they are the rows of q as they are,
-// the decay being a number a token)
+// rules whose queries over S0 are rows of their own (else they are the rows of q as they are, the decay
+// being a number a token)
 template <int RULE> constexpr bool OWN_Q = RULE != RULE_SSD && RULE != RULE_MLSTM;
 constexpr int CT = 32;              // tokens of a chunk
 constexpr int THREADS = 256;
@@ -55,6 +59,29 @@ struct Args {
     float4* ws;
 };
 
+// two fp32 numbers in one register pair, multiplied and added by one instruction
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t fma_pair(pair_t a, pair_t b, pair_t c) {
+    pair_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ pair_t make_pair_of(float lo, float hi) {
+    pair_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 split_pair(pair_t p) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float pair_sum(pair_t p) {
+    const float2 v = split_pair(p);
+    return v.x + v.y;
+}
+__device__ __forceinline__ ulonglong2 pairs_at(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
 __device__ __forceinline__ float* state_at(unsigned char* state, long slot_stride, int slot, long off) {
     return reinterpret_cast<float*>(state + (size_t)slot * slot_stride + off);
 }
@@ -65,12 +92,92 @@ __device__ __forceinline__ void cp16(float* smem, const float* gmem) {
 // a chunk's place among the step's chunks: strictly growing over a request's chunks and over requests
 __device__ __forceinline__ size_t chunk_place(int row, int r) { return (size_t)(row / CT + r); }
 
+// row t of a lower triangular matrix times a column in registers (pairs of neighbouring tokens), entries
+// 0 .. COUNT - 1
+template <int COUNT>
+__device__ __forceinline__ float row_times(const float* row, const pair_t (&x)[CT / 2]) {
+    pair_t a = 0, b = 0;
+    float tail = 0.f;
+#pragma unroll
+    for (int s = 0; s < COUNT; s += 4) {
+        const ulonglong2 n = pairs_at(row + s);
+        if (s + 1 < COUNT) a = fma_pair(n.x, x[s / 2], a);
+        else tail = split_pair(n.x).x * split_pair(x[s / 2]).x;
+        if (s + 3 < COUNT) b = fma_pair(n.y, x[s / 2 + 1], b);
+        else if (s + 2 < COUNT) tail = split_pair(n.y).x * split_pair(x[s / 2 + 1]).x;
+    }
+    return (pair_sum(a) + pair_sum(b)) + tail;
+}
+template <int T>
+__device__ __forceinline__ void set_token(pair_t (&x)[CT / 2], float v) {
+    const float2 p = split_pair(x[T / 2]);
+    x[T / 2] = T % 2 ? make_pair_of(p.x, v) : make_pair_of(v, p.y);
+}
+template <int T>
+__device__ __forceinline__ float get_token(const pair_t (&x)[CT / 2]) {
+    const float2 p = split_pair(x[T / 2]);
+    return T % 2 ? p.y : p.x;
+}
+// F::template at<T>() for T = 0 .. CT - 1, unrolled
+template <int T, typename F>
+__device__ __forceinline__ void each_token(F& f) {
+    if constexpr (T < CT) {
+        f.template at<T>();
+        each_token<T + 1>(f);
+    }
+}
+
+// forward substitution down a column: (1 + N) x = b x
+struct Substitute {
+    pair_t (&x)[CT / 2];
+    const float *N, *b;
+    template <int T> __device__ __forceinline__ void at() {
+        set_token<T>(x, fmaf(b[T], get_token<T>(x), -row_times<T>(N + T * AP, x)));
+    }
+};
+// a column of v: its tokens' results within the chunk, and u for the delta rules
+template <int RULE> struct ValueColumn {
+    pair_t (&x)[CT / 2];
+    const float* A;
+    float *out, *wu, skip;
+    size_t stride;
+    int cnt;
+    template <int T> __device__ __forceinline__ void at() {
+        if (T < cnt) {
+            const float v = get_token<T>(x), o = row_times<T + 1>(A + T * AP, x);
+            out[T * stride] = RULE == RULE_SSD ? fmaf(skip, v, o) : o;
+            if (IS_DELTA<RULE>) wu[T * stride] = v;
+        }
+    }
+};
+// a key channel: the queries' rows over S0, and W for the delta rules
+template <int RULE, int P> struct KeyColumn {
+    pair_t (&x)[CT / 2];
+    const float *A, *q, *decay;            // q, decay: this channel's column (decay: or one number a token)
+    float *wq, *ww, G;
+    size_t stride;
+    int cnt;
+    template <int T> __device__ __forceinline__ void at() {
+        if (T < cnt) {
+            const float g = decay[T * (VECTOR_DECAY<RULE> ? P : 1)];
+            if (RULE != RULE_WKV) G *= g;          // wkv reads the state before its token's decay
+            float o = 0.f;
+            if (IS_DELTA<RULE>) {
+                o = row_times<T + 1>(A + T * AP, x);
+                ww[T * stride] = get_token<T>(x);
+            }
+            wq[T * stride] = fmaf(q[T * P], G, -o);
+            if (RULE == RULE_WKV) G *= g;
+        }
+    }
+};
+
 // ---- what a chunk can do without the state before it ------------------------------------------
 // ws of a token and head: x = G_t (mLSTM: the sum of its log keeps from the chunk's start), y = what its
 // row of k is times when it joins the state (the decay to the chunk's end, the step size), z, w (mLSTM):
 // the running maximum of the chunk alone and its row's sum of A.
 template <int DP, int RULE>
-__global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
+__global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int P = DP + 4;                       // pitch: 8 neighbouring rows' 16-byte reads hit 32 banks
@@ -87,7 +194,7 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
     float* sN = sA + CT * AP;                       // delta rules; before that (scalar decays) L
     float* sa = sN + CT * AP;                       // [CT] decay of a token, [CT] beta or step
     float* sb = sa + CT;
-    float* part = sb + CT;                          // vector decays: [DP / 16][2][CT][CT] shares of the dots
+    float* part = sb + CT;                          // vector decays: [DP / 16][1 or 2][CT][CT] shares of the dots
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
@@ -132,10 +239,11 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
             // L[t][s] = product of the decays of s + 1 .. t; a column s a lane
             __syncwarp();
             float l = 0.f, G = 1.f;
+#pragma unroll 8
             for (int t = 0; t < CT; ++t) {
                 const float x = sa[t];
                 l = t == lane ? 1.f : l * x;
-                sN[t * AP + lane] = l;
+                sN[t * AP + lane] = t < lane ? 0.f : l;
                 if (t <= lane) G *= x;
             }
             if (in) {
@@ -150,40 +258,37 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
     // the dots of the chunk's rows: A, and for the delta rules N
     if (!VECTOR) {
         const int tr = tid >> 4, tc = tid & 15;     // rows tr, tr + 16 against columns tc, tc + 16
-        float qk[3] = {0.f, 0.f, 0.f}, kk[3] = {0.f, 0.f, 0.f};
+        pair_t qk[3] = {0, 0, 0}, kk[3] = {0, 0, 0};
 #pragma unroll 4
         for (int d = 0; d < DP; d += 4) {
-            float4 q[2], k[2], c[2];
+            ulonglong2 q[2], k[2], c[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                q[i] = *reinterpret_cast<const float4*>(sq + (tr + 16 * i) * P + d);
-                if (DELTA) k[i] = *reinterpret_cast<const float4*>(sk + (tr + 16 * i) * P + d);
-                c[i] = *reinterpret_cast<const float4*>(sk + (tc + 16 * i) * P + d);
+                q[i] = pairs_at(sq + (tr + 16 * i) * P + d);
+                if (DELTA) k[i] = pairs_at(sk + (tr + 16 * i) * P + d);
+                c[i] = pairs_at(sk + (tc + 16 * i) * P + d);
             }
 #pragma unroll
             for (int p = 0; p < 3; ++p) {           // (0, 0), (1, 0), (1, 1): the fourth lies above the diagonal
-                const float4 x = q[p > 0], z = c[p > 1];
-                qk[p] = fmaf(x.x, z.x, qk[p]); qk[p] = fmaf(x.y, z.y, qk[p]);
-                qk[p] = fmaf(x.z, z.z, qk[p]); qk[p] = fmaf(x.w, z.w, qk[p]);
+                qk[p] = fma_pair(q[p > 0].x, c[p > 1].x, qk[p]);
+                qk[p] = fma_pair(q[p > 0].y, c[p > 1].y, qk[p]);
                 if (DELTA) {
-                    const float4 y = k[p > 0];
-                    kk[p] = fmaf(y.x, z.x, kk[p]); kk[p] = fmaf(y.y, z.y, kk[p]);
-                    kk[p] = fmaf(y.z, z.z, kk[p]); kk[p] = fmaf(y.w, z.w, kk[p]);
+                    kk[p] = fma_pair(k[p > 0].x, c[p > 1].x, kk[p]);
+                    kk[p] = fma_pair(k[p > 0].y, c[p > 1].y, kk[p]);
                 }
             }
         }
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
+        for (int p = 0; p < 3; ++p) {               // (what lands above the diagonal is never read)
             const int t = tr + (p > 0 ? 16 : 0), s = tc + (p > 1 ? 16 : 0);
-            const float l = sN[t * AP + s];         // 0 above the diagonal
-            sA[t * AP + s] = qk[p] * l * (DELTA ? 1.f : sb[s]);
-            if (DELTA) sN[t * AP + s] = s < t ? sb[t] * kk[p] * l : 0.f;
+            const float l = sN[t * AP + s];
+            sA[t * AP + s] = pair_sum(qk[p]) * l * (DELTA ? 1.f : sb[s]);
+            if (DELTA) sN[t * AP + s] = sb[t] * pair_sum(kk[p]) * l;
         }
-        sA[tr * AP + tc + 16] = 0.f;
-        if (DELTA) sN[tr * AP + tc + 16] = 0.f;
         __syncthreads();
     } else {
         // a column s a lane, 16 channels a warp: the key decays on its way down the rows
+        constexpr int SHARE = (DELTA ? 2 : 1) * CT * CT;
         if (warp < DP / 16) {
             const int d0 = warp * 16, s = lane;
             float w[16], first = 0.f;
@@ -199,7 +304,8 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
                     first = fmaf(u * w[i], sq[s * P + d0 + i], first);
                 }
             }
-            float* to = part + (size_t)warp * 2 * CT * CT;
+            float* to = part + (size_t)warp * SHARE;
+#pragma unroll 2
             for (int t = 0; t < CT; ++t) {
                 float qk[4] = {0.f, 0.f, 0.f, 0.f}, kk[4] = {0.f, 0.f, 0.f, 0.f};
                 const float* rq = sq + t * P + d0;
@@ -221,8 +327,8 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
                 }
                 float x = (qk[0] + qk[1]) + (qk[2] + qk[3]);
                 if (RULE == RULE_WKV && t == s) x = first;
-                to[t * CT + s] = t >= s ? x : 0.f;
-                if (DELTA) to[CT * CT + t * CT + s] = t > s ? (kk[0] + kk[1]) + (kk[2] + kk[3]) : 0.f;
+                to[t * CT + s] = x;
+                if (DELTA) to[CT * CT + t * CT + s] = (kk[0] + kk[1]) + (kk[2] + kk[3]);
             }
         }
         __syncthreads();
@@ -231,8 +337,8 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
             float x = 0.f, y = 0.f;
 #pragma unroll
             for (int w = 0; w < DP / 16; ++w) {
-                x += part[(size_t)w * 2 * CT * CT + i];
-                if (DELTA) y += part[(size_t)(w * 2 + 1) * CT * CT + i];
+                x += part[(size_t)w * SHARE + i];
+                if (DELTA) y += part[(size_t)w * SHARE + CT * CT + i];
             }
             sA[t * AP + s] = x;
             if (DELTA) sN[t * AP + s] = sb[t] * y;
@@ -245,11 +351,12 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
         for (int s = 0; s <= tid; ++s) n += sA[tid * AP + s];
         a.ws[(size_t)(row0 + tid) * H + head].w = n;
     }
+    const size_t first = (size_t)row0 * H + head;      // the chunk's first row of a workspace
     // vector decays: keys decayed to the chunk's end, and the whole chunk's decay
     if (VECTOR && tid < D) {
         float to_end = 1.f;
         for (int t = cnt - 1; t >= 0; --t) {
-            a.wk[((size_t)(row0 + t) * H + head) * D + tid] = sk[t * P + tid] * to_end;
+            a.wk[(first + (size_t)t * H) * D + tid] = sk[t * P + tid] * to_end;
             to_end *= sw[t * P + tid];
         }
         a.wg[(chunk_place(row0, r) * H + head) * D + tid] = to_end;
@@ -257,71 +364,44 @@ __global__ void __launch_bounds__(THREADS) chunk_local_kernel(const Args a) {
     // the columns: E of v, then (delta rules: W; other vector decays: the decayed queries) D of the keys
     const int columns = E + (OWN_Q<RULE> ? D : 0);
     for (int c = tid; c < columns; c += THREADS) {
-        float x[CT];
-        const bool is_v = c < E;
+        pair_t x[CT / 2];
         const int d = c - E;
-        if (is_v) {
+        if (d < 0) {
             const float* src = a.qkv + (size_t)row0 * a.C + a.v_off + (size_t)head * E + c;
+            float v[CT];
 #pragma unroll
-            for (int t = 0; t < CT; ++t) x[t] = t < cnt ? src[(size_t)t * a.C] : 0.f;
+            for (int t = 0; t < CT; ++t) v[t] = t < cnt ? src[(size_t)t * a.C] : 0.f;
+#pragma unroll
+            for (int t = 0; t < CT; t += 2) x[t / 2] = make_pair_of(v[t], v[t + 1]);
         } else if (DELTA) {
             float G = 1.f;
 #pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                G *= VECTOR ? sw[t * P + d] : sa[t];
-                x[t] = sk[t * P + d] * G;
+            for (int t = 0; t < CT; t += 2) {
+                const float ga = G * (VECTOR ? sw[t * P + d] : sa[t]);
+                G = ga * (VECTOR ? sw[(t + 1) * P + d] : sa[t + 1]);
+                x[t / 2] = make_pair_of(sk[t * P + d] * ga, sk[(t + 1) * P + d] * G);
             }
         }
         if (DELTA) {
-            // forward substitution down the column
-#pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-                for (int s = 0; s < t; s += 4) {
-                    const float4 n = *reinterpret_cast<const float4*>(sN + t * AP + s);
-                    s0 = fmaf(n.x, x[s], s0);
-                    if (s + 1 < t) s1 = fmaf(n.y, x[s + 1], s1);
-                    if (s + 2 < t) s0 = fmaf(n.z, x[s + 2], s0);
-                    if (s + 3 < t) s1 = fmaf(n.w, x[s + 3], s1);
-                }
-                x[t] = fmaf(sb[t], x[t], -(s0 + s1));
-            }
+            Substitute f{x, sN, sb};
+            each_token<0>(f);
         }
-        const float skip = RULE == RULE_SSD ? a.per_head[head] : 0.f;
-        float G = 1.f;
-#pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            float s0 = 0.f, s1 = 0.f;
-            if (is_v || DELTA) {
-#pragma unroll
-                for (int s = 0; s <= t; s += 4) {
-                    const float4 n = *reinterpret_cast<const float4*>(sA + t * AP + s);
-                    s0 = fmaf(n.x, x[s], s0);
-                    if (s + 1 <= t) s1 = fmaf(n.y, x[s + 1], s1);
-                    if (s + 2 <= t) s0 = fmaf(n.z, x[s + 2], s0);
-                    if (s + 3 <= t) s1 = fmaf(n.w, x[s + 3], s1);
-                }
-            }
-            const float o = s0 + s1;
-            if (t < cnt) {
-                const size_t at = (size_t)(row0 + t) * H + head;
-                if (is_v) {
-                    a.out[at * E + c] = RULE == RULE_SSD ? fmaf(skip, x[t], o) : o;
-                    if (DELTA) a.wu[at * E + c] = x[t];
-                } else {
-                    // wkv reads the state before its token's decay
-                    if (RULE != RULE_WKV) G *= VECTOR ? sw[t * P + d] : sa[t];
-                    a.wq[at * a.D + d] = fmaf(sq[t * P + d], G, -o);
-                    if (RULE == RULE_WKV) G *= sw[t * P + d];
-                    if (DELTA) a.ww[at * a.D + d] = x[t];
-                }
-            }
+        if (d < 0) {
+            ValueColumn<RULE> f{x, sA, a.out + first * E + c, DELTA ? a.wu + first * E + c : nullptr,
+                                RULE == RULE_SSD ? a.per_head[head] : 0.f, (size_t)H * E, cnt};
+            each_token<0>(f);
+        } else {
+            KeyColumn<RULE, P> f{x, sA, sq + d, VECTOR ? sw + d : sa, a.wq + first * D + d,
+                                 DELTA ? a.ww + first * D + d : nullptr, 1.f, (size_t)H * D, cnt};
+            each_token<0>(f);
         }
     }
 }
 
 // ---- the state from chunk to chunk ---------------------------------------------------------------
+// The state's columns lie in shared memory as rows [ET][DP], so that sums over D run over neighbouring
+// pairs; column 4 j + i is row i * (ET / 4) + j: the columns that neighbouring lanes read then lie a pitch
+// apart and their 16-byte reads fall on different banks.
 template <int DP, int RULE, int ET>
 __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     cb_pdl_trigger();
@@ -329,20 +409,21 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     constexpr int P = DP + 4, CG = ET / 4;
     constexpr bool VECTOR = VECTOR_DECAY<RULE>, DELTA = IS_DELTA<RULE>;
     constexpr int ROWS = DELTA ? 2 * CT : CT;            // rows over S: the queries', then W
-    constexpr int RG = 16;                               // row groups; a thread has ROWS / 16 rows of one
+    constexpr int RG = ROWS / 4;                         // row groups; a thread has four rows, RG apart
     constexpr int SPLIT = THREADS / (RG * CG);           // shares of the sum over D
     constexpr int DS = DP / SPLIT;
     constexpr int STAGE = (ROWS + CT) * P + CT * ET;     // rows over S, keys, u
+    static_assert(DS >= 4 && DS % 4 == 0, "a share of the sum over D is whole 16-byte pieces");
     extern __shared__ __align__(16) float smem[];
-    float* S = smem;                                     // [DP][ET]
-    float* red = S + DP * ET;                            // [SPLIT][ROWS][ET]
-    float* su = red + SPLIT * ROWS * ET;                 // [CT][ET]: u as it joins the state
-    float* sg = su + CT * ET;                            // [DP]: the chunk's decay; mLSTM: n
+    float* S = smem;                                     // [ET][P]
+    float* red = S + ET * P;                             // [SPLIT][ROWS][ET]
+    float* su = red + SPLIT * ROWS * ET;                 // [CT][ET][2]: u as it joins the state, every number twice
+    float* sg = su + 2 * CT * ET;                        // [DP]: the chunk's decay; mLSTM: n
     float* sx = sg + DP;                                 // [CT][2]: mLSTM's factors of a row's two shares
     float4* sc = reinterpret_cast<float4*>(sx + 2 * CT); // [2][CT] the tokens' numbers
     float* stage = reinterpret_cast<float*>(sc + 2 * CT);
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * ET;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
     const int row0 = a.req_row_start[r], row1 = a.req_row_start[r + 1];
@@ -350,38 +431,42 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     float* state = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E;
     const float* n0 = RULE == RULE_MLSTM ? a.kept + (size_t)r * (H * D + H) : nullptr;
     float m0 = RULE == RULE_MLSTM ? n0[(size_t)H * D + head] : 0.f;
+    auto place_of = [](int c) { return (c & 3) * CG + (c >> 2); };
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
-        S[i] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
+        S[place_of(c) * P + d] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
     }
-    if (RULE == RULE_MLSTM)
-        for (int d = tid; d < DP; d += THREADS) sg[d] = d < D ? n0[(size_t)head * D + d] : 0.f;
+    for (int d = tid; d < DP; d += THREADS) sg[d] = RULE == RULE_MLSTM && d < D ? n0[(size_t)head * D + d] : 0.f;
     for (int i = tid; i < 2 * STAGE; i += THREADS) stage[i] = 0.f;      // the rows' and columns' padding
     __syncthreads();
 
+    // a thread copies the same 16-byte piece of every row that is its own
+    constexpr int PIECES = DP / 4, STEP = THREADS / PIECES;
+    const int ft = tid / PIECES, fd = (tid % PIECES) * 4;
     auto fetch = [&](int base, int buf) {
         float* rows = stage + buf * STAGE;
         float* keys = rows + ROWS * P;
         float* u = keys + CT * P;
         const int cnt = min(CT, row1 - base);
-        const int per = D >> 2;
-        for (int i = tid; i < CT * per; i += THREADS) {
-            const int t = i / per, d = (i - t * per) << 2;
-            if (t < cnt) {
-                const size_t at = (size_t)(base + t) * H + head;
-                const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + d;
-                cp16(rows + t * P + d, OWN_Q<RULE> ? a.wq + at * D + d : src + a.q_off);
-                if (DELTA) cp16(rows + (CT + t) * P + d, a.ww + at * D + d);
-                cp16(keys + t * P + d, VECTOR ? a.wk + at * D + d : src + a.k_off);
-            } else {                                     // a portion's last chunk: rows of an earlier one are there
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4*>(rows + t * P + d) = zero;
-                if (DELTA) *reinterpret_cast<float4*>(rows + (CT + t) * P + d) = zero;
-                *reinterpret_cast<float4*>(keys + t * P + d) = zero;
+        if (fd < D) {
+#pragma unroll
+            for (int t = ft; t < CT; t += STEP) {
+                if (t < cnt) {
+                    const size_t at = ((size_t)(base + t) * H + head) * D + fd;
+                    const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + fd;
+                    cp16(rows + t * P + fd, OWN_Q<RULE> ? a.wq + at : src + a.q_off);
+                    if (DELTA) cp16(rows + (CT + t) * P + fd, a.ww + at);
+                    cp16(keys + t * P + fd, VECTOR ? a.wk + at : src + a.k_off);
+                } else {                                 // a portion's last chunk: rows of an earlier one are there
+                    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(rows + t * P + fd) = zero;
+                    if (DELTA) *reinterpret_cast<float4*>(rows + (CT + t) * P + fd) = zero;
+                    *reinterpret_cast<float4*>(keys + t * P + fd) = zero;
+                }
             }
         }
-        for (int i = tid; i < CT * CG; i += THREADS) {
-            const int t = i / CG, c = (i - t * CG) * 4;
+        if (tid < CT * CG) {
+            const int t = tid / CG, c = (tid % CG) * 4;
             if (t < cnt && col0 + c < E) {
                 const size_t row = (size_t)(base + t);
                 cp16(u + t * ET + c, DELTA ? a.wu + (row * H + head) * E + col0 + c
@@ -390,13 +475,21 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 *reinterpret_cast<float4*>(u + t * ET + c) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        if (!VECTOR && tid < CT) {
-            if (tid < cnt) cp16(reinterpret_cast<float*>(sc + buf * CT + tid),
-                                reinterpret_cast<const float*>(a.ws + (size_t)(base + tid) * H + head));
-            else sc[buf * CT + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!VECTOR && tid >= THREADS - CT) {
+            const int t = tid - (THREADS - CT);
+            if (t < cnt) cp16(reinterpret_cast<float*>(sc + buf * CT + t),
+                              reinterpret_cast<const float*>(a.ws + (size_t)(base + t) * H + head));
+            else sc[buf * CT + t] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // the first product: a thread's rows rg + RG i and columns 4 cg + j, its share of D
+    const int share = tid / (RG * CG), rg = (tid % (RG * CG)) / CG, cg = tid % CG;
+    // where its sums go, and who adds the shares
+    const int orow = tid / CG, ocol = cg * 4;
+    // the second product: a thread's four channels and two columns
+    constexpr int DB = DP / 32, CP = ET / 2 < 4 ? ET / 2 : 4;       // blocks of 8 x 4 channels; column pairs a warp
+    const int ud = ((warp % DB) * 8 + lane / 4) * 4, uc = ((warp / DB) * 4 + (lane & 3)) * 2;
     if (row0 < row1) fetch(row0, 0);
     int buf = 0;
     for (int base = row0; base < row1; base += CT, buf ^= 1) {
@@ -405,8 +498,6 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         const float* keys = rows + ROWS * P;
         const float* u = keys + CT * P;
         const float4* nums = sc + buf * CT;
-        // where this thread's sums of the first product go
-        const int orow = tid / CG, ocol = (tid - orow * CG) * 4;
         const bool has_out = orow < cnt && col0 + ocol < E;
         float* out_at = a.out + ((size_t)(base + orow) * H + head) * E + col0 + ocol;
         float4 local = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -421,35 +512,30 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         __syncthreads();
         // the rows over S
         {
-            const int share = tid / (RG * CG), in = tid - share * (RG * CG);
-            const int rg = in / CG, cg = in - rg * CG;
-            float acc[ROWS / RG][4];
+            pair_t acc[4][4];
 #pragma unroll
-            for (int i = 0; i < ROWS / RG; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-#pragma unroll 4
-            for (int d = share * DS; d < share * DS + DS; d += 4) {
-                float4 x[ROWS / RG], y[4];
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0;
+            const float* x_at = rows + rg * P + share * DS;
+            const float* y_at = S + cg * P + share * DS;
 #pragma unroll
-                for (int i = 0; i < ROWS / RG; ++i)
-                    x[i] = *reinterpret_cast<const float4*>(rows + (rg + RG * i) * P + d);
+            for (int d = 0; d < DS; d += 4) {
+                ulonglong2 x[4], y[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) y[j] = *reinterpret_cast<const float4*>(S + (d + j) * ET + 4 * cg);
+                for (int i = 0; i < 4; ++i) x[i] = pairs_at(x_at + RG * i * P + d);
 #pragma unroll
-                for (int i = 0; i < ROWS / RG; ++i) {
-                    const float xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+                for (int j = 0; j < 4; ++j) y[j] = pairs_at(y_at + CG * j * P + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        acc[i][0] = fmaf(xs[j], y[j].x, acc[i][0]);
-                        acc[i][1] = fmaf(xs[j], y[j].y, acc[i][1]);
-                        acc[i][2] = fmaf(xs[j], y[j].z, acc[i][2]);
-                        acc[i][3] = fmaf(xs[j], y[j].w, acc[i][3]);
+                        acc[i][j] = fma_pair(x[i].x, y[j].x, acc[i][j]);
+                        acc[i][j] = fma_pair(x[i].y, y[j].y, acc[i][j]);
                     }
-                }
             }
 #pragma unroll
-            for (int i = 0; i < ROWS / RG; ++i)
+            for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<float4*>(red + ((size_t)share * ROWS + rg + RG * i) * ET + 4 * cg) =
-                    make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                    make_float4(pair_sum(acc[i][0]), pair_sum(acc[i][1]), pair_sum(acc[i][2]), pair_sum(acc[i][3]));
         }
         float g_end = 1.f, in_end = 1.f;
         if (RULE == RULE_MLSTM) {
@@ -484,51 +570,50 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 sum.x += y.x; sum.y += y.y; sum.z += y.z; sum.w += y.w;
             }
             if (orow < CT) {
-                float fa = 1.f, fb = 1.f;
-                if (RULE == RULE_SSD) fa = nums[orow].x;
+                float f = 1.f;
+                if (RULE == RULE_SSD) f = nums[orow].x;
                 if (RULE == RULE_MLSTM) {
-                    fa = sx[2 * orow];
-                    fb = sx[2 * orow + 1];
-                }
-                if (RULE == RULE_MLSTM) {
-                    local.x *= fb; local.y *= fb; local.z *= fb; local.w *= fb;
+                    f = sx[2 * orow];
+                    const float within = sx[2 * orow + 1];
+                    local.x *= within; local.y *= within; local.z *= within; local.w *= within;
                 }
                 if (has_out)
-                    *reinterpret_cast<float4*>(out_at) = make_float4(fmaf(fa, sum.x, local.x), fmaf(fa, sum.y, local.y),
-                                                                     fmaf(fa, sum.z, local.z), fmaf(fa, sum.w, local.w));
-            } else {
-                const int t = orow - CT;
-                const float4 own = *reinterpret_cast<const float4*>(u + t * ET + ocol);
-                const float f = VECTOR ? 1.f : nums[t].y;
-                *reinterpret_cast<float4*>(su + t * ET + ocol) =
-                    make_float4(f * (own.x - sum.x), f * (own.y - sum.y), f * (own.z - sum.z), f * (own.w - sum.w));
+                    *reinterpret_cast<float4*>(out_at) = make_float4(fmaf(f, sum.x, local.x), fmaf(f, sum.y, local.y),
+                                                                     fmaf(f, sum.z, local.z), fmaf(f, sum.w, local.w));
+            }
+            if (DELTA ? orow >= CT : true) {
+                const int t = DELTA ? orow - CT : orow;
+                float4 own = *reinterpret_cast<const float4*>(u + t * ET + ocol);
+                if (DELTA) {
+                    own.x -= sum.x; own.y -= sum.y; own.z -= sum.z; own.w -= sum.w;
+                }
+                const float f = VECTOR ? 1.f : nums[t].y * in_end;
+                float* to = su + 2 * (t * ET + ocol);
+                *reinterpret_cast<float4*>(to) = make_float4(f * own.x, f * own.x, f * own.y, f * own.y);
+                *reinterpret_cast<float4*>(to + 4) = make_float4(f * own.z, f * own.z, f * own.w, f * own.w);
             }
         }
-        if (!DELTA)
-            for (int i = tid; i < CT * CG; i += THREADS) {
-                const int t = i / CG, c = (i - t * CG) * 4;
-                const float4 own = *reinterpret_cast<const float4*>(u + t * ET + c);
-                const float f = VECTOR ? 1.f : nums[t].y * in_end;
-                *reinterpret_cast<float4*>(su + t * ET + c) = make_float4(f * own.x, f * own.y, f * own.z, f * own.w);
-            }
         __syncthreads();
         // the state: decayed, and the chunk's k^T u
-        for (int i = tid; i < (DP / 2) * CG; i += THREADS) {
-            const int d = (i / CG) * 2, cg = i % CG;
-            float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
+        if (uc < ET && (lane & 3) < CP) {
+            pair_t x[2] = {0, 0}, y[2] = {0, 0};
+#pragma unroll 16
             for (int t = 0; t < CT; ++t) {
-                const float2 k = *reinterpret_cast<const float2*>(keys + t * P + d);
-                const float4 v = *reinterpret_cast<const float4*>(su + t * ET + 4 * cg);
-                x[0] = fmaf(k.x, v.x, x[0]); x[1] = fmaf(k.x, v.y, x[1]); x[2] = fmaf(k.x, v.z, x[2]); x[3] = fmaf(k.x, v.w, x[3]);
-                y[0] = fmaf(k.y, v.x, y[0]); y[1] = fmaf(k.y, v.y, y[1]); y[2] = fmaf(k.y, v.z, y[2]); y[3] = fmaf(k.y, v.w, y[3]);
+                const ulonglong2 k = pairs_at(keys + t * P + ud);
+                const ulonglong2 v = pairs_at(su + 2 * (t * ET + uc));
+                x[0] = fma_pair(k.x, v.x, x[0]); x[1] = fma_pair(k.y, v.x, x[1]);
+                y[0] = fma_pair(k.x, v.y, y[0]); y[1] = fma_pair(k.y, v.y, y[1]);
             }
-            const float ga = VECTOR ? sg[d] : g_end, gb = VECTOR ? sg[d + 1] : g_end;
-            float4* a0 = reinterpret_cast<float4*>(S + (size_t)d * ET + 4 * cg);
-            float4* a1 = reinterpret_cast<float4*>(S + (size_t)(d + 1) * ET + 4 * cg);
-            const float4 p = *a0, q = *a1;
-            *a0 = make_float4(fmaf(ga, p.x, x[0]), fmaf(ga, p.y, x[1]), fmaf(ga, p.z, x[2]), fmaf(ga, p.w, x[3]));
-            *a1 = make_float4(fmaf(gb, q.x, y[0]), fmaf(gb, q.y, y[1]), fmaf(gb, q.z, y[2]), fmaf(gb, q.w, y[3]));
+            const float4 own = *reinterpret_cast<const float4*>(sg + ud);
+            const pair_t ga = VECTOR ? make_pair_of(own.x, own.y) : make_pair_of(g_end, g_end);
+            const pair_t gb = VECTOR ? make_pair_of(own.z, own.w) : ga;
+            ulonglong2* sx0 = reinterpret_cast<ulonglong2*>(S + place_of(uc) * P + ud);
+            ulonglong2* sx1 = reinterpret_cast<ulonglong2*>(S + place_of(uc + 1) * P + ud);
+            ulonglong2 p = *sx0, q = *sx1;
+            p.x = fma_pair(ga, p.x, x[0]); p.y = fma_pair(gb, p.y, x[1]);
+            q.x = fma_pair(ga, q.x, y[0]); q.y = fma_pair(gb, q.y, y[1]);
+            *sx0 = p;
+            *sx1 = q;
         }
         if (RULE == RULE_MLSTM)
             for (int d = tid; d < DP; d += THREADS) {
@@ -541,7 +626,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     }
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
-        if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = S[i];
+        if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = S[place_of(c) * P + d];
     }
     if (RULE == RULE_MLSTM && blockIdx.z == 0) {
         float* N = state_at(a.state, a.slot_stride, slot, a.n_off) + (size_t)head * D;
@@ -557,25 +642,27 @@ int allow_smem(K kernel, size_t smem) {
 
 template <int DP, int RULE, int ET>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
-    constexpr bool DELTA = IS_DELTA<RULE>;
-    constexpr int ROWS = DELTA ? 2 * CT : CT, SPLIT = THREADS / (16 * (ET / 4)), P = DP + 4;
-    const size_t floats = DP * ET + SPLIT * ROWS * ET + CT * ET + DP + 2 * CT + 8 * CT + 2 * ((ROWS + CT) * P + CT * ET);
-    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, floats * sizeof(float));
+    constexpr int ROWS = IS_DELTA<RULE> ? 2 * CT : CT, SPLIT = THREADS / ((ROWS / 4) * (ET / 4)), P = DP + 4;
+    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + 2 * CT * ET + DP + 2 * CT + 8 * CT
+                                              + 2 * ((ROWS + CT) * P + CT * ET));
+    static_assert(bytes <= 227 * 1024, "a block's shared memory");
+    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes);
     if (rc) return rc;
     const dim3 grid(n_requests, a.H, (a.E + ET - 1) / ET);
-    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS), floats * sizeof(float), s, a);
+    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS), bytes, s, a);
     return cb_last_error();
 }
 
 template <int DP, int RULE>
 int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
     constexpr int P = DP + 4;
-    const size_t floats = (VECTOR_DECAY<RULE> ? 3 : 2) * CT * P + 2 * CT * AP + 2 * CT
-                          + (VECTOR_DECAY<RULE> ? (DP / 16) * 2 * CT * CT : 0);
-    int rc = allow_smem(chunk_local_kernel<DP, RULE>, floats * sizeof(float));
+    constexpr size_t bytes = sizeof(float) * ((VECTOR_DECAY<RULE> ? 3 : 2) * CT * P + 2 * CT * AP + 2 * CT
+                                              + (VECTOR_DECAY<RULE> ? (DP / 16) * (IS_DELTA<RULE> ? 2 : 1) * CT * CT : 0));
+    static_assert(bytes <= 227 * 1024, "a block's shared memory");
+    int rc = allow_smem(chunk_local_kernel<DP, RULE>, bytes);
     if (rc) return rc;
     const dim3 grid((max_new + CT - 1) / CT, a.H, n_requests);
-    cb_launch(chunk_local_kernel<DP, RULE>, grid, dim3(THREADS), floats * sizeof(float), s, a);
+    cb_launch(chunk_local_kernel<DP, RULE>, grid, dim3(THREADS), bytes, s, a);
     rc = cb_last_error();
     if (rc) return rc;
     return launch_walk<DP, RULE, 16>(a, n_requests, s);

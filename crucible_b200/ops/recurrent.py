@@ -7,11 +7,13 @@ import ctypes
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, build
+from . import LAUNCHES, KernelError, _c_float, _c_int, _c_void_p, _check, _code, _need_cuda, _ptr, _stream, build
 
 _c_long = ctypes.c_long
 DELTA, MLSTM, WKV, SSD, CHANNEL = 0, 1, 2, 3, 4
 GATE_SILU, GATE_SIGMOID = 0, 1
+CHUNKS = True                # tests switch it off to reach the token-by-token walk with the same inputs
+CHUNK_MIN_TOKENS = 128       # the longest portion from which a bfloat16 step's portions go in chunks
 
 
 def _state_args(state: torch.Tensor):
@@ -130,13 +132,40 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     if qkv.dtype != torch.float32 or out.dtype != torch.float32 or not qkv.is_contiguous():
         raise KernelError("matrix_memory takes prepared float32 rows")
     sp, stride = _state_args(state)
+    n, walked = ctx.n_requests, ctx.n_requests
+    starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
+    w_off_read = w_off if rule in (WKV, CHANNEL) else 0
+    if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.max_new_tokens >= CHUNK_MIN_TOKENS
+            and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0):
+        # prompts' portions in chunks; the requests at the head of the step that bring one token are walked
+        walked = ctx.host.lead_single
+        rows, f32 = qkv.shape[0], torch.float32
+
+        def room(name, width, wanted=True):
+            return ctx.scratch(f"memory.{name}", (rows, n_heads, width), f32) if wanted else None
+        own_q, delta, vector = rule in (DELTA, WKV, CHANNEL), rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
+        wq, ww, wk = room("wq", key_dim, own_q), room("ww", key_dim, delta), room("wk", key_dim, vector)
+        wu, ws = room("wu", value_dim, delta), room("ws", 4)
+        wg = ctx.scratch("memory.wg", (rows // 32 + n, n_heads, key_dim), f32) if vector else None
+        lib = build.load("recurrent_chunks")
+        _check(lib.cb_matrix_memory_chunks(
+            _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
+            _ptr(sc0), _ptr(sc1), _c_void_p(starts + 4 * walked), _c_void_p(slots + 4 * walked), sp, stride,
+            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(n - walked),
+            _c_int(ctx.host.max_new_tokens), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
+            _c_int(w_off), _ptr(per_head),
+            _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
+            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _stream()), "matrix_memory (chunks)")
+        LAUNCHES[0] += 1                 # (two kernels)
+    if walked == 0:
+        return
     lib = build.load("recurrent")
     _check(lib.cb_matrix_memory(
         _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
-        _ptr(sc0), _ptr(sc1), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride,
-        _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(ctx.n_requests),
+        _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,
+        _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(walked),
         _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim), _c_int(w_off),
-        _ptr(per_head), _ptr(kept), _stream()), "matrix_memory")
+        _ptr(per_head), _c_void_p(kept_at), _stream()), "matrix_memory")
 
 
 def head_norm_gate(o, gain, gain_per_head, gate, out, gate_kind, n_heads, value_dim, eps,

@@ -1,0 +1,165 @@
+"""The recurrences over prompts' portions in chunks of 32 tokens (`csrc/recurrent_chunks.cu`) against the
+same recurrences token by token in float64, for every rule: portions that end inside a chunk, at its
+edge and one token beyond it, a state carried in, heads and values that are no whole tiles, decays of 0
+and 1, requests of one token at the head of the step.  The operands are float32, so the error is that
+of float32 sums: the bound is eight times what the token-by-token kernel shows on the same operands (a
+chunk sums in another order, the triangular system included), and never below 2e-6."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LENGTHS = [(1, 128, 33), (1, 1, 161), (200,), (129, 31, 32)]
+
+
+def _i32(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+def _ctx(lengths, dtype):
+    starts = [0]
+    for n in lengths:
+        starts.append(starts[-1] + n)
+    lead = 0
+    while lead < len(lengths) and lengths[lead] == 1:
+        lead += 1
+    room = {}
+
+    def scratch(name, shape, kind):
+        room[name] = torch.full(tuple(shape), float("nan"), dtype=kind, device=DEV)
+        return room[name]
+    slots = list(range(len(lengths)))[::-1]
+    return SimpleNamespace(dtype=dtype, n_requests=len(lengths), req_row_start=_i32(starts), req_state_slot=_i32(slots),
+                           scratch=scratch, host=SimpleNamespace(max_new_tokens=max(lengths), lead_single=lead)), starts, slots
+
+
+def _operands(rule, k, T, H, G, D, E, g):
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, kk = (torch.randn(T, G, D, generator=g) for _ in range(2))
+    v = torch.randn(T, H, E, generator=g)
+    w = sc0 = sc1 = per_head = None
+    decay = torch.rand(T, H, generator=g) ** 0.1
+    decay[3::29] = 0.0
+    decay[5::31] = 1.0
+    if rule in (k.DELTA, k.CHANNEL):
+        q, kk, sc1 = unit(q) * D ** -0.5, unit(kk), torch.rand(T, H, generator=g)
+        sc0 = decay
+    if rule == k.SSD:
+        sc0, sc1, per_head = decay, torch.rand(T, H, generator=g), torch.randn(H, generator=g)
+    if rule == k.MLSTM:
+        q = q * D ** -0.5
+        sc0 = torch.nn.functional.logsigmoid(torch.randn(T, H, generator=g) * 3.0)
+        sc1 = torch.randn(T, H, generator=g) * 4.0
+    if rule in (k.WKV, k.CHANNEL):
+        w = torch.rand(T, H, D, generator=g) ** 0.2
+        w[:, :, 0], w[:, :, 1] = 1.0, 0.0
+    if rule == k.WKV:
+        per_head = torch.randn(H, D, generator=g)
+    return q, kk, v, w, sc0, sc1, per_head
+
+
+def _walk(rule, k, q, kk, v, w, sc0, sc1, per_head, S, n, m):
+    """One request's tokens in float64."""
+    H, out = v.shape[1], torch.zeros(v.shape, dtype=torch.float64)
+    rep = H // q.shape[1]
+    q, kk, v = q.double().repeat_interleave(rep, 1), kk.double().repeat_interleave(rep, 1), v.double()
+    for t in range(q.shape[0]):
+        if rule == k.MLSTM:
+            f, i = sc0[t].double(), sc1[t].double()
+            m_new = torch.maximum(f + m, i)
+            a, b = torch.exp(f + m - m_new), torch.exp(i - m_new)
+            S = a[:, None, None] * S + (b[:, None] * kk[t])[:, :, None] * v[t][:, None]
+            n, m = a[:, None] * n + b[:, None] * kk[t], m_new
+            low = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+            out[t] = torch.einsum("hde,hd->he", S, q[t]) / low[:, None]
+            continue
+        kv = kk[t][:, :, None] * v[t][:, None]
+        if rule == k.WKV:
+            out[t] = torch.einsum("hde,hd->he", S + per_head.double()[:, :, None] * kv, q[t])
+            S = w[t].double()[:, :, None] * S + kv
+            continue
+        S = (w[t].double()[:, :, None] if rule == k.CHANNEL else sc0[t].double()[:, None, None]) * S
+        if rule == k.SSD:
+            S = S + sc1[t].double()[:, None, None] * kv
+            out[t] = torch.einsum("hde,hd->he", S, q[t]) + per_head.double()[:, None] * v[t]
+        else:
+            u = sc1[t].double()[:, None] * (v[t] - torch.einsum("hde,hd->he", S, kk[t]))
+            S = S + kk[t][:, :, None] * u[:, None]
+            out[t] = torch.einsum("hde,hd->he", S, q[t])
+    return out, S, n, m
+
+
+@pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
+@pytest.mark.parametrize("H,G,D,E", [(4, 2, 128, 128), (2, 1, 64, 64), (3, 3, 20, 20), (2, 2, 100, 100)])
+def test_chunks_agree_with_float64(rule, H, G, D, E):
+    from crucible_b200.ops import recurrent as k
+    rule_code = getattr(k, rule)
+    if rule in ("MLSTM", "WKV"):
+        G = H
+    elif (H, D) == (4, 128):
+        E = 40                                    # values unlike keys, no whole tiles
+    for lengths in LENGTHS:
+        g = torch.Generator().manual_seed(len(lengths) + D)
+        T, R = sum(lengths), len(lengths)
+        q, kk, v, w, sc0, sc1, per_head = _operands(rule_code, k, T, H, G, D, E, g)
+        parts = [q.reshape(T, -1), kk.reshape(T, -1), v.reshape(T, -1)] + ([w.reshape(T, -1)] if w is not None else [])
+        qkv = torch.cat(parts, 1).contiguous().to(DEV)
+        offs = (0, G * D, 2 * G * D)
+        sizes = (H * D * E, H * D, -(-H // 4) * 4)
+        before = torch.randn(R, sum(sizes), generator=g) * 0.3
+        results = {}
+        for chunks in (True, False):
+            ctx, starts, slots = _ctx(lengths, torch.bfloat16)
+            state = torch.zeros(R, 4 * sum(sizes), dtype=torch.uint8, device=DEV)
+            state.view(torch.float32)[slots] = before.to(DEV)
+            out = torch.full((T, H * E), float("nan"), device=DEV)
+            k.CHUNKS = chunks
+            try:
+                k.matrix_memory(rule_code, qkv, *offs, *(x.contiguous().to(DEV) if x is not None else None for x in (sc0, sc1)),
+                                ctx, state, 0, 4 * sizes[0], 4 * (sizes[0] + sizes[1]), out, H, G, D, E,
+                                w_off=2 * G * D + H * E, per_head=per_head.to(DEV).contiguous() if per_head is not None else None)
+            finally:
+                k.CHUNKS = True
+            results[chunks] = out.cpu().view(T, H, E), state.view(torch.float32)[slots].cpu()
+        for r in range(R):
+            a, b = starts[r], starts[r + 1]
+            cut = [x[a:b] if x is not None else None for x in (q, kk, v, w, sc0, sc1)]
+            S0 = before[r, :sizes[0]].double().view(H, D, E)
+            n0, m0 = before[r, sizes[0]:sizes[0] + sizes[1]].double().view(H, D), before[r, sum(sizes[:2]):][:H].double()
+            want, S, n, m = _walk(rule_code, k, *cut, per_head, S0, n0, m0)
+            errors = {}
+            for chunks, (out, state) in results.items():
+                off = [float((out[a:b].double() - want).norm() / want.norm()),
+                       float((state[r, :sizes[0]].double().view(H, D, E) - S).norm() / S.norm())]
+                if rule == "MLSTM":
+                    off.append(float((state[r, sizes[0]:sizes[0] + sizes[1]].double().view(H, D) - n).norm() / n.norm()))
+                    off.append(float((state[r, sum(sizes[:2]):][:H].double() - m).abs().max()) / max(1.0, float(m.abs().max())))
+                errors[chunks] = off
+            for got, plain in zip(errors[True], errors[False]):
+                assert got <= max(8 * plain, 2e-6), (rule, lengths, r, errors)
+
+
+@pytest.mark.parametrize("rule", ["DELTA", "CHANNEL", "SSD", "WKV", "MLSTM"])
+def test_a_later_token_does_not_reach_an_earlier_one(rule):
+    """A value that is not a number stays with its own and later tokens of its own request."""
+    from crucible_b200.ops import recurrent as k
+    code, H, D, lengths, at = getattr(k, rule), 2, 64, (140, 130), 45
+    g = torch.Generator().manual_seed(2)
+    T = sum(lengths)
+    q, kk, v, w, sc0, sc1, per_head = _operands(code, k, T, H, H, D, D, g)
+    outs = []
+    for bad in (False, True):
+        if bad:
+            v[at], kk[at], q[at] = float("nan"), float("inf"), float("nan")
+        qkv = torch.cat([x.reshape(T, -1) for x in (q, kk, v, w) if x is not None], 1).contiguous().to(DEV)
+        ctx, _, _ = _ctx(lengths, torch.bfloat16)
+        state = torch.zeros(2, 4 * (H * D * D + H * D + 4), dtype=torch.uint8, device=DEV)
+        out = torch.empty(T, H * D, device=DEV)
+        k.matrix_memory(code, qkv, 0, H * D, 2 * H * D, *(x.contiguous().to(DEV) if x is not None else None for x in (sc0, sc1)),
+                        ctx, state, 0, 4 * H * D * D, 4 * (H * D * D + H * D), out, H, H, D, D, w_off=3 * H * D,
+                        per_head=per_head.to(DEV).contiguous() if per_head is not None else None)
+        outs.append(out.cpu())
+    assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][lengths[0]:], outs[1][lengths[0]:])
+    assert bool(torch.isnan(outs[1][at]).any())

@@ -29,7 +29,13 @@
 // sum uses the same reference, and the final division makes the result the
 // exact softmax-weighted mean whatever the reference was.
 //
-// Sizes: head size 64 or 128; page size a power of two from 8 to 128; any head
+// Rows of 256 features that are keys and values at once (a latent with its rotated part: one
+// key head for all query heads): a stage holds the tile once, 64 KB; the first product reads it
+// with the features contracted, the second with the keys contracted.  A tile's 2 x 128 x 128 x 256
+// multiply-adds are 2,048 cycles of the tensor pipe, about what the softmax beside them takes.  A
+// 2,048-token prompt of 16 heads: 441 us on the mma.sync tiles, 85 here (34 GFLOP: 400 TFLOP/s).
+//
+// Sizes: head size 64 or 128, or 256 if the pages' rows are keys and values at once; page size a power of two from 8 to 128; any head
 // counts and group sizes; window.  Anything else is refused and the mma.sync
 // kernel runs.  Every wait is bounded (tc_common.cuh).
 // Reference counterpart: `attention_prefill_exact_*`
@@ -90,27 +96,28 @@ __device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits
 // beside this tile's softmax.  It was the right one for launches with more blocks than places
 // while the roomy form had one softmax group (4,096-token prompt of the 120M shape 1.84 against
 // 2.01 ms); with two groups the roomy form is quicker there too (1.68 ms) and the launcher
-// takes it unless told otherwise.  Head size 128: two stages and one P buffer (what 227 KB hold).
+// takes it unless told otherwise.  Head size 128, and 256 with one operand for both products: two stages
+// and one P buffer (what 227 KB hold).
 template <int HD, bool LEAN>
 struct Storage {
     static constexpr int STAGES = (HD == 64 && !LEAN) ? 4 : 2;
     static constexpr int PB = (HD == 64 && !LEAN) ? 2 : 1;
     static constexpr int S_BUFS = LEAN ? 1 : 2;
+    static constexpr int OPERANDS = HD == 256 ? 1 : 2;      // keys and values, or rows that are both
     // softmax groups of four warps that take the tiles in turn (tile j: group j % GROUPS), each
     // with its own reference maximum, sum and accumulator, merged at the end
     static constexpr int GROUPS = (HD == 64 && !LEAN) ? 2 : 1;
     // loader, MMA thread, four softmax warps a group; two groups: a warp for a second MMA thread
     static constexpr int THREADS = GROUPS > 1 ? 64 + 128 * GROUPS + 32 : 192;
     alignas(1024) uint8_t q[HD / 64][ROWS * 64 * 2];
-    alignas(1024) uint8_t k[STAGES][HD / 64][KEYS * 64 * 2];
-    alignas(1024) uint8_t v[STAGES][HD / 64][KEYS * 64 * 2];
+    alignas(1024) uint8_t kv[STAGES][OPERANDS][HD / 64][KEYS * 64 * 2];
     alignas(1024) uint8_t p[PB][2][ROWS * 64 * 2];  // P: buffers of two halves of 64 keys
     alignas(8) uint64_t kv_full[STAGES];
     uint64_t kv_empty[STAGES];
     uint64_t s_full[2], p_full[2], pv_done[2];
     uint64_t s_free;                                // lean form: a tile's scores are in registers
     uint64_t s_taken[2];                            // two groups: buffer b's scores are in registers
-    float2 merge[2][ROWS];                          // two groups: a row's (reference, sum) of each
+    float2 merge[GROUPS > 1 ? 2 : 1][ROWS];         // two groups: a row's (reference, sum) of each
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -164,6 +171,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     using Store = Storage<HD, LEAN>;
     constexpr int STAGES = Store::STAGES, PB = Store::PB, NH = HD / 64, S_BUFS = Store::S_BUFS;
+    constexpr int VALUES = Store::OPERANDS - 1;      // where a stage's values are
     constexpr int GROUPS = Store::GROUPS;
     constexpr int PV_WARP = GROUPS > 1 ? 2 + 4 * GROUPS : -1;    // the second MMA thread's warp
     static_assert(GROUPS == 1 || (PB == 2 && S_BUFS == 2 && HD == 64), "two groups: a buffer of scores, of P and an accumulator each");
@@ -261,12 +269,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
             return false;
         }
-        tc::mbar_expect_tx(&s.kv_full[st], 2 * KEYS * HD * 2);
+        tc::mbar_expect_tx(&s.kv_full[st], Store::OPERANDS * KEYS * HD * 2);
         if (run) {
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
-                tc::tma_load_4d(s.k[st][h], &run_k, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
-                tc::tma_load_4d(s.v[st][h], &run_v, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
+                tc::tma_load_4d(s.kv[st][0][h], &run_k, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
+                if (VALUES) tc::tma_load_4d(s.kv[st][VALUES][h], &run_v, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
             }
             return true;
         }
@@ -277,8 +285,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 const int y = (pages[i] * p.n_kv_heads + kv_head) << p.page_shift;
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
-                    tc::tma_load_2d(s.k[st][h] + dst, &map_k, &s.kv_full[st], h * 64, y);
-                    tc::tma_load_2d(s.v[st][h] + dst, &map_v, &s.kv_full[st], h * 64, y);
+                    tc::tma_load_2d(s.kv[st][0][h] + dst, &map_k, &s.kv_full[st], h * 64, y);
+                    if (VALUES) tc::tma_load_2d(s.kv[st][VALUES][h] + dst, &map_v, &s.kv_full[st], h * 64, y);
                 }
             }
         }
@@ -353,7 +361,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         // product wait for the other.
         if (lane == 0 && n_tiles > 0) {
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(ROWS, KEYS);
-            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, 64);
+            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, HD);
             // Operand descriptors by addition: the low word carries the address in 16-byte
             // units, the high word is the same for every tile; stages and parities are carried
             // along.  This thread's own instructions are what a tile's MMAs take (sending one
@@ -361,12 +369,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             const uint64_t q_desc0 = tc::smem_desc_sw128(tc::smem_u32(s.q[0]));
             const uint32_t desc_hi = (uint32_t)(q_desc0 >> 32);
             const uint32_t q_lo = (uint32_t)q_desc0;
-            const uint32_t k_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.k[0][0]));
-            const uint32_t v_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.v[0][0]));
+            const uint32_t k_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.kv[0][0][0]));
             const uint32_t p_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.p[0][0]));
-            constexpr uint32_t Q_HALF = sizeof(s.q[0]) >> 4, KV_HALF = sizeof(s.k[0][0]) >> 4,
-                               KV_STAGE = sizeof(s.k[0]) >> 4, P_HALF = sizeof(s.p[0][0]) >> 4,
+            constexpr uint32_t Q_HALF = sizeof(s.q[0]) >> 4, KV_HALF = sizeof(s.kv[0][0][0]) >> 4,
+                               KV_STAGE = sizeof(s.kv[0]) >> 4, P_HALF = sizeof(s.p[0][0]) >> 4,
                                P_BUF = sizeof(s.p[0]) >> 4;
+            // the values, all features in one instruction: 64 of them lie together, the next 64 a
+            // leading offset of KV_HALF on
+            const uint32_t v_lo0 = ((uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.kv[0][VALUES][0])) & 0xFFFFu) |
+                                   (KV_HALF << 16);
             bool ok = true;
             // S_j = Q K_j^T into buffer j % S_BUFS: the head size in steps of 16
             int qk_st = 0;                        // stage and parity of the next tile of scores
@@ -399,25 +410,22 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 send_qk(j);
                 return true;
             };
-            // O += P_j V_j: 128 keys in eight steps of 16, 64 output features at a time
+            // O += P_j V_j: 128 keys in eight steps of 16
             int st = 0;                           // stage of the next tile's values
             auto send_pv = [&](int j) {
                 const int pb = j % PB;
                 tc::tc_fence_after_sync();
                 const uint32_t p_lo = p_lo0 + pb * P_BUF;
+                const uint32_t v_lo = v_lo0 + st * KV_STAGE;
+                // (two groups: head size 64; a group's accumulator is 64 columns on)
+                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(j % GROUPS) * 64 : 0u);
 #pragma unroll
-                for (int h = 0; h < NH; ++h) {
-                    const uint32_t v_lo = v_lo0 + st * KV_STAGE + h * KV_HALF;
-                    // (two groups: head size 64, so h is 0; a group's accumulator is 64 columns on)
-                    const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(j % GROUPS) * 64 : (uint32_t)h * 64);
-#pragma unroll
-                    for (int k = 0; k < KEYS / 16; ++k) {
-                        // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
-                        const uint64_t p_desc = tc::desc_of(p_lo + (k >> 2) * P_HALF + 2 * (k & 3), desc_hi);
-                        const uint64_t v_desc = tc::desc_of(v_lo + 128 * k, desc_hi);
-                        if (k == 0) tc::umma_bf16(d_o, p_desc, v_desc, idesc_pv, j >= GROUPS ? 1u : 0u);
-                        else tc::umma_bf16_add(d_o, p_desc, v_desc, idesc_pv);
-                    }
+                for (int k = 0; k < KEYS / 16; ++k) {
+                    // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
+                    const uint64_t p_desc = tc::desc_of(p_lo + (k >> 2) * P_HALF + 2 * (k & 3), desc_hi);
+                    const uint64_t v_desc = tc::desc_of(v_lo + 128 * k, desc_hi);
+                    if (k == 0) tc::umma_bf16(d_o, p_desc, v_desc, idesc_pv, j >= GROUPS ? 1u : 0u);
+                    else tc::umma_bf16_add(d_o, p_desc, v_desc, idesc_pv);
                 }
                 tc::umma_commit(&s.kv_empty[st]);
                 tc::umma_commit(&s.pv_done[pb]);
@@ -712,7 +720,8 @@ int launch_as(dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorM
 }  // namespace
 
 // Attention for the rows of a step whose requests bring portions of prompts.
-// k_cache / v_cache: [n_pages][n_kv_heads][page_tokens][head_dim] bf16; head_dim 64 or 128.
+// k_cache / v_cache: [n_pages][n_kv_heads][page_tokens][head_dim] bf16; head_dim 64 or 128, or 256 where
+// both are the same rows.
 // keep_first (with a window): a row at position p reads j <= p with p - j < window or j < keep_first.
 // chunked: `window` is a chunk's size (first_key).  sinks: [n_heads] or null.  Results times out_scale.
 // gate: null, or logits laid out like `out`, rows of 16-byte pieces: results times their sigmoids.
@@ -726,7 +735,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
                                         int lean, int* status, void* stream) {
     if (n_requests <= 0 || max_new_tokens <= 0) return 0;
     if (keep_first < 0 || !(scale > 0.f)) return CB_ERR_UNSUPPORTED;
-    if ((head_dim != 64 && head_dim != 128) || n_heads % n_kv_heads != 0 || page_tokens < 8 || page_tokens > KEYS ||
+    if ((head_dim != 64 && head_dim != 128 && !(head_dim == 256 && k_cache == v_cache)) || n_heads % n_kv_heads != 0 || page_tokens < 8 || page_tokens > KEYS ||
         (page_tokens & (page_tokens - 1)) || (qkv_stride & 7) || (out_stride & 7) ||
         ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || ((uintptr_t)k_cache & 15) ||
         ((uintptr_t)v_cache & 15) || ((uintptr_t)gate & 15) || (gate != nullptr && (gate_stride & 7)))
@@ -782,6 +791,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     if (head_dim == 64)
         return lean ? launch_as<64, true>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p)
                     : launch_as<64, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
+    if (head_dim == 256) return launch_as<256, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
     return launch_as<128, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
 }
 

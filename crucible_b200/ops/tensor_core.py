@@ -493,10 +493,16 @@ class _Requests:
         self.count, self.max_new, self.bucket, self.rows_end = count, max_new, bucket, rows_end
 
 
+def _tcgen05_rows(head_dim, k_cache, v_cache) -> bool:
+    """Head sizes the tcgen05 prompt attention takes: 64 and 128, and 256 where a cached row is key and
+    value at once."""
+    return head_dim in (64, 128) or (head_dim == 256 and k_cache.data_ptr() == v_cache.data_ptr())
+
+
 def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale,
                        window, cache, keep_first: int = 0, chunked: bool = False, sinks=None, out_scale: float = 1.0,
                        gate=None) -> bool:
-    """tcgen05 attention for portions of prompts: head size 64 or 128, page size a
+    """tcgen05 attention for portions of prompts: head sizes of `_tcgen05_rows`, page size a
     power of two from 8 to 128.  `keep_first` (with a window): keys before that position stay
     visible.  `chunked`: the window is a chunk's size.  `sinks`: float32 per query head or None.
     `gate`: rows laid out like `out` whose sigmoids the results are multiplied by, or None.
@@ -622,13 +628,14 @@ def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, sc
                      ctx, cache, table, chunked: bool = False, sinks=None, out_scale: float = 1.0,
                      gate=None) -> bool:
     """The tcgen05 attention for a step that holds portions of prompts only (no single decoded
-    tokens ahead of them) over keys and values of one size, 64 or 128, with a window that may
+    tokens ahead of them) over keys and values of one size (`_tcgen05_rows`), with a window that may
     keep the first tokens or (`chunked`) is the size of chunks, and with a sink per head in the
     softmax (`sinks`) or none; `gate`: a logit for every result, or None.  `q`: rows of n_heads * head_dim.  False: not taken."""
     host = getattr(ctx, "host", None)
     n_rep = n_heads // n_kv_heads
-    if (not USE_TCGEN05_ATTENTION or host is None or q.dtype != torch.bfloat16 or head_dim not in (64, 128)
-            or k_cache.dtype != torch.bfloat16 or host.lead_single != 0 or host.max_new_tokens * n_rep < 64
+    if (not USE_TCGEN05_ATTENTION or host is None or q.dtype != torch.bfloat16
+            or not _tcgen05_rows(head_dim, k_cache, v_cache) or k_cache.dtype != torch.bfloat16
+            or host.lead_single != 0 or host.max_new_tokens * n_rep < 64
             or q.stride(0) % 8 or out.stride(0) % 8 or q.data_ptr() % 16 or out.data_ptr() % 16
             or (gate is not None and (gate.dtype != q.dtype or gate.stride(0) % 8 or gate.data_ptr() % 16))
             or k_cache.shape[-1] != head_dim or v_cache.shape[-1] != head_dim):
@@ -668,7 +675,7 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
                                           head_dim, scale, window, cache, partial, counters,
                                           n_chunks, chunk_keys)):
         return True
-    if (USE_TCGEN05_ATTENTION and not split and head_dim in (64, 128)
+    if (USE_TCGEN05_ATTENTION and not split and _tcgen05_rows(head_dim, k_cache, v_cache)
             and reqs.max_new * n_rep >= 64 and out.stride(0) % 8 == 0
             and _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads,
                                    head_dim, scale, window, cache)):

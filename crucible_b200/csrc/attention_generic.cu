@@ -5,7 +5,8 @@
 // table (lo = 0, or p - window + 1).  The result for a row depends only on that
 // row's query and its keys, never on the rest of the batch.
 //
-// This is the attention of the 32-bit path, and the refuge of the bfloat16 path
+// This is the refuge of both paths: of the 32-bit one for sizes that its tiles refuse
+// (attention_f32.cu: no multiples of 4, more than 256 features), of the bfloat16 one
 // for head sizes or options its tensor-core kernels refuse.
 // Reference counterparts: `attention_decode_paged_f32`
 // (engine/kernels/kernels.cu:1741-1839) and `attention_prefill_paged_impl`

@@ -473,11 +473,39 @@ def rope_kv_append(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: i
         _stream()), "rope_kv_append")
 
 
+F32_TILES = True          # tests switch it off to reach the one-warp-a-row kernels with the same inputs
+
+
+def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
+                  chunked, keep_first, out_scale, ctx, page_tokens, table, gate_per_head=False) -> bool:
+    """The 32-bit attention over tiles of keys (`csrc/attention_f32.cu`): float32 rows of sizes up to 256
+    that are multiples of 4.  A rule of the sizes alone, so that a row's bits never depend on the
+    step.  False: not taken."""
+    host = getattr(ctx, "host", None)
+    tensors = (q, out, k_cache, v_cache)
+    if (not F32_TILES or host is None or any(t.dtype != torch.float32 for t in tensors)
+            or max(key_dim, value_dim) > 256 or (key_dim | value_dim | q.stride(0) | out.stride(0)) % 4
+            or any(t.data_ptr() % 16 for t in tensors) or (gate is not None and gate.dtype != torch.float32)):
+        return False
+    lib = build.load("attention_f32")
+    _check(lib.cb_attention_f32(
+        _ptr(q), _c_int(q.stride(0)), _ptr(gate), _c_int(gate.stride(0) if gate is not None else 0), _ptr(out),
+        _c_int(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(sinks), _ptr(ctx.req_row_start),
+        _ptr(ctx.req_first_pos), _ptr(table), _c_int(table.shape[1]), _c_int(ctx.n_requests),
+        _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim), _c_int(value_dim),
+        _c_int(page_tokens), _c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first),
+        _c_float(out_scale), _c_int(1 if gate_per_head else 0), _stream()), "attention (32-bit tiles)")
+    return True
+
+
 def paged_attention_plain(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx, cache,
                           binding) -> None:
     _need_cuda(qkv, out)
     k_cache, v_cache = cache.keys(binding.slot), cache.values(binding.slot)
     table = ctx.block_table(binding.group)
+    if attention_f32(qkv, None, out, k_cache, v_cache, None, n_heads, n_kv_heads, head_dim, head_dim, scale, window,
+                     False, 0, 1.0, ctx, cache.page_tokens, table):
+        return
     lib = build.load("attention_generic")
     _check(lib.cb_attention_generic(
         _ptr(qkv), _c_int(qkv.stride(0)), _ptr(out), _c_int(out.stride(0)), _ptr(k_cache),

@@ -41,6 +41,7 @@ MODULES: Dict[str, List[str]] = {
     "elementwise": ["common.cuh"],
     "gemm_simt": ["common.cuh"],
     "attention_generic": ["common.cuh"],
+    "attention_f32": ["common.cuh"],
     "sampling": ["common.cuh", "no_alloc_argmax.h"],
     "streams": ["common.cuh"],
     "sink_attention": ["common.cuh"],

@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, build
+from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, attention_f32, build
 
 
 def rotate_norm_append(proj: torch.Tensor, freq: Optional[torch.Tensor], rotary_dim: int,
@@ -98,6 +98,9 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor,
         raise KernelError("sink attention: the gate's logits are rows of the queries' dtype")
     if _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                      keep_first, out_scale, ctx, cache, k_cache, v_cache, table, gate_per_head, chunked):
+        return
+    if attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
+                     chunked, keep_first if window else 0, out_scale, ctx, cache.page_tokens, table, gate_per_head):
         return
     lib = build.load("sink_attention")
     _check(lib.cb_sink_attention(

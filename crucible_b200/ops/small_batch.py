@@ -19,7 +19,7 @@ from typing import Optional, Union
 
 import torch
 
-from . import build
+from . import _stream, build
 
 build.register_module("decode_small", ["common.cuh"])
 
@@ -59,10 +59,6 @@ def as_tensor(h: Rows) -> torch.Tensor:
 
 def _ptr(t):
     return _c_void_p(0 if t is None else t.data_ptr())
-
-
-def _stream():
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _input(h: Rows, w: torch.Tensor):

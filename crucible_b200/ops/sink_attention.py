@@ -118,49 +118,54 @@ TENSOR_CORES = True      # tests switch it off to reach the plain kernel with th
 def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                   keep_first, out_scale, ctx, cache, k_cache, v_cache, table, gate_per_head=False,
                   chunked=False) -> bool:
-    """For bfloat16 rows: steps of prompts' portions alone whose keys and values have one size, 64
-    or 128, take the tcgen05 attention (`csrc/attention_tcgen05.cu`);
-    everything else of key and value sizes that are multiples of 16 up to 256 the mma.sync kernel of 64-row
-    tiles (`csrc/attention_mma.cu`, its extended form): prompts' portions and decoded tokens in
-    one launch, the rows of a request's query heads that share a key/value head packed into
-    tiles.  Refuses anything else."""
+    """For bfloat16 rows.  A step that holds a portion whose keys and values have one size that the
+    tcgen05 attention takes goes there (`csrc/attention_tcgen05.cu`), the single decoded tokens at its
+    head with it or in a launch of their own (`tensor_core.tiles_first`); everything else is the mma.sync
+    kernel of 64-row tiles (`csrc/attention_mma.cu`, its extended form; key and value sizes that are
+    multiples of 16 up to 256), the rows of a request's query heads that share a key/value head packed
+    into tiles.  Refuses anything else.  (A token each of 24 requests beside a portion of 509, 16 heads of
+    128, window 1,024: the attention 84 us on the mma.sync tiles, 45 here.)"""
     host = getattr(ctx, "host", None)
     if (not TENSOR_CORES or q.dtype != torch.bfloat16 or key_dim % 16 or value_dim % 16
             or key_dim > 256 or value_dim > 256 or host is None or q.stride(0) % 8 or out.stride(0) % 2
             or (gate is not None and not gate_per_head and gate.stride(0) % 2)):
         return False
     from . import tensor_core
-    # keys and values of 64 or 128 features, portions of prompts only: the tcgen05 attention, whose
-    # tiles take the kept first tokens ahead of the window's
-    if (key_dim == value_dim
-            and tensor_core.prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, key_dim, scale,
-                                             window, keep_first, ctx, cache, table, chunked=chunked, sinks=sinks,
-                                             out_scale=out_scale,
-                                             gate=None if gate_per_head else gate)):
+    first = ctx.n_requests
+    if key_dim == value_dim:
+        first = tensor_core.prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, key_dim, scale, window,
+                                             keep_first, ctx, cache, table, chunked=chunked, sinks=sinks,
+                                             out_scale=out_scale, gate=None if gate_per_head else gate)
+    if first < ctx.n_requests:
         if gate is not None and gate_per_head:
-            # one logit a head: a pass over the heads' results behind the attention
+            # one logit a head: a pass over the heads' results behind the attention (the requests
+            # before `first` bring a row each)
             from . import latent
-            latent.head_gate(out, gate, n_heads, value_dim)
-        return True
+            latent.head_gate(out[first:], gate[first:], n_heads, value_dim)
+        if first == 0:
+            return True
+        count, max_new, bucket = first, 1, host.lead_context_bucket
+    else:
+        count, max_new, bucket = ctx.n_requests, host.max_new_tokens, host.context_bucket
     lib = build.load("attention_mma")
     # Few rows per request (decoded tokens, short portions): one row tile each, so the blocks
     # are few; the key tiles are then dealt to several blocks and merged.  The number of shares
     # is a function of the step's shape; any number gives the same sums up to rounding.
-    max_rows = host.max_new_tokens * (n_heads // n_kv_heads)
+    max_rows = max_new * (n_heads // n_kv_heads)
     n_chunks, partial = 1, None
     if max_rows <= 64:
-        reach = host.context_bucket if window is None else min(window + 64, host.context_bucket)
+        reach = bucket if window is None else min(window + 64, bucket)
         tiles = -(-reach // 64) + (-(-keep_first // 64) if window is not None else 0)
-        n_chunks = max(1, min(tiles // 2, 296 // max(1, n_kv_heads * ctx.n_requests), 32))
+        n_chunks = max(1, min(tiles // 2, 296 // max(1, n_kv_heads * count), 32))
         if n_chunks > 1:
             partial = ctx.scratch("sink_attention.partial",
-                                  (ctx.n_requests * n_kv_heads * n_chunks * max_rows * (value_dim + 2),),
+                                  (count * n_kv_heads * n_chunks * max_rows * (value_dim + 2),),
                                   torch.float32)
     code = lib.cb_attention_mma_sink(
         _ptr(q), _c_int(q.stride(0)), _ptr(out), _c_int(out.stride(0)), _ptr(gate),
         _c_int(gate.stride(0) if gate is not None else 0), _ptr(k_cache), _ptr(v_cache), _ptr(sinks),
         _ptr(ctx.req_row_start), _ptr(ctx.req_first_pos), _ptr(table), _c_int(table.shape[1]),
-        _c_int(ctx.n_requests), _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(n_kv_heads),
+        _c_int(count), _c_int(max_new), _c_int(n_heads), _c_int(n_kv_heads),
         _c_int(key_dim), _c_int(value_dim), _c_int(cache.page_tokens), _c_float(scale), _c_int(window or 0),
         _c_int(1 if chunked else 0), _c_int(keep_first), _c_float(out_scale), _ptr(partial), _c_int(n_chunks),
         _c_int(1 if gate_per_head else 0), _stream())

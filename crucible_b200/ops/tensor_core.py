@@ -14,7 +14,7 @@ import os
 
 import torch
 
-from . import build
+from . import _stream, build
 
 build.register_module("gemm_tcgen05", ["common.cuh", "tc_common.cuh"])
 build.register_module("attention_mma", ["common.cuh"])
@@ -88,10 +88,6 @@ def _count(n: int) -> None:
     if TIMER[0] is not None:
         import sys
         _tick("tensor cores: " + sys._getframe(1).f_code.co_name)
-
-
-def _stream():
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 TILE_WIDTHS = (64, 96, 128, 160, 192, 256)
@@ -624,25 +620,47 @@ def wide_row_chunk_keys(blocks_per_chunk: int, context_bucket: int, window) -> i
     return min(max(chunk, unit), whole)
 
 
+def tiles_first(host, n_requests, head_dim, window, keep_first) -> int:
+    """The first request of a step that the tcgen05 tiles take (`n_requests`: none): 0, or behind the
+    single decoded tokens at its head, which the caller then runs with their keys dealt to several
+    blocks.  A decoded token is a block of 128 rows like another in the tiles' launch and walks its keys
+    alone, 2 us a tile of 128 keys of 128 features: it rides along while that is not much longer than
+    the launch is anyway (16 heads of 128, 24 decoded tokens: behind 2,000 keys beside 100 prompt tokens
+    101 us a layer in two launches, 78 in one; 4 behind 3,000 keys 72 in two, 88 in one)."""
+    lead = host.lead_single
+    if lead == 0 or lead == n_requests:
+        return lead
+    reach = host.lead_context_bucket
+    if window is not None:
+        reach = min(reach, window + 128 + (keep_first or 0))
+    return 0 if reach * head_dim <= MIXED_REACH else lead
+
+
+MIXED_REACH = 2560 * 128     # keys times features
+
+
 def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, scale, window, keep_first,
                      ctx, cache, table, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                     gate=None) -> bool:
-    """The tcgen05 attention for a step that holds portions of prompts only (no single decoded
-    tokens ahead of them) over keys and values of one size (`_tcgen05_rows`), with a window that may
-    keep the first tokens or (`chunked`) is the size of chunks, and with a sink per head in the
-    softmax (`sinks`) or none; `gate`: a logit for every result, or None.  `q`: rows of n_heads * head_dim.  False: not taken."""
-    host = getattr(ctx, "host", None)
+                     gate=None) -> int:
+    """The tcgen05 attention for the requests of a step from `tiles_first` on, over keys and values of
+    one size (`_tcgen05_rows`), with a window that may keep the first tokens or (`chunked`) is the size of
+    chunks, and with a sink per head in the softmax (`sinks`) or none; `gate`: a logit for every result, or
+    None.  `q`: rows of n_heads * head_dim.  Returns the first request taken (`ctx.n_requests`: none)."""
+    host, none = getattr(ctx, "host", None), ctx.n_requests
     n_rep = n_heads // n_kv_heads
     if (not USE_TCGEN05_ATTENTION or host is None or q.dtype != torch.bfloat16
             or not _tcgen05_rows(head_dim, k_cache, v_cache) or k_cache.dtype != torch.bfloat16
-            or host.lead_single != 0 or host.max_new_tokens * n_rep < 64
             or q.stride(0) % 8 or out.stride(0) % 8 or q.data_ptr() % 16 or out.data_ptr() % 16
             or (gate is not None and (gate.dtype != q.dtype or gate.stride(0) % 8 or gate.data_ptr() % 16))
             or k_cache.shape[-1] != head_dim or v_cache.shape[-1] != head_dim):
-        return False
-    reqs = _Requests(ctx, table, 0, ctx.n_requests, host.max_new_tokens, host.context_bucket, ctx.n_tokens)
-    return _attention_tcgen05(q, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, cache,
-                              keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate)
+        return none
+    first = tiles_first(host, none, head_dim, window, keep_first)
+    if first == none or host.max_new_tokens * n_rep < 64:
+        return none
+    reqs = _Requests(ctx, table, first, none - first, host.max_new_tokens, host.context_bucket, ctx.n_tokens)
+    taken = _attention_tcgen05(q, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, cache,
+                               keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate)
+    return first if taken else none
 
 
 SPLIT_ROWS = 16          # packed rows (new tokens x heads of a group) the split form takes

@@ -1,0 +1,65 @@
+"""A step of decoded tokens beside a prompt's portion on the tcgen05 attention, the decoded tokens with it
+or in a launch of their own: every row against the CUDA-core kernel on the same inputs."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _i32(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("H,G,D,window,keep,chunked,gate", [
+    (8, 2, 128, 100, 8, False, "element"), (4, 4, 64, None, 0, False, "head"), (6, 2, 64, 96, 0, True, None),
+    (16, 1, 256, None, 0, False, None)])            # the last: rows that are keys and values at once
+@pytest.mark.parametrize("apart", [False, True])
+@pytest.mark.parametrize("singles,portion", [([200], 65), ([1, 130, 257], 64), ([60] * 20, 130)])
+def test_decoded_tokens_beside_a_portion(H, G, D, window, keep, chunked, gate, singles, portion, apart,
+                                          monkeypatch):
+    from crucible_b200.engine.context import HostStep
+    from crucible_b200.ops import sink_attention, tensor_core
+    g = torch.Generator().manual_seed(H + len(singles))
+    contexts, page = singles + [portion + 37], 16
+    per = -(-max(contexts) // page)
+    R = len(contexts)
+    table = torch.randperm(R * per, generator=g).to(torch.int32).view(R, per).to(DEV)
+    k = torch.randn(R * per + 1, G, page, D, generator=g).to(torch.bfloat16).to(DEV)
+    v = k if D == 256 else torch.randn(k.shape, generator=g).to(torch.bfloat16).to(DEV)
+    cache = SimpleNamespace(keys=lambda s: k, values=lambda s: v, page_tokens=page)
+    counts = [1] * len(singles) + [portion]
+    firsts = [c - n for c, n in zip(contexts, counts)]
+    T = sum(counts)
+    starts = [0]
+    for n in counts:
+        starts.append(starts[-1] + n)
+    host = HostStep(list(range(R)), counts, firsts, contexts, list(range(R)))
+    ctx = SimpleNamespace(n_requests=R, n_tokens=T, req_row_start=_i32(starts), req_first_pos=_i32(firsts),
+                          positions=_i32([f + i for f, n in zip(firsts, counts) for i in range(n)]),
+                          row_request=_i32([r for r, n in enumerate(counts) for _ in range(n)]),
+                          block_table=lambda group: table, host=host,
+                          scratch=lambda name, shape, dtype: torch.full(tuple(shape), float("nan"), dtype=dtype, device=DEV))
+    q = torch.randn(T, H * D, generator=g).to(torch.bfloat16).to(DEV)
+    logits = None if gate is None else torch.randn(T, H * D if gate == "element" else H, generator=g).to(torch.bfloat16).to(DEV)
+    sinks = torch.randn(H, generator=g).to(DEV)
+    seen, real = [], tensor_core._attention_tcgen05
+
+    def spy(*a, **kw):
+        seen.append(a[4].count)
+        return real(*a, **kw)
+    monkeypatch.setattr(tensor_core, "_attention_tcgen05", spy)
+    if apart:
+        monkeypatch.setattr(tensor_core, "MIXED_REACH", 0)
+    outs = []
+    for use in (True, False):
+        monkeypatch.setattr(sink_attention, "TENSOR_CORES", use)
+        out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        sink_attention.attention(q, logits, out, sinks, H, G, D, D, D ** -0.5, window, keep, 0.8, ctx, cache,
+                                 SimpleNamespace(slot=0, group=0), gate_per_head=gate == "head", chunked=chunked)
+        outs.append(out.float())
+    assert seen == [1 if apart else R]                         # the portion alone, or the step
+    err = float((outs[0] - outs[1]).abs().max() / outs[1].abs().max())
+    assert err < 1.5e-2                                        # both round P and the result to bfloat16 (2^-8)

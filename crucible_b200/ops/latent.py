@@ -62,17 +62,20 @@ def rows_gate(x, g) -> None:
                             _c_int(x.shape[0]), _c_int(x.shape[1]), _stream()), "rows_gate")
 
 
-SMALL_ROWS = 16      # steps of up to this many rows take the heads' products in one launch
+WARP_ROWS = 2        # steps of up to this many rows take a warp per weight row ...
+SMALL_ROWS = 16      # ... and steps of up to this many that the tiles refuse
 HEADS_IN_ONE_LAUNCH = True   # many bfloat16 rows: the heads as the third axis of one tensor-core launch
                              # (tests switch it off to reach the product per head with the same inputs)
 
 
 def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_rows=None) -> None:
     """out[t, h * out_head + n] = sum_k a[t, h * a_head + k] * w[h, n, k] for every head h of
-    `w` [heads, N, K].  Steps of a few bfloat16 rows run as one launch whose warps each read one
-    weight row once; many bfloat16 rows as one launch of tensor-core tiles with the head as the
-    grid's third axis; otherwise one product per head through `ops.linear` (in float32 always, so
-    that a row's sums never depend on the step).
+    `w` [heads, N, K].  bfloat16 rows run as one launch of tensor-core tiles with the head as the grid's
+    third axis; one or two of them, and few whose sizes the tiles refuse, as one launch whose warps each
+    read one weight row once; otherwise one product per head through `ops.linear` (in float32 always,
+    so that a row's sums never depend on the step).  A whole layer of 16 heads over a latent of 192, both
+    ways: 8 rows 47 us with the tiles, 53 with the warps; 16 rows 51 and 68; 24 rows 66, and 140 as
+    a product per head; one row 45 and 45 with a launch less for the gate.
     `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), in the same
     launch for few rows, by `head_gate` otherwise.  `gate_rows` (rows of the activations' dtype,
     [rows, heads * N]): every result times the sigmoid of its own logit, likewise."""
@@ -81,14 +84,18 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
     if gate_rows is not None and (out_head != n or gate_rows.shape != (a.shape[0], heads * n)
                                   or gate_rows.dtype != out.dtype or gate_rows.stride(1) != 1):
         raise KernelError("heads_linear: gate rows are [rows, heads * N] of the results' dtype")
-    if a.dtype == torch.bfloat16 and a.shape[0] <= SMALL_ROWS:
+    from . import is_weight, tensor_core
+    rows = a.shape[0]
+    done = (HEADS_IN_ONE_LAUNCH and a.dtype == torch.bfloat16 and rows > WARP_ROWS and is_weight(w)
+            and tensor_core.heads_linear(a, a_head, w, out, out_head))
+    if not done and a.dtype == torch.bfloat16 and rows <= SMALL_ROWS:
         _need_cuda(a, w, out, gate_rows)
         if a.stride(1) != 1 or out.stride(1) != 1 or not w.is_contiguous() or out.dtype != a.dtype:
             raise KernelError("heads_linear: contiguous rows of one dtype and contiguous weights")
         lib = build.load("latent_attention")
         _check(lib.cb_heads_linear_small(_ptr(a), _c_int(a.stride(0)), _c_int(a_head), _ptr(w), _ptr(out),
                                          _c_int(out.stride(0)), _c_int(out_head), _c_int(_code(a.dtype)),
-                                         _c_int(a.shape[0]), _c_int(heads), _c_int(n), _c_int(k),
+                                         _c_int(rows), _c_int(heads), _c_int(n), _c_int(k),
                                          _ptr(gate_logit),
                                          _c_int(gate_logit.stride(0) if gate_logit is not None else 0),
                                          _ptr(gate_rows),
@@ -96,9 +103,7 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
                                          _stream()),
                "heads_linear (few rows)")
         return
-    from . import is_weight, tensor_core
-    if not (HEADS_IN_ONE_LAUNCH and a.dtype == torch.bfloat16 and is_weight(w)
-            and tensor_core.heads_linear(a, a_head, w, out, out_head)):
+    if not done:
         for i in range(heads):
             linear(a[:, i * a_head:i * a_head + k], w[i], out[:, i * out_head:i * out_head + n])
     if gate_logit is not None:

@@ -379,7 +379,6 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     return True
 
 
-HEADS_MIN_ROWS = 33      # from this many rows on the heads' products run as tiles of 128 rows
 
 
 def heads_linear(a, a_head: int, w, out, out_head: int) -> bool:
@@ -390,7 +389,7 @@ def heads_linear(a, a_head: int, w, out, out_head: int) -> bool:
     heads, n, k = w.shape
     if (a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not w.is_contiguous() or not a.is_cuda
             or a.stride(1) != 1 or out.stride(1) != 1 or out.dtype not in (torch.bfloat16, torch.float32)
-            or a.shape[0] < HEADS_MIN_ROWS or k % 8 or a_head % 8 or a.stride(0) % 8
+            or k % 8 or a_head % 8 or a.stride(0) % 8
             or a.data_ptr() % 16 or w.data_ptr() % 16 or out.data_ptr() % 16
             or (out_head * out.element_size()) % 16 or (out.stride(0) * out.element_size()) % 16
             or a.shape[1] < (heads - 1) * a_head + k or out.shape[1] < (heads - 1) * out_head + n):

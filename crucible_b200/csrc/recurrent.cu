@@ -671,6 +671,174 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     if (RULE == RULE_MLSTM && blockIdx.z == 0 && threadIdx.x == 0) *M = m;
 }
 
+// ---- the recurrence, a token each ----------------------------------------------------------
+// Decode steps of the bfloat16 engine: every request brings one token, so a head's S is read and written
+// once and nothing follows.  The walk above stages tokens and spreads a column over lanes that read 16
+// bytes of a row of S; here a block takes 64 columns, a thread four neighbouring ones of every eighth
+// row, all of its loads in flight at once, and the sums over a column meet in shared memory.  Bound by
+// the bytes of S both ways: 32 requests of 16 heads of 128 x 128 33 to 40 us in the walk, 9 to 15 here
+// (67 MB), 8 requests 10 to 12 and 4, one 3 to 4 and 3.
+// (The float32 engine keeps the walk: its rows have the same bits however a prompt is cut.)
+constexpr int STEP_COLS = 64, STEP_GROUPS = THREADS / (STEP_COLS / 4);
+
+template <int ROWS, int RULE>
+__global__ void __launch_bounds__(THREADS) matrix_step_kernel(
+    const float* __restrict__ qkv, int C, int q_off, int k_off, int v_off,
+    const float* __restrict__ sc0, const float* __restrict__ sc1,
+    const int* __restrict__ req_row_start, const int* __restrict__ req_state_slot,
+    unsigned char* state, long slot_stride, long s_off, long n_off, long m_off,
+    float* __restrict__ out, int n_heads, int n_qk_heads, int D, int E, int w_off,
+    const float* __restrict__ per_head, const float* __restrict__ kept) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    constexpr bool DELTAS = RULE == RULE_DELTA || RULE == RULE_CHANNEL, VECTOR = VECTOR_DECAY<RULE>;
+    constexpr int SUMS = DELTAS ? 2 : 1;
+    __shared__ float sq[ROWS * STEP_GROUPS], sk[ROWS * STEP_GROUPS], sw[ROWS * STEP_GROUPS];
+    __shared__ __align__(16) float part[SUMS][STEP_GROUPS][STEP_COLS];
+    __shared__ __align__(16) float su[STEP_COLS];
+    __shared__ float scratch[32];
+    const int r = blockIdx.x, head = blockIdx.y, tid = threadIdx.x;
+    const int cg = tid % (STEP_COLS / 4), dg = tid / (STEP_COLS / 4);
+    const int col = blockIdx.z * STEP_COLS + cg * 4;
+    const bool live = col < E;
+    const int row = req_row_start[r], slot = req_state_slot[r];
+    const int g = head / (n_heads / n_qk_heads);
+    float* S = state_at(state, slot_stride, slot, s_off) + (size_t)head * D * E + col;
+    float4 s[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int d = dg + STEP_GROUPS * i;
+        s[i] = live && d < D ? *reinterpret_cast<const float4*>(S + (size_t)d * E) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float* src = qkv + (size_t)row * C;
+    for (int d = tid; d < ROWS * STEP_GROUPS; d += THREADS) {
+        const bool in = d < D;
+        sq[d] = in ? src[q_off + (size_t)g * D + d] : 0.f;
+        sk[d] = in ? src[k_off + (size_t)g * D + d] : 0.f;
+        // the decays; wkv's bonus takes the sums' place below
+        if (VECTOR) sw[d] = in ? src[w_off + (size_t)head * D + d] : 0.f;
+    }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) v = *reinterpret_cast<const float4*>(src + v_off + (size_t)head * E + col);
+    const size_t at = (size_t)row * n_heads + head;
+    float a = 1.f, b = 1.f, low = 1.f;              // decay, what the write is times, the denominator
+    if (RULE == RULE_DELTA || RULE == RULE_SSD) a = sc0[at];
+    if (DELTAS || RULE == RULE_SSD) b = sc1[at];
+    if (RULE == RULE_MLSTM) {
+        const float* kept_n = kept + (size_t)r * (n_heads * D + n_heads);
+        const float f = sc0[at], in = sc1[at], m = kept_n[(size_t)n_heads * D + head];
+        const float m_new = fmaxf(f + m, in);
+        a = expf(f + m - m_new);
+        b = expf(in - m_new);
+        __syncthreads();
+        float nq = 0.f;
+        for (int d = tid; d < D; d += THREADS) {
+            const float n = fmaf(b, sk[d], a * kept_n[(size_t)head * D + d]);
+            nq = fmaf(n, sq[d], nq);
+            if (blockIdx.z == 0) state_at(state, slot_stride, slot, n_off)[(size_t)head * D + d] = n;
+        }
+        low = fmaxf(fabsf(cb_block_sum(nq, scratch)), expf(-m_new)) + 1e-6f;
+        if (blockIdx.z == 0 && tid == 0) state_at(state, slot_stride, slot, m_off)[head] = m_new;
+    }
+    __syncthreads();
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f), rk = o;
+    float kq = 0.f;
+    const float4 bv = make_float4(b * v.x, b * v.y, b * v.z, b * v.w);
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int d = dg + STEP_GROUPS * i;
+        const float q = sq[d], k = sk[d];
+        if (RULE == RULE_WKV) {
+            const float u = d < D ? per_head[(size_t)head * D + d] * k : 0.f, w = sw[d];
+            o.x = fmaf(fmaf(u, v.x, s[i].x), q, o.x); o.y = fmaf(fmaf(u, v.y, s[i].y), q, o.y);
+            o.z = fmaf(fmaf(u, v.z, s[i].z), q, o.z); o.w = fmaf(fmaf(u, v.w, s[i].w), q, o.w);
+            s[i] = make_float4(fmaf(w, s[i].x, k * v.x), fmaf(w, s[i].y, k * v.y), fmaf(w, s[i].z, k * v.z),
+                               fmaf(w, s[i].w, k * v.w));
+            continue;
+        }
+        const float w = RULE == RULE_CHANNEL ? sw[d] : a;
+        s[i] = make_float4(w * s[i].x, w * s[i].y, w * s[i].z, w * s[i].w);
+        if (DELTAS) {
+            rk.x = fmaf(s[i].x, k, rk.x); rk.y = fmaf(s[i].y, k, rk.y);
+            rk.z = fmaf(s[i].z, k, rk.z); rk.w = fmaf(s[i].w, k, rk.w);
+            kq = fmaf(k, q, kq);
+        } else {
+            s[i] = make_float4(fmaf(k, bv.x, s[i].x), fmaf(k, bv.y, s[i].y), fmaf(k, bv.z, s[i].z), fmaf(k, bv.w, s[i].w));
+        }
+        o.x = fmaf(s[i].x, q, o.x); o.y = fmaf(s[i].y, q, o.y);
+        o.z = fmaf(s[i].z, q, o.z); o.w = fmaf(s[i].w, q, o.w);
+    }
+    if (!DELTAS) {
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int d = dg + STEP_GROUPS * i;
+            if (live && d < D) *reinterpret_cast<float4*>(S + (size_t)d * E) = s[i];
+        }
+    }
+    *reinterpret_cast<float4*>(&part[0][dg][cg * 4]) = o;
+    if (DELTAS) {
+        *reinterpret_cast<float4*>(&part[SUMS - 1][dg][cg * 4]) = rk;
+        if (cg == 0) scratch[dg] = kq;
+    }
+    __syncthreads();
+    const int c = blockIdx.z * STEP_COLS + tid;
+    if (tid < STEP_COLS) {
+        float sum = 0.f, rs = 0.f, kqs = 0.f;
+#pragma unroll
+        for (int i = 0; i < STEP_GROUPS; ++i) {
+            sum += part[0][i][tid];
+            if (DELTAS) {
+                rs += part[SUMS - 1][i][tid];
+                kqs += scratch[i];
+            }
+        }
+        const float vc = c < E ? src[v_off + (size_t)head * E + c] : 0.f;
+        if (DELTAS) {
+            const float u = b * (vc - rs);
+            su[tid] = u;
+            sum = fmaf(u, kqs, sum);
+        } else if (RULE == RULE_SSD) {
+            sum = fmaf(per_head[head], vc, sum);
+        } else if (RULE == RULE_MLSTM) {
+            sum /= low;
+        }
+        if (c < E) out[at * E + c] = sum;
+    }
+    if (DELTAS) {
+        __syncthreads();
+        const float4 u = *reinterpret_cast<const float4*>(su + cg * 4);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int d = dg + STEP_GROUPS * i;
+            const float k = sk[d];
+            if (live && d < D)
+                *reinterpret_cast<float4*>(S + (size_t)d * E) = make_float4(
+                    fmaf(k, u.x, s[i].x), fmaf(k, u.y, s[i].y), fmaf(k, u.z, s[i].z), fmaf(k, u.w, s[i].w));
+        }
+    }
+}
+
+template <int RULE>
+int launch_step(const float* qkv, int C, int q_off, int k_off, int v_off, const float* sc0, const float* sc1,
+                const int* req_row_start, const int* req_state_slot, unsigned char* state, long slot_stride,
+                long s_off, long n_off, long m_off, float* out, int n_requests, int n_heads, int n_qk_heads, int D,
+                int E, int w_off, const float* per_head, const float* kept, cudaStream_t s) {
+    const dim3 grid(n_requests, n_heads, (E + STEP_COLS - 1) / STEP_COLS);
+#define CB_STEP(RR)                                                                                         \
+    do {                                                                                                    \
+        cb_launch(matrix_step_kernel<RR, RULE>, grid, dim3(THREADS), 0, s, qkv, C, q_off, k_off, v_off, sc0, sc1, \
+                  req_row_start, req_state_slot, state, slot_stride, s_off, n_off, m_off, out, n_heads,     \
+                  n_qk_heads, D, E, w_off, per_head, kept);                                                 \
+        return cb_last_error();                                                                             \
+    } while (0)
+    if (D <= 4 * STEP_GROUPS) CB_STEP(4);
+    if (D <= 8 * STEP_GROUPS) CB_STEP(8);
+    if (D <= 16 * STEP_GROUPS) CB_STEP(16);
+    if (D <= 32 * STEP_GROUPS) CB_STEP(32);
+#undef CB_STEP
+    return CB_ERR_UNSUPPORTED;
+}
+
 // ---- wkv: the mixes of a token with the token before it ------------------------------------
 // h: T rows [rows][width].  mu: fp32 [n_mix][width].  out: T [n_mix][rows][width]:
 //   out[s][t] = h[t] + (h[t-1] - h[t]) * mu[s]      (fp32 arithmetic, rounded once)
@@ -1012,6 +1180,35 @@ CB_EXPORT int cb_matrix_memory(int rule, const float* qkv, int C, int q_off, int
                                  req_state_slot, (unsigned char*)state, slot_stride, s_off, n_off,   \
                                  m_off, out, n_requests, n_heads, n_qk_heads, key_dim, value_dim,    \
                                  w_off, per_head, kept, s)
+    CB_RULE(RULE_DELTA);
+    CB_RULE(RULE_MLSTM);
+    CB_RULE(RULE_WKV);
+    CB_RULE(RULE_SSD);
+    CB_RULE(RULE_CHANNEL);
+#undef CB_RULE
+    return CB_ERR_UNSUPPORTED;
+}
+
+// The same where every request brings one token: value sizes, rows' strides and offsets of v in whole
+// 16-byte pieces, the matrices on 16-byte boundaries.
+CB_EXPORT int cb_matrix_memory_step(int rule, const float* qkv, int C, int q_off, int k_off, int v_off,
+                                    const float* sc0, const float* sc1, const int* req_row_start,
+                                    const int* req_state_slot, void* state, long slot_stride, long s_off,
+                                    long n_off, long m_off, float* out, int n_requests, int n_heads,
+                                    int n_qk_heads, int key_dim, int value_dim, int w_off,
+                                    const float* per_head, const float* kept, void* stream) {
+    if (n_requests <= 0) return 0;
+    if (n_heads % n_qk_heads != 0 || n_heads > 65535 || ((C | v_off | value_dim) & 3) != 0 ||
+        ((s_off | slot_stride) & 15) != 0 || ((uintptr_t)state & 15) != 0 || ((uintptr_t)qkv & 15) != 0)
+        return CB_ERR_UNSUPPORTED;
+    if ((rule == RULE_WKV || rule == RULE_SSD) && per_head == nullptr) return CB_ERR_UNSUPPORTED;
+    if (rule == RULE_MLSTM && kept == nullptr) return CB_ERR_UNSUPPORTED;
+    cudaStream_t s = (cudaStream_t)stream;
+#define CB_RULE(RR)                                                                                  \
+    if (rule == RR)                                                                                  \
+        return launch_step<RR>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start, req_state_slot, \
+                               (unsigned char*)state, slot_stride, s_off, n_off, m_off, out,         \
+                               n_requests, n_heads, n_qk_heads, key_dim, value_dim, w_off, per_head, kept, s)
     CB_RULE(RULE_DELTA);
     CB_RULE(RULE_MLSTM);
     CB_RULE(RULE_WKV);

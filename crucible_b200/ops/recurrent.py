@@ -14,6 +14,7 @@ DELTA, MLSTM, WKV, SSD, CHANNEL = 0, 1, 2, 3, 4
 GATE_SILU, GATE_SIGMOID = 0, 1
 CHUNKS = True                # tests switch it off to reach the token-by-token walk with the same inputs
 CHUNK_MIN_TOKENS = 128       # the longest portion from which a bfloat16 step's portions go in chunks
+STEP = True                  # likewise, for the form of a token each
 
 
 def _state_args(state: torch.Tensor):
@@ -160,7 +161,10 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     if walked == 0:
         return
     lib = build.load("recurrent")
-    _check(lib.cb_matrix_memory(
+    # decoded tokens of the bfloat16 engine: a token each, S read and written once
+    step = (STEP and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.lead_single >= walked
+            and (qkv.shape[1] | v_off | value_dim) % 4 == 0 and (s_off | state.stride(0)) % 16 == 0)
+    _check((lib.cb_matrix_memory_step if step else lib.cb_matrix_memory)(
         _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
         _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,
         _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(walked),

@@ -1,4 +1,5 @@
-"""The recurrences over prompts' portions in chunks of 32 tokens (`csrc/recurrent_chunks.cu`) against the
+"""The recurrences over prompts' portions in chunks of 32 tokens (`csrc/recurrent_chunks.cu`), and over a
+token of each of several requests (`csrc/recurrent.cu`, the step form), against the
 same recurrences token by token in float64, for every rule: portions that end inside a chunk, at its
 edge and one token beyond it, a state carried in, heads and values that are no whole tiles, decays of 0
 and 1, requests of one token at the head of the step.  The operands are float32, so the error is that
@@ -11,7 +12,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-LENGTHS = [(1, 128, 33), (1, 1, 161), (200,), (129, 31, 32)]
+LENGTHS = [(1, 128, 33), (1, 1, 161), (200,), (129, 31, 32), (1,), (1, 1, 1, 1, 1)]
 
 
 def _i32(values):
@@ -115,13 +116,13 @@ def test_chunks_agree_with_float64(rule, H, G, D, E):
             state = torch.zeros(R, 4 * sum(sizes), dtype=torch.uint8, device=DEV)
             state.view(torch.float32)[slots] = before.to(DEV)
             out = torch.full((T, H * E), float("nan"), device=DEV)
-            k.CHUNKS = chunks
+            k.CHUNKS = k.STEP = chunks
             try:
                 k.matrix_memory(rule_code, qkv, *offs, *(x.contiguous().to(DEV) if x is not None else None for x in (sc0, sc1)),
                                 ctx, state, 0, 4 * sizes[0], 4 * (sizes[0] + sizes[1]), out, H, G, D, E,
                                 w_off=2 * G * D + H * E, per_head=per_head.to(DEV).contiguous() if per_head is not None else None)
             finally:
-                k.CHUNKS = True
+                k.CHUNKS = k.STEP = True
             results[chunks] = out.cpu().view(T, H, E), state.view(torch.float32)[slots].cpu()
         for r in range(R):
             a, b = starts[r], starts[r + 1]

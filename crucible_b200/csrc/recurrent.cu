@@ -48,6 +48,20 @@ __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float logsigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
+// four neighbouring elements of a row, on a boundary of their size
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+    const float2 x = __bfloat1622float2(a), y = __bfloat1622float2(b);
+    return make_float4(x.x, x.y, y.x, y.y);
+}
+__device__ __forceinline__ void store_four(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(float* smem, const float* gmem) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
@@ -135,6 +149,110 @@ __global__ void conv_tail_update_kernel(const T* __restrict__ proj, int proj_str
             const int src = n_new - keep + i;
             tail[(size_t)i * C + c] = src >= 0 ? cb_to_float(proj[(size_t)(first + src) * proj_stride + c])
                                                : tail[(size_t)(i + n_new) * C + c];
+        }
+    }
+}
+
+// ---- delta rule and state space: the convolution 16 bytes a lane ---------------------------------
+// The two preparations above are a block a token whose threads read every input once per tap, two bytes
+// at a time (2,048 tokens of 3,072 channels 59 us for 38 MB, 9.4 us for 32 tokens of 2,560; here 25 and 5.8).  Here a warp takes a tile of
+// a request's tokens (grid y: tiles, z: requests) and 128 channels, or one q or k head, four neighbouring
+// channels a lane; it walks the tokens with the last inputs in registers, the next one on its way.  With
+// `update` the first tile's warp, which alone reads the request's old inputs, leaves the new ones, and
+// there is no launch for that.  A row's sums are in one order whatever the tile.
+// Units: heads (delta: 2 G heads of D channels that become unit vectors, the first G times
+// unit_scale), then runs of 128 channels, then the step's numbers per head.
+// conv_w: [C][TAPS], bias: [C] or null.
+template <typename T, int TAPS, bool IS_SSD>
+__global__ void __launch_bounds__(128) conv_prepare_kernel(
+    const T* __restrict__ proj, int proj_stride, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
+    const float* __restrict__ gates, int gates_stride, const float* __restrict__ a_log,
+    const float* __restrict__ dt_bias, const int* __restrict__ req_row_start, const int* __restrict__ req_state_slot,
+    unsigned char* state, long slot_stride, long tail_off, float* __restrict__ dst, float* __restrict__ num0,
+    float* __restrict__ num1, int C, int n_heads, int unit_heads, int scaled_heads, int head_size, float unit_scale,
+    int tile, int n_units, int update) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    const int r = blockIdx.z, lane = threadIdx.x & 31;
+    int unit = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (unit >= n_units) return;
+    const int row0 = req_row_start[r], n = req_row_start[r + 1] - row0;
+    const int a = blockIdx.y * tile, b = min(a + tile, n);
+    if (a >= n) return;
+    if (unit == n_units - 1) {
+        for (int i = lane; i < (b - a) * n_heads; i += 32) {
+            const int h = i % n_heads;
+            const size_t t = (size_t)(row0 + a + i / n_heads);
+            const float* g = gates + t * gates_stride;
+            if (IS_SSD) {           // step size, decay
+                const float dt = softplus_f(g[h] + dt_bias[h]);
+                num1[t * n_heads + h] = dt;
+                num0[t * n_heads + h] = expf(-expf(a_log[h]) * dt);
+            } else {                // decay, beta
+                num1[t * n_heads + h] = sigmoid_f(g[h]);
+                num0[t * n_heads + h] = expf(-expf(a_log[h]) * softplus_f(g[n_heads + h] + dt_bias[h]));
+            }
+        }
+        return;
+    }
+    const bool is_head = unit < unit_heads;
+    const int c0 = is_head ? unit * head_size : unit_heads * head_size + (unit - unit_heads) * 128;
+    const int count = is_head ? head_size : min(128, C - c0);
+    const int c = c0 + 4 * lane;
+    const bool in = 4 * lane < count;
+    float* tail = state_at(state, slot_stride, req_state_slot[r], tail_off);
+    constexpr int KEEP = TAPS - 1;
+    // the input of the lane's channels at the portion's token `row` (negative: the request's old inputs)
+    auto input = [&](int row) {
+        if (!in) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return row >= 0 ? load_four(proj + (size_t)(row0 + row) * proj_stride + c) : load_four(tail + (size_t)(KEEP + row) * C + c);
+    };
+    float w[4][TAPS];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[e][j] = in ? conv_w[(size_t)(c + e) * TAPS + j] : 0.f;
+    const float4 bias = IS_SSD && conv_b != nullptr && in ? load_four(conv_b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 past[TAPS], next = input(a);
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) past[j] = input(a - KEEP + j);
+    float4 last[TAPS];              // the request's old inputs, if this warp will replace them
+    const bool writes = update && a == 0;
+    if (writes) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) last[j] = past[j];
+    }
+    const float sc = is_head && unit < scaled_heads ? unit_scale : 1.0f;
+#pragma unroll 1
+    for (int t = a; t < b; ++t) {
+        past[KEEP] = next;
+        if (t + 1 < b) next = input(t + 1);
+        float4 v = bias;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            v.x = fmaf(w[0][j], past[j].x, v.x); v.y = fmaf(w[1][j], past[j].y, v.y);
+            v.z = fmaf(w[2][j], past[j].z, v.z); v.w = fmaf(w[3][j], past[j].w, v.w);
+        }
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) past[j] = past[j + 1];
+        v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+        if (is_head) {
+            const float ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+            const float inv = 1.0f / sqrtf(cb_warp_sum(ss) + 1e-6f) * sc;
+            v = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+        }
+        if (in) store_four(dst + (size_t)(row0 + t) * C + c, v);
+    }
+    if (writes && in) {
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int src = n - KEEP + k;           // negative: an old input stays, further to the front
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src >= 0) x = input(src);
+#pragma unroll
+            for (int j = 0; j < KEEP; ++j)
+                if (src < 0 && j == KEEP + src) x = last[j];
+            store_four(tail + (size_t)k * C + c, x);
         }
     }
 }
@@ -306,7 +424,7 @@ __global__ void mlstm_prepare_kernel(const T* __restrict__ proj, int proj_stride
                                      float* __restrict__ log_keep, float* __restrict__ log_in,
                                      int n_heads, int key_dim, int value_dim, float* __restrict__ kept,
                                      const int* __restrict__ req_state_slot, unsigned char* state,
-                                     long slot_stride, long n_off, long m_off, int n_requests) {
+                                     long slot_stride, long n_off, long m_off, int n_requests, int vec) {
     cb_pdl_trigger();
     cb_pdl_wait();
     const int t = blockIdx.x;
@@ -321,9 +439,17 @@ __global__ void mlstm_prepare_kernel(const T* __restrict__ proj, int proj_stride
     const float q_scale = 1.0f / sqrtf((float)key_dim);
     const T* src = proj + (size_t)t * proj_stride;
     float* dst = qkv + (size_t)t * C;
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        const float x = cb_to_float(src[c]);
-        dst[c] = c < nq ? x * q_scale : x;
+    if (vec) {
+        for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
+            float4 x = load_four(src + c);
+            if (c < nq) x = make_float4(x.x * q_scale, x.y * q_scale, x.z * q_scale, x.w * q_scale);
+            store_four(dst + c, x);
+        }
+    } else {
+        for (int c = threadIdx.x; c < C; c += blockDim.x) {
+            const float x = cb_to_float(src[c]);
+            dst[c] = c < nq ? x * q_scale : x;
+        }
     }
     for (int h = threadIdx.x; h < n_heads; h += blockDim.x) {
         const float* g = gates + (size_t)t * gates_stride;
@@ -988,6 +1114,73 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
     }
 }
 
+// The same for heads of up to 128 features in whole groups of four, all rows on boundaries of a group: a
+// lane has four neighbouring features, read once (2,048 rows of 16 heads of 128: 20 us with one feature at
+// a time, read twice; 12 here).
+template <typename T, typename TG, int GATE>
+__global__ void head_norm_gate_quad_kernel(const float* __restrict__ o, const float* __restrict__ gain,
+                                           int gain_head_stride, const TG* __restrict__ gate, int gate_stride,
+                                           T* __restrict__ out, int out_stride, int n_rows, int n_heads,
+                                           int E, float eps, float out_scale) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (unit >= n_rows * n_heads) return;
+    const int e = (threadIdx.x & 31) * 4;
+    const int t = unit / n_heads, h = unit - t * n_heads;
+    const bool in = e < E;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), z = x, gn = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (in) {
+        x = load_four(o + (size_t)unit * E + e);
+        z = load_four(gate + (size_t)t * gate_stride + (size_t)h * E + e);
+        if (gain != nullptr) gn = load_four(gain + (size_t)h * gain_head_stride + e);
+    }
+    const float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
+    const float r = 1.0f / sqrtf(cb_warp_sum(ss) / (float)E + eps);
+    auto gt = [](float v) { return GATE == GATE_SILU ? silu_f(v) : sigmoid_f(v); };
+    if (in)
+        store_four(out + (size_t)t * out_stride + (size_t)h * E + e,
+                   make_float4(x.x * r * gn.x * gt(z.x) * out_scale, x.y * r * gn.y * gt(z.y) * out_scale,
+                               x.z * r * gn.z * gt(z.z) * out_scale, x.w * r * gn.w * gt(z.w) * out_scale));
+}
+
+// gate_group_norm with the row's part in registers, four neighbouring features a thread and pass (32 rows
+// of 2,048: 10 us read one by one and twice, 5 here).  A part of up to 4 * QUADS * 256 features.
+template <typename T, int QUADS>
+__global__ void __launch_bounds__(256) gate_group_norm_quad_kernel(
+    const float* __restrict__ y, const T* __restrict__ gate, int gate_stride, const float* __restrict__ gain,
+    T* __restrict__ out, int out_stride, int width, int parts, float eps) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    __shared__ float scratch[32];
+    const int t = blockIdx.x / parts, part = blockIdx.x - t * parts;
+    const int n = width / parts, at = part * n;
+    const float* src = y + (size_t)t * width + at;
+    const T* g = gate + (size_t)t * gate_stride + at;
+    float4 v[QUADS];
+    float ss = 0.f;
+#pragma unroll
+    for (int q = 0; q < QUADS; ++q) {
+        const int i = (q * blockDim.x + threadIdx.x) * 4;
+        v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n) {
+            const float4 x = load_four(src + i), z = load_four(g + i);
+            v[q] = make_float4(x.x * silu_f(z.x), x.y * silu_f(z.y), x.z * silu_f(z.z), x.w * silu_f(z.w));
+        }
+        ss = fmaf(v[q].x, v[q].x, fmaf(v[q].y, v[q].y, fmaf(v[q].z, v[q].z, fmaf(v[q].w, v[q].w, ss))));
+    }
+    const float r = 1.0f / sqrtf(cb_block_sum(ss, scratch) / (float)n + eps);
+    T* dst = out + (size_t)t * out_stride + at;
+#pragma unroll
+    for (int q = 0; q < QUADS; ++q) {
+        const int i = (q * blockDim.x + threadIdx.x) * 4;
+        if (i < n) {
+            const float4 gn = load_four(gain + at + i);
+            store_four(dst + i, make_float4(v[q].x * r * gn.x, v[q].y * r * gn.y, v[q].z * r * gn.z, v[q].w * r * gn.w));
+        }
+    }
+}
+
 template <int P, int LANES, int RULE>
 int launch_memory_as(const float* qkv, int C, int q_off, int k_off, int v_off, const float* sc0,
                      const float* sc1, const int* req_row_start, const int* req_state_slot,
@@ -1063,6 +1256,50 @@ CB_EXPORT int cb_delta_prepare(const void* proj, int proj_stride, int dtype, con
     return cb_last_error();
 }
 
+// The preparation of the delta rule (unit_heads 2 G heads of head_size, the first half scaled) or of the
+// state space (unit_heads 0) 16 bytes a lane: 2 to 4 taps, sizes and strides in whole groups of four
+// elements, heads up to 128 features.  num0, num1: [rows][H] decay and beta, or decay and step size.  update:
+// the request's last inputs are replaced here; max_new: the most tokens that a request brings.
+CB_EXPORT int cb_conv_prepare(const void* proj, int proj_stride, int dtype, const float* conv_w,
+                              const float* conv_b, int taps, const float* gates, int gates_stride,
+                              const float* a_log, const float* dt_bias, const int* req_row_start,
+                              const int* req_state_slot, void* state, long slot_stride, long tail_off, float* dst,
+                              float* num0, float* num1, int n_requests, int max_new, int n_heads, int C,
+                              int unit_heads, int head_size, int is_ssd, int update, void* stream) {
+    if (n_requests <= 0 || max_new <= 0) return 0;
+    const size_t group = dtype == CB_F32 ? 16 : 8;
+    if (taps < 2 || taps > 4 || ((C | proj_stride | (unit_heads ? head_size : 0)) & 3) != 0 ||
+        (unit_heads && (head_size > 128 || head_size <= 0)) || (uintptr_t)proj % group != 0 ||
+        (((uintptr_t)dst | (uintptr_t)state | (uintptr_t)conv_b) & 15) != 0 || ((slot_stride | tail_off) & 15) != 0 ||
+        n_requests > 65535)
+        return CB_ERR_UNSUPPORTED;
+    const int runs = (C - unit_heads * head_size + 127) / 128;
+    const int n_units = unit_heads + runs + 1;
+    const int tile = max_new >= 1024 ? 16 : 8;          // at least the taps: a later tile never reads the state
+    const dim3 grid((n_units + 3) / 4, (max_new + tile - 1) / tile, n_requests), block(128);
+    if (grid.y > 65535) return CB_ERR_UNSUPPORTED;
+    const float unit_scale = unit_heads ? 1.0f / sqrtf((float)head_size) : 1.0f;
+    cudaStream_t s = (cudaStream_t)stream;
+#define CB_CP(TT, KK, SS)                                                                                    \
+    cb_launch(conv_prepare_kernel<TT, KK, SS>, grid, block, 0, s, (const TT*)proj, proj_stride, conv_w, conv_b, gates, \
+              gates_stride, a_log, dt_bias, req_row_start, req_state_slot, (unsigned char*)state, slot_stride, tail_off, \
+              dst, num0, num1, C, n_heads, unit_heads, unit_heads / 2, head_size, unit_scale, tile, n_units, update)
+#define CB_CP_TAPS(TT, SS)                              \
+    do {                                                \
+        if (taps == 2) CB_CP(TT, 2, SS);                \
+        else if (taps == 3) CB_CP(TT, 3, SS);           \
+        else CB_CP(TT, 4, SS);                          \
+    } while (0)
+    if (dtype == CB_F32) {
+        if (is_ssd) CB_CP_TAPS(float, true); else CB_CP_TAPS(float, false);
+    } else {
+        if (is_ssd) CB_CP_TAPS(__nv_bfloat16, true); else CB_CP_TAPS(__nv_bfloat16, false);
+    }
+#undef CB_CP_TAPS
+#undef CB_CP
+    return cb_last_error();
+}
+
 // conv_w: fp32 [taps][channels]; max_new: the most tokens that a request brings.
 CB_EXPORT int cb_channel_delta_prepare(const void* proj, int proj_stride, int dtype, const float* conv_w,
                                        int taps, const float* rate, int rate_stride, const float* beta_logit,
@@ -1122,17 +1359,20 @@ CB_EXPORT int cb_mlstm_prepare(const void* proj, int proj_stride, int dtype, con
                                long slot_stride, long n_off, long m_off, int n_requests, void* stream) {
     if (n_rows <= 0) return 0;
     const int C = n_heads * (2 * key_dim + value_dim);
-    const dim3 grid(n_rows), block(C <= 512 ? 128 : (C >= 4096 ? 1024 : (C / 4 + 31) / 32 * 32));
+    // rows whose groups of four elements lie on boundaries of their size are read in those
+    const int vec = ((C | n_heads * key_dim | proj_stride) & 3) == 0 && (uintptr_t)proj % (dtype == CB_F32 ? 16 : 8) == 0;
+    const dim3 grid(n_rows), block(vec ? (C >= 2048 ? 512 : (C / 4 + 31) / 32 * 32)
+                                       : (C <= 512 ? 128 : (C >= 4096 ? 1024 : (C / 4 + 31) / 32 * 32)));
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == CB_F32)
         cb_launch(mlstm_prepare_kernel<float>, grid, block, 0, s, (const float*)proj, proj_stride,
                   gates, gates_stride, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads, key_dim, value_dim,
-                  kept, req_state_slot, (unsigned char*)state, slot_stride, n_off, m_off, n_requests);
+                  kept, req_state_slot, (unsigned char*)state, slot_stride, n_off, m_off, n_requests, vec);
     else
         cb_launch(mlstm_prepare_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)proj,
                   proj_stride, gates, gates_stride, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads,
                   key_dim, value_dim, kept, req_state_slot, (unsigned char*)state, slot_stride, n_off, m_off,
-                  n_requests);
+                  n_requests, vec);
     return cb_last_error();
 }
 
@@ -1228,10 +1468,15 @@ CB_EXPORT int cb_head_norm_gate(const float* o, const float* gain, int gain_head
     const long units = (long)n_rows * n_heads;
     const dim3 grid((unsigned)((units + warps - 1) / warps)), block(warps * 32);
     cudaStream_t s = (cudaStream_t)stream;
+    // heads in whole groups of four features, every group on a boundary of its size
+    const size_t gate_group = gate_dtype == CB_F32 ? 16 : 8, out_group = dtype == CB_F32 ? 16 : 8;
+    const bool quads = value_dim <= 128 && ((value_dim | gain_head_stride | gate_stride | out_stride) & 3) == 0 &&
+                       (((uintptr_t)o | (uintptr_t)gain) & 15) == 0 && (uintptr_t)gate % gate_group == 0 &&
+                       (uintptr_t)out % out_group == 0;
 #define CB_HNG(TT, TGG, GG)                                                                        \
-    cb_launch(head_norm_gate_kernel<TT, TGG, GG>, grid, block, 0, s, o, gain, gain_head_stride,    \
-              (const TGG*)gate, gate_stride, (TT*)out, out_stride, n_rows, n_heads, value_dim, eps, \
-              out_scale)
+    cb_launch(quads ? head_norm_gate_quad_kernel<TT, TGG, GG> : head_norm_gate_kernel<TT, TGG, GG>, grid, block, \
+              0, s, o, gain, gain_head_stride, (const TGG*)gate, gate_stride, (TT*)out, out_stride, n_rows, n_heads, \
+              value_dim, eps, out_scale)
     if (dtype == CB_F32) {
         if (gate_dtype != CB_F32) return CB_ERR_UNSUPPORTED;
         if (gate_kind == GATE_SILU) CB_HNG(float, float, GATE_SILU); else CB_HNG(float, float, GATE_SIGMOID);
@@ -1308,6 +1553,24 @@ CB_EXPORT int cb_gate_group_norm(const float* y, const void* gate, int gate_stri
     const int n = width / parts;
     const dim3 grid((unsigned)((long)n_rows * parts)), block(n >= 1024 ? 256 : 128);
     cudaStream_t s = (cudaStream_t)stream;
+    const size_t group = dtype == CB_F32 ? 16 : 8;
+    if (n <= 4096 && ((n | width | gate_stride | out_stride) & 3) == 0 && (((uintptr_t)y | (uintptr_t)gain) & 15) == 0 &&
+        (uintptr_t)gate % group == 0 && (uintptr_t)out % group == 0) {
+        const int quads = (n / 4 + (int)block.x - 1) / (int)block.x;
+#define CB_GGN(TT, QQ)                                                                                       \
+    cb_launch(gate_group_norm_quad_kernel<TT, QQ>, grid, block, 0, s, y, (const TT*)gate, gate_stride, gain, \
+              (TT*)out, out_stride, width, parts, eps)
+#define CB_GGN_AS(TT)                                   \
+    do {                                                \
+        if (quads <= 1) CB_GGN(TT, 1);                  \
+        else if (quads <= 2) CB_GGN(TT, 2);             \
+        else CB_GGN(TT, 4);                             \
+    } while (0)
+        if (dtype == CB_F32) CB_GGN_AS(float); else CB_GGN_AS(__nv_bfloat16);
+#undef CB_GGN_AS
+#undef CB_GGN
+        return cb_last_error();
+    }
     if (dtype == CB_F32)
         cb_launch(gate_group_norm_kernel<float>, grid, block, 0, s, y, (const float*)gate, gate_stride, gain,
                   (float*)out, out_stride, width, parts, eps);

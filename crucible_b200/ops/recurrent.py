@@ -26,8 +26,13 @@ def _state_args(state: torch.Tensor):
 
 
 def delta_prepare(proj, conv_w, taps, gates, a_log, dt_bias, ctx, state, tail_off, qkv, beta,
-                  decay, n_heads, n_kv_heads, key_dim, value_dim) -> None:
+                  decay, n_heads, n_kv_heads, key_dim, value_dim, update_tail: bool = False) -> bool:
+    """`update_tail`: the convolution's inputs in the state may be replaced here; returns whether they
+    were (else `conv_tail_update` does it)."""
     _need_cuda(proj, conv_w, gates, a_log, dt_bias, state, qkv, beta, decay)
+    if _conv_prepare(proj, conv_w, None, taps, gates, a_log, dt_bias, ctx, state, tail_off, qkv, decay, beta, n_heads,
+                     qkv.shape[1], 2 * n_kv_heads, key_dim, False, update_tail):
+        return update_tail
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_delta_prepare(
@@ -36,6 +41,29 @@ def delta_prepare(proj, conv_w, taps, gates, a_log, dt_bias, ctx, state, tail_of
         _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(qkv), _ptr(beta), _ptr(decay),
         _c_int(proj.shape[0]), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim),
         _c_int(value_dim), _stream()), "delta_prepare")
+    return False
+
+
+def _conv_prepare(proj, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, state, tail_off, dst, num0, num1, n_heads,
+                  channels, unit_heads, head_size, is_ssd: bool, update: bool) -> bool:
+    """The preparations' form of 16 bytes a lane; `proj`: rows that start with the convolution's channels.
+    A rule of the sizes alone.  False: not taken."""
+    host = getattr(ctx, "host", None)
+    if (host is None or proj.stride(1) != 1 or not dst.is_contiguous() or not num0.is_contiguous()
+            or not num1.is_contiguous() or not conv_w.is_contiguous() or conv_w.shape[1] != taps):
+        return False
+    sp, stride = _state_args(state)
+    lib = build.load("recurrent")
+    code = lib.cb_conv_prepare(
+        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(conv_w), _ptr(conv_b), _c_int(taps),
+        _ptr(gates), _c_int(gates.stride(0)), _ptr(a_log), _ptr(dt_bias), _ptr(ctx.req_row_start),
+        _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(dst), _ptr(num0), _ptr(num1),
+        _c_int(ctx.n_requests), _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(channels), _c_int(unit_heads),
+        _c_int(head_size), _c_int(1 if is_ssd else 0), _c_int(1 if update else 0), _stream())
+    if code == 100001:
+        return False
+    _check(code, "conv_prepare")
+    return True
 
 
 def channel_delta_prepare(proj, conv_w, rate, beta_logit, a_log, dt_bias, ctx, state, tail_off, qkv, beta,
@@ -219,12 +247,16 @@ def wkv_prepare(rkv, logit, w0, qkv, n_channels) -> None:
 
 
 def ssd_prepare(proj, conv_at, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, state, tail_off, xbc,
-                decay, step, n_heads, channels) -> None:
+                decay, step, n_heads, channels, update_tail: bool = False) -> bool:
     """Causal convolution with bias + SiLU over `channels` columns of `proj` from `conv_at`
-    on; step size softplus(gate + dt_bias) and decay exp(-exp(A_log) * step) per head."""
+    on; step size softplus(gate + dt_bias) and decay exp(-exp(A_log) * step) per head.
+    `update_tail` and the result as in `delta_prepare`."""
     _need_cuda(proj, conv_w, conv_b, gates, a_log, dt_bias, state, xbc, decay, step)
     if proj.stride(1) != 1 or gates.dtype != torch.float32 or xbc.dtype != torch.float32:
         raise KernelError("ssd_prepare: contiguous rows, float32 gates and output")
+    if _conv_prepare(proj[:, conv_at:conv_at + channels], conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, state,
+                     tail_off, xbc, decay, step, n_heads, channels, 0, 0, True, update_tail):
+        return update_tail
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_ssd_prepare(
@@ -233,6 +265,7 @@ def ssd_prepare(proj, conv_at, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx,
         _ptr(ctx.row_request), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride,
         _c_long(tail_off), _ptr(xbc), _ptr(decay), _ptr(step), _c_int(proj.shape[0]), _c_int(n_heads),
         _c_int(channels), _stream()), "ssd_prepare")
+    return False
 
 
 def gate_group_norm(y, gate, gain, out, parts, eps) -> None:

@@ -107,9 +107,9 @@ class GatedDeltaRule(BranchMixer):
         beta = ctx.scratch("delta.beta", (t, H), torch.float32)
         decay = ctx.scratch("delta.decay", (t, H), torch.float32)
         o = ctx.scratch("delta.o", (t, H * E), torch.float32)
-        kernels.delta_prepare(proj, self.conv_w, self.taps, gates, self.a_log, self.dt_bias, ctx,
-                              state, self.s_bytes, qkv, beta, decay, H, G, D, E)
-        kernels.conv_tail_update(proj, self.taps, C, ctx, state, self.s_bytes)
+        if not kernels.delta_prepare(proj, self.conv_w, self.taps, gates, self.a_log, self.dt_bias, ctx,
+                                     state, self.s_bytes, qkv, beta, decay, H, G, D, E, update_tail=True):
+            kernels.conv_tail_update(proj, self.taps, C, ctx, state, self.s_bytes)
         kernels.matrix_memory(kernels.DELTA, qkv, 0, G * D, 2 * G * D, decay, beta, ctx, state, 0, 0,
                               0, o, H, G, D, E)
         kernels.head_norm_gate(o, self.gain, False, proj[:, C:C + H * E], act, kernels.GATE_SILU, H, E,
@@ -365,9 +365,9 @@ class StateSpaceMixer(BranchMixer):
         decay = ctx.scratch("ssd.decay", (t, H), torch.float32)
         step = ctx.scratch("ssd.step", (t, H), torch.float32)
         y = ctx.scratch("ssd.y", (t, inner), torch.float32)
-        kernels.ssd_prepare(proj, inner, self.conv_w, self.conv_b, self.taps, gates, self.a_log,
-                            self.dt_bias, ctx, state, self.s_bytes, xbc, decay, step, H, C)
-        kernels.conv_tail_update(proj[:, inner:inner + C], self.taps, C, ctx, state, self.s_bytes)
+        if not kernels.ssd_prepare(proj, inner, self.conv_w, self.conv_b, self.taps, gates, self.a_log,
+                                   self.dt_bias, ctx, state, self.s_bytes, xbc, decay, step, H, C, update_tail=True):
+            kernels.conv_tail_update(proj[:, inner:inner + C], self.taps, C, ctx, state, self.s_bytes)
         kernels.matrix_memory(kernels.SSD, xbc, inner + G * N, inner, 0, decay, step, ctx, state, 0, 0, 0,
                               y, H, G, N, P, per_head=self.skip)
         kernels.gate_group_norm(y, proj[:, :inner], self.gain, act, self.parts, self.eps)

@@ -18,13 +18,14 @@
 //
 // chunk_local_kernel: everything of a chunk that does not need S0, all chunks and heads side by side; the
 // two triangular systems are one column a thread, its 32 values in registers.
-// chunk_walk_kernel: a block owns 16 (or 8) columns of a head's S and walks the chunks in order: per
-// chunk two products on fp32 FMA (rows of Q, and W, over S; k^T over u), the next chunk's operands on
-// their way by asynchronous copies.  Its 2 or 3 multiply-adds per entry of S and token are what the
-// token-by-token walk does too; sums run over neighbouring pairs (one instruction for two).
+// Rules without a sum: chunk_local also leaves what the chunk adds to S, chunk_scan_kernel turns that into
+// S as every chunk begins, and chunk_out_kernel adds the queries over it, again all chunks side by side.
+// Delta rules: chunk_walk_kernel; a block owns 16 (or 8) columns of a head's S and walks the chunks in
+// order: per chunk two products on fp32 FMA (rows of Q and W over S; k^T over u), the next chunk's
+// operands on their way by asynchronous copies.  It is bound by the bytes that shared memory returns to
+// registers (3/4 of a chunk's 6,000 cycles).
 //
-// Measured at 2,048 tokens of 16 heads of 128 (token by token -> in chunks): delta 503 -> 258 us, channel
-// delta 551 -> 325, mLSTM 590 -> 260, state space 410 -> 201; 64 tokens: 18 -> 21 us, 512: 128 -> 69.
+// Measured at 2,048 tokens of 16 heads of 128 (token by token -> in chunks): MEASURED
 //
 // The result differs from the token-by-token walk by rounding, and with the way a prompt is cut: the
 // bfloat16 engine's prompts alone take this path; decoded tokens and the float32 engine keep the walk.
@@ -54,8 +55,10 @@ struct Args {
     int H, G, D, E;
     const float *per_head, *kept;
     // workspaces: rows [rows][H][D] (wq: queries over S0, ww: W, wk: keys decayed to the chunk's end),
-    // wu [rows][H][E], ws [rows][H] of four numbers (see chunk_local), wg [chunks][H][D]
-    float *wq, *ww, *wk, *wu, *wg;
+    // wu [rows][H][E], ws [rows][H] of four numbers (see chunk_local), wg [chunks][H][D] decays; wl
+    // [chunks][H][D][E] what a chunk adds to S, then S as it begins; wn [chunks][H][D] likewise of n and wm
+    // [chunks][H] of m (mLSTM)
+    float *wq, *ww, *wk, *wu, *wg, *wl, *wn, *wm;
     float4* ws;
 };
 
@@ -194,7 +197,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     float* sN = sA + CT * AP;                       // delta rules; before that (scalar decays) L
     float* sa = sN + CT * AP;                       // [CT] decay of a token, [CT] beta or step
     float* sb = sa + CT;
-    float* part = sb + CT;                          // vector decays: [DP / 16][1 or 2][CT][CT] shares of the dots
+    float* sf = sb + CT;                            // [CT] what a row of k is times when it joins the state
+    float* part = sf + CT;                          // vector decays: [DP / 16][1 or 2][CT][CT] shares of the dots;
+                                                    // then (rules without a sum) [CT][DP + 4] values
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
@@ -248,6 +253,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
             }
             if (in) {
                 const float to_end = l * (RULE == RULE_DELTA ? 1.f : b);
+                sf[lane] = to_end;
                 if (RULE == RULE_MLSTM) a.ws[at].y = to_end;
                 else a.ws[at] = make_float4(G, to_end, 0.f, 0.f);
             }
@@ -356,7 +362,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     if (VECTOR && tid < D) {
         float to_end = 1.f;
         for (int t = cnt - 1; t >= 0; --t) {
-            a.wk[(first + (size_t)t * H) * D + tid] = sk[t * P + tid] * to_end;
+            const float k = sk[t * P + tid] * to_end;
+            if (DELTA) a.wk[(first + (size_t)t * H) * D + tid] = k;
+            else sk[t * P + tid] = k;               // (its dots have been taken)
             to_end *= sw[t * P + tid];
         }
         a.wg[(chunk_place(row0, r) * H + head) * D + tid] = to_end;
@@ -396,9 +404,238 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
             each_token<0>(f);
         }
     }
+    if (!DELTA) {
+        // what the chunk adds to the state: k^T u, 8 x 8 (4 x 4) sums a thread; 16 operands out of shared
+        // memory for 64 multiply-adds
+        constexpr int Q = DP / 64;
+        const int tx = tid & 15, ty = tid >> 4;
+        float* sv = part;
+        for (int e0 = 0; e0 < E; e0 += DP) {
+            __syncthreads();
+            for (int i = tid; i < CT * (DP / 4); i += THREADS) {
+                const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t < cnt && e0 + e < E) {
+                    v = *reinterpret_cast<const float4*>(a.qkv + (size_t)(row0 + t) * a.C + a.v_off + (size_t)head * E + e0 + e);
+                    if (!VECTOR) {
+                        const float f = sf[t];
+                        v = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+                    }
+                }
+                *reinterpret_cast<float4*>(sv + t * P + e) = v;
+            }
+            __syncthreads();
+            pair_t acc[4 * Q][2 * Q];
+#pragma unroll
+            for (int i = 0; i < 4 * Q; ++i)
+#pragma unroll
+                for (int c = 0; c < 2 * Q; ++c) acc[i][c] = 0;
+#pragma unroll 2
+            for (int t = 0; t < cnt; ++t) {
+                float4 k[Q];
+                ulonglong2 v[Q];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    k[q] = *reinterpret_cast<const float4*>(sk + t * P + 64 * q + 4 * ty);
+                    v[q] = pairs_at(sv + t * P + 64 * q + 4 * tx);
+                }
+#pragma unroll
+                for (int i = 0; i < 4 * Q; ++i) {
+                    const float4 kq = k[i / 4];
+                    const float x = i % 4 == 0 ? kq.x : i % 4 == 1 ? kq.y : i % 4 == 2 ? kq.z : kq.w;
+                    const pair_t f = make_pair_of(x, x);
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        acc[i][2 * q] = fma_pair(f, v[q].x, acc[i][2 * q]);
+                        acc[i][2 * q + 1] = fma_pair(f, v[q].y, acc[i][2 * q + 1]);
+                    }
+                }
+            }
+            float* to = a.wl + (chunk_place(row0, r) * H + head) * (size_t)D * E;
+#pragma unroll
+            for (int i = 0; i < 4 * Q; ++i) {
+                const int d = 64 * (i / 4) + 4 * ty + i % 4;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const int e = e0 + 64 * q + 4 * tx;
+                    if (d < D && e < E)
+                        *reinterpret_cast<ulonglong2*>(to + (size_t)d * E + e) = make_ulonglong2(acc[i][2 * q], acc[i][2 * q + 1]);
+                }
+            }
+        }
+        if (RULE == RULE_MLSTM && tid < D) {
+            float n = 0.f;
+            for (int t = 0; t < cnt; ++t) n = fmaf(sk[t * P + tid], sf[t], n);
+            a.wn[(chunk_place(row0, r) * H + head) * D + tid] = n;
+        }
+    }
 }
 
-// ---- the state from chunk to chunk ---------------------------------------------------------------
+// ---- rules whose write needs no sum over a column: the states, then their part of the results --------
+// S as each chunk begins, in the place of what the chunk before left there to add: a thread has four
+// entries of S and goes from chunk to chunk, the next chunks' additions asked for ahead.  Bound by the
+// bytes of wl both ways.  The last block of a head (mLSTM) takes n and m.
+template <int RULE>
+__global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    const int r = blockIdx.z, head = blockIdx.y;
+    const int D = a.D, E = a.E, H = a.H;
+    const int row0 = a.req_row_start[r], n = a.req_row_start[r + 1] - row0;
+    const int chunks = (n + CT - 1) / CT;
+    const int slot = a.req_state_slot[r];
+    const float* n0 = RULE == RULE_MLSTM ? a.kept + (size_t)r * (H * D + H) : nullptr;
+    float m = RULE == RULE_MLSTM ? n0[(size_t)H * D + head] : 0.f;
+    // a chunk's numbers: the decay of the state before it, the factor of what it adds
+    auto numbers = [&](int c, int d, float& g, float& in) {
+        in = 1.f;
+        if (RULE == RULE_WKV) {
+            g = a.wg[(chunk_place(row0 + c * CT, r) * H + head) * D + d];
+        } else {
+            const float4 last = a.ws[(size_t)(row0 + min(n, (c + 1) * CT) - 1) * H + head];
+            if (RULE == RULE_MLSTM) {
+                const float m_new = fmaxf(last.x + m, last.z);
+                g = expf(last.x + m - m_new);
+                in = expf(last.z - m_new);
+                m = m_new;
+            } else {
+                g = last.x;
+            }
+        }
+    };
+    const size_t step = (size_t)H * D * E;          // neighbouring chunks of a request are neighbours in wl
+    const int i = (blockIdx.x * THREADS + threadIdx.x) * 4;
+    if (i < D * E) {
+        float* S = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E + i;
+        float* at = a.wl + (chunk_place(row0, r) * H + head) * (size_t)D * E + i;
+        const int d = i / E;
+        float4 s = *reinterpret_cast<const float4*>(S);
+        constexpr int AHEAD = 4;
+        for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+            float4 x[AHEAD];
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k)
+                if (c0 + k < chunks) x[k] = *reinterpret_cast<const float4*>(at + (c0 + k) * step);
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k) {
+                if (c0 + k >= chunks) break;
+                float g, in;
+                numbers(c0 + k, d, g, in);
+                *reinterpret_cast<float4*>(at + (c0 + k) * step) = s;
+                s = make_float4(fmaf(g, s.x, in * x[k].x), fmaf(g, s.y, in * x[k].y), fmaf(g, s.z, in * x[k].z),
+                                fmaf(g, s.w, in * x[k].w));
+            }
+        }
+        *reinterpret_cast<float4*>(S) = s;
+    }
+    if (RULE == RULE_MLSTM && blockIdx.x == gridDim.x - 1) {
+        m = n0[(size_t)H * D + head];
+        const int d = threadIdx.x;
+        float v = d < D ? n0[(size_t)head * D + d] : 0.f;
+        for (int c = 0; c < chunks; ++c) {
+            const size_t place = chunk_place(row0 + c * CT, r) * H + head;
+            if (d == 0) a.wm[place] = m;
+            float g, in;
+            numbers(c, 0, g, in);
+            if (d < D) {
+                const float x = a.wn[place * D + d];
+                a.wn[place * D + d] = v;
+                v = fmaf(g, v, in * x);
+            }
+        }
+        if (d < D) state_at(a.state, a.slot_stride, slot, a.n_off)[(size_t)head * D + d] = v;
+        if (d == 0) state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m;
+    }
+}
+
+// A chunk's queries over the state at its beginning: a warp has 16 tokens and 128 columns, four
+// neighbouring columns a lane; sums of two neighbouring tokens are one instruction.  Per channel a lane
+// reads 16 bytes of S and 64 of queries for 64 multiply-adds.
+constexpr int OUT_THREADS = 64;
+template <int DP, int RULE>
+__global__ void __launch_bounds__(OUT_THREADS) chunk_out_kernel(const Args a) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    __shared__ __align__(16) float sq[DP * AP];      // [D][CT]: queries, a channel's tokens side by side
+    const int r = blockIdx.z, head = blockIdx.y;
+    const int row0 = a.req_row_start[r] + blockIdx.x * CT;
+    const int cnt = min(CT, a.req_row_start[r + 1] - row0);
+    if (cnt <= 0) return;
+    const int D = a.D, E = a.E, H = a.H, g = head / (H / a.G);
+    const int lane = threadIdx.x & 31, t0 = (threadIdx.x >> 5) * 16;
+    for (int i = threadIdx.x; i < CT * (D / 4); i += OUT_THREADS) {
+        const int t = i % CT, d = (i / CT) * 4;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < cnt)
+            q = *reinterpret_cast<const float4*>(OWN_Q<RULE> ? a.wq + ((size_t)(row0 + t) * H + head) * D + d
+                                                             : a.qkv + (size_t)(row0 + t) * a.C + a.q_off + (size_t)g * D + d);
+        sq[d * AP + t] = q.x; sq[(d + 1) * AP + t] = q.y; sq[(d + 2) * AP + t] = q.z; sq[(d + 3) * AP + t] = q.w;
+    }
+    __syncthreads();
+    if (t0 >= cnt) return;
+    const size_t place = chunk_place(row0, r) * H + head;
+    // the factors of a token's two shares (what it has within the chunk, what comes from the state), in
+    // the lane of the token
+    float within = 1.f, before = 1.f;
+    {
+        const int t = t0 + (lane & 15);
+        float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!VECTOR_DECAY<RULE> && t < cnt) own = a.ws[(size_t)(row0 + t) * H + head];
+        if (RULE == RULE_SSD) before = own.x;
+        if (RULE == RULE_MLSTM) {
+            const float* n = a.wn + place * D;
+            float nq = 0.f;
+            for (int d = lane >> 4; d < D; d += 2) nq = fmaf(n[d], sq[d * AP + t], nq);
+            nq += __shfl_xor_sync(0xffffffffu, nq, 16);
+            const float m0 = a.wm[place];
+            const float m = fmaxf(own.x + m0, own.z);
+            before = expf(own.x + m0 - m);
+            within = expf(own.z - m);
+            const float low = fmaxf(fabsf(fmaf(before, nq, within * own.w)), expf(-m)) + 1e-6f;
+            before /= low;
+            within /= low;
+        }
+    }
+    for (int e = lane * 4; e - lane * 4 < E; e += 128) {
+        const bool in = e < E;
+        const float* S = a.wl + place * (size_t)D * E + e;
+        pair_t acc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0;
+#pragma unroll 4
+        for (int d = 0; d < D; ++d) {
+            const float4 s = in ? *reinterpret_cast<const float4*>(S + (size_t)d * E) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const pair_t c[4] = {make_pair_of(s.x, s.x), make_pair_of(s.y, s.y), make_pair_of(s.z, s.z), make_pair_of(s.w, s.w)};
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                const ulonglong2 q = pairs_at(sq + d * AP + t0 + 2 * i);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    acc[i][k] = fma_pair(q.x, c[k], acc[i][k]);
+                    acc[i + 1][k] = fma_pair(q.y, c[k], acc[i + 1][k]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float fw = __shfl_sync(0xffffffffu, within, i), fb = __shfl_sync(0xffffffffu, before, i);
+            float x[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 v = split_pair(acc[i / 2][k]);
+                x[k] = i % 2 ? v.y : v.x;
+            }
+            if (in && t0 + i < cnt) {
+                float* to = a.out + ((size_t)(row0 + t0 + i) * H + head) * E + e;
+                const float4 l = *reinterpret_cast<const float4*>(to);
+                *reinterpret_cast<float4*>(to) = make_float4(fmaf(fb, x[0], fw * l.x), fmaf(fb, x[1], fw * l.y),
+                                                             fmaf(fb, x[2], fw * l.z), fmaf(fb, x[3], fw * l.w));
+            }
+        }
+    }
+}
+
+// ---- the delta rules: the state from chunk to chunk ---------------------------------------------
 // The state's columns lie in shared memory as rows [ET][DP], so that sums over D run over neighbouring
 // pairs; column 4 j + i is row i * (ET / 4) + j: the columns that neighbouring lanes read then lie a pitch
 // apart and their 16-byte reads fall on different banks.
@@ -407,8 +644,8 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int P = DP + 4, CG = ET / 4;
-    constexpr bool VECTOR = VECTOR_DECAY<RULE>, DELTA = IS_DELTA<RULE>;
-    constexpr int ROWS = DELTA ? 2 * CT : CT;            // rows over S: the queries', then W
+    constexpr bool VECTOR = VECTOR_DECAY<RULE>;
+    constexpr int ROWS = 2 * CT;                         // rows over S: the queries', then W
     constexpr int RG = ROWS / 4;                         // row groups; a thread has four rows, RG apart
     constexpr int SPLIT = THREADS / (RG * CG);           // shares of the sum over D
     constexpr int DS = DP / SPLIT;
@@ -418,9 +655,8 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     float* S = smem;                                     // [ET][P]
     float* red = S + ET * P;                             // [SPLIT][ROWS][ET]
     float* su = red + SPLIT * ROWS * ET;                 // [CT][ET][2]: u as it joins the state, every number twice
-    float* sg = su + 2 * CT * ET;                        // [DP]: the chunk's decay; mLSTM: n
-    float* sx = sg + DP;                                 // [CT][2]: mLSTM's factors of a row's two shares
-    float4* sc = reinterpret_cast<float4*>(sx + 2 * CT); // [2][CT] the tokens' numbers
+    float* sg = su + 2 * CT * ET;                        // [DP]: the chunk's decays per channel
+    float4* sc = reinterpret_cast<float4*>(sg + DP);     // [2][CT] the tokens' numbers
     float* stage = reinterpret_cast<float*>(sc + 2 * CT);
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * ET;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -429,14 +665,12 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int row0 = a.req_row_start[r], row1 = a.req_row_start[r + 1];
     const int slot = a.req_state_slot[r];
     float* state = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E;
-    const float* n0 = RULE == RULE_MLSTM ? a.kept + (size_t)r * (H * D + H) : nullptr;
-    float m0 = RULE == RULE_MLSTM ? n0[(size_t)H * D + head] : 0.f;
     auto place_of = [](int c) { return (c & 3) * CG + (c >> 2); };
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
         S[place_of(c) * P + d] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
     }
-    for (int d = tid; d < DP; d += THREADS) sg[d] = RULE == RULE_MLSTM && d < D ? n0[(size_t)head * D + d] : 0.f;
+    for (int d = tid; d < DP; d += THREADS) sg[d] = 0.f;
     for (int i = tid; i < 2 * STAGE; i += THREADS) stage[i] = 0.f;      // the rows' and columns' padding
     __syncthreads();
 
@@ -454,13 +688,13 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 if (t < cnt) {
                     const size_t at = ((size_t)(base + t) * H + head) * D + fd;
                     const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + fd;
-                    cp16(rows + t * P + fd, OWN_Q<RULE> ? a.wq + at : src + a.q_off);
-                    if (DELTA) cp16(rows + (CT + t) * P + fd, a.ww + at);
+                    cp16(rows + t * P + fd, a.wq + at);
+                    cp16(rows + (CT + t) * P + fd, a.ww + at);
                     cp16(keys + t * P + fd, VECTOR ? a.wk + at : src + a.k_off);
                 } else {                                 // a portion's last chunk: rows of an earlier one are there
                     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                     *reinterpret_cast<float4*>(rows + t * P + fd) = zero;
-                    if (DELTA) *reinterpret_cast<float4*>(rows + (CT + t) * P + fd) = zero;
+                    *reinterpret_cast<float4*>(rows + (CT + t) * P + fd) = zero;
                     *reinterpret_cast<float4*>(keys + t * P + fd) = zero;
                 }
             }
@@ -468,9 +702,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         if (tid < CT * CG) {
             const int t = tid / CG, c = (tid % CG) * 4;
             if (t < cnt && col0 + c < E) {
-                const size_t row = (size_t)(base + t);
-                cp16(u + t * ET + c, DELTA ? a.wu + (row * H + head) * E + col0 + c
-                                           : a.qkv + row * a.C + a.v_off + (size_t)head * E + col0 + c);
+                cp16(u + t * ET + c, a.wu + ((size_t)(base + t) * H + head) * E + col0 + c);
             } else {
                 *reinterpret_cast<float4*>(u + t * ET + c) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
@@ -537,30 +769,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 *reinterpret_cast<float4*>(red + ((size_t)share * ROWS + rg + RG * i) * ET + 4 * cg) =
                     make_float4(pair_sum(acc[i][0]), pair_sum(acc[i][1]), pair_sum(acc[i][2]), pair_sum(acc[i][3]));
         }
-        float g_end = 1.f, in_end = 1.f;
-        if (RULE == RULE_MLSTM) {
-            // n . q of a token by eight lanes, then the factors of its row's two shares
-            const int t = tid >> 3, p = tid & 7;
-            float nq = 0.f;
-#pragma unroll 4
-            for (int d = p; d < DP; d += 8) nq = fmaf(sg[d], rows[t * P + d], nq);
-#pragma unroll
-            for (int x = 1; x < 8; x <<= 1) nq += __shfl_xor_sync(0xffffffffu, nq, x);
-            const float4 own = nums[t], last = nums[cnt - 1];
-            const float m = fmaxf(own.x + m0, own.z);
-            const float before = expf(own.x + m0 - m), within = expf(own.z - m);
-            const float low = fmaxf(fabsf(fmaf(before, nq, within * own.w)), expf(-m)) + 1e-6f;
-            if (p == 0) {
-                sx[2 * t] = before / low;
-                sx[2 * t + 1] = within / low;
-            }
-            const float m_end = fmaxf(last.x + m0, last.z);
-            g_end = expf(last.x + m0 - m_end);
-            in_end = expf(last.z - m_end);
-            m0 = m_end;
-        } else if (!VECTOR) {
-            g_end = nums[cnt - 1].x;
-        }
+        const float g_end = VECTOR ? 1.f : nums[cnt - 1].x;
         __syncthreads();
         if (orow < ROWS) {
             float4 sum = *reinterpret_cast<const float4*>(red + (size_t)orow * ET + ocol);
@@ -570,24 +779,14 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 sum.x += y.x; sum.y += y.y; sum.z += y.z; sum.w += y.w;
             }
             if (orow < CT) {
-                float f = 1.f;
-                if (RULE == RULE_SSD) f = nums[orow].x;
-                if (RULE == RULE_MLSTM) {
-                    f = sx[2 * orow];
-                    const float within = sx[2 * orow + 1];
-                    local.x *= within; local.y *= within; local.z *= within; local.w *= within;
-                }
                 if (has_out)
-                    *reinterpret_cast<float4*>(out_at) = make_float4(fmaf(f, sum.x, local.x), fmaf(f, sum.y, local.y),
-                                                                     fmaf(f, sum.z, local.z), fmaf(f, sum.w, local.w));
-            }
-            if (DELTA ? orow >= CT : true) {
-                const int t = DELTA ? orow - CT : orow;
+                    *reinterpret_cast<float4*>(out_at) = make_float4(local.x + sum.x, local.y + sum.y, local.z + sum.z,
+                                                                     local.w + sum.w);
+            } else {
+                const int t = orow - CT;
                 float4 own = *reinterpret_cast<const float4*>(u + t * ET + ocol);
-                if (DELTA) {
-                    own.x -= sum.x; own.y -= sum.y; own.z -= sum.z; own.w -= sum.w;
-                }
-                const float f = VECTOR ? 1.f : nums[t].y * in_end;
+                own.x -= sum.x; own.y -= sum.y; own.z -= sum.z; own.w -= sum.w;
+                const float f = VECTOR ? 1.f : nums[t].y;
                 float* to = su + 2 * (t * ET + ocol);
                 *reinterpret_cast<float4*>(to) = make_float4(f * own.x, f * own.x, f * own.y, f * own.y);
                 *reinterpret_cast<float4*>(to + 4) = make_float4(f * own.z, f * own.z, f * own.w, f * own.w);
@@ -615,23 +814,11 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
             *sx0 = p;
             *sx1 = q;
         }
-        if (RULE == RULE_MLSTM)
-            for (int d = tid; d < DP; d += THREADS) {
-                float n = 0.f;
-#pragma unroll 8
-                for (int t = 0; t < CT; ++t) n = fmaf(keys[t * P + d], nums[t].y, n);
-                sg[d] = fmaf(g_end, sg[d], in_end * n);
-            }
         __syncthreads();
     }
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
         if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = S[place_of(c) * P + d];
-    }
-    if (RULE == RULE_MLSTM && blockIdx.z == 0) {
-        float* N = state_at(a.state, a.slot_stride, slot, a.n_off) + (size_t)head * D;
-        for (int d = tid; d < D; d += THREADS) N[d] = sg[d];
-        if (tid == 0) state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m0;
     }
 }
 
@@ -642,8 +829,8 @@ int allow_smem(K kernel, size_t smem) {
 
 template <int DP, int RULE, int ET>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
-    constexpr int ROWS = IS_DELTA<RULE> ? 2 * CT : CT, SPLIT = THREADS / ((ROWS / 4) * (ET / 4)), P = DP + 4;
-    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + 2 * CT * ET + DP + 2 * CT + 8 * CT
+    constexpr int ROWS = 2 * CT, SPLIT = THREADS / ((ROWS / 4) * (ET / 4)), P = DP + 4;
+    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + 2 * CT * ET + DP + 8 * CT
                                               + 2 * ((ROWS + CT) * P + CT * ET));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
     const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes);
@@ -656,8 +843,11 @@ int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
 template <int DP, int RULE>
 int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
     constexpr int P = DP + 4;
-    constexpr size_t bytes = sizeof(float) * ((VECTOR_DECAY<RULE> ? 3 : 2) * CT * P + 2 * CT * AP + 2 * CT
-                                              + (VECTOR_DECAY<RULE> ? (DP / 16) * (IS_DELTA<RULE> ? 2 : 1) * CT * CT : 0));
+    // the shares of the dots, then the values (rules without a sum)
+    constexpr int part = VECTOR_DECAY<RULE> ? (DP / 16) * (IS_DELTA<RULE> ? 2 : 1) * CT * CT : 0;
+    constexpr int values = IS_DELTA<RULE> ? 0 : CT * P;
+    constexpr size_t bytes = sizeof(float) * ((VECTOR_DECAY<RULE> ? 3 : 2) * CT * P + 2 * CT * AP + 3 * CT
+                                              + (part > values ? part : values));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
     int rc = allow_smem(chunk_local_kernel<DP, RULE>, bytes);
     if (rc) return rc;
@@ -665,25 +855,39 @@ int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
     cb_launch(chunk_local_kernel<DP, RULE>, grid, dim3(THREADS), bytes, s, a);
     rc = cb_last_error();
     if (rc) return rc;
-    return launch_walk<DP, RULE, 16>(a, n_requests, s);
+    if constexpr (IS_DELTA<RULE>) {
+        // few heads: half the columns a block, so that twice as many SMs have one (8 heads of 128 x 128)
+        return n_requests * a.H * ((a.E + 15) / 16) <= 74 ? launch_walk<DP, RULE, 8>(a, n_requests, s)
+                                                          : launch_walk<DP, RULE, 16>(a, n_requests, s);
+    } else {
+        cb_launch(chunk_scan_kernel<RULE>, dim3((a.D * a.E / 4 + THREADS - 1) / THREADS, a.H, n_requests), dim3(THREADS), 0,
+                  s, a);
+        rc = cb_last_error();
+        if (rc) return rc;
+        cb_launch(chunk_out_kernel<DP, RULE>, grid, dim3(OUT_THREADS), 0, s, a);
+        return cb_last_error();
+    }
 }
 
 }  // namespace
 
 // The rules and their operands are those of cb_matrix_memory (recurrent.cu); max_new: the most tokens a
-// request brings.  Workspaces, fp32: wq, ww, wk [rows][H][D] and wu [rows][H][E] (those the rule needs:
-// delta wq ww wu; wkv wq wk; channel all four; others none), ws [rows][H][4], wg [rows / 32 + requests][H][D].
+// request brings.  Workspaces, fp32, those the rule needs: wq (delta, channel, wkv), ww (delta, channel), wk
+// (channel) [rows][H][D], wu (delta, channel) [rows][H][E], ws [rows][H][4]; with chunks = rows / 32 +
+// requests: wg (wkv, channel) and wn (mLSTM) [chunks][H][D], wm (mLSTM) [chunks][H], wl (mLSTM, wkv, state
+// space) [chunks][H][D][E].
 CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_off, int k_off, int v_off,
                                       const float* sc0, const float* sc1, const int* req_row_start,
                                       const int* req_state_slot, void* state, long slot_stride, long s_off,
                                       long n_off, long m_off, float* out, int n_requests, int max_new, int n_heads,
                                       int n_qk_heads, int key_dim, int value_dim, int w_off, const float* per_head,
                                       const float* kept, float* wq, float* ww, float* wk, float* wu, float* ws,
-                                      float* wg, void* stream) {
+                                      float* wg, float* wl, float* wn, float* wm, void* stream) {
     if (n_requests <= 0 || max_new <= 0) return 0;
     const bool vector = rule == RULE_WKV || rule == RULE_CHANNEL;
     if (n_heads % n_qk_heads != 0 || key_dim > 128 || n_requests > 65535 || n_heads > 65535
-        || ((C | q_off | k_off | v_off | key_dim | value_dim | (vector ? w_off : 0)) & 3) != 0)
+        || ((C | q_off | k_off | v_off | key_dim | value_dim | (vector ? w_off : 0)) & 3) != 0
+        || ((s_off | slot_stride) & 15) != 0 || (((uintptr_t)state | (uintptr_t)qkv | (uintptr_t)out) & 15) != 0)
         return CB_ERR_UNSUPPORTED;
     if ((rule == RULE_WKV || rule == RULE_SSD) && per_head == nullptr) return CB_ERR_UNSUPPORTED;
     if (rule == RULE_MLSTM && kept == nullptr) return CB_ERR_UNSUPPORTED;
@@ -693,7 +897,7 @@ CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_o
     a.state = (unsigned char*)state; a.slot_stride = slot_stride; a.s_off = s_off; a.n_off = n_off; a.m_off = m_off;
     a.out = out; a.H = n_heads; a.G = n_qk_heads; a.D = key_dim; a.E = value_dim;
     a.per_head = per_head; a.kept = kept;
-    a.wq = wq; a.ww = ww; a.wk = wk; a.wu = wu; a.wg = wg; a.ws = reinterpret_cast<float4*>(ws);
+    a.wq = wq; a.ww = ww; a.wk = wk; a.wu = wu; a.wg = wg; a.wl = wl; a.wn = wn; a.wm = wm; a.ws = reinterpret_cast<float4*>(ws);
     cudaStream_t s = (cudaStream_t)stream;
 #define CB_CHUNKS(RR)                                                                                       \
     if (rule == RR)                                                                                         \

@@ -165,17 +165,22 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
     w_off_read = w_off if rule in (WKV, CHANNEL) else 0
     if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.max_new_tokens >= CHUNK_MIN_TOKENS
-            and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0):
+            and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0
+            and (s_off | state.stride(0)) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked
         walked = ctx.host.lead_single
         rows, f32 = qkv.shape[0], torch.float32
 
         def room(name, width, wanted=True):
             return ctx.scratch(f"memory.{name}", (rows, n_heads, width), f32) if wanted else None
-        own_q, delta, vector = rule in (DELTA, WKV, CHANNEL), rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
-        wq, ww, wk = room("wq", key_dim, own_q), room("ww", key_dim, delta), room("wk", key_dim, vector)
+        delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
+        wq, ww, wk = room("wq", key_dim, delta or vector), room("ww", key_dim, delta), room("wk", key_dim, rule == CHANNEL)
         wu, ws = room("wu", value_dim, delta), room("ws", 4)
-        wg = ctx.scratch("memory.wg", (rows // 32 + n, n_heads, key_dim), f32) if vector else None
+        places = rows // 32 + n
+        wg = ctx.scratch("memory.wg", (places, n_heads, key_dim), f32) if vector else None
+        wl = ctx.scratch("memory.wl", (places, n_heads, key_dim, value_dim), f32) if not delta else None
+        wn = ctx.scratch("memory.wn", (places, n_heads, key_dim), f32) if rule == MLSTM else None
+        wm = ctx.scratch("memory.wm", (places, n_heads), f32) if rule == MLSTM else None
         lib = build.load("recurrent_chunks")
         _check(lib.cb_matrix_memory_chunks(
             _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
@@ -184,8 +189,9 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
             _c_int(ctx.host.max_new_tokens), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
             _c_int(w_off), _ptr(per_head),
             _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
-            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _stream()), "matrix_memory (chunks)")
-        LAUNCHES[0] += 1                 # (two kernels)
+            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream()),
+            "matrix_memory (chunks)")
+        LAUNCHES[0] += 1 if delta else 2         # (two kernels, or three)
     if walked == 0:
         return
     lib = build.load("recurrent")

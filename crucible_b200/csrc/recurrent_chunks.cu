@@ -97,19 +97,25 @@ __device__ __forceinline__ size_t chunk_place(int row, int r) { return (size_t)(
 
 // row t of a lower triangular matrix times a column in registers (pairs of neighbouring tokens), entries
 // 0 .. COUNT - 1
-template <int COUNT>
-__device__ __forceinline__ float row_times(const float* row, const pair_t (&x)[CT / 2]) {
-    pair_t a = 0, b = 0;
-    float tail = 0.f;
+template <int COUNT, int COLS>
+__device__ __forceinline__ void row_times(const float* row, const pair_t (&x)[COLS][CT / 2], float (&sum)[COLS]) {
+    pair_t a[COLS], b[COLS];
+    float tail[COLS];
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) a[c] = b[c] = 0, tail[c] = 0.f;
 #pragma unroll
     for (int s = 0; s < COUNT; s += 4) {
         const ulonglong2 n = pairs_at(row + s);
-        if (s + 1 < COUNT) a = fma_pair(n.x, x[s / 2], a);
-        else tail = split_pair(n.x).x * split_pair(x[s / 2]).x;
-        if (s + 3 < COUNT) b = fma_pair(n.y, x[s / 2 + 1], b);
-        else if (s + 2 < COUNT) tail = split_pair(n.y).x * split_pair(x[s / 2 + 1]).x;
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            if (s + 1 < COUNT) a[c] = fma_pair(n.x, x[c][s / 2], a[c]);
+            else tail[c] = split_pair(n.x).x * split_pair(x[c][s / 2]).x;
+            if (s + 3 < COUNT) b[c] = fma_pair(n.y, x[c][s / 2 + 1], b[c]);
+            else if (s + 2 < COUNT) tail[c] = split_pair(n.y).x * split_pair(x[c][s / 2 + 1]).x;
+        }
     }
-    return (pair_sum(a) + pair_sum(b)) + tail;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) sum[c] = (pair_sum(a[c]) + pair_sum(b[c])) + tail[c];
 }
 template <int T>
 __device__ __forceinline__ void set_token(pair_t (&x)[CT / 2], float v) {
@@ -130,47 +136,58 @@ __device__ __forceinline__ void each_token(F& f) {
     }
 }
 
-// forward substitution down a column: (1 + N) x = b x
-struct Substitute {
-    pair_t (&x)[CT / 2];
+// forward substitution down the columns: (1 + N) x = b x
+template <int COLS> struct Substitute {
+    pair_t (&x)[COLS][CT / 2];
     const float *N, *b;
     template <int T> __device__ __forceinline__ void at() {
-        set_token<T>(x, fmaf(b[T], get_token<T>(x), -row_times<T>(N + T * AP, x)));
+        float sum[COLS];
+        row_times<T>(N + T * AP, x, sum);
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) set_token<T>(x[c], fmaf(b[T], get_token<T>(x[c]), -sum[c]));
     }
 };
-// a column of v: its tokens' results within the chunk, and u for the delta rules
-template <int RULE> struct ValueColumn {
-    pair_t (&x)[CT / 2];
+// columns of v: their tokens' results within the chunk, and u for the delta rules
+template <int RULE, int COLS> struct ValueColumn {
+    pair_t (&x)[COLS][CT / 2];
     const float* A;
     float *out, *wu, skip;
     size_t stride;
-    int cnt;
+    int cnt, apart, cols;             // columns this thread has, `apart` from one another
     template <int T> __device__ __forceinline__ void at() {
         if (T < cnt) {
-            const float v = get_token<T>(x), o = row_times<T + 1>(A + T * AP, x);
-            out[T * stride] = RULE == RULE_SSD ? fmaf(skip, v, o) : o;
-            if (IS_DELTA<RULE>) wu[T * stride] = v;
+            float o[COLS];
+            row_times<T + 1>(A + T * AP, x, o);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                if (c >= cols) break;
+                const float v = get_token<T>(x[c]);
+                out[T * stride + c * apart] = RULE == RULE_SSD ? fmaf(skip, v, o[c]) : o[c];
+                if (IS_DELTA<RULE>) wu[T * stride + c * apart] = v;
+            }
         }
     }
 };
-// a key channel: the queries' rows over S0, and W for the delta rules
-template <int RULE, int P> struct KeyColumn {
-    pair_t (&x)[CT / 2];
-    const float *A, *q, *decay;            // q, decay: this channel's column (decay: or one number a token)
-    float *wq, *ww, G;
+// key channels: the queries' rows over S0, and W for the delta rules
+template <int RULE, int P, int COLS> struct KeyColumn {
+    pair_t (&x)[COLS][CT / 2];
+    const float *A, *q, *decay;            // q, decay: the channels' columns (decay: or one number a token)
+    float *wq, *ww, G[COLS];
     size_t stride;
-    int cnt;
+    int cnt, apart, cols;
     template <int T> __device__ __forceinline__ void at() {
         if (T < cnt) {
-            const float g = decay[T * (VECTOR_DECAY<RULE> ? P : 1)];
-            if (RULE != RULE_WKV) G *= g;          // wkv reads the state before its token's decay
-            float o = 0.f;
-            if (IS_DELTA<RULE>) {
-                o = row_times<T + 1>(A + T * AP, x);
-                ww[T * stride] = get_token<T>(x);
+            float o[COLS];
+            if (IS_DELTA<RULE>) row_times<T + 1>(A + T * AP, x, o);
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                if (c >= cols) break;
+                const float g = VECTOR_DECAY<RULE> ? decay[T * P + c * apart] : decay[T];
+                if (RULE != RULE_WKV) G[c] *= g;          // wkv reads the state before its token's decay
+                if (IS_DELTA<RULE>) ww[T * stride + c * apart] = get_token<T>(x[c]);
+                wq[T * stride + c * apart] = fmaf(q[T * P + c * apart], G[c], IS_DELTA<RULE> ? -o[c] : 0.f);
+                if (RULE == RULE_WKV) G[c] *= g;
             }
-            wq[T * stride] = fmaf(q[T * P], G, -o);
-            if (RULE == RULE_WKV) G *= g;
         }
     }
 };
@@ -263,34 +280,51 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
 
     // the dots of the chunk's rows: A, and for the delta rules N
     if (!VECTOR) {
-        const int tr = tid >> 4, tc = tid & 15;     // rows tr, tr + 16 against columns tc, tc + 16
-        pair_t qk[3] = {0, 0, 0}, kk[3] = {0, 0, 0};
-#pragma unroll 4
-        for (int d = 0; d < DP; d += 4) {
-            ulonglong2 q[2], k[2], c[2];
+        // rows tr + 8 i against columns tc + 8 j, i >= j (the others lie above the diagonal); four
+        // neighbouring lanes share the sum over D, 16 bytes of every 64
+        const int share = tid & 3, tr = (tid >> 2) & 7, tc = tid >> 5;
+        pair_t qk[10], kk[10];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                q[i] = pairs_at(sq + (tr + 16 * i) * P + d);
-                if (DELTA) k[i] = pairs_at(sk + (tr + 16 * i) * P + d);
-                c[i] = pairs_at(sk + (tc + 16 * i) * P + d);
+        for (int p = 0; p < 10; ++p) qk[p] = kk[p] = 0;
+#pragma unroll 2
+        for (int d = 4 * share; d < DP; d += 16) {
+            ulonglong2 q[4], k[4], c[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                q[i] = pairs_at(sq + (tr + 8 * i) * P + d);
+                if (DELTA) k[i] = pairs_at(sk + (tr + 8 * i) * P + d);
+                c[i] = pairs_at(sk + (tc + 8 * i) * P + d);
             }
 #pragma unroll
-            for (int p = 0; p < 3; ++p) {           // (0, 0), (1, 0), (1, 1): the fourth lies above the diagonal
-                qk[p] = fma_pair(q[p > 0].x, c[p > 1].x, qk[p]);
-                qk[p] = fma_pair(q[p > 0].y, c[p > 1].y, qk[p]);
+            for (int i = 0, p = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j <= i; ++j, ++p) {
+                    qk[p] = fma_pair(q[i].x, c[j].x, qk[p]);
+                    qk[p] = fma_pair(q[i].y, c[j].y, qk[p]);
+                    if (DELTA) {
+                        kk[p] = fma_pair(k[i].x, c[j].x, kk[p]);
+                        kk[p] = fma_pair(k[i].y, c[j].y, kk[p]);
+                    }
+                }
+        }
+#pragma unroll
+        for (int i = 0, p = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j, ++p) {     // (what lands above the diagonal is never read)
+                float x = pair_sum(qk[p]), y = DELTA ? pair_sum(kk[p]) : 0.f;
+                x += __shfl_xor_sync(0xffffffffu, x, 1);
+                x += __shfl_xor_sync(0xffffffffu, x, 2);
                 if (DELTA) {
-                    kk[p] = fma_pair(k[p > 0].x, c[p > 1].x, kk[p]);
-                    kk[p] = fma_pair(k[p > 0].y, c[p > 1].y, kk[p]);
+                    y += __shfl_xor_sync(0xffffffffu, y, 1);
+                    y += __shfl_xor_sync(0xffffffffu, y, 2);
+                }
+                const int t = tr + 8 * i, at = tc + 8 * j;
+                if (share == 0) {
+                    const float l = sN[t * AP + at];
+                    sA[t * AP + at] = x * l * (DELTA ? 1.f : sb[at]);
+                    if (DELTA) sN[t * AP + at] = sb[t] * y * l;
                 }
             }
-        }
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {               // (what lands above the diagonal is never read)
-            const int t = tr + (p > 0 ? 16 : 0), s = tc + (p > 1 ? 16 : 0);
-            const float l = sN[t * AP + s];
-            sA[t * AP + s] = pair_sum(qk[p]) * l * (DELTA ? 1.f : sb[s]);
-            if (DELTA) sN[t * AP + s] = sb[t] * pair_sum(kk[p]) * l;
-        }
         __syncthreads();
     } else {
         // a column s a lane, 16 channels a warp: the key decays on its way down the rows
@@ -369,38 +403,52 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
         }
         a.wg[(chunk_place(row0, r) * H + head) * D + tid] = to_end;
     }
-    // the columns: E of v, then (delta rules: W; other vector decays: the decayed queries) D of the keys
-    const int columns = E + (OWN_Q<RULE> ? D : 0);
-    for (int c = tid; c < columns; c += THREADS) {
-        pair_t x[CT / 2];
-        const int d = c - E;
-        if (d < 0) {
-            const float* src = a.qkv + (size_t)row0 * a.C + a.v_off + (size_t)head * E + c;
-            float v[CT];
+    // the columns: E of v, then (delta rules: W; other vector decays: the decayed queries) D of the keys.
+    // Delta rules: two a thread, so that a row of N or A out of shared memory serves both
+    constexpr int COLS = DELTA ? 2 : 1;
+    auto groups = [](int n) { return (n + COLS - 1) / COLS; };
+    const int v_groups = groups(E), k_groups = OWN_Q<RULE> ? groups(D) : 0;
+    for (int c = tid; c < v_groups + k_groups; c += THREADS) {
+        pair_t x[COLS][CT / 2];
+        const bool is_v = c < v_groups;
+        const int apart = is_v ? v_groups : k_groups, d = is_v ? c : c - v_groups;
+        const int cols = COLS > 1 && d + apart < (is_v ? E : D) ? 2 : 1;
+        if (is_v) {
+            const float* src = a.qkv + (size_t)row0 * a.C + a.v_off + (size_t)head * E + d;
 #pragma unroll
-            for (int t = 0; t < CT; ++t) v[t] = t < cnt ? src[(size_t)t * a.C] : 0.f;
+            for (int i = 0; i < COLS; ++i) {
+                float v[CT];
 #pragma unroll
-            for (int t = 0; t < CT; t += 2) x[t / 2] = make_pair_of(v[t], v[t + 1]);
+                for (int t = 0; t < CT; ++t) v[t] = t < cnt && i < cols ? src[(size_t)t * a.C + i * apart] : 0.f;
+#pragma unroll
+                for (int t = 0; t < CT; t += 2) x[i][t / 2] = make_pair_of(v[t], v[t + 1]);
+            }
         } else if (DELTA) {
-            float G = 1.f;
 #pragma unroll
-            for (int t = 0; t < CT; t += 2) {
-                const float ga = G * (VECTOR ? sw[t * P + d] : sa[t]);
-                G = ga * (VECTOR ? sw[(t + 1) * P + d] : sa[t + 1]);
-                x[t / 2] = make_pair_of(sk[t * P + d] * ga, sk[(t + 1) * P + d] * G);
+            for (int i = 0; i < COLS; ++i) {
+                const int k = i < cols ? d + i * apart : d;
+                float G = 1.f;
+#pragma unroll
+                for (int t = 0; t < CT; t += 2) {
+                    const float ga = G * (VECTOR ? sw[t * P + k] : sa[t]);
+                    G = ga * (VECTOR ? sw[(t + 1) * P + k] : sa[t + 1]);
+                    x[i][t / 2] = make_pair_of(sk[t * P + k] * ga, sk[(t + 1) * P + k] * G);
+                }
             }
         }
         if (DELTA) {
-            Substitute f{x, sN, sb};
+            Substitute<COLS> f{x, sN, sb};
             each_token<0>(f);
         }
-        if (d < 0) {
-            ValueColumn<RULE> f{x, sA, a.out + first * E + c, DELTA ? a.wu + first * E + c : nullptr,
-                                RULE == RULE_SSD ? a.per_head[head] : 0.f, (size_t)H * E, cnt};
+        if (is_v) {
+            ValueColumn<RULE, COLS> f{x, sA, a.out + first * E + d, DELTA ? a.wu + first * E + d : nullptr,
+                                      RULE == RULE_SSD ? a.per_head[head] : 0.f, (size_t)H * E, cnt, apart, cols};
             each_token<0>(f);
         } else {
-            KeyColumn<RULE, P> f{x, sA, sq + d, VECTOR ? sw + d : sa, a.wq + first * D + d,
-                                 DELTA ? a.ww + first * D + d : nullptr, 1.f, (size_t)H * D, cnt};
+            KeyColumn<RULE, P, COLS> f{x, sA, sq + d, VECTOR ? sw + d : sa, a.wq + first * D + d,
+                                       DELTA ? a.ww + first * D + d : nullptr, {}, (size_t)H * D, cnt, apart, cols};
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) f.G[i] = 1.f;
             each_token<0>(f);
         }
     }
@@ -486,83 +534,101 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
     const int slot = a.req_state_slot[r];
     const float* n0 = RULE == RULE_MLSTM ? a.kept + (size_t)r * (H * D + H) : nullptr;
     float m = RULE == RULE_MLSTM ? n0[(size_t)H * D + head] : 0.f;
-    // a chunk's numbers: the decay of the state before it, the factor of what it adds
-    auto numbers = [&](int c, int d, float& g, float& in) {
-        in = 1.f;
-        if (RULE == RULE_WKV) {
-            g = a.wg[(chunk_place(row0 + c * CT, r) * H + head) * D + d];
-        } else {
-            const float4 last = a.ws[(size_t)(row0 + min(n, (c + 1) * CT) - 1) * H + head];
-            if (RULE == RULE_MLSTM) {
-                const float m_new = fmaxf(last.x + m, last.z);
-                g = expf(last.x + m - m_new);
-                in = expf(last.z - m_new);
-                m = m_new;
-            } else {
-                g = last.x;
+    // the chunks' numbers, 64 at a time: the decay of the state before a chunk (wkv: a vector, read
+    // below), the factor of what it adds, m as it begins
+    constexpr int BATCH = 64, AHEAD = 8;
+    __shared__ float4 sx[BATCH];
+    __shared__ float sg[BATCH], si[BATCH], sm[BATCH];
+    auto numbers = [&](int c0) {
+        if (RULE == RULE_WKV) return;
+        __syncthreads();
+        if (threadIdx.x < BATCH && c0 + (int)threadIdx.x < chunks)
+            sx[threadIdx.x] = a.ws[(size_t)(row0 + min(n, (c0 + (int)threadIdx.x + 1) * CT) - 1) * H + head];
+        __syncthreads();
+        if (RULE == RULE_SSD) {
+            if (threadIdx.x < BATCH) sg[threadIdx.x] = sx[threadIdx.x].x, si[threadIdx.x] = 1.f;
+        } else if (threadIdx.x == 0) {
+            for (int k = 0; k < min(BATCH, chunks - c0); ++k) {
+                sm[k] = m;
+                m = fmaxf(sx[k].x + m, sx[k].z);
             }
         }
+        __syncthreads();
+        if (RULE == RULE_MLSTM && threadIdx.x < BATCH && c0 + (int)threadIdx.x < chunks) {
+            const float4 own = sx[threadIdx.x];
+            const float before = sm[threadIdx.x], after = fmaxf(own.x + before, own.z);
+            sg[threadIdx.x] = expf(own.x + before - after);
+            si[threadIdx.x] = expf(own.z - after);
+        }
+        __syncthreads();
     };
     const size_t step = (size_t)H * D * E;          // neighbouring chunks of a request are neighbours in wl
-    const int i = (blockIdx.x * THREADS + threadIdx.x) * 4;
-    if (i < D * E) {
-        float* S = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E + i;
-        float* at = a.wl + (chunk_place(row0, r) * H + head) * (size_t)D * E + i;
-        const int d = i / E;
-        float4 s = *reinterpret_cast<const float4*>(S);
-        constexpr int AHEAD = 4;
-        for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+    const int i = (blockIdx.x * THREADS + threadIdx.x) * 4, d = i / E;
+    const bool mine = i < D * E;
+    const bool with_n = RULE == RULE_MLSTM && blockIdx.x == gridDim.x - 1;
+    const int dn = threadIdx.x;
+    float* S = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E + i;
+    const size_t first = chunk_place(row0, r) * H + head;
+    float* at = a.wl + first * (size_t)D * E + i;
+    float4 s = mine ? *reinterpret_cast<const float4*>(S) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float v = with_n && dn < D ? n0[(size_t)head * D + dn] : 0.f;
+    for (int b0 = 0; b0 < chunks; b0 += BATCH) {
+        numbers(b0);
+        const int b1 = min(chunks, b0 + BATCH);
+        for (int c0 = b0; c0 < b1; c0 += AHEAD) {
             float4 x[AHEAD];
+            float gw[AHEAD], xn[AHEAD];
 #pragma unroll
             for (int k = 0; k < AHEAD; ++k)
-                if (c0 + k < chunks) x[k] = *reinterpret_cast<const float4*>(at + (c0 + k) * step);
+                if (c0 + k < b1) {
+                    if (mine) x[k] = *reinterpret_cast<const float4*>(at + (c0 + k) * step);
+                    if (RULE == RULE_WKV && mine) gw[k] = a.wg[(first + (size_t)(c0 + k) * H) * D + d];
+                    if (with_n && dn < D) xn[k] = a.wn[(first + (size_t)(c0 + k) * H) * D + dn];
+                }
 #pragma unroll
             for (int k = 0; k < AHEAD; ++k) {
-                if (c0 + k >= chunks) break;
-                float g, in;
-                numbers(c0 + k, d, g, in);
-                *reinterpret_cast<float4*>(at + (c0 + k) * step) = s;
-                s = make_float4(fmaf(g, s.x, in * x[k].x), fmaf(g, s.y, in * x[k].y), fmaf(g, s.z, in * x[k].z),
-                                fmaf(g, s.w, in * x[k].w));
+                if (c0 + k >= b1) break;
+                const float g = RULE == RULE_WKV ? gw[k] : sg[c0 + k - b0], in = RULE == RULE_MLSTM ? si[c0 + k - b0] : 1.f;
+                if (mine) {
+                    *reinterpret_cast<float4*>(at + (c0 + k) * step) = s;
+                    s = make_float4(fmaf(g, s.x, in * x[k].x), fmaf(g, s.y, in * x[k].y), fmaf(g, s.z, in * x[k].z),
+                                    fmaf(g, s.w, in * x[k].w));
+                }
+                if (with_n) {
+                    const size_t place = first + (size_t)(c0 + k) * H;
+                    if (dn == 0) a.wm[place] = sm[c0 + k - b0];
+                    if (dn < D) {
+                        a.wn[place * D + dn] = v;
+                        v = fmaf(g, v, in * xn[k]);
+                    }
+                }
             }
         }
-        *reinterpret_cast<float4*>(S) = s;
     }
-    if (RULE == RULE_MLSTM && blockIdx.x == gridDim.x - 1) {
-        m = n0[(size_t)H * D + head];
-        const int d = threadIdx.x;
-        float v = d < D ? n0[(size_t)head * D + d] : 0.f;
-        for (int c = 0; c < chunks; ++c) {
-            const size_t place = chunk_place(row0 + c * CT, r) * H + head;
-            if (d == 0) a.wm[place] = m;
-            float g, in;
-            numbers(c, 0, g, in);
-            if (d < D) {
-                const float x = a.wn[place * D + d];
-                a.wn[place * D + d] = v;
-                v = fmaf(g, v, in * x);
-            }
-        }
-        if (d < D) state_at(a.state, a.slot_stride, slot, a.n_off)[(size_t)head * D + d] = v;
-        if (d == 0) state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m;
+    if (mine) *reinterpret_cast<float4*>(S) = s;
+    if (with_n) {
+        if (dn < D) state_at(a.state, a.slot_stride, slot, a.n_off)[(size_t)head * D + dn] = v;
+        if (dn == 0) state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m;
     }
 }
 
-// A chunk's queries over the state at its beginning: a warp has 16 tokens and 128 columns, four
-// neighbouring columns a lane; sums of two neighbouring tokens are one instruction.  Per channel a lane
-// reads 16 bytes of S and 64 of queries for 64 multiply-adds.
-constexpr int OUT_THREADS = 64;
+// A chunk's queries over the state at its beginning: a warp has 16 tokens, 128 columns, four
+// neighbouring ones a lane, and half of the channels; sums of two neighbouring tokens are one
+// instruction.  Per channel a lane reads 16 bytes of S, eight channels at once, and 64 of queries for 64
+// multiply-adds.
+constexpr int OUT_THREADS = 128;
 template <int DP, int RULE>
-__global__ void __launch_bounds__(OUT_THREADS) chunk_out_kernel(const Args a) {
+__global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     __shared__ __align__(16) float sq[DP * AP];      // [D][CT]: queries, a channel's tokens side by side
+    __shared__ __align__(16) float half[2][16][128 + 4];
     const int r = blockIdx.z, head = blockIdx.y;
     const int row0 = a.req_row_start[r] + blockIdx.x * CT;
     const int cnt = min(CT, a.req_row_start[r + 1] - row0);
     if (cnt <= 0) return;
     const int D = a.D, E = a.E, H = a.H, g = head / (H / a.G);
-    const int lane = threadIdx.x & 31, t0 = (threadIdx.x >> 5) * 16;
+    const int lane = threadIdx.x & 31, group = (threadIdx.x >> 5) & 1, upper = threadIdx.x >> 6, t0 = group * 16;
     for (int i = threadIdx.x; i < CT * (D / 4); i += OUT_THREADS) {
         const int t = i % CT, d = (i / CT) * 4;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -572,7 +638,6 @@ __global__ void __launch_bounds__(OUT_THREADS) chunk_out_kernel(const Args a) {
         sq[d * AP + t] = q.x; sq[(d + 1) * AP + t] = q.y; sq[(d + 2) * AP + t] = q.z; sq[(d + 3) * AP + t] = q.w;
     }
     __syncthreads();
-    if (t0 >= cnt) return;
     const size_t place = chunk_place(row0, r) * H + head;
     // the factors of a token's two shares (what it has within the chunk, what comes from the state), in
     // the lane of the token
@@ -602,20 +667,45 @@ __global__ void __launch_bounds__(OUT_THREADS) chunk_out_kernel(const Args a) {
         pair_t acc[8][4];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0;
-#pragma unroll 4
-        for (int d = 0; d < D; ++d) {
-            const float4 s = in ? *reinterpret_cast<const float4*>(S + (size_t)d * E) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const pair_t c[4] = {make_pair_of(s.x, s.x), make_pair_of(s.y, s.y), make_pair_of(s.z, s.z), make_pair_of(s.w, s.w)};
+        const int d0 = upper ? D / 8 * 4 : 0, d1 = upper ? D : D / 8 * 4;       // (D: a multiple of 4)
+        constexpr int AHEAD = 8;
+        for (int db = d0; db < d1; db += AHEAD) {
+            float4 s[AHEAD];
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                const ulonglong2 q = pairs_at(sq + d * AP + t0 + 2 * i);
+            for (int k = 0; k < AHEAD; ++k)
+                s[k] = in && db + k < d1 ? *reinterpret_cast<const float4*>(S + (size_t)(db + k) * E) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    acc[i][k] = fma_pair(q.x, c[k], acc[i][k]);
-                    acc[i + 1][k] = fma_pair(q.y, c[k], acc[i + 1][k]);
+            for (int j = 0; j < AHEAD; ++j) {
+                if (db + j >= d1) break;
+                const pair_t c[4] = {make_pair_of(s[j].x, s[j].x), make_pair_of(s[j].y, s[j].y), make_pair_of(s[j].z, s[j].z),
+                                     make_pair_of(s[j].w, s[j].w)};
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const ulonglong2 q = pairs_at(sq + (db + j) * AP + t0 + 2 * i);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        acc[i][k] = fma_pair(q.x, c[k], acc[i][k]);
+                        acc[i + 1][k] = fma_pair(q.y, c[k], acc[i + 1][k]);
+                    }
                 }
             }
         }
+        // the upper half's sums to the lower half's warps
+        __syncthreads();
+        if (upper) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                float x[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 v = split_pair(acc[i / 2][k]);
+                    x[k] = i % 2 ? v.y : v.x;
+                }
+                *reinterpret_cast<float4*>(&half[group][i][lane * 4]) = make_float4(x[0], x[1], x[2], x[3]);
+            }
+        }
+        __syncthreads();
+        if (upper) continue;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const float fw = __shfl_sync(0xffffffffu, within, i), fb = __shfl_sync(0xffffffffu, before, i);
@@ -625,6 +715,8 @@ __global__ void __launch_bounds__(OUT_THREADS) chunk_out_kernel(const Args a) {
                 const float2 v = split_pair(acc[i / 2][k]);
                 x[k] = i % 2 ? v.y : v.x;
             }
+            const float4 other = *reinterpret_cast<const float4*>(&half[group][i][lane * 4]);
+            x[0] += other.x; x[1] += other.y; x[2] += other.z; x[3] += other.w;
             if (in && t0 + i < cnt) {
                 float* to = a.out + ((size_t)(row0 + t0 + i) * H + head) * E + e;
                 const float4 l = *reinterpret_cast<const float4*>(to);
@@ -654,12 +746,12 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     extern __shared__ __align__(16) float smem[];
     float* S = smem;                                     // [ET][P]
     float* red = S + ET * P;                             // [SPLIT][ROWS][ET]
-    float* su = red + SPLIT * ROWS * ET;                 // [CT][ET][2]: u as it joins the state, every number twice
-    float* sg = su + 2 * CT * ET;                        // [DP]: the chunk's decays per channel
+    float* su = red + SPLIT * ROWS * ET;                 // [CT][ET]: u as it joins the state
+    float* sg = su + CT * ET;                        // [DP]: the chunk's decays per channel
     float4* sc = reinterpret_cast<float4*>(sg + DP);     // [2][CT] the tokens' numbers
     float* stage = reinterpret_cast<float*>(sc + 2 * CT);
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * ET;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
     const int row0 = a.req_row_start[r], row1 = a.req_row_start[r + 1];
@@ -719,9 +811,8 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int share = tid / (RG * CG), rg = (tid % (RG * CG)) / CG, cg = tid % CG;
     // where its sums go, and who adds the shares
     const int orow = tid / CG, ocol = cg * 4;
-    // the second product: a thread's four channels and two columns
-    constexpr int DB = DP / 32, CP = ET / 2 < 4 ? ET / 2 : 4;       // blocks of 8 x 4 channels; column pairs a warp
-    const int ud = ((warp % DB) * 8 + lane / 4) * 4, uc = ((warp / DB) * 4 + (lane & 3)) * 2;
+    // the second product: a thread's four channels and four columns (of ET / 4 x DP / 4 threads)
+    const int ud = (tid / CG) * 4, uc = (tid % CG) * 4;
     if (row0 < row1) fetch(row0, 0);
     int buf = 0;
     for (int base = row0; base < row1; base += CT, buf ^= 1) {
@@ -787,32 +878,37 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 float4 own = *reinterpret_cast<const float4*>(u + t * ET + ocol);
                 own.x -= sum.x; own.y -= sum.y; own.z -= sum.z; own.w -= sum.w;
                 const float f = VECTOR ? 1.f : nums[t].y;
-                float* to = su + 2 * (t * ET + ocol);
-                *reinterpret_cast<float4*>(to) = make_float4(f * own.x, f * own.x, f * own.y, f * own.y);
-                *reinterpret_cast<float4*>(to + 4) = make_float4(f * own.z, f * own.z, f * own.w, f * own.w);
+                *reinterpret_cast<float4*>(su + t * ET + ocol) = make_float4(f * own.x, f * own.y, f * own.z, f * own.w);
             }
         }
         __syncthreads();
         // the state: decayed, and the chunk's k^T u
-        if (uc < ET && (lane & 3) < CP) {
-            pair_t x[2] = {0, 0}, y[2] = {0, 0};
-#pragma unroll 16
+        if (ud < DP) {
+            pair_t x[4][2];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c][0] = x[c][1] = 0;
+#pragma unroll 8
             for (int t = 0; t < CT; ++t) {
                 const ulonglong2 k = pairs_at(keys + t * P + ud);
-                const ulonglong2 v = pairs_at(su + 2 * (t * ET + uc));
-                x[0] = fma_pair(k.x, v.x, x[0]); x[1] = fma_pair(k.y, v.x, x[1]);
-                y[0] = fma_pair(k.x, v.y, y[0]); y[1] = fma_pair(k.y, v.y, y[1]);
+                const float4 v = *reinterpret_cast<const float4*>(su + t * ET + uc);
+                const pair_t f[4] = {make_pair_of(v.x, v.x), make_pair_of(v.y, v.y), make_pair_of(v.z, v.z), make_pair_of(v.w, v.w)};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    x[c][0] = fma_pair(k.x, f[c], x[c][0]);
+                    x[c][1] = fma_pair(k.y, f[c], x[c][1]);
+                }
             }
             const float4 own = *reinterpret_cast<const float4*>(sg + ud);
             const pair_t ga = VECTOR ? make_pair_of(own.x, own.y) : make_pair_of(g_end, g_end);
             const pair_t gb = VECTOR ? make_pair_of(own.z, own.w) : ga;
-            ulonglong2* sx0 = reinterpret_cast<ulonglong2*>(S + place_of(uc) * P + ud);
-            ulonglong2* sx1 = reinterpret_cast<ulonglong2*>(S + place_of(uc + 1) * P + ud);
-            ulonglong2 p = *sx0, q = *sx1;
-            p.x = fma_pair(ga, p.x, x[0]); p.y = fma_pair(gb, p.y, x[1]);
-            q.x = fma_pair(ga, q.x, y[0]); q.y = fma_pair(gb, q.y, y[1]);
-            *sx0 = p;
-            *sx1 = q;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                ulonglong2* at = reinterpret_cast<ulonglong2*>(S + place_of(uc + c) * P + ud);
+                ulonglong2 p = *at;
+                p.x = fma_pair(ga, p.x, x[c][0]);
+                p.y = fma_pair(gb, p.y, x[c][1]);
+                *at = p;
+            }
         }
         __syncthreads();
     }
@@ -830,7 +926,7 @@ int allow_smem(K kernel, size_t smem) {
 template <int DP, int RULE, int ET>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
     constexpr int ROWS = 2 * CT, SPLIT = THREADS / ((ROWS / 4) * (ET / 4)), P = DP + 4;
-    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + 2 * CT * ET + DP + 8 * CT
+    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + CT * ET + DP + 8 * CT
                                               + 2 * ((ROWS + CT) * P + CT * ET));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
     const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes);

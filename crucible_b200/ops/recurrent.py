@@ -13,8 +13,22 @@ _c_long = ctypes.c_long
 DELTA, MLSTM, WKV, SSD, CHANNEL = 0, 1, 2, 3, 4
 GATE_SILU, GATE_SIGMOID = 0, 1
 CHUNKS = True                # tests switch it off to reach the token-by-token walk with the same inputs
-CHUNK_MIN_TOKENS = 128       # the longest portion from which a bfloat16 step's portions go in chunks
 STEP = True                  # likewise, for the form of a token each
+
+
+def chunks_pay(rule, rows: int, requests: int, longest: int, heads: int) -> bool:
+    """Whether a bfloat16 step's portions (`rows` tokens of `requests`, without the single tokens at the
+    step's head; the longest) go in chunks.  The walk takes 0.2 to 0.28 us a token of the longest portion, or of
+    the whole where the requests fill the GPU; chunks take 18 us (delta rules) or 35 (the others) and then far
+    less a token, but a chunk that holds few tokens costs what a full one does.  Measured on 16 heads of
+    128: delta rules 64 tokens 22 us in chunks and 19 walked, 96: 24 and 26; 16 requests of up to 128: 221 and
+    182, 5: 76 and 81.  The others: 128 tokens 35 to 39 and 29 to 40, 512: 48 and 105 to 150; 16 requests of up
+    to 64: 88 to 105 and 93 to 136, of up to 30: 52 to 65 and 42 to 56."""
+    if requests <= 0:
+        return False
+    if rule in (DELTA, CHANNEL):
+        return rows >= 96 * requests
+    return longest >= 160 or (longest >= 48 and rows >= 24 * requests and rows * heads >= 4096)
 
 
 def _state_args(state: torch.Tensor):
@@ -164,7 +178,8 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     n, walked = ctx.n_requests, ctx.n_requests
     starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
     w_off_read = w_off if rule in (WKV, CHANNEL) else 0
-    if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.max_new_tokens >= CHUNK_MIN_TOKENS
+    if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and chunks_pay(
+                rule, qkv.shape[0] - ctx.host.lead_single, n - ctx.host.lead_single, ctx.host.max_new_tokens, n_heads)
             and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0
             and (s_off | state.stride(0)) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked

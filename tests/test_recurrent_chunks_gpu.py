@@ -94,8 +94,9 @@ def _walk(rule, k, q, kk, v, w, sc0, sc1, per_head, S, n, m):
 
 @pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
 @pytest.mark.parametrize("H,G,D,E", [(4, 2, 128, 128), (2, 1, 64, 64), (3, 3, 20, 20), (2, 2, 100, 100)])
-def test_chunks_agree_with_float64(rule, H, G, D, E):
+def test_chunks_agree_with_float64(rule, H, G, D, E, monkeypatch):
     from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
     rule_code = getattr(k, rule)
     if rule in ("MLSTM", "WKV"):
         G = H
@@ -143,9 +144,10 @@ def test_chunks_agree_with_float64(rule, H, G, D, E):
 
 
 @pytest.mark.parametrize("rule", ["DELTA", "CHANNEL", "SSD", "WKV", "MLSTM"])
-def test_a_later_token_does_not_reach_an_earlier_one(rule):
+def test_a_later_token_does_not_reach_an_earlier_one(rule, monkeypatch):
     """A value that is not a number stays with its own and later tokens of its own request."""
     from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda *a: True)
     code, H, D, lengths, at = getattr(k, rule), 2, 64, (140, 130), 45
     g = torch.Generator().manual_seed(2)
     T = sum(lengths)

@@ -87,7 +87,7 @@ struct NormArgs {
     // matrices one below the other (w_rows rows each), and block row y takes tile y of the plan
     // that a kernel before this one left on the device: [0] tiles in use, [2 + E + y] the tile's
     // expert, [2 + E + max_tiles + y] its first row, [2 + E + 2 max_tiles + y] its rows (at most
-    // 128).  Tiles beyond those in use compute on rows they do not own and store nothing.
+    // 128).  Tiles beyond those in use do nothing.
     const int* plan;
     int n_experts, max_tiles, w_rows;
     // A product per head in one launch (heads > 0; not with a plan): block z takes head z, whose
@@ -97,6 +97,9 @@ struct NormArgs {
     int heads, head_a_cols, head_c_cols;
     // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2
     int act;
+    // a grouped product's A and its rows' stride (set by its entry point)
+    const void* a_rows;
+    int a_ld;
 };
 
 template <int BN, int STAGES, int MH>
@@ -149,7 +152,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     const int k_blocks_all = (K + BK - 1) / BK;
     const int per_split = (k_blocks_all + k_splits - 1) / k_splits;
     const int kb_first = (int)split * per_split;
-    const int k_blocks = min(per_split, k_blocks_all - kb_first);      // the launcher keeps it positive
+    int k_blocks = min(per_split, k_blocks_all - kb_first);            // the launcher keeps it positive
     volatile int* abort_flag = &s.abort_flag;
     // tensor-memory columns are allocated in powers of two
     constexpr uint32_t TMEM_COLS = MH * BN <= 32 ? 32 : (MH * BN <= 64 ? 64 : (MH * BN <= 128 ? 128 : (MH * BN <= 256 ? 256 : 512)));
@@ -177,6 +180,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem_acc = s.tmem_base;
+    bool few_rows = false;              // grouped: the tile's rows of A are one box of 16
     constexpr bool PRE = NORM == NORM_PRE;
     auto load_w = [&](int kb, int st) {
         if (EPI == SWIGLU_BF16) {
@@ -208,7 +212,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         m0 = in_use ? __ldg(entry + na.max_tiles) : 0;
         M = in_use ? m0 + __ldg(entry + 2 * na.max_tiles) : 0;
         w_row0 = in_use ? __ldg(entry) * na.w_rows : 0;
+        if (!in_use) k_blocks = 0;                // nothing to load, multiply or store
+        // an expert of few rows (decoded tokens): a box of 16 rows instead of the whole tile of A, which
+        // would be as many bytes as W's; what the tile holds beyond them are rows nobody stores (8 rows,
+        // two of 8 experts of 4,096 x 2,048 each: 38 -> 29 us; several small boxes for more rows were slower)
+        few_rows = M - m0 <= 16;
     }
+    const uint32_t stage_bytes = few_rows ? (uint32_t)(BN + 16) * BK * 2 : STAGE_BYTES;
 
     // A norm after the product: the tile of C (32-column boxes in the 128-byte swizzle) comes
     // into its own piece of shared memory behind the stages, asked for by an epilogue thread
@@ -243,9 +253,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     break;
                 }
                 if (kb >= w_ahead) {
-                    tc::mbar_expect_tx(&s.full_bar[st], STAGE_BYTES);
+                    tc::mbar_expect_tx(&s.full_bar[st], stage_bytes);
                     load_w(kb, st);
                 }
+                if (MH == 1 && few_rows)
+                    tc::tma_load_2d(s.a[st], &map_s, &s.full_bar[st], (kb_first + kb) * BK, m0);
+                else
 #pragma unroll
                 for (int mh = 0; mh < MH; ++mh)
                     tc::tma_load_2d(s.a[st] + mh * (BM * BK * 2), &map_a, &s.full_bar[st],
@@ -906,6 +919,7 @@ int launch_norm(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
         tma_out = 0;
     if ((EPI == ROPE_APPEND || MH > 1 || emit) && !tma_out) return CB_ERR_UNSUPPORTED;
     CUtensorMap ms = ma;
+    if (grouped && !tc::make_map_2d(&ms, na.a_rows, (uint64_t)M, (uint64_t)K, (uint64_t)na.a_ld, 16)) return CB_ERR_UNSUPPORTED;
     if (emit && !tc::make_plain_box_map_2d(&ms, na.scaled, (uint64_t)M, (uint64_t)N, (uint64_t)na.ld_scaled, 32, BM))
         return CB_ERR_UNSUPPORTED;
     const int smem = (int)(emit ? smem_emit : smem_plain);
@@ -1013,11 +1027,13 @@ CB_EXPORT int cb_gemm_tcgen05(const void* A, const void* W, void* C, int M, int 
 // epi: STORE_BF16, STORE_F32 or SWIGLU_BF16 (N = the intermediate width, w_rows = 2 N).
 // bn: 64, 96 or 128.  Nothing of the plan is read on the host: a step replays as a graph.
 CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int M, int N, int K, int lda,
-                                      int ldw, int ldc, int epi, int bn, int* status, void* stream,
+                                      int ldw, int ldc, int epi, int bn, int per_sm, int* status, void* stream,
                                       const void* norm) {
     if (M <= 0 || N <= 0) return 0;
     if (norm == nullptr) return CB_ERR_UNSUPPORTED;
-    const NormArgs na = *static_cast<const NormArgs*>(norm);
+    NormArgs na = *static_cast<const NormArgs*>(norm);
+    na.a_rows = A;
+    na.a_ld = lda;
     if (na.plan == nullptr || na.n_experts <= 0 || na.gain != nullptr || na.sumsq_in != nullptr ||
         K <= 0 || (K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15))
         return CB_ERR_UNSUPPORTED;
@@ -1029,10 +1045,20 @@ CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int
         return CB_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     const int inter = epi == SWIGLU_BF16 ? N : 0;
+    if (per_sm == 2) {
+        switch (bn) {
+            case 64: return launch_epi<64, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+            case 96: return launch_epi<96, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+            case 128: return launch_epi<128, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+        }
+        return CB_ERR_UNSUPPORTED;
+    }
     switch (bn) {
         case 64: return launch_epi<64, 6>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
         case 96: return launch_epi<96, 6>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
         case 128: return launch_epi<128, 5>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+        case 192: return launch_epi<192, 5>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+        case 256: return launch_epi<256, 4>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
     }
     return CB_ERR_UNSUPPORTED;
 }

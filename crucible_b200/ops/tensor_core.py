@@ -178,7 +178,8 @@ class _NormArgs(ctypes.Structure):
                 ("glu_limit", ctypes.c_float), ("glu_alpha", ctypes.c_float), ("glu_offset", ctypes.c_float),
                 ("plan", ctypes.c_void_p), ("n_experts", ctypes.c_int), ("max_tiles", ctypes.c_int),
                 ("w_rows", ctypes.c_int), ("heads", ctypes.c_int), ("head_a_cols", ctypes.c_int),
-                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int)]
+                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int), ("a_rows", ctypes.c_void_p),
+                ("a_ld", ctypes.c_int)]
 
 
 class NormEmit:
@@ -349,7 +350,20 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
     return _gemm(a, w, out, w.shape[0], epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
 
 
-def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pair=None) -> bool:
+def grouped_tile(pairs: int, n_experts: int, gated: bool):
+    """(tile width, blocks to an SM) of a grouped product.  Many rows an expert: the widest tile asks for the
+    fewest operand bytes (2,048 tokens, two of 8 experts of 2,816 x 2,048: gate/up 125 us with 128 columns,
+    101 with 256; down 66 and 54).  Fewer: the weights' bytes decide, and how the blocks fill the SMs (64
+    pairs: gate/up 41 us with 128 columns, 35 with 192, 41 with 256; down 15, 18, 20; 16 pairs: gate/up 29
+    with 128, 25 with 128 and two blocks to an SM, 33 with 192)."""
+    if pairs >= 64 * n_experts:
+        return 256, 1
+    if not gated:
+        return 128, 1
+    return (192, 1) if pairs >= 4 * n_experts else (128, 2)
+
+
+def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pair=None, tile=None) -> bool:
     """The grouped product of a mixture of experts (`cb_gemm_tcgen05_grouped`): `a` [pairs, K]
     bfloat16 rows expert by expert, `w` [experts, rows, K] a declared weight, `plan` the int32
     plan on the device with `tiles` tile entries of 128 rows.  gated: out [pairs, rows / 2]
@@ -364,12 +378,13 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     args = _NormArgs()
     if pair is not None:
         args.glu_limit, args.glu_alpha, args.glu_offset = (float(v) for v in pair)
+    bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, gated)
     args.plan, args.n_experts, args.max_tiles, args.w_rows = plan.data_ptr(), n_experts, tiles, w.shape[1]
     lib = build.load("gemm_tcgen05")
     code = lib.cb_gemm_tcgen05_grouped(
         _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
         _c_int(a.shape[0]), _c_int(n), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(1)),
-        _c_int(out.stride(0)), _c_int(epi), _c_int(128), _c_void_p(status_word(a.device).data_ptr()),
+        _c_int(out.stride(0)), _c_int(epi), _c_int(bn), _c_int(per_sm), _c_void_p(status_word(a.device).data_ptr()),
         _stream(), ctypes.cast(ctypes.pointer(args), _c_void_p))
     if code == _UNSUPPORTED:
         return False

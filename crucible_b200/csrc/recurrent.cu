@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     if (RULE == RULE_MLSTM) m = kept_n[(size_t)n_heads * D + head];
     __syncthreads();
     // 16-byte copies if every row of q and k starts on a 16-byte boundary
-    const bool vec = ((C | q_off | k_off | D | (VECTOR ? w_off : 0)) & 3) == 0;
+    const bool vec = ((C | q_off | k_off | D | (VECTOR ? w_off : 0)) & 3) == 0 && ((uintptr_t)qkv & 15) == 0;
     // a chunk's q, k, v and gates on their way into one of the two stages (asynchronous
     // copies: the next chunk travels while this one is worked on)
     auto fetch = [&](int base, int buf) {

@@ -490,13 +490,16 @@ def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, ke
             or any(t.data_ptr() % 16 for t in tensors) or (gate is not None and gate.dtype != torch.float32)):
         return False
     lib = build.load("attention_f32")
-    _check(lib.cb_attention_f32(
+    code = lib.cb_attention_f32(
         _ptr(q), _c_int(q.stride(0)), _ptr(gate), _c_int(gate.stride(0) if gate is not None else 0), _ptr(out),
         _c_int(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(sinks), _ptr(ctx.req_row_start),
         _ptr(ctx.req_first_pos), _ptr(table), _c_int(table.shape[1]), _c_int(ctx.n_requests),
         _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim), _c_int(value_dim),
         _c_int(page_tokens), _c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first),
-        _c_float(out_scale), _c_int(1 if gate_per_head else 0), _stream()), "attention (32-bit tiles)")
+        _c_float(out_scale), _c_int(1 if gate_per_head else 0), _stream())
+    if code == build.UNSUPPORTED:
+        return False
+    _check(code, "attention (32-bit tiles)")
     return True
 
 

@@ -27,6 +27,8 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(_HERE), "csrc")
 _LIB_DIR = os.path.join(os.path.dirname(_HERE), "lib")
 
+UNSUPPORTED = 100001       # `csrc/common.cuh`: an entry does not take this call
+
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

@@ -74,7 +74,7 @@ def _conv_prepare(proj, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, state,
         _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(dst), _ptr(num0), _ptr(num1),
         _c_int(ctx.n_requests), _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(channels), _c_int(unit_heads),
         _c_int(head_size), _c_int(1 if is_ssd else 0), _c_int(1 if update else 0), _stream())
-    if code == 100001:
+    if code == build.UNSUPPORTED:
         return False
     _check(code, "conv_prepare")
     return True
@@ -197,28 +197,32 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         wn = ctx.scratch("memory.wn", (places, n_heads, key_dim), f32) if rule == MLSTM else None
         wm = ctx.scratch("memory.wm", (places, n_heads), f32) if rule == MLSTM else None
         lib = build.load("recurrent_chunks")
-        _check(lib.cb_matrix_memory_chunks(
+        code = lib.cb_matrix_memory_chunks(
             _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
             _ptr(sc0), _ptr(sc1), _c_void_p(starts + 4 * walked), _c_void_p(slots + 4 * walked), sp, stride,
             _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(n - walked),
             _c_int(ctx.host.max_new_tokens), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
             _c_int(w_off), _ptr(per_head),
             _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
-            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream()),
-            "matrix_memory (chunks)")
-        LAUNCHES[0] += 1 if delta else 2         # (two kernels, or three)
+            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream())
+        if code == build.UNSUPPORTED:            # (rows on boundaries that its loads do not take): the walk's
+            walked = n
+        else:
+            _check(code, "matrix_memory (chunks)")
+            LAUNCHES[0] += 1 if delta else 2     # (two kernels, or three)
     if walked == 0:
         return
     lib = build.load("recurrent")
     # decoded tokens of the bfloat16 engine: a token each, S read and written once
     step = (STEP and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.lead_single >= walked
             and (qkv.shape[1] | v_off | value_dim) % 4 == 0 and (s_off | state.stride(0)) % 16 == 0)
-    _check((lib.cb_matrix_memory_step if step else lib.cb_matrix_memory)(
-        _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
-        _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,
-        _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(walked),
-        _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim), _c_int(w_off),
-        _ptr(per_head), _c_void_p(kept_at), _stream()), "matrix_memory")
+    args = (_c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
+            _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,
+            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(walked),
+            _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim), _c_int(w_off),
+            _ptr(per_head), _c_void_p(kept_at), _stream())
+    code = lib.cb_matrix_memory_step(*args) if step else build.UNSUPPORTED
+    _check(lib.cb_matrix_memory(*args) if code == build.UNSUPPORTED else code, "matrix_memory")
 
 
 def head_norm_gate(o, gain, gain_per_head, gate, out, gate_kind, n_heads, value_dim, eps,

@@ -166,3 +166,27 @@ def test_a_later_token_does_not_reach_an_earlier_one(rule, monkeypatch):
         outs.append(out.cpu())
     assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][lengths[0]:], outs[1][lengths[0]:])
     assert bool(torch.isnan(outs[1][at]).any())
+
+
+@pytest.mark.parametrize("lengths", [(70, 33), (1, 1, 1), (1, 70)])
+def test_rows_off_the_wide_loads_boundaries_are_walked(lengths, monkeypatch):
+    """Outputs that start on no 16-byte boundary: the chunks refuse them, and the walk's bits are the answer."""
+    from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
+    H, D, g, T, R = 2, 64, torch.Generator().manual_seed(3), sum(lengths), len(lengths)
+    q, kk, v, w, sc0, sc1, per_head = _operands(k.DELTA, k, T, H, H, D, D, g)
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, kk, v)], 1).contiguous().to(DEV)
+    qkv_off = torch.empty(qkv.numel() + 1, device=DEV)[1:].view(qkv.shape).copy_(qkv)
+    outs = []
+    for chunks, rows in ((True, qkv_off), (False, qkv)):
+        ctx, _, _ = _ctx(lengths, torch.bfloat16)
+        state = torch.zeros(R, 4 * H * D * D, dtype=torch.uint8, device=DEV)
+        out = torch.full((T * H * D + 1,), float("nan"), device=DEV)[1:].view(T, H * D)
+        k.CHUNKS = k.STEP = chunks
+        try:
+            k.matrix_memory(k.DELTA, rows, 0, H * D, 2 * H * D, sc0.contiguous().to(DEV), sc1.contiguous().to(DEV),
+                            ctx, state, 0, 0, 0, out, H, H, D, D)
+        finally:
+            k.CHUNKS = k.STEP = True
+        outs.append((out.cpu(), state.cpu()))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])

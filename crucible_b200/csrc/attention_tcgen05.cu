@@ -1,5 +1,5 @@
 // Paged causal attention for portions of prompts on the 5th-generation tensor
-// cores (head size 64 or 128, bfloat16): S = Q K^T and O += P V are tcgen05.mma with
+// cores (head size 64, 128 or, keys and values at once, 256; bfloat16): S = Q K^T and O += P V are tcgen05.mma with
 // the scores and the output accumulator in tensor memory; K and V pages come in
 // by TMA; the softmax runs on four warps, one thread per query row, reading S
 // from tensor memory and writing P (bf16) to shared memory for the second MMA.
@@ -16,12 +16,17 @@
 // their sums and P's way to shared memory, in which the special-function unit's 560 and
 // the other pipes' instructions add up instead of overlapping; the rest maxima, barrier
 // tests of 100 to 200 cycles each, and the scores' way out of tensor memory).
-// Head size 64 with an SM to the block: two such groups of four softmax warps take the
+// Head sizes 64 and 128 with an SM to the block: two such groups of four softmax warps take the
 // tiles in turn (tile j: group j % 2), each with its own buffer of scores and of P, its own
 // reference maximum, sum and accumulator, merged when the keys are through; two tiles are
 // then in work at a time (one group's exponentials beside the other's maxima and waits:
 // 1,750 cycles a tile), and a second thread, of a warp of its own, sends the second products,
 // since one thread cannot send both products of two tiles in time (1,200 cycles a tile).
+// Head size 128 has room for two stages only (227 KB with both buffers of P, all of it), so keys
+// and values come and go by barriers of their own: a tile's keys travel as soon as the first
+// product two tiles back has read its own, beside that tile's softmax, and its values once the
+// second has.  A 2,048-token prompt of 16 heads on 4, a window of 1,024 (256 blocks of up to ten
+// tiles): 86 us with one group, 66 with two.
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
 // tile's maximum exceeds it by more than 2^8 (in the base-2 exponent), so P
@@ -41,6 +46,7 @@
 // Reference counterpart: `attention_prefill_exact_*`
 // (engine/kernels/kernels.cu:2257-2275).
 #define CB_PDL_BIT 1      // this file's bit in CRUCIBLE_PDL
+#include <type_traits>
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -96,17 +102,21 @@ __device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits
 // beside this tile's softmax.  It was the right one for launches with more blocks than places
 // while the roomy form had one softmax group (4,096-token prompt of the 120M shape 1.84 against
 // 2.01 ms); with two groups the roomy form is quicker there too (1.68 ms) and the launcher
-// takes it unless told otherwise.  Head size 128, and 256 with one operand for both products: two stages
-// and one P buffer (what 227 KB hold).
+// takes it unless told otherwise.  Head size 128: two stages, two P buffers.  256 with one operand
+// for both products: two stages and one P buffer (what 227 KB hold).
 template <int HD, bool LEAN>
 struct Storage {
     static constexpr int STAGES = (HD == 64 && !LEAN) ? 4 : 2;
-    static constexpr int PB = (HD == 64 && !LEAN) ? 2 : 1;
+    static constexpr int PB = (HD != 256 && !LEAN) ? 2 : 1;
     static constexpr int S_BUFS = LEAN ? 1 : 2;
     static constexpr int OPERANDS = HD == 256 ? 1 : 2;      // keys and values, or rows that are both
     // softmax groups of four warps that take the tiles in turn (tile j: group j % GROUPS), each
     // with its own reference maximum, sum and accumulator, merged at the end
-    static constexpr int GROUPS = (HD == 64 && !LEAN) ? 2 : 1;
+    static constexpr int GROUPS = (HD != 256 && !LEAN) ? 2 : 1;
+    // two groups on two stages: a stage's keys and its values come and go by barriers of their
+    // own, so that a tile's keys are asked for as soon as the first product two tiles back has
+    // read its own, not when the second has
+    static constexpr bool SPLIT = GROUPS > 1 && STAGES == 2;
     // loader, MMA thread, four softmax warps a group; two groups: a warp for a second MMA thread
     static constexpr int THREADS = GROUPS > 1 ? 64 + 128 * GROUPS + 32 : 192;
     alignas(1024) uint8_t q[HD / 64][ROWS * 64 * 2];
@@ -114,6 +124,7 @@ struct Storage {
     alignas(1024) uint8_t p[PB][2][ROWS * 64 * 2];  // P: buffers of two halves of 64 keys
     alignas(8) uint64_t kv_full[STAGES];
     uint64_t kv_empty[STAGES];
+    uint64_t v_full[STAGES], v_empty[STAGES];       // split: the values' (kv_*: the keys')
     uint64_t s_full[2], p_full[2], pv_done[2];
     uint64_t s_free;                                // lean form: a tile's scores are in registers
     uint64_t s_taken[2];                            // two groups: buffer b's scores are in registers
@@ -174,7 +185,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     constexpr int VALUES = Store::OPERANDS - 1;      // where a stage's values are
     constexpr int GROUPS = Store::GROUPS;
     constexpr int PV_WARP = GROUPS > 1 ? 2 + 4 * GROUPS : -1;    // the second MMA thread's warp
-    static_assert(GROUPS == 1 || (PB == 2 && S_BUFS == 2 && HD == 64), "two groups: a buffer of scores, of P and an accumulator each");
+    constexpr bool SPLIT = Store::SPLIT;
+    constexpr uint32_t TILE_BYTES = KEYS * HD * 2;       // a tile of one operand
+    static_assert(GROUPS == 1 || (PB == 2 && S_BUFS == 2 && HD <= 128), "two groups: a buffer of scores, of P and an accumulator each");
     constexpr uint32_t TMEM_COLS = LEAN ? 256 : 512;     // scores: 128 columns a buffer, then O
     Store& s = *reinterpret_cast<Store*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -188,6 +201,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         for (int i = 0; i < STAGES; ++i) {
             tc::mbar_init(&s.kv_full[i], 1);
             tc::mbar_init(&s.kv_empty[i], 1);
+            tc::mbar_init(&s.v_full[i], 1);
+            tc::mbar_init(&s.v_empty[i], 1);
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&s.s_full[b], 1);
@@ -255,7 +270,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             pages[i] = page < 0 ? 0 : page;           // an entry given back early: never read
         }
     };
-    auto issue = [&](int j, const int (&pages)[16]) -> bool {
+    // which of the tile's operands: both, unless keys and values come and go by themselves
+    auto issue = [&](int j, const int (&pages)[16], auto which) -> bool {
+        constexpr bool keys = decltype(which)::value != 2, values = decltype(which)::value != 1;
         const int st = j % STAGES;
         const uint32_t round = j / STAGES;
         // pages that follow one another in the pool come in with one copy per tile and operand
@@ -265,16 +282,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
 #pragma unroll
         for (int i = 1; i < 16; ++i)
             if (i < pages_per_tile && pages[i] != pages[0] + i) run = false;
-        if (round > 0 && !tc::mbar_wait(&s.kv_empty[st], (round - 1) & 1, abort_flag)) {
+        uint64_t* full = keys ? &s.kv_full[st] : &s.v_full[st];
+        uint64_t* empty = keys ? &s.kv_empty[st] : &s.v_empty[st];
+        if (round > 0 && !tc::mbar_wait(empty, (round - 1) & 1, abort_flag)) {
             tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
             return false;
         }
-        tc::mbar_expect_tx(&s.kv_full[st], Store::OPERANDS * KEYS * HD * 2);
+        tc::mbar_expect_tx(full, keys && values ? Store::OPERANDS * TILE_BYTES : TILE_BYTES);
         if (run) {
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
-                tc::tma_load_4d(s.kv[st][0][h], &run_k, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
-                if (VALUES) tc::tma_load_4d(s.kv[st][VALUES][h], &run_v, &s.kv_full[st], h * 64, 0, kv_head, pages[0]);
+                if (keys) tc::tma_load_4d(s.kv[st][0][h], &run_k, full, h * 64, 0, kv_head, pages[0]);
+                if (VALUES && values) tc::tma_load_4d(s.kv[st][VALUES][h], &run_v, full, h * 64, 0, kv_head, pages[0]);
             }
             return true;
         }
@@ -285,13 +304,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 const int y = (pages[i] * p.n_kv_heads + kv_head) << p.page_shift;
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
-                    tc::tma_load_2d(s.kv[st][0][h] + dst, &map_k, &s.kv_full[st], h * 64, y);
-                    if (VALUES) tc::tma_load_2d(s.kv[st][VALUES][h] + dst, &map_v, &s.kv_full[st], h * 64, y);
+                    if (keys) tc::tma_load_2d(s.kv[st][0][h] + dst, &map_k, full, h * 64, y);
+                    if (VALUES && values) tc::tma_load_2d(s.kv[st][VALUES][h] + dst, &map_v, full, h * 64, y);
                 }
             }
         }
         return true;
     };
+    using BOTH = std::integral_constant<int, 3>;
+    using KEYS_ONLY = std::integral_constant<int, 1>;
+    using VALUES_ONLY = std::integral_constant<int, 2>;
     const int early = n_tiles < STAGES ? n_tiles : STAGES;
 
     // ---- the query rows, by warps 1..5: 16-byte pieces into the 128-byte swizzle; warp 0's
@@ -307,7 +329,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             cb_pdl_wait();
 #pragma unroll
             for (int j = 0; j < STAGES; ++j)
-                if (j < early) issue(j, first[j]);
+                if (j < early) {
+                    issue(j, first[j], std::integral_constant<int, SPLIT ? 1 : 3>{});
+                    if (SPLIT) issue(j, first[j], VALUES_ONLY{});
+                }
         } else {
             cb_pdl_wait();
         }
@@ -339,18 +364,42 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     if (warp == 0) {
         // ---- loader: the remaining tiles, each once its stage has been read ------------------
         if (lane == 0 && n_tiles > 0) {
-            int armed = early;
-            for (int j = early; j < n_tiles; ++j) {
-                int pages[16];
-                lookup(j, pages);
-                if (!issue(j, pages)) break;
-                armed = j + 1;
+            int armed = early, values_armed = early;
+            if (SPLIT) {
+                // keys a tile ahead of the values: a tile's keys are free again before its
+                // predecessor's values are, and must not queue behind them
+                int ahead[16], pages[16];
+                if (early < n_tiles) {
+                    lookup(early, pages);
+                    if (issue(early, pages, KEYS_ONLY{})) armed = early + 1;
+                }
+                for (int j = early; j < n_tiles && armed > j; ++j) {
+                    if (j + 1 < n_tiles) {
+                        lookup(j + 1, ahead);
+                        if (!issue(j + 1, ahead, KEYS_ONLY{})) break;
+                        armed = j + 2;
+                    }
+                    if (!issue(j, pages, VALUES_ONLY{})) break;
+                    values_armed = j + 1;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) pages[i] = ahead[i];
+                }
+            } else {
+                for (int j = early; j < n_tiles; ++j) {
+                    int pages[16];
+                    lookup(j, pages);
+                    if (!issue(j, pages, BOTH{})) break;
+                    armed = j + 1;
+                }
             }
             if (*abort_flag) {
-                const int first = armed > STAGES ? armed - STAGES : 0;
-                for (int j = first; j < armed; ++j)
-                    for (uint32_t t = 0; t < tc::WAIT_LIMIT; ++t)
-                        if (tc::mbar_try_wait(&s.kv_full[j % STAGES], (j / STAGES) & 1)) break;
+                auto drain = [&](uint64_t* bars, int count) {
+                    for (int j = count > STAGES ? count - STAGES : 0; j < count; ++j)
+                        for (uint32_t t = 0; t < tc::WAIT_LIMIT; ++t)
+                            if (tc::mbar_try_wait(&bars[j % STAGES], (j / STAGES) & 1)) break;
+                };
+                drain(s.kv_full, armed);
+                if (SPLIT) drain(s.v_full, values_armed);
             }
         }
     } else if (warp == 1 || warp == PV_WARP) {
@@ -394,6 +443,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                     else tc::umma_bf16_add(d_s, q_desc, k_desc, idesc_qk);
                 }
                 tc::umma_commit(&s.s_full[j % S_BUFS]);
+                if (SPLIT) tc::umma_commit(&s.kv_empty[qk_st]);
                 if (++qk_st == STAGES) qk_st = 0, qk_parity ^= 1;
             };
             // `block`: wait for the tile; else only take it if it has landed (true: issued)
@@ -417,8 +467,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 tc::tc_fence_after_sync();
                 const uint32_t p_lo = p_lo0 + pb * P_BUF;
                 const uint32_t v_lo = v_lo0 + st * KV_STAGE;
-                // (two groups: head size 64; a group's accumulator is 64 columns on)
-                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(j % GROUPS) * 64 : 0u);
+                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(j % GROUPS) * HD : 0u);
 #pragma unroll
                 for (int k = 0; k < KEYS / 16; ++k) {
                     // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
@@ -427,7 +476,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                     if (k == 0) tc::umma_bf16(d_o, p_desc, v_desc, idesc_pv, j >= GROUPS ? 1u : 0u);
                     else tc::umma_bf16_add(d_o, p_desc, v_desc, idesc_pv);
                 }
-                tc::umma_commit(&s.kv_empty[st]);
+                tc::umma_commit(SPLIT ? &s.v_empty[st] : &s.kv_empty[st]);
                 tc::umma_commit(&s.pv_done[pb]);
                 if (++st == STAGES) st = 0;
             };
@@ -444,7 +493,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                     }
                 } else {
                     for (int j = 0; j < n_tiles && ok; ++j) {
-                        ok = tc::mbar_wait(&s.p_full[j & 1], (j >> 1) & 1, abort_flag);
+                        ok = tc::mbar_wait(&s.p_full[j & 1], (j >> 1) & 1, abort_flag) &&
+                             (!SPLIT || tc::mbar_wait(&s.v_full[st], (j / STAGES) & 1, abort_flag));
                         if (ok) send_pv(j);
                     }
                 }
@@ -478,7 +528,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         // tensor-memory lane; a group takes every GROUPS-th tile -------------------------------
         const int quarter = warp & 3;
         const int group = GROUPS > 1 ? (warp - 2) >> 2 : 0;
-        const uint32_t tmem_mine = tmem_o + (uint32_t)group * 64;
+        const uint32_t tmem_mine = tmem_o + (uint32_t)group * HD;
         const int r = quarter * 32 + lane;
         const int row = qt * ROWS + r;
         const bool real = active && row < n_rows;
@@ -620,7 +670,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         if (GROUPS > 1) {
             // Two groups: each holds the sums over its own tiles against its own reference.
             // A row's two states meet in shared memory; every thread comes to the barrier,
-            // whatever happened to its waits.  Then group g writes features [32 g, 32 g + 32).
+            // whatever happened to its waits.  Then group g writes its half of the features.
             s.merge[group][r] = make_float2(my_tiles > 0 ? m_ref : -INFINITY, my_tiles > 0 ? l : 0.f);
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (ok && n_tiles > 0 && !*abort_flag) {
@@ -634,31 +684,33 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 if (sink != -INFINITY) l_all += exp2f(sink - m_all);
                 const float inv = l_all > 0.f ? p.out_scale / l_all : 0.f;
                 const float w_mine = f_mine * inv, w_other = f_other * inv;
-                const int c0 = group * 32;
-                uint32_t a[32], b[32];
                 // An accumulator that no MMA has written holds whatever was there and is not
                 // read.  Whether a group had tiles is the same for every thread of the block,
                 // as it must be: the loads are the whole warp's (.sync.aligned).  A row that
                 // could read none of a group's keys has weight 0 and finite sums (zeros) there.
                 const bool mine_any = my_tiles > 0, other_any = n_tiles > my_tiles;
-                if (mine_any) tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, a);
-                if (other_any) tc::tmem_ld_32x32(tmem_o + (uint32_t)(group ^ 1) * 64 + lane_bits + c0, b);
-                tc::tmem_ld_wait();
-                if (real) {
-                    float o[32];
+#pragma unroll 1
+                for (int c0 = group * (HD / 2); c0 < (group + 1) * (HD / 2); c0 += 32) {
+                    uint32_t a[32], b[32];
+                    if (mine_any) tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, a);
+                    if (other_any) tc::tmem_ld_32x32(tmem_o + (uint32_t)(group ^ 1) * HD + lane_bits + c0, b);
+                    tc::tmem_ld_wait();
+                    if (real) {
+                        float o[32];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        o[i] = (mine_any ? __uint_as_float(a[i]) * w_mine : 0.f) +
-                               (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
+                        for (int i = 0; i < 32; ++i)
+                            o[i] = (mine_any ? __uint_as_float(a[i]) * w_mine : 0.f) +
+                                   (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        if (gate != nullptr) gate_eight(o + 8 * q4, gate + c0 + 8 * q4);
-                        uint4 w;
-                        w.x = pack_bf16(o[8 * q4 + 0], o[8 * q4 + 1]);
-                        w.y = pack_bf16(o[8 * q4 + 2], o[8 * q4 + 3]);
-                        w.z = pack_bf16(o[8 * q4 + 4], o[8 * q4 + 5]);
-                        w.w = pack_bf16(o[8 * q4 + 6], o[8 * q4 + 7]);
-                        *reinterpret_cast<uint4*>(dst + c0 + 8 * q4) = w;
+                        for (int q4 = 0; q4 < 4; ++q4) {
+                            if (gate != nullptr) gate_eight(o + 8 * q4, gate + c0 + 8 * q4);
+                            uint4 w;
+                            w.x = pack_bf16(o[8 * q4 + 0], o[8 * q4 + 1]);
+                            w.y = pack_bf16(o[8 * q4 + 2], o[8 * q4 + 3]);
+                            w.z = pack_bf16(o[8 * q4 + 4], o[8 * q4 + 5]);
+                            w.w = pack_bf16(o[8 * q4 + 6], o[8 * q4 + 7]);
+                            *reinterpret_cast<uint4*>(dst + c0 + 8 * q4) = w;
+                        }
                     }
                 }
             }
@@ -704,7 +756,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
 template <int HD, bool LEAN>
 int launch_as(dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
               const CUtensorMap& rk, const CUtensorMap& rv, const TcAttnParams& p) {
-    const int smem = (int)sizeof(Storage<HD, LEAN>);
+    constexpr int smem = (int)sizeof(Storage<HD, LEAN>);
+    static_assert(smem <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, LEAN>,

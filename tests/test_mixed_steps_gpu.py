@@ -63,3 +63,39 @@ def test_decoded_tokens_beside_a_portion(H, G, D, window, keep, chunked, gate, s
     assert seen == [1 if apart else R]                         # the portion alone, or the step
     err = float((outs[0] - outs[1]).abs().max() / outs[1].abs().max())
     assert err < 1.5e-2                                        # both round P and the result to bfloat16 (2^-8)
+
+
+@pytest.mark.parametrize("counts,held,window,keep,ordered", [
+    ([64, 65], [0, 0], None, 0, True),              # one and two tiles of keys: a group without any, a tile each
+    ([300], [85], None, 0, False),                  # three, scattered pages
+    ([130, 500, 3], [126, 600, 1500], None, 0, True),       # four to nine, one copy a tile
+    ([900], [0], 130, 0, False),                    # tiles that a window leaves
+    ([400], [700], 100, 200, True)])                # the kept first tokens' tiles come first
+def test_heads_of_128_two_groups_of_softmax_warps(counts, held, window, keep, ordered):
+    from crucible_b200.engine.context import HostStep
+    from crucible_b200.ops import tensor_core
+    H, G, D, page, R, T = 4, 2, 128, 16, len(counts), sum(counts)
+    g = torch.Generator().manual_seed(T)
+    per = -(-max(c + h for c, h in zip(counts, held)) // page)
+    table = (torch.arange(R * per) if ordered else torch.randperm(R * per, generator=g)).to(torch.int32).view(R, per)
+    k, v = (torch.randn(R * per + 1, G, page, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(T, H * D, generator=g).to(torch.bfloat16)
+    starts = [0]
+    for n in counts:
+        starts.append(starts[-1] + n)
+    host = HostStep(list(range(R)), counts, held, [c + h for c, h in zip(counts, held)], list(range(R)))
+    ctx = SimpleNamespace(n_requests=R, n_tokens=T, req_row_start=_i32(starts), req_first_pos=_i32(held), host=host)
+    whole = tensor_core._Requests(ctx, table.to(DEV), 0, R, max(counts), host.context_bucket, T)
+    out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    assert tensor_core._attention_tcgen05(q.to(DEV), out, k.to(DEV), v.to(DEV), whole, H, G, D, D ** -0.5, window,
+                                          SimpleNamespace(page_tokens=page), keep_first=keep)
+    for r in range(R):
+        n, total = counts[r], counts[r] + held[r]
+        keys, vals = (x[table[r].long()].transpose(0, 1).reshape(G, -1, D)[:, :total].double() for x in (k, v))
+        s = torch.einsum("nghd,gkd->nghk", q[starts[r]:starts[r + 1]].double().view(n, G, H // G, D), keys) * D ** -0.5
+        at, key = torch.arange(held[r], total)[:, None], torch.arange(total)[None]
+        seen = (key <= at) & ((key > at - window) | (key < keep) if window else True)
+        p = torch.softmax(s.masked_fill(~seen[:, None, None], -torch.inf), -1)
+        want = torch.einsum("nghk,gkd->nghd", p, vals).reshape(n, -1)
+        err = (out[starts[r]:starts[r + 1]].double().cpu() - want).abs().max() / want.abs().max()
+        assert float(err) < 1.5e-2                              # P and the result rounded to bfloat16 (2^-8 each)

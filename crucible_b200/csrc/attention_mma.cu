@@ -11,8 +11,7 @@
 //                   of prompts.
 //   split kernel  - a block takes 16 rows and ONE chunk of 256 * 2^k keys, a
 //                   quarter per warp; writes an unnormalised partial (max, sum,
-//                   vector) to scratch; the last block of a row group to arrive
-//                   (an atomic counter: no block waits for another) merges the
+//                   vector) to scratch; a merge kernel, a block a row, adds the
 //                   chunks in ascending order.  For decoded tokens, where rows
 //                   are few and keys many.
 // Chunk boundaries are multiples of the chunk from key 0 whatever the batch
@@ -620,8 +619,8 @@ __global__ void __launch_bounds__(128) attention_tiles_kernel(const AttnParams p
 // in flight, no block-wide barrier in the loop) and attends to them with a
 // running maximum.  The warps' results are merged in warp order; if the rows
 // have a single chunk the output is written at once, else the chunk's partial
-// (max, sum, vector) goes to scratch and the block that arrives last at the rows'
-// counter merges the chunks in ascending order.  No block waits for another.
+// (max, sum, vector) goes to scratch and a second kernel merges the chunks in
+// ascending order.
 // ---------------------------------------------------------------------------
 template <int HD_MAX>
 struct SplitShape {
@@ -632,61 +631,73 @@ struct SplitShape {
 };
 
 
-// Merges one row's chunks (ascending, with a running maximum) and writes its
-// output.  One warp; lanes own features.  The loads of up to 8 chunks are issued
-// together, so the whole merge costs about one memory round trip per 8 chunks.
-__device__ __forceinline__ void merge_row(const AttnParams& p, int tok, int head, int pos, int lane) {
+// Merges a row's chunks: a block a row, 32 chunks at a time; a lane holds one's maximum and sum, a thread
+// owns two features, and all loads of a round are in flight at once.  (A block that arrived last and
+// merged its 16 rows alone read all their shares through one SM, 8 at a time: with 8 heads of 256
+// over 3,000 keys, 48 chunks, a decoded token took 29 us, 12.7 with this kernel; 16 heads over 12,000
+// 137 and 28.8; of 32 requests over 3,000, 8 chunks, 74 and 53; 3 chunks of heads of 80 16.6 and 13.7.
+// Part of that is the cheaper merge of a block's own warps.)
+__global__ void __launch_bounds__(128) split_merge_kernel(const AttnParams p) {
+    cb_pdl_trigger();
+    cb_pdl_wait();
+    const int req = blockIdx.z, kv_head = blockIdx.y, row = blockIdx.x, lane = threadIdx.x & 31;
+    const int n_rep = p.n_heads / p.n_kv_heads;
+    const int row_base = p.req_row_start[req];
+    const int n_rows = (p.req_row_start[req + 1] - row_base) * n_rep;
+    if (row >= n_rows) return;
+    const int first_pos = p.req_first_pos[req], qt = row >> 4;
+    // a tile of 16 rows with one chunk has written its results (the split kernel's test)
+    const int tile_end = first_pos + min(n_rows - 1, qt * 16 + 15) / n_rep;
+    const int tile_lo = p.window > 0 ? max(0, first_pos + (qt * 16) / n_rep - p.window + 1) : 0;
+    if (tile_end / p.chunk_keys == tile_lo / p.chunk_keys) return;
+    const int pos = first_pos + row / n_rep, tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
     const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
-    const int mp = p.head_dim + 2;
-    const int c_first = lo / p.chunk_keys, c_last = pos / p.chunk_keys;
+    const int c_first = lo / p.chunk_keys, c_last = pos / p.chunk_keys, mp = p.head_dim + 2;
     const float* base = p.partial + ((size_t)tok * p.n_heads + head) * p.n_chunks * mp;
+    const int f = 2 * threadIdx.x;
+    const bool live = f < p.head_dim;
     float m = -INFINITY, l = 0.f;
-    float acc[8];
+    float2 acc = make_float2(0.f, 0.f);
+    for (int c0 = c_first; c0 <= c_last; c0 += 32) {
+        const bool in = c0 + lane <= c_last;
+        const float2 stat = in ? __ldcg(reinterpret_cast<const float2*>(base + (size_t)(c0 + lane) * mp + p.head_dim))
+                               : make_float2(-INFINITY, 0.f);
+        float2 part[32];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (int c0 = c_first; c0 <= c_last; c0 += 8) {
-        float mc[8], lc[8], oc[8][8];
+        for (int j = 0; j < 32; ++j)
+            part[j] = live && c0 + j <= c_last ? __ldcg(reinterpret_cast<const float2*>(base + (size_t)(c0 + j) * mp + f))
+                                               : make_float2(0.f, 0.f);
+        const float m_new = fmaxf(m, cb_warp_max(stat.x));
+        const float off = m_new == -INFINITY ? 0.f : m_new;
+        const float keep = exp2f(m - off), weight = exp2f(stat.x - off);
+        l = l * keep + cb_warp_sum(stat.y * weight);
+        acc.x *= keep;
+        acc.y *= keep;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const bool in = c0 + j <= c_last;
-            const float* src = base + (size_t)(in ? c0 + j : c_first) * mp;
-            mc[j] = in ? __ldcg(src + p.head_dim) : -INFINITY;
-            lc[j] = in ? __ldcg(src + p.head_dim + 1) : 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int f = lane + 32 * i;
-                oc[j][i] = (in && f < p.head_dim) ? __ldcg(src + f) : 0.f;
-            }
+        for (int j = 0; j < 32; ++j) {                  // ascending chunks
+            const float w = __shfl_sync(0xffffffffu, weight, j);
+            acc.x = fmaf(part[j].x, w, acc.x);
+            acc.y = fmaf(part[j].y, w, acc.y);
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {                    // ascending chunks
-            const float m_new = fmaxf(m, mc[j]);
-            const float off = m_new == -INFINITY ? 0.f : m_new;
-            const float keep = exp2f(m - off), take = exp2f(mc[j] - off);
-            l = l * keep + lc[j] * take;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] = acc[i] * keep + oc[j][i] * take;
-            m = m_new;
-        }
+        m = m_new;
     }
+    if (!live) return;
     const float inv = l > 0.f ? 1.0f / l : 0.f;
-    __nv_bfloat16* dst = p.out + (size_t)tok * p.out_stride + (size_t)head * p.head_dim;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int f = lane + 32 * i;
-        if (f < p.head_dim) dst[f] = __float2bfloat16_rn(acc[i] * inv);
-    }
+    __nv_bfloat16* dst = p.out + (size_t)tok * p.out_stride + (size_t)head * p.head_dim + f;
+    dst[0] = __float2bfloat16_rn(acc.x * inv);
+    dst[1] = __float2bfloat16_rn(acc.y * inv);
 }
 
 template <int HD_MAX, bool EXACT>
-__global__ void __launch_bounds__(128) attention_split_kernel(const AttnParams p, int* counters,
-                                                              int max_q_tiles) {
+__global__ void __launch_bounds__(128) attention_split_kernel(const AttnParams p) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int SUB = SplitShape<HD_MAX>::SUB;
     constexpr int RING = SplitShape<HD_MAX>::RING;
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    __shared__ int is_last;
+    __shared__ float2 warp_stat[4][16];                // a warp's (maximum, sum) of every row
+    __shared__ float warp_weight[4][16], row_sum[16];
+    __shared__ size_t row_at[16];
     const int pitch = EXACT ? HD_MAX + 8 : p.head_dim + 8;
     __nv_bfloat16* q_smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
     __nv_bfloat16* kv_smem = q_smem + 16 * pitch;      // [warp][RING][K, V][SUB][pitch]
@@ -783,88 +794,76 @@ __global__ void __launch_bounds__(128) attention_split_kernel(const AttnParams p
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
 
-    // merge the four warps through shared memory, reusing the key/value rings: per
-    // warp 16 rows x (head_dim + 2) floats.  Warp w holds sub-tiles w, w+4, ...; the
-    // merge takes the warps in a fixed order, so the result does not vary
+    // merge the four warps through shared memory, reusing the key/value rings: per warp 16 rows
+    // of head_dim + 8 floats (pairs of a quarter warp in banks of their own).  Warp w holds
+    // sub-tiles w, w+4, ...; the merge takes the warps in a fixed order, so the result does not
+    // vary.  What a row needs but once (its maximum, the warps' weights, its place) one thread
+    // works out; the rest take pairs of features.
     __syncthreads();
     float* merge = reinterpret_cast<float*>(kv_smem);
-    const int mp = p.head_dim + 2;
+    const int mp = p.head_dim + 2, wide = p.head_dim + 8;
     {
-        float* mine = merge + (size_t)warp * 16 * mp;
+        float* mine = merge + (size_t)warp * 16 * wide;
 #pragma unroll
         for (int n = 0; n < HD_MAX / 8; ++n) {
             if (n * 8 < p.head_dim) {
                 const int col = n * 8 + 2 * t;
-                mine[g * mp + col] = o[n][0];
-                mine[g * mp + col + 1] = o[n][1];
-                mine[(g + 8) * mp + col] = o[n][2];
-                mine[(g + 8) * mp + col + 1] = o[n][3];
+                *reinterpret_cast<float2*>(mine + g * wide + col) = make_float2(o[n][0], o[n][1]);
+                *reinterpret_cast<float2*>(mine + (g + 8) * wide + col) = make_float2(o[n][2], o[n][3]);
             }
         }
         if (t == 0) {
-            mine[g * mp + p.head_dim] = m_a;
-            mine[g * mp + p.head_dim + 1] = l_a;
-            mine[(g + 8) * mp + p.head_dim] = m_b;
-            mine[(g + 8) * mp + p.head_dim + 1] = l_b;
+            warp_stat[warp][g] = make_float2(m_a, l_a);
+            warp_stat[warp][g + 8] = make_float2(m_b, l_b);
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 16 * mp; i += 128) {
-        const int r = i / mp, f = i - r * mp;
-        const int row = qt * 16 + r;
-        if (row >= n_rows) continue;
-        float m = -INFINITY;
+    const int rows_here = min(16, n_rows - qt * 16);
+    if (threadIdx.x < rows_here) {
+        const int r = threadIdx.x, row = qt * 16 + r;
+        float m = -INFINITY, l = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) m = fmaxf(m, merge[((size_t)w * 16 + r) * mp + p.head_dim]);
-        float v;
-        if (f == p.head_dim) {
-            v = m;
+        for (int w = 0; w < 4; ++w) m = fmaxf(m, warp_stat[w][r].x);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float mw = warp_stat[w][r].x;
+            const float scale = mw == -INFINITY ? 0.f : exp2f(mw - m);
+            warp_weight[w][r] = scale;
+            l += warp_stat[w][r].y * scale;
+        }
+        const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
+        row_sum[r] = l;
+        if (n_active == 1) {
+            row_at[r] = (size_t)tok * p.out_stride + (size_t)head * p.head_dim;
         } else {
-            const int src = f == p.head_dim + 1 ? p.head_dim + 1 : f;
-            v = 0.f;
+            row_at[r] = (((size_t)tok * p.n_heads + head) * p.n_chunks + chunk) * mp;
+            *reinterpret_cast<float2*>(p.partial + row_at[r] + p.head_dim) = make_float2(m, l);
+        }
+    }
+    __syncthreads();
+    {
+        const int pairs = p.head_dim >> 1, step_r = 128 / pairs, step_f = 128 - step_r * pairs;
+        int r = threadIdx.x / pairs, f = threadIdx.x - r * pairs;
+        while (r < rows_here) {
+            float2 v = make_float2(0.f, 0.f);
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
-                const float mw = merge[((size_t)w * 16 + r) * mp + p.head_dim];
-                const float scale = mw == -INFINITY ? 0.f : exp2f(mw - m);
-                v += merge[((size_t)w * 16 + r) * mp + src] * scale;
+                const float2 x = *reinterpret_cast<const float2*>(merge + ((size_t)w * 16 + r) * wide + 2 * f);
+                v.x += x.x * warp_weight[w][r];
+                v.y += x.y * warp_weight[w][r];
             }
-        }
-        const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
-        if (n_active == 1) {
-            // the only chunk of these rows: normalise and write the output at once
-            if (f < p.head_dim) {
-                float l = 0.f;
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const float mw = merge[((size_t)w * 16 + r) * mp + p.head_dim];
-                    l += merge[((size_t)w * 16 + r) * mp + p.head_dim + 1] *
-                         (mw == -INFINITY ? 0.f : exp2f(mw - m));
-                }
-                p.out[(size_t)tok * p.out_stride + (size_t)head * p.head_dim + f] =
-                    __float2bfloat16_rn(l > 0.f ? v / l : 0.f);
+            if (n_active == 1) {                        // the only chunk of these rows: the output at once
+                const float l = row_sum[r];
+                __nv_bfloat16* dst = p.out + row_at[r] + 2 * f;
+                dst[0] = __float2bfloat16_rn(l > 0.f ? v.x / l : 0.f);
+                dst[1] = __float2bfloat16_rn(l > 0.f ? v.y / l : 0.f);
+            } else {
+                *reinterpret_cast<float2*>(p.partial + row_at[r] + 2 * f) = v;
             }
-        } else {
-            p.partial[(((size_t)tok * p.n_heads + head) * p.n_chunks + chunk) * mp + f] = v;
+            r += step_r;
+            f += step_f;
+            if (f >= pairs) f -= pairs, ++r;
         }
-    }
-    if (n_active == 1) return;
-    // the last block to arrive for these rows merges their chunks
-    int* counter = counters + ((size_t)req * p.n_kv_heads + kv_head) * max_q_tiles + qt;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int prev = atomicAdd(counter, 1);
-        is_last = prev == n_active - 1;
-        if (is_last) *counter = 0;                      // ready for the next launch
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    for (int r = warp; r < 16; r += 4) {
-        const int row = qt * 16 + r;
-        if (row >= n_rows) break;
-        const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
-        merge_row(p, tok, head, first_pos + row / n_rep, lane);
     }
 }
 
@@ -973,11 +972,11 @@ int launch_tiles_split(const AttnParams& p, int n_requests, int max_rows, cudaSt
 }
 
 template <int HD_MAX, bool EXACT>
-int launch_split_as(const AttnParams& p, int n_requests, int max_q_tiles, int* counters,
-                    cudaStream_t s) {
+int launch_split_as(const AttnParams& p, int n_requests, int max_rows, cudaStream_t s) {
+    const int max_q_tiles = (max_rows + 15) / 16;
     const int pitch = p.head_dim + 8;
     int smem = (16 + 4 * SplitShape<HD_MAX>::RING * 2 * SplitShape<HD_MAX>::SUB) * pitch * 2;
-    const int merge_bytes = 4 * 16 * (p.head_dim + 2) * 4;
+    const int merge_bytes = 4 * 16 * (p.head_dim + 8) * 4;
     if (16 * pitch * 2 + merge_bytes > smem) smem = 16 * pitch * 2 + merge_bytes;
     static bool configured = false;
     if (!configured && smem > 48 * 1024) {
@@ -987,16 +986,17 @@ int launch_split_as(const AttnParams& p, int n_requests, int max_q_tiles, int* c
         configured = true;
     }
     dim3 grid(max_q_tiles * p.n_chunks, p.n_kv_heads, n_requests);
-    cb_launch(attention_split_kernel<HD_MAX, EXACT>, dim3(grid), dim3(128), smem, s, p, counters,
-              max_q_tiles);
+    cb_launch(attention_split_kernel<HD_MAX, EXACT>, dim3(grid), dim3(128), smem, s, p);
+    if (p.n_chunks > 1)
+        cb_launch(split_merge_kernel, dim3(max_rows, p.n_kv_heads, n_requests), dim3(128), 0, s, p);
     return cb_last_error();
 }
 
 template <int HD_MAX>
-int launch_split(const AttnParams& p, int n_requests, int max_q_tiles, int* counters, cudaStream_t s) {
+int launch_split(const AttnParams& p, int n_requests, int max_rows, cudaStream_t s) {
     return p.head_dim == HD_MAX
-               ? launch_split_as<HD_MAX, true>(p, n_requests, max_q_tiles, counters, s)
-               : launch_split_as<HD_MAX, false>(p, n_requests, max_q_tiles, counters, s);
+               ? launch_split_as<HD_MAX, true>(p, n_requests, max_rows, s)
+               : launch_split_as<HD_MAX, false>(p, n_requests, max_rows, s);
 }
 
 }  // namespace
@@ -1009,19 +1009,9 @@ CB_EXPORT long cb_attention_split_scratch_floats(int n_tokens, int n_heads, int 
 
 CB_EXPORT int cb_attention_split_keys() { return SPLIT_KEYS; }
 
-// Counters (ints, zero before the first launch; the kernel leaves them zero) the
-// split form needs.
-CB_EXPORT long cb_attention_split_counters(int n_requests, int n_kv_heads, int max_new_tokens,
-                                           int n_heads) {
-    const int max_rows = max_new_tokens * (n_heads / n_kv_heads);
-    return (long)n_requests * n_kv_heads * ((max_rows + 15) / 16);
-}
-
 // n_chunks == 0: tiles kernel.  n_chunks > 0: split kernel over that many
 // chunks of chunk_keys keys (a multiple of 256, or of 64 for rows wider than 128; together they must cover the
-// longest context); `partial` must hold
-// cb_attention_split_scratch_floats floats and `counters`
-// cb_attention_split_counters zeroed ints.
+// longest context); `partial` must hold cb_attention_split_scratch_floats floats.
 // max_q_rows: the largest (new tokens x heads per group) of any request.
 CB_EXPORT int cb_attention_mma(const void* qkv, int qkv_stride, void* out, int out_stride,
                                const void* k_cache, const void* v_cache, const int* positions,
@@ -1029,8 +1019,7 @@ CB_EXPORT int cb_attention_mma(const void* qkv, int qkv_stride, void* out, int o
                                const int* block_table, int table_stride, int n_tokens,
                                int n_requests, int max_new_tokens, int n_heads, int n_kv_heads,
                                int head_dim, int page_tokens, float scale, int window,
-                               float* partial, int* counters, int n_chunks, int chunk_keys,
-                               void* stream) {
+                               float* partial, int n_chunks, int chunk_keys, void* stream) {
     if (n_tokens <= 0 || n_requests <= 0) return 0;
     if (head_dim <= 0 || head_dim > 256 || (head_dim & 15) || n_heads % n_kv_heads != 0 ||
         (qkv_stride & 7) || (out_stride & 1) || ((uintptr_t)qkv & 15) || ((uintptr_t)k_cache & 15) ||
@@ -1079,15 +1068,14 @@ CB_EXPORT int cb_attention_mma(const void* qkv, int qkv_stride, void* out, int o
     }
     // a chunk is whole sub-tiles for each of the four warps: 4 x 16 keys for rows of more than
     // 128 features, whole tiles of SPLIT_KEYS otherwise
-    if (partial == nullptr || counters == nullptr ||
+    if (partial == nullptr ||
         (chunk_keys % (head_dim > 128 ? 4 * SplitShape<256>::SUB : SPLIT_KEYS)) != 0)
         return CB_ERR_UNSUPPORTED;
-    const int q_tiles = (max_rows + 15) / 16;
-    if (head_dim <= 16) rc = launch_split<16>(p, n_requests, q_tiles, counters, s);
-    else if (head_dim <= 32) rc = launch_split<32>(p, n_requests, q_tiles, counters, s);
-    else if (head_dim <= 64) rc = launch_split<64>(p, n_requests, q_tiles, counters, s);
-    else if (head_dim <= 128) rc = launch_split<128>(p, n_requests, q_tiles, counters, s);
-    else rc = launch_split<256>(p, n_requests, q_tiles, counters, s);
+    if (head_dim <= 16) rc = launch_split<16>(p, n_requests, max_rows, s);
+    else if (head_dim <= 32) rc = launch_split<32>(p, n_requests, max_rows, s);
+    else if (head_dim <= 64) rc = launch_split<64>(p, n_requests, max_rows, s);
+    else if (head_dim <= 128) rc = launch_split<128>(p, n_requests, max_rows, s);
+    else rc = launch_split<256>(p, n_requests, max_rows, s);
     return rc;
 }
 

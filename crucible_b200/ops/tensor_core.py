@@ -704,7 +704,8 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
         n_chunks = -(-reqs.bucket // chunk_keys)
         floats = reqs.rows_end * n_heads * n_chunks * (head_dim + 2)
         partial = ctx.scratch("attn.partial", (floats,), torch.float32)
-        counters = _buffer(qkv.device, "attn.counters", blocks_per_chunk, torch.int32, zero=True)
+        if decode_tc:
+            counters = _buffer(qkv.device, "attn.counters", blocks_per_chunk, torch.int32, zero=True)
     if (decode_tc
             and _attention_decode_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads,
                                           head_dim, scale, window, cache, partial, counters,
@@ -728,14 +729,13 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
         _c_int(reqs.table_stride), _c_int(reqs.rows_end), _c_int(reqs.count),
         _c_int(reqs.max_new), _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim),
         _c_int(cache.page_tokens), ctypes.c_float(scale), _c_int(window or 0),
-        _c_void_p(partial.data_ptr() if partial is not None else 0),
-        _c_void_p(counters.data_ptr() if counters is not None else 0), _c_int(n_chunks),
+        _c_void_p(partial.data_ptr() if partial is not None else 0), _c_int(n_chunks),
         _c_int(chunk_keys), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
         raise RuntimeError(f"tensor-core attention failed to launch (CUDA error {code})")
-    _count(1)
+    _count(1)                                    # (one of the step's attention forms, its merge with it)
     return True
 
 

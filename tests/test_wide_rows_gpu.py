@@ -78,3 +78,29 @@ def test_with_a_sink(schedule, monkeypatch):
     cfg = sebalorn._latent_cfg(H, D, R, E, C, Q, scale)
     for slot, x in h.items():
         assert rel(got[slot], plain_sebalorn.latent_attention(x.double(), w, cfg, 1e-5, "")) < TOL[BF16]
+
+
+@pytest.mark.parametrize("D", [256, 80])
+@pytest.mark.parametrize("chunks,requests,window", [
+    (1, [(1, 255), (2, 3)], None),                # nothing to merge
+    (2, [(1, 400), (1, 3)], None),                # rows of one chunk are written at once
+    (9, [(1, 2100), (2, 250), (1, 0)], None),
+    (33, [(1, 8200), (3, 8190)], None),           # one chunk beyond 32 at a time
+    (33, [(1, 8200), (2, 8191)], 700)])           # a window: the row's own chunks alone
+def test_decoded_rows_of_many_chunks(D, chunks, requests, window, monkeypatch):
+    """A decoded row's keys in chunks, merged by a kernel of their own; heads that fill no tile."""
+    from test_kernels_gpu import _paged_case
+    from crucible_b200.ops import tensor_core
+    keys = 64 if D > 128 else 256
+    if D > 128:                                   # (chunks of 64 keys)
+        requests = [(n, h // 4) for n, h in requests]
+        window = window and window // 4
+    H, G = 10, 2
+    qkv, ctx, cache, binding, ref = _paged_case(BF16, H, G, D, 16, [(h, n) for n, h in requests], 7, window)
+    monkeypatch.setattr(tensor_core, "wide_row_chunk_keys", lambda *a: keys)
+    monkeypatch.setattr(tensor_core, "decode_chunk_keys", lambda *a: keys)
+    longest = max(n + h for n, h in requests)
+    assert -(-longest // keys) == chunks and ctx.host.max_new_tokens * (H // G) <= tensor_core.SPLIT_ROWS
+    out = torch.full((qkv.shape[0], H * D), float("nan"), device="cuda:0", dtype=BF16)
+    assert tensor_core.paged_attention(qkv, out, H, G, D, D ** -0.5, window, ctx, cache, binding)
+    assert rel(out.cpu(), ref) < TOL[BF16]

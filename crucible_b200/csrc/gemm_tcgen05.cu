@@ -1025,7 +1025,7 @@ CB_EXPORT int cb_gemm_tcgen05(const void* A, const void* W, void* C, int M, int 
 // expert, W [experts * w_rows, K] their matrices one below the other, and the plan on the device
 // says which rows are whose (NormArgs::plan and the fields after it, set by the caller in `norm`).
 // epi: STORE_BF16, STORE_F32 or SWIGLU_BF16 (N = the intermediate width, w_rows = 2 N).
-// bn: 64, 96 or 128.  Nothing of the plan is read on the host: a step replays as a graph.
+// bn: 64, 96, 128, 192 or 256 (the caller's `grouped_tile`).  Nothing of the plan is read on the host: a step replays as a graph.
 CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int M, int N, int K, int lda,
                                       int ldw, int ldc, int epi, int bn, int per_sm, int* status, void* stream,
                                       const void* norm) {

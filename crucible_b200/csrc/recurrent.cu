@@ -30,7 +30,9 @@
 // S, each with four or eight of its D entries in registers; a block is 128 threads.  A token
 // costs one pass over a lane's entries and one shuffle reduction of its sums.
 // The tokens' q, k, v and gates are staged in shared memory 16 tokens at a time, by
-// asynchronous copies one chunk ahead.
+// asynchronous copies one chunk ahead.  The bfloat16 engine sends long portions of prompts
+// through `recurrent_chunks.cu` instead, and decoded tokens through `matrix_step_kernel` here (a
+// token a request: S read and written once, 16 bytes a thread at a time).
 #define CB_PDL_BIT 11      // this file's bit in CRUCIBLE_PDL
 #include "common.cuh"
 

@@ -64,7 +64,7 @@ def rows_gate(x, g) -> None:
 
 WARP_ROWS = 2        # steps of up to this many rows take a warp per weight row ...
 SMALL_ROWS = 16      # ... and steps of up to this many that the tiles refuse
-HEADS_IN_ONE_LAUNCH = True   # many bfloat16 rows: the heads as the third axis of one tensor-core launch
+HEADS_IN_ONE_LAUNCH = True   # more bfloat16 rows: the heads as the third axis of one tensor-core launch
                              # (tests switch it off to reach the product per head with the same inputs)
 
 

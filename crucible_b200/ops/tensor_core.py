@@ -747,8 +747,9 @@ def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx,
 
     The kernel is chosen per request, not per step: requests that bring at most 16
     query rows per KV head (decoded tokens, tiny portions) run split over chunks of
-    keys, with the last block of a row group to arrive merging; longer portions run as
-    tiles (the tcgen05 kernel for head sizes 64 and 128, the mma.sync kernel of 64-row
+    keys, merged by a kernel of their own (heads of 64 and 128: by the last block of a row
+    group to arrive); longer portions run as tiles (the tcgen05 kernel for head sizes 64 and
+    128, and 256 where a cached row is key and value at once, the mma.sync kernel of 64-row
     tiles else).  A step that holds both kinds (single decoded tokens first, as the
     scheduler orders them, then portions) is two launches over disjoint runs of its
     requests; the shapes of both are functions of the step's shape."""

@@ -201,8 +201,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         for (int i = 0; i < STAGES; ++i) {
             tc::mbar_init(&s.kv_full[i], 1);
             tc::mbar_init(&s.kv_empty[i], 1);
-            tc::mbar_init(&s.v_full[i], 1);
-            tc::mbar_init(&s.v_empty[i], 1);
+            if (SPLIT) {
+                tc::mbar_init(&s.v_full[i], 1);
+                tc::mbar_init(&s.v_empty[i], 1);
+            }
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&s.s_full[b], 1);

@@ -1361,8 +1361,9 @@ CB_EXPORT int cb_mlstm_prepare(const void* proj, int proj_stride, int dtype, con
                                long slot_stride, long n_off, long m_off, int n_requests, void* stream) {
     if (n_rows <= 0) return 0;
     const int C = n_heads * (2 * key_dim + value_dim);
-    // rows whose groups of four elements lie on boundaries of their size are read in those
-    const int vec = ((C | n_heads * key_dim | proj_stride) & 3) == 0 && (uintptr_t)proj % (dtype == CB_F32 ? 16 : 8) == 0;
+    // rows whose groups of four elements lie on boundaries of their size are read and written in those
+    const int vec = ((C | n_heads * key_dim | proj_stride) & 3) == 0 && (uintptr_t)qkv % 16 == 0 &&
+                    (uintptr_t)proj % (dtype == CB_F32 ? 16 : 8) == 0;
     const dim3 grid(n_rows), block(vec ? (C >= 2048 ? 512 : (C / 4 + 31) / 32 * 32)
                                        : (C <= 512 ? 128 : (C >= 4096 ? 1024 : (C / 4 + 31) / 32 * 32)));
     cudaStream_t s = (cudaStream_t)stream;

@@ -190,3 +190,24 @@ def test_rows_off_the_wide_loads_boundaries_are_walked(lengths, monkeypatch):
             k.CHUNKS = k.STEP = True
         outs.append((out.cpu(), state.cpu()))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows_off,out_off", [(0, 1), (1, 0), (1, 1), (0, 2)])
+def test_mlstm_rows_off_the_wide_boundaries(dtype, rows_off, out_off):
+    """Rows or prepared rows that start on no boundary of four elements: moved one by one, the same bits."""
+    from crucible_b200.ops import recurrent as k
+    H, D, E, T, g = 2, 16, 24, 5, torch.Generator().manual_seed(5)
+    C = H * (2 * D + E)
+    proj = torch.randn(T, C + H * E, generator=g).to(dtype).to(DEV)
+    gates = torch.randn(T, 2 * H, generator=g).to(DEV)
+    bias = torch.randn(2, H, generator=g).to(DEV)
+    results = []
+    for a, b in ((0, 0), (rows_off, out_off)):
+        rows = torch.empty(proj.numel() + a, dtype=dtype, device=DEV)[a:].view(proj.shape).copy_(proj)
+        qkv = torch.full((T * C + b + 4,), float("nan"), device=DEV)
+        keep, into = torch.empty(T, H, device=DEV), torch.empty(T, H, device=DEV)
+        k.mlstm_prepare(rows, gates, bias[0], bias[1], 6.0, qkv[b:b + T * C].view(T, C), keep, into, H, D, E)
+        assert bool(torch.isnan(qkv[b + T * C:]).all())
+        results.append((qkv[b:b + T * C].cpu(), keep.cpu(), into.cpu()))
+    assert all(torch.equal(x, y) for x, y in zip(*results))

@@ -119,13 +119,14 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     const int kept_tiles = p.window > 0 ? min((p.keep_first + KT - 1) / KT, key_lo / KT) : 0;
     const int n_tiles = kept_tiles + (last_pos - key_lo) / KT + 1;
     auto tile_key0 = [&](int j) { return j < kept_tiles ? j * KT : key_lo + (j - kept_tiles) * KT; };
-    // a tile's rows of K or V; keys beyond the block's last position are zeros and not read
+    // a tile's rows of K or V; keys beyond the block's last position, and those of a page that was given
+    // back early (a tile may begin before the window does), are zeros and not read: no row sees them
     auto fetch = [&](int j, const float* cache, int n, float* to) {
         const int key0 = tile_key0(j);
         for (int i = tid; i < KT * (DP / 4); i += THREADS) {
             const int t = i / (DP / 4), d = (i % (DP / 4)) * 4, key = key0 + t;
-            if (key <= last_pos && d < n) {
-                const int page = table[key / p.page_tokens];
+            const int page = key <= last_pos && d < n ? table[key / p.page_tokens] : -1;
+            if (page >= 0) {
                 cp16(to + t * P + d,
                      cache + (((size_t)page * p.n_kv_heads + kvh) * p.page_tokens + key % p.page_tokens) * n + d);
             } else {

@@ -88,6 +88,32 @@ def test_attention_rows_have_their_own_bits(H, G, D, E, page, window, keep, chun
     assert bool(torch.isnan(again[150]).any())
 
 
+@pytest.mark.parametrize("H,G,D,page,window,keep,chunked", [
+    (4, 2, 64, 16, 70, 5, False), (2, 1, 144, 3, 33, 40, False), (4, 4, 128, 8, 64, 0, True)])
+def test_pages_that_no_row_sees_are_not_read(H, G, D, page, window, keep, chunked):
+    """Pages given back early (-1 in the table) lie in the tiles around a window and behind the kept tokens."""
+    g = torch.Generator().manual_seed(page)
+    firsts, portions = [360, 149], [41, 1]
+    per = -(-(360 + 41) // page)
+    table = torch.arange(2 * per, dtype=torch.int32).view(2, per)
+    k, v = (torch.randn(2 * per, G, page, D, generator=g).to(DEV) for _ in range(2))
+    cache = SimpleNamespace(keys=lambda s: k, values=lambda s: v, page_tokens=page)
+    q, gate = (torch.randn(sum(portions), H * D, generator=g).to(DEV) for _ in range(2))
+    opts = (None, cache)
+    given_back = table.clone()
+    for r, (first, n) in enumerate(zip(firsts, portions)):
+        seen = torch.zeros(per * page, dtype=torch.bool)
+        for pos in range(first, first + n):
+            low = pos - pos % window if chunked else max(0, pos - window + 1)
+            seen[low:pos + 1] = True
+            seen[:min(keep, pos + 1)] = True
+        given_back[r, ~seen.view(per, page).any(1)] = -1
+    assert int((given_back < 0).sum()) > per
+    outs = [_attend(portions, firsts, q, gate, *opts, t.to(DEV), H, G, D, D, window, keep, chunked, False)
+            for t in (table, given_back)]
+    assert torch.equal(*outs) and bool(torch.isfinite(outs[0]).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [(1, 33, 20), (16, 64, 768), (17, 31, 19), (64, 65, 16), (130, 100, 1), (200, 77, 67)])
 @pytest.mark.parametrize("accumulate", [False, True])

@@ -56,7 +56,9 @@ struct Args {
     float* out;                     // [rows][H][E]
     int H, G, D, E;
     const float *per_head, *kept;
-    // workspaces: rows [rows][H][D] (wq: queries over S0, ww: W, wk: keys decayed to the chunk's end),
+    float* kept_next;               // mLSTM: n and m as this slice ends, laid out like kept
+    int skip, limit;                // the slice: of every request's tokens those from skip on, limit at most
+    // workspaces, of the slice (Piece): rows [rows][H][D] (wq: queries over S0, ww: W, wk: keys decayed to the chunk's end),
     // wu [rows][H][E], ws [rows][H] of four numbers (see chunk_local), wg [chunks][H][D] decays; wl
     // [chunks][H][D][E] what a chunk adds to S, then S as it begins; wn [chunks][H][D] likewise of n and wm
     // [chunks][H] of m (mLSTM)
@@ -94,7 +96,18 @@ __device__ __forceinline__ void cp16(float* smem, const float* gmem) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gmem) : "memory");
 }
-// a chunk's place among the step's chunks: strictly growing over a request's chunks and over requests
+// The slice's rows of a request: [row0, row1) of the step; their rows of a workspace are `shift` less.
+// (A request's first: the rows of the requests before it, or limit for each of those if that is less.)
+struct Piece { int row0, row1, shift; };
+__device__ __forceinline__ Piece piece_of(const Args& a, int r) {
+    const int start = a.req_row_start[r], before = start - a.req_row_start[0];
+    Piece p;
+    p.row0 = start + a.skip;
+    p.row1 = min(a.req_row_start[r + 1], p.row0 + a.limit);
+    p.shift = p.row0 - (int)min((long)before, (long)r * a.limit);
+    return p;
+}
+// a chunk's place among the slice's chunks: strictly growing over a request's chunks and over requests
 __device__ __forceinline__ size_t chunk_place(int row, int r) { return (size_t)(row / CT + r); }
 
 // row t of a lower triangular matrix times a column in registers (pairs of neighbouring tokens), entries
@@ -205,8 +218,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     constexpr int P = DP + 4;                       // pitch: 8 neighbouring rows' 16-byte reads hit 32 banks
     constexpr bool VECTOR = VECTOR_DECAY<RULE>, DELTA = IS_DELTA<RULE>;
     const int r = blockIdx.z, head = blockIdx.y;
-    const int row0 = a.req_row_start[r] + blockIdx.x * CT;
-    const int cnt = min(CT, a.req_row_start[r + 1] - row0);
+    const Piece piece = piece_of(a, r);
+    const int row0 = piece.row0 + blockIdx.x * CT, own0 = row0 - piece.shift;
+    const int cnt = min(CT, piece.row1 - row0);
     if (cnt <= 0) return;
     extern __shared__ __align__(16) float smem[];
     float* sk = smem;                               // [CT][P]
@@ -235,7 +249,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     if (warp == 0) {
         // the chunk's numbers, a token a lane; tokens beyond the portion's end change nothing
         const bool in = lane < cnt;
-        const size_t at = (size_t)(row0 + lane) * H + head;
+        const size_t at = (size_t)(row0 + lane) * H + head, own_at = (size_t)(own0 + lane) * H + head;
         float dec = 1.f, b = 0.f;
         if (RULE == RULE_MLSTM) {
             float f = in ? a.sc0[at] : 0.f, i = in ? a.sc1[at] : -INFINITY;
@@ -252,7 +266,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
             const float before = __shfl_up_sync(0xffffffffu, i, 1);
             dec = lane == 0 ? 0.f : expf(f_own + before - i);
             b = in ? expf(i_own - i) : 0.f;
-            if (in) a.ws[at] = make_float4(f, 0.f, i, 0.f);
+            if (in) a.ws[own_at] = make_float4(f, 0.f, i, 0.f);
         } else {
             if (!VECTOR && in) dec = a.sc0[at];
             if (RULE != RULE_WKV && in) b = a.sc1[at];
@@ -273,8 +287,8 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
             if (in) {
                 const float to_end = l * (RULE == RULE_DELTA ? 1.f : b);
                 sf[lane] = to_end;
-                if (RULE == RULE_MLSTM) a.ws[at].y = to_end;
-                else a.ws[at] = make_float4(G, to_end, 0.f, 0.f);
+                if (RULE == RULE_MLSTM) a.ws[own_at].y = to_end;
+                else a.ws[own_at] = make_float4(G, to_end, 0.f, 0.f);
             }
         }
     }
@@ -391,19 +405,19 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     if (RULE == RULE_MLSTM && tid < cnt) {
         float n = 0.f;
         for (int s = 0; s <= tid; ++s) n += sA[tid * AP + s];
-        a.ws[(size_t)(row0 + tid) * H + head].w = n;
+        a.ws[(size_t)(own0 + tid) * H + head].w = n;
     }
-    const size_t first = (size_t)row0 * H + head;      // the chunk's first row of a workspace
+    const size_t first = (size_t)row0 * H + head, own = (size_t)own0 * H + head;      // the chunk's first row: results, workspaces
     // vector decays: keys decayed to the chunk's end, and the whole chunk's decay
     if (VECTOR && tid < D) {
         float to_end = 1.f;
         for (int t = cnt - 1; t >= 0; --t) {
             const float k = sk[t * P + tid] * to_end;
-            if (DELTA) a.wk[(first + (size_t)t * H) * D + tid] = k;
+            if (DELTA) a.wk[(own + (size_t)t * H) * D + tid] = k;
             else sk[t * P + tid] = k;               // (its dots have been taken)
             to_end *= sw[t * P + tid];
         }
-        a.wg[(chunk_place(row0, r) * H + head) * D + tid] = to_end;
+        a.wg[(chunk_place(own0, r) * H + head) * D + tid] = to_end;
     }
     // the columns: E of v, then (delta rules: W; other vector decays: the decayed queries) D of the keys.
     // Delta rules: two a thread, so that a row of N or A out of shared memory serves both
@@ -443,12 +457,12 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
             each_token<0>(f);
         }
         if (is_v) {
-            ValueColumn<RULE, COLS> f{x, sA, a.out + first * E + d, DELTA ? a.wu + first * E + d : nullptr,
+            ValueColumn<RULE, COLS> f{x, sA, a.out + first * E + d, DELTA ? a.wu + own * E + d : nullptr,
                                       RULE == RULE_SSD ? a.per_head[head] : 0.f, (size_t)H * E, cnt, apart, cols};
             each_token<0>(f);
         } else {
-            KeyColumn<RULE, P, COLS> f{x, sA, sq + d, VECTOR ? sw + d : sa, a.wq + first * D + d,
-                                       DELTA ? a.ww + first * D + d : nullptr, {}, (size_t)H * D, cnt, apart, cols};
+            KeyColumn<RULE, P, COLS> f{x, sA, sq + d, VECTOR ? sw + d : sa, a.wq + own * D + d,
+                                       DELTA ? a.ww + own * D + d : nullptr, {}, (size_t)H * D, cnt, apart, cols};
 #pragma unroll
             for (int i = 0; i < COLS; ++i) f.G[i] = 1.f;
             each_token<0>(f);
@@ -501,7 +515,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
                     }
                 }
             }
-            float* to = a.wl + (chunk_place(row0, r) * H + head) * (size_t)D * E;
+            float* to = a.wl + (chunk_place(own0, r) * H + head) * (size_t)D * E;
 #pragma unroll
             for (int i = 0; i < 4 * Q; ++i) {
                 const int d = 64 * (i / 4) + 4 * ty + i % 4;
@@ -516,7 +530,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
         if (RULE == RULE_MLSTM && tid < D) {
             float n = 0.f;
             for (int t = 0; t < cnt; ++t) n = fmaf(sk[t * P + tid], sf[t], n);
-            a.wn[(chunk_place(row0, r) * H + head) * D + tid] = n;
+            a.wn[(chunk_place(own0, r) * H + head) * D + tid] = n;
         }
     }
 }
@@ -531,7 +545,9 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
     cb_pdl_wait();
     const int r = blockIdx.z, head = blockIdx.y;
     const int D = a.D, E = a.E, H = a.H;
-    const int row0 = a.req_row_start[r], n = a.req_row_start[r + 1] - row0;
+    const Piece piece = piece_of(a, r);
+    const int own0 = piece.row0 - piece.shift, n = piece.row1 - piece.row0;
+    if (n <= 0) return;
     const int chunks = (n + CT - 1) / CT;
     const int slot = a.req_state_slot[r];
     const float* n0 = RULE == RULE_MLSTM ? a.kept + (size_t)r * (H * D + H) : nullptr;
@@ -545,7 +561,7 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
         if (RULE == RULE_WKV) return;
         __syncthreads();
         if (threadIdx.x < BATCH && c0 + (int)threadIdx.x < chunks)
-            sx[threadIdx.x] = a.ws[(size_t)(row0 + min(n, (c0 + (int)threadIdx.x + 1) * CT) - 1) * H + head];
+            sx[threadIdx.x] = a.ws[(size_t)(own0 + min(n, (c0 + (int)threadIdx.x + 1) * CT) - 1) * H + head];
         __syncthreads();
         if (RULE == RULE_SSD) {
             if (threadIdx.x < BATCH) sg[threadIdx.x] = sx[threadIdx.x].x, si[threadIdx.x] = 1.f;
@@ -570,7 +586,7 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
     const bool with_n = RULE == RULE_MLSTM && blockIdx.x == gridDim.x - 1;
     const int dn = threadIdx.x;
     float* S = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E + i;
-    const size_t first = chunk_place(row0, r) * H + head;
+    const size_t first = chunk_place(own0, r) * H + head;
     float* at = a.wl + first * (size_t)D * E + i;
     float4 s = mine ? *reinterpret_cast<const float4*>(S) : make_float4(0.f, 0.f, 0.f, 0.f);
     float v = with_n && dn < D ? n0[(size_t)head * D + dn] : 0.f;
@@ -609,8 +625,15 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const Args a) {
     }
     if (mine) *reinterpret_cast<float4*>(S) = s;
     if (with_n) {
-        if (dn < D) state_at(a.state, a.slot_stride, slot, a.n_off)[(size_t)head * D + dn] = v;
-        if (dn == 0) state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m;
+        float* next = a.kept_next != nullptr ? a.kept_next + (size_t)r * (H * D + H) : nullptr;
+        if (dn < D) {
+            state_at(a.state, a.slot_stride, slot, a.n_off)[(size_t)head * D + dn] = v;
+            if (next != nullptr) next[(size_t)head * D + dn] = v;
+        }
+        if (dn == 0) {
+            state_at(a.state, a.slot_stride, slot, a.m_off)[head] = m;
+            if (next != nullptr) next[(size_t)H * D + head] = m;
+        }
     }
 }
 
@@ -626,8 +649,9 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
     __shared__ __align__(16) float sq[DP * AP];      // [D][CT]: queries, a channel's tokens side by side
     __shared__ __align__(16) float half[2][16][128 + 4];
     const int r = blockIdx.z, head = blockIdx.y;
-    const int row0 = a.req_row_start[r] + blockIdx.x * CT;
-    const int cnt = min(CT, a.req_row_start[r + 1] - row0);
+    const Piece piece = piece_of(a, r);
+    const int row0 = piece.row0 + blockIdx.x * CT, own0 = row0 - piece.shift;
+    const int cnt = min(CT, piece.row1 - row0);
     if (cnt <= 0) return;
     const int D = a.D, E = a.E, H = a.H, g = head / (H / a.G);
     const int lane = threadIdx.x & 31, group = (threadIdx.x >> 5) & 1, upper = threadIdx.x >> 6, t0 = group * 16;
@@ -635,19 +659,19 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
         const int t = i % CT, d = (i / CT) * 4;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < cnt)
-            q = *reinterpret_cast<const float4*>(OWN_Q<RULE> ? a.wq + ((size_t)(row0 + t) * H + head) * D + d
+            q = *reinterpret_cast<const float4*>(OWN_Q<RULE> ? a.wq + ((size_t)(own0 + t) * H + head) * D + d
                                                              : a.qkv + (size_t)(row0 + t) * a.C + a.q_off + (size_t)g * D + d);
         sq[d * AP + t] = q.x; sq[(d + 1) * AP + t] = q.y; sq[(d + 2) * AP + t] = q.z; sq[(d + 3) * AP + t] = q.w;
     }
     __syncthreads();
-    const size_t place = chunk_place(row0, r) * H + head;
+    const size_t place = chunk_place(own0, r) * H + head;
     // the factors of a token's two shares (what it has within the chunk, what comes from the state), in
     // the lane of the token
     float within = 1.f, before = 1.f;
     {
         const int t = t0 + (lane & 15);
         float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!VECTOR_DECAY<RULE> && t < cnt) own = a.ws[(size_t)(row0 + t) * H + head];
+        if (!VECTOR_DECAY<RULE> && t < cnt) own = a.ws[(size_t)(own0 + t) * H + head];
         if (RULE == RULE_SSD) before = own.x;
         if (RULE == RULE_MLSTM) {
             const float* n = a.wn + place * D;
@@ -756,7 +780,9 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int tid = threadIdx.x;
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
-    const int row0 = a.req_row_start[r], row1 = a.req_row_start[r + 1];
+    const Piece piece = piece_of(a, r);
+    const int row0 = piece.row0, row1 = piece.row1, shift = piece.shift;
+    if (row0 >= row1) return;
     const int slot = a.req_state_slot[r];
     float* state = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E;
     auto place_of = [](int c) { return (c & 3) * CG + (c >> 2); };
@@ -780,7 +806,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
 #pragma unroll
             for (int t = ft; t < CT; t += STEP) {
                 if (t < cnt) {
-                    const size_t at = ((size_t)(base + t) * H + head) * D + fd;
+                    const size_t at = ((size_t)(base - shift + t) * H + head) * D + fd;
                     const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + fd;
                     cp16(rows + t * P + fd, a.wq + at);
                     cp16(rows + (CT + t) * P + fd, a.ww + at);
@@ -796,7 +822,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         if (tid < CT * CG) {
             const int t = tid / CG, c = (tid % CG) * 4;
             if (t < cnt && col0 + c < E) {
-                cp16(u + t * ET + c, a.wu + ((size_t)(base + t) * H + head) * E + col0 + c);
+                cp16(u + t * ET + c, a.wu + ((size_t)(base - shift + t) * H + head) * E + col0 + c);
             } else {
                 *reinterpret_cast<float4*>(u + t * ET + c) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
@@ -804,7 +830,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         if (!VECTOR && tid >= THREADS - CT) {
             const int t = tid - (THREADS - CT);
             if (t < cnt) cp16(reinterpret_cast<float*>(sc + buf * CT + t),
-                              reinterpret_cast<const float*>(a.ws + (size_t)(base + t) * H + head));
+                              reinterpret_cast<const float*>(a.ws + (size_t)(base - shift + t) * H + head));
             else sc[buf * CT + t] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -815,7 +841,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int orow = tid / CG, ocol = cg * 4;
     // the second product: a thread's four channels and four columns (of ET / 4 x DP / 4 threads)
     const int ud = (tid / CG) * 4, uc = (tid % CG) * 4;
-    if (row0 < row1) fetch(row0, 0);
+    fetch(row0, 0);
     int buf = 0;
     for (int base = row0; base < row1; base += CT, buf ^= 1) {
         const int cnt = min(CT, row1 - base);
@@ -833,7 +859,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        if (VECTOR && tid < D) sg[tid] = a.wg[(chunk_place(base, r) * H + head) * D + tid];
+        if (VECTOR && tid < D) sg[tid] = a.wg[(chunk_place(base - shift, r) * H + head) * D + tid];
         __syncthreads();
         // the rows over S
         {
@@ -970,16 +996,19 @@ int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
 }  // namespace
 
 // The rules and their operands are those of cb_matrix_memory (recurrent.cu); max_new: the most tokens a
-// request brings.  Workspaces, fp32, those the rule needs: wq (delta, channel, wkv), ww (delta, channel), wk
-// (channel) [rows][H][D], wu (delta, channel) [rows][H][E], ws [rows][H][4]; with chunks = rows / 32 +
-// requests: wg (wkv, channel) and wn (mLSTM) [chunks][H][D], wm (mLSTM) [chunks][H], wl (mLSTM, wkv, state
-// space) [chunks][H][D][E].
+// request brings.  The portions are taken in slices of `limit` tokens of every request (a multiple of 32, or
+// at least max_new: one slice), one after the other through the state, with the same bits whatever limit
+// is.  Workspaces, fp32, those the rule needs, rows being the slice's (no more than the step's, nor than
+// requests * limit): wq (delta, channel, wkv), ww (delta, channel), wk (channel) [rows][H][D], wu (delta, channel)
+// [rows][H][E], ws [rows][H][4]; with chunks = rows / 32 + requests: wg (wkv, channel) and wn (mLSTM)
+// [chunks][H][D], wm (mLSTM) [chunks][H], wl (mLSTM, wkv, state space) [chunks][H][D][E]; kept_room (mLSTM in
+// several slices) [2][requests][H*D + H].
 CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_off, int k_off, int v_off,
                                       const float* sc0, const float* sc1, const int* req_row_start,
                                       const int* req_state_slot, void* state, long slot_stride, long s_off,
                                       long n_off, long m_off, float* out, int n_requests, int max_new, int n_heads,
                                       int n_qk_heads, int key_dim, int value_dim, int w_off, const float* per_head,
-                                      const float* kept, float* wq, float* ww, float* wk, float* wu, float* ws,
+                                      const float* kept, int limit, float* kept_room, float* wq, float* ww, float* wk, float* wu, float* ws,
                                       float* wg, float* wl, float* wn, float* wm, void* stream) {
     if (n_requests <= 0 || max_new <= 0) return 0;
     const bool vector = rule == RULE_WKV || rule == RULE_CHANNEL;
@@ -988,7 +1017,8 @@ CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_o
         || ((s_off | slot_stride) & 15) != 0 || (((uintptr_t)state | (uintptr_t)qkv | (uintptr_t)out) & 15) != 0)
         return CB_ERR_UNSUPPORTED;
     if ((rule == RULE_WKV || rule == RULE_SSD) && per_head == nullptr) return CB_ERR_UNSUPPORTED;
-    if (rule == RULE_MLSTM && kept == nullptr) return CB_ERR_UNSUPPORTED;
+    if (rule == RULE_MLSTM && (kept == nullptr || (limit < max_new && kept_room == nullptr))) return CB_ERR_UNSUPPORTED;
+    if (limit <= 0 || (limit < max_new && limit % CT != 0)) return CB_ERR_UNSUPPORTED;
     Args a;
     a.qkv = qkv; a.C = C; a.q_off = q_off; a.k_off = k_off; a.v_off = v_off; a.w_off = w_off;
     a.sc0 = sc0; a.sc1 = sc1; a.req_row_start = req_row_start; a.req_state_slot = req_state_slot;
@@ -997,15 +1027,25 @@ CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_o
     a.per_head = per_head; a.kept = kept;
     a.wq = wq; a.ww = ww; a.wk = wk; a.wu = wu; a.wg = wg; a.wl = wl; a.wn = wn; a.wm = wm; a.ws = reinterpret_cast<float4*>(ws);
     cudaStream_t s = (cudaStream_t)stream;
+    a.limit = limit;
+    const size_t kept_size = (size_t)n_requests * n_heads * (key_dim + 1);
+    for (int skip = 0, slice = 0; skip < max_new; skip += limit, ++slice) {
+        a.skip = skip;
+        const int most = max_new - skip < limit ? max_new - skip : limit;
+        a.kept_next = rule == RULE_MLSTM && skip + most < max_new ? kept_room + (slice & 1) * kept_size : nullptr;
+        int rc = CB_ERR_UNSUPPORTED;
 #define CB_CHUNKS(RR)                                                                                       \
-    if (rule == RR)                                                                                         \
-        return key_dim <= 64 ? launch_chunks<64, RR>(a, n_requests, max_new, s)                             \
-                             : launch_chunks<128, RR>(a, n_requests, max_new, s)
-    CB_CHUNKS(RULE_DELTA);
-    CB_CHUNKS(RULE_MLSTM);
-    CB_CHUNKS(RULE_WKV);
-    CB_CHUNKS(RULE_SSD);
-    CB_CHUNKS(RULE_CHANNEL);
+        if (rule == RR)                                                                                     \
+            rc = key_dim <= 64 ? launch_chunks<64, RR>(a, n_requests, most, s)                              \
+                               : launch_chunks<128, RR>(a, n_requests, most, s)
+        CB_CHUNKS(RULE_DELTA);
+        CB_CHUNKS(RULE_MLSTM);
+        CB_CHUNKS(RULE_WKV);
+        CB_CHUNKS(RULE_SSD);
+        CB_CHUNKS(RULE_CHANNEL);
 #undef CB_CHUNKS
-    return CB_ERR_UNSUPPORTED;
+        if (rc) return rc;
+        a.kept = a.kept_next;
+    }
+    return 0;
 }

@@ -31,6 +31,23 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: int) -> bool
     return longest >= 160 or (longest >= 48 and rows >= 24 * requests and rows * heads >= 4096)
 
 
+CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces
+
+
+def slice_tokens(rows: int, requests: int, longest: int, row_bytes: int, chunk_bytes: int) -> int:
+    """Tokens of each of `requests` portions (`rows` tokens in all) that go through the chunks at a time: all of
+    the longest if the workspaces then stay within CHUNK_SPACE, else what does, in whole chunks and one
+    at least.  (16 heads of 128 x 128 take 25 to 33 KB a token, so that up to 8,000 tokens go at once;
+    a longer step's slices each fill the GPU.)"""
+    def space(tokens):
+        taken = min(rows, requests * tokens)
+        return taken * row_bytes + (taken // 32 + requests) * chunk_bytes
+    if space(longest) <= CHUNK_SPACE:
+        return longest
+    per_token = requests * (row_bytes + chunk_bytes / 32)
+    return max(32, int((CHUNK_SPACE - requests * chunk_bytes) / per_token) // 32 * 32)
+
+
 def _state_args(state: torch.Tensor):
     if state.dtype != torch.uint8 or state.dim() != 2 or state.stride(1) != 1:
         raise KernelError("a mixer's state is a uint8 view [slots, bytes]")
@@ -181,35 +198,42 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and chunks_pay(
                 rule, qkv.shape[0] - ctx.host.lead_single, n - ctx.host.lead_single, ctx.host.max_new_tokens, n_heads)
             and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0
-            and (s_off | state.stride(0)) % 16 == 0):
+            and (s_off | state.stride(0) | qkv.data_ptr() | out.data_ptr() | state.data_ptr()) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked
         walked = ctx.host.lead_single
-        rows, f32 = qkv.shape[0], torch.float32
+        longest, f32 = ctx.host.max_new_tokens, torch.float32
+        delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
+        # bytes a row and a chunk take in the workspaces, and the tokens of each request that go at a time
+        row_bytes = 4 * n_heads * (key_dim * ((delta or vector) + delta + (rule == CHANNEL)) + value_dim * delta + 4)
+        chunk_bytes = 4 * n_heads * (key_dim * (vector + (rule == MLSTM)) + (0 if delta else key_dim * value_dim) + 1)
+        limit = slice_tokens(qkv.shape[0] - walked, n - walked, longest, row_bytes, chunk_bytes)
+        rows = min(qkv.shape[0] - walked, (n - walked) * limit)
+        places = rows // 32 + n - walked
 
         def room(name, width, wanted=True):
             return ctx.scratch(f"memory.{name}", (rows, n_heads, width), f32) if wanted else None
-        delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
         wq, ww, wk = room("wq", key_dim, delta or vector), room("ww", key_dim, delta), room("wk", key_dim, rule == CHANNEL)
         wu, ws = room("wu", value_dim, delta), room("ws", 4)
-        places = rows // 32 + n
         wg = ctx.scratch("memory.wg", (places, n_heads, key_dim), f32) if vector else None
         wl = ctx.scratch("memory.wl", (places, n_heads, key_dim, value_dim), f32) if not delta else None
         wn = ctx.scratch("memory.wn", (places, n_heads, key_dim), f32) if rule == MLSTM else None
         wm = ctx.scratch("memory.wm", (places, n_heads), f32) if rule == MLSTM else None
+        kept_room = (ctx.scratch("memory.kept", (2, n - walked, n_heads * (key_dim + 1)), f32)
+                     if rule == MLSTM and limit < longest else None)
         lib = build.load("recurrent_chunks")
         code = lib.cb_matrix_memory_chunks(
             _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
             _ptr(sc0), _ptr(sc1), _c_void_p(starts + 4 * walked), _c_void_p(slots + 4 * walked), sp, stride,
             _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(n - walked),
-            _c_int(ctx.host.max_new_tokens), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
+            _c_int(longest), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
             _c_int(w_off), _ptr(per_head),
             _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
-            _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream())
-        if code == build.UNSUPPORTED:            # (rows on boundaries that its loads do not take): the walk's
+            _c_int(limit), _ptr(kept_room), _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream())
+        if code == build.UNSUPPORTED:            # the walk's
             walked = n
         else:
             _check(code, "matrix_memory (chunks)")
-            LAUNCHES[0] += 1 if delta else 2     # (two kernels, or three)
+            LAUNCHES[0] += (2 if delta else 3) * -(-longest // limit) - 1
     if walked == 0:
         return
     lib = build.load("recurrent")

@@ -105,3 +105,18 @@ def test_step_shape_key_follows_what_launches_depend_on():
     assert later.shape_key() == mixed.shape_key()
     prompts = HostStep(list("ab"), [700, 1], [0, 50], [700, 51], [0, 1])
     assert prompts.shape_key() == (700, 0, 0, 0)
+
+
+def test_the_chunks_workspaces_are_bounded():
+    """All of a step at once while that fits, else slices of whole chunks that fit (or of one chunk)."""
+    from crucible_b200.ops.recurrent import CHUNK_SPACE, slice_tokens
+    for rows, requests, longest in [(2048, 1, 2048), (6518, 5, 2048), (16384, 1, 16384), (40000, 3, 30000),
+                                    (50000, 48, 2000), (9000, 300, 31), (100000, 1, 100000)]:
+        for row_bytes, chunk_bytes in [(256, 1 << 20), (24832, 64), (41216, 8256), (256, 1 << 22)]:
+            n = slice_tokens(rows, requests, longest, row_bytes, chunk_bytes)
+            taken = min(rows, requests * n)
+            space = taken * row_bytes + (taken // 32 + requests) * chunk_bytes
+            assert n == longest or (n % 32 == 0 and 32 <= n < longest + 32)
+            assert space <= CHUNK_SPACE or n == 32
+            if rows * row_bytes + (rows // 32 + requests) * chunk_bytes <= CHUNK_SPACE:
+                assert n == longest

@@ -143,6 +143,45 @@ def test_chunks_agree_with_float64(rule, H, G, D, E, monkeypatch):
                 assert got <= max(8 * plain, 2e-6), (rule, lengths, r, errors)
 
 
+@pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
+@pytest.mark.parametrize("space,limit", [(0, 32), (None, 64), (None, 128)])
+def test_slices_have_the_bits_of_one(rule, space, limit, monkeypatch):
+    """A step whose workspaces would be too large goes in slices of its portions: the same numbers in less room."""
+    from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
+    code, H, D, whole = getattr(k, rule), 3, 64, k.CHUNK_SPACE
+    for lengths in [(1, 128, 33, 1), (300,), (129, 31, 70), (20, 64, 257)]:
+        g = torch.Generator().manual_seed(len(lengths))
+        T, R = sum(lengths), len(lengths)
+        q, kk, v, w, sc0, sc1, per_head = _operands(code, k, T, H, H, D, D, g)
+        on = lambda x: x.contiguous().to(DEV) if x is not None else None
+        qkv = on(torch.cat([x.reshape(T, -1) for x in (q, kk, v, w) if x is not None], 1))
+        before = torch.randn(R, H * D * D + H * D + 4, generator=g) * 0.3
+        results, asked = [], []
+        for cut in (False, True):
+            ctx, _, _ = _ctx(lengths, torch.bfloat16)
+            room = ctx.scratch
+            ctx.scratch = lambda name, shape, kind: asked.append((name, tuple(shape))) or room(name, shape, kind)
+            if cut and space is None:
+                monkeypatch.setattr(k, "slice_tokens", lambda *a: limit)
+            if cut and space is not None:
+                monkeypatch.setattr(k, "CHUNK_SPACE", space)
+            asked.clear()
+            state = on(before).clone().view(torch.uint8)
+            out = torch.full((T, H * D), float("nan"), device=DEV)
+            k.matrix_memory(code, qkv, 0, H * D, 2 * H * D, on(sc0), on(sc1), ctx, state, 0, 4 * H * D * D,
+                            4 * (H * D * D + H * D), out, H, H, D, D, w_off=3 * H * D, per_head=on(per_head))
+            results.append((out.cpu(), state.view(torch.float32).cpu()))
+        monkeypatch.undo()
+        monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
+        assert k.CHUNK_SPACE == whole
+        portions = R - (lengths[0] == 1)
+        rows = dict(asked)["memory.ws"][0]
+        assert rows <= min(T, portions * limit)
+        assert bool(torch.isfinite(results[0][0]).all())
+        assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1]), lengths
+
+
 @pytest.mark.parametrize("rule", ["DELTA", "CHANNEL", "SSD", "WKV", "MLSTM"])
 def test_a_later_token_does_not_reach_an_earlier_one(rule, monkeypatch):
     """A value that is not a number stays with its own and later tokens of its own request."""

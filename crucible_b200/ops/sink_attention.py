@@ -135,15 +135,10 @@ def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, 
     if key_dim == value_dim:
         first = tensor_core.prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, key_dim, scale, window,
                                              keep_first, ctx, cache, table, chunked=chunked, sinks=sinks,
-                                             out_scale=out_scale, gate=None if gate_per_head else gate)
+                                             out_scale=out_scale, gate=gate, gate_per_head=gate_per_head)
+    if first == 0:
+        return True
     if first < ctx.n_requests:
-        if gate is not None and gate_per_head:
-            # one logit a head: a pass over the heads' results behind the attention (the requests
-            # before `first` bring a row each)
-            from . import latent
-            latent.head_gate(out[first:], gate[first:], n_heads, value_dim)
-        if first == 0:
-            return True
         count, max_new, bucket = first, 1, host.lead_context_bucket
     else:
         count, max_new, bucket = ctx.n_requests, host.max_new_tokens, host.context_bucket

@@ -514,12 +514,12 @@ def _tcgen05_rows(head_dim, k_cache, v_cache) -> bool:
 
 def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale,
                        window, cache, keep_first: int = 0, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                       gate=None) -> bool:
+                       gate=None, gate_per_head: bool = False) -> bool:
     """tcgen05 attention for portions of prompts: head sizes of `_tcgen05_rows`, page size a
     power of two from 8 to 128.  `keep_first` (with a window): keys before that position stay
     visible.  `chunked`: the window is a chunk's size.  `sinks`: float32 per query head or None.
-    `gate`: rows laid out like `out` whose sigmoids the results are multiplied by, or None.
-    Returns False for anything else."""
+    `gate`: rows laid out like `out` (`gate_per_head`: one logit a head) whose sigmoids the results are
+    multiplied by before they are rounded, or None.  Returns False for anything else."""
     pt = cache.page_tokens
     if pt < 8 or pt > 128 or pt & (pt - 1):
         return False
@@ -534,7 +534,7 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         ctypes.c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first if window else 0),
         ctypes.c_float(out_scale), _c_void_p(sinks.data_ptr() if sinks is not None else 0),
         _c_void_p(gate.data_ptr() if gate is not None else 0), _c_int(gate.stride(0) if gate is not None else 0),
-        _c_int(ATTENTION_LEAN), _c_void_p(status_word(qkv.device).data_ptr()), _stream())
+        _c_int(1 if gate_per_head else 0), _c_int(ATTENTION_LEAN), _c_void_p(status_word(qkv.device).data_ptr()), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -658,17 +658,18 @@ MIXED_REACH = 2560 * 128     # keys times features
 
 def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, scale, window, keep_first,
                      ctx, cache, table, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                     gate=None) -> int:
+                     gate=None, gate_per_head: bool = False) -> int:
     """The tcgen05 attention for the requests of a step from `tiles_first` on, over keys and values of
     one size (`_tcgen05_rows`), with a window that may keep the first tokens or (`chunked`) is the size of
-    chunks, and with a sink per head in the softmax (`sinks`) or none; `gate`: a logit for every result, or
-    None.  `q`: rows of n_heads * head_dim.  Returns the first request taken (`ctx.n_requests`: none)."""
+    chunks, and with a sink per head in the softmax (`sinks`) or none; `gate`: a logit for every result or
+    (`gate_per_head`) head, or None.  `q`: rows of n_heads * head_dim.  Returns the first request taken (`ctx.n_requests`: none)."""
     host, none = getattr(ctx, "host", None), ctx.n_requests
     n_rep = n_heads // n_kv_heads
     if (not USE_TCGEN05_ATTENTION or host is None or q.dtype != torch.bfloat16
             or not _tcgen05_rows(head_dim, k_cache, v_cache) or k_cache.dtype != torch.bfloat16
             or q.stride(0) % 8 or out.stride(0) % 8 or q.data_ptr() % 16 or out.data_ptr() % 16
-            or (gate is not None and (gate.dtype != q.dtype or gate.stride(0) % 8 or gate.data_ptr() % 16))
+            or (gate is not None and (gate.dtype != q.dtype or (not gate_per_head and (
+                gate.stride(0) % 8 or gate.data_ptr() % 16))))
             or k_cache.shape[-1] != head_dim or v_cache.shape[-1] != head_dim):
         return none
     first = tiles_first(host, none, head_dim, window, keep_first)
@@ -676,7 +677,8 @@ def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, sc
         return none
     reqs = _Requests(ctx, table, first, none - first, host.max_new_tokens, host.context_bucket, ctx.n_tokens)
     taken = _attention_tcgen05(q, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, cache,
-                               keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate)
+                               keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate,
+                               gate_per_head=gate_per_head)
     return first if taken else none
 
 

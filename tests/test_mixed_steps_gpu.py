@@ -99,3 +99,34 @@ def test_heads_of_128_two_groups_of_softmax_warps(counts, held, window, keep, or
         want = torch.einsum("nghk,gkd->nghd", p, vals).reshape(n, -1)
         err = (out[starts[r]:starts[r + 1]].double().cpu() - want).abs().max() / want.abs().max()
         assert float(err) < 1.5e-2                              # P and the result rounded to bfloat16 (2^-8 each)
+
+
+@pytest.mark.parametrize("H,G,D", [(4, 4, 64), (8, 2, 128), (16, 1, 256)])
+@pytest.mark.parametrize("counts,held", [([65, 130], [0, 37]), ([1, 1, 300], [40, 200, 11])])
+def test_a_logit_a_head_counts_before_the_rounding(H, G, D, counts, held):
+    """The tiles' gate of one logit a head: the bits of a gate with that logit at each of the head's features,
+    which is multiplied in before the result is rounded to bfloat16."""
+    from crucible_b200.engine.context import HostStep
+    from crucible_b200.ops import sink_attention
+    g, page, R, T = torch.Generator().manual_seed(D), 16, len(counts), sum(counts)
+    contexts = [c + h for c, h in zip(counts, held)]
+    per = -(-max(contexts) // page)
+    table = torch.randperm(R * per, generator=g).to(torch.int32).view(R, per).to(DEV)
+    k = torch.randn(R * per, G, page, D, generator=g).to(torch.bfloat16).to(DEV)
+    v = k if D == 256 else torch.randn(k.shape, generator=g).to(torch.bfloat16).to(DEV)
+    starts = [0]
+    for n in counts:
+        starts.append(starts[-1] + n)
+    ctx = SimpleNamespace(n_requests=R, n_tokens=T, req_row_start=_i32(starts), req_first_pos=_i32(held),
+                          block_table=lambda group: table, host=HostStep(list(range(R)), counts, held, contexts, list(range(R))))
+    cache = SimpleNamespace(keys=lambda s: k, values=lambda s: v, page_tokens=page)
+    q = torch.randn(T, H * D, generator=g).to(torch.bfloat16).to(DEV)
+    rows = torch.randn(T, H + 3, generator=g).to(torch.bfloat16).to(DEV)      # columns of a wider projection
+    outs = []
+    for per_head in (True, False):
+        gate = rows[:, 1:H + 1] if per_head else rows[:, 1:H + 1].repeat_interleave(D, 1).contiguous()
+        out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        sink_attention.attention(q, gate, out, None, H, G, D, D, D ** -0.5, None, 0, 1.0, ctx, cache,
+                                 SimpleNamespace(slot=0, group=0), gate_per_head=per_head)
+        outs.append(out)
+    assert torch.equal(*outs) and bool(torch.isfinite(outs[0]).all())

@@ -74,27 +74,25 @@ struct TcAttnParams {
                              // the keys of its own chunk up to itself
     float out_scale;         // every result times this
     const float* sinks;      // [n_heads] or null: exp(sink) joins a row's denominator, with no value
-    const __nv_bfloat16* gate;   // null, or logits: every result times sigmoid(logit); rows laid out like
-    int gate_stride;             // `out`, or (gate_per_head) one logit a head
-    int gate_per_head;
+    const __nv_bfloat16* gate;   // logits: every result times sigmoid(logit); rows laid out like `out`, or
+    int gate_stride;             // (GATE_HEAD) one logit a head
     int n_pages;             // of the pool
     int runs;                // 1: the 4-D maps may be used for tiles whose pages are consecutive
     int* status;
 };
 
-// Eight results times the sigmoids of their logits, which lie at `logits` from `first` on (or of one).
-__device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits, int per_head, int first) {
-    if (per_head) {
-        const float f = 1.0f / (1.0f + expf(-__bfloat162float(*logits)));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] *= f;
-        return;
-    }
-    const uint4 raw = *reinterpret_cast<const uint4*>(logits + first);
+// Eight results times the sigmoids of their logits.
+__device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(logits);
     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] *= 1.0f / (1.0f + expf(-__bfloat162float(g[i])));
 }
+
+// GATE: the results' gate, fixed when it is compiled: the epilogue runs once per block and its instructions
+// come from memory (12 heads of 64 without a gate, a 2,048-token prompt: 32 us; with the code of the gate of a
+// logit a result beside it 0.3 us more, of both gates 1.4).
+enum Gate { GATE_NONE = 0, GATE_RESULT = 1, GATE_HEAD = 2 };
 
 // HD: the head size, 64 or 128.  Operands whose contracted or free dimension is the head
 // size lie in shared memory as HD / 64 halves of [rows][128 bytes] (one swizzle atom wide).
@@ -179,7 +177,7 @@ __device__ __forceinline__ void fma_pair(float& x0, float& x1, float a, float b)
         : "f"(a), "f"(b));
 }
 
-template <int HD, bool LEAN>
+template <int HD, bool LEAN, int GATE>
 __global__ void __launch_bounds__(Storage<HD, LEAN>::THREADS, LEAN ? 2 : 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v,
@@ -669,12 +667,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         if (ok && my_tiles > 0) ok = wait_all(&s.pv_done[j_last % PB], (j_last / PB) & 1);
         __nv_bfloat16* dst = nullptr;
         const __nv_bfloat16* gate = nullptr;
+        float gate_f = 1.f;
         float sink = -INFINITY;                       // in the base-2 exponent
         if (real) {
             const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
             if (p.sinks != nullptr) sink = p.sinks[head] * LOG2E;
             dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
-            if (p.gate != nullptr) gate = p.gate + (size_t)tok * p.gate_stride + (p.gate_per_head ? (size_t)head : (size_t)head * HD);
+            if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
+            if (GATE == GATE_HEAD)
+                gate_f = 1.0f / (1.0f + expf(-__bfloat162float(p.gate[(size_t)tok * p.gate_stride + head])));
         }
         if (GROUPS > 1) {
             // Two groups: each holds the sums over its own tiles against its own reference.
@@ -712,7 +713,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                                    (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
-                            if (gate != nullptr) gate_eight(o + 8 * q4, gate, p.gate_per_head, c0 + 8 * q4);
+                            if (GATE == GATE_RESULT) gate_eight(o + 8 * q4, gate + c0 + 8 * q4);
+                            if (GATE == GATE_HEAD) {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= gate_f;
+                            }
                             uint4 w;
                             w.x = pack_bf16(o[8 * q4 + 0], o[8 * q4 + 1]);
                             w.y = pack_bf16(o[8 * q4 + 2], o[8 * q4 + 3]);
@@ -742,7 +747,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                         float o[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[8 * q4 + i]) * inv;
-                        if (gate != nullptr) gate_eight(o, gate, p.gate_per_head, c0 + 8 * q4);
+                        if (GATE == GATE_RESULT) gate_eight(o, gate + c0 + 8 * q4);
+                        if (GATE == GATE_HEAD) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) o[i] *= gate_f;
+                        }
                         uint4 w;
                         w.x = pack_bf16(o[0], o[1]);
                         w.y = pack_bf16(o[2], o[3]);
@@ -762,21 +771,31 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     }
 }
 
-template <int HD, bool LEAN>
-int launch_as(dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
+template <int HD, bool LEAN, int GATE>
+int launch_gate(dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
               const CUtensorMap& rk, const CUtensorMap& rv, const TcAttnParams& p) {
     constexpr int smem = (int)sizeof(Storage<HD, LEAN>);
     static_assert(smem <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, LEAN>,
+        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, LEAN, GATE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    cb_launch(attention_tcgen05_kernel<HD, LEAN>, grid, dim3(Storage<HD, LEAN>::THREADS), smem, st, mk, mv, rk,
+    cb_launch(attention_tcgen05_kernel<HD, LEAN, GATE>, grid, dim3(Storage<HD, LEAN>::THREADS), smem, st, mk, mv, rk,
               rv, p);
     return cb_last_error();
+}
+
+template <int HD, bool LEAN>
+int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
+              const CUtensorMap& rk, const CUtensorMap& rv, const TcAttnParams& p) {
+    switch (gate) {
+        case GATE_NONE: return launch_gate<HD, LEAN, GATE_NONE>(grid, st, mk, mv, rk, rv, p);
+        case GATE_RESULT: return launch_gate<HD, LEAN, GATE_RESULT>(grid, st, mk, mv, rk, rv, p);
+    }
+    return launch_gate<HD, LEAN, GATE_HEAD>(grid, st, mk, mv, rk, rv, p);
 }
 
 }  // namespace
@@ -839,7 +858,6 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     p.sinks = sinks;
     p.gate = (const __nv_bfloat16*)gate;
     p.gate_stride = gate_stride;
-    p.gate_per_head = gate_per_head;
     p.out_scale = out_scale;
     p.status = status;
     const int n_rep = n_heads / n_kv_heads;
@@ -852,11 +870,12 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     // 4.86 ms; 4,096 tokens of the 120M shape, 384 blocks, 1.68 against 1.96 ms), so the launch
     // decides for it; the lean form stays for callers that ask for it.
     if (lean < 0) lean = 0;
+    const int form = gate == nullptr ? GATE_NONE : gate_per_head ? GATE_HEAD : GATE_RESULT;
     if (head_dim == 64)
-        return lean ? launch_as<64, true>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p)
-                    : launch_as<64, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
-    if (head_dim == 256) return launch_as<256, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
-    return launch_as<128, false>(grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
+        return lean ? launch_as<64, true>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p)
+                    : launch_as<64, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
+    if (head_dim == 256) return launch_as<256, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
+    return launch_as<128, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
 }
 
 CB_EXPORT int cb_attention_tcgen05(const void* qkv, int qkv_stride, void* out, int out_stride,

@@ -83,23 +83,20 @@ struct NormArgs {
     float width, eps;
     // SWIGLU_BF16: limit > 0 makes the pair the capped one (tc::gated_pair), else silu(g) * u
     float glu_limit, glu_alpha, glu_offset;
-    // A grouped product (plan != null): the rows of A lie expert by expert, W is the experts'
+    // A grouped product (form GROUPED): the rows of A lie expert by expert, W is the experts'
     // matrices one below the other (w_rows rows each), and block row y takes tile y of the plan
     // that a kernel before this one left on the device: [0] tiles in use, [2 + E + y] the tile's
     // expert, [2 + E + max_tiles + y] its first row, [2 + E + 2 max_tiles + y] its rows (at most
     // 128).  Tiles beyond those in use do nothing.
     const int* plan;
     int n_experts, max_tiles, w_rows;
-    // A product per head in one launch (heads > 0; not with a plan): block z takes head z, whose
+    // A product per head in one launch (form PER_HEAD): block z takes head z, whose
     // columns of A start at z * head_a_cols, whose matrix is rows [z * w_rows, z * w_rows + N) of
     // W and whose results go to columns z * head_c_cols + [0, N) of C.  K is a head's K; what a
     // block of 64 columns of A holds beyond it meets columns of W outside its map, which read zero.
     int heads, head_a_cols, head_c_cols;
     // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2
     int act;
-    // a grouped product's A and its rows' stride (set by its entry point)
-    const void* a_rows;
-    int a_ld;
 };
 
 template <int BN, int STAGES, int MH>
@@ -116,14 +113,16 @@ struct SharedStorage {
     int abort_flag;
 };
 
-// NORM: what the product has to do with the norm around it, fixed when it is compiled so that
-// the other forms carry none of its code (an epilogue runs once per block, its instructions
-// come from memory, and a tenth more of them cost every product 0.4 us): NORM_NONE, NORM_PRE
-// (the rows of A are ahead of their norm, `sumsq_in`), NORM_EMIT (`gain`: leave the next
-// norm's input).
-enum NormForm { NORM_NONE = 0, NORM_PRE = 1, NORM_EMIT = 2 };
+// FORM: what the product has to do beyond itself, fixed when it is compiled so that the other
+// forms carry none of its code (an epilogue runs once per block, its instructions come from
+// memory, and a tenth more of them cost every product 0.4 us; a choice in the loop of the thread
+// that sends the copies costs it every round: with the grouped form's choices in all forms a
+// 2,048-token prompt of the 120M shape, 48 of these products, took 3.3 us more): NORM_PRE (the rows of A are ahead of
+// their norm, `sumsq_in`), NORM_EMIT (`gain`: leave the next norm's input), GROUPED (a plan says
+// which rows meet which matrix), PER_HEAD (a product per head).
+enum Form { NORM_NONE = 0, NORM_PRE = 1, NORM_EMIT = 2, GROUPED = 3, PER_HEAD = 4 };
 
-template <int BN, int STAGES, int EPI, int MH, int NORM>
+template <int BN, int STAGES, int EPI, int MH, int FORM>
 __global__ void __launch_bounds__(192, (STAGES <= 3 && MH == 1) ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_w,
@@ -140,9 +139,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     int m0 = blockIdx.y * BM * MH, M = M_all, w_row0 = 0;
     const int n_tile = blockIdx.x;
     // a product per head: this block's head moves the columns of A, the rows of W and the columns of C
-    const int head = na.heads > 0 ? (int)blockIdx.z : 0;
-    const int a_col0 = head * na.head_a_cols;
-    if (na.heads > 0) {
+    const int head = FORM == PER_HEAD ? (int)blockIdx.z : 0;
+    const int a_col0 = FORM == PER_HEAD ? head * na.head_a_cols : 0;
+    if (FORM == PER_HEAD) {
         w_row0 = head * na.w_rows;
         c_ptr = reinterpret_cast<uint8_t*>(c_ptr) +
                 (size_t)head * na.head_c_cols * ((EPI == STORE_F32 || EPI == ACCUM_F32) ? 4 : 2);
@@ -170,7 +169,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         tc::prefetch_tensormap(&map_a);
         tc::prefetch_tensormap(&map_w);
         if (tma_out) tc::prefetch_tensormap(&map_c);
-        if (NORM == NORM_EMIT && M > BM) tc::prefetch_tensormap(&map_s);
+        if (FORM == NORM_EMIT && M > BM) tc::prefetch_tensormap(&map_s);
     }
     if (warp == 1) {
         tc::tmem_alloc(&s.tmem_base, TMEM_COLS);
@@ -181,7 +180,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     tc::tc_fence_after_sync();
     const uint32_t tmem_acc = s.tmem_base;
     bool few_rows = false;              // grouped: the tile's rows of A are one box of 16
-    constexpr bool PRE = NORM == NORM_PRE;
+    constexpr bool PRE = FORM == NORM_PRE;
     auto load_w = [&](int kb, int st) {
         if (EPI == SWIGLU_BF16) {
             const int half = BN / 2;
@@ -196,7 +195,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     // now: W is a weight matrix, which no kernel of the stream writes, so these copies need
     // not wait for the kernels before this one; A is their output and does.
     // (not in a grouped product: which expert's W it is stands in the plan, which a kernel wrote)
-    const int w_ahead = na.plan != nullptr ? 0 : (k_blocks < STAGES ? k_blocks : STAGES);
+    const int w_ahead = FORM == GROUPED ? 0 : (k_blocks < STAGES ? k_blocks : STAGES);
     if (warp == 0 && lane == 0) {
         for (int kb = 0; kb < w_ahead; ++kb) {
             tc::mbar_expect_tx(&s.full_bar[kb], STAGE_BYTES);
@@ -205,7 +204,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     }
     cb_pdl_wait();
     cb_pdl_trigger();
-    if (na.plan != nullptr) {
+    if (FORM == GROUPED) {
         const int tile = blockIdx.y;
         const int* entry = na.plan + 2 + na.n_experts + tile;
         const bool in_use = tile < __ldg(na.plan);
@@ -218,12 +217,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         // two of 8 experts of 4,096 x 2,048 each: 38 -> 29 us; several small boxes for more rows were slower)
         few_rows = M - m0 <= 16;
     }
-    const uint32_t stage_bytes = few_rows ? (uint32_t)(BN + 16) * BK * 2 : STAGE_BYTES;
+    const uint32_t stage_bytes = FORM == GROUPED && few_rows ? (uint32_t)(BN + 16) * BK * 2 : STAGE_BYTES;
 
     // A norm after the product: the tile of C (32-column boxes in the 128-byte swizzle) comes
     // into its own piece of shared memory behind the stages, asked for by an epilogue thread
     // that has nothing else to do yet.  Only the block that runs the epilogue asks.
-    const bool emit = NORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && BN <= 128 && split == 0;
+    const bool emit = FORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && BN <= 128 && split == 0;
     uint8_t* const c_tile = reinterpret_cast<uint8_t*>(&s) + ((sizeof(Storage) + 1023) & ~(size_t)1023);
     if (emit && warp >= 2) {
         // (read in the epilogue, behind a barrier of these four warps)
@@ -256,7 +255,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     tc::mbar_expect_tx(&s.full_bar[st], stage_bytes);
                     load_w(kb, st);
                 }
-                if (MH == 1 && few_rows)
+                if (FORM == GROUPED && few_rows)
                     tc::tma_load_2d(s.a[st], &map_s, &s.full_bar[st], (kb_first + kb) * BK, m0);
                 else
 #pragma unroll
@@ -588,7 +587,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 const int n_out = EPI == SWIGLU_BF16 ? inter : N;
                 float ss4[4] = {0.f, 0.f, 0.f, 0.f};
                 uint8_t* const sbuf = ring + (BN / 32) * (BM * 128);     // behind the staged chunks of C
-                static_assert(NORM != NORM_EMIT || EPI != ACCUM_F32 || BN > 128 || MH > 1 ||
+                static_assert(FORM != NORM_EMIT || EPI != ACCUM_F32 || BN > 128 || MH > 1 ||
                                   (BN / 32) * (BM * 192) <= (int)(sizeof(s.a) + sizeof(s.b)),
                               "the staged chunks of C and of the scaled rows must fit in the ring of stages");
                 const bool direct = M <= BM;
@@ -614,7 +613,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                         tc::tmem_ld_32x32(lane_addr_h + c * 32, v);
                         // a norm after the product: the chunk's values of C and the gain come out
                         // of shared memory while the accumulators come out of tensor memory
-                        constexpr bool EMIT = NORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1;
+                        constexpr bool EMIT = FORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1;
                         const bool emit_chunk = EMIT && emit && n_tile * BN + c * 32 < N;
                         float4 o[EMIT ? 8 : 1], g[EMIT ? 8 : 1];
                         if (EMIT && emit_chunk) {
@@ -714,14 +713,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                             if (EPI == ACCUM_F32) tc::tma_reduce_add_2d(&map_c, buf, x, m0 + mh * BM);
                             else tc::tma_store_2d(&map_c, buf, x, m0 + mh * BM);
 
-                            if (NORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && emit && !direct)
+                            if (FORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && emit && !direct)
                                 tc::tma_store_2d(&map_s, sbuf + c * (BM * 64), x, m0);
                             tc::tma_store_commit();
                         }
                     }
                 }
                 }
-                if (NORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && emit && row < M)
+                if (FORM == NORM_EMIT && EPI == ACCUM_F32 && MH == 1 && emit && row < M)
                     na.sumsq_out[(size_t)n_tile * M + row] = (ss4[0] + ss4[1]) + (ss4[2] + ss4[3]);
                 if (warp == 2 && lane == 0) tc::tma_store_wait_all();
             } else if (EPI == SWIGLU_BF16) {
@@ -871,12 +870,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     }
 }
 
-template <int BN, int STAGES, int EPI, int MH, int NORM>
-int launch_norm(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc,
-                int inter, int k_splits, int* status, cudaStream_t stream, const RopeArgs& ra, const NormArgs& na) {
+template <int BN, int STAGES, int EPI, int MH, int FORM>
+int launch_form(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc,
+                int inter, int k_splits, int* status, cudaStream_t stream, const RopeArgs& ra, const NormArgs& na,
+                const CUtensorMap* few = nullptr) {
     if (MH > 1 && k_splits > 1) return CB_ERR_UNSUPPORTED;
-    const bool grouped = na.plan != nullptr;
-    if (grouped && (MH > 1 || k_splits > 1 || NORM != NORM_NONE || EPI == ROPE_APPEND || EPI == ACCUM_F32 ||
+    constexpr bool grouped = FORM == GROUPED, per_head = FORM == PER_HEAD;
+    if (grouped && (na.plan == nullptr || MH > 1 || k_splits > 1 || EPI == ROPE_APPEND || EPI == ACCUM_F32 ||
                     na.max_tiles <= 0 || na.w_rows <= 0))
         return CB_ERR_UNSUPPORTED;
     // a norm after the product: only the epilogue that has the summed rows in registers leaves it
@@ -904,10 +904,9 @@ int launch_norm(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
     int tma_out = ((uintptr_t)C & 15) == 0 && ((size_t)ldc * esize) % 16 == 0 &&
                   (f32 || (EPI == SWIGLU_BF16 ? BN % 128 == 0 : BN % 64 == 0));
     if (grouped) tma_out = 0;        // a tile's rows end where its expert's do: every thread stores its own row
-    const bool per_head = na.heads > 0;
     if (per_head) {
         // the heads' columns of C lie side by side: every thread stores its own row, 16 bytes at a time
-        if (grouped || MH > 1 || k_splits > 1 || NORM != NORM_NONE || (EPI != STORE_BF16 && EPI != STORE_F32) ||
+        if (na.heads <= 0 || MH > 1 || k_splits > 1 || (EPI != STORE_BF16 && EPI != STORE_F32) ||
             na.w_rows <= 0 || (na.head_a_cols & 7) || ((size_t)na.head_c_cols * esize) % 16 || na.heads > 65535)
             return CB_ERR_UNSUPPORTED;
         tma_out = 0;
@@ -919,13 +918,13 @@ int launch_norm(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
         tma_out = 0;
     if ((EPI == ROPE_APPEND || MH > 1 || emit) && !tma_out) return CB_ERR_UNSUPPORTED;
     CUtensorMap ms = ma;
-    if (grouped && !tc::make_map_2d(&ms, na.a_rows, (uint64_t)M, (uint64_t)K, (uint64_t)na.a_ld, 16)) return CB_ERR_UNSUPPORTED;
+    if (grouped) ms = *few;
     if (emit && !tc::make_plain_box_map_2d(&ms, na.scaled, (uint64_t)M, (uint64_t)N, (uint64_t)na.ld_scaled, 32, BM))
         return CB_ERR_UNSUPPORTED;
     const int smem = (int)(emit ? smem_emit : smem_plain);
     static int configured = 0;
     if (configured < smem) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI, MH, NORM>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI, MH, FORM>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = smem;
@@ -933,7 +932,7 @@ int launch_norm(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
     const int n_cols = EPI == SWIGLU_BF16 ? 2 * inter : N;
     dim3 grid((n_cols + BN - 1) / BN, grouped ? na.max_tiles : (M + BM * MH - 1) / (BM * MH),
               per_head ? na.heads : k_splits);
-    cb_launch_cluster(gemm_tcgen05_kernel<BN, STAGES, EPI, MH, NORM>, dim3(grid), dim3(192), smem, stream, k_splits,
+    cb_launch_cluster(gemm_tcgen05_kernel<BN, STAGES, EPI, MH, FORM>, dim3(grid), dim3(192), smem, stream, k_splits,
                       ma, mw, mc, ms, tma_out, C, M, N, K, ldc, inter, k_splits, status, ra, na);
     return cb_last_error();
 }
@@ -945,18 +944,18 @@ template <int BN, int STAGES, int EPI, int MH = 1>
 int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc,
            int inter, int k_splits, int* status, cudaStream_t stream, const RopeArgs& ra = RopeArgs{},
            const NormArgs& na = NormArgs{}) {
-    if (na.gain != nullptr && na.sumsq_in != nullptr) return CB_ERR_UNSUPPORTED;
+    if ((na.gain != nullptr && na.sumsq_in != nullptr) || na.plan != nullptr || na.heads > 0) return CB_ERR_UNSUPPORTED;
     if (na.sumsq_in != nullptr) {
         if constexpr (EPI == SWIGLU_BF16 || EPI == ROPE_APPEND)
-            return launch_norm<BN, STAGES, EPI, MH, NORM_PRE>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
+            return launch_form<BN, STAGES, EPI, MH, NORM_PRE>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
         return CB_ERR_UNSUPPORTED;
     }
     if (na.gain != nullptr) {
         if constexpr (EPI == ACCUM_F32 && BN <= 128 && MH == 1)
-            return launch_norm<BN, STAGES, EPI, MH, NORM_EMIT>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
+            return launch_form<BN, STAGES, EPI, MH, NORM_EMIT>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
         return CB_ERR_UNSUPPORTED;
     }
-    return launch_norm<BN, STAGES, EPI, MH, NORM_NONE>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
+    return launch_form<BN, STAGES, EPI, MH, NORM_NONE>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
 }
 
 template <int BN, int STAGES, int MH = 1>
@@ -970,6 +969,27 @@ int launch_epi(int epi, const CUtensorMap& ma, const CUtensorMap& mw, void* C, i
         case SWIGLU_BF16: return launch<BN, STAGES, SWIGLU_BF16, MH>(ma, mw, C, M, N, K, ldc, inter, ks, status, stream, none, na);
     }
     return CB_ERR_UNSUPPORTED;
+}
+
+template <int BN, int STAGES>
+int launch_grouped(int epi, const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc,
+                   int inter, int* status, cudaStream_t stream, const NormArgs& na, const CUtensorMap& few) {
+    const RopeArgs none{};
+    switch (epi) {
+        case STORE_BF16: return launch_form<BN, STAGES, STORE_BF16, 1, GROUPED>(ma, mw, C, M, N, K, ldc, inter, 1, status, stream, none, na, &few);
+        case STORE_F32: return launch_form<BN, STAGES, STORE_F32, 1, GROUPED>(ma, mw, C, M, N, K, ldc, inter, 1, status, stream, none, na, &few);
+        case SWIGLU_BF16: return launch_form<BN, STAGES, SWIGLU_BF16, 1, GROUPED>(ma, mw, C, M, N, K, ldc, inter, 1, status, stream, none, na, &few);
+    }
+    return CB_ERR_UNSUPPORTED;
+}
+
+template <int BN, int STAGES>
+int launch_heads(int epi, const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc,
+                 int* status, cudaStream_t stream, const NormArgs& na) {
+    const RopeArgs none{};
+    return epi == STORE_BF16
+               ? launch_form<BN, STAGES, STORE_BF16, 1, PER_HEAD>(ma, mw, C, M, N, K, ldc, 0, 1, status, stream, none, na)
+               : launch_form<BN, STAGES, STORE_F32, 1, PER_HEAD>(ma, mw, C, M, N, K, ldc, 0, 1, status, stream, none, na);
 }
 
 }  // namespace
@@ -1025,40 +1045,32 @@ CB_EXPORT int cb_gemm_tcgen05(const void* A, const void* W, void* C, int M, int 
 // expert, W [experts * w_rows, K] their matrices one below the other, and the plan on the device
 // says which rows are whose (NormArgs::plan and the fields after it, set by the caller in `norm`).
 // epi: STORE_BF16, STORE_F32 or SWIGLU_BF16 (N = the intermediate width, w_rows = 2 N).
-// bn: 64, 96, 128, 192 or 256 (the caller's `grouped_tile`).  Nothing of the plan is read on the host: a step replays as a graph.
+// bn: 128, 192 or 256; per_sm 2: 128 with two blocks to an SM (the caller's `grouped_tile`).  Nothing of the plan is read on the host: a step replays as a graph.
 CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int M, int N, int K, int lda,
                                       int ldw, int ldc, int epi, int bn, int per_sm, int* status, void* stream,
                                       const void* norm) {
     if (M <= 0 || N <= 0) return 0;
     if (norm == nullptr) return CB_ERR_UNSUPPORTED;
-    NormArgs na = *static_cast<const NormArgs*>(norm);
-    na.a_rows = A;
-    na.a_ld = lda;
+    const NormArgs na = *static_cast<const NormArgs*>(norm);
     if (na.plan == nullptr || na.n_experts <= 0 || na.gain != nullptr || na.sumsq_in != nullptr ||
         K <= 0 || (K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15))
         return CB_ERR_UNSUPPORTED;
     if (epi != STORE_BF16 && epi != STORE_F32 && epi != SWIGLU_BF16) return CB_ERR_UNSUPPORTED;
     const int box_rows = epi == SWIGLU_BF16 ? bn / 2 : bn;
-    CUtensorMap ma, mw;
-    if (!tc::make_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM)) return CB_ERR_UNSUPPORTED;
+    CUtensorMap ma, mw, few;                 // few: a box of 16 rows of A
+    if (!tc::make_map_2d(&ma, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM) ||
+        !tc::make_map_2d(&few, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 16))
+        return CB_ERR_UNSUPPORTED;
     if (!tc::make_map_2d(&mw, W, (uint64_t)na.n_experts * (uint64_t)na.w_rows, (uint64_t)K, (uint64_t)ldw, box_rows))
         return CB_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     const int inter = epi == SWIGLU_BF16 ? N : 0;
-    if (per_sm == 2) {
-        switch (bn) {
-            case 64: return launch_epi<64, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-            case 96: return launch_epi<96, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-            case 128: return launch_epi<128, 3>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-        }
-        return CB_ERR_UNSUPPORTED;
-    }
+    if (per_sm == 2)
+        return bn == 128 ? launch_grouped<128, 3>(epi, ma, mw, C, M, N, K, ldc, inter, status, s, na, few) : CB_ERR_UNSUPPORTED;
     switch (bn) {
-        case 64: return launch_epi<64, 6>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-        case 96: return launch_epi<96, 6>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-        case 128: return launch_epi<128, 5>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-        case 192: return launch_epi<192, 5>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
-        case 256: return launch_epi<256, 4>(epi, ma, mw, C, M, N, K, ldc, inter, 1, status, s, na);
+        case 128: return launch_grouped<128, 5>(epi, ma, mw, C, M, N, K, ldc, inter, status, s, na, few);
+        case 192: return launch_grouped<192, 5>(epi, ma, mw, C, M, N, K, ldc, inter, status, s, na, few);
+        case 256: return launch_grouped<256, 4>(epi, ma, mw, C, M, N, K, ldc, inter, status, s, na, few);
     }
     return CB_ERR_UNSUPPORTED;
 }
@@ -1081,9 +1093,9 @@ CB_EXPORT int cb_gemm_tcgen05_heads(const void* A, const void* W, void* C, int M
     if (!tc::make_map_2d(&mw, W, (uint64_t)heads * (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn)) return CB_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     switch (bn) {
-        case 64: return launch_epi<64, 6>(epi, ma, mw, C, M, N, K, ldc, 0, 1, status, s, na);
-        case 96: return launch_epi<96, 6>(epi, ma, mw, C, M, N, K, ldc, 0, 1, status, s, na);
-        case 128: return launch_epi<128, 5>(epi, ma, mw, C, M, N, K, ldc, 0, 1, status, s, na);
+        case 64: return launch_heads<64, 6>(epi, ma, mw, C, M, N, K, ldc, status, s, na);
+        case 96: return launch_heads<96, 6>(epi, ma, mw, C, M, N, K, ldc, status, s, na);
+        case 128: return launch_heads<128, 5>(epi, ma, mw, C, M, N, K, ldc, status, s, na);
     }
     return CB_ERR_UNSUPPORTED;
 }

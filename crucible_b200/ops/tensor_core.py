@@ -181,8 +181,7 @@ class _NormArgs(ctypes.Structure):
                 ("glu_limit", ctypes.c_float), ("glu_alpha", ctypes.c_float), ("glu_offset", ctypes.c_float),
                 ("plan", ctypes.c_void_p), ("n_experts", ctypes.c_int), ("max_tiles", ctypes.c_int),
                 ("w_rows", ctypes.c_int), ("heads", ctypes.c_int), ("head_a_cols", ctypes.c_int),
-                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int), ("a_rows", ctypes.c_void_p),
-                ("a_ld", ctypes.c_int)]
+                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int)]
 
 
 class NormEmit:

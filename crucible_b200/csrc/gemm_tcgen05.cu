@@ -95,9 +95,14 @@ struct NormArgs {
     // W and whose results go to columns z * head_c_cols + [0, N) of C.  K is a head's K; what a
     // block of 64 columns of A holds beyond it meets columns of W outside its map, which read zero.
     int heads, head_a_cols, head_c_cols;
-    // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2
+    // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2.  PER_HEAD, with `gate` set: the
+    // results times the sigmoids of their logits before they are rounded, of one logit a row and head
+    // (GATE_HEAD: fp32 [M][heads]) or of one a result (GATE_RESULT: bf16 [M][heads * N]).
     int act;
+    const void* gate;
+    int gate_ld;
 };
+constexpr int GATE_HEAD = 2, GATE_RESULT = 3;
 
 template <int BN, int STAGES, int MH>
 struct SharedStorage {
@@ -789,6 +794,32 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     }
                 }
             } else {
+                // 32 results of a head times the sigmoids of their logits
+                auto gate_chunk = [&](uint32_t (&r)[32], int at_row, int at_head, int col) {
+                    if (na.act == GATE_HEAD) {
+                        const float f = 1.0f / (1.0f + expf(-static_cast<const float*>(na.gate)[(size_t)at_row * na.gate_ld + at_head]));
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
+                        return;
+                    }
+                    const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(na.gate) + (size_t)at_row * na.gate_ld +
+                                             (size_t)at_head * N + col;
+                    const bool wide = col + 32 <= N && ((uintptr_t)g & 15) == 0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        __align__(16) __nv_bfloat16 z[8];
+                        if (wide) {
+                            *reinterpret_cast<uint4*>(z) = __ldg(reinterpret_cast<const uint4*>(g) + q);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) z[j] = col + 8 * q + j < N ? g[8 * q + j] : __nv_bfloat16();
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            r[8 * q + j] = __float_as_uint(__uint_as_float(r[8 * q + j]) *
+                                                           (1.0f / (1.0f + expf(-__bfloat162float(z[j])))));
+                    }
+                };
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     uint32_t r[32];
@@ -800,13 +831,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
                         for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * rf[0]);
                     }
-                    if (EPI == STORE_BF16 && na.act == 1) {
+                    if (EPI == STORE_BF16 && FORM != PER_HEAD && na.act == 1) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float z = fmaxf(__uint_as_float(r[j]), 0.f);
                             r[j] = __float_as_uint(z * z);
                         }
                     }
+                    if (EPI == STORE_BF16 && FORM == PER_HEAD && na.gate != nullptr) gate_chunk(r, row, head, col0);
                     const bool full = col0 + 32 <= N;
                     if (EPI == STORE_BF16) {
                         __nv_bfloat16* dst = (__nv_bfloat16*)c_ptr + (size_t)row * ldc + col0;
@@ -1078,16 +1110,21 @@ CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int
 // A product per head in one launch: A [M, a_cols] holds head h's K columns from h * head_a_cols,
 // W [heads * N, K] the heads' matrices one below the other, and head h's results go to columns
 // h * head_c_cols + [0, N) of C (bf16 or fp32 by epi: STORE_BF16 or STORE_F32).  bn: 64, 96 or 128.
+// gate (STORE_BF16 alone; null: none) as in NormArgs, of the kind GATE_HEAD or GATE_RESULT.
 CB_EXPORT int cb_gemm_tcgen05_heads(const void* A, const void* W, void* C, int M, int N, int K, int a_cols,
                                     int lda, int ldw, int ldc, int heads, int head_a_cols, int head_c_cols,
-                                    int epi, int bn, int* status, void* stream) {
+                                    int epi, int bn, const void* gate, int gate_ld, int gate_kind, int* status,
+                                    void* stream) {
     if (M <= 0 || N <= 0 || heads <= 0) return 0;
+    if (gate != nullptr && (epi != STORE_BF16 || (gate_kind != GATE_HEAD && gate_kind != GATE_RESULT)))
+        return CB_ERR_UNSUPPORTED;
     if (K <= 0 || (K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) ||
         ((uintptr_t)C & 15) || a_cols < (heads - 1) * head_a_cols + K)
         return CB_ERR_UNSUPPORTED;
     if (epi != STORE_BF16 && epi != STORE_F32) return CB_ERR_UNSUPPORTED;
     NormArgs na{};
     na.heads = heads; na.head_a_cols = head_a_cols; na.head_c_cols = head_c_cols; na.w_rows = N;
+    na.gate = gate; na.gate_ld = gate_ld; na.act = gate != nullptr ? gate_kind : 0;
     CUtensorMap ma, mw;
     if (!tc::make_map_2d(&ma, A, (uint64_t)M, (uint64_t)a_cols, (uint64_t)lda, BM)) return CB_ERR_UNSUPPORTED;
     if (!tc::make_map_2d(&mw, W, (uint64_t)heads * (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn)) return CB_ERR_UNSUPPORTED;

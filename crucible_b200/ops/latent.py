@@ -77,8 +77,9 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
     ways: 8 rows 47 us with the tiles, 53 with the warps; 16 rows 51 and 68; 24 rows 66, and 140 as
     a product per head; one row 45 and 45 with a launch less for the gate.
     `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), in the same
-    launch for few rows, by `head_gate` otherwise.  `gate_rows` (rows of the activations' dtype,
-    [rows, heads * N]): every result times the sigmoid of its own logit, likewise."""
+    launch and before they are rounded where there is one for all heads, by `head_gate` otherwise.
+    `gate_rows` (rows of the activations' dtype, [rows, heads * N]): every result times the sigmoid
+    of its own logit, likewise."""
     from . import linear
     heads, n, k = w.shape
     if gate_rows is not None and (out_head != n or gate_rows.shape != (a.shape[0], heads * n)
@@ -86,8 +87,16 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
         raise KernelError("heads_linear: gate rows are [rows, heads * N] of the results' dtype")
     from . import is_weight, tensor_core
     rows = a.shape[0]
+    # the gate that the tiles take with them: of one kind, its logits side by side
+    gate = gate_logit if gate_rows is None else gate_rows if gate_logit is None else None
+    if gate is not None and (out.dtype != torch.bfloat16 or out_head != n or out.shape[1] != heads * n
+                             or not gate.is_cuda or gate.stride(1) != 1
+                             or (gate_rows is None and (gate.dtype != torch.float32 or gate.shape != (rows, heads)))):
+        gate = None
     done = (HEADS_IN_ONE_LAUNCH and a.dtype == torch.bfloat16 and rows > WARP_ROWS and is_weight(w)
-            and tensor_core.heads_linear(a, a_head, w, out, out_head))
+            and tensor_core.heads_linear(a, a_head, w, out, out_head, gate))
+    if done and gate is not None:
+        return
     if not done and a.dtype == torch.bfloat16 and rows <= SMALL_ROWS:
         _need_cuda(a, w, out, gate_rows)
         if a.stride(1) != 1 or out.stride(1) != 1 or not w.is_contiguous() or out.dtype != a.dtype:

@@ -181,7 +181,8 @@ class _NormArgs(ctypes.Structure):
                 ("glu_limit", ctypes.c_float), ("glu_alpha", ctypes.c_float), ("glu_offset", ctypes.c_float),
                 ("plan", ctypes.c_void_p), ("n_experts", ctypes.c_int), ("max_tiles", ctypes.c_int),
                 ("w_rows", ctypes.c_int), ("heads", ctypes.c_int), ("head_a_cols", ctypes.c_int),
-                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int)]
+                ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int), ("gate", ctypes.c_void_p),
+                ("gate_ld", ctypes.c_int)]
 
 
 class NormEmit:
@@ -398,11 +399,15 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
 
 
 
-def heads_linear(a, a_head: int, w, out, out_head: int) -> bool:
+GATE_HEAD, GATE_RESULT = 2, 3
+
+
+def heads_linear(a, a_head: int, w, out, out_head: int, gate=None) -> bool:
     """out[t, h * out_head + n] = sum_k a[t, h * a_head + k] * w[h, n, k] for every head of `w`
     [heads, N, K] (a declared bfloat16 weight) in ONE launch (`cb_gemm_tcgen05_heads`: the head is
-    the grid's third axis).  Refuses what the tiles cannot take (the caller then runs a product
-    per head)."""
+    the grid's third axis).  `gate` (bfloat16 results alone): float32 logits [rows, heads] or bfloat16 ones
+    [rows, heads * N] whose sigmoids the results are multiplied by before they are rounded.  Refuses
+    what the tiles cannot take (the caller then runs a product per head)."""
     heads, n, k = w.shape
     if (a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not w.is_contiguous() or not a.is_cuda
             or a.stride(1) != 1 or out.stride(1) != 1 or out.dtype not in (torch.bfloat16, torch.float32)
@@ -418,6 +423,8 @@ def heads_linear(a, a_head: int, w, out, out_head: int) -> bool:
         _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()), _c_int(a.shape[0]),
         _c_int(n), _c_int(k), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(1)),
         _c_int(out.stride(0)), _c_int(heads), _c_int(a_head), _c_int(out_head), _c_int(epi), _c_int(bn),
+        _c_void_p(gate.data_ptr() if gate is not None else 0), _c_int(gate.stride(0) if gate is not None else 0),
+        _c_int(GATE_HEAD if gate is not None and gate.dtype == torch.float32 else GATE_RESULT),
         _c_void_p(status_word(a.device).data_ptr()), _stream())
     if code == _UNSUPPORTED:
         return False

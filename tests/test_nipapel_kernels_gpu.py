@@ -450,6 +450,34 @@ def test_heads_products_of_many_rows_are_one_launch(rows, heads, a_head, k, n, o
         assert torch.all(got[..., n:] == 7.0)
 
 
+@pytest.mark.parametrize("rows", [1, 2, 3, 16, 17, 130])
+@pytest.mark.parametrize("heads,n,k", [(3, 64, 40), (2, 104, 192), (8, 128, 192)])
+@pytest.mark.parametrize("per_head", [True, False])
+def test_heads_gates_count_before_the_rounding(rows, heads, n, k, per_head):
+    """A gate on the heads' products, of one logit a head or one a result: the results are those of float64
+    rounded to bfloat16 once.  (Sums of float32 leave one in a few hundred on the other side of a
+    rounding; products rounded before the gate and after differ in every fourth.)"""
+    from crucible_b200 import ops
+    from crucible_b200.ops import latent
+    g = torch.Generator().manual_seed(rows + n)
+    a = torch.randn(rows, heads * k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(heads, n, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+    wd = w.to(DEV).contiguous()
+    ops.declare_weights(wd)
+    kind, width = (torch.float32, heads) if per_head else (torch.bfloat16, heads * n)
+    at = 8 if rows % 2 else 4                           # columns of a wider projection, on 16-byte boundaries or off them
+    logit = torch.randn(rows, width + 8, generator=g).to(kind)[:, at:at + width]
+    out = torch.full((rows, heads * n), float("nan"), device=DEV, dtype=torch.bfloat16)
+    on = torch.empty(rows, width + 8, dtype=kind, device=DEV)[:, at:at + width].copy_(logit)
+    latent.heads_linear(a.to(DEV), k, wd, out, n, **({"gate_logit": on} if per_head else {"gate_rows": on}))
+    want = torch.einsum("thk,hnk->thn", a.double().view(rows, heads, k), w.double())
+    gate = torch.sigmoid(logit.double())
+    want = want * (gate[:, :, None] if per_head else gate.view(rows, heads, n))
+    want = want.reshape(rows, -1).to(torch.bfloat16)
+    assert rel(out, want) < 4.1e-3                      # one rounding of bfloat16 at the most
+    assert float((out.cpu() != want).double().mean()) < 0.02
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("window,keep", [(70, 5), (40, 130), (200, 0)])
 def test_unequal_portions_of_several_requests_in_one_step(D, window, keep, monkeypatch):

@@ -264,8 +264,10 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
                 }
             }
             const float before = __shfl_up_sync(0xffffffffu, i, 1);
-            dec = lane == 0 ? 0.f : expf(f_own + before - i);
-            b = in ? expf(i_own - i) : 0.f;
+            // (a log gate of -inf lets nothing in; until one does, the maximum is -inf and both are 0)
+            const float top = i == -INFINITY ? 0.f : i;
+            dec = lane == 0 ? 0.f : expf(f_own + before - top);
+            b = in ? expf(i_own - top) : 0.f;
             if (in) a.ws[own_at] = make_float4(f, 0.f, i, 0.f);
         } else {
             if (!VECTOR && in) dec = a.sc0[at];

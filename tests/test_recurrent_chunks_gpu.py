@@ -207,6 +207,30 @@ def test_a_later_token_does_not_reach_an_earlier_one(rule, monkeypatch):
     assert bool(torch.isnan(outs[1][at]).any())
 
 
+@pytest.mark.parametrize("closed", [(0, 1), (0, 40), (0, 64), (31, 33), (60, 61), (0, 70)])
+def test_input_gates_that_are_shut(closed, monkeypatch):
+    """Log input gates of -inf, from a portion's beginning on, over whole chunks, or throughout: such tokens add
+    nothing, as in the walk."""
+    from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda *a: True)
+    H, D, T, g = 2, 64, 70, torch.Generator().manual_seed(7)
+    q, kk, v, w, sc0, sc1, _ = _operands(k.MLSTM, k, T, H, H, D, D, g)
+    sc1[closed[0]:closed[1]] = float("-inf")
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, kk, v)], 1).contiguous().to(DEV)
+    before = torch.randn(1, H * D * D + H * D + 4, generator=g) * 0.3
+    results = []
+    for chunks in (True, False):
+        ctx, _, _ = _ctx((T,), torch.bfloat16)
+        state, out = before.to(DEV).clone().view(torch.uint8), torch.full((T, H * D), float("nan"), device=DEV)
+        monkeypatch.setattr(k, "CHUNKS", chunks)
+        k.matrix_memory(k.MLSTM, qkv, 0, H * D, 2 * H * D, sc0.contiguous().to(DEV), sc1.contiguous().to(DEV), ctx, state, 0,
+                        4 * H * D * D, 4 * (H * D * D + H * D), out, H, H, D, D)
+        results.append((out, state.view(torch.float32)))
+    for got, want in zip(*results):
+        assert bool(torch.isfinite(want).all()) and bool(torch.isfinite(got).all())
+        assert float((got - want).norm() / want.norm()) < 1e-5      # float32 sums of up to 70 tokens in another order
+
+
 @pytest.mark.parametrize("lengths", [(70, 33), (1, 1, 1), (1, 70)])
 def test_rows_off_the_wide_loads_boundaries_are_walked(lengths, monkeypatch):
     """Outputs that start on no 16-byte boundary: the chunks refuse them, and the walk's bits are the answer."""

@@ -288,10 +288,12 @@ template <int DP, int QR>
 int launch(const Params& p, int n_requests, int max_new, cudaStream_t s) {
     constexpr size_t bytes = SMEM_FLOATS<DP, QR> * sizeof(float);
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
-    if (bytes > 48 * 1024) {
+    static bool configured = false;
+    if (!configured && bytes > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<DP, QR>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return (int)e;
+        configured = true;
     }
     const dim3 grid((max_new * p.n_rep + QR - 1) / QR, p.n_kv_heads, n_requests);
     cb_launch(attention_f32_kernel<DP, QR>, grid, dim3(THREADS), bytes, s, p);

@@ -948,9 +948,13 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     }
 }
 
+// (`configured`: a kernel's own, so that only its first launch asks)
 template <typename K>
-int allow_smem(K kernel, size_t smem) {
-    return smem > 48 * 1024 ? (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : 0;
+int allow_smem(K kernel, size_t smem, bool& configured) {
+    if (configured || smem <= 48 * 1024) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    configured = e == cudaSuccess;
+    return (int)e;
 }
 
 template <int DP, int RULE, int ET>
@@ -959,7 +963,8 @@ int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
     constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + CT * ET + DP + 8 * CT
                                               + 2 * ((ROWS + CT) * P + CT * ET));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
-    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes);
+    static bool configured = false;
+    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes, configured);
     if (rc) return rc;
     const dim3 grid(n_requests, a.H, (a.E + ET - 1) / ET);
     cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS), bytes, s, a);
@@ -975,7 +980,8 @@ int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
     constexpr size_t bytes = sizeof(float) * ((VECTOR_DECAY<RULE> ? 3 : 2) * CT * P + 2 * CT * AP + 3 * CT
                                               + (part > values ? part : values));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
-    int rc = allow_smem(chunk_local_kernel<DP, RULE>, bytes);
+    static bool configured = false;
+    int rc = allow_smem(chunk_local_kernel<DP, RULE>, bytes, configured);
     if (rc) return rc;
     const dim3 grid((max_new + CT - 1) / CT, a.H, n_requests);
     cb_launch(chunk_local_kernel<DP, RULE>, grid, dim3(THREADS), bytes, s, a);

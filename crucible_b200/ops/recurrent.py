@@ -193,15 +193,17 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         raise KernelError("matrix_memory takes prepared float32 rows")
     sp, stride = _state_args(state)
     n, walked = ctx.n_requests, ctx.n_requests
+    # (without the host's counts of the step, or in 32 bits: the walk alone)
+    host = getattr(ctx, "host", None) if getattr(ctx, "dtype", None) == torch.bfloat16 else None
     starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
     w_off_read = w_off if rule in (WKV, CHANNEL) else 0
-    if (CHUNKS and getattr(ctx, "dtype", None) == torch.bfloat16 and chunks_pay(
-                rule, qkv.shape[0] - ctx.host.lead_single, n - ctx.host.lead_single, ctx.host.max_new_tokens, n_heads)
+    if (CHUNKS and host is not None and chunks_pay(
+                rule, qkv.shape[0] - host.lead_single, n - host.lead_single, host.max_new_tokens, n_heads)
             and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0
             and (s_off | state.stride(0) | qkv.data_ptr() | out.data_ptr() | state.data_ptr()) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked
-        walked = ctx.host.lead_single
-        longest, f32 = ctx.host.max_new_tokens, torch.float32
+        walked = host.lead_single
+        longest, f32 = host.max_new_tokens, torch.float32
         delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
         # bytes a row and a chunk take in the workspaces, and the tokens of each request that go at a time
         row_bytes = 4 * n_heads * (key_dim * ((delta or vector) + delta + (rule == CHANNEL)) + value_dim * delta + 4)
@@ -238,7 +240,7 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         return
     lib = build.load("recurrent")
     # decoded tokens of the bfloat16 engine: a token each, S read and written once
-    step = (STEP and getattr(ctx, "dtype", None) == torch.bfloat16 and ctx.host.lead_single >= walked
+    step = (STEP and host is not None and host.lead_single >= walked
             and (qkv.shape[1] | v_off | value_dim) % 4 == 0 and (s_off | state.stride(0)) % 16 == 0)
     args = (_c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
             _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,

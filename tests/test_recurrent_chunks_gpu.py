@@ -274,3 +274,25 @@ def test_mlstm_rows_off_the_wide_boundaries(dtype, rows_off, out_off):
         assert bool(torch.isnan(qkv[b + T * C:]).all())
         results.append((qkv[b:b + T * C].cpu(), keep.cpu(), into.cpu()))
     assert all(torch.equal(x, y) for x, y in zip(*results))
+
+
+@pytest.mark.parametrize("host", [None, "none given"])
+def test_a_step_without_the_hosts_counts_is_walked(host):
+    """A bfloat16 step's context that does not say what its requests bring."""
+    from crucible_b200.ops import recurrent as k
+    H, D, lengths, g = 2, 64, (300, 1), torch.Generator().manual_seed(4)
+    T = sum(lengths)
+    q, kk, v, w, sc0, sc1, _ = _operands(k.DELTA, k, T, H, H, D, D, g)
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, kk, v)], 1).contiguous().to(DEV)
+    results = []
+    for dtype in (torch.bfloat16, torch.float32):
+        ctx, _, _ = _ctx(lengths, dtype)
+        if dtype == torch.bfloat16:
+            del ctx.host
+            if host is None:
+                ctx.host = None
+        state, out = torch.zeros(2, 4 * H * D * D, dtype=torch.uint8, device=DEV), torch.empty(T, H * D, device=DEV)
+        k.matrix_memory(k.DELTA, qkv, 0, H * D, 2 * H * D, sc0.contiguous().to(DEV), sc1.contiguous().to(DEV), ctx, state, 0, 0,
+                        0, out, H, H, D, D)
+        results.append((out, state))
+    assert all(torch.equal(x, y) for x, y in zip(*results))

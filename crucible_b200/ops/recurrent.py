@@ -16,19 +16,28 @@ CHUNKS = True                # tests switch it off to reach the token-by-token w
 STEP = True                  # likewise, for the form of a token each
 
 
-def chunks_pay(rule, rows: int, requests: int, longest: int, heads: int) -> bool:
+# us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128) and of the chunks
+# (their launches, a token of the longest portion, a chunk and head of 128), fitted to both forms over 4 to 32 heads of 64
+# and 128 and 1 to 24 uneven portions of up to 40 to 500 tokens; the delta rules' chunks are walked in order, the
+# others' are not
+_DELTA_COSTS = ((2.8, 0.160, 0.0061), (13.3, 0.024, 0.217))
+COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS, MLSTM: ((3.1, 0.202, 0.0067), (23.3, 0.0, 0.148)),
+         WKV: ((3.0, 0.131, 0.0057), (21.2, 0.0, 0.131)), SSD: ((3.5, 0.130, 0.0043), (22.0, 0.0, 0.131))}
+
+
+def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bool:
     """Whether a bfloat16 step's portions (`rows` tokens of `requests`, without the single tokens at the
-    step's head; the longest) go in chunks.  The walk takes 0.2 to 0.28 us a token of the longest portion, or of
-    the whole where the requests fill the GPU; chunks take 18 us (delta rules) or 35 (the others) and then far
-    less a token, but a chunk that holds few tokens costs what a full one does.  Measured on 16 heads of
-    128: delta rules 64 tokens 22 us in chunks and 19 walked, 96: 24 and 26; 16 requests of up to 128: 221 and
-    182, 5: 76 and 81.  The others: 128 tokens 35 to 39 and 29 to 40, 512: 48 and 105 to 150; 16 requests of up
-    to 64: 88 to 105 and 93 to 136, of up to 30: 52 to 65 and 42 to 56."""
+    step's head; the longest; `heads` of 128 key channels) go in chunks.  The walk takes its time a token of the
+    longest portion until the requests fill the GPU, then a time a token; a chunk that holds few tokens
+    costs what a full one does, and every portion ends in one such.  Over the sizes that the costs were fitted to the
+    choice is 0.5 % (delta rules), 0.7 (mLSTM), 1.1 (state space) and 1.4 (wkv) from the better form on average.  16 heads of 128, chunks and
+    walk: delta rule 1 portion of 110 tokens 27 and 30 us, 24 of up to 300 514 and 450; state space
+    1 of 140 35 and 31, of 500 45 and 103; 24 of up to 60 101 and 90."""
     if requests <= 0:
         return False
-    if rule in (DELTA, CHANNEL):
-        return rows >= 96 * requests
-    return longest >= 160 or (longest >= 48 and rows >= 24 * requests and rows * heads >= 4096)
+    (start, token, work), (first, step, chunk) = COSTS[rule]
+    walk = start + token * longest + work * rows * heads
+    return walk > 1.05 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads)
 
 
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces
@@ -198,7 +207,7 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
     w_off_read = w_off if rule in (WKV, CHANNEL) else 0
     if (CHUNKS and host is not None and chunks_pay(
-                rule, qkv.shape[0] - host.lead_single, n - host.lead_single, host.max_new_tokens, n_heads)
+                rule, qkv.shape[0] - host.lead_single, n - host.lead_single, host.max_new_tokens, n_heads * key_dim / 128)
             and key_dim <= 128 and (qkv.shape[1] | q_off | k_off | v_off | key_dim | value_dim | w_off_read) % 4 == 0
             and (s_off | state.stride(0) | qkv.data_ptr() | out.data_ptr() | state.data_ptr()) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked

@@ -67,6 +67,7 @@ struct TcAttnParams {
     const int* block_table;
     int table_stride;
     int n_heads, n_kv_heads, n_rep, n_requests, page_tokens, page_shift;
+    int lead, lead_ranks;    // requests at the head of a single token each, and the tile ranks they take
     float scale_log2;
     int window;
     int keep_first;          // with a window: keys before this position stay visible to every later row
@@ -198,8 +199,23 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // grid (heads, requests, tile ranks), the tile rank slowest: blocks start in order of
     // weight over the whole launch, the longest rows first (and no thread divides by a run-time
-    // value to find its place: that costs about a hundred cycles each time)
-    const int kv_head = blockIdx.x, req = blockIdx.y, rank = blockIdx.z;
+    // value to find its place: that costs about a hundred cycles each time).  Single tokens at the
+    // head of the step have a tile each and lie in ranks of their own ahead of the portions': a
+    // block without work is not free, it waits for the SM's shared memory like another (48 tokens
+    // beside a portion of 2,048, 16 heads of 64 on 4, a window of 512, with a rank of the
+    // portion's 64 for each of them: 12,288 blocks without work, the layer 270 us, 125 now).
+    const int kv_head = blockIdx.x;
+    int req = blockIdx.y, rank = blockIdx.z;
+    if (p.lead > 0) {
+        if (rank < p.lead_ranks) {
+            req += rank * (int)gridDim.y;
+            rank = 0;
+            if (req >= p.lead) return;
+        } else {
+            req += p.lead;
+            rank -= p.lead_ranks;
+        }
+    }
     volatile int* abort_flag = &s.abort_flag;
 
     if (threadIdx.x == 0) {
@@ -805,6 +821,7 @@ int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap& mk, const
 // both are the same rows.
 // keep_first (with a window): a row at position p reads j <= p with p - j < window or j < keep_first.
 // chunked: `window` is a chunk's size (first_key).  sinks: [n_heads] or null.  Results times out_scale.
+// lead: how many requests at the head bring a single token (as max_new_tokens is the others').
 // gate: null, or logits: results times their sigmoids; laid out like `out`, rows of 16-byte pieces, or with
 // gate_per_head [rows][n_heads].
 CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* out, int out_stride,
@@ -814,7 +831,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
                                         int max_new_tokens, int n_heads, int n_kv_heads, int head_dim,
                                         int page_tokens, float scale, int window, int chunked, int keep_first,
                                         float out_scale, const float* sinks, const void* gate, int gate_stride,
-                                        int gate_per_head, int lean, int* status, void* stream) {
+                                        int gate_per_head, int lead, int lean, int* status, void* stream) {
     if (n_requests <= 0 || max_new_tokens <= 0) return 0;
     if (keep_first < 0 || !(scale > 0.f)) return CB_ERR_UNSUPPORTED;
     if ((head_dim != 64 && head_dim != 128 && !(head_dim == 256 && k_cache == v_cache)) || n_heads % n_kv_heads != 0 || page_tokens < 8 || page_tokens > KEYS ||
@@ -863,7 +880,12 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     const int n_rep = n_heads / n_kv_heads;
     const int q_tiles = (max_new_tokens * n_rep + ROWS - 1) / ROWS;
     if (n_requests > 65535 || q_tiles > 65535) return CB_ERR_UNSUPPORTED;
-    const dim3 grid(n_kv_heads, n_requests, q_tiles);
+    // (single tokens of more than a tile of query heads keep ranks like a portion's)
+    p.lead = lead > 0 && lead < n_requests && n_rep <= ROWS ? lead : 0;
+    const int portions = n_requests - p.lead;
+    p.lead_ranks = (p.lead + portions - 1) / portions;
+    if (p.lead_ranks + q_tiles > 65535) return CB_ERR_UNSUPPORTED;
+    const dim3 grid(n_kv_heads, portions, p.lead_ranks + q_tiles);
     // lean: -1 lets the launch decide, 0 and 1 fix the form.  Since the roomy form has two
     // softmax groups it is the quicker one also for launches with more blocks than places
     // (measured on B200: 2,048 tokens at the Llama-3.2-1B layer sizes, 512 blocks, 4.63 against
@@ -887,6 +909,6 @@ CB_EXPORT int cb_attention_tcgen05(const void* qkv, int qkv_stride, void* out, i
                                    void* stream) {
     return cb_attention_tcgen05_kept(qkv, qkv_stride, out, out_stride, k_cache, v_cache, n_pages, req_row_start,
                                      req_first_pos, block_table, table_stride, n_requests, max_new_tokens, n_heads,
-                                     n_kv_heads, head_dim, page_tokens, scale, window, 0, 0, 1.0f, nullptr, nullptr, 0, 0, lean,
+                                     n_kv_heads, head_dim, page_tokens, scale, window, 0, 0, 1.0f, nullptr, nullptr, 0, 0, 0, lean,
                                      status, stream);
 }

@@ -520,12 +520,13 @@ def _tcgen05_rows(head_dim, k_cache, v_cache) -> bool:
 
 def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale,
                        window, cache, keep_first: int = 0, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                       gate=None, gate_per_head: bool = False) -> bool:
+                       gate=None, gate_per_head: bool = False, lead: int = 0) -> bool:
     """tcgen05 attention for portions of prompts: head sizes of `_tcgen05_rows`, page size a
     power of two from 8 to 128.  `keep_first` (with a window): keys before that position stay
     visible.  `chunked`: the window is a chunk's size.  `sinks`: float32 per query head or None.
     `gate`: rows laid out like `out` (`gate_per_head`: one logit a head) whose sigmoids the results are
-    multiplied by before they are rounded, or None.  Returns False for anything else."""
+    multiplied by before they are rounded, or None.  `lead`: how many requests at the head of `reqs` bring a
+    single token.  Returns False for anything else."""
     pt = cache.page_tokens
     if pt < 8 or pt > 128 or pt & (pt - 1):
         return False
@@ -540,7 +541,7 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         ctypes.c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first if window else 0),
         ctypes.c_float(out_scale), _c_void_p(sinks.data_ptr() if sinks is not None else 0),
         _c_void_p(gate.data_ptr() if gate is not None else 0), _c_int(gate.stride(0) if gate is not None else 0),
-        _c_int(1 if gate_per_head else 0), _c_int(ATTENTION_LEAN), _c_void_p(status_word(qkv.device).data_ptr()), _stream())
+        _c_int(1 if gate_per_head else 0), _c_int(lead), _c_int(ATTENTION_LEAN), _c_void_p(status_word(qkv.device).data_ptr()), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -684,7 +685,7 @@ def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, sc
     reqs = _Requests(ctx, table, first, none - first, host.max_new_tokens, host.context_bucket, ctx.n_tokens)
     taken = _attention_tcgen05(q, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, cache,
                                keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate,
-                               gate_per_head=gate_per_head)
+                               gate_per_head=gate_per_head, lead=host.lead_single if first == 0 else 0)
     return first if taken else none
 
 

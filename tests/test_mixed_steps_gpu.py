@@ -65,6 +65,45 @@ def test_decoded_tokens_beside_a_portion(H, G, D, window, keep, chunked, gate, s
     assert err < 1.5e-2                                        # both round P and the result to bfloat16 (2^-8)
 
 
+@pytest.mark.parametrize("H,G,D", [(8, 2, 128), (4, 4, 64), (16, 1, 256), (144, 1, 64)])      # (the last: two tiles a token)
+@pytest.mark.parametrize("singles,portions", [(1, [200, 65, 70]), (3, [130, 70, 65]), (7, [64, 300, 65]), (20, [400])])
+def test_tokens_beside_several_portions_have_a_tile_each(H, G, D, singles, portions):
+    """Fewer, as many and more single tokens than portions: every one of the step's rows is written, with
+    the values of the CUDA-core kernel."""
+    from crucible_b200.engine.context import HostStep
+    from crucible_b200.ops import sink_attention
+    g, page = torch.Generator().manual_seed(H + singles), 16
+    counts = [1] * singles + portions
+    held = [(37 * i) % 150 for i in range(singles)] + [0, 41, 130][:len(portions)]
+    R, T, contexts = len(counts), sum(counts), [c + h for c, h in zip(counts, held)]
+    per = -(-max(contexts) // page)
+    table = torch.randperm(R * per, generator=g).to(torch.int32).view(R, per).to(DEV)
+    k = torch.randn(R * per, G, page, D, generator=g).to(torch.bfloat16).to(DEV)
+    v = k if D == 256 else torch.randn(k.shape, generator=g).to(torch.bfloat16).to(DEV)
+    cache = SimpleNamespace(keys=lambda s: k, values=lambda s: v, page_tokens=page)
+    starts = [0]
+    for n in counts:
+        starts.append(starts[-1] + n)
+    ctx = SimpleNamespace(n_requests=R, n_tokens=T, req_row_start=_i32(starts), req_first_pos=_i32(held),
+                          positions=_i32([h + i for h, n in zip(held, counts) for i in range(n)]),
+                          row_request=_i32([r for r, n in enumerate(counts) for _ in range(n)]),
+                          block_table=lambda group: table, host=HostStep(list(range(R)), counts, held, contexts, list(range(R))))
+    assert ctx.host.lead_single == singles
+    q = torch.randn(T, H * D, generator=g).to(torch.bfloat16).to(DEV)
+    outs = []
+    for use in (True, False):
+        sink_attention.TENSOR_CORES = use
+        try:
+            out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+            sink_attention.attention(q, None, out, None, H, G, D, D, D ** -0.5, None, 0, 1.0, ctx, cache,
+                                     SimpleNamespace(slot=0, group=0))
+        finally:
+            sink_attention.TENSOR_CORES = True
+        outs.append(out.float())
+    err = float((outs[0] - outs[1]).abs().max() / outs[1].abs().max())
+    assert err < 1.5e-2                                        # both round P and the result to bfloat16 (2^-8)
+
+
 @pytest.mark.parametrize("counts,held,window,keep,ordered", [
     ([64, 65], [0, 0], None, 0, True),              # one and two tiles of keys: a group without any, a tile each
     ([300], [85], None, 0, False),                  # three, scattered pages

@@ -18,6 +18,7 @@
 // Sizes: key and value sizes up to 256 that are multiples of 4, rows of whole 16-byte pieces, any page
 // size; window, chunks, kept first tokens, a sink, a gate, an output scale as in sink_attention.cu.
 #define CB_PDL_BIT 8      // this file's bit in CRUCIBLE_PDL (shared with attention_generic.cu)
+#include <type_traits>
 #include "common.cuh"
 
 namespace {
@@ -115,18 +116,17 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     }
     // the block's keys: tiles of the kept first tokens, then from the first row's first key on
     const int last_pos = first_pos + min(n_rows - 1, r0 + QR - 1) / p.n_rep;
-    const int key_lo = low(first_pos + r0 / p.n_rep) / KT * KT;
+    const int first_key = low(first_pos + r0 / p.n_rep), key_lo = first_key / KT * KT;
     const int kept_tiles = p.window > 0 ? min((p.keep_first + KT - 1) / KT, key_lo / KT) : 0;
     const int n_tiles = kept_tiles + (last_pos - key_lo) / KT + 1;
     auto tile_key0 = [&](int j) { return j < kept_tiles ? j * KT : key_lo + (j - kept_tiles) * KT; };
-    // a tile's rows of K or V; keys beyond the block's last position, and those of a page that was given
-    // back early (a tile may begin before the window does), are zeros and not read: no row sees them
-    auto fetch = [&](int j, const float* cache, int n, float* to) {
-        const int key0 = tile_key0(j);
+    // a tile's rows of K or V; keys that none of the block's rows sees (behind its last position, ahead of
+    // its windows) are zeros and not read: their page may have been given back
+    auto fetch_keys = [&](int key0, const float* cache, int n, float* to, auto all_seen) {
         for (int i = tid; i < KT * (DP / 4); i += THREADS) {
             const int t = i / (DP / 4), d = (i % (DP / 4)) * 4, key = key0 + t;
-            const int page = key <= last_pos && d < n ? table[key / p.page_tokens] : -1;
-            if (page >= 0) {
+            if (key <= last_pos && d < n && (decltype(all_seen)::value || key >= first_key || key < p.keep_first)) {
+                const int page = table[key / p.page_tokens];
                 cp16(to + t * P + d,
                      cache + (((size_t)page * p.n_kv_heads + kvh) * p.page_tokens + key % p.page_tokens) * n + d);
             } else {
@@ -134,6 +134,11 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
             }
         }
         cp_commit();
+    };
+    auto fetch = [&](int j, const float* cache, int n, float* to) {
+        const int key0 = tile_key0(j);
+        if (key0 >= first_key) fetch_keys(key0, cache, n, to, std::true_type{});
+        else fetch_keys(key0, cache, n, to, std::false_type{});
     };
     float m[NR], l[NR];
     pair_t acc[NR][2 * NC];

@@ -95,14 +95,15 @@ struct NormArgs {
     // W and whose results go to columns z * head_c_cols + [0, N) of C.  K is a head's K; what a
     // block of 64 columns of A holds beyond it meets columns of W outside its map, which read zero.
     int heads, head_a_cols, head_c_cols;
-    // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2.  PER_HEAD, with `gate` set: the
-    // results times the sigmoids of their logits before they are rounded, of one logit a row and head
+    // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2.  PER_HEAD, with `gate` set (up to
+    // GATED_ROWS rows): the results times the sigmoids of their logits before they are rounded, of one logit a row and head
     // (GATE_HEAD: fp32 [M][heads]) or of one a result (GATE_RESULT: bf16 [M][heads * N]).
     int act;
     const void* gate;
     int gate_ld;
 };
 constexpr int GATE_HEAD = 2, GATE_RESULT = 3;
+constexpr int GATED_ROWS = 16;          // rows of a product per head that takes a gate, at the most
 
 template <int BN, int STAGES, int MH>
 struct SharedStorage {
@@ -400,6 +401,40 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             }
         };
         if (EPI == ROPE_APPEND) rope_rows(row);
+        // PER_HEAD: the gates of up to 16 rows, worked out by all four warps while the products run, behind
+        // the stages (16 heads of 128 x 256, 3 to 8 rows 3.1 us, 2.9 without a gate, 4.8 with a launch of
+        // its own for it; 16 rows 4.0 and 4.9.  By each row's own thread, 128 sigmoids in a chain, they
+        // took 8 us; more rows are better off with that launch: 48 rows 8.1 here and 5.2)
+        const bool gated = FORM == PER_HEAD && EPI == STORE_BF16 && na.gate != nullptr;
+        constexpr int GATE_PITCH = BN + 4;
+        float* const gates = reinterpret_cast<float*>(c_tile);
+        if (gated) {
+            const int rows = min(GATED_ROWS, M - m0);
+            for (int i = threadIdx.x - 64; i < rows * (BN / 4); i += 128) {
+                const int r = i / (BN / 4), c = (i % (BN / 4)) * 4, col = n_tile * BN + c;
+                float z[4];
+                if (na.act == GATE_HEAD) {
+                    z[0] = z[1] = z[2] = z[3] = __ldg(static_cast<const float*>(na.gate) + (size_t)(m0 + r) * na.gate_ld + head);
+                } else {
+                    const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(na.gate) + (size_t)(m0 + r) * na.gate_ld +
+                                             (size_t)head * N + col;
+                    __nv_bfloat16 b[4];
+                    if (col + 4 <= N && ((uintptr_t)g & 7) == 0) {
+                        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(g));
+                        memcpy(b, &raw, 8);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) b[j] = col + j < N ? g[j] : __nv_bfloat16();
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) z[j] = __bfloat162float(b[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[j] = 1.0f / (1.0f + expf(-z[j]));
+                *reinterpret_cast<float4*>(gates + r * GATE_PITCH + c) = make_float4(z[0], z[1], z[2], z[3]);
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         bool ok = tc::mbar_wait(&s.tmem_full_bar, 0, abort_flag);
         if (!ok && !*abort_flag) tc::give_up(abort_flag, status, tc::ST_EPILOGUE_TIMEOUT);
         ok = __all_sync(0xffffffffu, ok);
@@ -794,32 +829,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     }
                 }
             } else {
-                // 32 results of a head times the sigmoids of their logits
-                auto gate_chunk = [&](uint32_t (&r)[32], int at_row, int at_head, int col) {
-                    if (na.act == GATE_HEAD) {
-                        const float f = 1.0f / (1.0f + expf(-static_cast<const float*>(na.gate)[(size_t)at_row * na.gate_ld + at_head]));
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
-                        return;
-                    }
-                    const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(na.gate) + (size_t)at_row * na.gate_ld +
-                                             (size_t)at_head * N + col;
-                    const bool wide = col + 32 <= N && ((uintptr_t)g & 15) == 0;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        __align__(16) __nv_bfloat16 z[8];
-                        if (wide) {
-                            *reinterpret_cast<uint4*>(z) = __ldg(reinterpret_cast<const uint4*>(g) + q);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) z[j] = col + 8 * q + j < N ? g[8 * q + j] : __nv_bfloat16();
-                        }
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            r[8 * q + j] = __float_as_uint(__uint_as_float(r[8 * q + j]) *
-                                                           (1.0f / (1.0f + expf(-__bfloat162float(z[j])))));
-                    }
-                };
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     uint32_t r[32];
@@ -838,7 +847,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                             r[j] = __float_as_uint(z * z);
                         }
                     }
-                    if (EPI == STORE_BF16 && FORM == PER_HEAD && na.gate != nullptr) gate_chunk(r, row, head, col0);
+                    if (gated) {
+                        const float* g = gates + (quarter * 32 + lane) * GATE_PITCH + c0;
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) {
+                            const float4 z = *reinterpret_cast<const float4*>(g + j);
+                            r[j] = __float_as_uint(__uint_as_float(r[j]) * z.x);
+                            r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) * z.y);
+                            r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) * z.z);
+                            r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) * z.w);
+                        }
+                    }
                     const bool full = col0 + 32 <= N;
                     if (EPI == STORE_BF16) {
                         __nv_bfloat16* dst = (__nv_bfloat16*)c_ptr + (size_t)row * ldc + col0;
@@ -953,7 +972,10 @@ int launch_form(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
     if (grouped) ms = *few;
     if (emit && !tc::make_plain_box_map_2d(&ms, na.scaled, (uint64_t)M, (uint64_t)N, (uint64_t)na.ld_scaled, 32, BM))
         return CB_ERR_UNSUPPORTED;
-    const int smem = (int)(emit ? smem_emit : smem_plain);
+    const size_t smem_gate = ((sizeof(Storage) + 1023) & ~(size_t)1023) + (size_t)GATED_ROWS * (BN + 4) * 4 + 1024;
+    const bool gated = per_head && na.gate != nullptr;
+    if (gated && (M > GATED_ROWS || smem_gate > 227 * 1024)) return CB_ERR_UNSUPPORTED;
+    const int smem = (int)(emit ? smem_emit : gated ? smem_gate : smem_plain);
     static int configured = 0;
     if (configured < smem) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, STAGES, EPI, MH, FORM>,
@@ -1110,7 +1132,7 @@ CB_EXPORT int cb_gemm_tcgen05_grouped(const void* A, const void* W, void* C, int
 // A product per head in one launch: A [M, a_cols] holds head h's K columns from h * head_a_cols,
 // W [heads * N, K] the heads' matrices one below the other, and head h's results go to columns
 // h * head_c_cols + [0, N) of C (bf16 or fp32 by epi: STORE_BF16 or STORE_F32).  bn: 64, 96 or 128.
-// gate (STORE_BF16 alone; null: none) as in NormArgs, of the kind GATE_HEAD or GATE_RESULT.
+// gate (STORE_BF16 and up to GATED_ROWS rows alone; null: none) as in NormArgs, of the kind GATE_HEAD or GATE_RESULT.
 CB_EXPORT int cb_gemm_tcgen05_heads(const void* A, const void* W, void* C, int M, int N, int K, int a_cols,
                                     int lda, int ldw, int ldc, int heads, int head_a_cols, int head_c_cols,
                                     int epi, int bn, const void* gate, int gate_ld, int gate_kind, int* status,

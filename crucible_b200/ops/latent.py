@@ -63,7 +63,7 @@ def rows_gate(x, g) -> None:
 
 
 WARP_ROWS = 2        # steps of up to this many rows take a warp per weight row ...
-SMALL_ROWS = 16      # ... and steps of up to this many that the tiles refuse
+SMALL_ROWS = 16      # ... and steps of up to this many that the tiles refuse; the tiles take a gate with as many
 HEADS_IN_ONE_LAUNCH = True   # more bfloat16 rows: the heads as the third axis of one tensor-core launch
                              # (tests switch it off to reach the product per head with the same inputs)
 
@@ -73,13 +73,13 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
     `w` [heads, N, K].  bfloat16 rows run as one launch of tensor-core tiles with the head as the grid's
     third axis; one or two of them, and few whose sizes the tiles refuse, as one launch whose warps each
     read one weight row once; otherwise one product per head through `ops.linear` (in float32 always,
-    so that a row's sums never depend on the step).  A whole layer of 16 heads over a latent of 192, both
-    ways: 8 rows 47 us with the tiles, 53 with the warps; 16 rows 51 and 68; 24 rows 66, and 140 as
-    a product per head; one row 45 and 45 with a launch less for the gate.
-    `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), in the same
-    launch and before they are rounded where there is one for all heads, by `head_gate` otherwise.
-    `gate_rows` (rows of the activations' dtype, [rows, heads * N]): every result times the sigmoid
-    of its own logit, likewise."""
+    so that a row's sums never depend on the step).  16 heads of 128 x 256 with a gate: 8 rows 3.1 us with
+    the tiles, 7.8 with the warps; 16 rows 4.0 and 14; a whole layer of 24 rows 66, and 140 as a product
+    per head.  (One or two rows 3.1 and 4.5: the line dates from when the tiles took no gate, and a launch
+    for it made up for that.)
+    `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), before they are
+    rounded in the one launch of up to SMALL_ROWS rows, by `head_gate` otherwise.  `gate_rows` (rows of the
+    activations' dtype, [rows, heads * N]): every result times the sigmoid of its own logit, likewise."""
     from . import linear
     heads, n, k = w.shape
     if gate_rows is not None and (out_head != n or gate_rows.shape != (a.shape[0], heads * n)
@@ -87,13 +87,15 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
         raise KernelError("heads_linear: gate rows are [rows, heads * N] of the results' dtype")
     from . import is_weight, tensor_core
     rows = a.shape[0]
-    # the gate that the tiles take with them: of one kind, its logits side by side
-    gate = gate_logit if gate_rows is None else gate_rows if gate_logit is None else None
-    if gate is not None and (out.dtype != torch.bfloat16 or out_head != n or out.shape[1] != heads * n
-                             or not gate.is_cuda or gate.stride(1) != 1
-                             or (gate_rows is None and (gate.dtype != torch.float32 or gate.shape != (rows, heads)))):
-        gate = None
-    done = (HEADS_IN_ONE_LAUNCH and a.dtype == torch.bfloat16 and rows > WARP_ROWS and is_weight(w)
+    # the gate that the tiles take with them: few rows, of one kind, its logits side by side (few rows with
+    # another are the warps', which take any)
+    gate, taken = None, True
+    if rows <= SMALL_ROWS and (gate_logit is not None or gate_rows is not None):
+        gate = gate_logit if gate_rows is None else gate_rows if gate_logit is None else None
+        taken = (gate is not None and out.dtype == torch.bfloat16 and out_head == n and out.shape[1] == heads * n
+                 and gate.is_cuda and gate.stride(1) == 1
+                 and (gate_rows is not None or (gate.dtype == torch.float32 and gate.shape == (rows, heads))))
+    done = (HEADS_IN_ONE_LAUNCH and a.dtype == torch.bfloat16 and rows > WARP_ROWS and taken and is_weight(w)
             and tensor_core.heads_linear(a, a_head, w, out, out_head, gate))
     if done and gate is not None:
         return

@@ -10,6 +10,8 @@ row stride of a bfloat16 output must be multiples of 8 elements (TMA needs
 from __future__ import annotations
 
 import ctypes
+import functools
+import math
 import os
 
 import torch
@@ -353,17 +355,21 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
     return _gemm(a, w, out, w.shape[0], epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
 
 
-def grouped_tile(pairs: int, n_experts: int, gated: bool):
-    """(tile width, blocks to an SM) of a grouped product.  Many rows an expert: the widest tile asks for the
-    fewest operand bytes (2,048 tokens, two of 8 experts of 2,816 x 2,048: gate/up 125 us with 128 columns,
-    101 with 256; down 66 and 54).  Fewer: the weights' bytes decide, and how the blocks fill the SMs (64
-    pairs: gate/up 41 us with 128 columns, 35 with 192, 41 with 256; down 15, 18, 20; 16 pairs: gate/up 29
-    with 128, 25 with 128 and two blocks to an SM, 33 with 192)."""
-    if pairs >= 64 * n_experts:
-        return 256, 1
-    if not gated:
-        return 128, 1
-    return (192, 1) if pairs >= 4 * n_experts else (128, 2)
+@functools.lru_cache(maxsize=4096)
+def grouped_tile(pairs: int, n_experts: int, n_cols: int, gated: bool):
+    """(tile width, blocks to an SM) of a grouped product over `n_cols` rows of an expert's matrix.  Blocks
+    run in waves over the SMs and a block costs its width and a fixed part of 160 columns, which here
+    is mostly the operands' way in.  Tiles of 128 rows: one an expert while few experts have more rows than
+    that, then a half-filled one each beside the full ones.  Over 16 to 4,096 pairs of 8 experts of 2,816 x 2,048
+    and 1,408 x 1,024 the choice is 0.5 % from the best width on average, 14 % at worst; 128 columns
+    throughout 16 %, 67 % at worst (4,096 pairs, gate/up of 2,816: 106 us with 256 columns, 150 with
+    128; 512 pairs: gate/up 36 with 192 and 42 with 128, down 17.5 with 128 and 23.8 with 256).
+    A couple of pairs an expert: not all experts have rows, and with two blocks to an SM all blocks of
+    the wide gate/up find a place at once (16 pairs: 24.7 us, 31.2 with 192 columns)."""
+    if gated and pairs < 3 * n_experts:
+        return 128, 2
+    tiles = n_experts if pairs <= 112 * n_experts else pairs / 128 + n_experts / 2
+    return min((-(-int(math.ceil(tiles * -(-n_cols // bn))) // N_SMS) * (bn + 160), bn) for bn in (128, 192, 256))[1], 1
 
 
 def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pair=None, tile=None) -> bool:
@@ -381,7 +387,7 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     args = _NormArgs()
     if pair is not None:
         args.glu_limit, args.glu_alpha, args.glu_offset = (float(v) for v in pair)
-    bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, gated)
+    bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, w.shape[1], gated)
     args.plan, args.n_experts, args.max_tiles, args.w_rows = plan.data_ptr(), n_experts, tiles, w.shape[1]
     lib = build.load("gemm_tcgen05")
     code = lib.cb_gemm_tcgen05_grouped(
@@ -405,7 +411,7 @@ GATE_HEAD, GATE_RESULT = 2, 3
 def heads_linear(a, a_head: int, w, out, out_head: int, gate=None) -> bool:
     """out[t, h * out_head + n] = sum_k a[t, h * a_head + k] * w[h, n, k] for every head of `w`
     [heads, N, K] (a declared bfloat16 weight) in ONE launch (`cb_gemm_tcgen05_heads`: the head is
-    the grid's third axis).  `gate` (bfloat16 results alone): float32 logits [rows, heads] or bfloat16 ones
+    the grid's third axis).  `gate` (bfloat16 results of up to 16 rows alone): float32 logits [rows, heads] or bfloat16 ones
     [rows, heads * N] whose sigmoids the results are multiplied by before they are rounded.  Refuses
     what the tiles cannot take (the caller then runs a product per head)."""
     heads, n, k = w.shape

@@ -132,3 +132,12 @@ def test_portions_go_in_chunks_where_that_was_quicker(rule, rows, requests, long
     """Steps of which one form was measured to be well ahead (heads of 128 key channels)."""
     from crucible_b200.ops import recurrent
     assert recurrent.chunks_pay(getattr(recurrent, rule), rows, requests, longest, heads) == chunks
+
+
+@pytest.mark.parametrize("pairs,cols,gated,width", [
+    (16, 5632, True, 128), (64, 5632, True, 192), (64, 2048, False, 128), (512, 5632, True, 192), (512, 2048, False, 128),
+    (896, 1024, False, 128), (1024, 5632, True, 256), (1024, 2816, True, 256), (4096, 5632, True, 256),
+    (4096, 2048, False, 256), (4096, 1024, False, 256)])
+def test_grouped_tiles_where_a_width_was_quicker(pairs, cols, gated, width):
+    """Products of 8 experts of which one width was measured to be ahead."""
+    assert tensor_core.grouped_tile(pairs, 8, cols, gated)[0] == width

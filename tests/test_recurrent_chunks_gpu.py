@@ -3,8 +3,9 @@ token of each of several requests (`csrc/recurrent.cu`, the step form), against 
 same recurrences token by token in float64, for every rule: portions that end inside a chunk, at its
 edge and one token beyond it, a state carried in, heads and values that are no whole tiles, decays of 0
 and 1, requests of one token at the head of the step.  The operands are float32, so the error is that
-of float32 sums: the bound is eight times what the token-by-token kernel shows on the same operands (a
-chunk sums in another order, the triangular system included), and never below 2e-6."""
+of float32 sums: the bound is twice what the token-by-token kernel shows on the same operands (a
+chunk sums in another order, the triangular system included; up to 64 chunks showed 1.5 times), or four roundings
+of float32.  The mLSTM divides by a sum that may all but cancel, in either form: four times, or eight roundings."""
 from types import SimpleNamespace
 
 import pytest
@@ -13,6 +14,7 @@ import torch
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 LENGTHS = [(1, 128, 33), (1, 1, 161), (200,), (129, 31, 32), (1,), (1, 1, 1, 1, 1)]
+ROUNDING = 2.0 ** -23
 
 
 def _i32(values):
@@ -102,7 +104,7 @@ def test_chunks_agree_with_float64(rule, H, G, D, E, monkeypatch):
         G = H
     elif (H, D) == (4, 128):
         E = 40                                    # values unlike keys, no whole tiles
-    for lengths in LENGTHS:
+    for lengths in LENGTHS + ([(2048,)] if (H, D) == (4, 128) else []):
         g = torch.Generator().manual_seed(len(lengths) + D)
         T, R = sum(lengths), len(lengths)
         q, kk, v, w, sc0, sc1, per_head = _operands(rule_code, k, T, H, G, D, E, g)
@@ -140,7 +142,8 @@ def test_chunks_agree_with_float64(rule, H, G, D, E, monkeypatch):
                     off.append(float((state[r, sum(sizes[:2]):][:H].double() - m).abs().max()) / max(1.0, float(m.abs().max())))
                 errors[chunks] = off
             for got, plain in zip(errors[True], errors[False]):
-                assert got <= max(8 * plain, 2e-6), (rule, lengths, r, errors)
+                times, least = (4, 8 * ROUNDING) if rule == "MLSTM" else (2, 4 * ROUNDING)
+                assert got <= max(times * plain, least), (rule, lengths, r, errors)
 
 
 @pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])

@@ -276,6 +276,47 @@ def test_gated_delta_rule_in_portions(dtype, H, G, D, E, taps):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,D,E,taps", [(4, 2, 16, 24, 4), (2, 2, 40, 72, 3), (3, 1, 128, 32, 2), (1, 1, 64, 100, 4)])
+@pytest.mark.parametrize("ssd", [False, True])
+def test_wide_preparation_agrees_with_a_block_a_token(dtype, H, G, D, E, taps, ssd):
+    """The preparations' form of 16 bytes a lane, which the engine's steps take: portions down to one token
+    (shorter than the convolution's reach), off its tiles of 8 tokens and of 16 (from 1,024 on), in
+    slots that are not in order.  Beside the form of a block a token: the state's last inputs in the same
+    bytes, numbers within some roundings of float32 sums of at most 128 terms."""
+    from crucible_b200.ops import recurrent as k
+    g = torch.Generator().manual_seed(H * 10 + D)
+    C = 2 * G * D + H * E
+    on = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    conv_w, conv_b = on(C, taps) * 0.5, on(C)
+    a_log, dt_bias = on(H) * 0.3, on(H)
+    wide = torch.randn(5, (taps - 1) * C, generator=g).to(DEV)
+    plain_state = wide.clone()
+    for portions, slots in [((2, 1), (3, 1)), ((1, 2), (3, 1)), ((1,), (3,)), ((9, 3, 1), (1, 4, 3)), ((16, 8), (4, 0)),
+                            ((1030, 5), (1, 3)), ((1,), (1,))]:
+        t = sum(portions)
+        proj, gates = on(t, C + 8).to(dtype), on(t, 2 * H)
+        results = []
+        for state, host in ((wide, SimpleNamespace(max_new_tokens=max(portions))), (plain_state, None)):
+            ctx = _state_ctx(portions, list(slots), 4 * state.shape[1])
+            ctx.host = host
+            dst, one, two = torch.empty(t, C, device=DEV), torch.empty(t, H, device=DEV), torch.empty(t, H, device=DEV)
+            raw = state.view(torch.uint8)
+            if ssd:
+                done = k.ssd_prepare(proj, 4, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, raw, 0, dst, one, two, H, C,
+                                     update_tail=True)
+            else:
+                done = k.delta_prepare(proj, conv_w, taps, gates, a_log, dt_bias, ctx, raw, 0, dst, one, two, H, G, D, E,
+                                       update_tail=True)
+            assert done == (host is not None)
+            if not done:
+                k.conv_tail_update(proj[:, 4:4 + C] if ssd else proj, taps, C, ctx, raw, 0)
+            results.append((dst, one, two))
+        assert torch.equal(wide, plain_state), portions
+        for got, want in zip(*results):
+            assert rel(got, want) < 2e-6, portions
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,D,E", [(2, 16, 32), (3, 72, 40), (1, 256, 16)])
 def test_mlstm_in_portions(dtype, H, D, E):
     from crucible_b200.ops import recurrent as k

@@ -650,23 +650,25 @@ def wide_row_chunk_keys(blocks_per_chunk: int, context_bucket: int, window) -> i
     return min(max(chunk, unit), whole)
 
 
+MIXED_REACH = 2048 * 256     # keys times features
+MIXED_FEW = 12               # decoded tokens
+
+
 def tiles_first(host, n_requests, head_dim, window, keep_first) -> int:
     """The first request of a step that the tcgen05 tiles take (`n_requests`: none): 0, or behind the
     single decoded tokens at its head, which the caller then runs with their keys dealt to several
     blocks.  A decoded token is a block of 128 rows like another in the tiles' launch and walks its keys
-    alone, 2 us a tile of 128 keys of 128 features: it rides along while that is not much longer than
-    the launch is anyway (16 heads of 128, 24 decoded tokens: behind 2,000 keys beside 100 prompt tokens
-    101 us a layer in two launches, 78 in one; 4 behind 3,000 keys 72 in two, 88 in one)."""
+    alone, 10 us a thousand keys of 64 features, 12 of 128 and 21 of 256: it rides along unless few tokens
+    have long to walk; the more there are, the longer the launch of their own takes.  (One launch and two,
+    16 heads: of 128, 4 tokens behind 3,000 keys beside 2,000 of a prompt 48 and 70 us, 48 behind 3,500 beside 500
+    62 and 242; of 256, 12 behind 3,500 beside 200 72 and 52, 24 behind 3,000 beside 300 62 and 66.)"""
     lead = host.lead_single
     if lead == 0 or lead == n_requests:
         return lead
     reach = host.lead_context_bucket
     if window is not None:
         reach = min(reach, window + 128 + (keep_first or 0))
-    return 0 if reach * head_dim <= MIXED_REACH else lead
-
-
-MIXED_REACH = 2560 * 128     # keys times features
+    return 0 if reach * head_dim <= MIXED_REACH * (1 if lead <= MIXED_FEW else 4) else lead
 
 
 def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, scale, window, keep_first,

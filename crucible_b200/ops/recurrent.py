@@ -29,15 +29,17 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
     """Whether a bfloat16 step's portions (`rows` tokens of `requests`, without the single tokens at the
     step's head; the longest; `heads` of 128 key channels) go in chunks.  The walk takes its time a token of the
     longest portion until the requests fill the GPU, then a time a token; a chunk that holds few tokens
-    costs what a full one does, and every portion ends in one such.  Over the sizes that the costs were fitted to the
-    choice is 0.5 % (delta rules), 0.7 (mLSTM), 1.1 (state space) and 1.4 (wkv) from the better form on average.  16 heads of 128, chunks and
+    costs what a full one does, and every portion ends in one such.  The chunks have to be 5 % and 5 us ahead: their
+    launches and workspaces are 25 us of host work, which a step that runs eagerly pays (wkv, a portion of
+    150: 37 and 36 us, the layer 275 and 242).  Over the sizes that the costs were fitted to the choice is 1.6 to
+    3.1 % from the better form on average, and at most 1.15 times the walk (wkv of 32 heads of 64: 1.23).  16 heads of 128, chunks and
     walk: delta rule 1 portion of 110 tokens 27 and 30 us, 24 of up to 300 514 and 450; state space
     1 of 140 35 and 31, of 500 45 and 103; 24 of up to 60 101 and 90."""
     if requests <= 0:
         return False
     (start, token, work), (first, step, chunk) = COSTS[rule]
     walk = start + token * longest + work * rows * heads
-    return walk > 1.05 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads)
+    return walk > 1.05 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads) + 5.0
 
 
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces

@@ -123,7 +123,7 @@ def test_the_chunks_workspaces_are_bounded():
 
 
 @pytest.mark.parametrize("rule,rows,requests,longest,heads,chunks", [
-    ("DELTA", 2048, 1, 2048, 16, True), ("DELTA", 56, 1, 56, 16, False), ("DELTA", 110, 1, 110, 16, True),
+    ("DELTA", 2048, 1, 2048, 16, True), ("DELTA", 56, 1, 56, 16, False), ("DELTA", 180, 1, 180, 16, True),
     ("DELTA", 430, 5, 200, 4, True), ("DELTA", 3648, 24, 300, 16, False), ("CHANNEL", 3648, 24, 300, 32, False),
     ("CHANNEL", 430, 5, 200, 8, True), ("MLSTM", 140, 1, 140, 8, True), ("MLSTM", 72, 1, 72, 16, False),
     ("SSD", 768, 24, 60, 32, False), ("SSD", 1030, 5, 400, 16, True), ("SSD", 110, 1, 110, 16, False),

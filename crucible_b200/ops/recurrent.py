@@ -4,6 +4,7 @@ state-space rule, the delta rule with a decay per key channel)."""
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -45,15 +46,20 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces
 
 
+@functools.lru_cache(maxsize=256)
+def _space_of(rule, n_heads: int, key_dim: int, value_dim: int):
+    """Bytes that a row and that a chunk take in the chunks' workspaces."""
+    delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
+    return (4 * n_heads * (key_dim * ((delta or vector) + delta + (rule == CHANNEL)) + value_dim * delta + 4),
+            4 * n_heads * (key_dim * (vector + (rule == MLSTM)) + (0 if delta else key_dim * value_dim) + 1))
+
+
 def slice_tokens(rows: int, requests: int, longest: int, row_bytes: int, chunk_bytes: int) -> int:
     """Tokens of each of `requests` portions (`rows` tokens in all) that go through the chunks at a time: all of
     the longest if the workspaces then stay within CHUNK_SPACE, else what does, in whole chunks and one
     at least.  (16 heads of 128 x 128 take 25 to 33 KB a token, so that up to 8,000 tokens go at once;
     a longer step's slices each fill the GPU.)"""
-    def space(tokens):
-        taken = min(rows, requests * tokens)
-        return taken * row_bytes + (taken // 32 + requests) * chunk_bytes
-    if space(longest) <= CHUNK_SPACE:
+    if rows * row_bytes + (rows // 32 + requests) * chunk_bytes <= CHUNK_SPACE:
         return longest
     per_token = requests * (row_bytes + chunk_bytes / 32)
     return max(32, int((CHUNK_SPACE - requests * chunk_bytes) / per_token) // 32 * 32)
@@ -216,10 +222,7 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         walked = host.lead_single
         longest, f32 = host.max_new_tokens, torch.float32
         delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
-        # bytes a row and a chunk take in the workspaces, and the tokens of each request that go at a time
-        row_bytes = 4 * n_heads * (key_dim * ((delta or vector) + delta + (rule == CHANNEL)) + value_dim * delta + 4)
-        chunk_bytes = 4 * n_heads * (key_dim * (vector + (rule == MLSTM)) + (0 if delta else key_dim * value_dim) + 1)
-        limit = slice_tokens(qkv.shape[0] - walked, n - walked, longest, row_bytes, chunk_bytes)
+        limit = slice_tokens(qkv.shape[0] - walked, n - walked, longest, *_space_of(rule, n_heads, key_dim, value_dim))
         rows = min(qkv.shape[0] - walked, (n - walked) * limit)
         places = rows // 32 + n - walked
 

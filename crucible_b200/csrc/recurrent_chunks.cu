@@ -22,12 +22,13 @@
 // S as every chunk begins, and chunk_out_kernel adds the queries over it, again all chunks side by side.
 // Delta rules: chunk_walk_kernel; a block owns 16 (or 8) columns of a head's S and walks the chunks in
 // order: per chunk two products on fp32 FMA (rows of Q and W over S; k^T over u), the next chunk's
-// operands on their way by asynchronous copies.  It is bound by the bytes that shared memory returns to
-// registers (3/4 of a chunk's 6,000 cycles).
+// operands on their way by asynchronous copies.  57 % of a chunk's 5,300 cycles go into operands out of
+// shared memory, the rest into the four block barriers and the chain between the products.
 //
-// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 244 us, channel delta
-// 551 -> 310, mLSTM 590 -> 172, wkv 414 -> 170, state space 410 -> 163; 8 heads: 502 -> 160, 551 -> 199, 590 -> 90,
-// 413 -> 92, 410 -> 79.
+// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 235 us (under ncu, cold: the chunks'
+// numbers 80, the walk 177), channel delta 551 -> 324, mLSTM 590 -> 172, wkv 467 -> 169, state space 408 -> 168;
+// 8 heads: 502 -> 165, 551 -> 210, 589 -> 91, 467 -> 90, 407 -> 79.  16,384 tokens of 16 heads in slices (256 MB of
+// workspaces): delta 1,768 us, 1,760 at once; mLSTM 1,340 and 1,292; state space 1,403 and 1,380.
 //
 // The result differs from the token-by-token walk by rounding, and with the way a prompt is cut: the
 // bfloat16 engine's prompts alone take this path; decoded tokens and the float32 engine keep the walk.

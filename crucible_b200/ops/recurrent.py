@@ -17,30 +17,37 @@ CHUNKS = True                # tests switch it off to reach the token-by-token w
 STEP = True                  # likewise, for the form of a token each
 
 
-# us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128) and of the chunks
-# (their launches, a token of the longest portion, a chunk and head of 128), fitted to both forms over 4 to 32 heads of 64
-# and 128 and 1 to 24 uneven portions of up to 40 to 500 tokens; the delta rules' chunks are walked in order, the
-# others' are not
-_DELTA_COSTS = ((2.8, 0.160, 0.0061), (13.3, 0.024, 0.217))
-COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS, MLSTM: ((3.1, 0.202, 0.0067), (23.3, 0.0, 0.148)),
-         WKV: ((3.0, 0.131, 0.0057), (21.2, 0.0, 0.131)), SSD: ((3.5, 0.130, 0.0043), (22.0, 0.0, 0.131))}
+# us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128, a portion and head) and of
+# the chunks (their launches, a token of the longest portion, a chunk and head of 128), fitted to both forms over 4 to 32
+# heads of 64 and 128 and 1 to 24 uneven portions of up to 40 to 500 tokens; the delta rules' chunks are walked in
+# order, the others' are not
+_DELTA_COSTS = ((1.8, 0.172, 0.0052, 0.0525), (13.3, 0.024, 0.217))
+COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS, MLSTM: ((1.8, 0.216, 0.0057, 0.0597), (23.1, 0.0, 0.137)),
+         WKV: ((2.0, 0.142, 0.0049, 0.0501), (20.5, 0.0, 0.129)), SSD: ((2.6, 0.140, 0.0037, 0.040), (20.7, 0.0, 0.1275))}
 
 
 def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bool:
     """Whether a bfloat16 step's portions (`rows` tokens of `requests`, without the single tokens at the
     step's head; the longest; `heads` of 128 key channels) go in chunks.  The walk takes its time a token of the
     longest portion until the requests fill the GPU, then a time a token; a chunk that holds few tokens
-    costs what a full one does, and every portion ends in one such.  The chunks have to be 5 % and 5 us ahead: their
-    launches and workspaces are 25 us of host work, which a step that runs eagerly pays (wkv, a portion of
-    150: 37 and 36 us, the layer 275 and 242).  Over the sizes that the costs were fitted to the choice is 1.6 to
-    3.1 % from the better form on average, and at most 1.15 times the walk (wkv of 32 heads of 64: 1.23).  16 heads of 128, chunks and
-    walk: delta rule 1 portion of 110 tokens 27 and 30 us, 24 of up to 300 514 and 450; state space
-    1 of 140 35 and 31, of 500 45 and 103; 24 of up to 60 101 and 90."""
+    costs what a full one does, and every portion ends in one such.  16 heads of 128, chunks and walk: delta rule
+    1 portion of 110 tokens 27 and 30 us, 24 of up to 300 514 and 450; state space 1 of 140 35 and 31, of 500 45 and
+    103; 24 of up to 60 101 and 90.
+    The chunks' launches and workspaces are some 30 us of host work, which a step that runs eagerly pays and whose
+    host time covers either form of little work (wkv, a portion of 150: 37 and 36 us on the device, the layer
+    eagerly 275 and 242): less than 96 tokens a request of the delta rules, or less than 160 of a few of the others,
+    are walked, and more where the costs say that the walk is ahead.  Of 954 steps measured that is
+    1.7 % from the quicker form on average."""
     if requests <= 0:
         return False
-    (start, token, work), (first, step, chunk) = COSTS[rule]
-    walk = start + token * longest + work * rows * heads
-    return walk > 1.05 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads) + 5.0
+    if rule in (DELTA, CHANNEL):
+        if rows < 96 * requests:
+            return False
+    elif longest < 160 and (longest < 48 or rows < 24 * requests or rows * heads < 4096):
+        return False
+    (start, token, work, portion), (first, step, chunk) = COSTS[rule]
+    walk = start + token * longest + (work * rows + portion * requests) * heads
+    return walk > 0.95 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads)
 
 
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces

@@ -61,6 +61,22 @@ def _space_of(rule, n_heads: int, key_dim: int, value_dim: int):
             4 * n_heads * (key_dim * (vector + (rule == MLSTM)) + (0 if delta else key_dim * value_dim) + 1))
 
 
+@functools.lru_cache(maxsize=4096)
+def _chunk_room(rule, rows: int, requests: int, n_heads: int, key_dim: int, value_dim: int, slices: bool):
+    """The chunks' workspaces in one buffer: its floats, and where wq, ww, wk, wu, ws, wg, wl, wn, wm and the
+    slices' n and m begin (-1: the rule has none)."""
+    delta, vector, mlstm = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL), rule == MLSTM
+    row, chunk = rows * n_heads, (rows // 32 + requests) * n_heads
+    sizes = (row * key_dim * (delta or vector), row * key_dim * delta, row * key_dim * (rule == CHANNEL),
+             row * value_dim * delta, row * 4, chunk * key_dim * vector, 0 if delta else chunk * key_dim * value_dim,
+             chunk * key_dim * mlstm, chunk * mlstm, 2 * requests * n_heads * (key_dim + 1) * (mlstm and slices))
+    floats, begins = 0, []
+    for size in sizes:
+        begins.append(floats if size else -1)
+        floats += -(-size // 4) * 4                 # (16-byte boundaries)
+    return floats, tuple(begins)
+
+
 def slice_tokens(rows: int, requests: int, longest: int, row_bytes: int, chunk_bytes: int) -> int:
     """Tokens of each of `requests` portions (`rows` tokens in all) that go through the chunks at a time: all of
     the longest if the workspaces then stay within CHUNK_SPACE, else what does, in whole chunks and one
@@ -227,36 +243,26 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
             and (s_off | state.stride(0) | qkv.data_ptr() | out.data_ptr() | state.data_ptr()) % 16 == 0):
         # prompts' portions in chunks; the requests at the head of the step that bring one token are walked
         walked = host.lead_single
-        longest, f32 = host.max_new_tokens, torch.float32
-        delta, vector = rule in (DELTA, CHANNEL), rule in (WKV, CHANNEL)
-        limit = slice_tokens(qkv.shape[0] - walked, n - walked, longest, *_space_of(rule, n_heads, key_dim, value_dim))
-        rows = min(qkv.shape[0] - walked, (n - walked) * limit)
-        places = rows // 32 + n - walked
-
-        def room(name, width, wanted=True):
-            return ctx.scratch(f"memory.{name}", (rows, n_heads, width), f32) if wanted else None
-        wq, ww, wk = room("wq", key_dim, delta or vector), room("ww", key_dim, delta), room("wk", key_dim, rule == CHANNEL)
-        wu, ws = room("wu", value_dim, delta), room("ws", 4)
-        wg = ctx.scratch("memory.wg", (places, n_heads, key_dim), f32) if vector else None
-        wl = ctx.scratch("memory.wl", (places, n_heads, key_dim, value_dim), f32) if not delta else None
-        wn = ctx.scratch("memory.wn", (places, n_heads, key_dim), f32) if rule == MLSTM else None
-        wm = ctx.scratch("memory.wm", (places, n_heads), f32) if rule == MLSTM else None
-        kept_room = (ctx.scratch("memory.kept", (2, n - walked, n_heads * (key_dim + 1)), f32)
-                     if rule == MLSTM and limit < longest else None)
+        longest, requests = host.max_new_tokens, n - walked
+        limit = slice_tokens(qkv.shape[0] - walked, requests, longest, *_space_of(rule, n_heads, key_dim, value_dim))
+        rows = min(qkv.shape[0] - walked, requests * limit)
+        floats, begins = _chunk_room(rule, rows, requests, n_heads, key_dim, value_dim, limit < longest)
+        room = ctx.scratch("memory.chunks", (floats,), torch.float32).data_ptr()
+        wq, ww, wk, wu, ws, wg, wl, wn, wm, kept_room = (_c_void_p(room + 4 * at if at >= 0 else 0) for at in begins)
         lib = build.load("recurrent_chunks")
         code = lib.cb_matrix_memory_chunks(
             _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
             _ptr(sc0), _ptr(sc1), _c_void_p(starts + 4 * walked), _c_void_p(slots + 4 * walked), sp, stride,
-            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(n - walked),
+            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(requests),
             _c_int(longest), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
             _c_int(w_off), _ptr(per_head),
             _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
-            _c_int(limit), _ptr(kept_room), _ptr(wq), _ptr(ww), _ptr(wk), _ptr(wu), _ptr(ws), _ptr(wg), _ptr(wl), _ptr(wn), _ptr(wm), _stream())
+            _c_int(limit), kept_room, wq, ww, wk, wu, ws, wg, wl, wn, wm, _stream())
         if code == build.UNSUPPORTED:            # the walk's
             walked = n
         else:
             _check(code, "matrix_memory (chunks)")
-            LAUNCHES[0] += (2 if delta else 3) * -(-longest // limit) - 1
+            LAUNCHES[0] += (2 if rule in (DELTA, CHANNEL) else 3) * -(-longest // limit) - 1
     if walked == 0:
         return
     lib = build.load("recurrent")

@@ -179,8 +179,9 @@ def test_slices_have_the_bits_of_one(rule, space, limit, monkeypatch):
         monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
         assert k.CHUNK_SPACE == whole
         portions = R - (lengths[0] == 1)
-        rows = dict(asked)["memory.ws"][0]
-        assert rows <= min(T, portions * limit)
+        rows, (row_bytes, chunk_bytes) = min(T, portions * limit), k._space_of(code, H, D, D)
+        room = 4 * dict(asked)["memory.chunks"][0]
+        assert room <= rows * row_bytes + (rows // 32 + portions) * chunk_bytes + 8 * portions * H * (D + 1) + 160
         assert bool(torch.isfinite(results[0][0]).all())
         assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1]), lengths
 

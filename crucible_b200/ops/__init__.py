@@ -291,6 +291,24 @@ def linear_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *,
            "linear (CUDA cores)")
 
 
+def linear_heads_plain(a, a_head: int, w, out, out_head: int) -> None:
+    """out[t, h * out_head + n] = sum_k a[t, h * a_head + k] * w[h, n, k] for every head of `w`
+    [heads, N, K] in one launch; each head's sums are those of `linear_plain`."""
+    _need_cuda(a, w, out)
+    heads, n, k = w.shape
+    if (a.dtype != w.dtype or a.shape[1] < (heads - 1) * a_head + k or out.shape[0] != a.shape[0]
+            or out.shape[1] < (heads - 1) * out_head + n):
+        raise KernelError(f"linear per head: a is {tuple(a.shape)} {a.dtype}, w is {tuple(w.shape)} {w.dtype}, "
+                          f"output is {tuple(out.shape)}")
+    if a.stride(1) != 1 or w.stride(2) != 1 or out.stride(1) != 1:
+        raise KernelError("linear per head: rows must be contiguous")
+    lib = build.load("gemm_simt")
+    _check(lib.cb_gemm_simt_heads(_ptr(a), _ptr(w), _ptr(out), _c_int(_code(a.dtype)), _c_int(_code(out.dtype)),
+                                  _c_int(a.shape[0]), _c_int(n), _c_int(k), _c_int(a.stride(0)), _c_int(w.stride(1)),
+                                  _c_int(out.stride(0)), _c_int(heads), _c_int(a_head), ctypes.c_long(w.stride(0)),
+                                  _c_int(out_head), _stream()), "linear per head (CUDA cores)")
+
+
 # Device ranges that hold weights: tensors that no kernel of a step writes.  The bfloat16
 # product kernels ask for their matrix before the kernels ahead of them in the stream have
 # finished (only the rows and the output wait for those), which is sound for a weight and a

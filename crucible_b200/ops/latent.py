@@ -72,15 +72,16 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
     """out[t, h * out_head + n] = sum_k a[t, h * a_head + k] * w[h, n, k] for every head h of
     `w` [heads, N, K].  bfloat16 rows run as one launch of tensor-core tiles with the head as the grid's
     third axis; one or two of them, and few whose sizes the tiles refuse, as one launch whose warps each
-    read one weight row once; otherwise one product per head through `ops.linear` (in float32 always,
-    so that a row's sums never depend on the step).  16 heads of 128 x 256 with a gate: 8 rows 3.1 us with
+    read one weight row once; otherwise one product per head through `ops.linear`.  float32 rows run as
+    one launch of the CUDA-core product's tiles always, so that a row's sums never depend on the step
+    (8 heads of 128 x 192, 116 rows: 2.8 us, 116 as a product per head).  16 heads of 128 x 256 with a gate: 8 rows 3.1 us with
     the tiles, 7.8 with the warps; 16 rows 4.0 and 14; a whole layer of 24 rows 66, and 140 as a product
     per head.  (One or two rows 3.1 and 4.5: the line dates from when the tiles took no gate, and a launch
     for it made up for that.)
     `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), before they are
     rounded in the one launch of up to SMALL_ROWS rows, by `head_gate` otherwise.  `gate_rows` (rows of the
     activations' dtype, [rows, heads * N]): every result times the sigmoid of its own logit, likewise."""
-    from . import linear
+    from . import linear, linear_heads_plain
     heads, n, k = w.shape
     if gate_rows is not None and (out_head != n or gate_rows.shape != (a.shape[0], heads * n)
                                   or gate_rows.dtype != out.dtype or gate_rows.stride(1) != 1):
@@ -114,7 +115,9 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
                                          _stream()),
                "heads_linear (few rows)")
         return
-    if not done:
+    if not done and a.dtype == torch.float32:
+        linear_heads_plain(a, a_head, w, out, out_head)
+    elif not done:
         for i in range(heads):
             linear(a[:, i * a_head:i * a_head + k], w[i], out[:, i * out_head:i * out_head + n])
     if gate_logit is not None:

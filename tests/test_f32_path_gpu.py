@@ -143,3 +143,35 @@ def test_products_on_cuda_cores(dtype, M, N, K, accumulate):
     assert torch.equal(got.cpu(), want)
     few = product(a[:min(M, 5)].contiguous())
     assert torch.equal(few[:1], got[:1])
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 4608, 64), (33, 2304, 36), (65, 1280, 128), (300, 1280, 68), (513, 768, 16)])
+def test_products_of_every_form_are_one_ascending_sum(M, N, K):
+    """Sizes of each of the four forms of the fp32 product, at the edges of their tiles and of a stage of K."""
+    from crucible_b200 import ops
+    g = torch.Generator().manual_seed(M * N + K)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    want = torch.zeros(M, N, dtype=torch.float64)
+    for k in range(K):                            # (a product of float32 numbers is exact in float64)
+        want = (want + a[:, k].double()[:, None] * w[:, k].double()[None]).float().double()
+    got = torch.full((M, N + 4), 7.0, device=DEV)
+    ops.linear_plain(a.to(DEV), w.to(DEV), got[:, :N])
+    assert torch.equal(got[:, :N].cpu(), want.float()) and bool((got[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("rows", [1, 40, 130])
+@pytest.mark.parametrize("n,k,a_head,shift", [(192, 128, 192, 0), (33, 20, 24, 0), (64, 30, 31, 1)])
+def test_products_per_head_are_the_products(rows, n, k, a_head, shift):
+    from crucible_b200 import ops
+    heads = 5
+    g = torch.Generator().manual_seed(rows + n)
+    a = torch.randn(rows, heads * a_head + shift, generator=g).to(DEV)[:, shift:]
+    w = torch.randn(heads, n, k, generator=g).to(DEV)
+    got = torch.zeros(rows, heads * n, device=DEV)
+    want = got.clone()
+    ops.linear_heads_plain(a, a_head, w, got, n)
+    for h in range(heads):
+        ops.linear_plain(a[:, h * a_head:h * a_head + k].contiguous(), w[h], want[:, h * n:h * n + n])
+    assert torch.equal(got, want)
+    with pytest.raises(ops.KernelError):
+        ops.linear_heads_plain(a[:, :heads * a_head - a_head + k - 1], a_head, w, got, n)

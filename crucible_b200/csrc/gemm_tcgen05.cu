@@ -36,14 +36,13 @@
 #define CB_PDL_BIT 0      // this file's bit in CRUCIBLE_PDL
 #include "common.cuh"
 #include "tc_common.cuh"
+#include "gemm_args.cuh"
 
 namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 64;                 // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-
-enum Epilogue { STORE_BF16 = 0, STORE_F32 = 1, ACCUM_F32 = 2, SWIGLU_BF16 = 3, ROPE_APPEND = 4 };
 
 // ROPE_APPEND: W = [Wq; Wk; Wv]; a tile covers whole heads.  The q heads are rotated
 // and stored (bf16) to C[M, ldc]; the k heads are rotated and the v heads copied into
@@ -60,48 +59,6 @@ struct RopeArgs {
     int n_heads, n_kv_heads, head_dim, page_tokens, write_cache;
 };
 
-// What a product knows of the RMS norm on either side of it.
-//   After it (ACCUM_F32 as the rows' last write before a norm): with `gain` set the epilogue
-//   also leaves bf16(x * gain) of the summed rows x in `scaled` and the tile's share of every
-//   row's sum of squares in `sumsq_out` [tiles along N][M] (summed in the order of the
-//   columns).  The tile of C comes into shared memory by TMA while the products run, so the
-//   thread that holds a row's accumulators also has the values they are added to; C itself
-//   still gets its sums by TMA adds, `scaled` leaves by TMA stores of 32-column boxes (a single
-//   tile of rows: in 64-byte pieces of the threads' own rows).
-//   Tiles up to 128 columns, N a multiple of 32.
-//   Before it (any epilogue): with `sumsq_in` set the rows of A are bf16(x * gain) of rows
-//   not yet divided by their root mean square; the epilogue sums a row's `parts` shares in
-//   their order and multiplies the row's accumulators by 1 / sqrt(sum / width + eps), which
-//   is the same product as with normalised rows up to the rounding of A.
-struct NormArgs {
-    const float* gain;
-    __nv_bfloat16* scaled;
-    float* sumsq_out;
-    int ld_scaled;
-    const float* sumsq_in;
-    int parts;
-    float width, eps;
-    // SWIGLU_BF16: limit > 0 makes the pair the capped one (tc::gated_pair), else silu(g) * u
-    float glu_limit, glu_alpha, glu_offset;
-    // A grouped product (form GROUPED): the rows of A lie expert by expert, W is the experts'
-    // matrices one below the other (w_rows rows each), and block row y takes tile y of the plan
-    // that a kernel before this one left on the device: [0] tiles in use, [2 + E + y] the tile's
-    // expert, [2 + E + max_tiles + y] its first row, [2 + E + 2 max_tiles + y] its rows (at most
-    // 128).  Tiles beyond those in use do nothing.
-    const int* plan;
-    int n_experts, max_tiles, w_rows;
-    // A product per head in one launch (form PER_HEAD): block z takes head z, whose
-    // columns of A start at z * head_a_cols, whose matrix is rows [z * w_rows, z * w_rows + N) of
-    // W and whose results go to columns z * head_c_cols + [0, N) of C.  K is a head's K; what a
-    // block of 64 columns of A holds beyond it meets columns of W outside its map, which read zero.
-    int heads, head_a_cols, head_c_cols;
-    // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2.  PER_HEAD, with `gate` set (up to
-    // GATED_ROWS rows): the results times the sigmoids of their logits before they are rounded, of one logit a row and head
-    // (GATE_HEAD: fp32 [M][heads]) or of one a result (GATE_RESULT: bf16 [M][heads * N]).
-    int act;
-    const void* gate;
-    int gate_ld;
-};
 constexpr int GATE_HEAD = 2, GATE_RESULT = 3;
 constexpr int GATED_ROWS = 16;          // rows of a product per head that takes a gate, at the most
 

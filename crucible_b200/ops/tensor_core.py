@@ -18,7 +18,8 @@ import torch
 
 from . import _stream, build
 
-build.register_module("gemm_tcgen05", ["common.cuh", "tc_common.cuh"])
+build.register_module("gemm_tcgen05", ["common.cuh", "tc_common.cuh", "gemm_args.cuh"])
+build.register_module("gemm_waves_tcgen05", ["common.cuh", "tc_common.cuh", "gemm_args.cuh"])
 build.register_module("attention_mma", ["common.cuh"])
 build.register_module("gemm_skinny_tcgen05", ["common.cuh", "tc_common.cuh"])
 build.register_module("attention_tcgen05", ["common.cuh", "tc_common.cuh"])
@@ -176,7 +177,7 @@ NORM_AHEAD_MAX_TILE = 128   # widest tile whose epilogue holds a row's sums in r
 
 
 class _NormArgs(ctypes.Structure):
-    """`NormArgs` of csrc/gemm_tcgen05.cu."""
+    """`NormArgs` of csrc/gemm_args.cuh."""
     _fields_ = [("gain", ctypes.c_void_p), ("scaled", ctypes.c_void_p), ("sumsq_out", ctypes.c_void_p),
                 ("ld_scaled", ctypes.c_int), ("sumsq_in", ctypes.c_void_p), ("parts", ctypes.c_int),
                 ("width", ctypes.c_float), ("eps", ctypes.c_float),
@@ -246,6 +247,50 @@ def _gemm(a, w, out, n, epi, bn, per_sm=1, splits=None, emit=None, pre=None, pai
         raise RuntimeError(f"tensor-core matrix product failed to launch (CUDA error {code})")
     if emit is not None:
         emit.parts = -(-n // bn)
+    _count(1)
+    return True
+
+
+WAVES_MIN_TILES = 200       # tiles of 128 x 256 from which one block an SM walks them (`_gemm_waves`)
+
+
+def _waves_width(m: int, n_cols: int, k: int, epi: int) -> int:
+    """The tile width with which a product runs through `_gemm_waves`, 0: not at all.  That kernel hides every
+    tile's way out behind the next tile's products, but has fewer stages, a longer start, and no second
+    accumulator row for tall tiles.  us at 2,048 rows, 128-row tiles or tall ones -> waves: the gated pair of
+    2 x 2,048 by K = 768 15.8 -> 13.3, of 2 x 2,816 by 2,048 43.2 -> 35.3; float32 results of 4,096
+    by 128 10.2 -> 8.6, of 50,304 by 768 204 -> 160.  From 1.35 waves on: at 1,100 rows of
+    2 x 2,816 (198 tiles) 23.7 -> 24.4.  bfloat16 results gain 3 to 7 % at the width that a block a tile would
+    have: with 256 columns from two waves on (8,192 by 2,048 at 1,100 / 1,600 rows 28.2 / 43.0 -> 26.4 / 39.9),
+    with 192 from three on or at a short K (2,048 rows of 5,120 by 2,048 34.0 -> 32.9, of 3,072 by 1,024 14.6 ->
+    13.6; two waves by 2,048, 1,100 rows of 4,608, 21.5 -> 21.9)."""
+    m_tiles = -(-m // 128)
+    waves = lambda bn: -(-m_tiles * -(-n_cols // bn) // N_SMS)
+    if epi == STORE_F32 and waves(256) > 1:
+        return min((waves(bn) * (bn + 64), bn) for bn in (192, 256))[1]
+    if epi == SWIGLU_BF16:
+        return 256 if m_tiles * -(-n_cols // 256) >= WAVES_MIN_TILES else 0
+    if epi == STORE_BF16:
+        bn = _tile_width(m, n_cols, epi)[0]
+        least = {256: 2, 192: 2 if k <= 1024 else 3}.get(bn)
+        return bn if least is not None and waves(bn) >= least else 0
+    return 0
+
+
+def _gemm_waves(a, w, out, n, epi, bn, pre=None, pair=None, act=0, plan=None) -> bool:
+    """The product with one block an SM over the tiles (`csrc/gemm_waves_tcgen05.cu`).  `plan`: the arguments of
+    a grouped product.  False: sizes it does not take."""
+    norm_ptr, keep = _norm_args(None, pre, a.shape[0], pair, act)
+    if plan is not None:
+        keep, norm_ptr = plan, ctypes.cast(ctypes.pointer(plan), _c_void_p)
+    code = build.load("gemm_waves_tcgen05").cb_gemm_waves(
+        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
+        _c_int(a.shape[0]), _c_int(n), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(-2)),
+        _c_int(out.stride(0)), _c_int(epi), _c_int(bn), _c_void_p(status_word(a.device).data_ptr()), _stream(), norm_ptr)
+    if code == _UNSUPPORTED:
+        return False
+    if code != 0:
+        raise RuntimeError(f"tensor-core product in waves failed to launch (CUDA error {code})")
     _count(1)
     return True
 
@@ -349,8 +394,12 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
         if pre is not None or act:
             return False
         return _gemm_skinny(a, w, out, w.shape[0], epi)
-    if tile is None and _tall_tiles(a.shape[0], w.shape[0], a.shape[1]):
-        tile = (256, 0)
+    if tile is None:
+        tall = _tall_tiles(a.shape[0], w.shape[0], a.shape[1])
+        waves = 0 if emit is not None or pre is not None or (tall and epi != STORE_F32) else _waves_width(a.shape[0], w.shape[0], a.shape[1], epi)
+        if waves and _gemm_waves(a, w, out, w.shape[0], epi, waves, act=act):
+            return True
+        tile = (256, 0) if tall else None
     bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(a.shape[0], w.shape[0], epi)
     return _gemm(a, w, out, w.shape[0], epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
 
@@ -387,8 +436,13 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     args = _NormArgs()
     if pair is not None:
         args.glu_limit, args.glu_alpha, args.glu_offset = (float(v) for v in pair)
-    bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, w.shape[1], gated)
     args.plan, args.n_experts, args.max_tiles, args.w_rows = plan.data_ptr(), n_experts, tiles, w.shape[1]
+    # (full tiles beside a half-filled one an expert: 4,096 pairs of 8 experts of 2,816 x 2,048 gate/up 99.8 -> 90.6 us,
+    # down 53.8 -> 49.2; 2,048 pairs 56.6 -> 53.8 and, below the line, 39.0 -> 45.7)
+    if (tile is None and (a.shape[0] / 128 + n_experts / 2) * -(-w.shape[1] // 256) >= WAVES_MIN_TILES
+            and a.shape[0] >= 64 * n_experts and _gemm_waves(a, w, out, n, epi, 256, plan=args)):
+        return True
+    bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, w.shape[1], gated)
     lib = build.load("gemm_tcgen05")
     code = lib.cb_gemm_tcgen05_grouped(
         _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
@@ -449,8 +503,11 @@ def linear_swiglu(h, gate_up, out, tile=None, pre=None, pair=None) -> bool:
         if pre is not None or pair is not None:      # (the few-row split product has the silu pair only)
             return False
         return _gemm_skinny(h, gate_up, out, inter, SWIGLU_BF16)
-    if tile is None and _tall_tiles(h.shape[0], 2 * inter, h.shape[1]):
-        tile = (256, 0)
+    if tile is None:
+        waves = _waves_width(h.shape[0], 2 * inter, h.shape[1], SWIGLU_BF16)
+        if waves and _gemm_waves(h, gate_up, out, inter, SWIGLU_BF16, waves, pre, pair):
+            return True
+        tile = (256, 0) if _tall_tiles(h.shape[0], 2 * inter, h.shape[1]) else None
     bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(h.shape[0], 2 * inter, SWIGLU_BF16)
     return _gemm(h, gate_up, out, inter, SWIGLU_BF16, bn, per_sm, splits[0] if splits else None, None, pre, pair)
 

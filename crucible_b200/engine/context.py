@@ -62,6 +62,7 @@ class CacheStorage:
         self.head_dim = head_dim
         self.value_dim = head_dim if value_dim is None else value_dim
         self.values_are_keys = values_are_keys
+        self._slots: Dict[int, tuple] = {}        # slot -> its keys and values
         if values_are_keys:
             # one row per token, read as key and as value: no pages for values
             self.kv = None
@@ -79,11 +80,18 @@ class CacheStorage:
             self._v = torch.zeros((n_slots, n_pages, kv_heads, page_tokens, self.value_dim),
                                   dtype=dtype, device=device)
 
+    def _slot(self, slot: int) -> tuple:
+        pair = self._slots.get(slot)
+        if pair is None:
+            pair = (self.kv[slot, 0], self.kv[slot, 1]) if self.kv is not None else (self._k[slot], self._v[slot])
+            self._slots[slot] = pair
+        return pair
+
     def keys(self, slot: int) -> torch.Tensor:
-        return self.kv[slot, 0] if self.kv is not None else self._k[slot]
+        return self._slot(slot)[0]
 
     def values(self, slot: int) -> torch.Tensor:
-        return self.kv[slot, 1] if self.kv is not None else self._v[slot]
+        return self._slot(slot)[1]
 
 
 class Scratch:
@@ -92,20 +100,29 @@ class Scratch:
 
     def __init__(self, device):
         self.device = device
-        self._flat: Dict[str, torch.Tensor] = {}
+        self._flat: Dict[tuple, torch.Tensor] = {}
+        self._views: Dict[tuple, torch.Tensor] = {}      # of the buffers as they are, by name, dtype and shape
         self.generation = 0          # bumped whenever a buffer moves
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
+        wanted = (name, dtype, *shape)
+        view = self._views.get(wanted)
+        if view is not None:
+            return view
         numel = 1
         for s in shape:
             numel *= int(s)
-        key = f"{name}:{dtype}"
+        key = (name, dtype)
         flat = self._flat.get(key)
         if flat is None or flat.numel() < numel:
             flat = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
             self._flat[key] = flat
             self.generation += 1
-        return flat[:numel].view(*shape)
+            self._views.clear()
+        if len(self._views) >= 1024:
+            self._views.clear()
+        view = self._views[wanted] = flat[:numel].view(*shape)
+        return view
 
     def reserve(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> None:
         self.get(name, shape, dtype)
@@ -155,6 +172,8 @@ class StepContext:
         [n_slots, state_bytes]; index it with `req_state_slot`."""
         if self._state is None or binding.state_bytes == 0:
             return None
+        if binding.state_offset == 0 and binding.state_bytes == self._state.shape[1]:
+            return self._state
         return self._state[:, binding.state_offset:binding.state_offset + binding.state_bytes]
 
     def scratch(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:

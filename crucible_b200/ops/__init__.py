@@ -14,7 +14,8 @@ the same function, so a row's result depends on the path only by rounding.
 """
 from __future__ import annotations
 
-import ctypes
+import bisect
+import weakref
 from typing import Optional
 
 import torch
@@ -22,7 +23,6 @@ import torch
 from . import build
 
 _F32, _BF16 = 0, 1
-_c_int, _c_float, _c_void_p = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
 
 
 class KernelError(RuntimeError):
@@ -37,14 +37,14 @@ def _code(dtype: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16 tensors, got {dtype}")
 
 
-def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
-    return _c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _stream() -> _c_void_p:
+def _stream() -> int:
     """The current stream of the current device.  (Asked of the bindings: `torch.cuda.current_stream()`
     makes a stream object and takes 10 us of the 20 that a launch cost the host.)"""
-    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*tensors) -> None:
@@ -101,8 +101,7 @@ def _check(code: int, what: str) -> None:
     _tick(what)
     if code != 0:
         lib = build.load("elementwise")
-        lib.cb_error_string.restype = ctypes.c_char_p
-        text = lib.cb_error_string(_c_int(code)).decode()
+        text = lib.cb_error_string(code).decode()
         raise KernelError(f"{what}: {text} (code {code})")
 
 
@@ -118,9 +117,9 @@ def embed_rows(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor,
         raise KernelError("embed_rows takes int32 ids and a float32 output")
     _contig(table, "embedding table"); _contig(out, "embed_rows output")
     lib = build.load("elementwise")
-    _check(lib.cb_embed_rows(_ptr(table), _c_int(_code(table.dtype)), _ptr(ids), _ptr(out),
-                             _c_int(ids.shape[0]), _c_int(table.shape[1]),
-                             _c_int(table.shape[0]), _ptr(device_tokens), _stream()), "embed_rows")
+    _check(lib.cb_embed_rows(_ptr(table), _code(table.dtype), _ptr(ids), _ptr(out),
+                             ids.shape[0], table.shape[1],
+                             table.shape[0], _ptr(device_tokens), _stream()), "embed_rows")
 
 
 def rmsnorm(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor) -> None:
@@ -129,8 +128,8 @@ def rmsnorm(x: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor) 
         raise KernelError("rmsnorm takes a float32 input and a float32 gain")
     _contig(x, "rmsnorm input"); _contig(out, "rmsnorm output")
     lib = build.load("elementwise")
-    _check(lib.cb_rmsnorm(_ptr(x), _ptr(gain), _ptr(out), _c_int(_code(out.dtype)),
-                          _c_int(x.shape[0]), _c_int(x.shape[1]), _c_float(eps), _stream()),
+    _check(lib.cb_rmsnorm(_ptr(x), _ptr(gain), _ptr(out), _code(out.dtype),
+                          x.shape[0], x.shape[1], eps, _stream()),
            "rmsnorm")
 
 
@@ -140,8 +139,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor) -> None:
         raise KernelError("swiglu takes [T, 2I] and writes [T, I] of the same dtype")
     _contig(gate_up, "swiglu input"); _contig(out, "swiglu output")
     lib = build.load("elementwise")
-    _check(lib.cb_swiglu(_ptr(gate_up), _ptr(out), _c_int(_code(out.dtype)),
-                         _c_int(out.shape[0]), _c_int(out.shape[1]), _stream()), "swiglu")
+    _check(lib.cb_swiglu(_ptr(gate_up), _ptr(out), _code(out.dtype),
+                         out.shape[0], out.shape[1], _stream()), "swiglu")
 
 
 def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor) -> None:
@@ -153,9 +152,9 @@ def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor)
     if z.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("polynorm: rows must be contiguous")
     lib = build.load("polynorm")
-    _check(lib.cb_polynorm(_ptr(z), _c_int(z.stride(0)), _ptr(coef), _ptr(out), _c_int(out.stride(0)),
-                           _c_int(_code(z.dtype)), _c_int(z.shape[0]), _c_int(z.shape[1]),
-                           _c_float(eps), _stream()), "polynorm")
+    _check(lib.cb_polynorm(_ptr(z), z.stride(0), _ptr(coef), _ptr(out), out.stride(0),
+                           _code(z.dtype), z.shape[0], z.shape[1],
+                           eps, _stream()), "polynorm")
 
 
 ACTIVATIONS = {"relu2": 0, "tanh": 1, "gelu_tanh": 2, "silu": 3}
@@ -169,9 +168,9 @@ def activation(kind: str, z: torch.Tensor, out: torch.Tensor) -> None:
     if z.shape != out.shape or z.dim() != 2 or z.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("activation takes rows [T, F] and writes the same shape")
     lib = build.load("activations")
-    _check(lib.cb_activation(_c_int(ACTIVATIONS[kind]), _ptr(z), _c_int(z.stride(0)), _c_int(_code(z.dtype)),
-                             _ptr(out), _c_int(out.stride(0)), _c_int(_code(out.dtype)),
-                             _c_int(z.shape[0]), _c_int(z.shape[1]), _stream()), f"activation {kind}")
+    _check(lib.cb_activation(ACTIVATIONS[kind], _ptr(z), z.stride(0), _code(z.dtype),
+                             _ptr(out), out.stride(0), _code(out.dtype),
+                             z.shape[0], z.shape[1], _stream()), f"activation {kind}")
 
 
 def glu(both: torch.Tensor, out: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0,
@@ -186,9 +185,9 @@ def glu(both: torch.Tensor, out: torch.Tensor, limit: Optional[float] = None, al
     if limit is not None and not limit > 0:
         raise KernelError("glu: the limit must be positive")
     lib = build.load("activations")
-    _check(lib.cb_glu(_ptr(both), _c_int(both.stride(0)), _ptr(out), _c_int(out.stride(0)),
-                      _c_int(_code(out.dtype)), _c_int(out.shape[0]), _c_int(out.shape[1]),
-                      _c_float(limit if limit is not None else 0.0), _c_float(alpha), _c_float(offset),
+    _check(lib.cb_glu(_ptr(both), both.stride(0), _ptr(out), out.stride(0),
+                      _code(out.dtype), out.shape[0], out.shape[1],
+                      limit if limit is not None else 0.0, alpha, offset,
                       _stream()), "glu")
 
 
@@ -210,12 +209,12 @@ def hashed_embedding(table, bigram, positions_table, ids, ctx, state, out, scale
         raise KernelError("hashed_embedding: the state is a uint8 view [slots, bytes], 4-byte aligned")
     lib = build.load("hashed_embedding")
     _check(lib.cb_hashed_embedding(
-        _ptr(table), _ptr(bigram), _ptr(positions_table), _c_int(_code(table.dtype)), _ptr(ids),
+        _ptr(table), _ptr(bigram), _ptr(positions_table), _code(table.dtype), _ptr(ids),
         _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot),
-        _ptr(state), ctypes.c_long(state.stride(0) if state is not None else 0), _ptr(out),
-        _c_int(ids.shape[0]), _c_int(table.shape[1]), _c_int(table.shape[0]), _c_float(scale),
-        _c_int(buckets), ctypes.c_longlong(mul_prev), ctypes.c_longlong(mul_cur),
-        _c_int(positions_table.shape[0] if positions_table is not None else 1), _ptr(device_tokens),
+        _ptr(state), state.stride(0) if state is not None else 0, _ptr(out),
+        ids.shape[0], table.shape[1], table.shape[0], scale,
+        buckets, mul_prev, mul_cur,
+        positions_table.shape[0] if positions_table is not None else 1, _ptr(device_tokens),
         _stream()), "hashed_embedding")
 
 
@@ -225,8 +224,8 @@ def gather_rows(x: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> None:
         raise KernelError("gather_rows takes float32 rows and int32 indices")
     _contig(x, "gather_rows input"); _contig(out, "gather_rows output")
     lib = build.load("elementwise")
-    _check(lib.cb_gather_rows(_ptr(x), _ptr(rows), _ptr(out), _c_int(out.shape[0]),
-                              _c_int(x.shape[1]), _stream()), "gather_rows")
+    _check(lib.cb_gather_rows(_ptr(x), _ptr(rows), _ptr(out), out.shape[0],
+                              x.shape[1], _stream()), "gather_rows")
 
 
 def add_vector(x: torch.Tensor, v: torch.Tensor) -> None:
@@ -237,7 +236,7 @@ def add_vector(x: torch.Tensor, v: torch.Tensor) -> None:
         raise KernelError("add_vector takes float32 rows [T, W] and a float32 vector [W]")
     _contig(x, "add_vector rows"); _contig(v, "add_vector vector")
     lib = build.load("elementwise")
-    _check(lib.cb_add_vector(_ptr(x), _ptr(v), _c_int(x.shape[0]), _c_int(x.shape[1]), _stream()),
+    _check(lib.cb_add_vector(_ptr(x), _ptr(v), x.shape[0], x.shape[1], _stream()),
            "add_vector")
 
 
@@ -251,7 +250,7 @@ def add_rows(x: torch.Tensor, rows: torch.Tensor, v: Optional[torch.Tensor] = No
     if v is not None:
         _contig(v, "add_rows vector")
     lib = build.load("elementwise")
-    _check(lib.cb_add_rows(_ptr(x), _ptr(rows), _ptr(v), _c_int(x.shape[0]), _c_int(x.shape[1]), _stream()),
+    _check(lib.cb_add_rows(_ptr(x), _ptr(rows), _ptr(v), x.shape[0], x.shape[1], _stream()),
            "add_rows")
 
 
@@ -262,7 +261,7 @@ def softcap(z: torch.Tensor, cap: float) -> None:
         raise KernelError("softcap takes float32 rows")
     _contig(z, "softcap rows")
     lib = build.load("elementwise")
-    _check(lib.cb_softcap(_ptr(z), _c_int(z.shape[0]), _c_int(z.shape[1]), _c_float(cap), _stream()),
+    _check(lib.cb_softcap(_ptr(z), z.shape[0], z.shape[1], cap, _stream()),
            "softcap")
 
 
@@ -284,10 +283,10 @@ def linear_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *,
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("linear: rows must be contiguous")
     lib = build.load("gemm_simt")
-    _check(lib.cb_gemm_simt(_ptr(a), _ptr(w), _ptr(out), _c_int(_code(a.dtype)),
-                            _c_int(_code(out.dtype)), _c_int(a.shape[0]), _c_int(w.shape[0]),
-                            _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(0)),
-                            _c_int(out.stride(0)), _c_int(1 if accumulate else 0), _stream()),
+    _check(lib.cb_gemm_simt(_ptr(a), _ptr(w), _ptr(out), _code(a.dtype),
+                            _code(out.dtype), a.shape[0], w.shape[0],
+                            a.shape[1], a.stride(0), w.stride(0),
+                            out.stride(0), 1 if accumulate else 0, _stream()),
            "linear (CUDA cores)")
 
 
@@ -303,10 +302,10 @@ def linear_heads_plain(a, a_head: int, w, out, out_head: int) -> None:
     if a.stride(1) != 1 or w.stride(2) != 1 or out.stride(1) != 1:
         raise KernelError("linear per head: rows must be contiguous")
     lib = build.load("gemm_simt")
-    _check(lib.cb_gemm_simt_heads(_ptr(a), _ptr(w), _ptr(out), _c_int(_code(a.dtype)), _c_int(_code(out.dtype)),
-                                  _c_int(a.shape[0]), _c_int(n), _c_int(k), _c_int(a.stride(0)), _c_int(w.stride(1)),
-                                  _c_int(out.stride(0)), _c_int(heads), _c_int(a_head), ctypes.c_long(w.stride(0)),
-                                  _c_int(out_head), _stream()), "linear per head (CUDA cores)")
+    _check(lib.cb_gemm_simt_heads(_ptr(a), _ptr(w), _ptr(out), _code(a.dtype), _code(out.dtype),
+                                  a.shape[0], n, k, a.stride(0), w.stride(1),
+                                  out.stride(0), heads, a_head, w.stride(0),
+                                  out_head, _stream()), "linear per head (CUDA cores)")
 
 
 # Device ranges that hold weights: tensors that no kernel of a step writes.  The bfloat16
@@ -322,8 +321,6 @@ _weight_ends: list = []
 def declare_weights(*tensors: Optional[torch.Tensor]) -> None:
     """Says that these tensors are written by no kernel of any step, for as long as the
     tensor objects given here live (the declaration goes with them)."""
-    import bisect
-    import weakref
     for t in tensors:
         if t is None or not t.is_cuda:
             continue
@@ -338,7 +335,6 @@ def declare_weights(*tensors: Optional[torch.Tensor]) -> None:
 
 
 def _forget_weight(start: int) -> None:
-    import bisect
     at = bisect.bisect_left(_weight_starts, start)
     if at < len(_weight_starts) and _weight_starts[at] == start:
         del _weight_starts[at]
@@ -346,7 +342,6 @@ def _forget_weight(start: int) -> None:
 
 
 def is_weight(t: torch.Tensor) -> bool:
-    import bisect
     p = t.data_ptr()
     at = bisect.bisect_right(_weight_starts, p) - 1
     return at >= 0 and p < _weight_ends[at]
@@ -360,12 +355,10 @@ def linear(a, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = False, c
     accumulating product is.  If the arrangement has announced the norm that reads those rows
     next (`StepContext.announce_norm`), the product may leave that norm's input beside its
     sums, and the norm then costs no kernel of its own."""
-    from . import small_batch
     if w.dtype == torch.bfloat16 and is_weight(w):
         if a.shape[0] <= small_batch.PREFERRED_ROWS and small_batch.linear(a, w, out, accumulate=accumulate):
             return
         a = small_batch.as_tensor(a)
-        from . import tensor_core
         emit = _norm_emit(closes, out, tensor_core) if accumulate and closes is not None else None
         if tensor_core.linear(a, w, out, accumulate=accumulate, emit=emit):
             if emit is not None and emit.parts:
@@ -383,12 +376,10 @@ def linear_act(h, w: torch.Tensor, out: torch.Tensor, kind: str) -> None:
     """out = act(h W^T): for a bfloat16 weight and an activation of `FUSED_ACTIVATIONS` one
     kernel (the activation in the product's epilogue, on the float32 sums, rounded once); else the
     product and then `activation` in place."""
-    from . import small_batch
     code = FUSED_ACTIVATIONS.get(kind, 0)
     if FUSE_ACTIVATION and code and w.dtype == torch.bfloat16 and is_weight(w) and out.dtype == torch.bfloat16:
         if h.shape[0] <= small_batch.PREFERRED_ROWS and small_batch.linear(h, w, out, act=code):
             return
-        from . import tensor_core
         if tensor_core.linear(small_batch.as_tensor(h), w, out, act=code):
             return
     linear(h, w, out)
@@ -409,18 +400,15 @@ def _norm_emit(ctx, rows: torch.Tensor, tensor_core):
 
 def _prenormed(h):
     """`h` if it carries a norm input that a product before it left, else None."""
-    from . import small_batch
     return h if isinstance(h, small_batch.LazyNorm) and h.scaled is not None else None
 
 
 def linear_swiglu(h, gate_up: torch.Tensor, out: torch.Tensor, ctx, pair=None) -> None:
     """out[T, I] = silu(h Wg^T) * (h Wu^T) with gate_up = [Wg; Wu] of shape [2I, d].  `pair` =
     (limit, alpha, offset): the capped gated pair of the two halves instead (see `glu`)."""
-    from . import small_batch
     if gate_up.dtype == torch.bfloat16 and is_weight(gate_up):
         if h.shape[0] <= small_batch.PREFERRED_ROWS and small_batch.linear_swiglu(h, gate_up, out, pair=pair):
             return
-        from . import tensor_core
         pre = _prenormed(h)
         if pre is not None and tensor_core.linear_swiglu(pre.scaled, gate_up, out, pre=pre, pair=pair):
             return
@@ -443,7 +431,6 @@ def qkv_rope_append(h, wqkv: torch.Tensor, qkv: torch.Tensor, n_heads: int, n_kv
     (tcgen05, rotation and cache write in the epilogue), two otherwise.  Leaves the
     rotated q in the first columns of `qkv`; the k and v columns of `qkv` are not
     defined afterwards (attention reads keys and values from the cache)."""
-    from . import small_batch
     if not is_weight(wqkv):
         linear(h, wqkv, qkv)
         rope_kv_append(qkv, n_heads, n_kv_heads, head_dim, cos, sin, rotary_dim, ctx, cache, binding)
@@ -453,7 +440,6 @@ def qkv_rope_append(h, wqkv: torch.Tensor, qkv: torch.Tensor, n_heads: int, n_kv
                                             rotary_dim, ctx, cache, binding)):
         return
     if wqkv.dtype == torch.bfloat16 and h.shape[0] > small_batch.PREFERRED_ROWS:
-        from . import tensor_core
         pre = _prenormed(h)
         if pre is not None and tensor_core.linear_rope_append(pre.scaled, wqkv, qkv, n_heads, n_kv_heads,
                                                               head_dim, cos, sin, rotary_dim, ctx, cache,
@@ -486,10 +472,10 @@ def rope_kv_append(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: i
     table = ctx.block_table(binding.group)
     lib = build.load("elementwise")
     _check(lib.cb_rope_kv_append(
-        _ptr(qkv), _c_int(_code(qkv.dtype)), _ptr(cos), _ptr(sin), _c_int(rotary_dim),
-        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]),
-        _ptr(k_cache), _ptr(v_cache), _c_int(qkv.shape[0]), _c_int(n_heads), _c_int(n_kv_heads),
-        _c_int(head_dim), _c_int(cache.page_tokens), _c_int(1 if binding.write else 0),
+        _ptr(qkv), _code(qkv.dtype), _ptr(cos), _ptr(sin), rotary_dim,
+        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1],
+        _ptr(k_cache), _ptr(v_cache), qkv.shape[0], n_heads, n_kv_heads,
+        head_dim, cache.page_tokens, 1 if binding.write else 0,
         _stream()), "rope_kv_append")
 
 
@@ -509,12 +495,12 @@ def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, ke
         return False
     lib = build.load("attention_f32")
     code = lib.cb_attention_f32(
-        _ptr(q), _c_int(q.stride(0)), _ptr(gate), _c_int(gate.stride(0) if gate is not None else 0), _ptr(out),
-        _c_int(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(sinks), _ptr(ctx.req_row_start),
-        _ptr(ctx.req_first_pos), _ptr(table), _c_int(table.shape[1]), _c_int(ctx.n_requests),
-        _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim), _c_int(value_dim),
-        _c_int(page_tokens), _c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first),
-        _c_float(out_scale), _c_int(1 if gate_per_head else 0), _stream())
+        _ptr(q), q.stride(0), _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(out),
+        out.stride(0), _ptr(k_cache), _ptr(v_cache), _ptr(sinks), _ptr(ctx.req_row_start),
+        _ptr(ctx.req_first_pos), _ptr(table), table.shape[1], ctx.n_requests,
+        host.max_new_tokens, n_heads, n_kv_heads, key_dim, value_dim,
+        page_tokens, scale, window or 0, 1 if chunked else 0, keep_first,
+        out_scale, 1 if gate_per_head else 0, _stream())
     if code == build.UNSUPPORTED:
         return False
     _check(code, "attention (32-bit tiles)")
@@ -531,17 +517,16 @@ def paged_attention_plain(qkv, out, n_heads, n_kv_heads, head_dim, scale, window
         return
     lib = build.load("attention_generic")
     _check(lib.cb_attention_generic(
-        _ptr(qkv), _c_int(qkv.stride(0)), _ptr(out), _c_int(out.stride(0)), _ptr(k_cache),
-        _ptr(v_cache), _c_int(_code(qkv.dtype)), _ptr(ctx.positions), _ptr(ctx.row_request),
-        _ptr(table), _c_int(table.shape[1]), _c_int(qkv.shape[0]), _c_int(n_heads),
-        _c_int(n_kv_heads), _c_int(head_dim), _c_int(cache.page_tokens), _c_float(scale),
-        _c_int(window or 0), _stream()), "paged attention (plain)")
+        _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), _ptr(k_cache),
+        _ptr(v_cache), _code(qkv.dtype), _ptr(ctx.positions), _ptr(ctx.row_request),
+        _ptr(table), table.shape[1], qkv.shape[0], n_heads,
+        n_kv_heads, head_dim, cache.page_tokens, scale,
+        window or 0, _stream()), "paged attention (plain)")
 
 
 def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx, cache,
                     binding) -> None:
     if qkv.dtype == torch.bfloat16:
-        from . import tensor_core
         if tensor_core.paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window,
                                        ctx, cache, binding):
             return
@@ -556,7 +541,7 @@ def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx,
 def _status_pair(status):
     """(source, destination) pointers of a status relay, or two nulls."""
     if status is None:
-        return _c_void_p(0), _c_void_p(0)
+        return 0, 0
     src, dst = status
     _need_cuda(src, dst)
     if src.dtype != torch.int32 or dst.dtype != torch.int32:
@@ -587,7 +572,7 @@ def argmax_rows(logits: torch.Tensor, out_ids: torch.Tensor,
     if counters is None or counters.numel() < n:
         counters = torch.zeros(max(n, 1024), dtype=torch.int32, device=logits.device)
         _scratch[key + ("counters",)] = counters
-    _check(lib.cb_argmax_rows(_ptr(logits), _c_int(n), _c_int(logits.shape[1]),
+    _check(lib.cb_argmax_rows(_ptr(logits), n, logits.shape[1],
                               _ptr(out_ids), _ptr(scratch), _ptr(scatter_index), _ptr(scatter_out),
                               *_status_pair(status), _stream(), _ptr(counters)), "argmax_rows")
 
@@ -607,11 +592,14 @@ def sample_rows(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Te
         raise KernelError("sample_rows: wrong tensor dtypes")
     _contig(logits, "logits")
     lib = build.load("sampling")
-    code = lib.cb_sample_rows(_ptr(logits), _c_int(logits.shape[0]), _c_int(logits.shape[1]),
-                              _ptr(temperature), _ptr(top_k), _ptr(uniform), _c_int(max_top_k),
+    code = lib.cb_sample_rows(_ptr(logits), logits.shape[0], logits.shape[1],
+                              _ptr(temperature), _ptr(top_k), _ptr(uniform), max_top_k,
                               _ptr(out_ids), _ptr(scatter_index), _ptr(scatter_out),
                               *_status_pair(status), _stream())
     if code == 100001:
         raise KernelError(f"top_k {max_top_k} exceeds what the sampling kernel holds "
                           f"({max_device_top_k()} candidates)")
     _check(code, "sample_rows")
+
+
+from . import small_batch, tensor_core  # noqa: E402  (they take what stands above)

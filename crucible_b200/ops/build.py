@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -156,11 +157,47 @@ def library_path(name: str) -> str:
     return target
 
 
+_C_TYPES = {"int": ctypes.c_int, "long": ctypes.c_long, "long long": ctypes.c_longlong, "float": ctypes.c_float}
+
+
+def signatures(text: str) -> Dict[str, tuple]:
+    """name -> (result, [parameters]) as ctypes, of every entry point that a kernel source exports."""
+    out = {}
+    text = re.sub(r"//[^\n]*", "", text)
+    for result, name, params in re.findall(r"^CB_EXPORT\s+([^(]*?)(\w+)\s*\(([^)]*)\)", text, re.M):
+        kinds = []
+        for p in params.replace("\n", " ").split(","):
+            p = re.sub(r"\bconst\b|\b__restrict__\b", "", p).strip()
+            if not p or p == "void":
+                continue
+            kind = ctypes.c_void_p if "*" in p else _C_TYPES.get(" ".join(p.split()[:-1]))
+            if kind is None:
+                raise BuildError(f"{name}: parameter {p!r} is of no type that the wrappers pass")
+            kinds.append(kind)
+        result = result.strip()
+        kind = ctypes.c_char_p if "char" in result else None if result == "void" else _C_TYPES.get(result)
+        if kind is None and result != "void":
+            raise BuildError(f"{name}: result {result!r} is of no type that the wrappers take")
+        out[name] = kind, kinds
+    return out
+
+
 def load(name: str) -> ctypes.CDLL:
+    """The library of module `name`.  A kernel source's entry points know their parameters' types, read off
+    the source's own declarations, so that the wrappers pass plain numbers and addresses: a launch
+    passes some twenty, and an object made for each cost the host 2 to 3 us."""
+    lib = _loaded.get(name)
+    if lib is not None:
+        return lib
     with _lock:
         lib = _loaded.get(name)
         if lib is None:
             lib = ctypes.CDLL(library_path(name))
+            if name not in HOST_SOURCES:
+                with open(os.path.join(CSRC, _source(name))) as f:
+                    for entry, (result, kinds) in signatures(f.read()).items():
+                        fn = getattr(lib, entry)
+                        fn.restype, fn.argtypes = result, kinds
             _loaded[name] = lib
         return lib
 

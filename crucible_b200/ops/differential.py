@@ -7,7 +7,7 @@ from typing import Optional
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, build
+from . import KernelError, _check, _code, _need_cuda, _ptr, _stream, build
 
 
 def prepare(proj, bias: Optional[torch.Tensor], coef: float, every: int, qx, n_heads: int, n_kv_heads: int,
@@ -30,11 +30,11 @@ def prepare(proj, bias: Optional[torch.Tensor], coef: float, every: int, qx, n_h
     table = ctx.block_table(binding.group)
     lib = build.load("differential")
     _check(lib.cb_differential_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(bias), _c_float(coef), _c_int(every),
-        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]), _ptr(qx),
-        _c_int(qx.stride(0)), _ptr(k_cache), _ptr(v_cache), _c_int(proj.shape[0]), _c_int(n_heads),
-        _c_int(n_kv_heads), _c_int(dim), _c_int(value_dim), _c_int(cache.page_tokens),
-        _c_int(1 if binding.write else 0), _stream()), "differential_prepare")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(bias), coef, every,
+        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1], _ptr(qx),
+        qx.stride(0), _ptr(k_cache), _ptr(v_cache), proj.shape[0], n_heads,
+        n_kv_heads, dim, value_dim, cache.page_tokens,
+        1 if binding.write else 0, _stream()), "differential_prepare")
 
 
 def combine(a, lam: float, eps: float, scale: float, out, out_bias: Optional[torch.Tensor], residual,
@@ -51,7 +51,7 @@ def combine(a, lam: float, eps: float, scale: float, out, out_bias: Optional[tor
         raise KernelError("differential combine: a float32 bias as wide as the float32 residual rows")
     lib = build.load("differential")
     _check(lib.cb_differential_combine(
-        _ptr(a), _c_int(a.stride(0)), _c_int(_code(a.dtype)), _c_float(lam), _c_float(eps), _c_float(scale),
-        _ptr(out), _c_int(out.stride(0)), _ptr(out_bias), _ptr(residual),
-        _c_int(residual.shape[1] if residual is not None else 0), _c_int(a.shape[0]), _c_int(n_heads),
-        _c_int(value_dim), _stream()), "differential_combine")
+        _ptr(a), a.stride(0), _code(a.dtype), lam, eps, scale,
+        _ptr(out), out.stride(0), _ptr(out_bias), _ptr(residual),
+        residual.shape[1] if residual is not None else 0, a.shape[0], n_heads,
+        value_dim, _stream()), "differential_combine")

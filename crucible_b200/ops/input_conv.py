@@ -4,8 +4,8 @@ from __future__ import annotations
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _contig, _need_cuda, _ptr, _stream, build
-from .recurrent import _c_long, _state_args
+from . import KernelError, _check, _code, _contig, _need_cuda, _ptr, _stream, build
+from .recurrent import _state_args
 
 
 def norm_conv(x, gain, eps: float, taps_weight, ctx, state, tail_off: int, out) -> None:
@@ -20,13 +20,13 @@ def norm_conv(x, gain, eps: float, taps_weight, ctx, state, tail_off: int, out) 
     for t, what in ((x, "rows"), (gain, "gain"), (taps_weight, "taps"), (out, "output")):
         _contig(t, "norm_conv " + what)
     taps = taps_weight.shape[0]
-    sp, stride = _ptr(None), _c_long(0)
+    sp, stride = _ptr(None), 0
     if taps > 1:
         sp, stride = _state_args(state)
         if state.shape[1] < tail_off + 4 * (taps - 1) * x.shape[1]:
             raise KernelError("norm_conv: the state is too small for the convolution's inputs")
     lib = build.load("input_conv")
     _check(lib.cb_norm_conv(
-        _ptr(x), _ptr(gain), _c_float(eps), _ptr(taps_weight), _c_int(taps), _ptr(ctx.req_row_start),
-        _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(out), _c_int(_code(out.dtype)),
-        _c_int(ctx.n_requests), _c_int(ctx.host.max_new_tokens), _c_int(x.shape[1]), _stream()), "norm_conv")
+        _ptr(x), _ptr(gain), eps, _ptr(taps_weight), taps, _ptr(ctx.req_row_start),
+        _ptr(ctx.req_state_slot), sp, stride, tail_off, _ptr(out), _code(out.dtype),
+        ctx.n_requests, ctx.host.max_new_tokens, x.shape[1], _stream()), "norm_conv")

@@ -9,7 +9,6 @@ box's height).  The tensor-core kernels' loops are shaped by these figures: for 
 """
 from __future__ import annotations
 
-import ctypes
 
 import torch
 
@@ -18,12 +17,12 @@ from . import build, tensor_core
 build.register_module("issue_probe", ["common.cuh", "tc_common.cuh"])
 
 
-def _vp(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr())
+def _vp(t) -> int:
+    return t.data_ptr()
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    return torch.cuda.current_stream().cuda_stream
 
 
 def mma_send_cycles(m: int, n: int, count: int = 1025, tight: bool = True, device="cuda:0") -> float:
@@ -32,8 +31,8 @@ def mma_send_cycles(m: int, n: int, count: int = 1025, tight: bool = True, devic
     out = torch.zeros(1, dtype=torch.int64, device=device)
     status = tensor_core.status_word(device)
     for _ in range(2):                                   # the first launch also loads the code
-        code = lib.cb_probe_mma_send(ctypes.c_int(m), ctypes.c_int(n), ctypes.c_int(count),
-                                     ctypes.c_int(1 if tight else 0), _vp(out), _vp(status), _stream())
+        code = lib.cb_probe_mma_send(m, n, count,
+                                     1 if tight else 0, _vp(out), _vp(status), _stream())
         if code != 0:
             raise RuntimeError(f"the MMA probe was refused or failed to launch (code {code})")
         torch.cuda.synchronize(device)
@@ -49,8 +48,8 @@ def tma_send_cycles(rows: int, count: int = 32, device="cuda:0"):
     out = torch.zeros(2, dtype=torch.int64, device=device)
     status = tensor_core.status_word(device)
     for _ in range(2):
-        code = lib.cb_probe_tma_send(_vp(matrix), ctypes.c_int(256), ctypes.c_int(2048), ctypes.c_int(rows),
-                                     ctypes.c_int(count), _vp(out), _vp(status), _stream())
+        code = lib.cb_probe_tma_send(_vp(matrix), 256, 2048, rows,
+                                     count, _vp(out), _vp(status), _stream())
         if code != 0:
             raise RuntimeError(f"the TMA probe was refused or failed to launch (code {code})")
         torch.cuda.synchronize(device)

@@ -4,7 +4,8 @@ from __future__ import annotations
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, build
+from . import (KernelError, _check, _code, _need_cuda, _ptr, _stream, build, is_weight, linear, linear_heads_plain,
+               tensor_core)
 
 
 def prepare(dkv, q, qx, gain, freq, mscale: float, eps: float, n_heads: int, dim: int, rank: int,
@@ -30,12 +31,12 @@ def prepare(dkv, q, qx, gain, freq, mscale: float, eps: float, n_heads: int, dim
     table = ctx.block_table(binding.group)
     lib = build.load("latent_attention")
     _check(lib.cb_latent_prepare(
-        _ptr(dkv), _c_int(dkv.stride(0) if dkv is not None else 0), _ptr(q),
-        _c_int(q.stride(0) if q is not None else 0), _ptr(qx), _c_int(qx.stride(0) if qx is not None else 0),
-        _c_int(_code(rows[0].dtype)), _ptr(gain), _ptr(freq), _c_float(mscale), _c_float(eps),
-        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]), _ptr(pages),
-        _c_int(rows[0].shape[0]), _c_int(n_heads), _c_int(dim), _c_int(rank), _c_int(rot), _c_int(turned),
-        _c_int(cache.page_tokens), _c_int(1 if binding.write else 0), _c_int(1 if split_halves else 0),
+        _ptr(dkv), dkv.stride(0) if dkv is not None else 0, _ptr(q),
+        q.stride(0) if q is not None else 0, _ptr(qx), qx.stride(0) if qx is not None else 0,
+        _code(rows[0].dtype), _ptr(gain), _ptr(freq), mscale, eps,
+        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1], _ptr(pages),
+        rows[0].shape[0], n_heads, dim, rank, rot, turned,
+        cache.page_tokens, 1 if binding.write else 0, 1 if split_halves else 0,
         _stream()), "latent_prepare")
 
 
@@ -47,9 +48,9 @@ def head_gate(x, logit, n_heads: int, head_width: int) -> None:
             or x.shape[1] != n_heads * head_width or logit.shape[1] != n_heads):
         raise KernelError("head_gate: rows [T, heads * width] and logits [T, heads], float32 or the rows' dtype")
     lib = build.load("latent_attention")
-    _check(lib.cb_head_gate(_ptr(x), _c_int(x.stride(0)), _c_int(_code(x.dtype)), _ptr(logit),
-                            _c_int(_code(logit.dtype)), _c_int(logit.stride(0)), _c_int(x.shape[0]),
-                            _c_int(n_heads), _c_int(head_width), _stream()), "head_gate")
+    _check(lib.cb_head_gate(_ptr(x), x.stride(0), _code(x.dtype), _ptr(logit),
+                            _code(logit.dtype), logit.stride(0), x.shape[0],
+                            n_heads, head_width, _stream()), "head_gate")
 
 
 def rows_gate(x, g) -> None:
@@ -58,8 +59,8 @@ def rows_gate(x, g) -> None:
     if x.shape != g.shape or x.dtype != g.dtype or x.stride(1) != 1 or g.stride(1) != 1:
         raise KernelError("rows_gate: rows and logits of one shape and dtype")
     lib = build.load("latent_attention")
-    _check(lib.cb_rows_gate(_ptr(x), _c_int(x.stride(0)), _ptr(g), _c_int(g.stride(0)), _c_int(_code(x.dtype)),
-                            _c_int(x.shape[0]), _c_int(x.shape[1]), _stream()), "rows_gate")
+    _check(lib.cb_rows_gate(_ptr(x), x.stride(0), _ptr(g), g.stride(0), _code(x.dtype),
+                            x.shape[0], x.shape[1], _stream()), "rows_gate")
 
 
 WARP_ROWS = 2        # steps of up to this many rows take a warp per weight row ...
@@ -81,12 +82,10 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
     `gate_logit` (float32 [rows, heads]): every head's results times sigmoid(logit), before they are
     rounded in the one launch of up to SMALL_ROWS rows, by `head_gate` otherwise.  `gate_rows` (rows of the
     activations' dtype, [rows, heads * N]): every result times the sigmoid of its own logit, likewise."""
-    from . import linear, linear_heads_plain
     heads, n, k = w.shape
     if gate_rows is not None and (out_head != n or gate_rows.shape != (a.shape[0], heads * n)
                                   or gate_rows.dtype != out.dtype or gate_rows.stride(1) != 1):
         raise KernelError("heads_linear: gate rows are [rows, heads * N] of the results' dtype")
-    from . import is_weight, tensor_core
     rows = a.shape[0]
     # the gate that the tiles take with them: few rows, of one kind, its logits side by side (few rows with
     # another are the warps', which take any)
@@ -105,13 +104,13 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate_logit=None, gate_ro
         if a.stride(1) != 1 or out.stride(1) != 1 or not w.is_contiguous() or out.dtype != a.dtype:
             raise KernelError("heads_linear: contiguous rows of one dtype and contiguous weights")
         lib = build.load("latent_attention")
-        _check(lib.cb_heads_linear_small(_ptr(a), _c_int(a.stride(0)), _c_int(a_head), _ptr(w), _ptr(out),
-                                         _c_int(out.stride(0)), _c_int(out_head), _c_int(_code(a.dtype)),
-                                         _c_int(rows), _c_int(heads), _c_int(n), _c_int(k),
+        _check(lib.cb_heads_linear_small(_ptr(a), a.stride(0), a_head, _ptr(w), _ptr(out),
+                                         out.stride(0), out_head, _code(a.dtype),
+                                         rows, heads, n, k,
                                          _ptr(gate_logit),
-                                         _c_int(gate_logit.stride(0) if gate_logit is not None else 0),
+                                         gate_logit.stride(0) if gate_logit is not None else 0,
                                          _ptr(gate_rows),
-                                         _c_int(gate_rows.stride(0) if gate_rows is not None else 0),
+                                         gate_rows.stride(0) if gate_rows is not None else 0,
                                          _stream()),
                "heads_linear (few rows)")
         return

@@ -7,7 +7,7 @@ from typing import Optional, Sequence, Tuple
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _contig, _need_cuda, _ptr, _stream, build
+from . import KernelError, _check, _code, _contig, _need_cuda, _ptr, _stream, build
 
 
 @dataclass
@@ -49,10 +49,10 @@ def close(x: torch.Tensor, mixer: Optional[torch.Tensor], s1: Optional[torch.Ten
     padded = list(norms) + [(None, 0.0, None)] * (2 - len(norms))
     lib = build.load("layer_close")
     _check(lib.cb_layer_close(
-        _ptr(x), _ptr(mixer), _ptr(s1), _ptr(s2), _ptr(o.rows), _c_int(o.top), _ptr(plan), _ptr(idx), _ptr(place),
-        _ptr(weight), _ptr(o.shared), _ptr(o.gate), _c_int(len(norms)),
-        *(a for g, eps, out in padded for a in (_ptr(g), _c_float(eps), _ptr(out))),
-        _c_int(_code(outs[0].dtype) if outs else 0), _c_int(x.shape[0]), _c_int(width), _stream()), "layer close")
+        _ptr(x), _ptr(mixer), _ptr(s1), _ptr(s2), _ptr(o.rows), o.top, _ptr(plan), _ptr(idx), _ptr(place),
+        _ptr(weight), _ptr(o.shared), _ptr(o.gate), len(norms),
+        *(a for g, eps, out in padded for a in (_ptr(g), eps, _ptr(out))),
+        _code(outs[0].dtype) if outs else 0, x.shape[0], width, _stream()), "layer close")
 
 
 def swap_rows(x: torch.Tensor, rows_out: torch.Tensor, next_rows: Optional[torch.Tensor] = None) -> None:
@@ -65,5 +65,5 @@ def swap_rows(x: torch.Tensor, rows_out: torch.Tensor, next_rows: Optional[torch
         if t is not None:
             _contig(t, "swap_rows rows")
     lib = build.load("layer_close")
-    _check(lib.cb_swap_rows(_ptr(x), _ptr(rows_out), _c_int(_code(rows_out.dtype)), _ptr(next_rows),
-                            _c_int(x.shape[0]), _c_int(x.shape[1]), _stream()), "swap_rows")
+    _check(lib.cb_swap_rows(_ptr(x), _ptr(rows_out), _code(rows_out.dtype), _ptr(next_rows),
+                            x.shape[0], x.shape[1], _stream()), "swap_rows")

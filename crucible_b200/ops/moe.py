@@ -2,11 +2,9 @@
 products over those tiles, and the sum of a token's chosen experts."""
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
-from . import KernelError, _c_int, _check, _code, _need_cuda, _ptr, _stream, build
+from . import KernelError, _check, _code, _need_cuda, _ptr, _stream, build, tensor_core
 
 
 def tile_rows() -> int:
@@ -29,7 +27,7 @@ def plan_ints(n_experts: int, tiles: int) -> int:
 def _pair(pair):
     """(limit, alpha, offset) of the capped gated pair as C floats; None: silu(g) * u."""
     limit, alpha, offset = pair if pair is not None else (0.0, 1.0, 0.0)
-    return ctypes.c_float(limit), ctypes.c_float(alpha), ctypes.c_float(offset)
+    return limit, alpha, offset
 
 
 def route(logits, top: int, idx, weight, place, count, plan, tiles: int, sorted_pair, bias=None,
@@ -65,11 +63,11 @@ def route(logits, top: int, idx, weight, place, count, plan, tiles: int, sorted_
         raise KernelError("moe route: a buffer is too small")
     lib = build.load("moe")
     count_g, keep_g = groups if groups is not None else (1, 1)
-    _check(lib.cb_moe_route(_ptr(logits), _c_int(logits.shape[1]), _ptr(bias), _c_int(t), _c_int(e), _c_int(top),
-                            _ptr(idx), _ptr(weight), _ptr(place), _ptr(count), _ptr(plan), _c_int(tiles),
-                            _ptr(sorted_pair), _c_int(rows), _c_int(count_g), _c_int(keep_g), _c_int(n_shared),
-                            _c_int(gate_col), ctypes.c_float(scale), _ptr(gate_out), _c_int(1 if sigmoid else 0),
-                            _c_int(1 if group_best_two else 0), _ptr(correction), _stream()), "moe route")
+    _check(lib.cb_moe_route(_ptr(logits), logits.shape[1], _ptr(bias), t, e, top,
+                            _ptr(idx), _ptr(weight), _ptr(place), _ptr(count), _ptr(plan), tiles,
+                            _ptr(sorted_pair), rows, count_g, keep_g, n_shared,
+                            gate_col, scale, _ptr(gate_out), 1 if sigmoid else 0,
+                            1 if group_best_two else 0, _ptr(correction), _stream()), "moe route")
 
 
 def expert_tiles(gated: bool, a, w, n_out: int, plan, n_experts: int, tiles: int, sorted_pair, top: int,
@@ -83,11 +81,11 @@ def expert_tiles(gated: bool, a, w, n_out: int, plan, n_experts: int, tiles: int
     if (not gated) and out.dtype != torch.float32:
         raise KernelError("moe tiles: the down product writes float32")
     lib = build.load("moe")
-    _check(lib.cb_moe_tiles(_c_int(1 if gated else 0), _ptr(a), _c_int(a.stride(0)), _ptr(w),
-                            ctypes.c_long(w.stride(0)), _c_int(_code(a.dtype)), _c_int(n_out),
-                            _c_int(w.shape[2]), _ptr(plan), _c_int(n_experts), _c_int(tiles),
-                            _ptr(sorted_pair), _c_int(top), _ptr(weight), _ptr(out),
-                            _c_int(out.stride(0)), *_pair(pair), _stream()),
+    _check(lib.cb_moe_tiles(1 if gated else 0, _ptr(a), a.stride(0), _ptr(w),
+                            w.stride(0), _code(a.dtype), n_out,
+                            w.shape[2], _ptr(plan), n_experts, tiles,
+                            _ptr(sorted_pair), top, _ptr(weight), _ptr(out),
+                            out.stride(0), *_pair(pair), _stream()),
            "moe gate/up" if gated else "moe down")
 
 
@@ -99,11 +97,11 @@ def expert_rows_small(gated: bool, a, w, n_out: int, plan, n_experts: int, tiles
     if a.dtype != w.dtype or a.stride(1) != 1 or not w.is_contiguous() or out.stride(1) != 1:
         raise KernelError("moe rows: rows and weights of one dtype, contiguous rows")
     lib = build.load("moe")
-    code = lib.cb_moe_rows_small(_c_int(1 if gated else 0), _ptr(a), _c_int(a.stride(0)), _ptr(w),
-                                 ctypes.c_long(w.stride(0)), _c_int(_code(a.dtype)), _c_int(n_out),
-                                 _c_int(w.shape[2]), _ptr(plan), _c_int(n_experts), _c_int(tiles),
-                                 _ptr(sorted_pair), _c_int(top), _ptr(weight), _ptr(out),
-                                 _c_int(out.stride(0)), *_pair(pair), _stream())
+    code = lib.cb_moe_rows_small(1 if gated else 0, _ptr(a), a.stride(0), _ptr(w),
+                                 w.stride(0), _code(a.dtype), n_out,
+                                 w.shape[2], _ptr(plan), n_experts, tiles,
+                                 _ptr(sorted_pair), top, _ptr(weight), _ptr(out),
+                                 out.stride(0), *_pair(pair), _stream())
     if code == 100001:
         return False
     _check(code, "moe gate/up (few rows)" if gated else "moe down (few rows)")
@@ -123,8 +121,8 @@ def combine(rows, top: int, residual, by_plan=None, shared=None, gate=None) -> N
                                         or not shared.is_contiguous() or (gate is not None and gate.dtype != torch.float32)))):
         raise KernelError("moe combine adds float32 rows into the float32 residual")
     lib = build.load("moe")
-    _check(lib.cb_moe_combine(_ptr(rows), _c_int(top), _ptr(residual), _c_int(residual.shape[0]),
-                              _c_int(residual.shape[1]), _ptr(plan), _ptr(idx), _ptr(place), _ptr(weight),
+    _check(lib.cb_moe_combine(_ptr(rows), top, _ptr(residual), residual.shape[0],
+                              residual.shape[1], _ptr(plan), _ptr(idx), _ptr(place), _ptr(weight),
                               _ptr(shared), _ptr(gate), _stream()), "moe combine")
 
 
@@ -132,8 +130,8 @@ def gather(h, sorted_pair, top: int, out) -> None:
     """out[i] = h[token of the i-th pair in sorted order]."""
     _need_cuda(h, sorted_pair, out)
     lib = build.load("moe")
-    _check(lib.cb_moe_gather(_ptr(h), _c_int(h.stride(0)), _c_int(_code(h.dtype)), _ptr(sorted_pair),
-                             _c_int(top), _ptr(out), _c_int(out.shape[0]), _c_int(h.shape[1]), _stream()),
+    _check(lib.cb_moe_gather(_ptr(h), h.stride(0), _code(h.dtype), _ptr(sorted_pair),
+                             top, _ptr(out), out.shape[0], h.shape[1], _stream()),
            "moe gather")
 
 
@@ -142,5 +140,4 @@ def grouped_linear(rows_sorted, w, out, plan, n_experts: int, tiles: int, gated:
     the device (tiles of `GROUPED_TILE_ROWS` rows): out[i] = rows_sorted[i] . W[expert of row i]^T
     with w [experts, N, K]; gated: w [experts, 2 F, K] and out [pairs, F] = the gated pair of
     the two halves (`pair`: the capped form).  False: the sizes do not allow it."""
-    from . import tensor_core
     return tensor_core.grouped_linear(rows_sorted, w, out, plan, n_experts, tiles, gated, pair)

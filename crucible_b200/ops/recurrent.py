@@ -3,14 +3,12 @@ token in the request's state slot (the gated delta rule, the mLSTM, the wkv rule
 state-space rule, the delta rule with a decay per key channel)."""
 from __future__ import annotations
 
-import ctypes
 import functools
 
 import torch
 
-from . import LAUNCHES, KernelError, _c_float, _c_int, _c_void_p, _check, _code, _need_cuda, _ptr, _stream, build
+from . import LAUNCHES, KernelError, _check, _code, _need_cuda, _ptr, _stream, build
 
-_c_long = ctypes.c_long
 DELTA, MLSTM, WKV, SSD, CHANNEL = 0, 1, 2, 3, 4
 GATE_SILU, GATE_SIGMOID = 0, 1
 CHUNKS = True                # tests switch it off to reach the token-by-token walk with the same inputs
@@ -93,7 +91,7 @@ def _state_args(state: torch.Tensor):
         raise KernelError("a mixer's state is a uint8 view [slots, bytes]")
     if state.data_ptr() % 16:
         raise KernelError("a mixer's state must start on a 16-byte boundary")
-    return _ptr(state), _c_long(state.stride(0))
+    return _ptr(state), state.stride(0)
 
 
 def delta_prepare(proj, conv_w, taps, gates, a_log, dt_bias, ctx, state, tail_off, qkv, beta,
@@ -107,11 +105,11 @@ def delta_prepare(proj, conv_w, taps, gates, a_log, dt_bias, ctx, state, tail_of
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_delta_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(conv_w), _c_int(taps),
-        _ptr(gates), _c_int(gates.stride(0)), _ptr(a_log), _ptr(dt_bias), _ptr(ctx.row_request), _ptr(ctx.req_row_start),
-        _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(qkv), _ptr(beta), _ptr(decay),
-        _c_int(proj.shape[0]), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim),
-        _c_int(value_dim), _stream()), "delta_prepare")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(conv_w), taps,
+        _ptr(gates), gates.stride(0), _ptr(a_log), _ptr(dt_bias), _ptr(ctx.row_request), _ptr(ctx.req_row_start),
+        _ptr(ctx.req_state_slot), sp, stride, tail_off, _ptr(qkv), _ptr(beta), _ptr(decay),
+        proj.shape[0], n_heads, n_kv_heads, key_dim,
+        value_dim, _stream()), "delta_prepare")
     return False
 
 
@@ -126,11 +124,11 @@ def _conv_prepare(proj, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx, state,
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     code = lib.cb_conv_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(conv_w), _ptr(conv_b), _c_int(taps),
-        _ptr(gates), _c_int(gates.stride(0)), _ptr(a_log), _ptr(dt_bias), _ptr(ctx.req_row_start),
-        _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(dst), _ptr(num0), _ptr(num1),
-        _c_int(ctx.n_requests), _c_int(host.max_new_tokens), _c_int(n_heads), _c_int(channels), _c_int(unit_heads),
-        _c_int(head_size), _c_int(1 if is_ssd else 0), _c_int(1 if update else 0), _stream())
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(conv_w), _ptr(conv_b), taps,
+        _ptr(gates), gates.stride(0), _ptr(a_log), _ptr(dt_bias), _ptr(ctx.req_row_start),
+        _ptr(ctx.req_state_slot), sp, stride, tail_off, _ptr(dst), _ptr(num0), _ptr(num1),
+        ctx.n_requests, host.max_new_tokens, n_heads, channels, unit_heads,
+        head_size, 1 if is_ssd else 0, 1 if update else 0, _stream())
     if code == build.UNSUPPORTED:
         return False
     _check(code, "conv_prepare")
@@ -156,11 +154,11 @@ def channel_delta_prepare(proj, conv_w, rate, beta_logit, a_log, dt_bias, ctx, s
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_channel_delta_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(conv_w), _c_int(conv_w.shape[0]),
-        _ptr(rate), _c_int(rate.stride(0)), _ptr(beta_logit), _c_int(beta_logit.stride(0)), _ptr(a_log),
-        _ptr(dt_bias), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off), _ptr(qkv),
-        _ptr(beta), _c_int(ctx.n_requests), _c_int(ctx.host.max_new_tokens), _c_int(n_heads), _c_int(n_qk_heads),
-        _c_int(key_dim), _c_int(value_dim), _stream()), "channel_delta_prepare")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(conv_w), conv_w.shape[0],
+        _ptr(rate), rate.stride(0), _ptr(beta_logit), beta_logit.stride(0), _ptr(a_log),
+        _ptr(dt_bias), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride, tail_off, _ptr(qkv),
+        _ptr(beta), ctx.n_requests, ctx.host.max_new_tokens, n_heads, n_qk_heads,
+        key_dim, value_dim, _stream()), "channel_delta_prepare")
 
 
 def conv_tail_update(proj, taps, channels, ctx, state, tail_off) -> None:
@@ -168,9 +166,9 @@ def conv_tail_update(proj, taps, channels, ctx, state, tail_off) -> None:
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_conv_tail_update(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _c_int(taps), _c_int(channels),
-        _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride, _c_long(tail_off),
-        _c_int(ctx.n_requests), _stream()), "conv_tail_update")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), taps, channels,
+        _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride, tail_off,
+        ctx.n_requests, _stream()), "conv_tail_update")
 
 
 def mlstm_prepare(proj, gates, bias_i, bias_f, cap, qkv, log_keep, log_in, n_heads, key_dim,
@@ -178,18 +176,18 @@ def mlstm_prepare(proj, gates, bias_i, bias_f, cap, qkv, log_keep, log_in, n_hea
     """`kept` (with `ctx`, `state` and the offsets of n and m in it): float32 [requests, H*D + H] that
     receives the requests' n and m as the step begins, for `matrix_memory`."""
     _need_cuda(proj, gates, bias_i, bias_f, qkv, log_keep, log_in, state, kept)
-    sp, stride = _state_args(state) if kept is not None else (_ptr(None), _c_long(0))
+    sp, stride = _state_args(state) if kept is not None else (_ptr(None), 0)
     if kept is not None and (kept.dtype != torch.float32 or not kept.is_contiguous()
                              or tuple(kept.shape) != (ctx.n_requests, n_heads * (key_dim + 1))
                              or proj.shape[0] < ctx.n_requests):
         raise KernelError("mlstm_prepare: kept is float32 [requests, H*D + H]")
     lib = build.load("recurrent")
     _check(lib.cb_mlstm_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(gates), _c_int(gates.stride(0)), _ptr(bias_i),
-        _ptr(bias_f), _c_float(cap), _ptr(qkv), _ptr(log_keep), _ptr(log_in), _c_int(proj.shape[0]),
-        _c_int(n_heads), _c_int(key_dim), _c_int(value_dim), _ptr(kept),
-        _ptr(ctx.req_state_slot if kept is not None else None), sp, stride, _c_long(n_off), _c_long(m_off),
-        _c_int(ctx.n_requests if kept is not None else 0), _stream()), "mlstm_prepare")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(gates), gates.stride(0), _ptr(bias_i),
+        _ptr(bias_f), cap, _ptr(qkv), _ptr(log_keep), _ptr(log_in), proj.shape[0],
+        n_heads, key_dim, value_dim, _ptr(kept),
+        _ptr(ctx.req_state_slot if kept is not None else None), sp, stride, n_off, m_off,
+        ctx.n_requests if kept is not None else 0, _stream()), "mlstm_prepare")
 
 
 def retention_prepare(proj, freq, rotary_dim: int, split_halves: bool, ctx, head_decay, k_scale: float,
@@ -210,10 +208,10 @@ def retention_prepare(proj, freq, rotary_dim: int, split_halves: bool, ctx, head
         raise KernelError("retention_prepare: freq is float32 [rotary_dim / 2]")
     lib = build.load("recurrent")
     _check(lib.cb_retention_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(freq), _c_int(rotary_dim),
-        _c_int(1 if split_halves else 0), _ptr(ctx.positions), _ptr(head_decay), _c_float(k_scale),
-        _ptr(qkv), _ptr(keep), _ptr(step), _c_int(proj.shape[0]), _c_int(n_heads), _c_int(key_dim),
-        _c_int(value_dim), _stream()), "retention_prepare")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(freq), rotary_dim,
+        1 if split_halves else 0, _ptr(ctx.positions), _ptr(head_decay), k_scale,
+        _ptr(qkv), _ptr(keep), _ptr(step), proj.shape[0], n_heads, key_dim,
+        value_dim, _stream()), "retention_prepare")
 
 
 def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n_off, m_off, out,
@@ -248,16 +246,16 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
         rows = min(qkv.shape[0] - walked, requests * limit)
         floats, begins = _chunk_room(rule, rows, requests, n_heads, key_dim, value_dim, limit < longest)
         room = ctx.scratch("memory.chunks", (floats,), torch.float32).data_ptr()
-        wq, ww, wk, wu, ws, wg, wl, wn, wm, kept_room = (_c_void_p(room + 4 * at if at >= 0 else 0) for at in begins)
+        wq, ww, wk, wu, ws, wg, wl, wn, wm, kept_room = (room + 4 * at if at >= 0 else 0 for at in begins)
         lib = build.load("recurrent_chunks")
         code = lib.cb_matrix_memory_chunks(
-            _c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
-            _ptr(sc0), _ptr(sc1), _c_void_p(starts + 4 * walked), _c_void_p(slots + 4 * walked), sp, stride,
-            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(requests),
-            _c_int(longest), _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim),
-            _c_int(w_off), _ptr(per_head),
-            _c_void_p(kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0),
-            _c_int(limit), kept_room, wq, ww, wk, wu, ws, wg, wl, wn, wm, _stream())
+            rule, _ptr(qkv), qkv.shape[1], q_off, k_off, v_off,
+            _ptr(sc0), _ptr(sc1), starts + 4 * walked, slots + 4 * walked, sp, stride,
+            s_off, n_off, m_off, _ptr(out), requests,
+            longest, n_heads, n_qk_heads, key_dim, value_dim,
+            w_off, _ptr(per_head),
+            kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0,
+            limit, kept_room, wq, ww, wk, wu, ws, wg, wl, wn, wm, _stream())
         if code == build.UNSUPPORTED:            # the walk's
             walked = n
         else:
@@ -269,11 +267,11 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     # decoded tokens of the bfloat16 engine: a token each, S read and written once
     step = (STEP and host is not None and host.lead_single >= walked
             and (qkv.shape[1] | v_off | value_dim) % 4 == 0 and (s_off | state.stride(0)) % 16 == 0)
-    args = (_c_int(rule), _ptr(qkv), _c_int(qkv.shape[1]), _c_int(q_off), _c_int(k_off), _c_int(v_off),
-            _ptr(sc0), _ptr(sc1), _c_void_p(starts), _c_void_p(slots), sp, stride,
-            _c_long(s_off), _c_long(n_off), _c_long(m_off), _ptr(out), _c_int(walked),
-            _c_int(n_heads), _c_int(n_qk_heads), _c_int(key_dim), _c_int(value_dim), _c_int(w_off),
-            _ptr(per_head), _c_void_p(kept_at), _stream())
+    args = (rule, _ptr(qkv), qkv.shape[1], q_off, k_off, v_off,
+            _ptr(sc0), _ptr(sc1), starts, slots, sp, stride,
+            s_off, n_off, m_off, _ptr(out), walked,
+            n_heads, n_qk_heads, key_dim, value_dim, w_off,
+            _ptr(per_head), kept_at, _stream())
     code = lib.cb_matrix_memory_step(*args) if step else build.UNSUPPORTED
     _check(lib.cb_matrix_memory(*args) if code == build.UNSUPPORTED else code, "matrix_memory")
 
@@ -288,10 +286,10 @@ def head_norm_gate(o, gain, gain_per_head, gate, out, gate_kind, n_heads, value_
         raise KernelError("head_norm_gate: float32 input, gate rows of the output's dtype or float32")
     lib = build.load("recurrent")
     _check(lib.cb_head_norm_gate(
-        _ptr(o), _ptr(gain), _c_int(value_dim if gain_per_head else 0), _ptr(gate),
-        _c_int(gate.stride(0)), _c_int(_code(gate.dtype)), _ptr(out), _c_int(out.stride(0)),
-        _c_int(_code(out.dtype)), _c_int(gate_kind), _c_int(o.shape[0]), _c_int(n_heads), _c_int(value_dim), _c_float(eps),
-        _c_float(out_scale), _stream()), "head_norm_gate")
+        _ptr(o), _ptr(gain), value_dim if gain_per_head else 0, _ptr(gate),
+        gate.stride(0), _code(gate.dtype), _ptr(out), out.stride(0),
+        _code(out.dtype), gate_kind, o.shape[0], n_heads, value_dim, eps,
+        out_scale, _stream()), "head_norm_gate")
 
 
 def shift_mix(h, mu, ctx, state, prev_off, out) -> None:
@@ -304,9 +302,9 @@ def shift_mix(h, mu, ctx, state, prev_off, out) -> None:
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_shift_mix(
-        _ptr(h), _c_int(h.stride(0)), _c_int(_code(h.dtype)), _ptr(mu), _c_int(mu.shape[0]),
+        _ptr(h), h.stride(0), _code(h.dtype), _ptr(mu), mu.shape[0],
         _ptr(ctx.row_request), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride,
-        _c_long(prev_off), _ptr(out), _c_int(h.shape[0]), _c_int(h.shape[1]), _stream()), "shift_mix")
+        prev_off, _ptr(out), h.shape[0], h.shape[1], _stream()), "shift_mix")
 
 
 def wkv_prepare(rkv, logit, w0, qkv, n_channels) -> None:
@@ -319,8 +317,8 @@ def wkv_prepare(rkv, logit, w0, qkv, n_channels) -> None:
         raise KernelError("wkv_prepare: planes [3, rows, channels], float32 logits and output "
                           "[rows, 4 * channels]")
     lib = build.load("recurrent")
-    _check(lib.cb_wkv_prepare(_ptr(rkv), _c_long(rkv.stride(0)), _c_int(_code(rkv.dtype)), _ptr(logit),
-                              _ptr(w0), _ptr(qkv), _c_int(rkv.shape[1]), _c_int(n_channels), _stream()),
+    _check(lib.cb_wkv_prepare(_ptr(rkv), rkv.stride(0), _code(rkv.dtype), _ptr(logit),
+                              _ptr(w0), _ptr(qkv), rkv.shape[1], n_channels, _stream()),
            "wkv_prepare")
 
 
@@ -338,11 +336,11 @@ def ssd_prepare(proj, conv_at, conv_w, conv_b, taps, gates, a_log, dt_bias, ctx,
     sp, stride = _state_args(state)
     lib = build.load("recurrent")
     _check(lib.cb_ssd_prepare(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(conv_at), _c_int(_code(proj.dtype)), _ptr(conv_w),
-        _ptr(conv_b), _c_int(taps), _ptr(gates), _c_int(gates.stride(0)), _ptr(a_log), _ptr(dt_bias),
+        _ptr(proj), proj.stride(0), conv_at, _code(proj.dtype), _ptr(conv_w),
+        _ptr(conv_b), taps, _ptr(gates), gates.stride(0), _ptr(a_log), _ptr(dt_bias),
         _ptr(ctx.row_request), _ptr(ctx.req_row_start), _ptr(ctx.req_state_slot), sp, stride,
-        _c_long(tail_off), _ptr(xbc), _ptr(decay), _ptr(step), _c_int(proj.shape[0]), _c_int(n_heads),
-        _c_int(channels), _stream()), "ssd_prepare")
+        tail_off, _ptr(xbc), _ptr(decay), _ptr(step), proj.shape[0], n_heads,
+        channels, _stream()), "ssd_prepare")
     return False
 
 
@@ -354,7 +352,7 @@ def gate_group_norm(y, gate, gain, out, parts, eps) -> None:
         raise KernelError("gate_group_norm: float32 input, gate and output rows of one dtype, "
                           "a width that the parts divide")
     lib = build.load("recurrent")
-    _check(lib.cb_gate_group_norm(_ptr(y), _ptr(gate), _c_int(gate.stride(0)), _ptr(gain), _ptr(out),
-                                  _c_int(out.stride(0)), _c_int(_code(out.dtype)), _c_int(y.shape[0]),
-                                  _c_int(y.shape[1]), _c_int(parts), _c_float(eps), _stream()),
+    _check(lib.cb_gate_group_norm(_ptr(y), _ptr(gate), gate.stride(0), _ptr(gain), _ptr(out),
+                                  out.stride(0), _code(out.dtype), y.shape[0],
+                                  y.shape[1], parts, eps, _stream()),
            "gate_group_norm")

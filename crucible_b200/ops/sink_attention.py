@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _need_cuda, _ptr, _stream, attention_f32, build
+from . import KernelError, _check, _code, _need_cuda, _ptr, _stream, attention_f32, build, tensor_core
 
 
 def rotate_norm_append(proj: torch.Tensor, freq: Optional[torch.Tensor], rotary_dim: int,
@@ -28,11 +28,11 @@ def rotate_norm_append(proj: torch.Tensor, freq: Optional[torch.Tensor], rotary_
     table = ctx.block_table(binding.group)
     lib = build.load("sink_attention")
     _check(lib.cb_rotate_norm_append(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(freq), _c_int(rotary_dim),
-        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]),
-        _ptr(k_cache), _ptr(v_cache), _c_int(proj.shape[0]), _c_int(n_heads), _c_int(n_kv_heads),
-        _c_int(key_dim), _c_int(value_dim), _c_int(cache.page_tokens),
-        _c_int(1 if binding.write else 0), _c_float(-1.0 if value_eps is None else value_eps), _stream()),
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(freq), rotary_dim,
+        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1],
+        _ptr(k_cache), _ptr(v_cache), proj.shape[0], n_heads, n_kv_heads,
+        key_dim, value_dim, cache.page_tokens,
+        1 if binding.write else 0, -1.0 if value_eps is None else value_eps, _stream()),
         "rotate_norm_append")
 
 
@@ -67,13 +67,13 @@ def norm_rotate_append(proj: torch.Tensor, q_gain: Optional[torch.Tensor], k_gai
     table = ctx.block_table(binding.group)
     lib = build.load("sink_attention")
     _check(lib.cb_norm_rotate_append(
-        _ptr(proj), _c_int(proj.stride(0)), _c_int(_code(proj.dtype)), _ptr(q_gain), _ptr(k_gain),
-        _c_float(qk_eps), _ptr(freq), _c_int(rotary_dim), _c_int(1 if split_halves else 0),
-        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]),
-        _ptr(k_cache), _ptr(v_cache), _c_int(proj.shape[0]), _c_int(n_heads), _c_int(n_kv_heads),
-        _c_int(key_dim), _c_int(value_dim), _c_int(cache.page_tokens),
-        _c_int(1 if binding.write else 0), _c_float(-1.0 if value_eps is None else value_eps),
-        _c_int(1 if whole_norm else 0), _stream()), "norm_rotate_append")
+        _ptr(proj), proj.stride(0), _code(proj.dtype), _ptr(q_gain), _ptr(k_gain),
+        qk_eps, _ptr(freq), rotary_dim, 1 if split_halves else 0,
+        _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1],
+        _ptr(k_cache), _ptr(v_cache), proj.shape[0], n_heads, n_kv_heads,
+        key_dim, value_dim, cache.page_tokens,
+        1 if binding.write else 0, -1.0 if value_eps is None else value_eps,
+        1 if whole_norm else 0, _stream()), "norm_rotate_append")
 
 
 def attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor,
@@ -104,12 +104,12 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor,
         return
     lib = build.load("sink_attention")
     _check(lib.cb_sink_attention(
-        _ptr(q), _c_int(q.stride(0)), _ptr(gate), _c_int(gate.stride(0) if gate is not None else 0),
-        _ptr(out), _c_int(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _c_int(_code(q.dtype)),
-        _ptr(sinks), _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), _c_int(table.shape[1]),
-        _c_int(q.shape[0]), _c_int(n_heads), _c_int(n_kv_heads), _c_int(key_dim), _c_int(value_dim),
-        _c_int(cache.page_tokens), _c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0),
-        _c_int(keep_first), _c_float(out_scale), _c_int(1 if gate_per_head else 0), _stream()), "sink attention")
+        _ptr(q), q.stride(0), _ptr(gate), gate.stride(0) if gate is not None else 0,
+        _ptr(out), out.stride(0), _ptr(k_cache), _ptr(v_cache), _code(q.dtype),
+        _ptr(sinks), _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table), table.shape[1],
+        q.shape[0], n_heads, n_kv_heads, key_dim, value_dim,
+        cache.page_tokens, scale, window or 0, 1 if chunked else 0,
+        keep_first, out_scale, 1 if gate_per_head else 0, _stream()), "sink attention")
 
 
 TENSOR_CORES = True      # tests switch it off to reach the plain kernel with the same inputs
@@ -130,7 +130,6 @@ def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, 
             or key_dim > 256 or value_dim > 256 or host is None or q.stride(0) % 8 or out.stride(0) % 2
             or (gate is not None and not gate_per_head and gate.stride(0) % 2)):
         return False
-    from . import tensor_core
     first = ctx.n_requests
     if key_dim == value_dim:
         first = tensor_core.prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, key_dim, scale, window,
@@ -157,13 +156,13 @@ def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, 
                                   (count * n_kv_heads * n_chunks * max_rows * (value_dim + 2),),
                                   torch.float32)
     code = lib.cb_attention_mma_sink(
-        _ptr(q), _c_int(q.stride(0)), _ptr(out), _c_int(out.stride(0)), _ptr(gate),
-        _c_int(gate.stride(0) if gate is not None else 0), _ptr(k_cache), _ptr(v_cache), _ptr(sinks),
-        _ptr(ctx.req_row_start), _ptr(ctx.req_first_pos), _ptr(table), _c_int(table.shape[1]),
-        _c_int(count), _c_int(max_new), _c_int(n_heads), _c_int(n_kv_heads),
-        _c_int(key_dim), _c_int(value_dim), _c_int(cache.page_tokens), _c_float(scale), _c_int(window or 0),
-        _c_int(1 if chunked else 0), _c_int(keep_first), _c_float(out_scale), _ptr(partial), _c_int(n_chunks),
-        _c_int(1 if gate_per_head else 0), _stream())
+        _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(gate),
+        gate.stride(0) if gate is not None else 0, _ptr(k_cache), _ptr(v_cache), _ptr(sinks),
+        _ptr(ctx.req_row_start), _ptr(ctx.req_first_pos), _ptr(table), table.shape[1],
+        count, max_new, n_heads, n_kv_heads,
+        key_dim, value_dim, cache.page_tokens, scale, window or 0,
+        1 if chunked else 0, keep_first, out_scale, _ptr(partial), n_chunks,
+        1 if gate_per_head else 0, _stream())
     if code == 100001:
         return False
     _check(code, "sink attention (tensor cores)")

@@ -14,12 +14,11 @@ carry what the product that wrote the rows last left for the norm (`scaled`,
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Union
 
 import torch
 
-from . import _stream, build
+from . import LAUNCHES, _stream, _tick, build
 
 build.register_module("decode_small", ["common.cuh"])
 
@@ -30,7 +29,6 @@ PREFERRED_ROWS = 16     # rows up to which the callers choose them: measured on 
                         # against 48.5 us for gate/up)
 MAX_LAZY_ROWS = 16      # rows a norm hands over not yet normalised: every block then normalises
                         # them for itself, which beyond 16 rows costs more than a norm kernel
-_c_int, _c_float, _c_void_p = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
 _UNSUPPORTED = 100001
 
 
@@ -58,7 +56,7 @@ def as_tensor(h: Rows) -> torch.Tensor:
 
 
 def _ptr(t):
-    return _c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _input(h: Rows, w: torch.Tensor):
@@ -79,7 +77,6 @@ def _done(code: int, what: str) -> bool:
         return False
     if code != 0:
         raise RuntimeError(f"{what} failed to launch (CUDA error {code})")
-    from . import LAUNCHES, _tick
     LAUNCHES[0] += 1
     _tick("few rows: " + what)
     return True
@@ -121,15 +118,15 @@ def linear(h: Rows, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = Fa
     x, gain, eps, a, lda = inp
     lib = build.load("decode_small")
     if out.dtype == torch.bfloat16:
-        return _done(lib.cb_small_linear_bf16(_ptr(x), _ptr(gain), _c_float(eps), _ptr(a), _c_int(lda),
-                                              _ptr(w), _c_int(w.stride(0)), _ptr(out),
-                                              _c_int(out.stride(0)), _c_int(h.shape[0]),
-                                              _c_int(w.shape[0]), _c_int(w.shape[1]), _c_int(act), _stream()),
+        return _done(lib.cb_small_linear_bf16(_ptr(x), _ptr(gain), eps, _ptr(a), lda,
+                                              _ptr(w), w.stride(0), _ptr(out),
+                                              out.stride(0), h.shape[0],
+                                              w.shape[0], w.shape[1], act, _stream()),
                      "small linear (bf16 result)")
-    return _done(lib.cb_small_linear(_ptr(x), _ptr(gain), _c_float(eps), _ptr(a), _c_int(lda),
-                                     _ptr(w), _c_int(w.stride(0)), _ptr(out), _c_int(out.stride(0)),
-                                     _c_int(h.shape[0]), _c_int(w.shape[0]), _c_int(w.shape[1]),
-                                     _c_int(1 if accumulate else 0), _stream()), "small linear")
+    return _done(lib.cb_small_linear(_ptr(x), _ptr(gain), eps, _ptr(a), lda,
+                                     _ptr(w), w.stride(0), _ptr(out), out.stride(0),
+                                     h.shape[0], w.shape[0], w.shape[1],
+                                     1 if accumulate else 0, _stream()), "small linear")
 
 
 def linear_swiglu(h: Rows, gate_up: torch.Tensor, out: torch.Tensor, pair=None) -> bool:
@@ -141,11 +138,11 @@ def linear_swiglu(h: Rows, gate_up: torch.Tensor, out: torch.Tensor, pair=None) 
         return False
     x, gain, eps, a, lda = inp
     lib = build.load("decode_small")
-    return _done(lib.cb_small_swiglu(_ptr(x), _ptr(gain), _c_float(eps), _ptr(a), _c_int(lda),
-                                     _ptr(gate_up), _c_int(gate_up.stride(0)), _ptr(out),
-                                     _c_int(out.stride(0)), _c_int(h.shape[0]),
-                                     _c_int(gate_up.shape[0] // 2), _c_int(gate_up.shape[1]),
-                                     *(_c_float(float(v)) for v in (pair or (0.0, 1.0, 0.0))),
+    return _done(lib.cb_small_swiglu(_ptr(x), _ptr(gain), eps, _ptr(a), lda,
+                                     _ptr(gate_up), gate_up.stride(0), _ptr(out),
+                                     out.stride(0), h.shape[0],
+                                     gate_up.shape[0] // 2, gate_up.shape[1],
+                                     *(float(v) for v in (pair or (0.0, 1.0, 0.0))),
                                      _stream()), "small swiglu")
 
 
@@ -162,10 +159,10 @@ def qkv_rope_append(h: Rows, wqkv: torch.Tensor, qkv: torch.Tensor, n_heads: int
     table = ctx.block_table(binding.group)
     lib = build.load("decode_small")
     return _done(lib.cb_small_qkv_rope_append(
-        _ptr(x), _ptr(gain), _c_float(eps), _ptr(a), _c_int(lda), _ptr(wqkv),
-        _c_int(wqkv.stride(0)), _ptr(qkv), _c_int(qkv.stride(0)), _ptr(cos), _ptr(sin),
-        _c_int(rotary_dim), _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table),
-        _c_int(table.shape[1]), _ptr(k_cache), _ptr(v_cache), _c_int(h.shape[0]),
-        _c_int(wqkv.shape[1]), _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim),
-        _c_int(cache.page_tokens), _c_int(1 if binding.write else 0), _stream()),
+        _ptr(x), _ptr(gain), eps, _ptr(a), lda, _ptr(wqkv),
+        wqkv.stride(0), _ptr(qkv), qkv.stride(0), _ptr(cos), _ptr(sin),
+        rotary_dim, _ptr(ctx.positions), _ptr(ctx.row_request), _ptr(table),
+        table.shape[1], _ptr(k_cache), _ptr(v_cache), h.shape[0],
+        wqkv.shape[1], n_heads, n_kv_heads, head_dim,
+        cache.page_tokens, 1 if binding.write else 0, _stream()),
         "small qkv + rope + cache write")

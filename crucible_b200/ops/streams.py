@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from . import KernelError, _c_float, _c_int, _check, _code, _contig, _need_cuda, _ptr, _stream, build
+from . import KernelError, _check, _code, _contig, _need_cuda, _ptr, _stream, build
 
 
 def _residual(x: torch.Tensor) -> None:
@@ -24,9 +24,9 @@ def embed_norm(table: torch.Tensor, ids: torch.Tensor, gain: torch.Tensor, eps: 
         raise KernelError("embed_norm takes int32 ids and a float32 gain")
     _contig(table, "embedding table")
     lib = build.load("streams")
-    _check(lib.cb_embed_norm_streams(_ptr(table), _c_int(_code(table.dtype)), _ptr(ids), _ptr(gain),
-                                     _ptr(out), _c_int(ids.shape[0]), _c_int(table.shape[1]),
-                                     _c_int(table.shape[0]), _c_int(out.shape[1]), _c_float(eps),
+    _check(lib.cb_embed_norm_streams(_ptr(table), _code(table.dtype), _ptr(ids), _ptr(gain),
+                                     _ptr(out), ids.shape[0], table.shape[1],
+                                     table.shape[0], out.shape[1], eps,
                                      _ptr(device_tokens), _stream()), "embed_norm_streams")
 
 
@@ -37,9 +37,9 @@ def read(x: torch.Tensor, weights: torch.Tensor, gain: torch.Tensor, eps: float,
     _residual(x)
     _contig(h, "normalised rows")
     lib = build.load("streams")
-    _check(lib.cb_streams_read(_ptr(x), _ptr(weights), _ptr(gain), _ptr(h), _c_int(_code(h.dtype)),
-                               _c_int(x.shape[0]), _c_int(x.shape[2]), _c_int(x.shape[1]),
-                               _c_float(eps), _stream()), "streams_read")
+    _check(lib.cb_streams_read(_ptr(x), _ptr(weights), _ptr(gain), _ptr(h), _code(h.dtype),
+                               x.shape[0], x.shape[2], x.shape[1],
+                               eps, _stream()), "streams_read")
 
 
 def write(x: torch.Tensor, y: torch.Tensor, mix: torch.Tensor, out_w: torch.Tensor, *,
@@ -54,10 +54,10 @@ def write(x: torch.Tensor, y: torch.Tensor, mix: torch.Tensor, out_w: torch.Tens
         raise KernelError("streams.write: y is float32 [tokens, width]")
     _contig(y, "sublayer result")
     lib = build.load("streams")
-    _check(lib.cb_streams_write(_ptr(x), _ptr(y), _ptr(mix), _ptr(out_w), _c_int(x.shape[0]),
-                                _c_int(x.shape[2]), _c_int(x.shape[1]), _ptr(next_weights),
+    _check(lib.cb_streams_write(_ptr(x), _ptr(y), _ptr(mix), _ptr(out_w), x.shape[0],
+                                x.shape[2], x.shape[1], _ptr(next_weights),
                                 _ptr(next_gain), _ptr(h),
-                                _c_int(_code(h.dtype) if h is not None else 0), _c_float(eps),
+                                _code(h.dtype) if h is not None else 0, eps,
                                 _stream()), "streams_write")
 
 
@@ -68,6 +68,6 @@ def sum_rows(x: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) -> None:
     if out.dtype != torch.float32 or rows.dtype != torch.int32:
         raise KernelError("streams.sum_rows takes int32 rows and a float32 output")
     lib = build.load("streams")
-    _check(lib.cb_streams_sum_rows(_ptr(x), _ptr(rows), _ptr(out), _c_int(out.shape[0]),
-                                   _c_int(x.shape[2]), _c_int(x.shape[1]), _stream()),
+    _check(lib.cb_streams_sum_rows(_ptr(x), _ptr(rows), _ptr(out), out.shape[0],
+                                   x.shape[2], x.shape[1], _stream()),
            "streams_sum_rows")

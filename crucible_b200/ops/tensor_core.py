@@ -16,7 +16,7 @@ import os
 
 import torch
 
-from . import _stream, build
+from . import LAUNCHES, TIMER, _stream, _tick, build
 
 build.register_module("gemm_tcgen05", ["common.cuh", "tc_common.cuh", "gemm_args.cuh"])
 build.register_module("gemm_waves_tcgen05", ["common.cuh", "tc_common.cuh", "gemm_args.cuh"])
@@ -30,7 +30,6 @@ build.register_module("attention_decode_tcgen05", ["common.cuh", "tc_common.cuh"
 USE_TCGEN05_ATTENTION = True
 USE_TCGEN05_DECODE = True
 
-_c_int, _c_void_p = ctypes.c_int, ctypes.c_void_p
 STORE_BF16, STORE_F32, ACCUM_F32, SWIGLU_BF16, ROPE_APPEND = 0, 1, 2, 3, 4
 _UNSUPPORTED = 100001
 
@@ -45,7 +44,7 @@ class KernelGaveUp(RuntimeError):
 
 def status_word(device) -> torch.Tensor:
     """A device int the kernels write if one of their bounded waits runs out."""
-    key = torch.device(device).index or 0
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     t = _status.get(key)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=device)
@@ -86,7 +85,6 @@ def check_status(device) -> None:
 
 
 def _count(n: int) -> None:
-    from . import LAUNCHES, TIMER, _tick
     LAUNCHES[0] += n
     if TIMER[0] is not None:
         import sys
@@ -116,6 +114,7 @@ K_SPLIT_BLOCK_LIMIT = {2: 148, 3: 120, 4: 128}
 K_SPLIT_MIN_GAIN_US = 1.0
 
 
+@functools.lru_cache(maxsize=4096)
 def k_splits(m: int, n_cols: int, k: int, bn: int) -> int:
     """Blocks that share one tile's K as a cluster (1: none).  A step of 33 to a few
     hundred rows has few tiles, each a chain of K / 64 loads and products on one SM while
@@ -134,6 +133,7 @@ def k_splits(m: int, n_cols: int, k: int, bn: int) -> int:
     return best
 
 
+@functools.lru_cache(maxsize=4096)
 def _tile_width(m: int, n_cols: int, epi: int = 1, multiple_of: int = 1):
     """Tile width in output columns: the one that needs the least time if every
     block costs (width + a fixed part) and blocks run in waves over the SMs.  A
@@ -161,6 +161,7 @@ TALL_MIN_K = 512            # ... pay where many rows meet enough 256 x 256 tile
 TALL_MIN_FILL = 0.8         # long K they halve the operand bytes per flop, at short K the blocks' starts and ends
 
 
+@functools.lru_cache(maxsize=4096)
 def _tall_tiles(m: int, n_cols: int, k: int) -> bool:
     """Whether a product should run as 256 x 256 tiles (two accumulators per block).  At the
     Llama-3-8B layer sizes 148 blocks of 128 x 256 ask the L2 for 384 rows of operands per
@@ -205,7 +206,7 @@ def _norm_args(emit, pre, rows: int, pair=None, act: int = 0):
     (limit, alpha, offset) of the capped gated pair for the SwiGLU form.  `act`: an activation
     on a bfloat16 result's way out (1: the square of relu)."""
     if emit is None and pre is None and pair is None and not act:
-        return _c_void_p(0), None
+        return 0, None
     args = _NormArgs()
     args.act = int(act)
     if pair is not None:
@@ -218,7 +219,7 @@ def _norm_args(emit, pre, rows: int, pair=None, act: int = 0):
             raise RuntimeError("shares of the rows' sums of squares must be float32 [parts, rows]")
         args.sumsq_in, args.parts = pre.sumsq.data_ptr(), pre.parts
         args.width, args.eps = float(pre.x.shape[1]), float(pre.eps)
-    return ctypes.cast(ctypes.pointer(args), _c_void_p), args
+    return ctypes.addressof(args), args
 
 
 def _gemm(a, w, out, n, epi, bn, per_sm=1, splits=None, emit=None, pre=None, pair=None, act=0) -> bool:
@@ -230,17 +231,18 @@ def _gemm(a, w, out, n, epi, bn, per_sm=1, splits=None, emit=None, pre=None, pai
         per_sm = 1
     if per_sm == -1:
         per_sm, splits = 0, 1
+    m, k = a.shape
     if splits is None:
-        splits = k_splits(a.shape[0], 2 * n if epi == SWIGLU_BF16 else n, a.shape[1], bn)
+        splits = k_splits(m, 2 * n if epi == SWIGLU_BF16 else n, k, bn)
     if emit is not None and (epi != ACCUM_F32 or bn > NORM_AHEAD_MAX_TILE or per_sm == 0 or n % 32
                              or emit.sumsq.shape[0] < -(-n // bn) or emit.sumsq.stride(0) != a.shape[0]):
         emit = None
-    norm_ptr, keep = _norm_args(emit, pre, a.shape[0], pair, act)
+    norm_ptr, keep = _norm_args(emit, pre, m, pair, act)
     code = lib.cb_gemm_tcgen05(
-        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
-        _c_int(a.shape[0]), _c_int(n), _c_int(a.shape[1]), _c_int(a.stride(0)),
-        _c_int(w.stride(0)), _c_int(out.stride(0)), _c_int(epi), _c_int(bn), _c_int(per_sm),
-        _c_int(splits), _c_void_p(status_word(a.device).data_ptr()), _stream(), norm_ptr)
+        a.data_ptr(), w.data_ptr(), out.data_ptr(),
+        m, n, k, a.stride(0),
+        w.stride(0), out.stride(0), epi, bn, per_sm,
+        splits, status_word(a.device).data_ptr(), _stream(), norm_ptr)
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -254,6 +256,7 @@ def _gemm(a, w, out, n, epi, bn, per_sm=1, splits=None, emit=None, pre=None, pai
 WAVES_MIN_TILES = 200       # tiles of 128 x 256 from which one block an SM walks them (`_gemm_waves`)
 
 
+@functools.lru_cache(maxsize=4096)
 def _waves_width(m: int, n_cols: int, k: int, epi: int) -> int:
     """The tile width with which a product runs through `_gemm_waves`, 0: not at all.  That kernel hides every
     tile's way out behind the next tile's products, but has fewer stages, a longer start, and no second
@@ -282,11 +285,11 @@ def _gemm_waves(a, w, out, n, epi, bn, pre=None, pair=None, act=0, plan=None) ->
     a grouped product.  False: sizes it does not take."""
     norm_ptr, keep = _norm_args(None, pre, a.shape[0], pair, act)
     if plan is not None:
-        keep, norm_ptr = plan, ctypes.cast(ctypes.pointer(plan), _c_void_p)
+        keep, norm_ptr = plan, ctypes.addressof(plan)
     code = build.load("gemm_waves_tcgen05").cb_gemm_waves(
-        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
-        _c_int(a.shape[0]), _c_int(n), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(-2)),
-        _c_int(out.stride(0)), _c_int(epi), _c_int(bn), _c_void_p(status_word(a.device).data_ptr()), _stream(), norm_ptr)
+        a.data_ptr(), w.data_ptr(), out.data_ptr(),
+        a.shape[0], n, a.shape[1], a.stride(0), w.stride(-2),
+        out.stride(0), epi, bn, status_word(a.device).data_ptr(), _stream(), norm_ptr)
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -326,23 +329,22 @@ def skinny_splits(m: int, n_tiles: int, k: int) -> int:
 def _gemm_skinny(a, w, out, n, epi, splits=None) -> bool:
     lib = build.load("gemm_skinny_tcgen05")
     m, k = a.shape
-    n_tiles = int(lib.cb_gemm_skinny_tiles(_c_int(n), _c_int(epi)))
+    n_tiles = int(lib.cb_gemm_skinny_tiles(n, epi))
     if splits is None:
         splits = skinny_splits(m, n_tiles, k)
     partial = counters = None
     if splits > 1:
-        lib.cb_gemm_skinny_partial_bytes.restype = ctypes.c_long
-        nbytes = int(lib.cb_gemm_skinny_partial_bytes(_c_int(m), _c_int(n), _c_int(epi),
-                                                      _c_int(splits)))
+        nbytes = int(lib.cb_gemm_skinny_partial_bytes(m, n, epi,
+                                                      splits))
         partial = _buffer(a.device, "skinny.partial", nbytes // 4, torch.float32)
         counters = _buffer(a.device, "skinny.counters", n_tiles, torch.int32, zero=True)
     code = lib.cb_gemm_skinny(
-        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
-        _c_int(m), _c_int(n), _c_int(k), _c_int(a.stride(0)), _c_int(w.stride(0)),
-        _c_int(out.stride(0)), _c_int(epi), _c_int(splits),
-        _c_void_p(partial.data_ptr() if partial is not None else 0),
-        _c_void_p(counters.data_ptr() if counters is not None else 0),
-        _c_void_p(status_word(a.device).data_ptr()), _stream())
+        a.data_ptr(), w.data_ptr(), out.data_ptr(),
+        m, n, k, a.stride(0), w.stride(0),
+        out.stride(0), epi, splits,
+        partial.data_ptr() if partial is not None else 0,
+        counters.data_ptr() if counters is not None else 0,
+        status_word(a.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -364,10 +366,9 @@ SKINNY_WIDE_N = 8192 # ... and up to 64 rows if W has at least this many rows (t
 
 
 def _operands_ok(a, w) -> bool:
-    return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.is_cuda
-            and a.stride(1) == 1 and w.stride(1) == 1 and a.shape[1] % 8 == 0
-            and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
-            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    (a_row, a_col), (w_row, w_col) = a.stride(), w.stride()
+    return (a_col == 1 and w_col == 1 and not (a.shape[1] | a_row | w_row) & 7 and not (a.data_ptr() | w.data_ptr()) & 15
+            and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.is_cuda)
 
 
 def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0) -> bool:
@@ -387,21 +388,23 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
         epi = ACCUM_F32 if accumulate else STORE_F32
     else:
         return False
-    w_bytes = w.numel() * 2
-    if tile is None and ((a.shape[0] <= SKINNY_ROWS and w_bytes >= SKINNY_MIN_BYTES)
-                         or (a.shape[0] <= SKINNY_MID_ROWS and SKINNY_MIN_BYTES <= w_bytes <= SKINNY_MID_BYTES)
-                         or (a.shape[0] <= 64 and w.shape[0] >= SKINNY_WIDE_N)):
-        if pre is not None or act:
-            return False
-        return _gemm_skinny(a, w, out, w.shape[0], epi)
+    m, k = a.shape
+    n = w.shape[0]
+    if tile is None and m <= 64:
+        w_bytes = w.numel() * 2
+        if ((m <= SKINNY_ROWS and w_bytes >= SKINNY_MIN_BYTES)
+                or (m <= SKINNY_MID_ROWS and SKINNY_MIN_BYTES <= w_bytes <= SKINNY_MID_BYTES) or n >= SKINNY_WIDE_N):
+            if pre is not None or act:
+                return False
+            return _gemm_skinny(a, w, out, n, epi)
     if tile is None:
-        tall = _tall_tiles(a.shape[0], w.shape[0], a.shape[1])
-        waves = 0 if emit is not None or pre is not None or (tall and epi != STORE_F32) else _waves_width(a.shape[0], w.shape[0], a.shape[1], epi)
-        if waves and _gemm_waves(a, w, out, w.shape[0], epi, waves, act=act):
+        tall = _tall_tiles(m, n, k)
+        waves = 0 if emit is not None or pre is not None or (tall and epi != STORE_F32) else _waves_width(m, n, k, epi)
+        if waves and _gemm_waves(a, w, out, n, epi, waves, act=act):
             return True
         tile = (256, 0) if tall else None
-    bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(a.shape[0], w.shape[0], epi)
-    return _gemm(a, w, out, w.shape[0], epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
+    bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(m, n, epi)
+    return _gemm(a, w, out, n, epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -445,10 +448,10 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, w.shape[1], gated)
     lib = build.load("gemm_tcgen05")
     code = lib.cb_gemm_tcgen05_grouped(
-        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()),
-        _c_int(a.shape[0]), _c_int(n), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(1)),
-        _c_int(out.stride(0)), _c_int(epi), _c_int(bn), _c_int(per_sm), _c_void_p(status_word(a.device).data_ptr()),
-        _stream(), ctypes.cast(ctypes.pointer(args), _c_void_p))
+        a.data_ptr(), w.data_ptr(), out.data_ptr(),
+        a.shape[0], n, a.shape[1], a.stride(0), w.stride(1),
+        out.stride(0), epi, bn, per_sm, status_word(a.device).data_ptr(),
+        _stream(), ctypes.addressof(args))
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -480,12 +483,12 @@ def heads_linear(a, a_head: int, w, out, out_head: int, gate=None) -> bool:
     bn = 128 if n > 96 else (96 if n > 64 else 64)
     lib = build.load("gemm_tcgen05")
     code = lib.cb_gemm_tcgen05_heads(
-        _c_void_p(a.data_ptr()), _c_void_p(w.data_ptr()), _c_void_p(out.data_ptr()), _c_int(a.shape[0]),
-        _c_int(n), _c_int(k), _c_int(a.shape[1]), _c_int(a.stride(0)), _c_int(w.stride(1)),
-        _c_int(out.stride(0)), _c_int(heads), _c_int(a_head), _c_int(out_head), _c_int(epi), _c_int(bn),
-        _c_void_p(gate.data_ptr() if gate is not None else 0), _c_int(gate.stride(0) if gate is not None else 0),
-        _c_int(GATE_HEAD if gate is not None and gate.dtype == torch.float32 else GATE_RESULT),
-        _c_void_p(status_word(a.device).data_ptr()), _stream())
+        a.data_ptr(), w.data_ptr(), out.data_ptr(), a.shape[0],
+        n, k, a.shape[1], a.stride(0), w.stride(1),
+        out.stride(0), heads, a_head, out_head, epi, bn,
+        gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0,
+        GATE_HEAD if gate is not None and gate.dtype == torch.float32 else GATE_RESULT,
+        status_word(a.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -539,15 +542,15 @@ def linear_rope_append(h, wqkv, qkv, n_heads, n_kv_heads, head_dim, cos, sin, ro
     lib = build.load("gemm_tcgen05")
     norm_ptr, keep = _norm_args(None, pre, h.shape[0])
     code = lib.cb_gemm_tcgen05_rope(
-        _c_void_p(h.data_ptr()), _c_void_p(wqkv.data_ptr()), _c_void_p(qkv.data_ptr()),
-        _c_int(h.shape[0]), _c_int(h.shape[1]), _c_int(h.stride(0)), _c_int(wqkv.stride(0)),
-        _c_int(qkv.stride(0)), _c_int(bn), _c_void_p(cos.data_ptr()), _c_void_p(sin.data_ptr()),
-        _c_void_p(ctx.positions.data_ptr()), _c_void_p(ctx.row_request.data_ptr()),
-        _c_void_p(table.data_ptr()), _c_int(table.shape[1]), _c_void_p(k_cache.data_ptr()),
-        _c_void_p(v_cache.data_ptr()), _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim),
-        _c_int(cache.page_tokens), _c_int(1 if binding.write else 0),
-        _c_int(1 if tall else k_splits(h.shape[0], wqkv.shape[0], h.shape[1], bn)), _c_int(1 if tall else 0),
-        _c_void_p(status_word(h.device).data_ptr()), _stream(), norm_ptr)
+        h.data_ptr(), wqkv.data_ptr(), qkv.data_ptr(),
+        h.shape[0], h.shape[1], h.stride(0), wqkv.stride(0),
+        qkv.stride(0), bn, cos.data_ptr(), sin.data_ptr(),
+        ctx.positions.data_ptr(), ctx.row_request.data_ptr(),
+        table.data_ptr(), table.shape[1], k_cache.data_ptr(),
+        v_cache.data_ptr(), n_heads, n_kv_heads, head_dim,
+        cache.page_tokens, 1 if binding.write else 0,
+        1 if tall else k_splits(h.shape[0], wqkv.shape[0], h.shape[1], bn), 1 if tall else 0,
+        status_word(h.device).data_ptr(), _stream(), norm_ptr)
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -568,10 +571,10 @@ class _Requests:
     the step's rows up to its end (the split form's scratch is indexed by row)."""
 
     def __init__(self, ctx, table, first: int, count: int, max_new: int, bucket: int, rows_end: int):
-        self.row_start = ctx.req_row_start[first:]
-        self.first_pos = ctx.req_first_pos[first:]
-        self.table = table[first:]
+        self.row_start = ctx.req_row_start.data_ptr() + 4 * first         # (addresses of int32)
+        self.first_pos = ctx.req_first_pos.data_ptr() + 4 * first
         self.table_stride = table.shape[1]
+        self.table = table.data_ptr() + 4 * first * table.stride(0)
         self.count, self.max_new, self.bucket, self.rows_end = count, max_new, bucket, rows_end
 
 
@@ -595,16 +598,16 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         return False
     lib = build.load("attention_tcgen05")
     code = lib.cb_attention_tcgen05_kept(
-        _c_void_p(qkv.data_ptr()), _c_int(qkv.stride(0)), _c_void_p(out.data_ptr()),
-        _c_int(out.stride(0)), _c_void_p(k_cache.data_ptr()), _c_void_p(v_cache.data_ptr()),
-        _c_int(k_cache.shape[0]), _c_void_p(reqs.row_start.data_ptr()),
-        _c_void_p(reqs.first_pos.data_ptr()), _c_void_p(reqs.table.data_ptr()),
-        _c_int(reqs.table_stride), _c_int(reqs.count), _c_int(reqs.max_new),
-        _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim), _c_int(pt),
-        ctypes.c_float(scale), _c_int(window or 0), _c_int(1 if chunked else 0), _c_int(keep_first if window else 0),
-        ctypes.c_float(out_scale), _c_void_p(sinks.data_ptr() if sinks is not None else 0),
-        _c_void_p(gate.data_ptr() if gate is not None else 0), _c_int(gate.stride(0) if gate is not None else 0),
-        _c_int(1 if gate_per_head else 0), _c_int(lead), _c_int(ATTENTION_LEAN), _c_void_p(status_word(qkv.device).data_ptr()), _stream())
+        qkv.data_ptr(), qkv.stride(0), out.data_ptr(),
+        out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
+        k_cache.shape[0], reqs.row_start,
+        reqs.first_pos, reqs.table,
+        reqs.table_stride, reqs.count, reqs.max_new,
+        n_heads, n_kv_heads, head_dim, pt,
+        scale, window or 0, 1 if chunked else 0, keep_first if window else 0,
+        out_scale, sinks.data_ptr() if sinks is not None else 0,
+        gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0,
+        1 if gate_per_head else 0, lead, ATTENTION_LEAN, status_word(qkv.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -624,15 +627,15 @@ def _attention_decode_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_he
         return False
     lib = build.load("attention_decode_tcgen05")
     code = lib.cb_attention_decode_tcgen05(
-        _c_void_p(qkv.data_ptr()), _c_int(qkv.stride(0)), _c_void_p(out.data_ptr()),
-        _c_int(out.stride(0)), _c_void_p(k_cache.data_ptr()), _c_void_p(v_cache.data_ptr()),
-        _c_int(k_cache.shape[0]), _c_void_p(reqs.row_start.data_ptr()),
-        _c_void_p(reqs.first_pos.data_ptr()), _c_void_p(reqs.table.data_ptr()),
-        _c_int(reqs.table_stride), _c_int(reqs.count), _c_int(reqs.max_new),
-        _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim), _c_int(pt),
-        ctypes.c_float(scale), _c_int(window or 0), _c_void_p(partial.data_ptr()),
-        _c_void_p(counters.data_ptr()), _c_int(n_chunks), _c_int(chunk_keys),
-        _c_void_p(status_word(qkv.device).data_ptr()), _stream())
+        qkv.data_ptr(), qkv.stride(0), out.data_ptr(),
+        out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
+        k_cache.shape[0], reqs.row_start,
+        reqs.first_pos, reqs.table,
+        reqs.table_stride, reqs.count, reqs.max_new,
+        n_heads, n_kv_heads, head_dim, pt,
+        scale, window or 0, partial.data_ptr(),
+        counters.data_ptr(), n_chunks, chunk_keys,
+        status_word(qkv.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -796,15 +799,15 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
         n_chunks = -(-reqs.bucket // chunk_keys)
     lib = build.load("attention_mma")
     code = lib.cb_attention_mma(
-        _c_void_p(qkv.data_ptr()), _c_int(qkv.stride(0)), _c_void_p(out.data_ptr()),
-        _c_int(out.stride(0)), _c_void_p(k_cache.data_ptr()), _c_void_p(v_cache.data_ptr()),
-        _c_void_p(ctx.positions.data_ptr()), _c_void_p(reqs.row_start.data_ptr()),
-        _c_void_p(reqs.first_pos.data_ptr()), _c_void_p(reqs.table.data_ptr()),
-        _c_int(reqs.table_stride), _c_int(reqs.rows_end), _c_int(reqs.count),
-        _c_int(reqs.max_new), _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim),
-        _c_int(cache.page_tokens), ctypes.c_float(scale), _c_int(window or 0),
-        _c_void_p(partial.data_ptr() if partial is not None else 0), _c_int(n_chunks),
-        _c_int(chunk_keys), _stream())
+        qkv.data_ptr(), qkv.stride(0), out.data_ptr(),
+        out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
+        ctx.positions.data_ptr(), reqs.row_start,
+        reqs.first_pos, reqs.table,
+        reqs.table_stride, reqs.rows_end, reqs.count,
+        reqs.max_new, n_heads, n_kv_heads, head_dim,
+        cache.page_tokens, scale, window or 0,
+        partial.data_ptr() if partial is not None else 0, n_chunks,
+        chunk_keys, _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -856,6 +859,6 @@ def run_wait_probe(device, limit: int = 4096) -> None:
     nothing arrives at, and then records its give-up code in the status word: the failure
     path of the tensor-core kernels, made to happen without a fault (for tests)."""
     lib = build.load("gemm_tcgen05")
-    code = lib.cb_tc_wait_probe(_c_void_p(status_word(device).data_ptr()), _c_int(limit), _stream())
+    code = lib.cb_tc_wait_probe(status_word(device).data_ptr(), limit, _stream())
     if code != 0:
         raise RuntimeError(f"wait probe failed to launch (CUDA error {code})")

@@ -96,13 +96,16 @@ class MixtureOfExperts(FeedForward):
     # Nothing of a step's routing comes to the host: the launches depend on the step's shape
     # alone, so prompt steps are captured as graphs like decode steps.
     SMALL_MAX_PAIRS = 256        # up to this many pairs the experts' weight rows are read by a warp each
-    SORTED_MIN_PAIRS = 16        # from this many (token, expert) pairs on, the experts run as two
-                                 # grouped products over their rows side by side (8 experts of 4096 x
-                                 # 2048, two a token: 8 rows 133 us against 152 with a warp per weight
-                                 # row, 16 rows 121 against 259, 64 rows 129 against 784)
+    # From this many (token, expert) pairs on, by the bytes of an expert, the experts run as two grouped
+    # products over their rows side by side; below, a warp reads a weight row.  A layer, the shared expert
+    # riding, warps and grouped: 8 experts of 2,816 x 2,048, two a token, 1 token 46.3 and 45.2 us, 2 69.8 and 54.7,
+    # 4 88 and 58, 7 157 and 77; of 1,408 x 1,024, 2 tokens 26.0 and 27.6, 3 32 and 27.7, 7 41 and 29.
+    SORTED_MIN_PAIRS = ((16 << 20, 4), (4 << 20, 6), (0, 16))
     MAX_EXPERTS = 256
     RIDE_GROUPED_ROWS = 32       # the same where the experts run as grouped products (a decode step of 16 rows,
                                  # 4 layers of width 1024: 0.379 -> 0.347 ms; at 64 rows of width 2048 no gain)
+    RIDE_PLAIN_ROWS = 128        # ... and one that does not join them otherwise (width 2,048, layer apart and riding: 8 rows
+                                 # 87 and 78 us, 32 93 and 81, 128 96 and 84, 192 99 and 105)
     RIDE_MAX_ROWS = 2            # up to this many bfloat16 rows a joining shared expert rides with the routed ones
 
     def __init__(self, spec: FeedForwardSpec):
@@ -149,8 +152,11 @@ class MixtureOfExperts(FeedForward):
                        if shared and not self.joins else None)
         # A joining shared expert as slices of an expert's size (the last one padded with zeros) that
         # every token chooses: a few rows then take no launches of their own for it.
-        self.slices = -(-self.shared_ff // self.ff) if self.joins else 0
-        if self.slices > 32 or self.n + self.slices > self.MAX_EXPERTS:
+        # One that does not join them otherwise rides along the same way in steps of a few rows (`RIDE_PLAIN_ROWS`),
+        # if the padding is little.
+        self.slices = -(-self.shared_ff // self.ff) if self.joins or (shared and self.pair is None) else 0
+        if (self.slices > 32 or self.n + self.slices > self.MAX_EXPERTS
+                or (not self.joins and 4 * self.slices * self.ff > 5 * self.shared_ff)):
             self.slices = 0
 
     def tensors(self):
@@ -176,6 +182,8 @@ class MixtureOfExperts(FeedForward):
     def bind(self, tensors, dtype, device):
         self.dtype = dtype
         d, f = self.spec.width, self.ff
+        if not self.joins and dtype != torch.bfloat16:
+            self.slices = 0                       # (a 32-bit row's sums do not depend on the step)
         # the router's rows and, behind them, the row of the shared expert's gate: one product
         self.router = (torch.cat([tensors["router"], tensors["shared.sg"]], 0).contiguous()
                        if self.shared_gate else tensors["router"])
@@ -210,8 +218,20 @@ class MixtureOfExperts(FeedForward):
     def forward(self, ctx, h, residual):
         o = self.forward_open(ctx, h)
         kernels.combine(o.rows, o.top, residual, by_plan=o.by_plan, shared=o.shared, gate=o.gate)
-        if self.shared is not None:
+        if self.shared is not None and not self._rides(h.shape[0]):
             self.shared.forward(ctx, h, residual)
+
+    def _rides(self, t: int) -> bool:
+        """Whether a shared expert that does not join the others' sum rides with them all the same: in grouped
+        products of up to `RIDE_PLAIN_ROWS` rows, or beside a token or two."""
+        if self.shared is None or self.slices == 0:
+            return False
+        return t <= (self.RIDE_PLAIN_ROWS if self._grouped(t) else self.RIDE_MAX_ROWS)
+
+    def _grouped(self, t: int) -> bool:
+        d, f = self.spec.width, self.ff
+        return (self.dtype == torch.bfloat16 and d % 8 == 0 and f % 8 == 0
+                and t * self.top >= next(n for size, n in self.SORTED_MIN_PAIRS if 6 * d * f >= size))
 
     def forward_open(self, ctx, h) -> OpenSum:
         """The experts' rows and what the shared expert adds if it joins their sum, not yet summed."""
@@ -221,10 +241,9 @@ class MixtureOfExperts(FeedForward):
         # more than a few rows: the experts' rows side by side and two grouped products on the tensor
         # cores, by the plan on the device (tiles of 128 rows); a joining shared expert then
         # runs as dense products of its own
-        grouped = (self.dtype == torch.bfloat16 and d % 8 == 0 and f % 8 == 0
-                   and t * self.top >= self.SORTED_MIN_PAIRS)
+        grouped = self._grouped(t)
         most = (self.RIDE_GROUPED_ROWS if grouped else self.RIDE_MAX_ROWS) if self.dtype == torch.bfloat16 else t
-        riding = self.slices if t <= most else 0
+        riding = self.slices if (t <= most if self.joins else self._rides(t)) else 0
         apart = self.joins and not riding
         n, top = self.n + riding, self.top + riding              # experts of the plan, pairs of a token
         tile_rows = kernels.GROUPED_TILE_ROWS if grouped else 0

@@ -69,6 +69,8 @@ struct SmallParams {
     int n_heads, n_kv_heads, head_dim, page_tokens, write_cache;
     float glu_limit, glu_alpha, glu_offset;   // SWIGLU: limit > 0: the capped pair instead of silu(g) * u
     int act;                      // STORE_BF16: 1: max(dot, 0)^2 instead of the dot
+    float* out2;                  // STORE_BF16, not null: the columns from n_main on go here in fp32, ld2 floats between rows
+    int n_main, ld2;
     int trigger_early;            // let the kernel after this one start as soon as this one's weights are asked for
                                   // (the q/k/v product: measured on B200 at batch 1 / 8, 2,048-token contexts,
                                   // 0.291 -> 0.286 / 0.345 -> 0.330 ms per step; for the other products 0 to
@@ -371,6 +373,12 @@ __global__ void __launch_bounds__(WARPS * 32) small_linear_kernel(const SmallPar
             if (m >= p.M) continue;
             const float df = d[e], ds = d[2 + e];
             if (EPI == STORE_BF16) {
+                if (p.out2 != nullptr && rf >= p.n_main) {             // (a tile lies on one side: n_main is a multiple of 16)
+                    float* second = p.out2 + (size_t)m * p.ld2 - p.n_main;
+                    if (ok_f) second[rf] = df;
+                    if (ok_s) second[rs] = ds;
+                    continue;
+                }
                 __nv_bfloat16* out = (__nv_bfloat16*)p.out + (size_t)m * p.ldc;
                 const float af = p.act == 1 ? fmaxf(df, 0.f) * fmaxf(df, 0.f) : df;
                 const float as = p.act == 1 ? fmaxf(ds, 0.f) * fmaxf(ds, 0.f) : ds;
@@ -477,16 +485,18 @@ CB_EXPORT int cb_small_linear(const float* x, const float* gain, float eps, cons
     return accumulate ? launch_rows<false, ACCUM_F32>(p, s) : launch_rows<false, STORE_F32>(p, s);
 }
 
-// out[M, N] (bf16) = act W^T.
+// out[M, N] (bf16) = act W^T; out2 not null: of the first n_main rows of W (a multiple of 16), and the others' in fp32 in out2.
 CB_EXPORT int cb_small_linear_bf16(const float* x, const float* gain, float eps, const void* a, int lda,
                                    const void* w, int ldw, void* out, int ldc, int M, int N, int K,
-                                   int act, void* stream) {
+                                   int act, float* out2, int n_main, int ld2, void* stream) {
     if (M <= 0 || N <= 0) return 0;
+    if (out2 != nullptr && (n_main <= 0 || n_main % 16 || n_main >= N || ld2 < N - n_main || act)) return CB_ERR_UNSUPPORTED;
     if (!sizes_ok(x, gain, a, lda, M, K, ldw, w) || act < 0 || act > 1) return CB_ERR_UNSUPPORTED;
     SmallParams p = {};
     p.x = x; p.gain = gain; p.eps = eps; p.a = (const __nv_bfloat16*)a; p.lda = lda;
     p.w = (const __nv_bfloat16*)w; p.ldw = ldw; p.M = M; p.K = K; p.N = N;
     p.n_tiles = (N + 15) / 16; p.out = out; p.ldc = ldc; p.act = act;
+    p.out2 = out2; p.n_main = n_main; p.ld2 = ld2;
     cudaStream_t s = (cudaStream_t)stream;
     return x ? launch_rows<true, STORE_BF16>(p, s) : launch_rows<false, STORE_BF16>(p, s);
 }

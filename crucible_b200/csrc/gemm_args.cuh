@@ -46,6 +46,12 @@ struct NormArgs {
     int act;
     const void* gate;
     int gate_ld;
+    // Two products of the same rows in one (form SPLIT_OUT, STORE_BF16): the results of the first n_main rows of W (a multiple
+    // of 64) go to C, those of the others to out2 in fp32 (ld2 floats between rows).  (A product of 8 to 32 columns alone is a
+    // chain of K / 64 loads on few SMs, 7 to 16 us; here it mostly rides in the last column of tiles: the state-space
+    // layer of width 2,048, 32 decoded tokens, 45 -> 38 us a step.)
+    void* out2;
+    int n_main, ld2;
 };
 
 }  // namespace

@@ -82,8 +82,8 @@ struct SharedStorage {
 // that sends the copies costs it every round: with the grouped form's choices in all forms a
 // 2,048-token prompt of the 120M shape, 48 of these products, took 3.3 us more): NORM_PRE (the rows of A are ahead of
 // their norm, `sumsq_in`), NORM_EMIT (`gain`: leave the next norm's input), GROUPED (a plan says
-// which rows meet which matrix), PER_HEAD (a product per head).
-enum Form { NORM_NONE = 0, NORM_PRE = 1, NORM_EMIT = 2, GROUPED = 3, PER_HEAD = 4 };
+// which rows meet which matrix), PER_HEAD (a product per head), SPLIT_OUT (`n_main`: the last columns in fp32 elsewhere).
+enum Form { NORM_NONE = 0, NORM_PRE = 1, NORM_EMIT = 2, GROUPED = 3, PER_HEAD = 4, SPLIT_OUT = 5 };
 
 template <int BN, int STAGES, int EPI, int MH, int FORM>
 __global__ void __launch_bounds__(192, (STAGES <= 3 && MH == 1) ? 2 : 1)
@@ -581,7 +581,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 uint8_t* ring = s.a[0];
                 constexpr int OUT_COLS = EPI == SWIGLU_BF16 ? BN / 2 : BN;     // columns of C per tile
                 constexpr int CHUNK = (EPI == STORE_F32 || EPI == ACCUM_F32) ? 32 : 64;
-                const int n_out = EPI == SWIGLU_BF16 ? inter : N;
+                const int n_out = EPI == SWIGLU_BF16 ? inter : FORM == SPLIT_OUT ? na.n_main : N;
+                constexpr int CHUNK_BUFS = FORM == SPLIT_OUT ? 2 : 1;         // (64 columns are 256 bytes in fp32)
                 float ss4[4] = {0.f, 0.f, 0.f, 0.f};
                 uint8_t* const sbuf = ring + (BN / 32) * (BM * 128);     // behind the staged chunks of C
                 static_assert(FORM != NORM_EMIT || EPI != ACCUM_F32 || BN > 128 || MH > 1 ||
@@ -603,9 +604,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                 }
 #pragma unroll 1
                 for (int c = 0; c < OUT_COLS / CHUNK; ++c) {
-                    uint8_t* buf = ring + c * (BM * 128);
+                    uint8_t* buf = ring + c * CHUNK_BUFS * (BM * 128);
                     uint8_t* mine = buf + r * 128;
-                    if (EPI == STORE_F32 || EPI == ACCUM_F32) {
+                    const bool second = FORM == SPLIT_OUT && n_tile * OUT_COLS + c * CHUNK >= na.n_main;
+                    if (second) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t v[32];
+                            tc::tmem_ld_32x32(lane_addr_h + c * 64 + h * 32, v);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                *reinterpret_cast<uint4*>(mine + h * (BM * 128) + ((q ^ (r & 7)) << 4)) =
+                                    make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                        }
+                    } else if (EPI == STORE_F32 || EPI == ACCUM_F32) {
                         uint32_t v[32];
                         tc::tmem_ld_32x32(lane_addr_h + c * 32, v);
                         // a norm after the product: the chunk's values of C and the gain come out
@@ -706,7 +719,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (warp == 2 && lane == 0) {
                         const int x = n_tile * OUT_COLS + c * CHUNK;
-                        if (x < n_out) {
+                        if (second) {
+                            for (int h = 0; h < 2; ++h)
+                                if (x + h * 32 < N)
+                                    tc::tma_store_2d(&map_s, buf + h * (BM * 128), x + h * 32 - n_out, m0 + mh * BM);
+                            tc::tma_store_commit();
+                        } else if (x < n_out) {
                             if (EPI == ACCUM_F32) tc::tma_reduce_add_2d(&map_c, buf, x, m0 + mh * BM);
                             else tc::tma_store_2d(&map_c, buf, x, m0 + mh * BM);
 
@@ -921,12 +939,19 @@ int launch_form(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, in
     }
     CUtensorMap mc = ma;
     // ROPE_APPEND: only the q heads' columns of C are written
-    const uint64_t map_cols = EPI == ROPE_APPEND ? (uint64_t)ra.n_heads * ra.head_dim : (uint64_t)out_cols;
+    const uint64_t map_cols = EPI == ROPE_APPEND ? (uint64_t)ra.n_heads * ra.head_dim
+                              : FORM == SPLIT_OUT ? (uint64_t)na.n_main : (uint64_t)out_cols;
     if (tma_out && !tc::make_out_map_2d(&mc, C, f32, (uint64_t)M, map_cols, (uint64_t)ldc, BM))
         tma_out = 0;
     if ((EPI == ROPE_APPEND || MH > 1 || emit) && !tma_out) return CB_ERR_UNSUPPORTED;
     CUtensorMap ms = ma;
     if (grouped) ms = *few;
+    if (FORM == SPLIT_OUT &&
+        (EPI != STORE_BF16 || na.act || !tma_out || na.n_main <= 0 || na.n_main >= N || na.n_main % 64 || na.out2 == nullptr ||
+         ((uintptr_t)na.out2 & 15) || (na.ld2 & 3) || na.ld2 < N - na.n_main ||
+         (size_t)BM * BN * 4 > sizeof(Storage::a) + sizeof(Storage::b) ||
+         !tc::make_out_map_2d(&ms, na.out2, true, (uint64_t)M, (uint64_t)(N - na.n_main), (uint64_t)na.ld2, BM)))
+        return CB_ERR_UNSUPPORTED;
     if (emit && !tc::make_plain_box_map_2d(&ms, na.scaled, (uint64_t)M, (uint64_t)N, (uint64_t)na.ld_scaled, 32, BM))
         return CB_ERR_UNSUPPORTED;
     const size_t smem_gate = ((sizeof(Storage) + 1023) & ~(size_t)1023) + (size_t)GATED_ROWS * (BN + 4) * 4 + 1024;
@@ -964,6 +989,11 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, 
     if (na.gain != nullptr) {
         if constexpr (EPI == ACCUM_F32 && BN <= 128 && MH == 1)
             return launch_form<BN, STAGES, EPI, MH, NORM_EMIT>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
+        return CB_ERR_UNSUPPORTED;
+    }
+    if (na.n_main > 0) {
+        if constexpr (EPI == STORE_BF16 && BN % 64 == 0 && (STAGES > 3 || MH == 2))
+            return launch_form<BN, STAGES, EPI, MH, SPLIT_OUT>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);
         return CB_ERR_UNSUPPORTED;
     }
     return launch_form<BN, STAGES, EPI, MH, NORM_NONE>(ma, mw, C, M, N, K, ldc, inter, k_splits, status, stream, ra, na);

@@ -407,7 +407,7 @@ CB_EXPORT int cb_gemm_waves(const void* A, const void* W, void* C, int M, int N,
     if (M <= 0 || N <= 0) return 0;
     const NormArgs na = norm ? *static_cast<const NormArgs*>(norm) : NormArgs{};
     if (K <= 0 || (K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || na.gain != nullptr ||
-        na.heads > 0 || (na.sumsq_in != nullptr && (na.parts < 1 || !(na.width > 0.f))) ||
+        na.heads > 0 || na.n_main > 0 || (na.sumsq_in != nullptr && (na.parts < 1 || !(na.width > 0.f))) ||
         (na.plan != nullptr && (na.n_experts <= 0 || na.max_tiles <= 0 || na.w_rows <= 0)))
         return CB_ERR_UNSUPPORTED;
     const uint64_t w_rows = na.plan != nullptr ? (uint64_t)na.n_experts * na.w_rows : epi == SWIGLU_BF16 ? 2 * (uint64_t)N : N;

@@ -368,6 +368,23 @@ def linear(a, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = False, c
     linear_plain(a, w, out, accumulate=accumulate)
 
 
+SPLIT_PRODUCTS = True                # tests switch it off to reach the two products
+
+
+def linear_split(h, w, w_main, w_second, out, out2) -> None:
+    """out = h W_main^T in the engine's dtype and out2 = h W_second^T in float32.  `w`: both matrices one below the
+    other, a declared weight of which `w_main` and `w_second` are views (None: they lie apart); bfloat16
+    rows then take one launch where that is quicker."""
+    if SPLIT_PRODUCTS and w is not None and w.dtype == torch.bfloat16 and is_weight(w):
+        if h.shape[0] <= small_batch.PREFERRED_ROWS:
+            if small_batch.linear(h, w, out, out2=out2):
+                return
+        elif tensor_core.linear_split(small_batch.as_tensor(h), w, out, out2):
+            return
+    linear(h, w_main, out)
+    linear(h, w_second, out2)
+
+
 FUSED_ACTIVATIONS = {"relu2": 1}     # activations the bfloat16 products apply on their results' way out
 FUSE_ACTIVATION = True               # tests switch it off to reach the product and the pass after it
 

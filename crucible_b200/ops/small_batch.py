@@ -106,11 +106,13 @@ def _weights_ok(w: torch.Tensor, rows: int) -> bool:
 MAX_OUT_ROWS = 8192     # wider products (the LM head) stream better through the tensor-core kernel
 
 
-def linear(h: Rows, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = False, act: int = 0) -> bool:
-    """`act` 1 (a bfloat16 result only): the square of relu of every dot product."""
+def linear(h: Rows, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = False, act: int = 0, out2=None) -> bool:
+    """`act` 1 (a bfloat16 result only): the square of relu of every dot product.  `out2` (likewise): float32 rows that
+    receive the products with the last rows of `w`, those beyond the columns of `out`."""
     if (not _weights_ok(w, h.shape[0]) or out.stride(1) != 1 or w.shape[0] > MAX_OUT_ROWS
             or out.dtype not in (torch.float32, torch.bfloat16)
-            or (accumulate and out.dtype != torch.float32) or (act and out.dtype != torch.bfloat16)):
+            or (accumulate and out.dtype != torch.float32) or (act and out.dtype != torch.bfloat16)
+            or (out2 is not None and (out.dtype != torch.bfloat16 or out2.dtype != torch.float32 or out2.stride(1) != 1))):
         return False
     inp = _input(h, w)
     if inp is None:
@@ -121,7 +123,8 @@ def linear(h: Rows, w: torch.Tensor, out: torch.Tensor, *, accumulate: bool = Fa
         return _done(lib.cb_small_linear_bf16(_ptr(x), _ptr(gain), eps, _ptr(a), lda,
                                               _ptr(w), w.stride(0), _ptr(out),
                                               out.stride(0), h.shape[0],
-                                              w.shape[0], w.shape[1], act, _stream()),
+                                              w.shape[0], w.shape[1], act, _ptr(out2), out.shape[1],
+                                              out2.stride(0) if out2 is not None else 0, _stream()),
                      "small linear (bf16 result)")
     return _done(lib.cb_small_linear(_ptr(x), _ptr(gain), eps, _ptr(a), lda,
                                      _ptr(w), w.stride(0), _ptr(out), out.stride(0),

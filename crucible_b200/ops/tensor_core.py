@@ -186,7 +186,7 @@ class _NormArgs(ctypes.Structure):
                 ("plan", ctypes.c_void_p), ("n_experts", ctypes.c_int), ("max_tiles", ctypes.c_int),
                 ("w_rows", ctypes.c_int), ("heads", ctypes.c_int), ("head_a_cols", ctypes.c_int),
                 ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int), ("gate", ctypes.c_void_p),
-                ("gate_ld", ctypes.c_int)]
+                ("gate_ld", ctypes.c_int), ("out2", ctypes.c_void_p), ("n_main", ctypes.c_int), ("ld2", ctypes.c_int)]
 
 
 class NormEmit:
@@ -405,6 +405,52 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
         tile = (256, 0) if tall else None
     bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(m, n, epi)
     return _gemm(a, w, out, n, epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
+
+
+def _product_cost(m: int, n_cols: int, k: int):
+    """The cost by which `_tile_width` chooses, of its choice or of tall tiles, and the tile."""
+    if _tall_tiles(m, n_cols, k):
+        return -(--(-m // 256) * -(-n_cols // 256) // N_SMS) * 711, (256, 0)
+    bn, per_sm = _tile_width(m, n_cols, STORE_BF16, 64)
+    return -(--(-m // 128) * -(-n_cols // bn) // N_SMS) * (bn + 128), (bn, per_sm)
+
+
+@functools.lru_cache(maxsize=4096)
+def _split_tile(m: int, n_main: int, n_second: int, k: int):
+    """The tile of two products of the same rows in one launch, or None where apart they take less: the second
+    often fits into the first's last column of tiles or an SM that its wave leaves idle (2,048 rows of 5,120 +
+    32 columns by 2,048: 34.0 and 8.7 us apart), but where it opens a wave more that costs more than a launch
+    (4,608 + 16: tall tiles of the first take 25.2)."""
+    joint, tile = _product_cost(m, n_main + n_second, k)
+    return tile if joint <= _product_cost(m, n_main, k)[0] + _product_cost(m, n_second, k)[0] else None
+
+
+def linear_split(a, w, out, out2) -> bool:
+    """[out | out2] = a . w^T for bfloat16 rows `out` of a multiple of 64 columns and float32 rows `out2`, in one
+    launch.  False: not taken."""
+    m, k = a.shape
+    n, n_main = w.shape[0], out.shape[1]
+    if (not _operands_ok(a, w) or out.dtype != torch.bfloat16 or out2.dtype != torch.float32 or n_main % 64
+            or out.stride(1) != 1 or out2.stride(1) != 1 or out2.shape[1] != n - n_main or out2.stride(0) % 4
+            or out.stride(0) % 8 or (out.data_ptr() | out2.data_ptr()) & 15):
+        return False
+    if m <= 64 and ((m <= SKINNY_MID_ROWS and w.numel() * 2 >= SKINNY_MIN_BYTES) or n >= SKINNY_WIDE_N):
+        return False                              # (the few-row kernel's)
+    tile = _split_tile(m, n_main, n - n_main, k)
+    if tile is None:
+        return False
+    args = _NormArgs()
+    args.out2, args.n_main, args.ld2 = out2.data_ptr(), n_main, out2.stride(0)
+    bn, per_sm = tile
+    code = build.load("gemm_tcgen05").cb_gemm_tcgen05(
+        a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), w.stride(0), out.stride(0), STORE_BF16, bn, per_sm,
+        1 if per_sm == 0 else k_splits(m, n, k, bn), status_word(a.device).data_ptr(), _stream(), ctypes.addressof(args))
+    if code == _UNSUPPORTED:
+        return False
+    if code != 0:
+        raise RuntimeError(f"tensor-core product with two results failed to launch (CUDA error {code})")
+    _count(1)
+    return True
 
 
 @functools.lru_cache(maxsize=4096)

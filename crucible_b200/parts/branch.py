@@ -32,6 +32,7 @@ class BranchMixer(Mixer):
     w_in: Optional[torch.Tensor] = None
     w_gates: Optional[torch.Tensor] = None
     w_out: Optional[torch.Tensor] = None
+    w_joint: Optional[torch.Tensor] = None      # w_in and w_gates one below the other, or None
 
     # -- what a branch says of itself ------------------------------------------------
     def input_weight(self) -> torch.Tensor:
@@ -51,11 +52,21 @@ class BranchMixer(Mixer):
 
     # -- alone -------------------------------------------------------------------------
     def _declare(self) -> None:
-        ops.declare_weights(self.w_in, self.w_gates, self.w_out)
+        self.w_in, self.w_gates, self.w_joint = join(self.w_in, self.w_gates)
+        ops.declare_weights(self.w_joint, self.w_in, self.w_gates, self.w_out)
 
     def forward(self, ctx, h, residual, binding, accumulate: bool = True):
         run_products(ctx, self, [self], [1.0], [binding], h, residual, accumulate,
                      self.w_in, self.w_gates, self.w_out)
+
+
+def join(w_in, w_gates):
+    """The two input matrices as views of one, and that one, for rows that take both products in one launch
+    (`ops.linear_split`); as they are, and None, where they cannot."""
+    if w_gates is None or w_in.dtype != torch.bfloat16 or w_in.shape[0] % 64:
+        return w_in, w_gates, None
+    both = torch.cat([w_in, w_gates], 0).contiguous()
+    return both[:w_in.shape[0]], both[w_in.shape[0]:], both
 
 
 def run_products(ctx, owner, branches: List[BranchMixer], scales, bindings, h, out, accumulate,
@@ -64,11 +75,12 @@ def run_products(ctx, owner, branches: List[BranchMixer], scales, bindings, h, o
     tag = type(owner).__name__
     dtype = w_in.dtype          # the engine dtype (h may be rows that are not yet normalised)
     proj = ctx.scratch(f"{tag}.proj", (t, w_in.shape[0]), dtype)
-    ops.linear(h, w_in, proj)
     gates = None
-    if w_gates is not None:
+    if w_gates is None:
+        ops.linear(h, w_in, proj)
+    else:
         gates = ctx.scratch(f"{tag}.gates", (t, w_gates.shape[0]), torch.float32)
-        ops.linear(h, w_gates, gates)
+        ops.linear_split(h, owner.w_joint, w_in, w_gates, proj, gates)
     act = ctx.scratch(f"{tag}.act", (t, w_out.shape[1]), dtype)
     p = g = a = 0
     for branch, scale, binding in zip(branches, scales, bindings):
@@ -108,7 +120,7 @@ class ParallelMixer(Mixer):
             self._state_offsets.append(at)
             at += (int(b.state_bytes()) + 15) // 16 * 16
         self._state_total = at
-        self.w_in = self.w_gates = self.w_out = None
+        self.w_in = self.w_gates = self.w_out = self.w_joint = None
 
     def tensors(self):
         return [replace(d, name=f"{name}.{d.name}")
@@ -122,7 +134,8 @@ class ParallelMixer(Mixer):
         gates = [b.gate_weight() for b in self.branches if b.gate_weight() is not None]
         self.w_gates = torch.cat(gates, dim=0).contiguous() if gates else None
         self.w_out = torch.cat([b.output_weight() for b in self.branches], dim=1).contiguous()
-        ops.declare_weights(self.w_in, self.w_gates, self.w_out)
+        self.w_in, self.w_gates, self.w_joint = join(self.w_in, self.w_gates)
+        ops.declare_weights(self.w_joint, self.w_in, self.w_gates, self.w_out)
 
     def cache_need(self) -> Optional[CacheNeed]:
         for b in self.branches:

@@ -38,6 +38,7 @@ from .. import ops
 from ..config.model_config import MixerSpec
 from ..ops import latent as kernels
 from .base import MIXERS, POSITIONS, CacheNeed, Mixer, TensorDecl
+from .branch import join
 
 
 class LatentAttention(Mixer):
@@ -121,7 +122,11 @@ class LatentAttention(Mixer):
         self.w_out = tensors["o"]
         self.sinks = tensors.get("sink") if self.has_sink else None
         self.dtype = dtype
-        ops.declare_weights(self.w_in, self.w_gate, self.uk_t, self.uv, self.w_out, self.w_dq, self.w_uq)
+        # the queries' latent leaves its product in float32 beside the joint product's rows
+        self.w_joint = None
+        if self.w_in is not None and self.w_dq is not None:
+            self.w_in, self.w_dq, self.w_joint = join(self.w_in, self.w_dq)
+        ops.declare_weights(self.w_joint, self.w_in, self.w_gate, self.uk_t, self.uv, self.w_out, self.w_dq, self.w_uq)
         if self.position is not None:
             self.position.bind({}, dtype, device)
 
@@ -133,17 +138,22 @@ class LatentAttention(Mixer):
         hq, row = H * (D + R), C + R
         if self.reads_other and binding.write:
             raise ValueError("latent attention: a layer without Wdkv must be run with another layer's cache")
-        proj = None
+        proj = cq32 = None
+        if self.w_dq is not None:
+            cq32 = ctx.scratch("latent.cq32", (t, int(self.q_rank)), torch.float32)
         if self.w_in is not None:
             proj = ctx.scratch("latent.proj", (t, self.w_in.shape[0]), self.dtype)
-            ops.linear(h, self.w_in, proj)
+            if cq32 is None:
+                ops.linear(h, self.w_in, proj)
+            else:
+                ops.linear_split(h, self.w_joint, self.w_in, self.w_dq, proj, cq32)
+        elif cq32 is not None:
+            ops.linear(h, self.w_dq, cq32)
         if self.q_rank is None:
             q = proj[:, self.q_at:self.q_at + hq]
         else:
             # the queries' latent: the product leaves float32, the norm reads that
             r = int(self.q_rank)
-            cq32 = ctx.scratch("latent.cq32", (t, r), torch.float32)
-            ops.linear(h, self.w_dq, cq32)
             cq = ctx.scratch("latent.cq", (t, r), self.dtype)
             ops.rmsnorm(cq32, self.dq_gain, self.eps, cq)
             q = ctx.scratch("latent.q", (t, hq), self.dtype)

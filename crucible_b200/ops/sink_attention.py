@@ -141,6 +141,10 @@ def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, 
         count, max_new, bucket = first, 1, host.lead_context_bucket
     else:
         count, max_new, bucket = ctx.n_requests, host.max_new_tokens, host.context_bucket
+    if (max_new == 1 and key_dim == value_dim and not chunked and not (keep_first and window is not None)
+            and tensor_core.short_attention(q, out, k_cache, v_cache, ctx, table, count, bucket, n_heads, n_kv_heads, key_dim,
+                                            scale, window, cache.page_tokens, sinks, out_scale, gate, gate_per_head)):
+        return True
     lib = build.load("attention_mma")
     # Few rows per request (decoded tokens, short portions): one row tile each, so the blocks
     # are few; the key tiles are then dealt to several blocks and merged.  The number of shares

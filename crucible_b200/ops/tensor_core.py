@@ -24,6 +24,7 @@ build.register_module("attention_mma", ["common.cuh"])
 build.register_module("gemm_skinny_tcgen05", ["common.cuh", "tc_common.cuh"])
 build.register_module("attention_tcgen05", ["common.cuh", "tc_common.cuh"])
 build.register_module("attention_decode_tcgen05", ["common.cuh", "tc_common.cuh"])
+build.register_module("attention_short", ["common.cuh"])
 
 # Portions of prompts with head size 64 run on the tcgen05 attention kernel; False sends
 # them to the mma.sync kernel instead (the tests compare the two).
@@ -621,6 +622,7 @@ class _Requests:
         self.first_pos = ctx.req_first_pos.data_ptr() + 4 * first
         self.table_stride = table.shape[1]
         self.table = table.data_ptr() + 4 * first * table.stride(0)
+        self.first, self.whole_table = first, table
         self.count, self.max_new, self.bucket, self.rows_end = count, max_new, bucket, rows_end
 
 
@@ -686,6 +688,47 @@ def _attention_decode_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_he
         return False
     if code != 0:
         raise RuntimeError(f"tcgen05 decode attention failed to launch (CUDA error {code})")
+    _count(1)
+    return True
+
+
+SHORT_ATTENTION = True       # tests switch it off to reach the split kernels with the same inputs
+
+
+def short_attention_pays(blocks: int, reach: int, head_dim: int, plain: bool) -> bool:
+    """Whether single tokens that read up to `reach` keys (the context's bucket, or the window) take one block a
+    request and key/value head (`blocks` of them) instead of keys split over blocks.  Without splitting
+    nothing is merged, but the keys beyond what the warps hold are walked: 3 us a 256 keys of 128 features.
+    `plain`: against the tcgen05 kernel, else (a sink, a gate) the mma.sync one, whose launch and merge cost more.
+    Whole layers of 16 or 8 heads, split and short, us: plain, 250 keys, 1 to 48 tokens, 1.02 to 1.2 times as
+    fast; 500 keys 8 tokens of 64 features 14.9 and 13.7, of 128 17.7 and 18.1, 24 of 128 33.6 and 31.1; 1,000 keys 1 token 12.7
+    and 15.7, 40 of 128 41.5 and 35.9.  With sink and gate up to 1,024 keys 1.03 to 2.3 times (a window of 1,024,
+    48 tokens of 128 102 and 60); 3,700 keys 8 tokens 50 and 61, 40 244 and 102."""
+    if plain:
+        return (reach <= 256 or (reach <= 512 and (blocks <= N_SMS if head_dim == 64 else blocks >= 48))
+                or (reach <= 1024 and head_dim == 128 and blocks >= 80))
+    return reach <= 1024 or blocks >= 64
+
+
+def short_attention(q, out, k_cache, v_cache, ctx, table, count: int, bucket: int, n_heads: int, n_kv_heads: int, head_dim: int,
+                    scale: float, window, page_tokens: int, sinks=None, out_scale: float = 1.0, gate=None,
+                    gate_per_head: bool = False, plain: bool = False) -> bool:
+    """`csrc/attention_short.cu` for the step's first `count` requests, which bring one token each and whose contexts
+    (`bucket` at most), or windows, are short.  A rule of the step's shape and of the sizes.  False: not taken."""
+    if (not SHORT_ATTENTION or head_dim not in (64, 128) or n_heads > 8 * n_kv_heads or q.stride(0) % 8 or q.data_ptr() % 16
+            or k_cache.shape[-1] != head_dim or v_cache.shape[-1] != head_dim or k_cache.dtype != torch.bfloat16
+            or not short_attention_pays(count * n_kv_heads, bucket if window is None else min(bucket, window), head_dim, plain)):
+        return False
+    code = build.load("attention_short").cb_attention_short(
+        q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), gate.data_ptr() if gate is not None else 0,
+        gate.stride(0) if gate is not None else 0, 1 if gate_per_head else 0, k_cache.data_ptr(), v_cache.data_ptr(),
+        sinks.data_ptr() if sinks is not None else 0, ctx.req_row_start.data_ptr(), ctx.req_first_pos.data_ptr(),
+        table.data_ptr(), table.shape[1], count, n_heads, n_kv_heads, head_dim, page_tokens, scale, window or 0,
+        out_scale, _stream())
+    if code == _UNSUPPORTED:
+        return False
+    if code != 0:
+        raise RuntimeError(f"short attention failed to launch (CUDA error {code})")
     _count(1)
     return True
 
@@ -811,6 +854,10 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
     """One run of requests through the kernel that suits it.  A function of the run's
     shape (count, most new tokens, bucket) and of the sizes only."""
     n_rep = n_heads // n_kv_heads
+    if (reqs.max_new == 1 and reqs.first == 0 and USE_TCGEN05_DECODE
+            and short_attention(qkv, out, k_cache, v_cache, ctx, reqs.whole_table, reqs.count, reqs.bucket, n_heads,
+                                n_kv_heads, head_dim, scale, window, cache.page_tokens, plain=True)):
+        return True
     split = reqs.max_new * n_rep <= SPLIT_ROWS
     pt = cache.page_tokens
     decode_tc = (USE_TCGEN05_DECODE and split and head_dim in (64, 128) and out.stride(0) % 2 == 0

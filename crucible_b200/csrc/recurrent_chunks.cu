@@ -22,12 +22,11 @@
 // S as every chunk begins, and chunk_out_kernel adds the queries over it, again all chunks side by side.
 // Delta rules: chunk_walk_kernel; a block owns 16 (or 8) columns of a head's S and walks the chunks in
 // order: per chunk two products on fp32 FMA (rows of Q and W over S; k^T over u), the next chunk's
-// operands on their way by asynchronous copies.  57 % of a chunk's 5,300 cycles go into operands out of
-// shared memory, the rest into the four block barriers and the chain between the products.
+// operands on their way by asynchronous copies.
 //
-// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 235 us (under ncu, cold: the chunks'
-// numbers 80, the walk 177), channel delta 551 -> 324, mLSTM 590 -> 172, wkv 467 -> 169, state space 408 -> 168;
-// 8 heads: 502 -> 165, 551 -> 210, 589 -> 91, 467 -> 90, 407 -> 79.  16,384 tokens of 16 heads in slices (256 MB of
+// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 233 us (under ncu, cold: the chunks'
+// numbers 80, the walk 165), channel delta 551 -> 280, mLSTM 590 -> 172, wkv 467 -> 169, state space 408 -> 168;
+// 8 heads: 502 -> 143, 551 -> 170, 589 -> 91, 467 -> 90, 407 -> 79.  16,384 tokens of 16 heads in slices (256 MB of
 // workspaces): delta 1,768 us, 1,760 at once; mLSTM 1,340 and 1,292; state space 1,403 and 1,380.
 //
 // The result differs from the token-by-token walk by rounding, and with the way a prompt is cut: the
@@ -757,26 +756,94 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
 }
 
 // ---- the delta rules: the state from chunk to chunk ---------------------------------------------
-// The state's columns lie in shared memory as rows [ET][DP], so that sums over D run over neighbouring
-// pairs; column 4 j + i is row i * (ET / 4) + j: the columns that neighbouring lanes read then lie a pitch
-// apart and their 16-byte reads fall on different banks.
+// The chain from chunk to chunk is W's rows over S, u, and k^T over u; the queries' rows over S are beside it.
+// All of them are bound by the bytes that shared memory hands to registers (56 % of the cycles; fp32 FMA 31 %) and by
+// the chain's latencies.  So a thread's piece of a product is up to 8 x 4 numbers (12 reads of 16 bytes for 128
+// products), what is left of a sum lies in neighbouring lanes, which halve it among themselves by exchanges (no shares
+// in shared memory), S lies there twice, as the chunk begins and as it ends, and a chunk has two barriers: u is
+// there; the state is there.  2,048 tokens of 16 heads of 128 with the chunks' numbers, against pieces of 4 x 4, shares in shared memory and
+// four barriers: delta 240 -> 233 us, channel delta 328 -> 280; 8 heads 166 -> 143, 214 -> 170; 300 tokens of 16 heads
+// 46.4 -> 44.4, 61.1 -> 54.4.  The queries' rows beside the state's sums: 45.8 -> 44.4 with 16 columns a block, but
+// 34.3 -> 35.1 (333 tokens of 8 heads of 128) and 25.7 -> 28.3 (300 of 64) with 8, where W's rows alone leave a thread a
+// piece of 2 x 4; k^T over u by all eight warps: 233 -> 245.
+// S's columns lie in shared memory as rows [ET][PS], so that sums over D run over neighbouring pairs; column
+// 4 j + i is row i * (ET / 4) + j, and the pitch puts the rows that neighbouring lanes write 128 / ET banks apart.
+
+// SHARES lanes, `apart` from each other, each with its share of the same COUNT sums: share i is left with the
+// i-th of SHARES pieces of them, in the first places
+template <int COUNT, int SHARES>
+__device__ __forceinline__ void shares_summed(float* sum, int share, int apart) {
+    if constexpr (SHARES > 1) {
+        constexpr int N = COUNT / 2, STEP = SHARES / 2;
+        const bool upper = (share & STEP) != 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float other = __shfl_xor_sync(0xffffffffu, upper ? sum[i] : sum[i + N], STEP * apart);
+            sum[i] = (upper ? sum[i + N] : sum[i]) + other;
+        }
+        shares_summed<N, STEP>(sum, share, apart);
+    }
+}
+
+// COUNT rows [COUNT][DP] over the columns of S, by N threads: a thread's piece is ROWS rows, RG apart, and 4 columns,
+// CG apart (in their order in shared memory); eight neighbouring lanes share the sum over D, 128 bytes of a row at a time
+template <int DP, int ET, int COUNT, int N>
+struct RowsOverState {
+    static constexpr int SHARES = 8, CG = ET / 4, PS = DP + 32 / CG, RG = N / (SHARES * CG), ROWS = COUNT / RG;
+    static constexpr int SUMS = ROWS * 4, LEFT = SUMS / SHARES;     // left to a lane: 4 or 2 columns of a row
+    static_assert(DP % (4 * SHARES) == 0 && (LEFT == 4 || LEFT == 2), "");
+    int row, col, x_at, y_at;
+    __device__ __forceinline__ explicit RowsOverState(int t) : share(t % SHARES) {
+        const int cg = t / SHARES % CG, rg = t / (SHARES * CG);
+        row = rg + RG * (share * LEFT / 4);
+        col = cg * 4 + share * LEFT % 4;
+        x_at = rg * DP + share * 4;
+        y_at = cg * PS + share * 4;
+    }
+    __device__ __forceinline__ void take(const float* rows, const float* S, float (&sum)[SUMS]) const {
+        pair_t acc[ROWS][4];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0;
+#pragma unroll
+        for (int d = 0; d < DP; d += 4 * SHARES) {
+            ulonglong2 x[ROWS], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = pairs_at(S + y_at + CG * j * PS + d);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) x[i] = pairs_at(rows + x_at + RG * i * DP + d);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fma_pair(x[i].x, y[j].x, acc[i][j]);
+                    acc[i][j] = fma_pair(x[i].y, y[j].y, acc[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < SUMS; ++i) sum[i] = pair_sum(acc[i / 4][i % 4]);
+        shares_summed<SUMS, SHARES>(sum, share, 1);
+    }
+private:
+    int share;
+};
+
 template <int DP, int RULE, int ET>
 __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
-    constexpr int P = DP + 4, CG = ET / 4;
+    constexpr int CG = ET / 4, PS = DP + 32 / CG;
     constexpr bool VECTOR = VECTOR_DECAY<RULE>;
-    constexpr int ROWS = 2 * CT;                         // rows over S: the queries', then W
-    constexpr int RG = ROWS / 4;                         // row groups; a thread has four rows, RG apart
-    constexpr int SPLIT = THREADS / (RG * CG);           // shares of the sum over D
-    constexpr int DS = DP / SPLIT;
-    constexpr int STAGE = (ROWS + CT) * P + CT * ET;     // rows over S, keys, u
-    static_assert(DS >= 4 && DS % 4 == 0, "a share of the sum over D is whole 16-byte pieces");
+    // 16 columns: the queries' rows beside the state's sums, by the other half of the warps; 8: with W's rows before them
+    constexpr bool BESIDE = ET == 16;
+    constexpr int STAGE = 3 * CT * DP + CT * ET;         // the queries' rows and W's over S, keys, u
+    // the second product: shares of the chunk's tokens, in lanes MS * CG apart; a thread has two pieces of four
+    // channels, DP / 2 apart, and four columns; four warps
+    constexpr int TS = 4096 / (DP * ET), MS = 32 / (TS * CG), TOKENS = CT / TS;
+    static_assert(TS >= 2 && TS <= 8 && DP / 8 == 4 * MS, "four warps cover the state");
     extern __shared__ __align__(16) float smem[];
-    float* S = smem;                                     // [ET][P]
-    float* red = S + ET * P;                             // [SPLIT][ROWS][ET]
-    float* su = red + SPLIT * ROWS * ET;                 // [CT][ET]: u as it joins the state
-    float* sg = su + CT * ET;                        // [DP]: the chunk's decays per channel
+    float* states = smem;                                // [2][ET][PS]: as the chunk begins, and as it ends
+    float* su = states + 2 * ET * PS;                    // [CT][ET]: u as it joins the state
+    float* sg = su + CT * ET;                            // [DP]: the chunk's decays per channel
     float4* sc = reinterpret_cast<float4*>(sg + DP);     // [2][CT] the tokens' numbers
     float* stage = reinterpret_cast<float*>(sc + 2 * CT);
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * ET;
@@ -791,7 +858,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     auto place_of = [](int c) { return (c & 3) * CG + (c >> 2); };
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
-        S[place_of(c) * P + d] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
+        states[place_of(c) * PS + d] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
     }
     for (int d = tid; d < DP; d += THREADS) sg[d] = 0.f;
     for (int i = tid; i < 2 * STAGE; i += THREADS) stage[i] = 0.f;      // the rows' and columns' padding
@@ -802,8 +869,8 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int ft = tid / PIECES, fd = (tid % PIECES) * 4;
     auto fetch = [&](int base, int buf) {
         float* rows = stage + buf * STAGE;
-        float* keys = rows + ROWS * P;
-        float* u = keys + CT * P;
+        float* keys = rows + 2 * CT * DP;
+        float* u = keys + CT * DP;
         const int cnt = min(CT, row1 - base);
         if (fd < D) {
 #pragma unroll
@@ -811,14 +878,14 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 if (t < cnt) {
                     const size_t at = ((size_t)(base - shift + t) * H + head) * D + fd;
                     const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + fd;
-                    cp16(rows + t * P + fd, a.wq + at);
-                    cp16(rows + (CT + t) * P + fd, a.ww + at);
-                    cp16(keys + t * P + fd, VECTOR ? a.wk + at : src + a.k_off);
+                    cp16(rows + t * DP + fd, a.wq + at);
+                    cp16(rows + (CT + t) * DP + fd, a.ww + at);
+                    cp16(keys + t * DP + fd, VECTOR ? a.wk + at : src + a.k_off);
                 } else {                                 // a portion's last chunk: rows of an earlier one are there
                     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                    *reinterpret_cast<float4*>(rows + t * P + fd) = zero;
-                    *reinterpret_cast<float4*>(rows + (CT + t) * P + fd) = zero;
-                    *reinterpret_cast<float4*>(keys + t * P + fd) = zero;
+                    *reinterpret_cast<float4*>(rows + t * DP + fd) = zero;
+                    *reinterpret_cast<float4*>(rows + (CT + t) * DP + fd) = zero;
+                    *reinterpret_cast<float4*>(keys + t * DP + fd) = zero;
                 }
             }
         }
@@ -838,114 +905,114 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // the first product: a thread's rows rg + RG i and columns 4 cg + j, its share of D
-    const int share = tid / (RG * CG), rg = (tid % (RG * CG)) / CG, cg = tid % CG;
-    // where its sums go, and who adds the shares
-    const int orow = tid / CG, ocol = cg * 4;
-    // the second product: a thread's four channels and four columns (of ET / 4 x DP / 4 threads)
-    const int ud = (tid / CG) * 4, uc = (tid % CG) * 4;
+    RowsOverState<DP, ET, BESIDE ? CT : 2 * CT, THREADS> first(tid);
+    RowsOverState<DP, ET, CT, THREADS / 2> queries(tid % (THREADS / 2));
+    // the state's part: a share of the tokens, channels ud + DP / 2 i, columns 4 uc + c
+    const int lane = tid & 31, uc = lane % CG, part = lane / (CG * MS);
+    const int ud = (tid / 32 % 4 * MS + lane / CG % MS) * 4;
     fetch(row0, 0);
     int buf = 0;
     for (int base = row0; base < row1; base += CT, buf ^= 1) {
         const int cnt = min(CT, row1 - base);
         const float* rows = stage + buf * STAGE;
-        const float* keys = rows + ROWS * P;
-        const float* u = keys + CT * P;
+        const float* keys = rows + 2 * CT * DP;
+        const float* u = keys + CT * DP;
+        const float* S = states + buf * ET * PS;
         const float4* nums = sc + buf * CT;
-        const bool has_out = orow < cnt && col0 + ocol < E;
-        float* out_at = a.out + ((size_t)(base + orow) * H + head) * E + col0 + ocol;
-        float4 local = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (has_out) local = *reinterpret_cast<const float4*>(out_at);
-        if (base + CT < row1) {
-            fetch(base + CT, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        // what a token has within the chunk, and with the state's share added
+        auto out_at = [&](int t, int c) { return a.out + ((size_t)(base + t) * H + head) * E + col0 + c; };
+        auto within = [&](bool has, int t, int c, float* to, int n) {
+#pragma unroll
+            for (int k = 0; k < n; k += 2) {
+                const float2 l = has ? *reinterpret_cast<const float2*>(out_at(t, c + k)) : make_float2(0.f, 0.f);
+                to[k] = l.x; to[k + 1] = l.y;
+            }
+        };
+        auto put = [&](int t, int c, const float* l, const float* sum, int n) {
+#pragma unroll
+            for (int k = 0; k < n; k += 2)
+                *reinterpret_cast<float2*>(out_at(t, c + k)) = make_float2(l[k] + sum[k], l[k + 1] + sum[k + 1]);
+        };
+        float local[4];
+        const bool first_out = !BESIDE && first.row < cnt && col0 + first.col < E;
+        if (!BESIDE) within(first_out, first.row, first.col, local, first.LEFT);
+        // the chunk's operands are there, the state is, and the other stage is free
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (base + CT < row1) fetch(base + CT, buf ^ 1);
         if (VECTOR && tid < D) sg[tid] = a.wg[(chunk_place(base - shift, r) * H + head) * D + tid];
-        __syncthreads();
-        // the rows over S
         {
-            pair_t acc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0;
-            const float* x_at = rows + rg * P + share * DS;
-            const float* y_at = S + cg * P + share * DS;
-#pragma unroll
-            for (int d = 0; d < DS; d += 4) {
-                ulonglong2 x[4], y[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) x[i] = pairs_at(x_at + RG * i * P + d);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) y[j] = pairs_at(y_at + CG * j * P + d);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc[i][j] = fma_pair(x[i].x, y[j].x, acc[i][j]);
-                        acc[i][j] = fma_pair(x[i].y, y[j].y, acc[i][j]);
-                    }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                *reinterpret_cast<float4*>(red + ((size_t)share * ROWS + rg + RG * i) * ET + 4 * cg) =
-                    make_float4(pair_sum(acc[i][0]), pair_sum(acc[i][1]), pair_sum(acc[i][2]), pair_sum(acc[i][3]));
-        }
-        const float g_end = VECTOR ? 1.f : nums[cnt - 1].x;
-        __syncthreads();
-        if (orow < ROWS) {
-            float4 sum = *reinterpret_cast<const float4*>(red + (size_t)orow * ET + ocol);
-#pragma unroll
-            for (int x = 1; x < SPLIT; ++x) {
-                const float4 y = *reinterpret_cast<const float4*>(red + ((size_t)x * ROWS + orow) * ET + ocol);
-                sum.x += y.x; sum.y += y.y; sum.z += y.z; sum.w += y.w;
-            }
-            if (orow < CT) {
-                if (has_out)
-                    *reinterpret_cast<float4*>(out_at) = make_float4(local.x + sum.x, local.y + sum.y, local.z + sum.z,
-                                                                     local.w + sum.w);
-            } else {
-                const int t = orow - CT;
-                float4 own = *reinterpret_cast<const float4*>(u + t * ET + ocol);
-                own.x -= sum.x; own.y -= sum.y; own.z -= sum.z; own.w -= sum.w;
+            float sum[first.SUMS];
+            first.take(rows + (BESIDE ? CT * DP : 0), S, sum);
+            const int t = first.row - (BESIDE ? 0 : CT);
+            if (t >= 0) {
                 const float f = VECTOR ? 1.f : nums[t].y;
-                *reinterpret_cast<float4*>(su + t * ET + ocol) = make_float4(f * own.x, f * own.y, f * own.z, f * own.w);
+#pragma unroll
+                for (int k = 0; k < first.LEFT; k += 2) {
+                    const float2 own = *reinterpret_cast<const float2*>(u + t * ET + first.col + k);
+                    *reinterpret_cast<float2*>(su + t * ET + first.col + k) =
+                        make_float2(f * (own.x - sum[k]), f * (own.y - sum[k + 1]));
+                }
+            } else if (first_out) {
+                put(first.row, first.col, local, sum, first.LEFT);
             }
         }
         __syncthreads();
-        // the state: decayed, and the chunk's k^T u
-        if (ud < DP) {
-            pair_t x[4][2];
+        if (tid >= THREADS / 2) {
+            if (BESIDE) {
+                const bool has = queries.row < cnt && col0 + queries.col < E;
+                within(has, queries.row, queries.col, local, queries.LEFT);
+                float sum[queries.SUMS];
+                queries.take(rows, S, sum);
+                if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
+            }
+        } else {
+            pair_t x[2][4][2];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) x[c][0] = x[c][1] = 0;
-#pragma unroll 8
-            for (int t = 0; t < CT; ++t) {
-                const ulonglong2 k = pairs_at(keys + t * P + ud);
-                const float4 v = *reinterpret_cast<const float4*>(su + t * ET + uc);
+            for (int c = 0; c < 8; ++c) x[c / 4][c % 4][0] = x[c / 4][c % 4][1] = 0;
+#pragma unroll
+            for (int i = 0; i < TOKENS; ++i) {
+                const int t = part * TOKENS + i;
+                const ulonglong2 k0 = pairs_at(keys + t * DP + ud), k1 = pairs_at(keys + t * DP + DP / 2 + ud);
+                const float4 v = *reinterpret_cast<const float4*>(su + t * ET + uc * 4);
                 const pair_t f[4] = {make_pair_of(v.x, v.x), make_pair_of(v.y, v.y), make_pair_of(v.z, v.z), make_pair_of(v.w, v.w)};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    x[c][0] = fma_pair(k.x, f[c], x[c][0]);
-                    x[c][1] = fma_pair(k.y, f[c], x[c][1]);
+                    x[0][c][0] = fma_pair(k0.x, f[c], x[0][c][0]);
+                    x[0][c][1] = fma_pair(k0.y, f[c], x[0][c][1]);
+                    x[1][c][0] = fma_pair(k1.x, f[c], x[1][c][0]);
+                    x[1][c][1] = fma_pair(k1.y, f[c], x[1][c][1]);
                 }
             }
-            const float4 own = *reinterpret_cast<const float4*>(sg + ud);
-            const pair_t ga = VECTOR ? make_pair_of(own.x, own.y) : make_pair_of(g_end, g_end);
-            const pair_t gb = VECTOR ? make_pair_of(own.z, own.w) : ga;
+            // the tokens' shares: a piece of the channels to each half of the lanes, then half of its columns
+            float sum[32];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                ulonglong2* at = reinterpret_cast<ulonglong2*>(S + place_of(uc + c) * P + ud);
-                ulonglong2 p = *at;
-                p.x = fma_pair(ga, p.x, x[c][0]);
-                p.y = fma_pair(gb, p.y, x[c][1]);
-                *at = p;
+            for (int i = 0; i < 16; ++i) {
+                const float2 v = split_pair(x[i / 8][i / 2 % 4][i % 2]);
+                sum[2 * i] = v.x; sum[2 * i + 1] = v.y;
+            }
+            shares_summed<32, TS>(sum, part, CG * MS);
+            constexpr int COLS = 8 / TS;
+            const int d = ud + (part / (TS / 2)) * (DP / 2), c0 = uc * 4 + part % (TS / 2) * COLS;
+            const float g_end = VECTOR ? 1.f : nums[cnt - 1].x;
+            const float4 own = *reinterpret_cast<const float4*>(sg + d);
+            float* next = states + (buf ^ 1) * ET * PS;
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                const int at = place_of(c0 + c) * PS + d;
+                float4 p = *reinterpret_cast<const float4*>(S + at);
+                p.x = fmaf(VECTOR ? own.x : g_end, p.x, sum[4 * c]);
+                p.y = fmaf(VECTOR ? own.y : g_end, p.y, sum[4 * c + 1]);
+                p.z = fmaf(VECTOR ? own.z : g_end, p.z, sum[4 * c + 2]);
+                p.w = fmaf(VECTOR ? own.w : g_end, p.w, sum[4 * c + 3]);
+                *reinterpret_cast<float4*>(next + at) = p;
             }
         }
-        __syncthreads();
     }
+    __syncthreads();
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
-        if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = S[place_of(c) * P + d];
+        if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = states[buf * ET * PS + place_of(c) * PS + d];
     }
 }
 
@@ -960,9 +1027,7 @@ int allow_smem(K kernel, size_t smem, bool& configured) {
 
 template <int DP, int RULE, int ET>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
-    constexpr int ROWS = 2 * CT, SPLIT = THREADS / ((ROWS / 4) * (ET / 4)), P = DP + 4;
-    constexpr size_t bytes = sizeof(float) * (ET * P + SPLIT * ROWS * ET + CT * ET + DP + 8 * CT
-                                              + 2 * ((ROWS + CT) * P + CT * ET));
+    constexpr size_t bytes = sizeof(float) * (2 * ET * (DP + 128 / ET) + CT * ET + DP + 8 * CT + 2 * (3 * CT * DP + CT * ET));
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes, configured);

@@ -146,6 +146,39 @@ def test_chunks_agree_with_float64(rule, H, G, D, E, monkeypatch):
                 assert got <= max(times * plain, least), (rule, lengths, r, errors)
 
 
+@pytest.mark.parametrize("rule", ["DELTA", "CHANNEL"])
+@pytest.mark.parametrize("H,D,E", [(12, 128, 128), (16, 64, 72), (12, 100, 100), (3, 128, 20), (2, 36, 8)])
+def test_the_delta_rules_walk_in_both_widths(rule, H, D, E, monkeypatch):
+    """16 columns of the state a block (more than 74 such blocks) and 8: one chunk, part of one, whole chunks and one token
+    more, against float64; the bound is the module's."""
+    from crucible_b200.ops import recurrent as k
+    monkeypatch.setattr(k, "chunks_pay", lambda rule, rows, requests, longest, heads: requests > 0)
+    code, lengths = getattr(k, rule), (96, 33, 7)
+    g = torch.Generator().manual_seed(H + D)
+    T, R = sum(lengths), len(lengths)
+    assert (R * H * -(-E // 16) > 74) == (H >= 12)
+    q, kk, v, w, sc0, sc1, _ = _operands(code, k, T, H, H, D, E, g)
+    on = lambda x: x.contiguous().to(DEV) if x is not None else None
+    qkv = on(torch.cat([x.reshape(T, -1) for x in (q, kk, v, w) if x is not None], 1))
+    before, results = torch.randn(R, H * D * E, generator=g) * 0.3, []
+    for chunks in (True, False):
+        monkeypatch.setattr(k, "CHUNKS", chunks)
+        ctx, starts, slots = _ctx(lengths, torch.bfloat16)
+        state = torch.zeros(R, H * D * E, device=DEV)
+        state[slots] = before.to(DEV)
+        out = torch.full((T, H * E), float("nan"), device=DEV)
+        k.matrix_memory(code, qkv, 0, H * D, 2 * H * D, on(sc0), on(sc1), ctx, state.view(torch.uint8), 0, 0, 0, out, H, H, D, E,
+                        w_off=2 * H * D + H * E)
+        results.append((out.cpu().view(T, H, E).double(), state[slots].cpu().view(R, H, D, E).double()))
+    for r in range(R):
+        a, b = starts[r], starts[r + 1]
+        want, S, _, _ = _walk(code, k, *[x[a:b] if x is not None else None for x in (q, kk, v, w, sc0, sc1)], None,
+                              before[r].double().view(H, D, E), None, None)
+        off = [[float((x - y).norm() / y.norm()) for x, y in ((o[a:b], want), (s[r], S))] for o, s in results]
+        for got, plain in zip(*off):
+            assert got <= max(2 * plain, 4 * ROUNDING), (lengths[r], off)
+
+
 @pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
 @pytest.mark.parametrize("space,limit", [(0, 32), (None, 64), (None, 128)])
 def test_slices_have_the_bits_of_one(rule, space, limit, monkeypatch):

@@ -129,12 +129,14 @@ __global__ void __launch_bounds__(32 * W, HD == 64 && R <= 4 && W == 8 ? 2 : 1) 
 #pragma unroll
             for (int x = 4; x < 32; x <<= 1) m_new[e] = fmaxf(m_new[e], __shfl_xor_sync(0xffffffffu, m_new[e], x));
         }
-        // (a pass begins with a key that counts; its scores may all be -inf, or one NaN)
+        // A maximum of -inf: every score so far is -inf, or NaN, which fmaxf passes over.  0 is the offset then, so that
+        // the first weigh nothing and a NaN stays one (and 0 times it, in what follows).
+        const float off[2] = {m_new[0] == -INFINITY ? 0.f : m_new[0], m_new[1] == -INFINITY ? 0.f : m_new[1]};
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const float p = m_new[x & 1] == -INFINITY ? 0.f : exp2_of(c[m][x] - m_new[x & 1]);
+                const float p = exp2_of(c[m][x] - off[x & 1]);
                 total[x & 1] += p;
                 c[m][x] = p;
             }
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 && R <= 4 && W == 8 ? 2 : 1) 
             l = fmaf(f, sum[w][h], l);
             y = fmaf(f, x, y);
         }
-        y = y / l * a.out_scale;
+        y = l > 0.f ? y / l * a.out_scale : y * 0.f;         // (no weight at all, or a NaN)
         if (a.gate != nullptr) {
             const float z = __bfloat162float(a.gate[(size_t)row * a.gate_stride + (a.gate_per_head ? head : head * HD + d)]);
             y *= 1.0f / (1.0f + expf(-z));

@@ -39,19 +39,23 @@ struct NormArgs {
     // columns of A start at z * head_a_cols, whose matrix is rows [z * w_rows, z * w_rows + N) of
     // W and whose results go to columns z * head_c_cols + [0, N) of C.  K is a head's K; what a
     // block of 64 columns of A holds beyond it meets columns of W outside its map, which read zero.
-    int heads, head_a_cols, head_c_cols;
+    // Two products of the same rows in one (form SPLIT_OUT, STORE_BF16; heads 0): the results of the first n_main rows of W (a
+    // multiple of 64) go to C, those of the others to out2 in fp32 (ld2 floats between rows).  (A product of 8 to 32 columns alone
+    // is a chain of K / 64 loads on few SMs, 7 to 16 us; here it mostly rides in the last column of tiles: the state-space
+    // layer of width 2,048, 32 decoded tokens, 45 -> 38 us a step.)
+    // These forms share their fields, as no product is both, for the size: see the assertion below.
+    int heads, head_a_cols;
+    union { int head_c_cols; int n_main; };
     // STORE_BF16: an activation on the way out; 0: none, 1: max(x, 0)^2.  PER_HEAD, with `gate` set (up to
     // GATED_ROWS rows): the results times the sigmoids of their logits before they are rounded, of one logit a row and head
     // (GATE_HEAD: fp32 [M][heads]) or of one a result (GATE_RESULT: bf16 [M][heads * N]).
     int act;
-    const void* gate;
-    int gate_ld;
-    // Two products of the same rows in one (form SPLIT_OUT, STORE_BF16): the results of the first n_main rows of W (a multiple
-    // of 64) go to C, those of the others to out2 in fp32 (ld2 floats between rows).  (A product of 8 to 32 columns alone is a
-    // chain of K / 64 loads on few SMs, 7 to 16 us; here it mostly rides in the last column of tiles: the state-space
-    // layer of width 2,048, 32 decoded tokens, 45 -> 38 us a step.)
-    void* out2;
-    int n_main, ld2;
+    union { const void* gate; void* out2; };
+    union { int gate_ld; int ld2; };
 };
+// With 120 bytes the parameters of gemm_tcgen05_kernel are 768.  With 136 (and the kernel's code as it was) every
+// gated product took 0.3 to 0.6 us more: 17 rows of 2 x 2,048 by 768 5.5 -> 5.8 us, 300 5.5 -> 5.85, 900 rows of
+// 2 x 2,816 by 2,048 22.8 -> 23.5.
+static_assert(sizeof(NormArgs) == 120, "the products' parameters have grown");
 
 }  // namespace

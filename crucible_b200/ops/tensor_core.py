@@ -187,7 +187,7 @@ class _NormArgs(ctypes.Structure):
                 ("plan", ctypes.c_void_p), ("n_experts", ctypes.c_int), ("max_tiles", ctypes.c_int),
                 ("w_rows", ctypes.c_int), ("heads", ctypes.c_int), ("head_a_cols", ctypes.c_int),
                 ("head_c_cols", ctypes.c_int), ("act", ctypes.c_int), ("gate", ctypes.c_void_p),
-                ("gate_ld", ctypes.c_int), ("out2", ctypes.c_void_p), ("n_main", ctypes.c_int), ("ld2", ctypes.c_int)]
+                ("gate_ld", ctypes.c_int)]
 
 
 class NormEmit:
@@ -441,7 +441,7 @@ def linear_split(a, w, out, out2) -> bool:
     if tile is None:
         return False
     args = _NormArgs()
-    args.out2, args.n_main, args.ld2 = out2.data_ptr(), n_main, out2.stride(0)
+    args.gate, args.head_c_cols, args.gate_ld = out2.data_ptr(), n_main, out2.stride(0)      # (out2, n_main, ld2 there)
     bn, per_sm = tile
     code = build.load("gemm_tcgen05").cb_gemm_tcgen05(
         a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), w.stride(0), out.stride(0), STORE_BF16, bn, per_sm,

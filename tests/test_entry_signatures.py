@@ -47,3 +47,11 @@ def test_scratch_views_follow_their_buffer():
     for i in range(3000):
         s.get("x", (1, 1 + i % 40, 1), torch.float32)
     assert len(s._views) <= 1024
+
+
+def test_what_a_product_is_told_keeps_its_size():
+    """The kernel's copy is asserted beside its declaration: with 16 bytes more every gated product took 0.3 us more."""
+    from crucible_b200.ops import build, tensor_core
+    assert ctypes.sizeof(tensor_core._NormArgs) == 120
+    with open(os.path.join(build.CSRC, "gemm_args.cuh")) as f:
+        assert "static_assert(sizeof(NormArgs) == 120" in f.read()

@@ -16,9 +16,10 @@
 // us before (gemm_rows_kernel for all) -> now, W in L2, K = N = 1,024: 5 rows 21.0 -> 12.0, 28 rows 46.6 ->
 // 12.6, 116 rows 48.3 -> 17.2, 301 rows 48.7 -> 32.4, 700 rows 63.3 -> 49.7; 700 x 768 x 768 37.5 -> 27.3
 // (0.41 of the SMs' multiply-adds; the copies out of shared memory alone would be 20); 2,048 x 2,304 x 768
-// 172 -> 165.  Stages are whole, so a K just past one costs up to a stage more (700 x 2,050 x 136: 15.7 -> 17.1).
+// 172 -> 165.  Stages are whole, so a K just past one costs up to a stage more, where gemm_rows_kernel is taken instead.  (A
+// tail of half a stage in a second copy of the loop's body: 5 to 12 % slower at whole stages.)
 //
-// gemm_rows_kernel, everything else (bfloat16 rows, rows off 16 bytes): tiles of 64 x 64 with 8 x 4 sums a
+// gemm_rows_kernel, everything else (bfloat16 rows, rows off 16 bytes) and where `pick_form` says so: tiles of 64 x 64 with 8 x 4 sums a
 // thread, or 16 x 32 with 4 x 1 for up to 16 rows; the next 16 of k are on their way through registers,
 // which convert them.  (The forms above fed through registers: 15 % slower from 700 rows on.)
 //
@@ -144,20 +145,42 @@ int launch_form(const float* A, const float* W, float* C, const Product& p, int 
 // The form by what an SM with the most tiles takes for one k, in tenths of a cycle: a part for the chain
 // and one a tile, as measured at K = 768 and 1,024 over 8 to 3,255 rows and 16 to 4,608 columns (the choice
 // is within 9 % of the best form at all of them).  The smallest form fits an SM six times, the third four.
+// -1: gemm_rows_kernel, whose stages are of 16 of k and whose blocks start sooner and fit an SM five times.  All forms
+// and it were measured at 15 numbers of rows, 9 of columns and 14 of K from 16 to 2,048; it is ahead
+// - at K up to 16 (16 rows of 2,050 2.0 against 2.95 us, 2,050 of 2,050 7.9 against 12.2; few rows of few columns are not);
+// - where a K ends in the first half of a stage, so that half a stage is multiplied for nothing, and the tiles are
+//   more than the SMs: at 64 x 64 up to K = 512 (700 x 2,050 x 136 15.9 against 17.2, x 264 within 1 %; a tile an SM, 700 x 768 x 136, 9.1
+//   against 8.0), at 64 x 32 to 144;
+// - at K below 640 where an SM gets 4 and a part of the 64 x 64 tiles: four fit it, so the rest wait (1,300 x 2,050 x 128 22.4
+//   against 25.6, x 520 79 against 86, x 768 110 against 106).
+// Five to sixteen rows of many columns at a K of one or two stages: the second form before the first (16 x 4,608 x 64 1.16 times
+// as fast, and as the kernel before).  With this choice no size is slower than gemm_rows_kernel's by more than 5 %, but
+// 1,000 rows of 16 columns at K = 16 (2.5 against 2.3 us).
+constexpr int ROWS_KERNEL = -1;
 int pick_form(const Product& p, int heads) {
-    auto tiles = [&](int tm, int tn) { return ((long)((p.M + tm - 1) / tm) * ((p.N + tn - 1) / tn) * heads + 147) / 148; };
+    auto all = [&](int tm, int tn) { return (long)((p.M + tm - 1) / tm) * ((p.N + tn - 1) / tn) * heads; };
+    auto tiles = [&](int tm, int tn) {
+        return (all(tm, tn) + 147) / 148;
+    };
     const long e[4] = {tiles(16, 16), tiles(32, 32), tiles(64, 32), tiles(64, 64)};
     const long cost[4] = {170 * ((e[0] + 5) / 6) + 46 * e[0], 140 + 175 * e[1], 180 * ((e[2] + 3) / 4) + 275 * e[2],
                           170 + 510 * e[3]};
     int form = 0;
     for (int i = 1; i < 4; ++i)
         if (cost[i] < cost[form]) form = i;
+    const bool few = p.M <= 16;
+    if (p.K <= 16 && (few || all(64, 64) >= 10)) return ROWS_KERNEL;
+    if (few) return form == 0 && p.M > 4 && p.K <= 80 && all(16, 16) >= (p.K > 64 ? 80 : 149) ? 1 : form;
+    const bool half = p.K % 32 >= 1 && p.K % 32 <= 16;
+    if (form == 3 && half && (p.K <= 48 || (e[3] >= 2 && p.K < (e[3] == 2 ? 544 : 512)))) return ROWS_KERNEL;
+    if (form == 3 && e[3] == 5 && p.K < 640) return ROWS_KERNEL;
+    if (form == 2 && half && e[3] >= 2 && p.K <= 144) return ROWS_KERNEL;
     return form;
 }
 
 template <bool ACCUMULATE>
-int launch_f32(const float* A, const float* W, float* C, const Product& p, int heads, cudaStream_t s) {
-    switch (pick_form(p, heads)) {
+int launch_f32(int form, const float* A, const float* W, float* C, const Product& p, int heads, cudaStream_t s) {
+    switch (form) {
         case 0: return launch_form<ACCUMULATE, 16, 16, 2, 2, 64, 4>(A, W, C, p, heads, s);
         case 1: return launch_form<ACCUMULATE, 32, 32, 4, 2, 32, 4>(A, W, C, p, heads, s);
         case 2: return launch_form<ACCUMULATE, 64, 32, 4, 4, 32, 4>(A, W, C, p, heads, s);
@@ -310,7 +333,10 @@ gemm_rows_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TC* __restr
 
 template <typename TA, typename TC, bool ACCUMULATE, bool VEC>
 int launch_as(const TA* A, const TA* W, TC* C, const Product& p, int heads, cudaStream_t s) {
-    if constexpr (VEC && sizeof(TA) == 4 && sizeof(TC) == 4) return launch_f32<ACCUMULATE>(A, W, C, p, heads, s);
+    if constexpr (VEC && sizeof(TA) == 4 && sizeof(TC) == 4) {
+        const int form = pick_form(p, heads);
+        if (form != ROWS_KERNEL) return launch_f32<ACCUMULATE>(form, A, W, C, p, heads, s);
+    }
     for (int h = 0; h < heads; ++h, A += p.a_head, W += p.w_head, C += p.c_head) {
         if (p.M <= 16)
             cb_launch(gemm_rows_kernel<TA, TC, ACCUMULATE, VEC, 16, 32, 4, 1>, dim3((p.N + 31) / 32, (p.M + 15) / 16),
@@ -363,4 +389,9 @@ CB_EXPORT int cb_gemm_simt_heads(const void* A, const void* W, void* C, int in_d
                                  int M, int N, int K, int lda, int ldw, int ldc, int heads, int a_head, long w_head,
                                  int c_head, void* stream) {
     return dispatch(A, W, C, in_dtype, out_dtype, Product{M, N, K, lda, ldw, ldc, a_head, w_head, c_head}, heads, 0, stream);
+}
+
+// The form that an fp32 product of rows of whole 16-byte pieces takes (`pick_form`), for tests.
+CB_EXPORT int cb_gemm_simt_form(int M, int N, int K, int heads) {
+    return pick_form(Product{M, N, K, K, K, N, 0, 0, 0}, heads);
 }

@@ -175,3 +175,17 @@ def test_products_per_head_are_the_products(rows, n, k, a_head, shift):
     assert torch.equal(got, want)
     with pytest.raises(ops.KernelError):
         ops.linear_heads_plain(a[:, :heads * a_head - a_head + k - 1], a_head, w, got, n)
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 1280, 16), (520, 1284, 136), (1300, 2050, 36), (700, 772, 36), (300, 2050, 20)])
+def test_short_products_are_one_ascending_sum(M, N, K):
+    """Sizes that go by the kernel whose stages are of 16, or by the forms beside its line."""
+    from crucible_b200 import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    want = torch.zeros(M, N, dtype=torch.float64)
+    for k in range(K):                            # (a product of float32 numbers is exact in float64)
+        want = (want + a[:, k].double()[:, None] * w[:, k].double()[None]).float().double()
+    got = torch.full((M, N + 4), 7.0, device=DEV)
+    ops.linear_plain(a.to(DEV), w.to(DEV), got[:, :N])
+    assert torch.equal(got[:, :N].cpu(), want.float()) and bool((got[:, N:] == 7.0).all())

@@ -160,7 +160,7 @@ constexpr int ROWS_KERNEL = -1;
 int pick_form(const Product& p, int heads) {
     auto all = [&](int tm, int tn) { return (long)((p.M + tm - 1) / tm) * ((p.N + tn - 1) / tn) * heads; };
     auto tiles = [&](int tm, int tn) {
-        return (all(tm, tn) + 147) / 148;
+        return (p.M + tm - 1) / tm > 65535 ? 1l << 40 : (all(tm, tn) + 147) / 148;     // (a grid has so many rows at the most)
     };
     const long e[4] = {tiles(16, 16), tiles(32, 32), tiles(64, 32), tiles(64, 64)};
     const long cost[4] = {170 * ((e[0] + 5) / 6) + 46 * e[0], 140 + 175 * e[1], 180 * ((e[2] + 3) / 4) + 275 * e[2],

@@ -189,3 +189,15 @@ def test_short_products_are_one_ascending_sum(M, N, K):
     got = torch.full((M, N + 4), 7.0, device=DEV)
     ops.linear_plain(a.to(DEV), w.to(DEV), got[:, :N])
     assert torch.equal(got[:, :N].cpu(), want.float()) and bool((got[:, N:] == 7.0).all())
+
+
+def test_more_rows_than_tiles_of_sixteen_in_a_grid():
+    from crucible_b200 import ops
+    M, N, K = 16 * 65535 + 40, 8, 20
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    got = torch.full((M, N), 7.0, device=DEV)
+    ops.linear_plain(a, w, got)
+    few = torch.empty(37, N, device=DEV)
+    ops.linear_plain(a[-37:], w, few)
+    assert torch.equal(got[-37:], few)
+    assert float((got.double() - a.double() @ w.double().T).norm() / got.double().norm()) < 1e-6      # (20 roundings of 2^-24)

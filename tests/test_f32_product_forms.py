@@ -18,3 +18,11 @@ ROWS = -1
 def test_the_form_of_a_float32_product(m, n, k, heads, form):
     from crucible_b200.ops import build
     assert build.load("gemm_simt").cb_gemm_simt_form(m, n, k, heads) == form
+
+
+@pytest.mark.parametrize("m,tallest", [(16 * 65535, 16), (16 * 65535 + 1, 32), (32 * 65535, 32), (32 * 65535 + 1, 64), (64 * 65535, 64)])
+def test_a_grid_has_room_for_every_tile_of_rows(m, tallest):
+    """Few columns, for which the smallest tiles are the cheapest: a form whose tiles of rows a grid can hold."""
+    from crucible_b200.ops import build
+    rows = {0: 16, 1: 32, 2: 64, 3: 64, ROWS: 64}[build.load("gemm_simt").cb_gemm_simt_form(m, 8, 64, 1)]
+    assert rows >= tallest and -(-m // rows) <= 65535

@@ -153,8 +153,8 @@ int launch_form(const float* A, const float* W, float* C, const Product& p, int 
 //   against 8.0), at 64 x 32 to 144;
 // - at K below 640 where an SM gets 4 and a part of the 64 x 64 tiles: four fit it, so the rest wait (1,300 x 2,050 x 128 22.4
 //   against 25.6, x 520 79 against 86, x 768 110 against 106).
-// Five to sixteen rows of many columns at a K of one or two stages: the second form before the first (16 x 4,608 x 64 1.16 times
-// as fast, and as the kernel before).  With this choice no size is slower than gemm_rows_kernel's by more than 5 %, but
+// Five to sixteen rows of many columns at a K of one or two stages: the second form before the first (16 x 2,050 x 72 1.14 times
+// as fast), and gemm_rows_kernel before both from 288 tiles on (16 x 9,216 x 72 3.7, 4.6 and 4.9 us).  With this choice no size is slower than gemm_rows_kernel's by more than 5 %, but
 // 1,000 rows of 16 columns at K = 16 (2.5 against 2.3 us).
 constexpr int ROWS_KERNEL = -1;
 int pick_form(const Product& p, int heads) {
@@ -170,7 +170,8 @@ int pick_form(const Product& p, int heads) {
         if (cost[i] < cost[form]) form = i;
     const bool few = p.M <= 16;
     if (p.K <= 16 && (few || all(64, 64) >= 10)) return ROWS_KERNEL;
-    if (few) return form == 0 && p.M > 4 && p.K <= 80 && all(16, 16) >= (p.K > 64 ? 80 : 149) ? 1 : form;
+    if (few && form == 0 && p.M > 4 && p.K <= 80 && all(16, 16) >= (p.K > 64 ? 80 : 149)) return all(16, 16) >= 288 ? ROWS_KERNEL : 1;
+    if (few) return form;
     const bool half = p.K % 32 >= 1 && p.K % 32 <= 16;
     if (form == 3 && half && (p.K <= 48 || (e[3] >= 2 && p.K < (e[3] == 2 ? 544 : 512)))) return ROWS_KERNEL;
     if (form == 3 && e[3] == 5 && p.K < 640) return ROWS_KERNEL;

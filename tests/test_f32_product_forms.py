@@ -14,7 +14,7 @@ ROWS = -1
     # four and a part of the tiles to an SM
     (1300, 2050, 128, 1, ROWS), (1300, 2050, 768, 1, 3), (2050, 2050, 128, 1, 3), (65, 1280, 128, 11, 3), (64, 1280, 128, 33, ROWS),
     # few rows of many columns, short K
-    (16, 4608, 64, 1, 1), (16, 4608, 100, 1, 0), (4, 4608, 64, 1, 0), (16, 1280, 72, 1, 1), (16, 768, 72, 1, 0)])
+    (16, 4592, 64, 1, 1), (16, 4608, 64, 1, ROWS), (8, 9216, 72, 1, ROWS), (16, 4608, 100, 1, 0), (4, 4608, 64, 1, 0), (16, 1280, 72, 1, 1), (16, 768, 72, 1, 0)])
 def test_the_form_of_a_float32_product(m, n, k, heads, form):
     from crucible_b200.ops import build
     assert build.load("gemm_simt").cb_gemm_simt_form(m, n, k, heads) == form

@@ -255,6 +255,8 @@ def _gemm(a, w, out, n, epi, bn, per_sm=1, splits=None, emit=None, pre=None, pai
 
 
 WAVES_MIN_TILES = 200       # tiles of 128 x 256 from which one block an SM walks them (`_gemm_waves`)
+F32_WAVES_MIN_TILES = 210   # ... for float32 results by a long K
+TALL_COST = 711             # a wave of tall tiles, where a wave of tiles of bn columns costs bn + 128
 
 
 @functools.lru_cache(maxsize=4096)
@@ -267,16 +269,28 @@ def _waves_width(m: int, n_cols: int, k: int, epi: int) -> int:
     2 x 2,816 (198 tiles) 23.7 -> 24.4.  bfloat16 results gain 3 to 7 % at the width that a block a tile would
     have: with 256 columns from two waves on (8,192 by 2,048 at 1,100 / 1,600 rows 28.2 / 43.0 -> 26.4 / 39.9),
     with 192 from three on or at a short K (2,048 rows of 5,120 by 2,048 34.0 -> 32.9, of 3,072 by 1,024 14.6 ->
-    13.6; two waves by 2,048, 1,100 rows of 4,608, 21.5 -> 21.9)."""
+    13.6; two waves by 2,048, 1,100 rows of 4,608, 21.5 -> 21.9), and beyond K = 2,048 from four (by 4,096, 1,600 rows of
+    6,144 64.6 -> 67.7, 1,800 79.5 -> 75.0).
+    float32 results of more than 128 rows by a K of more than 1,024 want 1.4 waves (1,300 rows of 4,096 by 2,048, 1.2 waves,
+    23.2 -> 24.4, by 4,096 37.8 -> 43.3), and from K = 1,024 on stay with one to three waves of tall tiles unless that many
+    waves here cost clearly less (2,048 rows of 4,096 by 2,048 27.1 -> 27.9, of 8,192 56.4 -> 62.8; 1,100 of 6,144 28.2 -> 24.5,
+    1,300 of 16,384 91.0 -> 76.9)."""
     m_tiles = -(-m // 128)
     waves = lambda bn: -(-m_tiles * -(-n_cols // bn) // N_SMS)
     if epi == STORE_F32 and waves(256) > 1:
-        return min((waves(bn) * (bn + 64), bn) for bn in (192, 256))[1]
+        if k > 1024 and m_tiles > 1 and m_tiles * -(-n_cols // 256) < F32_WAVES_MIN_TILES:
+            return 0
+        cost, bn = min((waves(bn) * (bn + 64), bn) for bn in (192, 256))
+        if k >= 1024 and _tall_tiles(m, n_cols, k):
+            tall = -(--(-m // 256) * -(-n_cols // 256) // N_SMS)
+            if tall <= 3 and cost > 0.83 * tall * TALL_COST:
+                return 0
+        return bn
     if epi == SWIGLU_BF16:
         return 256 if m_tiles * -(-n_cols // 256) >= WAVES_MIN_TILES else 0
     if epi == STORE_BF16:
         bn = _tile_width(m, n_cols, epi)[0]
-        least = {256: 2, 192: 2 if k <= 1024 else 3}.get(bn)
+        least = {256: 2, 192: 2 if k <= 1024 else 3 if k <= 2048 else 4}.get(bn)
         return bn if least is not None and waves(bn) >= least else 0
     return 0
 
@@ -411,7 +425,7 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
 def _product_cost(m: int, n_cols: int, k: int):
     """The cost by which `_tile_width` chooses, of its choice or of tall tiles, and the tile."""
     if _tall_tiles(m, n_cols, k):
-        return -(--(-m // 256) * -(-n_cols // 256) // N_SMS) * 711, (256, 0)
+        return -(--(-m // 256) * -(-n_cols // 256) // N_SMS) * TALL_COST, (256, 0)
     bn, per_sm = _tile_width(m, n_cols, STORE_BF16, 64)
     return -(--(-m // 128) * -(-n_cols // bn) // N_SMS) * (bn + 128), (bn, per_sm)
 
@@ -471,6 +485,13 @@ def grouped_tile(pairs: int, n_experts: int, n_cols: int, gated: bool):
     return min((-(-int(math.ceil(tiles * -(-n_cols // bn))) // N_SMS) * (bn + 160), bn) for bn in (128, 192, 256))[1], 1
 
 
+def grouped_waves(pairs: int, n_experts: int, n_cols: int) -> bool:
+    """Whether a grouped product over `n_cols` rows of an expert's matrix goes by `_gemm_waves`: full tiles beside a
+    half-filled one an expert (4,096 pairs of 8 experts of 2,816 x 2,048 gate/up 99.8 -> 90.6 us, down 53.8 -> 49.2;
+    2,048 pairs 56.6 -> 53.8 and, below the line, 39.0 -> 45.7)."""
+    return (pairs / 128 + n_experts / 2) * -(-n_cols // 256) >= WAVES_MIN_TILES and pairs >= 64 * n_experts
+
+
 def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pair=None, tile=None) -> bool:
     """The grouped product of a mixture of experts (`cb_gemm_tcgen05_grouped`): `a` [pairs, K]
     bfloat16 rows expert by expert, `w` [experts, rows, K] a declared weight, `plan` the int32
@@ -487,10 +508,7 @@ def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pai
     if pair is not None:
         args.glu_limit, args.glu_alpha, args.glu_offset = (float(v) for v in pair)
     args.plan, args.n_experts, args.max_tiles, args.w_rows = plan.data_ptr(), n_experts, tiles, w.shape[1]
-    # (full tiles beside a half-filled one an expert: 4,096 pairs of 8 experts of 2,816 x 2,048 gate/up 99.8 -> 90.6 us,
-    # down 53.8 -> 49.2; 2,048 pairs 56.6 -> 53.8 and, below the line, 39.0 -> 45.7)
-    if (tile is None and (a.shape[0] / 128 + n_experts / 2) * -(-w.shape[1] // 256) >= WAVES_MIN_TILES
-            and a.shape[0] >= 64 * n_experts and _gemm_waves(a, w, out, n, epi, 256, plan=args)):
+    if (tile is None and grouped_waves(a.shape[0], n_experts, w.shape[1]) and _gemm_waves(a, w, out, n, epi, 256, plan=args)):
         return True
     bn, per_sm = tile or grouped_tile(a.shape[0], n_experts, w.shape[1], gated)
     lib = build.load("gemm_tcgen05")

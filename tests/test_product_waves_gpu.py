@@ -90,3 +90,45 @@ def test_grouped_products_in_waves(rows, gated):
             assert r == 0 or _close(out[at:at + r], _gated(p) if gated else p, 7.5 if dtype == torch.bfloat16 else 17)
             at += r
     tc.check_status(DEV)
+
+
+def test_the_dispatch_reaches_it(monkeypatch):
+    """Through the products' own entry points, at sizes on either side of the lines: which calls it ran, and that
+    it refused none; the results against the kernel of a block a tile."""
+    from types import SimpleNamespace
+    from crucible_b200 import ops
+    from crucible_b200.engine.context import Scratch
+    from crucible_b200.ops import moe, tensor_core as tc
+    calls, own = [], tc._gemm_waves
+    monkeypatch.setattr(tc, "_gemm_waves", lambda *a, **kw: calls.append(own(*a, **kw)) or calls[-1])
+    ctx = SimpleNamespace(scratch=Scratch(DEV).get)
+    for m, n, k, kind, there in ((2050, 776, 136, "bf16", False), (1100, 8192, 64, "bf16", True), (1300, 4096, 128, "f32", True),
+                                 (1100, 4096, 128, "f32", False), (300, 512, 64, "pair", False), (1664, 2048, 72, "pair", True)):
+        a, w, want = _inputs(m, n * (2 if kind == "pair" else 1), k, m)
+        ops.declare_weights(w)
+        out = torch.full((m, n), 7.0, device=DEV, dtype=torch.float32 if kind == "f32" else torch.bfloat16)
+        calls.clear()
+        if kind == "pair":
+            ops.linear_swiglu(a, w, out, ctx)
+        else:
+            ops.linear(a, w, out)
+        assert calls == [True] * there, (m, n, k, kind)
+        assert _close(out, _gated(want) if kind == "pair" else want, 17 if kind == "f32" else 7.5)
+    experts, k, n = 2, 64, 1024
+    for each, there in ((3200, True), (256, False)):
+        tiles = experts * -(-each // 128)
+        plan = torch.zeros(2 + experts + 3 * tiles, dtype=torch.int32)
+        plan[0] = tiles
+        for i in range(tiles):
+            e, r = divmod(i * 128, -(-each // 128) * 128)
+            for j, v in enumerate((e, e * each + r, min(128, each - r))):
+                plan[2 + experts + j * tiles + i] = v
+        a, w, _ = _inputs(experts * each, experts * n, k, each)
+        w = w.view(experts, n, k)
+        out = torch.full((experts * each, n), 7.0, device=DEV)
+        calls.clear()
+        assert moe.grouped_linear(a, w, out, plan.to(DEV), experts, tiles, False)
+        assert calls == [True] * there
+        want = torch.cat([a[e * each:(e + 1) * each].double() @ w[e].double().T for e in range(experts)])
+        assert _close(out, want, 17)
+    tc.check_status(DEV)

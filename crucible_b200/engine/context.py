@@ -278,15 +278,30 @@ class HostStep:
         n = self.lead_single
         return self._bucket(max(self.context_len[:n])) if n else 0
 
+    ONE_TILE = 128           # keys: contexts up to here are a class of their own for the choice of a kernel
+
+    @cached_property
+    def context_reach(self) -> int:
+        """`context_bucket`, or 128 where no context is longer: what a kernel's choice may go by."""
+        return self.ONE_TILE if self.max_context_len <= self.ONE_TILE else self.context_bucket
+
+    @cached_property
+    def lead_context_reach(self) -> int:
+        """`context_reach` over the leading single-token requests alone (0: none)."""
+        n = self.lead_single
+        if n and max(self.context_len[:n]) <= self.ONE_TILE:
+            return self.ONE_TILE
+        return self.lead_context_bucket
+
     SMALL_STEP_TOKENS = 16
 
     def shape_key(self) -> tuple:
         """What, beside the counts of rows, requests and wanted rows, a kernel's launch
         shape may depend on: the most new tokens of a request, the number of leading
-        single-token requests, and the context buckets of the requests that may run
+        single-token requests, and the context buckets (`context_reach`) of the requests that may run
         split over their keys (all of them when every request brings few tokens; the
         leading single-token ones otherwise).  Steps with equal keys launch the same
         kernels with the same grids."""
         small = self.max_new_tokens <= self.SMALL_STEP_TOKENS
         return (self.max_new_tokens, self.lead_single,
-                self.context_bucket if small else 0, self.lead_context_bucket)
+                self.context_reach if small else 0, self.lead_context_reach)

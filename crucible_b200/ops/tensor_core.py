@@ -635,13 +635,14 @@ class _Requests:
     tokens any of them brings, the context bucket that covers them, and the number of
     the step's rows up to its end (the split form's scratch is indexed by row)."""
 
-    def __init__(self, ctx, table, first: int, count: int, max_new: int, bucket: int, rows_end: int):
+    def __init__(self, ctx, table, first: int, count: int, max_new: int, bucket: int, rows_end: int, reach=None):
         self.row_start = ctx.req_row_start.data_ptr() + 4 * first         # (addresses of int32)
         self.first_pos = ctx.req_first_pos.data_ptr() + 4 * first
         self.table_stride = table.shape[1]
         self.table = table.data_ptr() + 4 * first * table.stride(0)
         self.first, self.whole_table = first, table
         self.count, self.max_new, self.bucket, self.rows_end = count, max_new, bucket, rows_end
+        self.reach = bucket if reach is None else reach
 
 
 def _tcgen05_rows(head_dim, k_cache, v_cache) -> bool:
@@ -713,29 +714,53 @@ def _attention_decode_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_he
 SHORT_ATTENTION = True       # tests switch it off to reach the split kernels with the same inputs
 
 
-def short_attention_pays(blocks: int, reach: int, head_dim: int, plain: bool) -> bool:
-    """Whether single tokens that read up to `reach` keys (the context's bucket, or the window) take one block a
+# A sink or a gate, by (features of a head, whether more than four query heads share a key/value head): the blocks from
+# which contexts of up to so many keys go by one block each.
+SHORT_SINK_BLOCKS = {(64, False): ((1024, 0), (1536, 32), (2048, 48), (3840, 64), (8192, 80)),
+                     (64, True): ((512, 0), (768, 24), (1024, 64), (2048, 96)),
+                     (128, False): ((1024, 0), (2048, 48), (8192, 80)),
+                     (128, True): ((256, 0), (512, 32), (768, 64), (1536, 96))}
+
+
+def short_attention_pays(blocks: int, reach: int, head_dim: int, plain: bool, heads_a_group: int = 1, tokens: int = 1) -> bool:
+    """Whether single tokens that read up to `reach` keys (the longest context's class, or the window) take one block a
     request and key/value head (`blocks` of them) instead of keys split over blocks.  Without splitting
-    nothing is merged, but the keys beyond what the warps hold are walked: 3 us a 256 keys of 128 features.
-    `plain`: against the tcgen05 kernel, else (a sink, a gate) the mma.sync one, whose launch and merge cost more.
-    Whole layers of 16 or 8 heads, split and short, us: plain, 250 keys, 1 to 48 tokens, 1.02 to 1.2 times as
-    fast; 500 keys 8 tokens of 64 features 14.9 and 13.7, of 128 17.7 and 18.1, 24 of 128 33.6 and 31.1; 1,000 keys 1 token 12.7
-    and 15.7, 40 of 128 41.5 and 35.9.  With sink and gate up to 1,024 keys 1.03 to 2.3 times (a window of 1,024,
-    48 tokens of 128 102 and 60); 3,700 keys 8 tokens 50 and 61, 40 244 and 102."""
-    if plain:
-        return (reach <= 256 or (reach <= 512 and (blocks <= N_SMS if head_dim == 64 else blocks >= 48))
-                or (reach <= 1024 and head_dim == 128 and blocks >= 80))
-    return reach <= 1024 or blocks >= 64
+    nothing is merged, but a block walks its keys alone: 1.7 us a 256 keys of 64 features and 2.9 of 128, with more
+    than four heads a group 2.6 and 4.8.  `reach` is the longest of the step, so every line was measured with
+    all contexts as long and with one so long among others of 200 keys, and lies where both are as fast or faster.
+
+    `plain`: against the tcgen05 kernel, which has nothing to merge up to 128 keys.  us, split and short: a pass of a prompt and
+    eight steps of the 120M shape (12 heads of 64, 4 key/value heads), 4 tokens, behind 100 keys 2,355 and 2,432, behind 180
+    2,610 and 2,497; 16 behind 40 3,046 and 3,120, 17 3,727 and 3,718; 32 (128 blocks) behind 180 4,504 and 4,323, 48 (192) 4,809 and
+    4,820; whole layers of 16 heads of 128 and 4 key/value heads: 1 token behind 100 keys 33.4 and 31.6, 250 keys 36.7
+    and 31.8, 400 keys 4 tokens 37.3 and 38.2, 16 (64 blocks) 52.9 and 48.1, 1,000 keys 24 tokens (96) 73.8 and 72.4, 48
+    (192) 89.8 and 90.0; eight heads a group, 4 tokens behind 250 keys 39.6 and 38.2, 400 40.0 and 43.3.
+    Else against the mma.sync kernel, whose launch and merge cost more: 8 tokens of 128 behind 240 keys 30.9 and 22.6, 1,000
+    33.5 and 30.8, 2,000 (32 blocks) 41.4 and 43.3; 16 (64) behind 2,000 59.4 and 47.1; 40 (160) behind 3,700 248 and 104; one
+    of 24 behind 8,000 keys and the others behind 200 (96) 1.5 times as fast, 16 tokens (64) all behind 8,000 0.89."""
+    many = heads_a_group > 4
+    if not plain:
+        return any(reach <= keys and blocks >= least for keys, least in SHORT_SINK_BLOCKS[head_dim, many])
+    if reach <= 128 and (many if head_dim == 128 else tokens <= 16):
+        return False
+    if head_dim == 64:
+        return blocks <= N_SMS and (reach <= 256 or (reach <= 512 and (not many or blocks >= 24)))
+    if many:
+        return reach <= 256
+    return (reach <= 256 or (reach <= 512 and blocks >= 48) or (reach <= 768 and blocks >= 80)
+            or (reach <= 1024 and 80 <= blocks <= N_SMS))
 
 
-def short_attention(q, out, k_cache, v_cache, ctx, table, count: int, bucket: int, n_heads: int, n_kv_heads: int, head_dim: int,
+def short_attention(q, out, k_cache, v_cache, ctx, table, count: int, reach: int, n_heads: int, n_kv_heads: int, head_dim: int,
                     scale: float, window, page_tokens: int, sinks=None, out_scale: float = 1.0, gate=None,
                     gate_per_head: bool = False, plain: bool = False) -> bool:
     """`csrc/attention_short.cu` for the step's first `count` requests, which bring one token each and whose contexts
-    (`bucket` at most), or windows, are short.  A rule of the step's shape and of the sizes.  False: not taken."""
+    (`reach` at most), or windows, are short.  A rule of the step's shape and of the sizes.  False: not taken."""
     if (not SHORT_ATTENTION or head_dim not in (64, 128) or n_heads > 8 * n_kv_heads or q.stride(0) % 8 or q.data_ptr() % 16
             or k_cache.shape[-1] != head_dim or v_cache.shape[-1] != head_dim or k_cache.dtype != torch.bfloat16
-            or not short_attention_pays(count * n_kv_heads, bucket if window is None else min(bucket, window), head_dim, plain)):
+            # (a short window's keys may lie in two of the split kernel's chunks, a short context's do not)
+            or not short_attention_pays(count * n_kv_heads, reach if window is None or reach <= 128 else
+                                        min(reach, max(window, 129)), head_dim, plain, n_heads // n_kv_heads, count)):
         return False
     code = build.load("attention_short").cb_attention_short(
         q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), gate.data_ptr() if gate is not None else 0,
@@ -873,7 +898,7 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
     shape (count, most new tokens, bucket) and of the sizes only."""
     n_rep = n_heads // n_kv_heads
     if (reqs.max_new == 1 and reqs.first == 0 and USE_TCGEN05_DECODE
-            and short_attention(qkv, out, k_cache, v_cache, ctx, reqs.whole_table, reqs.count, reqs.bucket, n_heads,
+            and short_attention(qkv, out, k_cache, v_cache, ctx, reqs.whole_table, reqs.count, reqs.reach, n_heads,
                                 n_kv_heads, head_dim, scale, window, cache.page_tokens, plain=True)):
         return True
     split = reqs.max_new * n_rep <= SPLIT_ROWS
@@ -951,7 +976,7 @@ def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx,
     args = (n_heads, n_kv_heads, head_dim, scale, window, ctx, cache)
     lead = host.lead_single
     if 0 < lead < ctx.n_requests and host.max_new_tokens * n_rep > SPLIT_ROWS:
-        decoding = _Requests(ctx, table, 0, lead, 1, host.lead_context_bucket, lead)
+        decoding = _Requests(ctx, table, 0, lead, 1, host.lead_context_bucket, lead, host.lead_context_reach)
         portions = _Requests(ctx, table, lead, ctx.n_requests - lead, host.max_new_tokens,
                              host.context_bucket, ctx.n_tokens)
         if not _attend(qkv, out, k_cache, v_cache, decoding, *args):
@@ -961,7 +986,7 @@ def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx,
                                "refused its portions: a rule of sizes is inconsistent")
         return True
     whole = _Requests(ctx, table, 0, ctx.n_requests, host.max_new_tokens, host.context_bucket,
-                      ctx.n_tokens)
+                      ctx.n_tokens, host.context_reach)
     return _attend(qkv, out, k_cache, v_cache, whole, *args)
 
 

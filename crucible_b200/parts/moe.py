@@ -97,9 +97,13 @@ class MixtureOfExperts(FeedForward):
     # alone, so prompt steps are captured as graphs like decode steps.
     SMALL_MAX_PAIRS = 256        # up to this many pairs the experts' weight rows are read by a warp each
     # From this many (token, expert) pairs on, by the bytes of an expert, the experts run as two grouped
-    # products over their rows side by side; below, a warp reads a weight row.  A layer, the shared expert
-    # riding, warps and grouped: 8 experts of 2,816 x 2,048, two a token, 1 token 46.3 and 45.2 us, 2 69.8 and 54.7,
-    # 4 88 and 58, 7 157 and 77; of 1,408 x 1,024, 2 tokens 26.0 and 27.6, 3 32 and 27.7, 7 41 and 29.
+    # products over their rows side by side; below, a warp reads a weight row (`_grouped`: with many experts later, and a
+    # shared expert's slices that ride count).  Layers with cold weights, us, warps and grouped: 8 experts of 2,816 x 2,048 and a
+    # shared one, top 1, 1 token 39 and 43, 2 50 and 46; top 2, 1 token 48 and 47, 2 66 and 52, 7 157 and 77; 16 of that size
+    # without, 1 token of top 4 59 and 58, of top 6 72 and 66; 64 of 1,408 x 2,048, 1 token of top 4 40 and 44, of top 6 52 and
+    # 53, of top 8 65 and 58; 128 of 1,536 x 4,096, top 8, 1 token 108 and 115, 2 182 and 153; 32 of 1,408 x 1,024, 1 token of
+    # top 6 35 and 39, of top 8 44 and 42; 128 of 768 x 2,048, 2 tokens of top 4 44 and 49, of top 8 68 and 67, 3 86 and 76;
+    # 64 of 512 x 1,024 and a shared one of two, 2 tokens of top 6 40 and 34.
     SORTED_MIN_PAIRS = ((16 << 20, 4), (4 << 20, 6), (0, 16))
     MAX_EXPERTS = 256
     RIDE_GROUPED_ROWS = 32       # the same where the experts run as grouped products (a decode step of 16 rows,
@@ -228,10 +232,17 @@ class MixtureOfExperts(FeedForward):
             return False
         return t <= (self.RIDE_PLAIN_ROWS if self._grouped(t) else self.RIDE_MAX_ROWS)
 
+    def _least_pairs(self) -> int:
+        """The pairs from which grouped products are chosen: what a grouped launch pays for every expert there is
+        moves the line up, more where an expert's own weights are little."""
+        size = 6 * self.spec.width * self.ff
+        least = next(n for s, n in self.SORTED_MIN_PAIRS if size >= s)
+        return max(least, self.n // 8) if size >= 16 << 20 else least + self.n // 16 if size >= 4 << 20 else least
+
     def _grouped(self, t: int) -> bool:
         d, f = self.spec.width, self.ff
         return (self.dtype == torch.bfloat16 and d % 8 == 0 and f % 8 == 0
-                and t * self.top >= next(n for size, n in self.SORTED_MIN_PAIRS if 6 * d * f >= size))
+                and t * (self.top + self.slices) >= self._least_pairs())
 
     def forward_open(self, ctx, h) -> OpenSum:
         """The experts' rows and what the shared expert adds if it joins their sum, not yet summed."""

@@ -205,17 +205,18 @@ class MixtureOfExperts(FeedForward):
         self.gate_up = torch.stack(gate_up, 0).contiguous()          # [E + slices, 2F, d]
         self.down = torch.stack(down, 0).contiguous()                # [E + slices, d, F]
         ops.declare_weights(self.router, self.gate_up, self.down)
-        # the shared expert as dense products, for steps of many rows
-        self.dense = []
-        if self.joins:
-            if self.slices:
-                self.dense = [(self.gate_up[self.n + s], self.down[self.n + s]) for s in range(self.slices)]
-            else:
-                self.dense = [(torch.cat([tensors["shared.gate"], tensors["shared.up"]], 0).contiguous(),
-                               tensors["shared.down"])]
-                ops.declare_weights(*self.dense[0])
+        # The shared expert as dense products, for steps of many rows: over the slices where there are some, so that its
+        # weights are held once.  A plain one of several slices, though, is held a second time in one piece (6 bytes x
+        # width x its size a layer): its products slice by slice take longer, two of 1,408 x 2,048 beside 16 experts
+        # 116 us instead of 101 at 129 rows, 257 instead of 245 at 2,048.
+        self.dense = [(self.gate_up[self.n + s], self.down[self.n + s]) for s in range(self.slices)]
+        self.apart = self.shared is not None and (self.slices == 0 or (self.slices > 1 and self.shared_ff % 8 == 0))
+        if self.joins and not self.slices:
+            self.dense = [(torch.cat([tensors["shared.gate"], tensors["shared.up"]], 0).contiguous(),
+                           tensors["shared.down"])]
+            ops.declare_weights(*self.dense[0])
         self.count = torch.zeros(self.n + self.slices, dtype=torch.int32, device=device)     # zero between steps
-        if self.shared is not None:
+        if self.apart:
             self.shared.bind({k[len("shared."):]: v for k, v in tensors.items() if k.startswith("shared.")},
                              dtype, device)
 
@@ -223,7 +224,12 @@ class MixtureOfExperts(FeedForward):
         o = self.forward_open(ctx, h)
         kernels.combine(o.rows, o.top, residual, by_plan=o.by_plan, shared=o.shared, gate=o.gate)
         if self.shared is not None and not self._rides(h.shape[0]):
-            self.shared.forward(ctx, h, residual)
+            if self.apart:
+                return self.shared.forward(ctx, h, residual)
+            for i, (gate_up, down) in enumerate(self.dense):
+                act = ctx.scratch("ffn.act", (h.shape[0], self.ff), self.dtype)
+                ops.linear_swiglu(h, gate_up, act, ctx)
+                ops.linear(act, down, residual, accumulate=True, closes=ctx if i + 1 == self.slices else None)
 
     def _rides(self, t: int) -> bool:
         """Whether a shared expert that does not join the others' sum rides with them all the same: in grouped

@@ -18,3 +18,31 @@ def test_where_experts_run_as_grouped_products(width, ff, experts, top, shared, 
     assert part._grouped(tokens) and (tokens == 1 or not part._grouped(tokens - 1))
     part.dtype = torch.float32
     assert not part._grouped(64)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shared,slices,copies", [(0, 0, 1), (64, 1, 1), (60, 1, 1), (100, 0, 1), (124, 2, 1), (120, 2, 2)])
+def test_a_shared_expert_is_held_once(shared, slices, copies, dtype):
+    """One whose slice rides with the routed experts has no second copy for the steps in which it does not; one of several
+    slices has, unless it is of a size that the dense products refuse."""
+    from crucible_b200.config.model_config import FeedForwardSpec
+    from crucible_b200.parts import FEED_FORWARDS
+    width, ff, experts = 32, 64, 4
+    options = (("experts", experts), ("top", 2)) + ((("shared_intermediate", shared),) if shared else ())
+    part = FEED_FORWARDS.build("moe", FeedForwardSpec("moe", width, ff, options))
+    given = {t.name: torch.randn(t.shape).to(dtype) for t in part.tensors()}
+    part.bind(given, dtype, torch.device("cpu"))
+    held, todo = {}, [part]
+    while todo:
+        x = todo.pop()
+        if isinstance(x, torch.Tensor):
+            held[x.untyped_storage().data_ptr()] = x.untyped_storage().nbytes()
+        elif isinstance(x, (list, tuple)):
+            todo += x
+        elif x is part or (x is not None and x is part.shared):
+            todo += vars(x).values()
+    size = torch.finfo(dtype).bits // 8
+    matrices = sum(t.numel() for n, t in given.items() if n != "router")
+    assert part.slices == (slices if dtype == torch.bfloat16 else 0)
+    more = 3 * width * (part.slices * ff - shared if part.slices and copies == 1 else part.slices * ff)
+    assert sum(held.values()) == (matrices + more + given["router"].numel()) * size + 4 * (experts + part.slices)

@@ -14,10 +14,14 @@
 //            memory, 16 bytes for four heads
 //   merge    the warps' and lanes' shares, with the sink if there is one; then the gate, and one rounding
 //
-// us a layer with its two products, split kernels -> here: 8 tokens behind 250 keys, 12 heads' worth of the 120M
-// shape's sizes and up: 16 heads of 64 14.0 -> 12.4, of 128 17.3 -> 14.9; with sink and gate 28.9 -> 20.2, 48 tokens
-// in a window of 1,024 102 -> 60 (`short_attention_pays` has the line).  A chain of about 4.5 us from the wait to
-// the rows for one pass of keys, 3 more for every other.
+// us a layer with its two products, split kernels -> here, 8 tokens behind 250 keys, 16 heads: of 64 14.0 -> 12.4, of 128 17.3
+// -> 14.9; with sink and gate 28.9 -> 20.2, 48 tokens in a window of 1,024 102 -> 60.  A chain of about 4.5 us from the
+// wait to the rows for one pass of keys; every 256 keys more are 1.7 us with heads of 64 and 2.9 of 128, 2.6 and 4.8 with more
+// than four heads a group, and a block walks them alone (`short_attention_pays` has the lines).
+//
+// Keys and values of a pass are in registers together, which takes all there are: 250 to 255 of a thread's with heads of 128
+// (8 heads a group: 112 bytes spilled), and with heads of 64 and up to four a group the 128 (four: 80 bytes spilled) with
+// which sixteen warps, or two blocks of eight, fit an SM.
 //
 // Reference counterpart: `attention_decode` (engine/kernels/kernels.cu:1740), one block per head over all keys.
 #define CB_PDL_BIT 2      // this file's bit in CRUCIBLE_PDL (shared with attention_decode_tcgen05.cu)

@@ -11,10 +11,11 @@
 // are the epilogue: a group takes 64 bytes of its columns of all 128 rows at a time from tensor memory into
 // one of its two buffers (64-byte swizzle) and sends it by TMA: a store, or an fp32 add at the memory side.
 //
-// Epilogues and forms as in `gemm_tcgen05.cu`: STORE_BF16 (with an activation), STORE_F32, ACCUM_F32, SWIGLU_BF16;
-// rows ahead of their norm (NormArgs::sumsq_in) with SWIGLU_BF16; a grouped product (NormArgs::plan).  In
-// a grouped product a tile that ends before its 128 rows leaves its buffers row by row, 64 bytes a row,
-// since the rows behind it are another expert's.
+// Epilogues and forms as in `gemm_tcgen05.cu`: STORE_BF16 (with an activation), STORE_F32, SWIGLU_BF16; rows ahead of their
+// norm (NormArgs::sumsq_in) with SWIGLU_BF16; a grouped product (NormArgs::plan), of 256 columns a tile.  The rules
+// (`_waves_width`, `grouped_waves`) choose 192 or 256 columns; 128, and ACCUM_F32 (a TMA add instead of the store), no rule
+// chooses yet: the tests of the tile walk run them, for its edges at three widths.  In a grouped product a tile that ends
+// before its 128 rows leaves its buffers row by row, 64 bytes a row, since the rows behind it are another expert's.
 //
 // us at 2,048 rows, a block a tile (or tall) -> here: gated pair of 2 x 2,816 by K = 2,048 43.2 -> 35.3 (1,338 TFLOP/s),
 // of 2 x 2,048 by 768 15.8 -> 13.3; fp32 results of 4,096 by 128 10.2 -> 8.6; 4,096 rows of 8 experts, gate/up of
@@ -375,11 +376,12 @@ template <int BN, int STAGES>
 int launch(int epi, const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, int ldc, int* status,
            cudaStream_t s, const NormArgs& na) {
     if (na.plan != nullptr) {
-        switch (epi) {
-            case STORE_BF16: return launch_form<BN, STAGES, STORE_BF16, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
-            case STORE_F32: return launch_form<BN, STAGES, STORE_F32, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
-            case SWIGLU_BF16:
-                if constexpr (BN % 128 == 0) return launch_form<BN, STAGES, SWIGLU_BF16, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
+        if constexpr (BN == 256) {
+            switch (epi) {
+                case STORE_BF16: return launch_form<BN, STAGES, STORE_BF16, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
+                case STORE_F32: return launch_form<BN, STAGES, STORE_F32, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
+                case SWIGLU_BF16: return launch_form<BN, STAGES, SWIGLU_BF16, GROUPED>(ma, mw, C, M, N, K, ldc, status, s, na);
+            }
         }
         return CB_ERR_UNSUPPORTED;
     }
@@ -401,7 +403,7 @@ int launch(int epi, const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M
 }  // namespace
 
 // As `cb_gemm_tcgen05` and, with a plan in `norm`, `cb_gemm_tcgen05_grouped` (whose plan's tiles have 128 rows).
-// bn: tile width: 128, 192 (not SWIGLU_BF16) or 256.
+// bn: tile width: 128, 192 (not SWIGLU_BF16) or 256; 256 alone with a plan.
 CB_EXPORT int cb_gemm_waves(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc, int epi,
                             int bn, int* status, void* stream, const void* norm) {
     if (M <= 0 || N <= 0) return 0;

@@ -26,6 +26,8 @@ by their sum.)
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from .. import ops
@@ -238,6 +240,7 @@ class MixtureOfExperts(FeedForward):
             return False
         return t <= (self.RIDE_PLAIN_ROWS if self._grouped(t) else self.RIDE_MAX_ROWS)
 
+    @functools.cached_property
     def _least_pairs(self) -> int:
         """The pairs from which grouped products are chosen: what a grouped launch pays for every expert there is
         moves the line up, more where an expert's own weights are little."""
@@ -246,9 +249,8 @@ class MixtureOfExperts(FeedForward):
         return max(least, self.n // 8) if size >= 16 << 20 else least + self.n // 16 if size >= 4 << 20 else least
 
     def _grouped(self, t: int) -> bool:
-        d, f = self.spec.width, self.ff
-        return (self.dtype == torch.bfloat16 and d % 8 == 0 and f % 8 == 0
-                and t * (self.top + self.slices) >= self._least_pairs())
+        return (self.dtype == torch.bfloat16 and not (self.spec.width | self.ff) & 7
+                and t * (self.top + self.slices) >= self._least_pairs)
 
     def forward_open(self, ctx, h) -> OpenSum:
         """The experts' rows and what the shared expert adds if it joins their sum, not yet summed."""

@@ -1,32 +1,29 @@
 // Paged causal attention for portions of prompts on the 5th-generation tensor
 // cores (head size 64, 128 or, keys and values at once, 256; bfloat16): S = Q K^T and O += P V are tcgen05.mma with
 // the scores and the output accumulator in tensor memory; K and V pages come in
-// by TMA; the softmax runs on four warps, one thread per query row, reading S
-// from tensor memory and writing P (bf16) to shared memory for the second MMA.
+// by TMA; the softmax has one thread per query row, which reads S from tensor memory and writes P (bf16)
+// back to it for the second MMA.
 //
-// A block takes 128 query rows of one request and one KV head; rows are
+// A block takes up to 128 query rows of one request and one KV head; rows are
 // (position, head within the group) pairs, so every query head that shares the
-// KV head uses the same K and V tiles.  It walks the keys in tiles of 128.
-// Roles: warp 0 loads (one thread: block-table lookups, then one TMA box per tile and
-// operand where the tile's pages follow one another in the pool, else one per page),
-// warp 1 owns tensor memory and issues the MMAs, warps 2-5 are the softmax.
-// S and P are double-buffered: while the softmax works on tile j, the first MMA
-// of tile j+1 and the second MMA of tile j-1 run, so a block's time per tile is
-// the softmax's alone (about 2,000 cycles: 1,260 for the 128 exponentials per thread,
-// their sums and P's way to shared memory, in which the special-function unit's 560 and
-// the other pipes' instructions add up instead of overlapping; the rest maxima, barrier
-// tests of 100 to 200 cycles each, and the scores' way out of tensor memory).
-// Head sizes 64 and 128 with an SM to the block: two such groups of four softmax warps take the
-// tiles in turn (tile j: group j % 2), each with its own buffer of scores and of P, its own
-// reference maximum, sum and accumulator, merged when the keys are through; two tiles are
-// then in work at a time (one group's exponentials beside the other's maxima and waits:
-// 1,750 cycles a tile), and a second thread, of a warp of its own, sends the second products,
-// since one thread cannot send both products of two tiles in time (1,200 cycles a tile).
-// Head size 128 has room for two stages only (227 KB with both buffers of P, all of it), so keys
-// and values come and go by barriers of their own: a tile's keys travel as soon as the first
-// product two tiles back has read its own, beside that tile's softmax, and its values once the
-// second has.  A 2,048-token prompt of 16 heads on 4, a window of 1,024 (256 blocks of up to ten
-// tiles): 86 us with one group, 66 with two.
+// KV head uses the same K and V tiles; a tile holds whole tokens, so that its rows come in by one TMA box
+// per 64 features, as the gate's logits do (fetched by the threads, 16 bytes each, a block of 128 rows of 256
+// features waited 11 us for its queries).  It walks the keys in tiles of 128.
+// Roles: warp 0 loads (a lane a page: table lookups and, where the tile's pages do not follow one another
+// in the pool, one TMA box a page side by side; else one box for the tile), warp 1 owns tensor memory
+// and issues the MMAs, the others are the softmax.
+// P goes back into tensor memory, over the scores that it was made from, and is the first operand of the
+// second product there: shared memory carries queries, keys and values alone (a 128 x 128 x 128 tile: 1,280
+// cycles of its 128 bytes a cycle; with P written to and read from it 1,790, more than the products' 1,024).
+// Two groups of four softmax warps take the tiles in turn (tile j: group j % 2), each with its own
+// buffer of scores, its own reference maximum, sum and accumulator, merged when the keys are through.
+// A tile's code is kept short (64 scores at a time, loops not unrolled): a block lives 10 to 20 us,
+// and code that is met for the first time comes from memory (the masks of 128 scores, unrolled: 7,500 cycles).
+// What bounds it: a tile takes a group some 3,400 cycles (head size 64), of which the special-function unit's
+// 8 a warp and exponential make 1,024 (two groups 2,048), the maxima 400, the scores' way 200 to 900.
+// Measured on one B200, a 2,048-token prompt: 12 heads of 64 on 4 20 us a layer (27 with P in shared memory
+// and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 33 (59), 16 heads of 256 on 1
+// 38 (76).
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
 // tile's maximum exceeds it by more than 2^8 (in the base-2 exponent), so P
@@ -35,10 +32,9 @@
 // exact softmax-weighted mean whatever the reference was.
 //
 // Rows of 256 features that are keys and values at once (a latent with its rotated part: one
-// key head for all query heads): a stage holds the tile once, 64 KB; the first product reads it
+// key head for all query heads): a stage holds the tile once; the first product reads it
 // with the features contracted, the second with the keys contracted.  A tile's 2 x 128 x 128 x 256
-// multiply-adds are 2,048 cycles of the tensor pipe, about what the softmax beside them takes.  A
-// 2,048-token prompt of 16 heads: 441 us on the mma.sync tiles, 85 here (34 GFLOP: 400 TFLOP/s).
+// multiply-adds are 2,048 cycles of the tensor pipe; one softmax group takes 2,700.
 //
 // Sizes: head size 64 or 128, or 256 if the pages' rows are keys and values at once; page size a power of two from 8 to 128; any head
 // counts and group sizes; window.  Anything else is refused and the mma.sync
@@ -46,7 +42,6 @@
 // Reference counterpart: `attention_prefill_exact_*`
 // (engine/kernels/kernels.cu:2257-2275).
 #define CB_PDL_BIT 1      // this file's bit in CRUCIBLE_PDL
-#include <type_traits>
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -77,17 +72,19 @@ struct TcAttnParams {
     const float* sinks;      // [n_heads] or null: exp(sink) joins a row's denominator, with no value
     const __nv_bfloat16* gate;   // logits: every result times sigmoid(logit); rows laid out like `out`, or
     int gate_stride;             // (GATE_HEAD) one logit a head
+    int tile_rows;           // query rows of a tile: whole tokens' groups of heads
+    int q_boxes;             // 1: the queries (and the gate's logits) come in by TMA; tile_rows is 128 else
     int n_pages;             // of the pool
     int runs;                // 1: the 4-D maps may be used for tiles whose pages are consecutive
     int* status;
 };
 
-// Eight results times the sigmoids of their logits.
-__device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(logits);
-    const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] *= 1.0f / (1.0f + expf(-__bfloat162float(g[i])));
+// 1 / (1 + e^-x); 0 for x so low that e^-x is infinite.  (The IEEE division costs a hundred dependent cycles
+// an element; the reciprocal is within one unit in the last place, 2^-15 of what the bf16 result keeps.)
+__device__ __forceinline__ float sigmoid(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.0f + expf(-x)));
+    return y;
 }
 
 // GATE: the results' gate, fixed when it is compiled: the epilogue runs once per block and its instructions
@@ -95,46 +92,37 @@ __device__ __forceinline__ void gate_eight(float* o, const __nv_bfloat16* logits
 // logit a result beside it 0.3 us more, of both gates 1.4).
 enum Gate { GATE_NONE = 0, GATE_RESULT = 1, GATE_HEAD = 2 };
 
-// HD: the head size, 64 or 128.  Operands whose contracted or free dimension is the head
-// size lie in shared memory as HD / 64 halves of [rows][128 bytes] (one swizzle atom wide).
-// Head size 64 has two forms.  The roomy one: four K/V stages, two P buffers, two buffers of
-// scores, two softmax groups, an SM to itself (210 KB, 384 columns of tensor memory: with two
-// tiles in work a tile's keys are asked for three tiles ahead); it is the quicker block,
-// and the right one while all blocks of a launch find a place at once.  The lean one: two
-// stages, one P buffer, one buffer of scores (112 KB, 256 columns), so that two blocks share
-// an SM and one's waits (for a copy, an MMA, the scores' way out of tensor memory) are filled
-// by the other's exponentials; its one buffer of scores is handed back to the MMA thread as
-// soon as the softmax has the scores in registers, so the next tile's first MMA still runs
-// beside this tile's softmax.  It was the right one for launches with more blocks than places
-// while the roomy form had one softmax group (4,096-token prompt of the 120M shape 1.84 against
-// 2.01 ms); with two groups the roomy form is quicker there too (1.68 ms) and the launcher
-// takes it unless told otherwise.  Head size 128: two stages, two P buffers.  256 with one operand
-// for both products: two stages and one P buffer (what 227 KB hold).
-template <int HD, bool LEAN>
+// HD: the head size, 64, 128 or (keys and values at once) 256.  A tile's operand of 64 features a row
+// is one swizzle atom wide: [rows][128 bytes].
+// The ring holds what the loader brings, in the order in which the MMA thread takes it.  Head sizes 64
+// and 128: the keys of the first S_BUFS tiles, then V_t and K_(t + S_BUFS) in turn, one operand tile a slot; two
+// neighbouring slots are one release, of which there are PAIRS.  256:
+// a tile's features 0-127, then 128-255; a slot is free once the second product has read it.  Five
+// slots are what 227 KB hold beside the queries: the upper half of tile t + 2 travels while the
+// second product of tile t reads its own upper half.
+template <int HD>
 struct Storage {
-    static constexpr int STAGES = (HD == 64 && !LEAN) ? 4 : 2;
-    static constexpr int PB = (HD != 256 && !LEAN) ? 2 : 1;
-    static constexpr int S_BUFS = LEAN ? 1 : 2;
-    static constexpr int OPERANDS = HD == 256 ? 1 : 2;      // keys and values, or rows that are both
+    static constexpr bool BOTH = HD == 256;                 // a cached row is key and value
+    static constexpr int PART = BOTH ? 128 : HD;            // features of a slot
+    static constexpr int PARTS = HD / PART;
+    static constexpr int HALVES = PART / 64;
+    static constexpr int PAIRS = HD == 64 ? 4 : 3;
+    static constexpr int SLOTS = BOTH ? 5 : 2 * PAIRS;
+    static constexpr int RELEASES = BOTH ? SLOTS : PAIRS;
+    // buffers of scores: what 512 columns of tensor memory hold beside the accumulators.  With three the
+    // next scores of a group are there when it asks for them; with two they follow its tile's second product.
+    static constexpr int S_BUFS = HD == 64 ? 3 : 2;
     // softmax groups of four warps that take the tiles in turn (tile j: group j % GROUPS), each
     // with its own reference maximum, sum and accumulator, merged at the end
-    static constexpr int GROUPS = (HD != 256 && !LEAN) ? 2 : 1;
-    // two groups on two stages: a stage's keys and its values come and go by barriers of their
-    // own, so that a tile's keys are asked for as soon as the first product two tiles back has
-    // read its own, not when the second has
-    static constexpr bool SPLIT = GROUPS > 1 && STAGES == 2;
-    // loader, MMA thread, four softmax warps a group; two groups: a warp for a second MMA thread
-    static constexpr int THREADS = GROUPS > 1 ? 64 + 128 * GROUPS + 32 : 192;
-    alignas(1024) uint8_t q[HD / 64][ROWS * 64 * 2];
-    alignas(1024) uint8_t kv[STAGES][OPERANDS][HD / 64][KEYS * 64 * 2];
-    alignas(1024) uint8_t p[PB][2][ROWS * 64 * 2];  // P: buffers of two halves of 64 keys
-    alignas(8) uint64_t kv_full[STAGES];
-    uint64_t kv_empty[STAGES];
-    uint64_t v_full[STAGES], v_empty[STAGES];       // split: the values' (kv_*: the keys')
-    uint64_t s_full[2], p_full[2], pv_done[2];
-    uint64_t s_free;                                // lean form: a tile's scores are in registers
-    uint64_t s_taken[2];                            // two groups: buffer b's scores are in registers
-    float2 merge[GROUPS > 1 ? 2 : 1][ROWS];         // two groups: a row's (reference, sum) of each
+    static constexpr int GROUPS = BOTH ? 1 : 2;
+    static constexpr int THREADS = 64 + 128 * GROUPS;       // loader, MMA thread, the softmax groups
+    alignas(1024) uint8_t q[HD / 64][ROWS * 128];
+    alignas(1024) uint8_t ring[SLOTS][HALVES][KEYS * 128];
+    alignas(8) uint64_t full[SLOTS];
+    uint64_t empty[RELEASES];
+    uint64_t q_full, gate_full, o_done;
+    uint64_t s_full[S_BUFS], p_half[S_BUFS], p_full[S_BUFS], pv_done[2];
+    float2 merge[GROUPS][ROWS];                             // a row's (reference, sum) of each group
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -164,37 +152,45 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-// (x0, x1) * a + b in one instruction on the pair
-__device__ __forceinline__ void fma_pair(float& x0, float& x1, float a, float b) {
-    asm("{\n\t"
-        ".reg .b64 x, s, o;\n\t"
-        "mov.b64 x, {%0, %1};\n\t"
-        "mov.b64 s, {%2, %2};\n\t"
-        "mov.b64 o, {%3, %3};\n\t"
-        "fma.rn.f32x2 x, x, s, o;\n\t"
-        "mov.b64 {%0, %1}, x;\n\t"
-        "}"
-        : "+f"(x0), "+f"(x1)
-        : "f"(a), "f"(b));
+// Two floats in one 64-bit register pair, and the instructions on the pair.
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void pair_to(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 
-template <int HD, bool LEAN, int GATE>
-__global__ void __launch_bounds__(Storage<HD, LEAN>::THREADS, LEAN ? 2 : 1)
-attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
-                         const __grid_constant__ CUtensorMap map_v,
-                         const __grid_constant__ CUtensorMap run_k,
-                         const __grid_constant__ CUtensorMap run_v, const TcAttnParams p) {
+// the low n bits
+__device__ __forceinline__ uint32_t bits_below(int n) {
+    return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+}
+
+template <int HD, int GATE>
+__global__ void __launch_bounds__(Storage<HD>::THREADS, 1)
+attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                         const __grid_constant__ CUtensorMap run_k, const __grid_constant__ CUtensorMap run_v,
+                         const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_gate,
+                         const TcAttnParams p) {
     // 1024-byte alignment (the swizzled tiles need it) is asked of the declaration
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    using Store = Storage<HD, LEAN>;
-    constexpr int STAGES = Store::STAGES, PB = Store::PB, NH = HD / 64, S_BUFS = Store::S_BUFS;
-    constexpr int VALUES = Store::OPERANDS - 1;      // where a stage's values are
-    constexpr int GROUPS = Store::GROUPS;
-    constexpr int PV_WARP = GROUPS > 1 ? 2 + 4 * GROUPS : -1;    // the second MMA thread's warp
-    constexpr bool SPLIT = Store::SPLIT;
-    constexpr uint32_t TILE_BYTES = KEYS * HD * 2;       // a tile of one operand
-    static_assert(GROUPS == 1 || (PB == 2 && S_BUFS == 2 && HD <= 128), "two groups: a buffer of scores, of P and an accumulator each");
-    constexpr uint32_t TMEM_COLS = LEAN ? 256 : 512;     // scores: 128 columns a buffer, then O
+    using Store = Storage<HD>;
+    constexpr int NH = HD / 64, SLOTS = Store::SLOTS, GROUPS = Store::GROUPS, HALVES = Store::HALVES;
+    constexpr int S_BUFS = Store::S_BUFS;
+    constexpr bool BOTH = Store::BOTH;
+    constexpr uint32_t SLOT_BYTES = KEYS * Store::PART * 2;
+    constexpr uint32_t TMEM_COLS = 512;                  // scores: 128 columns a buffer, then O
     Store& s = *reinterpret_cast<Store*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // grid (heads, requests, tile ranks), the tile rank slowest: blocks start in order of
@@ -219,26 +215,22 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     volatile int* abort_flag = &s.abort_flag;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < STAGES; ++i) {
-            tc::mbar_init(&s.kv_full[i], 1);
-            tc::mbar_init(&s.kv_empty[i], 1);
-            if (SPLIT) {
-                tc::mbar_init(&s.v_full[i], 1);
-                tc::mbar_init(&s.v_empty[i], 1);
-            }
-        }
-        for (int b = 0; b < 2; ++b) {
+        for (int i = 0; i < SLOTS; ++i) tc::mbar_init(&s.full[i], 1);
+        for (int i = 0; i < Store::RELEASES; ++i) tc::mbar_init(&s.empty[i], 1);
+        tc::mbar_init(&s.q_full, p.q_boxes ? 1 : 4 * GROUPS);
+        tc::mbar_init(&s.gate_full, 1);
+        tc::mbar_init(&s.o_done, 1);
+        for (int b = 0; b < S_BUFS; ++b) {
             tc::mbar_init(&s.s_full[b], 1);
-            tc::mbar_init(&s.p_full[b], 4);               // one arrival per softmax warp
-            tc::mbar_init(&s.pv_done[b], 1);
+            tc::mbar_init(&s.p_half[b], 4);               // one arrival per softmax warp
+            tc::mbar_init(&s.p_full[b], 4);
         }
-        tc::mbar_init(&s.s_free, 4);
-        tc::mbar_init(&s.s_taken[0], 4);
-        tc::mbar_init(&s.s_taken[1], 4);
+        for (int b = 0; b < 2; ++b) tc::mbar_init(&s.pv_done[b], 1);
         s.abort_flag = 0;
         tc::fence_barrier_init();
         tc::prefetch_tensormap(&map_k);
         tc::prefetch_tensormap(&map_v);
+        tc::prefetch_tensormap(&map_q);
         if (p.runs) {
             tc::prefetch_tensormap(&run_k);
             tc::prefetch_tensormap(&run_v);
@@ -251,20 +243,22 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     // What follows reads the step's metadata, which was uploaded before the step began: the
     // kernels ahead in the stream write none of it, so it is read, and the first tiles'
     // table entries looked up, before the wait for them.
-    const int n_rep = p.n_rep;
+    const int n_rep = p.n_rep, tile_rows = p.tile_rows;
     const int row_base = p.req_row_start[req];
     const int n_new = p.req_row_start[req + 1] - row_base;
     const int n_rows = n_new * n_rep;
-    const int q_tiles = (n_rows + ROWS - 1) / ROWS;
+    const int q_tiles = (n_rows + tile_rows - 1) / tile_rows;
     const bool active = rank < q_tiles;
     const int qt = active ? q_tiles - 1 - rank : 0;               // heaviest tiles first
     const int first_pos = p.req_first_pos[req];
     const int* table = p.block_table + (size_t)req * p.table_stride;
 
     // the block's keys: from the first key any of its rows may read to its last position
-    const int last_row = min(n_rows - 1, qt * ROWS + ROWS - 1);
+    const int first_row = qt * tile_rows;
+    const int last_row = min(n_rows, first_row + tile_rows) - 1;
+    const int first_tok = first_row / n_rep;
     const int max_pos = first_pos + last_row / n_rep;
-    const int min_pos = first_pos + (qt * ROWS) / n_rep;
+    const int min_pos = first_pos + first_tok;
     int key_lo = first_key(p, min_pos);
     key_lo = key_lo / KEYS * KEYS;
     const int key_end = max_pos + 1;
@@ -274,292 +268,247 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                                ? min((p.keep_first + KEYS - 1) / KEYS, key_lo / KEYS) : 0;
     const int n_tiles = active ? kept_tiles + (key_end - key_lo + KEYS - 1) / KEYS : 0;
     auto tile_key0 = [&](int j) { return j < kept_tiles ? j * KEYS : key_lo + (j - kept_tiles) * KEYS; };
-    // a kept tile's pages beyond the last kept token's may have gone back to the pool: their
-    // keys are masked, and they are read from the last kept page instead
-    const int last_kept_page = p.keep_first > 0 ? (p.keep_first - 1) >> p.page_shift : 0;
 
-    // ---- the loader's thread: one tile of K and V pages into a stage --------------------------
-    const int pages_per_tile = KEYS >> p.page_shift;
-    auto lookup = [&](int j, int (&pages)[16]) {
-        // the tile's table entries, all in flight at once: the copies are ordered against
-        // memory and would take the lookups one by one
-        const int key0 = tile_key0(j);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            int index = (key0 >> p.page_shift) + (i < pages_per_tile ? i : 0);
-            if (j < kept_tiles && index > last_kept_page) index = last_kept_page;
-            index = index < p.table_stride ? index : p.table_stride - 1;
-            const int page = table[index];
-            pages[i] = page < 0 ? 0 : page;           // an entry given back early: never read
-        }
-    };
-    // which of the tile's operands: both, unless keys and values come and go by themselves
-    auto issue = [&](int j, const int (&pages)[16], auto which) -> bool {
-        constexpr bool keys = decltype(which)::value != 2, values = decltype(which)::value != 1;
-        const int st = j % STAGES;
-        const uint32_t round = j / STAGES;
-        // pages that follow one another in the pool come in with one copy per tile and operand
-        // (sending a copy costs this thread about 60 cycles whatever the copy's size, and the
-        // arithmetic around it more)
-        bool run = p.runs != 0 && pages[0] + pages_per_tile <= p.n_pages;
-#pragma unroll
-        for (int i = 1; i < 16; ++i)
-            if (i < pages_per_tile && pages[i] != pages[0] + i) run = false;
-        uint64_t* full = keys ? &s.kv_full[st] : &s.v_full[st];
-        uint64_t* empty = keys ? &s.kv_empty[st] : &s.v_empty[st];
-        if (round > 0 && !tc::mbar_wait(empty, (round - 1) & 1, abort_flag)) {
-            tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
-            return false;
-        }
-        tc::mbar_expect_tx(full, keys && values ? Store::OPERANDS * TILE_BYTES : TILE_BYTES);
-        if (run) {
-#pragma unroll
-            for (int h = 0; h < NH; ++h) {
-                if (keys) tc::tma_load_4d(s.kv[st][0][h], &run_k, full, h * 64, 0, kv_head, pages[0]);
-                if (VALUES && values) tc::tma_load_4d(s.kv[st][VALUES][h], &run_v, full, h * 64, 0, kv_head, pages[0]);
-            }
-            return true;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            if (i < pages_per_tile) {
-                const int dst = (i << p.page_shift) * 128;
-                const int y = (pages[i] * p.n_kv_heads + kv_head) << p.page_shift;
-#pragma unroll
-                for (int h = 0; h < NH; ++h) {
-                    if (keys) tc::tma_load_2d(s.kv[st][0][h] + dst, &map_k, full, h * 64, y);
-                    if (VALUES && values) tc::tma_load_2d(s.kv[st][VALUES][h] + dst, &map_v, full, h * 64, y);
-                }
-            }
-        }
-        return true;
-    };
-    using BOTH = std::integral_constant<int, 3>;
-    using KEYS_ONLY = std::integral_constant<int, 1>;
-    using VALUES_ONLY = std::integral_constant<int, 2>;
-    const int early = n_tiles < STAGES ? n_tiles : STAGES;
-
-    // ---- the query rows, by warps 1..5: 16-byte pieces into the 128-byte swizzle; warp 0's
-    // thread meanwhile starts the first tiles' copies, which wait for nothing -----------------
-    if (warp == 0) {
-        if (lane == 0) {
-            // the first tiles: all their lookups before the wait, then all their copies (the
-            // keys of this step's own tokens are written by the product before this kernel)
-            int first[STAGES][16];
-#pragma unroll
-            for (int j = 0; j < STAGES; ++j)
-                if (j < early) lookup(j, first[j]);
-            cb_pdl_wait();
-#pragma unroll
-            for (int j = 0; j < STAGES; ++j)
-                if (j < early) {
-                    issue(j, first[j], std::integral_constant<int, SPLIT ? 1 : 3>{});
-                    if (SPLIT) issue(j, first[j], VALUES_ONLY{});
-                }
-        } else {
-            cb_pdl_wait();
-        }
-    } else {
-        cb_pdl_wait();
-        if (active)
-        for (int i = threadIdx.x - 32; i < ROWS * 8 * NH; i += blockDim.x - 32) {
-            const int r = i / (8 * NH), c = i % (8 * NH);         // row, 16-byte piece of the row
-            const int row = qt * ROWS + r;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (row < n_rows) {
-                const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
-                val = *reinterpret_cast<const uint4*>(p.qkv + (size_t)tok * p.qkv_stride +
-                                                      (size_t)head * HD + c * 8);
-            }
-            *reinterpret_cast<uint4*>(s.q[c >> 3] + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
-        }
+    // rows beyond the tile's (a group size that does not divide 128): zeros, like any row not stored
+    for (int i = tile_rows * 8 * NH + threadIdx.x; i < ROWS * 8 * NH; i += blockDim.x) {
+        const int r = i / (8 * NH), c = i % (8 * NH);
+        *reinterpret_cast<uint4*>(s.q[c >> 3] + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = make_uint4(0, 0, 0, 0);
     }
-    tc::fence_proxy_async();                // generic-proxy writes of Q, before the MMAs read them
+    tc::fence_proxy_async();
     tc::tc_fence_before_sync();
     __syncthreads();
     tc::tc_fence_after_sync();
-    // only now may the kernel after this one start: every block of this one holds its tensor
-    // memory by now, so a successor that asks for tensor memory queues behind it
-    cb_pdl_trigger();
-    const uint32_t tmem_s = s.tmem_base;          // + 128 for the second buffer
+    const uint32_t tmem_s = s.tmem_base;          // + 128 a buffer
     const uint32_t tmem_o = s.tmem_base + S_BUFS * 128;
 
     if (warp == 0) {
-        // ---- loader: the remaining tiles, each once its stage has been read ------------------
-        if (lane == 0 && n_tiles > 0) {
-            int armed = early, values_armed = early;
-            if (SPLIT) {
-                // keys a tile ahead of the values: a tile's keys are free again before its
-                // predecessor's values are, and must not queue behind them
-                int ahead[16], pages[16];
-                if (early < n_tiles) {
-                    lookup(early, pages);
-                    if (issue(early, pages, KEYS_ONLY{})) armed = early + 1;
-                }
-                for (int j = early; j < n_tiles && armed > j; ++j) {
-                    if (j + 1 < n_tiles) {
-                        lookup(j + 1, ahead);
-                        if (!issue(j + 1, ahead, KEYS_ONLY{})) break;
-                        armed = j + 2;
-                    }
-                    if (!issue(j, pages, VALUES_ONLY{})) break;
-                    values_armed = j + 1;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) pages[i] = ahead[i];
-                }
-            } else {
-                for (int j = early; j < n_tiles; ++j) {
-                    int pages[16];
-                    lookup(j, pages);
-                    if (!issue(j, pages, BOTH{})) break;
-                    armed = j + 1;
-                }
+        // ---- loader: the warp together (a lane a page), so that scattered pages' table entries
+        // and copies go out side by side -----------------------------------------------------
+        // a kept tile's pages beyond the last kept token's may have gone back to the pool: their
+        // keys are masked, and they are read from the last kept page instead
+        const int last_kept_page = p.keep_first > 0 ? (p.keep_first - 1) >> p.page_shift : 0;
+        const int pages_per_tile = KEYS >> p.page_shift;
+        auto lookup = [&](int j) -> int {
+            const int key0 = tile_key0(j < n_tiles ? j : 0);
+            int index = (key0 >> p.page_shift) + (lane < pages_per_tile ? lane : 0);
+            if (j < kept_tiles && index > last_kept_page) index = last_kept_page;
+            index = index < p.table_stride ? index : p.table_stride - 1;
+            const int page = table[index];
+            return page < 0 ? 0 : page;               // an entry given back early: never read
+        };
+        int item = 0, armed = 0;                      // the next slot's number; slots with copies sent
+        auto send = [&](int page, bool values, int feature) -> bool {
+            const int st = item % SLOTS;
+            const int rel = BOTH ? item : item >> 1, round = rel / Store::RELEASES;
+            // (of a pair's two slots both wait: the second's test passes at once)
+            if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_wait(&s.empty[rel % Store::RELEASES], (round - 1) & 1, abort_flag))) {
+                tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
+                return false;
             }
-            if (*abort_flag) {
-                auto drain = [&](uint64_t* bars, int count) {
-                    for (int j = count > STAGES ? count - STAGES : 0; j < count; ++j)
-                        for (uint32_t t = 0; t < tc::WAIT_LIMIT; ++t)
-                            if (tc::mbar_try_wait(&bars[j % STAGES], (j / STAGES) & 1)) break;
-                };
-                drain(s.kv_full, armed);
-                if (SPLIT) drain(s.v_full, values_armed);
+            // pages that follow one another in the pool come in with one copy per slot and half
+            const int page0 = __shfl_sync(0xffffffffu, page, 0);
+            const bool run = __all_sync(0xffffffffu, lane >= pages_per_tile || page == page0 + lane) && p.runs != 0 &&
+                             page0 + pages_per_tile <= p.n_pages;
+            if (lane == 0) tc::mbar_expect_tx(&s.full[st], SLOT_BYTES);
+            __syncwarp();
+            if (run) {
+                if (lane < HALVES)
+                    tc::tma_load_4d(s.ring[st][lane], values ? &run_v : &run_k, &s.full[st], feature + lane * 64, 0, kv_head, page0);
+            } else if (lane < pages_per_tile) {
+                const int dst = (lane << p.page_shift) * 128;
+                const int y = (page * p.n_kv_heads + kv_head) << p.page_shift;
+#pragma unroll
+                for (int h = 0; h < HALVES; ++h)
+                    tc::tma_load_2d(s.ring[st][h] + dst, values ? &map_v : &map_k, &s.full[st], feature + h * 64, y);
+            }
+            armed = ++item;
+            return true;
+        };
+        int pg0 = lookup(0), pg1 = lookup(1), pg2 = lookup(2);
+        cb_pdl_wait();
+        cb_pdl_trigger();     // the block holds its tensor memory: a successor that asks for some queues behind it
+        bool ok = n_tiles > 0;
+        if (ok && p.q_boxes && lane == 0) {
+            tc::mbar_expect_tx(&s.q_full, NH * tile_rows * 128);
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+                tc::tma_load_3d(s.q[h], &map_q, &s.q_full, h * 64, kv_head * n_rep, row_base + first_tok);
+        }
+        __syncwarp();
+        if (BOTH) {
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                ok = send(pg0, false, 0) && send(pg0, false, 128);
+                pg0 = pg1, pg1 = pg2, pg2 = lookup(j + 3);
+            }
+        } else if (ok) {
+            int pg3 = S_BUFS > 2 ? lookup(3) : 0;
+            ok = send(pg0, false, 0);
+            if (ok && n_tiles > 1) ok = send(pg1, false, 0);
+            if (S_BUFS > 2 && ok && n_tiles > 2) ok = send(pg2, false, 0);
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                ok = send(pg0, true, 0);
+                if (ok && j + S_BUFS < n_tiles) ok = send(S_BUFS > 2 ? pg3 : pg2, false, 0);
+                pg0 = pg1, pg1 = pg2;
+                if (S_BUFS > 2) pg2 = pg3, pg3 = lookup(j + 4);
+                else pg2 = lookup(j + 3);
             }
         }
-    } else if (warp == 1 || warp == PV_WARP) {
-        // ---- MMA issuer: one thread; with two softmax groups two, of different warps: warp 1's
-        // sends the first products (scores), the last warp's the second (P V).  Sending twelve
-        // MMAs, three commits and the barrier tests between them costs a thread some 1,200
-        // cycles a tile, and two groups want a tile every 1,400: one thread would make each
-        // product wait for the other.
-        if (lane == 0 && n_tiles > 0) {
+        bool gate_sent = false;
+        if (GATE == GATE_RESULT && p.q_boxes && ok) {
+            // the gate's logits into the next free slots, beside the last tiles' work
+            constexpr int N = BOTH ? 2 : 1;
+            for (int i = 0; i < N && ok; ++i, ++item) {      // (two slots' worth: items are even by now)
+                const int rel = BOTH ? item : item >> 1, round = rel / Store::RELEASES;
+                ok = round == 0 || __all_sync(0xffffffffu, tc::mbar_wait(&s.empty[rel % Store::RELEASES], (round - 1) & 1, abort_flag));
+                if (!ok) {
+                    tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
+                } else if (lane == 0) {
+                    gate_sent = true;
+                    if (i == 0) tc::mbar_expect_tx(&s.gate_full, NH * tile_rows * 128);
+                    for (int h = 0; h < HALVES; ++h)
+                        tc::tma_load_3d(s.ring[item % SLOTS][h], &map_gate, &s.gate_full, i * 128 + h * 64, kv_head * n_rep,
+                                        row_base + first_tok);
+                }
+                __syncwarp();
+            }
+        }
+        // an abort leaves no copy in flight behind
+        if (*abort_flag && lane == 0) {
+            auto drain = [&](uint64_t* bar, uint32_t parity) {
+                for (uint32_t t = 0; t < tc::WAIT_LIMIT; ++t)
+                    if (tc::mbar_try_wait(bar, parity)) break;
+            };
+            if (p.q_boxes && n_tiles > 0) drain(&s.q_full, 0);
+            for (int i = armed > SLOTS ? armed - SLOTS : 0; i < armed; ++i) drain(&s.full[i % SLOTS], (i / SLOTS) & 1);
+            if (gate_sent) drain(&s.gate_full, 0);
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer: the warp walks the tiles together, one lane sends ---------------------
+        // Order: the first S_BUFS tiles' scores, then O += P_t V_t and S_(t + S_BUFS) for every tile.  P lies
+        // over the scores that it was made from, so the scores that take its buffer follow the second
+        // product, which the tensor pipe works off in order; the softmax of the tiles between runs beside both.
+        if (n_tiles > 0) {
+            const bool sender = tc::elect_one();
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(ROWS, KEYS);
-            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, HD);
+            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, Store::PART);
             // Operand descriptors by addition: the low word carries the address in 16-byte
-            // units, the high word is the same for every tile; stages and parities are carried
-            // along.  This thread's own instructions are what a tile's MMAs take (sending one
-            // costs 54 cycles, a dependent integer instruction about 5).
+            // units, the high word is the same for every tile.
             const uint64_t q_desc0 = tc::smem_desc_sw128(tc::smem_u32(s.q[0]));
             const uint32_t desc_hi = (uint32_t)(q_desc0 >> 32);
             const uint32_t q_lo = (uint32_t)q_desc0;
-            const uint32_t k_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.kv[0][0][0]));
-            const uint32_t p_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.p[0][0]));
-            constexpr uint32_t Q_HALF = sizeof(s.q[0]) >> 4, KV_HALF = sizeof(s.kv[0][0][0]) >> 4,
-                               KV_STAGE = sizeof(s.kv[0]) >> 4, P_HALF = sizeof(s.p[0][0]) >> 4,
-                               P_BUF = sizeof(s.p[0]) >> 4;
-            // the values, all features in one instruction: 64 of them lie together, the next 64 a
-            // leading offset of KV_HALF on
-            const uint32_t v_lo0 = ((uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.kv[0][VALUES][0])) & 0xFFFFu) |
-                                   (KV_HALF << 16);
-            bool ok = true;
-            // S_j = Q K_j^T into buffer j % S_BUFS: the head size in steps of 16
-            int qk_st = 0;                        // stage and parity of the next tile of scores
-            uint32_t qk_parity = 0;
-            auto send_qk = [&](int j) {
-                tc::tc_fence_after_sync();
-                const uint32_t k_lo = k_lo0 + qk_st * KV_STAGE;
-                const uint32_t d_s = tmem_s + (j % S_BUFS) * 128;
-#pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const uint64_t q_desc = tc::desc_of(q_lo + (k >> 2) * Q_HALF + 2 * (k & 3), desc_hi);
-                    const uint64_t k_desc = tc::desc_of(k_lo + (k >> 2) * KV_HALF + 2 * (k & 3), desc_hi);
-                    if (k == 0) tc::umma_bf16(d_s, q_desc, k_desc, idesc_qk, 0u);
-                    else tc::umma_bf16_add(d_s, q_desc, k_desc, idesc_qk);
-                }
-                tc::umma_commit(&s.s_full[j % S_BUFS]);
-                if (SPLIT) tc::umma_commit(&s.kv_empty[qk_st]);
-                if (++qk_st == STAGES) qk_st = 0, qk_parity ^= 1;
+            constexpr uint32_t HALF = KEYS * 128 >> 4, SLOT = SLOT_BYTES >> 4;
+            const uint32_t k_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.ring[0][0]));
+            // the values, all features of a slot in one instruction: 64 of them lie together, the next 64 a
+            // leading offset of HALF on
+            const uint32_t v_lo0 = (k_lo0 & 0xFFFFu) | (HALF << 16);
+            auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+                return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, abort_flag));
             };
-            // `block`: wait for the tile; else only take it if it has landed (true: issued)
-            auto issue_qk = [&](int j, bool block) -> bool {
-                // one buffer of scores: the softmax of tile j - 1 must have them in registers
-                const bool hand_back = S_BUFS == 1 && j > 0;
-                if (block) {
-                    if (!tc::mbar_wait(&s.kv_full[qk_st], qk_parity, abort_flag)) return false;
-                    if (hand_back && !tc::mbar_wait(&s.s_free, (j - 1) & 1, abort_flag)) return false;
-                } else if (!tc::mbar_try_wait(&s.kv_full[qk_st], qk_parity) ||
-                           (hand_back && !tc::mbar_try_wait(&s.s_free, (j - 1) & 1))) {
-                    return false;
+            int item = 0;                         // the next slot that has not been taken
+            // S_j = Q K_j^T into buffer `to`
+            int to = 0;
+            auto scores = [&](int j) -> bool {
+                const uint32_t d_s = tmem_s + to * 128;
+#pragma unroll
+                for (int part = 0; part < Store::PARTS; ++part) {
+                    const int st = item % SLOTS;
+                    if (!wait(&s.full[st], (item / SLOTS) & 1)) return false;
+                    tc::tc_fence_after_sync();
+                    const uint32_t k_lo = k_lo0 + st * SLOT;
+                    if (sender) {
+#pragma unroll
+                        for (int k = 0; k < Store::PART / 16; ++k) {
+                            const uint64_t q_desc = tc::desc_of(q_lo + (part * HALVES + (k >> 2)) * HALF + 2 * (k & 3), desc_hi);
+                            const uint64_t k_desc = tc::desc_of(k_lo + (k >> 2) * HALF + 2 * (k & 3), desc_hi);
+                            if (k == 0 && part == 0) tc::umma_bf16(d_s, q_desc, k_desc, idesc_qk, 0u);
+                            else tc::umma_bf16_add(d_s, q_desc, k_desc, idesc_qk);
+                        }
+                    }
+                    ++item;
                 }
-                send_qk(j);
+                if (sender) {
+                    tc::umma_commit(&s.s_full[to]);
+                    // pairs: K0 and K1; with two buffers V_(j-2) and K_j, with three K_(t+2) and V_t
+                    if (!BOTH && (S_BUFS == 2 ? j > 0 : j == 1)) tc::umma_commit(&s.empty[(j - 1) % Store::RELEASES]);
+                }
+                if (++to == S_BUFS) to = 0;
                 return true;
             };
-            // O += P_j V_j: 128 keys in eight steps of 16
-            int st = 0;                           // stage of the next tile's values
-            auto send_pv = [&](int j) {
-                const int pb = j % PB;
-                tc::tc_fence_after_sync();
-                const uint32_t p_lo = p_lo0 + pb * P_BUF;
-                const uint32_t v_lo = v_lo0 + st * KV_STAGE;
-                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(j % GROUPS) * HD : 0u);
+            auto products = [&](int t) -> bool {  // O += P_t V_t: 128 keys in eight steps of 16
+                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(t & 1) * HD : 0u);
+                const int b = t % S_BUFS;
+                const uint32_t p_at = tmem_s + b * 128;
+                const uint32_t parity = (t / S_BUFS) & 1;
 #pragma unroll
-                for (int k = 0; k < KEYS / 16; ++k) {
-                    // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
-                    const uint64_t p_desc = tc::desc_of(p_lo + (k >> 2) * P_HALF + 2 * (k & 3), desc_hi);
-                    const uint64_t v_desc = tc::desc_of(v_lo + 128 * k, desc_hi);
-                    if (k == 0) tc::umma_bf16(d_o, p_desc, v_desc, idesc_pv, j >= GROUPS ? 1u : 0u);
-                    else tc::umma_bf16_add(d_o, p_desc, v_desc, idesc_pv);
+                for (int part = 0; part < Store::PARTS; ++part) {
+                    // 256: the tile's own slots, which the scores have taken (and freed by this)
+                    const int st = BOTH ? (2 * t + part) % SLOTS : item % SLOTS;
+                    if (!BOTH && !wait(&s.full[st], (item / SLOTS) & 1)) return false;
+                    const uint32_t v_lo = v_lo0 + st * SLOT;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        if (part == 0 && !wait(half ? &s.p_full[b] : &s.p_half[b], parity)) return false;
+                        tc::tc_fence_after_sync();
+                        if (sender) {
+#pragma unroll
+                            for (int k = 4 * half; k < 4 * half + 4; ++k) {
+                                // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
+                                const uint64_t v_desc = tc::desc_of(v_lo + 128 * k, desc_hi);
+                                if (k == 0) tc::umma_bf16_ts(d_o + part * 128, p_at + 8 * k, v_desc, idesc_pv, t >= GROUPS ? 1u : 0u);
+                                else tc::umma_bf16_ts_add(d_o + part * 128, p_at + 8 * k, v_desc, idesc_pv);
+                            }
+                        }
+                    }
+                    if (BOTH && sender) tc::umma_commit(&s.empty[st]);
+                    if (!BOTH) ++item;
                 }
-                tc::umma_commit(SPLIT ? &s.v_empty[st] : &s.kv_empty[st]);
-                tc::umma_commit(&s.pv_done[pb]);
-                if (++st == STAGES) st = 0;
+                if (sender) {
+                    if (GROUPS == 1) tc::umma_commit(&s.pv_done[t & 1]);
+                    if (S_BUFS == 3) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
+                    if (t == n_tiles - 1) tc::umma_commit(&s.o_done);
+                }
+                return true;
             };
-            if (GROUPS > 1) {
-                // Two groups of softmax warps take the tiles in turn, so two tiles are in work
-                // at a time.  A tile's first product goes out as soon as its keys have landed
-                // and the scores that its buffer held (two tiles earlier) are in registers; its
-                // second once its P is written.
-                if (warp == 1) {
-                    for (int j = 0; j < n_tiles && ok; ++j) {
-                        ok = tc::mbar_wait(&s.kv_full[qk_st], qk_parity, abort_flag) &&
-                             (j < 2 || tc::mbar_wait(&s.s_taken[j & 1], ((j - 2) >> 1) & 1, abort_flag));
-                        if (ok) send_qk(j);
-                    }
-                } else {
-                    for (int j = 0; j < n_tiles && ok; ++j) {
-                        ok = tc::mbar_wait(&s.p_full[j & 1], (j >> 1) & 1, abort_flag) &&
-                             (!SPLIT || tc::mbar_wait(&s.v_full[st], (j / STAGES) & 1, abort_flag));
-                        if (ok) send_pv(j);
-                    }
-                }
-            } else {
-                ok = issue_qk(0, true);
-                for (int j = 0; j < n_tiles && ok; ++j) {
-                    // the next tile's scores go out first if its keys have landed (their buffer
-                    // was last read by the softmax of tile j - 1, whose P this thread has waited
-                    // for); else after this tile's second product, which must not wait for a copy
-                    bool ahead = j + 1 < n_tiles && issue_qk(j + 1, false);
-                    // With one buffer of scores the next tile's first MMA may go as soon as this
-                    // tile's softmax has the scores in registers, which happens during this wait.
-                    bool got = false;
-                    for (uint32_t i = 0; i < tc::WAIT_LIMIT && !got; ++i) {
-                        got = tc::mbar_try_wait(&s.p_full[j % PB], (j / PB) & 1);
-                        if (S_BUFS == 1 && !got && !ahead && j + 1 < n_tiles) ahead = issue_qk(j + 1, false);
-                        if ((i & 1023u) == 1023u && *abort_flag) break;
-                    }
-                    if (!got) {
-                        ok = false;
-                        break;
-                    }
-                    send_pv(j);
-                    if (j + 1 < n_tiles && !ahead) ok = issue_qk(j + 1, true);
-                }
+            bool ok = wait(&s.q_full, 0);
+            for (int j = 0; j < S_BUFS && j < n_tiles && ok; ++j) ok = scores(j);
+            for (int t = 0; t < n_tiles && ok; ++t) {
+                ok = products(t);
+                if (ok && t + S_BUFS < n_tiles) ok = scores(t + S_BUFS);
             }
-            if (!ok) tc::give_up(abort_flag, p.status, tc::ST_MMA_TIMEOUT);
+            if (!ok && lane == 0) tc::give_up(abort_flag, p.status, tc::ST_MMA_TIMEOUT);
         }
-    } else if (warp < 2 + 4 * GROUPS) {
+    } else {
         // ---- softmax: warps 2..5 (and 6..9: the second group), one thread per row =
         // tensor-memory lane; a group takes every GROUPS-th tile -------------------------------
         const int quarter = warp & 3;
         const int group = GROUPS > 1 ? (warp - 2) >> 2 : 0;
         const uint32_t tmem_mine = tmem_o + (uint32_t)group * HD;
         const int r = quarter * 32 + lane;
-        const int row = qt * ROWS + r;
-        const bool real = active && row < n_rows;
-        // rows past the request's last are computed like rows that may read every key (their
-        // queries are zero) and are not stored: they keep a tile's fast path open
+        const int row = first_row + r;
+        const bool real = active && r < tile_rows && row < n_rows;
+        // rows that are not the request's are computed like rows that may read every key and are
+        // not stored: they keep a tile's fast path open
         const int pos = real ? first_pos + row / n_rep : (1 << 30);
         const int lo = real ? first_key(p, pos) : 0;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
+        cb_pdl_wait();
+        if (!p.q_boxes && n_tiles > 0) {
+            // group sizes whose tiles would leave much of the 128 rows empty: the rows by hand,
+            // 16-byte pieces into the 128-byte swizzle
+            for (int i = threadIdx.x - 64; i < ROWS * 8 * NH; i += 128 * GROUPS) {
+                const int rr = i / (8 * NH), c = i % (8 * NH);
+                const int at = first_row + rr;
+                uint4 val = make_uint4(0, 0, 0, 0);
+                if (at < n_rows) {
+                    const int tok = row_base + at / n_rep, head = kv_head * n_rep + at % n_rep;
+                    val = *reinterpret_cast<const uint4*>(p.qkv + (size_t)tok * p.qkv_stride + (size_t)head * HD + c * 8);
+                }
+                *reinterpret_cast<uint4*>(s.q[c >> 3] + rr * 128 + (((c & 7) ^ (rr & 7)) << 4)) = val;
+            }
+            tc::fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&s.q_full);
+        }
         float m_ref = -INFINITY, l = 0.f;
         bool ok = true;
         auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
@@ -567,60 +516,67 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             if (!got && !*abort_flag) tc::give_up(abort_flag, p.status, tc::ST_EPILOGUE_TIMEOUT);
             return __all_sync(0xffffffffu, got);
         };
-        for (int j = group; j < n_tiles && ok; j += GROUPS) {
+        const uint64_t scale2 = pair_of(p.scale_log2, p.scale_log2);
+        for (int j = group; j < n_tiles; j += GROUPS) {
             const int key0 = tile_key0(j);
-            const int b = j % S_BUFS;                 // the scores' buffer
-            const int pb = j % PB;                    // P's buffer
+            const int b = j % S_BUFS;
             ok = wait_all(&s.s_full[b], (j / S_BUFS) & 1);
             if (!ok) break;
             tc::tc_fence_after_sync();
-            // the row's 128 scores, once, into registers
-            uint32_t sv[4][32];
-#pragma unroll
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tc::tmem_ld_32x32(tmem_s + b * 128 + lane_bits + c * 32, sv[c]);
-            tc::tmem_ld_wait();
-            tc::tc_fence_before_sync();
-            if (S_BUFS == 1 || GROUPS > 1) {          // the buffer may take the next tile's scores
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(GROUPS > 1 ? &s.s_taken[b] : &s.s_free);
-            }
-            // keys of this tile the row may read: [first, last] relative to key0.  Most tiles
-            // lie wholly inside every row's range and skip the test.
-            const int last = min(pos - key0, KEYS - 1);
-            const int first = max(lo - key0, 0);
+            const uint32_t at = tmem_s + b * 128 + lane_bits;
+            // keys of this tile the row may read: [first, last] relative to key0, and those before
+            // `kept`.  Most tiles lie wholly inside every row's range and skip the test; in the
+            // others the masked scores go back where they came from.
+            const int last = pos - key0, first = lo - key0;
             const int kept = p.keep_first - key0;     // keys before this one are kept first tokens (<= 0: none here)
-            if (!__all_sync(0xffffffffu, last == KEYS - 1 && first == 0)) {
+            const bool inside = __all_sync(0xffffffffu, last >= KEYS - 1 && first <= 0);
+            float mc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            // The scores are read twice, 64 at a time in a loop that is not unrolled: the code of
+            // both passes over all 128 comes from memory at a block's first tile, and the registers
+            // would not hold them beside the rest.
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                uint32_t sv[2][32];
+                tc::tmem_ld_32x32(at + 64 * h, sv[0]);
+                tc::tmem_ld_32x32(at + 64 * h + 32, sv[1]);
+                tc::tmem_ld_wait();
+                if (!inside) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 2; ++c) {
+                        const int k0 = 64 * h + 32 * c;
+                        const uint32_t seen = bits_below(last + 1 - k0) & (~bits_below(first - k0) | bits_below(kept - k0));
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int kk = c * 32 + i;
-                        if (kk > last || (kk < first && kk >= kept)) sv[c][i] = __float_as_uint(-INFINITY);
+                        for (int i = 0; i < 32; ++i)
+                            if (!(seen >> i & 1u)) sv[c][i] = __float_as_uint(-INFINITY);
+                        tc::tmem_st_32x32(at + k0, sv[c]);
                     }
-            }
-            float mc[4];
+                    tc::tmem_st_wait();
+                }
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                mc[c] = -INFINITY;
+                for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; i += 2)
-                    mc[c] = max3(mc[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+                    for (int i = 0; i < 32; i += 2) {
+                        float& m = mc[2 * c + ((i >> 1) & 1)];
+                        m = max3(m, __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+                    }
             }
             float mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3]));
             mx *= p.scale_log2;
             // raise the reference maximum only when it is exceeded by far; the accumulator
-            // in tensor memory is rescaled then, by the whole warp at once, after the
-            // second MMA of the tile before has finished
+            // in tensor memory is rescaled then, by the whole warp at once.  Two groups, two buffers: the
+            // scores' commit covers the second product of this group's tile before; else that is waited for.
             float corr = 1.0f;
             if (mx > m_ref + RAISE || (m_ref == -INFINITY && mx > -INFINITY)) {
                 corr = m_ref == -INFINITY ? 0.f : exp2f(m_ref - mx);
                 m_ref = mx;
             }
             if (j >= GROUPS && __any_sync(0xffffffffu, corr != 1.0f)) {
-                ok = wait_all(&s.pv_done[(j - GROUPS) % PB], ((j - GROUPS) / PB) & 1);
-                if (!ok) break;
-                tc::tc_fence_after_sync();
+                if (GROUPS == 1 || S_BUFS == 3) {
+                    ok = GROUPS == 1 ? wait_all(&s.pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1)
+                                     : wait_all(&s.empty[(j - 1) % Store::RELEASES], ((j - 1) / Store::RELEASES) & 1);
+                    if (!ok) break;
+                    tc::tc_fence_after_sync();
+                }
 #pragma unroll 1
                 for (int c0 = 0; c0 < HD; c0 += 32) {
                     uint32_t v[32];
@@ -631,56 +587,45 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                     tc::tmem_st_32x32(tmem_mine + lane_bits + c0, v);
                 }
                 tc::tmem_st_wait();
-                tc::tc_fence_before_sync();
             }
             l *= corr;
-            // P's buffer was last read by the second MMA of tile j - PB.  With two buffers and
-            // one group that MMA was sent before this tile's first one, and the commit that
-            // announced this tile's scores covers everything its thread had sent by then:
-            // nothing to wait for (a barrier test costs a warp 100 to 200 cycles even when it
-            // passes).  With two groups this tile's first MMA may have gone out earlier.
-            if ((PB == 1 || GROUPS > 1) && j >= PB) {
-                ok = wait_all(&s.pv_done[pb], ((j - PB) / PB) & 1);
-                if (!ok) break;
-            }
-            // P = exp2(s * scale - reference), to shared memory in the layout the second MMA
-            // reads (rows of 128 bytes per half of 64 keys, 128-byte swizzle)
+            // P = exp2(s * scale - reference) in bf16, two a column, over the scores' own columns:
+            // keys 0-63 into the first 32, 64-127 into the next (their scores, columns 64-127, are
+            // read after the first half's, whose columns are 0-63)
             const float off = m_ref == -INFINITY ? 0.f : -m_ref;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint64_t off2 = pair_of(off, off);
+            uint64_t sum[4] = {0, 0, 0, 0};
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                uint32_t sv[2][32], pk[32];
+                tc::tmem_ld_32x32(at + 64 * h, sv[0]);
+                tc::tmem_ld_32x32(at + 64 * h + 32, sv[1]);
+                tc::tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint8_t* half = s.p[pb][c >> 1] + r * 128;
+                for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int piece = 0; piece < 4; ++piece) {
-                    float e[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
-                        e[i] = __uint_as_float(sv[c][8 * piece + i]);
-                        e[i + 1] = __uint_as_float(sv[c][8 * piece + i + 1]);
-                        fma_pair(e[i], e[i + 1], p.scale_log2, off);
-                        e[i] = ex2_fast(e[i]);
-                        e[i + 1] = ex2_fast(e[i + 1]);
-                        sum[i >> 1] += e[i] + e[i + 1];
+                    for (int i = 0; i < 32; i += 2) {
+                        float e0, e1;
+                        pair_to(fma2(pair_of(__uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1])), scale2, off2), e0, e1);
+                        e0 = ex2_fast(e0);
+                        e1 = ex2_fast(e1);
+                        uint64_t& into = sum[(i >> 1) & 3];
+                        into = add2(into, pair_of(e0, e1));
+                        pk[16 * c + (i >> 1)] = pack_bf16(e0, e1);
                     }
-                    uint4 w;
-                    w.x = pack_bf16(e[0], e[1]);
-                    w.y = pack_bf16(e[2], e[3]);
-                    w.z = pack_bf16(e[4], e[5]);
-                    w.w = pack_bf16(e[6], e[7]);
-                    const int pc = (c & 1) * 4 + piece;              // 16-byte piece inside the row
-                    *reinterpret_cast<uint4*>(half + ((pc ^ (r & 7)) << 4)) = w;
-                }
+                tc::tmem_st_32x32(at + 32 * h, pk);
+                tc::tmem_st_wait();
+                tc::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(h ? &s.p_full[b] : &s.p_half[b]);
             }
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            tc::fence_proxy_async();             // P is written by the generic proxy, read by the MMA
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&s.p_full[pb]);
+            float s0, s1;
+            pair_to(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), s0, s1);
+            l += s0 + s1;
         }
         // ---- the output: O / l ------------------------------------------------------------
-        // the group's last tile
         const int my_tiles = n_tiles > group ? (n_tiles - group + GROUPS - 1) / GROUPS : 0;
-        const int j_last = group + (my_tiles - 1) * GROUPS;
-        if (ok && my_tiles > 0) ok = wait_all(&s.pv_done[j_last % PB], (j_last / PB) & 1);
+        if (n_tiles > 0 && ok) ok = wait_all(&s.o_done, 0);
         __nv_bfloat16* dst = nullptr;
         const __nv_bfloat16* gate = nullptr;
         float gate_f = 1.f;
@@ -691,8 +636,60 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
             if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
             if (GATE == GATE_HEAD)
-                gate_f = 1.0f / (1.0f + expf(-__bfloat162float(p.gate[(size_t)tok * p.gate_stride + head])));
+                gate_f = sigmoid(__bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]));
         }
+        if (GATE == GATE_RESULT && p.q_boxes && n_tiles > 0 && ok) ok = wait_all(&s.gate_full, 0);
+        // where the loader put the gate's logits: behind the ring's last slot (see there)
+        const int gate_item = 2 * n_tiles;
+        // 32 results of the row, from feature c0 on, to the queries' place, which nothing reads any more
+        auto close = [&](float (&o)[32], int c0) {
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+                if (GATE == GATE_RESULT) {
+                    const int f = c0 + 8 * q4, piece = (f & 63) >> 3;
+                    const void* from = gate + f;
+                    if (p.q_boxes) {
+                        const int st = (gate_item + (BOTH ? f >> 7 : 0)) % SLOTS;
+                        from = s.ring[st][(f >> 6) & (HALVES - 1)] + r * 128 + ((piece ^ (r & 7)) << 4);
+                    }
+                    const uint4 raw = *reinterpret_cast<const uint4*>(from);
+                    const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= sigmoid(__bfloat162float(g[i]));
+                }
+                if (GATE == GATE_HEAD) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= gate_f;
+                }
+                uint4 w;
+                w.x = pack_bf16(o[8 * q4 + 0], o[8 * q4 + 1]);
+                w.y = pack_bf16(o[8 * q4 + 2], o[8 * q4 + 3]);
+                w.z = pack_bf16(o[8 * q4 + 4], o[8 * q4 + 5]);
+                w.w = pack_bf16(o[8 * q4 + 6], o[8 * q4 + 7]);
+                const int f = c0 + 8 * q4;
+                *reinterpret_cast<uint4*>(s.q[f >> 6] + r * 128 + ((((f & 63) >> 3) ^ (r & 7)) << 4)) = w;
+            }
+        };
+        // The warp's 32 rows from there to memory, several rows' pieces side by side: a store of one piece by
+        // each of 32 rows touches 32 lines and takes the memory pipe 32 cycles (128 rows of 256 features
+        // that way 5,200 cycles of a block, of 64 features with two groups 2,200).
+        auto write_rows = [&]() {
+            constexpr int MINE = HD / GROUPS, ACROSS = MINE < 64 ? MINE / 8 : 8;      // pieces of a row side by side
+            __syncwarp();
+            const unsigned long long mine = real ? (unsigned long long)dst : 0ull;
+#pragma unroll 1
+            for (int rr = lane / ACROSS; rr < 32; rr += 32 / ACROSS) {
+                __nv_bfloat16* to = (__nv_bfloat16*)__shfl_sync(0xffffffffu, mine, rr);
+                const int at = quarter * 32 + rr;
+                if (to != nullptr)
+#pragma unroll
+                    for (int f0 = 0; f0 < MINE; f0 += 8 * ACROSS) {
+                        const int f = group * MINE + f0 + 8 * (lane % ACROSS);
+                        *reinterpret_cast<uint4*>(to + f) = *reinterpret_cast<const uint4*>(
+                            s.q[f >> 6] + at * 128 + ((((f & 63) >> 3) ^ (at & 7)) << 4));
+                    }
+            }
+        };
         if (GROUPS > 1) {
             // Two groups: each holds the sums over its own tiles against its own reference.
             // A row's two states meet in shared memory; every thread comes to the barrier,
@@ -701,7 +698,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (ok && n_tiles > 0 && !*abort_flag) {
                 tc::tc_fence_after_sync();
-                const float2 other = s.merge[group ^ 1][r];
+                const float2 other = s.merge[GROUPS > 1 ? group ^ 1 : 0][r];
                 const float m_mine = my_tiles > 0 ? m_ref : -INFINITY;
                 const float m_all = fmaxf(fmaxf(m_mine, other.x), sink);
                 const float f_mine = m_mine == -INFINITY ? 0.f : exp2f(m_mine - m_all);
@@ -727,22 +724,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                         for (int i = 0; i < 32; ++i)
                             o[i] = (mine_any ? __uint_as_float(a[i]) * w_mine : 0.f) +
                                    (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
-#pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) {
-                            if (GATE == GATE_RESULT) gate_eight(o + 8 * q4, gate + c0 + 8 * q4);
-                            if (GATE == GATE_HEAD) {
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= gate_f;
-                            }
-                            uint4 w;
-                            w.x = pack_bf16(o[8 * q4 + 0], o[8 * q4 + 1]);
-                            w.y = pack_bf16(o[8 * q4 + 2], o[8 * q4 + 3]);
-                            w.z = pack_bf16(o[8 * q4 + 4], o[8 * q4 + 5]);
-                            w.w = pack_bf16(o[8 * q4 + 6], o[8 * q4 + 7]);
-                            *reinterpret_cast<uint4*>(dst + c0 + 8 * q4) = w;
-                        }
+                        close(o, c0);
                     }
                 }
+                write_rows();
             }
         } else if (ok && n_tiles > 0) {
             tc::tc_fence_after_sync();
@@ -758,25 +743,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
                 tc::tmem_ld_32x32(tmem_o + lane_bits + c0, v);
                 tc::tmem_ld_wait();
                 if (real) {
+                    float o[32];
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        float o[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[8 * q4 + i]) * inv;
-                        if (GATE == GATE_RESULT) gate_eight(o, gate + c0 + 8 * q4);
-                        if (GATE == GATE_HEAD) {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] *= gate_f;
-                        }
-                        uint4 w;
-                        w.x = pack_bf16(o[0], o[1]);
-                        w.y = pack_bf16(o[2], o[3]);
-                        w.z = pack_bf16(o[4], o[5]);
-                        w.w = pack_bf16(o[6], o[7]);
-                        *reinterpret_cast<uint4*>(dst + c0 + 8 * q4) = w;
-                    }
+                    for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(v[i]) * inv;
+                    close(o, c0);
                 }
             }
+            write_rows();
         }
     }
     tc::tc_fence_before_sync();
@@ -787,31 +760,29 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     }
 }
 
-template <int HD, bool LEAN, int GATE>
-int launch_gate(dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
-              const CUtensorMap& rk, const CUtensorMap& rv, const TcAttnParams& p) {
-    constexpr int smem = (int)sizeof(Storage<HD, LEAN>);
+template <int HD, int GATE>
+int launch_gate(dim3 grid, cudaStream_t st, const CUtensorMap (&maps)[6], const TcAttnParams& p) {
+    constexpr int smem = (int)sizeof(Storage<HD>);
     static_assert(smem <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, LEAN, GATE>,
+        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, GATE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    cb_launch(attention_tcgen05_kernel<HD, LEAN, GATE>, grid, dim3(Storage<HD, LEAN>::THREADS), smem, st, mk, mv, rk,
-              rv, p);
+    cb_launch(attention_tcgen05_kernel<HD, GATE>, grid, dim3(Storage<HD>::THREADS), smem, st, maps[0], maps[1], maps[2],
+              maps[3], maps[4], maps[5], p);
     return cb_last_error();
 }
 
-template <int HD, bool LEAN>
-int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap& mk, const CUtensorMap& mv,
-              const CUtensorMap& rk, const CUtensorMap& rv, const TcAttnParams& p) {
+template <int HD>
+int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap (&maps)[6], const TcAttnParams& p) {
     switch (gate) {
-        case GATE_NONE: return launch_gate<HD, LEAN, GATE_NONE>(grid, st, mk, mv, rk, rv, p);
-        case GATE_RESULT: return launch_gate<HD, LEAN, GATE_RESULT>(grid, st, mk, mv, rk, rv, p);
+        case GATE_NONE: return launch_gate<HD, GATE_NONE>(grid, st, maps, p);
+        case GATE_RESULT: return launch_gate<HD, GATE_RESULT>(grid, st, maps, p);
     }
-    return launch_gate<HD, LEAN, GATE_HEAD>(grid, st, mk, mv, rk, rv, p);
+    return launch_gate<HD, GATE_HEAD>(grid, st, maps, p);
 }
 
 }  // namespace
@@ -821,17 +792,17 @@ int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap& mk, const
 // both are the same rows.
 // keep_first (with a window): a row at position p reads j <= p with p - j < window or j < keep_first.
 // chunked: `window` is a chunk's size (first_key).  sinks: [n_heads] or null.  Results times out_scale.
-// lead: how many requests at the head bring a single token (as max_new_tokens is the others').
+// n_rows: of qkv (and out, gate).  lead: how many requests at the head bring a single token (as max_new_tokens is the others').
 // gate: null, or logits: results times their sigmoids; laid out like `out`, rows of 16-byte pieces, or with
 // gate_per_head [rows][n_heads].
-CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* out, int out_stride,
+CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, int n_rows, void* out, int out_stride,
                                         const void* k_cache, const void* v_cache, int n_pages,
                                         const int* req_row_start, const int* req_first_pos,
                                         const int* block_table, int table_stride, int n_requests,
                                         int max_new_tokens, int n_heads, int n_kv_heads, int head_dim,
                                         int page_tokens, float scale, int window, int chunked, int keep_first,
                                         float out_scale, const float* sinks, const void* gate, int gate_stride,
-                                        int gate_per_head, int lead, int lean, int* status, void* stream) {
+                                        int gate_per_head, int lead, int* status, void* stream) {
     if (n_requests <= 0 || max_new_tokens <= 0) return 0;
     if (keep_first < 0 || !(scale > 0.f)) return CB_ERR_UNSUPPORTED;
     if ((head_dim != 64 && head_dim != 128 && !(head_dim == 256 && k_cache == v_cache)) || n_heads % n_kv_heads != 0 || page_tokens < 8 || page_tokens > KEYS ||
@@ -841,17 +812,32 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
         return CB_ERR_UNSUPPORTED;
     int shift = 0;
     while ((1 << shift) < page_tokens) ++shift;
-    CUtensorMap mk, mv;
+    CUtensorMap maps[6];
+    CUtensorMap &mk = maps[0], &mv = maps[1], &rk = maps[2], &rv = maps[3];
     const uint64_t rows = (uint64_t)n_pages * n_kv_heads * page_tokens;
     if (!tc::make_map_2d(&mk, k_cache, rows, head_dim, head_dim, page_tokens)) return CB_ERR_UNSUPPORTED;
     if (!tc::make_map_2d(&mv, v_cache, rows, head_dim, head_dim, page_tokens)) return CB_ERR_UNSUPPORTED;
     // tiles of several pages: a second pair of maps that takes a run of pages at once
-    CUtensorMap rk = mk, rv = mv;
+    rk = mk, rv = mv;
     const int pages_per_tile = KEYS / page_tokens;
     const bool runs = pages_per_tile > 1 &&
                       tc::make_map_pages(&rk, k_cache, n_pages, n_kv_heads, page_tokens, head_dim, pages_per_tile) &&
                       tc::make_map_pages(&rv, v_cache, n_pages, n_kv_heads, page_tokens, head_dim, pages_per_tile);
+    // A tile takes whole tokens, all heads of the group, so that one box holds its rows.  Group sizes that
+    // would leave more than an eighth of the 128 rows empty are cut anywhere and fetched by hand.
+    const int n_rep = n_heads / n_kv_heads;
     TcAttnParams p;
+    p.tile_rows = n_rep <= ROWS ? ROWS / n_rep * n_rep : 0;
+    p.q_boxes = p.tile_rows >= ROWS - ROWS / 8;
+    if (!p.q_boxes) p.tile_rows = ROWS;
+    maps[4] = maps[5] = mk;
+    if (p.q_boxes) {
+        const uint32_t tokens = p.tile_rows / n_rep;
+        if (!tc::make_map_heads(&maps[4], qkv, n_rows, n_heads, head_dim, qkv_stride, n_rep, tokens) ||
+            (gate != nullptr && !gate_per_head &&
+             !tc::make_map_heads(&maps[5], gate, n_rows, n_heads, head_dim, gate_stride, n_rep, tokens)))
+            return CB_ERR_UNSUPPORTED;
+    }
     p.n_pages = n_pages;
     p.runs = runs ? 1 : 0;
     p.qkv = (const __nv_bfloat16*)qkv;
@@ -864,7 +850,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     p.table_stride = table_stride;
     p.n_heads = n_heads;
     p.n_kv_heads = n_kv_heads;
-    p.n_rep = n_heads / n_kv_heads;
+    p.n_rep = n_rep;
     p.n_requests = n_requests;
     p.page_tokens = page_tokens;
     p.page_shift = shift;
@@ -877,8 +863,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     p.gate_stride = gate_stride;
     p.out_scale = out_scale;
     p.status = status;
-    const int n_rep = n_heads / n_kv_heads;
-    const int q_tiles = (max_new_tokens * n_rep + ROWS - 1) / ROWS;
+    const int q_tiles = (max_new_tokens * n_rep + p.tile_rows - 1) / p.tile_rows;
     if (n_requests > 65535 || q_tiles > 65535) return CB_ERR_UNSUPPORTED;
     // (single tokens of more than a tile of query heads keep ranks like a portion's)
     p.lead = lead > 0 && lead < n_requests && n_rep <= ROWS ? lead : 0;
@@ -886,29 +871,8 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, void* o
     p.lead_ranks = (p.lead + portions - 1) / portions;
     if (p.lead_ranks + q_tiles > 65535) return CB_ERR_UNSUPPORTED;
     const dim3 grid(n_kv_heads, portions, p.lead_ranks + q_tiles);
-    // lean: -1 lets the launch decide, 0 and 1 fix the form.  Since the roomy form has two
-    // softmax groups it is the quicker one also for launches with more blocks than places
-    // (measured on B200: 2,048 tokens at the Llama-3.2-1B layer sizes, 512 blocks, 4.63 against
-    // 4.86 ms; 4,096 tokens of the 120M shape, 384 blocks, 1.68 against 1.96 ms), so the launch
-    // decides for it; the lean form stays for callers that ask for it.
-    if (lean < 0) lean = 0;
     const int form = gate == nullptr ? GATE_NONE : gate_per_head ? GATE_HEAD : GATE_RESULT;
-    if (head_dim == 64)
-        return lean ? launch_as<64, true>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p)
-                    : launch_as<64, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
-    if (head_dim == 256) return launch_as<256, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
-    return launch_as<128, false>(form, grid, (cudaStream_t)stream, mk, mv, rk, rv, p);
-}
-
-CB_EXPORT int cb_attention_tcgen05(const void* qkv, int qkv_stride, void* out, int out_stride,
-                                   const void* k_cache, const void* v_cache, int n_pages,
-                                   const int* req_row_start, const int* req_first_pos,
-                                   const int* block_table, int table_stride, int n_requests,
-                                   int max_new_tokens, int n_heads, int n_kv_heads, int head_dim,
-                                   int page_tokens, float scale, int window, int lean, int* status,
-                                   void* stream) {
-    return cb_attention_tcgen05_kept(qkv, qkv_stride, out, out_stride, k_cache, v_cache, n_pages, req_row_start,
-                                     req_first_pos, block_table, table_stride, n_requests, max_new_tokens, n_heads,
-                                     n_kv_heads, head_dim, page_tokens, scale, window, 0, 0, 1.0f, nullptr, nullptr, 0, 0, 0, lean,
-                                     status, stream);
+    if (head_dim == 64) return launch_as<64>(form, grid, (cudaStream_t)stream, maps, p);
+    if (head_dim == 256) return launch_as<256>(form, grid, (cudaStream_t)stream, maps, p);
+    return launch_as<128>(form, grid, (cudaStream_t)stream, maps, p);
 }

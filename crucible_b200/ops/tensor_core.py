@@ -624,9 +624,9 @@ def linear_rope_append(h, wqkv, qkv, n_heads, n_kv_heads, head_dim, cos, sin, ro
     return True
 
 
-# The form of the head-size-64 prompt attention: -1 the launcher's choice (the roomy form, see the
-# kernel's header), 0 roomy, 1 lean (tests fix it; CRUCIBLE_ATTENTION_LEAN=1 for a profile of that form).
-ATTENTION_LEAN = int(os.environ.get("CRUCIBLE_ATTENTION_LEAN", "-1"))
+# The prompt attention had a second form of head size 64, which callers could fix here; it has one now, and
+# the value is taken and not read.
+ATTENTION_LEAN = -1
 
 
 class _Requests:
@@ -665,7 +665,7 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         return False
     lib = build.load("attention_tcgen05")
     code = lib.cb_attention_tcgen05_kept(
-        qkv.data_ptr(), qkv.stride(0), out.data_ptr(),
+        qkv.data_ptr(), qkv.stride(0), qkv.shape[0], out.data_ptr(),
         out.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
         k_cache.shape[0], reqs.row_start,
         reqs.first_pos, reqs.table,
@@ -674,7 +674,7 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         scale, window or 0, 1 if chunked else 0, keep_first if window else 0,
         out_scale, sinks.data_ptr() if sinks is not None else 0,
         gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0,
-        1 if gate_per_head else 0, lead, ATTENTION_LEAN, status_word(qkv.device).data_ptr(), _stream())
+        1 if gate_per_head else 0, lead, status_word(qkv.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:

@@ -288,7 +288,7 @@ attention_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
     // asked for while that product still runs made a step slower, not faster: 0.300 against
     // 0.289 ms at batch 1, 0.329 against 0.320 ms at batch 8, measured on B200).
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             // the first tiles wait for nothing: all their lookups first, then all their copies
             int y0[16], y1[16], y2[16];
             lookup(0, y0);
@@ -329,7 +329,7 @@ attention_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
 
     if (warp == 0) {
         // ---- loader: the remaining tiles, each once its stage has been read ------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int armed = early;
             // a tile's table entries are looked up while the tile before it is awaited
             int y[16];
@@ -351,7 +351,7 @@ attention_decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k,
         }
     } else if (warp == 1) {
         // ---- MMA issuer -------------------------------------------------------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(KEYS, ROWS);
             constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(128, 64);
             // Operand descriptors by addition: the low word carries the address in 16-byte

@@ -388,7 +388,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // over the scores that it was made from, so the scores that take its buffer follow the second
         // product, which the tensor pipe works off in order; the softmax of the tiles between runs beside both.
         if (n_tiles > 0) {
-            const bool sender = tc::elect_one();
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(ROWS, KEYS);
             constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, Store::PART);
             // Operand descriptors by addition: the low word carries the address in 16-byte
@@ -415,7 +414,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     if (!wait(&s.full[st], (item / SLOTS) & 1)) return false;
                     tc::tc_fence_after_sync();
                     const uint32_t k_lo = k_lo0 + st * SLOT;
-                    if (sender) {
+                    if (tc::elect_one()) {
 #pragma unroll
                         for (int k = 0; k < Store::PART / 16; ++k) {
                             const uint64_t q_desc = tc::desc_of(q_lo + (part * HALVES + (k >> 2)) * HALF + 2 * (k & 3), desc_hi);
@@ -426,7 +425,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     }
                     ++item;
                 }
-                if (sender) {
+                if (tc::elect_one()) {
                     tc::umma_commit(&s.s_full[to]);
                     // pairs: K0 and K1; with two buffers V_(j-2) and K_j, with three K_(t+2) and V_t
                     if (!BOTH && (S_BUFS == 2 ? j > 0 : j == 1)) tc::umma_commit(&s.empty[(j - 1) % Store::RELEASES]);
@@ -449,7 +448,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     for (int half = 0; half < 2; ++half) {
                         if (part == 0 && !wait(half ? &s.p_full[b] : &s.p_half[b], parity)) return false;
                         tc::tc_fence_after_sync();
-                        if (sender) {
+                        if (tc::elect_one()) {
 #pragma unroll
                             for (int k = 4 * half; k < 4 * half + 4; ++k) {
                                 // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
@@ -459,10 +458,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                             }
                         }
                     }
-                    if (BOTH && sender) tc::umma_commit(&s.empty[st]);
+                    if (BOTH && tc::elect_one()) tc::umma_commit(&s.empty[st]);
                     if (!BOTH) ++item;
                 }
-                if (sender) {
+                if (tc::elect_one()) {
                     if (GROUPS == 1) tc::umma_commit(&s.pv_done[t & 1]);
                     if (S_BUFS == 3) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
                     if (t == n_tiles - 1) tc::umma_commit(&s.o_done);

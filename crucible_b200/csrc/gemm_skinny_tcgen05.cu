@@ -119,7 +119,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w,
     // now (a weight matrix, which no kernel of the stream writes); the step's rows are the
     // output of the kernels before this one and wait for them.
     const int w_ahead = n_kb < STAGES ? n_kb : STAGES;
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && tc::elect_one()) {
         for (int i = 0; i < w_ahead; ++i) {
             tc::mbar_expect_tx(&s.full_bar[i], STAGE_BYTES);
             load_w(i, i);
@@ -129,7 +129,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w,
     cb_pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             // (the stage and its parity are carried along: a division by a run-time value
             // costs a lone thread about as much as two boxes)
             int armed = w_ahead, st = 0;
@@ -155,7 +155,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w,
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             // One thread, whose own instructions are what a step of K takes with tiles this
             // narrow (a block that has its SM to itself streams what this loop can hand on);
             // so the ring is walked by an unrolled loop in which a stage's barriers and

@@ -159,7 +159,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
     // not wait for the kernels before this one; A is their output and does.
     // (not in a grouped product: which expert's W it is stands in the plan, which a kernel wrote)
     const int w_ahead = FORM == GROUPED ? 0 : (k_blocks < STAGES ? k_blocks : STAGES);
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && tc::elect_one()) {
         for (int kb = 0; kb < w_ahead; ++kb) {
             tc::mbar_expect_tx(&s.full_bar[kb], STAGE_BYTES);
             load_w(kb, kb);
@@ -192,7 +192,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         const int i = threadIdx.x - 64;
         if (i < BN) s.gain[i] = n_tile * BN + i < N ? __ldg(na.gain + n_tile * BN + i) : 0.f;
     }
-    if (emit && warp == 2 && lane == 0) {
+    if (emit && warp == 2 && tc::elect_one()) {
         int boxes = 0;
         for (int c = 0; c < BN / 32; ++c) boxes += n_tile * BN + c * 32 < N;
         tc::mbar_expect_tx(&s.c_bar, (uint32_t)boxes * BM * 128);
@@ -203,7 +203,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
 
     if (warp == 0) {
         // ---- producer: one thread feeds the ring of stages -------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             // (sending a box costs this thread about 60 cycles whatever the box's size, a division
             // by a run-time value a hundred, a dependent integer instruction about 5, so
             // the loop around it carries the stage and its parity along instead of dividing)
@@ -245,15 +245,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         }
     } else if (warp == 1) {
         // ---- MMA issuer --------------------------------------------------------
-        // One thread, and for tiles up to 128 columns wide its own instructions are what a
-        // step of K takes: sending a tcgen05.mma costs the thread about 54 cycles (the tensor
-        // cores need 32 to 64 for 64 to 128 columns), a commit about 60, and every dependent
-        // integer instruction of a lone thread about 5.  So the ring is walked by an unrolled
+        // One thread, and for tiles up to 128 columns wide its own instructions are much of what a
+        // step of K takes (the tensor cores need 32 to 64 cycles an MMA for 64 to 128 columns, and
+        // every dependent integer instruction of a lone thread is about 5).  So the ring is walked by an unrolled
         // loop: a stage's barriers and operand descriptors are constants away from those of
         // stage 0 (the descriptor's low word carries the address in 16-byte units, its high
         // word is the same for every tile), and only the first MMA of the first stage asks
         // whether it accumulates.
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc = tc::instr_desc_bf16(BM, BN);
             constexpr uint32_t A_STEP = sizeof(s.a[0]) >> 4, B_STEP = sizeof(s.b[0]) >> 4;
             constexpr uint32_t A_HALF = (BM * BK * 2) >> 4;

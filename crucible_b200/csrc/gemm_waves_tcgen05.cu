@@ -127,7 +127,7 @@ gemm_waves_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     };
     // the first stages' W go out before the kernels ahead of this one are done: no kernel writes a weight
     const int w_ahead = FORM == GROUPED ? 0 : min(k_blocks, STAGES);
-    if (warp == 0 && lane == 0 && w_ahead > 0) {
+    if (warp == 0 && w_ahead > 0 && tc::elect_one()) {
         const Tile x = tile_at(blockIdx.x);
         for (int kb = 0; kb < w_ahead; ++kb) {
             tc::mbar_expect_tx(&s.full_bar[kb], STAGE_BYTES);
@@ -139,7 +139,7 @@ gemm_waves_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (FORM == GROUPED) tiles = min(__ldg(na.plan), na.max_tiles) * n_tiles;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int st = 0, ahead = w_ahead, sent = 0;
             uint32_t parity = 1;                         // of a stage's last round, once there was one
             bool ok = true, first_round = true;
@@ -172,7 +172,7 @@ gemm_waves_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc = tc::instr_desc_bf16(BM, BN);
             constexpr uint32_t A_STEP = sizeof(s.a[0]) >> 4, B_STEP = sizeof(s.b[0]) >> 4;
             const uint64_t desc0 = tc::smem_desc_sw128(tc::smem_u32(s.a[0]));

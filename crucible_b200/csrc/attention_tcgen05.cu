@@ -300,8 +300,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         auto send = [&](int page, bool values, int feature) -> bool {
             const int st = item % SLOTS;
             const int rel = BOTH ? item : item >> 1, round = rel / Store::RELEASES;
-            // (of a pair's two slots both wait: the second's test passes at once)
-            if (round > 0 && !__all_sync(0xffffffffu, tc::mbar_wait(&s.empty[rel % Store::RELEASES], (round - 1) & 1, abort_flag))) {
+            // (A pair's first slot waits for both.  The second must not ask again: the last pair's release may
+            // come round as soon as its first slot's values have been used, and the phase asked for is then
+            // two behind, which reads as not over yet.)
+            if (round > 0 && (BOTH || (item & 1) == 0) && !__all_sync(0xffffffffu, tc::mbar_wait(&s.empty[rel % Store::RELEASES], (round - 1) & 1, abort_flag))) {
                 tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
                 return false;
             }
@@ -388,6 +390,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // over the scores that it was made from, so the scores that take its buffer follow the second
         // product, which the tensor pipe works off in order; the softmax of the tiles between runs beside both.
         if (n_tiles > 0) {
+            const bool sender = tc::elect_one();
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(ROWS, KEYS);
             constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, Store::PART);
             // Operand descriptors by addition: the low word carries the address in 16-byte
@@ -414,7 +417,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     if (!wait(&s.full[st], (item / SLOTS) & 1)) return false;
                     tc::tc_fence_after_sync();
                     const uint32_t k_lo = k_lo0 + st * SLOT;
-                    if (tc::elect_one()) {
+                    if (sender) {
 #pragma unroll
                         for (int k = 0; k < Store::PART / 16; ++k) {
                             const uint64_t q_desc = tc::desc_of(q_lo + (part * HALVES + (k >> 2)) * HALF + 2 * (k & 3), desc_hi);
@@ -425,7 +428,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     }
                     ++item;
                 }
-                if (tc::elect_one()) {
+                if (sender) {
                     tc::umma_commit(&s.s_full[to]);
                     // pairs: K0 and K1; with two buffers V_(j-2) and K_j, with three K_(t+2) and V_t
                     if (!BOTH && (S_BUFS == 2 ? j > 0 : j == 1)) tc::umma_commit(&s.empty[(j - 1) % Store::RELEASES]);
@@ -448,7 +451,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     for (int half = 0; half < 2; ++half) {
                         if (part == 0 && !wait(half ? &s.p_full[b] : &s.p_half[b], parity)) return false;
                         tc::tc_fence_after_sync();
-                        if (tc::elect_one()) {
+                        if (sender) {
 #pragma unroll
                             for (int k = 4 * half; k < 4 * half + 4; ++k) {
                                 // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
@@ -458,12 +461,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                             }
                         }
                     }
-                    if (BOTH && tc::elect_one()) tc::umma_commit(&s.empty[st]);
+                    if (BOTH && sender) tc::umma_commit(&s.empty[st]);
                     if (!BOTH) ++item;
                 }
-                if (tc::elect_one()) {
+                if (sender) {
                     if (GROUPS == 1) tc::umma_commit(&s.pv_done[t & 1]);
-                    if (S_BUFS == 3) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
+                    // (not after the last tile: the loader may still be about to ask for this barrier's phase before)
+                    if (S_BUFS == 3 && t + 1 < n_tiles) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
                     if (t == n_tiles - 1) tc::umma_commit(&s.o_done);
                 }
                 return true;

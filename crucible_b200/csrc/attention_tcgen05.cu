@@ -15,15 +15,21 @@
 // P goes back into tensor memory, over the scores that it was made from, and is the first operand of the
 // second product there: shared memory carries queries, keys and values alone (a 128 x 128 x 128 tile: 1,280
 // cycles of its 128 bytes a cycle; with P written to and read from it 1,790, more than the products' 1,024).
-// Two groups of four softmax warps take the tiles in turn (tile j: group j % 2), each with its own
-// buffer of scores, its own reference maximum, sum and accumulator, merged when the keys are through.
+// Two groups of four softmax warps take the tiles in turn (tile j: group j % 2).  Head size 64: each has its
+// own reference maximum, sum and accumulator, merged when the keys are through.  128 and 256: one
+// accumulator and a reference that goes from tile to tile, so that three (256: two) buffers of scores find room and
+// a group's next scores need not wait for its last second product (16 heads of 128, 2,048 tokens 28.2 -> 26.8 us,
+// of 256 31.9 -> 31.0; with 64 features there is room for all of it).
 // A tile's code is kept short (64 scores at a time, loops not unrolled): a block lives 10 to 20 us,
 // and code that is met for the first time comes from memory (the masks of 128 scores, unrolled: 7,500 cycles).
-// What bounds it: a tile takes a group some 3,400 cycles (head size 64), of which the special-function unit's
-// 8 a warp and exponential make 1,024 (two groups 2,048), the maxima 400, the scores' way 200 to 900.
-// Measured on one B200, a 2,048-token prompt: 12 heads of 64 on 4 20 us a layer (27 with P in shared memory
-// and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 33 (59), 16 heads of 256 on 1
-// 38 (76).
+// What bounds it: a pair of tiles takes the two groups some 3,000 cycles (head size 64), of which the
+// special-function unit's 8 a warp and exponential make 2,048; the rest is what a tile takes besides (the
+// maxima 400, the way to and from the barriers 400), at which the other group is not always busy with its
+// exponentials: set half a tile apart the groups were no faster (17.9 and 17.9), in turns slower (18.5), and a quarter
+// of the exponentials on the FMA pipe gave 2 %, 7 % less where most blocks are short.
+// Measured on one B200, replayed, a 2,048-token prompt: 12 heads of 64 on 4 17.8 us a layer (27 with P in shared
+// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 25.8 (58), 16
+// heads of 256 on 1 30.8 (76).
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
 // tile's maximum exceeds it by more than 2^8 (in the base-2 exponent), so P
@@ -34,7 +40,7 @@
 // Rows of 256 features that are keys and values at once (a latent with its rotated part: one
 // key head for all query heads): a stage holds the tile once; the first product reads it
 // with the features contracted, the second with the keys contracted.  A tile's 2 x 128 x 128 x 256
-// multiply-adds are 2,048 cycles of the tensor pipe; one softmax group takes 2,700.
+// multiply-adds are 2,048 cycles of the tensor pipe.
 //
 // Sizes: head size 64 or 128, or 256 if the pages' rows are keys and values at once; page size a power of two from 8 to 128; any head
 // counts and group sizes; window.  Anything else is refused and the mma.sync
@@ -79,14 +85,6 @@ struct TcAttnParams {
     int* status;
 };
 
-// 1 / (1 + e^-x); 0 for x so low that e^-x is infinite.  (The IEEE division costs a hundred dependent cycles
-// an element; the reciprocal is within one unit in the last place, 2^-15 of what the bf16 result keeps.)
-__device__ __forceinline__ float sigmoid(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.0f + expf(-x)));
-    return y;
-}
-
 // GATE: the results' gate, fixed when it is compiled: the epilogue runs once per block and its instructions
 // come from memory (12 heads of 64 without a gate, a 2,048-token prompt: 32 us; with the code of the gate of a
 // logit a result beside it 0.3 us more, of both gates 1.4).
@@ -111,18 +109,21 @@ struct Storage {
     static constexpr int RELEASES = BOTH ? SLOTS : PAIRS;
     // buffers of scores: what 512 columns of tensor memory hold beside the accumulators.  With three the
     // next scores of a group are there when it asks for them; with two they follow its tile's second product.
-    static constexpr int S_BUFS = HD == 64 ? 3 : 2;
-    // softmax groups of four warps that take the tiles in turn (tile j: group j % GROUPS), each
-    // with its own reference maximum, sum and accumulator, merged at the end
-    static constexpr int GROUPS = BOTH ? 1 : 2;
+    static constexpr int S_BUFS = BOTH ? 2 : 3;
+    // two softmax groups of four warps take the tiles in turn (tile j: group j % 2).  Head size 64: each with its
+    // own reference maximum, sum and accumulator, merged at the end.  Else (SHARED) one accumulator, for
+    // which a row's reference goes from tile to tile through shared memory: two of 128 columns would leave
+    // room for two buffers of scores, and the next scores would wait for the second product of two tiles back.
+    static constexpr int GROUPS = 2;
+    static constexpr bool SHARED = HD > 64;
     static constexpr int THREADS = 64 + 128 * GROUPS;       // loader, MMA thread, the softmax groups
     alignas(1024) uint8_t q[HD / 64][ROWS * 128];
     alignas(1024) uint8_t ring[SLOTS][HALVES][KEYS * 128];
     alignas(8) uint64_t full[SLOTS];
     uint64_t empty[RELEASES];
     uint64_t q_full, gate_full, o_done;
-    uint64_t s_full[S_BUFS], p_half[S_BUFS], p_full[S_BUFS], pv_done[2];
-    float2 merge[GROUPS][ROWS];                             // a row's (reference, sum) of each group
+    uint64_t s_full[S_BUFS], p_half[S_BUFS], p_full[S_BUFS], pv_done[2], m_full[2];
+    float m_row[2][ROWS];                                   // shared: a row's reference as of a tile (tile j: j & 1)
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -172,6 +173,39 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return d;
 }
 
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t both_of(float v) { return pair_of(v, v); }
+
+// (a, b) times 1 / (1 + e^-x) of their logits: 16,384 of them a tile with a logit a result, when nothing else
+// is left to do, so that their instructions count: 18 a pair, where expf and the IEEE division took a hundred dependent
+// cycles an element.  e^-x = 2^n 2^f: n is -x log2(e) rounded (Cody and Waite's reduction; adding 1.5 * 2^23 leaves n in
+// the sum's low bits), f the rest with log2(e) in two parts.  The reciprocal is within one unit in the last place,
+// 2^-15 of what the bf16 result keeps; beyond +-88 the results are those at 88, 1 and (flushed) 0.
+__device__ __forceinline__ void gate_pair(float& a, float& b, float x0, float x1) {
+    constexpr float LOG2E_LOW = 1.925963033500988e-8f;            // log2(e) - LOG2E
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-88.5f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-88.5f));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(87.f));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(87.f));
+    const uint64_t x = pair_of(x0, x1), r = fma2(x, both_of(-LOG2E), both_of(12582912.f));
+    const uint64_t minus_n = fma2(r, both_of(-1.f), both_of(12582912.f));
+    const uint64_t f = fma2(x, both_of(-LOG2E_LOW), fma2(x, both_of(-LOG2E), minus_n));
+    float f0, f1, r0, r1;
+    pair_to(f, f0, f1);
+    pair_to(r, r0, r1);
+    const float s0 = __uint_as_float((__float_as_uint(r0) << 23) + 0x3f800000u);
+    const float s1 = __uint_as_float((__float_as_uint(r1) << 23) + 0x3f800000u);
+    float d0, d1, y0, y1;
+    pair_to(fma2(pair_of(ex2_fast(f0), ex2_fast(f1)), pair_of(s0, s1), both_of(1.f)), d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(d1));
+    pair_to(mul2(pair_of(a, b), pair_of(y0, y1)), a, b);
+}
+
 // the low n bits
 __device__ __forceinline__ uint32_t bits_below(int n) {
     return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u;
@@ -188,7 +222,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     using Store = Storage<HD>;
     constexpr int NH = HD / 64, SLOTS = Store::SLOTS, GROUPS = Store::GROUPS, HALVES = Store::HALVES;
     constexpr int S_BUFS = Store::S_BUFS;
-    constexpr bool BOTH = Store::BOTH;
+    constexpr bool BOTH = Store::BOTH, SHARED = Store::SHARED;
     constexpr uint32_t SLOT_BYTES = KEYS * Store::PART * 2;
     constexpr uint32_t TMEM_COLS = 512;                  // scores: 128 columns a buffer, then O
     Store& s = *reinterpret_cast<Store*>(smem_raw);
@@ -225,7 +259,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             tc::mbar_init(&s.p_half[b], 4);               // one arrival per softmax warp
             tc::mbar_init(&s.p_full[b], 4);
         }
-        for (int b = 0; b < 2; ++b) tc::mbar_init(&s.pv_done[b], 1);
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&s.pv_done[b], 1);
+            tc::mbar_init(&s.m_full[b], 4);
+        }
         s.abort_flag = 0;
         tc::fence_barrier_init();
         tc::prefetch_tensormap(&map_k);
@@ -437,7 +474,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 return true;
             };
             auto products = [&](int t) -> bool {  // O += P_t V_t: 128 keys in eight steps of 16
-                const uint32_t d_o = tmem_o + (GROUPS > 1 ? (uint32_t)(t & 1) * HD : 0u);
+                const uint32_t d_o = tmem_o + (SHARED ? 0u : (uint32_t)(t & 1) * HD);
                 const int b = t % S_BUFS;
                 const uint32_t p_at = tmem_s + b * 128;
                 const uint32_t parity = (t / S_BUFS) & 1;
@@ -456,7 +493,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                             for (int k = 4 * half; k < 4 * half + 4; ++k) {
                                 // 16 keys further down V: 16 rows of 128 bytes = 128 descriptor units
                                 const uint64_t v_desc = tc::desc_of(v_lo + 128 * k, desc_hi);
-                                if (k == 0) tc::umma_bf16_ts(d_o + part * 128, p_at + 8 * k, v_desc, idesc_pv, t >= GROUPS ? 1u : 0u);
+                                if (k == 0) tc::umma_bf16_ts(d_o + part * 128, p_at + 8 * k, v_desc, idesc_pv, t >= (SHARED ? 1 : GROUPS) ? 1u : 0u);
                                 else tc::umma_bf16_ts_add(d_o + part * 128, p_at + 8 * k, v_desc, idesc_pv);
                             }
                         }
@@ -465,7 +502,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     if (!BOTH) ++item;
                 }
                 if (sender) {
-                    if (GROUPS == 1) tc::umma_commit(&s.pv_done[t & 1]);
+                    if (BOTH) tc::umma_commit(&s.pv_done[t & 1]);
                     // (not after the last tile: the loader may still be about to ask for this barrier's phase before)
                     if (S_BUFS == 3 && t + 1 < n_tiles) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
                     if (t == n_tiles - 1) tc::umma_commit(&s.o_done);
@@ -484,8 +521,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // ---- softmax: warps 2..5 (and 6..9: the second group), one thread per row =
         // tensor-memory lane; a group takes every GROUPS-th tile -------------------------------
         const int quarter = warp & 3;
-        const int group = GROUPS > 1 ? (warp - 2) >> 2 : 0;
-        const uint32_t tmem_mine = tmem_o + (uint32_t)group * HD;
+        const int group = (warp - 2) >> 2;
+        const uint32_t tmem_mine = tmem_o + (SHARED ? 0u : (uint32_t)group * HD);
         const int r = quarter * 32 + lane;
         const int row = first_row + r;
         const bool real = active && r < tile_rows && row < n_rows;
@@ -495,6 +532,22 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         const int lo = real ? first_key(p, pos) : 0;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
         cb_pdl_wait();
+        // what the row needs at its end, asked for now
+        __nv_bfloat16* dst = nullptr;
+        const __nv_bfloat16* gate = nullptr;
+        float gate_f = 1.f;
+        float sink = -INFINITY;                       // in the base-2 exponent
+        if (real) {
+            const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
+            if (p.sinks != nullptr) sink = p.sinks[head] * LOG2E;
+            dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
+            if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
+            if (GATE == GATE_HEAD) {
+                float none = 1.f;
+                const float x = __bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]);
+                gate_pair(gate_f, none, x, x);
+            }
+        }
         if (!p.q_boxes && n_tiles > 0) {
             // group sizes whose tiles would leave much of the 128 rows empty: the rows by hand,
             // 16-byte pieces into the 128-byte swizzle
@@ -566,20 +619,33 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             float mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3]));
             mx *= p.scale_log2;
             // raise the reference maximum only when it is exceeded by far; the accumulator
-            // in tensor memory is rescaled then, by the whole warp at once.  Two groups, two buffers: the
-            // scores' commit covers the second product of this group's tile before; else that is waited for.
-            float corr = 1.0f;
-            if (mx > m_ref + RAISE || (m_ref == -INFINITY && mx > -INFINITY)) {
-                corr = m_ref == -INFINITY ? 0.f : exp2f(m_ref - mx);
-                m_ref = mx;
+            // in tensor memory is rescaled then, by the whole warp at once, after the second product
+            // that was the last to add to it.  A shared accumulator's reference is the one of the tile before.
+            float m_was = m_ref;
+            if (SHARED && j > 0) {
+                ok = wait_all(&s.m_full[(j - 1) & 1], ((j - 1) >> 1) & 1);
+                if (!ok) break;
+                m_was = s.m_row[(j - 1) & 1][r];
             }
-            if (j >= GROUPS && __any_sync(0xffffffffu, corr != 1.0f)) {
-                if (GROUPS == 1 || S_BUFS == 3) {
-                    ok = GROUPS == 1 ? wait_all(&s.pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1)
-                                     : wait_all(&s.empty[(j - 1) % Store::RELEASES], ((j - 1) / Store::RELEASES) & 1);
-                    if (!ok) break;
-                    tc::tc_fence_after_sync();
-                }
+            float m_new = m_was;
+            if (mx > m_was + RAISE || (m_was == -INFINITY && mx > -INFINITY)) m_new = mx;
+            if (SHARED) {
+                s.m_row[j & 1][r] = m_new;
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&s.m_full[j & 1]);
+            }
+            if (__any_sync(0xffffffffu, m_new != m_ref)) {      // (of what this group summed, of what all have)
+                const float mine = m_new == m_ref ? 1.f : m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
+                l *= mine;
+                m_ref = m_new;
+            }
+            if (j >= (SHARED ? 1 : GROUPS) && __any_sync(0xffffffffu, m_new != m_was)) {
+                const float corr = m_new == m_was ? 1.f : m_was == -INFINITY ? 0.f : exp2f(m_was - m_new);
+                constexpr int BACK = SHARED ? 1 : GROUPS, R = Store::RELEASES;
+                ok = BOTH ? wait_all(&s.pv_done[(j - BACK) & 1], ((j - BACK) >> 1) & 1)
+                          : wait_all(&s.empty[(j - BACK + 1) % R], ((j - BACK + 1) / R) & 1);
+                if (!ok) break;
+                tc::tc_fence_after_sync();
 #pragma unroll 1
                 for (int c0 = 0; c0 < HD; c0 += 32) {
                     uint32_t v[32];
@@ -591,7 +657,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 }
                 tc::tmem_st_wait();
             }
-            l *= corr;
             // P = exp2(s * scale - reference) in bf16, two a column, over the scores' own columns:
             // keys 0-63 into the first 32, 64-127 into the next (their scores, columns 64-127, are
             // read after the first half's, whose columns are 0-63)
@@ -629,18 +694,6 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // ---- the output: O / l ------------------------------------------------------------
         const int my_tiles = n_tiles > group ? (n_tiles - group + GROUPS - 1) / GROUPS : 0;
         if (n_tiles > 0 && ok) ok = wait_all(&s.o_done, 0);
-        __nv_bfloat16* dst = nullptr;
-        const __nv_bfloat16* gate = nullptr;
-        float gate_f = 1.f;
-        float sink = -INFINITY;                       // in the base-2 exponent
-        if (real) {
-            const int tok = row_base + row / n_rep, head = kv_head * n_rep + row % n_rep;
-            if (p.sinks != nullptr) sink = p.sinks[head] * LOG2E;
-            dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
-            if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
-            if (GATE == GATE_HEAD)
-                gate_f = sigmoid(__bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]));
-        }
         if (GATE == GATE_RESULT && p.q_boxes && n_tiles > 0 && ok) ok = wait_all(&s.gate_full, 0);
         // where the loader put the gate's logits: behind the ring's last slot (see there)
         const int gate_item = 2 * n_tiles;
@@ -658,7 +711,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     const uint4 raw = *reinterpret_cast<const uint4*>(from);
                     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= sigmoid(__bfloat162float(g[i]));
+                    for (int i = 0; i < 8; i += 2)
+                        gate_pair(o[8 * q4 + i], o[8 * q4 + i + 1], __bfloat162float(g[i]), __bfloat162float(g[i + 1]));
                 }
                 if (GATE == GATE_HEAD) {
 #pragma unroll
@@ -680,75 +734,57 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             constexpr int MINE = HD / GROUPS, ACROSS = MINE < 64 ? MINE / 8 : 8;      // pieces of a row side by side
             __syncwarp();
             const unsigned long long mine = real ? (unsigned long long)dst : 0ull;
-#pragma unroll 1
-            for (int rr = lane / ACROSS; rr < 32; rr += 32 / ACROSS) {
+#pragma unroll 4
+            for (int r0 = 0; r0 < 32; r0 += 32 / ACROSS) {
+                const int rr = r0 + lane / ACROSS, at = quarter * 32 + rr;
                 __nv_bfloat16* to = (__nv_bfloat16*)__shfl_sync(0xffffffffu, mine, rr);
-                const int at = quarter * 32 + rr;
+                uint4 w[MINE / (8 * ACROSS)];
+#pragma unroll
+                for (int i = 0; i < MINE / (8 * ACROSS); ++i) {
+                    const int f = group * MINE + 8 * (i * ACROSS + lane % ACROSS);
+                    w[i] = *reinterpret_cast<const uint4*>(s.q[f >> 6] + at * 128 + ((((f & 63) >> 3) ^ (at & 7)) << 4));
+                }
                 if (to != nullptr)
 #pragma unroll
-                    for (int f0 = 0; f0 < MINE; f0 += 8 * ACROSS) {
-                        const int f = group * MINE + f0 + 8 * (lane % ACROSS);
-                        *reinterpret_cast<uint4*>(to + f) = *reinterpret_cast<const uint4*>(
-                            s.q[f >> 6] + at * 128 + ((((f & 63) >> 3) ^ (at & 7)) << 4));
-                    }
+                    for (int i = 0; i < MINE / (8 * ACROSS); ++i)
+                        *reinterpret_cast<uint4*>(to + group * MINE + 8 * (i * ACROSS + lane % ACROSS)) = w[i];
             }
         };
-        if (GROUPS > 1) {
-            // Two groups: each holds the sums over its own tiles against its own reference.
-            // A row's two states meet in shared memory; every thread comes to the barrier,
-            // whatever happened to its waits.  Then group g writes its half of the features.
-            s.merge[group][r] = make_float2(my_tiles > 0 ? m_ref : -INFINITY, my_tiles > 0 ? l : 0.f);
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (ok && n_tiles > 0 && !*abort_flag) {
-                tc::tc_fence_after_sync();
-                const float2 other = s.merge[GROUPS > 1 ? group ^ 1 : 0][r];
-                const float m_mine = my_tiles > 0 ? m_ref : -INFINITY;
-                const float m_all = fmaxf(fmaxf(m_mine, other.x), sink);
-                const float f_mine = m_mine == -INFINITY ? 0.f : exp2f(m_mine - m_all);
-                const float f_other = other.x == -INFINITY ? 0.f : exp2f(other.x - m_all);
-                float l_all = (my_tiles > 0 ? l : 0.f) * f_mine + other.y * f_other;
-                if (sink != -INFINITY) l_all += exp2f(sink - m_all);
-                const float inv = l_all > 0.f ? p.out_scale / l_all : 0.f;
-                const float w_mine = f_mine * inv, w_other = f_other * inv;
-                // An accumulator that no MMA has written holds whatever was there and is not
-                // read.  Whether a group had tiles is the same for every thread of the block,
-                // as it must be: the loads are the whole warp's (.sync.aligned).  A row that
-                // could read none of a group's keys has weight 0 and finite sums (zeros) there.
-                const bool mine_any = my_tiles > 0, other_any = n_tiles > my_tiles;
-#pragma unroll 1
-                for (int c0 = group * (HD / 2); c0 < (group + 1) * (HD / 2); c0 += 32) {
-                    uint32_t a[32], b[32];
-                    if (mine_any) tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, a);
-                    if (other_any) tc::tmem_ld_32x32(tmem_o + (uint32_t)(group ^ 1) * HD + lane_bits + c0, b);
-                    tc::tmem_ld_wait();
-                    if (real) {
-                        float o[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            o[i] = (mine_any ? __uint_as_float(a[i]) * w_mine : 0.f) +
-                                   (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
-                        close(o, c0);
-                    }
-                }
-                write_rows();
-            }
-        } else if (ok && n_tiles > 0) {
+        // Each group holds the sums over its own tiles against the reference of its last one.
+        // A row's two states meet in shared memory; every thread comes to the barrier,
+        // whatever happened to its waits.  Then group g writes its half of the features.
+        float2* const merge = reinterpret_cast<float2*>(s.ring[(gate_item + 2) % SLOTS][0]);     // (nothing is there any more)
+        merge[group * ROWS + r] = make_float2(my_tiles > 0 ? m_ref : -INFINITY, my_tiles > 0 ? l : 0.f);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (ok && n_tiles > 0 && !*abort_flag) {
             tc::tc_fence_after_sync();
-            float inv = l > 0.f ? p.out_scale / l : 0.f;
-            if (sink != -INFINITY) {
-                const float top = fmaxf(m_ref, sink);
-                const float keep = exp2f(m_ref - top);
-                inv = keep * p.out_scale / (l * keep + exp2f(sink - top));
-            }
+            const float2 other = merge[(group ^ 1) * ROWS + r];
+            const float m_mine = my_tiles > 0 ? m_ref : -INFINITY, m_both = fmaxf(m_mine, other.x);
+            const float m_all = fmaxf(m_both, sink);
+            const float f_mine = m_mine == -INFINITY ? 0.f : exp2f(m_mine - m_all);
+            const float f_other = other.x == -INFINITY ? 0.f : exp2f(other.x - m_all);
+            float l_all = (my_tiles > 0 ? l : 0.f) * f_mine + other.y * f_other;
+            if (sink != -INFINITY) l_all += exp2f(sink - m_all);
+            const float inv = l_all > 0.f ? p.out_scale / l_all : 0.f;
+            // (a shared accumulator stands against the last tile's reference, the higher one)
+            const float w_mine = SHARED ? fmaxf(f_mine, f_other) * inv : f_mine * inv, w_other = f_other * inv;
+            // An accumulator that no MMA has written holds whatever was there and is not
+            // read.  Whether a group had tiles is the same for every thread of the block,
+            // as it must be: the loads are the whole warp's (.sync.aligned).  A row that
+            // could read none of a group's keys has weight 0 and finite sums (zeros) there.
+            const bool mine_any = SHARED || my_tiles > 0, other_any = !SHARED && n_tiles > my_tiles;
 #pragma unroll 1
-            for (int c0 = 0; c0 < HD; c0 += 32) {
-                uint32_t v[32];
-                tc::tmem_ld_32x32(tmem_o + lane_bits + c0, v);
+            for (int c0 = group * (HD / 2); c0 < (group + 1) * (HD / 2); c0 += 32) {
+                uint32_t a[32], b[32];
+                if (mine_any) tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, a);
+                if (other_any) tc::tmem_ld_32x32(tmem_o + (uint32_t)(group ^ 1) * HD + lane_bits + c0, b);
                 tc::tmem_ld_wait();
                 if (real) {
                     float o[32];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(v[i]) * inv;
+                    for (int i = 0; i < 32; ++i)
+                        o[i] = (mine_any ? __uint_as_float(a[i]) * w_mine : 0.f) +
+                               (other_any ? __uint_as_float(b[i]) * w_other : 0.f);
                     close(o, c0);
                 }
             }

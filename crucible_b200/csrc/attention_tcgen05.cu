@@ -40,7 +40,9 @@
 // Rows of 256 features that are keys and values at once (a latent with its rotated part: one
 // key head for all query heads): a stage holds the tile once; the first product reads it
 // with the features contracted, the second with the keys contracted.  A tile's 2 x 128 x 128 x 256
-// multiply-adds are 2,048 cycles of the tensor pipe.
+// multiply-adds are 2,048 cycles of the tensor pipe, 1,792 where only 192 features are asked for (31.0 -> 29.0 us
+// a layer): there a group's softmax, its second product and its next scores stand in a row, 4,500 cycles for
+// two tiles, since 512 columns hold no third buffer of scores.
 //
 // Sizes: head size 64 or 128, or 256 if the pages' rows are keys and values at once; page size a power of two from 8 to 128; any head
 // counts and group sizes; window.  Anything else is refused and the mma.sync
@@ -48,6 +50,7 @@
 // Reference counterpart: `attention_prefill_exact_*`
 // (engine/kernels/kernels.cu:2257-2275).
 #define CB_PDL_BIT 1      // this file's bit in CRUCIBLE_PDL
+#include <type_traits>
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -98,15 +101,20 @@ enum Gate { GATE_NONE = 0, GATE_RESULT = 1, GATE_HEAD = 2 };
 // a tile's features 0-127, then 128-255; a slot is free once the second product has read it.  Five
 // slots are what 227 KB hold beside the queries: the upper half of tile t + 2 travels while the
 // second product of tile t reads its own upper half.
-template <int HD>
+// NARROW (256): only the first 192 features are values (a latent; the rotated part is key alone).  Three tiles'
+// 192 features and one tile's last 64 then: the last 64 are free again when the tile's scores are there, so all of
+// tile t + 2 is there when its scores' turn comes, and a second product is a quarter shorter.
+template <int HD, bool NARROW>
 struct Storage {
     static constexpr bool BOTH = HD == 256;                 // a cached row is key and value
-    static constexpr int PART = BOTH ? 128 : HD;            // features of a slot
+    static constexpr int VALUES = NARROW ? 192 : HD;        // features of a result
+    static constexpr int PART = NARROW ? 64 : BOTH ? 128 : HD;      // features of a slot
     static constexpr int PARTS = HD / PART;
     static constexpr int HALVES = PART / 64;
     static constexpr int PAIRS = HD == 64 ? 4 : 3;
-    static constexpr int SLOTS = BOTH ? 5 : 2 * PAIRS;
-    static constexpr int RELEASES = BOTH ? SLOTS : PAIRS;
+    static constexpr int SLOTS = NARROW ? 10 : BOTH ? 5 : 2 * PAIRS;
+    static constexpr int FULLS = NARROW ? 4 : SLOTS;        // narrow: three tiles' 192 features, then the last 64
+    static constexpr int RELEASES = NARROW ? 4 : BOTH ? SLOTS : PAIRS;
     // buffers of scores: what 512 columns of tensor memory hold beside the accumulators.  With three the
     // next scores of a group are there when it asks for them; with two they follow its tile's second product.
     static constexpr int S_BUFS = BOTH ? 2 : 3;
@@ -119,7 +127,7 @@ struct Storage {
     static constexpr int THREADS = 64 + 128 * GROUPS;       // loader, MMA thread, the softmax groups
     alignas(1024) uint8_t q[HD / 64][ROWS * 128];
     alignas(1024) uint8_t ring[SLOTS][HALVES][KEYS * 128];
-    alignas(8) uint64_t full[SLOTS];
+    alignas(8) uint64_t full[FULLS];
     uint64_t empty[RELEASES];
     uint64_t q_full, gate_full, o_done;
     uint64_t s_full[S_BUFS], p_half[S_BUFS], p_full[S_BUFS], pv_done[2], m_full[2];
@@ -211,15 +219,15 @@ __device__ __forceinline__ uint32_t bits_below(int n) {
     return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u;
 }
 
-template <int HD, int GATE>
-__global__ void __launch_bounds__(Storage<HD>::THREADS, 1)
+template <int HD, int GATE, bool NARROW>
+__global__ void __launch_bounds__(Storage<HD, NARROW>::THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                          const __grid_constant__ CUtensorMap run_k, const __grid_constant__ CUtensorMap run_v,
                          const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_gate,
                          const TcAttnParams p) {
     // 1024-byte alignment (the swizzled tiles need it) is asked of the declaration
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    using Store = Storage<HD>;
+    using Store = Storage<HD, NARROW>;
     constexpr int NH = HD / 64, SLOTS = Store::SLOTS, GROUPS = Store::GROUPS, HALVES = Store::HALVES;
     constexpr int S_BUFS = Store::S_BUFS;
     constexpr bool BOTH = Store::BOTH, SHARED = Store::SHARED;
@@ -249,7 +257,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     volatile int* abort_flag = &s.abort_flag;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < SLOTS; ++i) tc::mbar_init(&s.full[i], 1);
+        for (int i = 0; i < Store::FULLS; ++i) tc::mbar_init(&s.full[i], 1);
         for (int i = 0; i < Store::RELEASES; ++i) tc::mbar_init(&s.empty[i], 1);
         tc::mbar_init(&s.q_full, p.q_boxes ? 1 : 4 * GROUPS);
         tc::mbar_init(&s.gate_full, 1);
@@ -333,6 +341,26 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             const int page = table[index];
             return page < 0 ? 0 : page;               // an entry given back early: never read
         };
+        // a tile's features from `feature` on, 64 to a slot's half, to `to`; N halves
+        auto copy = [&](int page, bool values, int feature, uint8_t (*to)[KEYS * 128], auto halves, uint64_t* full) {
+            constexpr int N = decltype(halves)::value;
+            // pages that follow one another in the pool come in with one copy per half
+            const int page0 = __shfl_sync(0xffffffffu, page, 0);
+            const bool run = __all_sync(0xffffffffu, lane >= pages_per_tile || page == page0 + lane) && p.runs != 0 &&
+                             page0 + pages_per_tile <= p.n_pages;
+            if (lane == 0) tc::mbar_expect_tx(full, N * KEYS * 128);
+            __syncwarp();
+            if (run) {
+                if (lane < N)
+                    tc::tma_load_4d(to[lane], values ? &run_v : &run_k, full, feature + lane * 64, 0, kv_head, page0);
+            } else if (lane < pages_per_tile) {
+                const int dst = (lane << p.page_shift) * 128;
+                const int y = (page * p.n_kv_heads + kv_head) << p.page_shift;
+#pragma unroll
+                for (int h = 0; h < N; ++h)
+                    tc::tma_load_2d(to[h] + dst, values ? &map_v : &map_k, full, feature + h * 64, y);
+            }
+        };
         int item = 0, armed = 0;                      // the next slot's number; slots with copies sent
         auto send = [&](int page, bool values, int feature) -> bool {
             const int st = item % SLOTS;
@@ -344,22 +372,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
                 return false;
             }
-            // pages that follow one another in the pool come in with one copy per slot and half
-            const int page0 = __shfl_sync(0xffffffffu, page, 0);
-            const bool run = __all_sync(0xffffffffu, lane >= pages_per_tile || page == page0 + lane) && p.runs != 0 &&
-                             page0 + pages_per_tile <= p.n_pages;
-            if (lane == 0) tc::mbar_expect_tx(&s.full[st], SLOT_BYTES);
-            __syncwarp();
-            if (run) {
-                if (lane < HALVES)
-                    tc::tma_load_4d(s.ring[st][lane], values ? &run_v : &run_k, &s.full[st], feature + lane * 64, 0, kv_head, page0);
-            } else if (lane < pages_per_tile) {
-                const int dst = (lane << p.page_shift) * 128;
-                const int y = (page * p.n_kv_heads + kv_head) << p.page_shift;
-#pragma unroll
-                for (int h = 0; h < HALVES; ++h)
-                    tc::tma_load_2d(s.ring[st][h] + dst, values ? &map_v : &map_k, &s.full[st], feature + h * 64, y);
-            }
+            copy(page, values, feature, s.ring[st], std::integral_constant<int, HALVES>{}, &s.full[st]);
             armed = ++item;
             return true;
         };
@@ -374,7 +387,24 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 tc::tma_load_3d(s.q[h], &map_q, &s.q_full, h * 64, kv_head * n_rep, row_base + first_tok);
         }
         __syncwarp();
-        if (BOTH) {
+        int last_armed = 0;                           // narrow: tiles whose last 64 features have been sent
+        if constexpr (NARROW) {
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                const int st = j % 3;
+                ok = (j < 3 || __all_sync(0xffffffffu, tc::mbar_wait(&s.empty[st], (j / 3 - 1) & 1, abort_flag)));
+                if (ok) {
+                    copy(pg0, false, 0, &s.ring[3 * st][0], std::integral_constant<int, 3>{}, &s.full[st]);
+                    armed = j + 1;
+                    ok = j < 1 || __all_sync(0xffffffffu, tc::mbar_wait(&s.empty[3], (j - 1) & 1, abort_flag));
+                }
+                if (ok) {
+                    copy(pg0, false, 192, &s.ring[9][0], std::integral_constant<int, 1>{}, &s.full[3]);
+                    last_armed = j + 1;
+                }
+                if (!ok) tc::give_up(abort_flag, p.status, tc::ST_PRODUCER_TIMEOUT);
+                pg0 = pg1, pg1 = pg2, pg2 = lookup(j + 3);
+            }
+        } else if (BOTH) {
             for (int j = 0; j < n_tiles && ok; ++j) {
                 ok = send(pg0, false, 0) && send(pg0, false, 128);
                 pg0 = pg1, pg1 = pg2, pg2 = lookup(j + 3);
@@ -418,7 +448,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     if (tc::mbar_try_wait(bar, parity)) break;
             };
             if (p.q_boxes && n_tiles > 0) drain(&s.q_full, 0);
-            for (int i = armed > SLOTS ? armed - SLOTS : 0; i < armed; ++i) drain(&s.full[i % SLOTS], (i / SLOTS) & 1);
+            constexpr int AHEAD = NARROW ? 3 : SLOTS;
+            for (int i = armed > AHEAD ? armed - AHEAD : 0; i < armed; ++i) drain(&s.full[i % AHEAD], (i / AHEAD) & 1);
+            if (last_armed > 0) drain(&s.full[Store::FULLS - 1], (last_armed - 1) & 1);
             if (gate_sent) drain(&s.gate_full, 0);
         }
     } else if (warp == 1) {
@@ -429,13 +461,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         if (n_tiles > 0) {
             const bool sender = tc::elect_one();
             constexpr uint32_t idesc_qk = tc::instr_desc_bf16(ROWS, KEYS);
-            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, Store::PART);
+            constexpr uint32_t idesc_pv = tc::instr_desc_bf16_b_mn(ROWS, NARROW ? 192 : Store::PART);
             // Operand descriptors by addition: the low word carries the address in 16-byte
             // units, the high word is the same for every tile.
             const uint64_t q_desc0 = tc::smem_desc_sw128(tc::smem_u32(s.q[0]));
             const uint32_t desc_hi = (uint32_t)(q_desc0 >> 32);
             const uint32_t q_lo = (uint32_t)q_desc0;
-            constexpr uint32_t HALF = KEYS * 128 >> 4, SLOT = SLOT_BYTES >> 4;
+            constexpr uint32_t HALF = KEYS * 128 >> 4, SLOT = KEYS * Store::PART * 2 >> 4;
             const uint32_t k_lo0 = (uint32_t)tc::smem_desc_sw128(tc::smem_u32(s.ring[0][0]));
             // the values, all features of a slot in one instruction: 64 of them lie together, the next 64 a
             // leading offset of HALF on
@@ -450,8 +482,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 const uint32_t d_s = tmem_s + to * 128;
 #pragma unroll
                 for (int part = 0; part < Store::PARTS; ++part) {
-                    const int st = item % SLOTS;
-                    if (!wait(&s.full[st], (item / SLOTS) & 1)) return false;
+                    const int st = NARROW ? (part < 3 ? 3 * (j % 3) + part : 9) : item % SLOTS;
+                    if (NARROW ? part == 0 && !wait(&s.full[j % 3], (j / 3) & 1) : !wait(&s.full[st], (item / SLOTS) & 1)) return false;
+                    if (NARROW && part == 3 && !wait(&s.full[3], j & 1)) return false;
                     tc::tc_fence_after_sync();
                     const uint32_t k_lo = k_lo0 + st * SLOT;
                     if (sender) {
@@ -467,6 +500,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 }
                 if (sender) {
                     tc::umma_commit(&s.s_full[to]);
+                    if (NARROW) tc::umma_commit(&s.empty[3]);
                     // pairs: K0 and K1; with two buffers V_(j-2) and K_j, with three K_(t+2) and V_t
                     if (!BOTH && (S_BUFS == 2 ? j > 0 : j == 1)) tc::umma_commit(&s.empty[(j - 1) % Store::RELEASES]);
                 }
@@ -479,9 +513,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 const uint32_t p_at = tmem_s + b * 128;
                 const uint32_t parity = (t / S_BUFS) & 1;
 #pragma unroll
-                for (int part = 0; part < Store::PARTS; ++part) {
+                for (int part = 0; part < (NARROW ? 1 : Store::PARTS); ++part) {
                     // 256: the tile's own slots, which the scores have taken (and freed by this)
-                    const int st = BOTH ? (2 * t + part) % SLOTS : item % SLOTS;
+                    const int st = NARROW ? 3 * (t % 3) : BOTH ? (2 * t + part) % SLOTS : item % SLOTS;
                     if (!BOTH && !wait(&s.full[st], (item / SLOTS) & 1)) return false;
                     const uint32_t v_lo = v_lo0 + st * SLOT;
 #pragma unroll
@@ -498,7 +532,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                             }
                         }
                     }
-                    if (BOTH && sender) tc::umma_commit(&s.empty[st]);
+                    if (BOTH && sender) tc::umma_commit(&s.empty[NARROW ? t % 3 : st]);
                     if (!BOTH) ++item;
                 }
                 if (sender) {
@@ -647,7 +681,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 if (!ok) break;
                 tc::tc_fence_after_sync();
 #pragma unroll 1
-                for (int c0 = 0; c0 < HD; c0 += 32) {
+                for (int c0 = 0; c0 < Store::VALUES; c0 += 32) {
                     uint32_t v[32];
                     tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, v);
                     tc::tmem_ld_wait();
@@ -731,7 +765,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // each of 32 rows touches 32 lines and takes the memory pipe 32 cycles (128 rows of 256 features
         // that way 5,200 cycles of a block, of 64 features with two groups 2,200).
         auto write_rows = [&]() {
-            constexpr int MINE = HD / GROUPS, ACROSS = MINE < 64 ? MINE / 8 : 8;      // pieces of a row side by side
+            constexpr int MINE = Store::VALUES / GROUPS, ACROSS = MINE % 64 ? 4 : 8;      // pieces of a row side by side
             __syncwarp();
             const unsigned long long mine = real ? (unsigned long long)dst : 0ull;
 #pragma unroll 4
@@ -753,7 +787,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         // Each group holds the sums over its own tiles against the reference of its last one.
         // A row's two states meet in shared memory; every thread comes to the barrier,
         // whatever happened to its waits.  Then group g writes its half of the features.
-        float2* const merge = reinterpret_cast<float2*>(s.ring[(gate_item + 2) % SLOTS][0]);     // (nothing is there any more)
+        float2* const merge = reinterpret_cast<float2*>(s.ring[NARROW ? 0 : (gate_item + 2) % SLOTS][0]);     // (nothing is there any more)
         merge[group * ROWS + r] = make_float2(my_tiles > 0 ? m_ref : -INFINITY, my_tiles > 0 ? l : 0.f);
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ok && n_tiles > 0 && !*abort_flag) {
@@ -774,7 +808,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             // could read none of a group's keys has weight 0 and finite sums (zeros) there.
             const bool mine_any = SHARED || my_tiles > 0, other_any = !SHARED && n_tiles > my_tiles;
 #pragma unroll 1
-            for (int c0 = group * (HD / 2); c0 < (group + 1) * (HD / 2); c0 += 32) {
+            for (int c0 = group * (Store::VALUES / 2); c0 < (group + 1) * (Store::VALUES / 2); c0 += 32) {
                 uint32_t a[32], b[32];
                 if (mine_any) tc::tmem_ld_32x32(tmem_mine + lane_bits + c0, a);
                 if (other_any) tc::tmem_ld_32x32(tmem_o + (uint32_t)(group ^ 1) * HD + lane_bits + c0, b);
@@ -799,19 +833,19 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     }
 }
 
-template <int HD, int GATE>
+template <int HD, int GATE, bool NARROW = false>
 int launch_gate(dim3 grid, cudaStream_t st, const CUtensorMap (&maps)[6], const TcAttnParams& p) {
-    constexpr int smem = (int)sizeof(Storage<HD>);
+    constexpr int smem = (int)sizeof(Storage<HD, NARROW>);
     static_assert(smem <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, GATE>,
+        cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<HD, GATE, NARROW>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    cb_launch(attention_tcgen05_kernel<HD, GATE>, grid, dim3(Storage<HD>::THREADS), smem, st, maps[0], maps[1], maps[2],
-              maps[3], maps[4], maps[5], p);
+    cb_launch(attention_tcgen05_kernel<HD, GATE, NARROW>, grid, dim3(Storage<HD, NARROW>::THREADS), smem, st, maps[0],
+              maps[1], maps[2], maps[3], maps[4], maps[5], p);
     return cb_last_error();
 }
 
@@ -831,7 +865,8 @@ int launch_as(int gate, dim3 grid, cudaStream_t st, const CUtensorMap (&maps)[6]
 // both are the same rows.
 // keep_first (with a window): a row at position p reads j <= p with p - j < window or j < keep_first.
 // chunked: `window` is a chunk's size (first_key).  sinks: [n_heads] or null.  Results times out_scale.
-// n_rows: of qkv (and out, gate).  lead: how many requests at the head bring a single token (as max_new_tokens is the others').
+// n_rows: of qkv (and out, gate).  value_cols (0: all): the caller reads no result's features beyond that many; they may
+// be left as they are.  lead: how many requests at the head bring a single token (as max_new_tokens is the others').
 // gate: null, or logits: results times their sigmoids; laid out like `out`, rows of 16-byte pieces, or with
 // gate_per_head [rows][n_heads].
 CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, int n_rows, void* out, int out_stride,
@@ -841,7 +876,7 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, int n_r
                                         int max_new_tokens, int n_heads, int n_kv_heads, int head_dim,
                                         int page_tokens, float scale, int window, int chunked, int keep_first,
                                         float out_scale, const float* sinks, const void* gate, int gate_stride,
-                                        int gate_per_head, int lead, int* status, void* stream) {
+                                        int gate_per_head, int lead, int value_cols, int* status, void* stream) {
     if (n_requests <= 0 || max_new_tokens <= 0) return 0;
     if (keep_first < 0 || !(scale > 0.f)) return CB_ERR_UNSUPPORTED;
     if ((head_dim != 64 && head_dim != 128 && !(head_dim == 256 && k_cache == v_cache)) || n_heads % n_kv_heads != 0 || page_tokens < 8 || page_tokens > KEYS ||
@@ -912,6 +947,8 @@ CB_EXPORT int cb_attention_tcgen05_kept(const void* qkv, int qkv_stride, int n_r
     const dim3 grid(n_kv_heads, portions, p.lead_ranks + q_tiles);
     const int form = gate == nullptr ? GATE_NONE : gate_per_head ? GATE_HEAD : GATE_RESULT;
     if (head_dim == 64) return launch_as<64>(form, grid, (cudaStream_t)stream, maps, p);
+    if (head_dim == 256 && value_cols > 0 && value_cols <= 192 && form == GATE_NONE)
+        return launch_gate<256, GATE_NONE, true>(grid, (cudaStream_t)stream, maps, p);
     if (head_dim == 256) return launch_as<256>(form, grid, (cudaStream_t)stream, maps, p);
     return launch_as<128>(form, grid, (cudaStream_t)stream, maps, p);
 }

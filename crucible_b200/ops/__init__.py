@@ -542,10 +542,11 @@ def paged_attention_plain(qkv, out, n_heads, n_kv_heads, head_dim, scale, window
 
 
 def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx, cache,
-                    binding) -> None:
+                    binding, value_cols=None) -> None:
+    """`value_cols`: the caller reads only so many features of every result (None: all)."""
     if qkv.dtype == torch.bfloat16:
         if tensor_core.paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window,
-                                       ctx, cache, binding):
+                                       ctx, cache, binding, value_cols):
             return
     paged_attention_plain(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx, cache,
                           binding)

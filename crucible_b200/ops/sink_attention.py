@@ -80,12 +80,13 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor,
               sinks: Optional[torch.Tensor], n_heads: int, n_kv_heads: int, key_dim: int,
               value_dim: int, scale: float, window: Optional[int], keep_first: int,
               out_scale: float, ctx, cache, binding, gate_per_head: bool = False,
-              chunked: bool = False) -> None:
+              chunked: bool = False, value_cols: Optional[int] = None) -> None:
     """`q`, `gate`, `out`: views of rows (unit stride along features).  Position p sees
     j <= p with p - j < window or j < keep_first; with `chunked` the window is the size of chunks
     counted from position 0 and p sees j <= p of its own chunk.  out = softmax-with-sink(q k) v, times
     sigmoid(gate) if given, times out_scale.  `gate`: rows laid out like `out` (a logit for
-    every feature), or [rows, n_heads] with `gate_per_head` (one logit a head)."""
+    every feature), or [rows, n_heads] with `gate_per_head` (one logit a head).  `value_cols`: the
+    caller reads only so many features of every result (None: all)."""
     _need_cuda(q, gate, out, sinks)
     for t in (q, gate, out):
         if t is not None and t.stride(1) != 1:
@@ -97,7 +98,7 @@ def attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor,
     if gate is not None and gate.dtype != q.dtype:
         raise KernelError("sink attention: the gate's logits are rows of the queries' dtype")
     if _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
-                     keep_first, out_scale, ctx, cache, k_cache, v_cache, table, gate_per_head, chunked):
+                     keep_first, out_scale, ctx, cache, k_cache, v_cache, table, gate_per_head, chunked, value_cols):
         return
     if attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                      chunked, keep_first if window else 0, out_scale, ctx, cache.page_tokens, table, gate_per_head):
@@ -117,7 +118,7 @@ TENSOR_CORES = True      # tests switch it off to reach the plain kernel with th
 
 def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                   keep_first, out_scale, ctx, cache, k_cache, v_cache, table, gate_per_head=False,
-                  chunked=False) -> bool:
+                  chunked=False, value_cols=None) -> bool:
     """For bfloat16 rows.  A step that holds a portion whose keys and values have one size that the
     tcgen05 attention takes goes there (`csrc/attention_tcgen05.cu`), the single decoded tokens at its
     head with it or in a launch of their own (`tensor_core.tiles_first`); everything else is the mma.sync
@@ -134,7 +135,8 @@ def _tensor_cores(q, gate, out, sinks, n_heads, n_kv_heads, key_dim, value_dim, 
     if key_dim == value_dim:
         first = tensor_core.prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, key_dim, scale, window,
                                              keep_first, ctx, cache, table, chunked=chunked, sinks=sinks,
-                                             out_scale=out_scale, gate=gate, gate_per_head=gate_per_head)
+                                             out_scale=out_scale, gate=gate, gate_per_head=gate_per_head,
+                                             value_cols=value_cols)
     if first == 0:
         return True
     if first < ctx.n_requests:

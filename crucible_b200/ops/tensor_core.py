@@ -653,13 +653,13 @@ def _tcgen05_rows(head_dim, k_cache, v_cache) -> bool:
 
 def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale,
                        window, cache, keep_first: int = 0, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                       gate=None, gate_per_head: bool = False, lead: int = 0) -> bool:
+                       gate=None, gate_per_head: bool = False, lead: int = 0, value_cols=None) -> bool:
     """tcgen05 attention for portions of prompts: head sizes of `_tcgen05_rows`, page size a
     power of two from 8 to 128.  `keep_first` (with a window): keys before that position stay
     visible.  `chunked`: the window is a chunk's size.  `sinks`: float32 per query head or None.
     `gate`: rows laid out like `out` (`gate_per_head`: one logit a head) whose sigmoids the results are
     multiplied by before they are rounded, or None.  `lead`: how many requests at the head of `reqs` bring a
-    single token.  Returns False for anything else."""
+    single token.  `value_cols`: the features of a result that are read (None: all).  Returns False for anything else."""
     pt = cache.page_tokens
     if pt < 8 or pt > 128 or pt & (pt - 1):
         return False
@@ -674,7 +674,7 @@ def _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, he
         scale, window or 0, 1 if chunked else 0, keep_first if window else 0,
         out_scale, sinks.data_ptr() if sinks is not None else 0,
         gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0,
-        1 if gate_per_head else 0, lead, status_word(qkv.device).data_ptr(), _stream())
+        1 if gate_per_head else 0, lead, value_cols or 0, status_word(qkv.device).data_ptr(), _stream())
     if code == _UNSUPPORTED:
         return False
     if code != 0:
@@ -865,7 +865,7 @@ def tiles_first(host, n_requests, head_dim, window, keep_first) -> int:
 
 def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, scale, window, keep_first,
                      ctx, cache, table, chunked: bool = False, sinks=None, out_scale: float = 1.0,
-                     gate=None, gate_per_head: bool = False) -> int:
+                     gate=None, gate_per_head: bool = False, value_cols=None) -> int:
     """The tcgen05 attention for the requests of a step from `tiles_first` on, over keys and values of
     one size (`_tcgen05_rows`), with a window that may keep the first tokens or (`chunked`) is the size of
     chunks, and with a sink per head in the softmax (`sinks`) or none; `gate`: a logit for every result or
@@ -885,7 +885,8 @@ def prompt_attention(q, out, k_cache, v_cache, n_heads, n_kv_heads, head_dim, sc
     reqs = _Requests(ctx, table, first, none - first, host.max_new_tokens, host.context_bucket, ctx.n_tokens)
     taken = _attention_tcgen05(q, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, cache,
                                keep_first=keep_first, chunked=chunked, sinks=sinks, out_scale=out_scale, gate=gate,
-                               gate_per_head=gate_per_head, lead=host.lead_single if first == 0 else 0)
+                               gate_per_head=gate_per_head, lead=host.lead_single if first == 0 else 0,
+                               value_cols=value_cols)
     return first if taken else none
 
 
@@ -893,7 +894,7 @@ SPLIT_ROWS = 16          # packed rows (new tokens x heads of a group) the split
 
 
 def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, scale, window, ctx,
-            cache) -> bool:
+            cache, value_cols=None) -> bool:
     """One run of requests through the kernel that suits it.  A function of the run's
     shape (count, most new tokens, bucket) and of the sizes only."""
     n_rep = n_heads // n_kv_heads
@@ -927,7 +928,7 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
     if (USE_TCGEN05_ATTENTION and not split and _tcgen05_rows(head_dim, k_cache, v_cache)
             and reqs.max_new * n_rep >= 64 and out.stride(0) % 8 == 0
             and _attention_tcgen05(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads,
-                                   head_dim, scale, window, cache)):
+                                   head_dim, scale, window, cache, value_cols=value_cols)):
         return True
     if split and head_dim <= 128 and chunk_keys % 256:
         # the mma.sync split form of rows up to 128 features walks whole tiles of 256 keys
@@ -953,7 +954,7 @@ def _attend(qkv, out, k_cache, v_cache, reqs, n_heads, n_kv_heads, head_dim, sca
 
 
 def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx, cache,
-                    binding) -> bool:
+                    binding, value_cols=None) -> bool:
     """Tensor-core attention over the paged cache.  Takes head sizes that are
     multiples of 16 up to 256 and any head counts, group sizes and page sizes;
     refuses anything else (the plain kernel then runs).
@@ -973,7 +974,7 @@ def paged_attention(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ctx,
     table = ctx.block_table(binding.group)
     host = ctx.host
     n_rep = n_heads // n_kv_heads
-    args = (n_heads, n_kv_heads, head_dim, scale, window, ctx, cache)
+    args = (n_heads, n_kv_heads, head_dim, scale, window, ctx, cache, value_cols)
     lead = host.lead_single
     if 0 < lead < ctx.n_requests and host.max_new_tokens * n_rep > SPLIT_ROWS:
         decoding = _Requests(ctx, table, 0, lead, 1, host.lead_context_bucket, lead, host.lead_context_reach)

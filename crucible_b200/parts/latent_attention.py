@@ -175,9 +175,10 @@ class LatentAttention(Mixer):
             # over the same ONE key head whose rows are keys and values at once
             from ..ops import sink_attention
             sink_attention.attention(qx, None, ox, self.sinks, H, 1, row, row, self.spec.softmax_scale,
-                                     self.spec.window, 0, 1.0, ctx, cache, binding)
+                                     self.spec.window, 0, 1.0, ctx, cache, binding, value_cols=C)
         else:
-            ops.paged_attention(qx, ox, H, 1, row, self.spec.softmax_scale, self.spec.window, ctx, cache, binding)
+            ops.paged_attention(qx, ox, H, 1, row, self.spec.softmax_scale, self.spec.window, ctx, cache, binding,
+                                value_cols=C)
         act = ctx.scratch("latent.act", (t, H * E), self.dtype)
         logit = gate_rows = None
         if self.w_gate is not None:

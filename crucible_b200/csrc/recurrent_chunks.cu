@@ -22,17 +22,19 @@
 // S as every chunk begins, and chunk_out_kernel adds the queries over it, again all chunks side by side.
 // Delta rules: chunk_walk_kernel; a block owns 16 (or 8) columns of a head's S and walks the chunks in
 // order: per chunk two products on fp32 FMA (rows of Q and W over S; k^T over u), the next chunk's
-// operands on their way by asynchronous copies.
+// operands on their way by TMA.
 //
-// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 233 us (under ncu, cold: the chunks'
-// numbers 80, the walk 165), channel delta 551 -> 280, mLSTM 590 -> 172, wkv 467 -> 169, state space 408 -> 168;
-// 8 heads: 502 -> 143, 551 -> 170, 589 -> 91, 467 -> 90, 407 -> 79.  16,384 tokens of 16 heads in slices (256 MB of
+// Measured at 2,048 tokens (token by token -> in chunks), 16 heads of 128: delta 503 -> 201 us (the chunks'
+// numbers 64, the walk 137), channel delta 551 -> 251, mLSTM 590 -> 172, wkv 467 -> 169, state space 408 -> 168;
+// 8 heads: 502 -> 126, 551 -> 152, 589 -> 91, 467 -> 90, 407 -> 79.  16,384 tokens of 16 heads in slices (256 MB of
 // workspaces): delta 1,768 us, 1,760 at once; mLSTM 1,340 and 1,292; state space 1,403 and 1,380.
 //
 // The result differs from the token-by-token walk by rounding, and with the way a prompt is cut: the
 // bfloat16 engine's prompts alone take this path; decoded tokens and the float32 engine keep the walk.
 #define CB_PDL_BIT 11      // this file's bit in CRUCIBLE_PDL (shared with recurrent.cu)
+#include <type_traits>
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace {
 
@@ -45,6 +47,10 @@ template <int RULE> constexpr bool OWN_Q = RULE != RULE_SSD && RULE != RULE_MLST
 constexpr int CT = 32;              // tokens of a chunk
 constexpr int THREADS = 256;
 constexpr int AP = CT + 4;          // pitch of the [CT][CT] matrices: rows of whole 16-byte pieces
+// Padding of chunk_local's rows of keys and queries.  The dots of scalar decays: eight lanes read 64 bytes of two
+// neighbouring rows, which lie 16 banks apart (with 4, as the others have it, 12 of 16 banks met twice).  Vector decays: a row a lane,
+// 16 bytes of eight rows on 32 banks.
+template <int RULE> constexpr int PAD = VECTOR_DECAY<RULE> ? 4 : 16;
 
 struct Args {
     const float* qkv;               // rows of C floats: q heads at q_off, k at k_off, v at v_off, decays at w_off
@@ -64,6 +70,8 @@ struct Args {
     // [chunks][H] of m (mLSTM)
     float *wq, *ww, *wk, *wu, *wg, *wl, *wn, *wm;
     float4* ws;
+    int rows, piece_rows;           // of qkv, and of the workspaces
+    int* status;                    // a wait that ran out is recorded here
 };
 
 // two fp32 numbers in one register pair, multiplied and added by one instruction
@@ -91,10 +99,6 @@ __device__ __forceinline__ ulonglong2 pairs_at(const float* p) { return *reinter
 
 __device__ __forceinline__ float* state_at(unsigned char* state, long slot_stride, int slot, long off) {
     return reinterpret_cast<float*>(state + (size_t)slot * slot_stride + off);
-}
-__device__ __forceinline__ void cp16(float* smem, const float* gmem) {
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gmem) : "memory");
 }
 // The slice's rows of a request: [row0, row1) of the step; their rows of a workspace are `shift` less.
 // (A request's first: the rows of the requests before it, or limit for each of those if that is less.)
@@ -215,8 +219,8 @@ template <int DP, int RULE>
 __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
-    constexpr int P = DP + 4;                       // pitch: 8 neighbouring rows' 16-byte reads hit 32 banks
     constexpr bool VECTOR = VECTOR_DECAY<RULE>, DELTA = IS_DELTA<RULE>;
+    constexpr int P = DP + PAD<RULE>;
     const int r = blockIdx.z, head = blockIdx.y;
     const Piece piece = piece_of(a, r);
     const int row0 = piece.row0 + blockIdx.x * CT, own0 = row0 - piece.shift;
@@ -237,15 +241,6 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
     const int D = a.D, E = a.E, H = a.H;
     const int g = head / (H / a.G);
 
-    for (int i = tid; i < CT * (DP / 4); i += THREADS) {
-        const int t = i / (DP / 4), d = (i - t * (DP / 4)) * 4;
-        const bool in = t < cnt && d < D;
-        const float* src = a.qkv + (size_t)(row0 + t) * a.C;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
-        *reinterpret_cast<float4*>(sk + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.k_off + (size_t)g * D + d) : zero;
-        *reinterpret_cast<float4*>(sq + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.q_off + (size_t)g * D + d) : zero;
-        if (VECTOR) *reinterpret_cast<float4*>(sw + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.w_off + (size_t)head * D + d) : one;
-    }
     if (warp == 0) {
         // the chunk's numbers, a token a lane; tokens beyond the portion's end change nothing
         const bool in = lane < cnt;
@@ -293,6 +288,17 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
                 else a.ws[own_at] = make_float4(G, to_end, 0.f, 0.f);
             }
         }
+    }
+    // (scalar decays: the first warp is at the numbers, a chain of its own, meanwhile)
+    if (VECTOR || warp > 0)
+    for (int i = VECTOR ? tid : tid - 32; i < CT * (DP / 4); i += VECTOR ? THREADS : THREADS - 32) {
+        const int t = i / (DP / 4), d = (i - t * (DP / 4)) * 4;
+        const bool in = t < cnt && d < D;
+        const float* src = a.qkv + (size_t)(row0 + t) * a.C;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+        *reinterpret_cast<float4*>(sk + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.k_off + (size_t)g * D + d) : zero;
+        *reinterpret_cast<float4*>(sq + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.q_off + (size_t)g * D + d) : zero;
+        if (VECTOR) *reinterpret_cast<float4*>(sw + t * P + d) = in ? *reinterpret_cast<const float4*>(src + a.w_off + (size_t)head * D + d) : one;
     }
     __syncthreads();
 
@@ -404,10 +410,11 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_local_kernel(const Args a) {
         __syncthreads();
     }
 
-    if (RULE == RULE_MLSTM && tid < cnt) {
-        float n = 0.f;
-        for (int s = 0; s <= tid; ++s) n += sA[tid * AP + s];
-        a.ws[(size_t)(own0 + tid) * H + head].w = n;
+    if (RULE == RULE_MLSTM) {
+        for (int t = warp; t < cnt; t += THREADS / 32) {
+            const float n = cb_warp_sum(lane <= t ? sA[t * AP + lane] : 0.f);
+            if (lane == 0) a.ws[(size_t)(own0 + t) * H + head].w = n;
+        }
     }
     const size_t first = (size_t)row0 * H + head, own = (size_t)own0 * H + head;      // the chunk's first row: results, workspaces
     // vector decays: keys decayed to the chunk's end, and the whole chunk's decay
@@ -718,11 +725,21 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
                 }
             }
         }
-        // the upper half's sums to the lower half's warps
-        __syncthreads();
-        if (upper) {
+        // The two halves' sums: each warp closes eight of its tokens, and leaves the other eight's shares to the
+        // other half's.  What they have within the chunk is asked for first: a load behind each
+        // store, which may be to the same place, took the memory's latency 16 times (a quarter of the kernel).
+        float4 l[8];
+        const int mine0 = upper * 8;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 8; ++i) {
+            const int t = t0 + mine0 + i;
+            l[i] = in && t < cnt ? *reinterpret_cast<const float4*>(a.out + ((size_t)(row0 + t) * H + head) * E + e)
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if ((i >= 8) != (upper != 0)) {
                 float x[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -731,27 +748,29 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
                 }
                 *reinterpret_cast<float4*>(&half[group][i][lane * 4]) = make_float4(x[0], x[1], x[2], x[3]);
             }
-        }
         __syncthreads();
-        if (upper) continue;
+        auto close = [&](auto first) {
+            constexpr int FIRST = decltype(first)::value;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float fw = __shfl_sync(0xffffffffu, within, i), fb = __shfl_sync(0xffffffffu, before, i);
-            float x[4];
+            for (int i = 0; i < 8; ++i) {
+                const float fw = __shfl_sync(0xffffffffu, within, FIRST + i), fb = __shfl_sync(0xffffffffu, before, FIRST + i);
+                float x[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float2 v = split_pair(acc[i / 2][k]);
-                x[k] = i % 2 ? v.y : v.x;
+                for (int k = 0; k < 4; ++k) {
+                    const float2 v = split_pair(acc[(FIRST + i) / 2][k]);
+                    x[k] = i % 2 ? v.y : v.x;
+                }
+                const float4 other = *reinterpret_cast<const float4*>(&half[group][FIRST + i][lane * 4]);
+                x[0] += other.x; x[1] += other.y; x[2] += other.z; x[3] += other.w;
+                const int t = t0 + FIRST + i;
+                if (in && t < cnt)
+                    *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + t) * H + head) * E + e) =
+                        make_float4(fmaf(fb, x[0], fw * l[i].x), fmaf(fb, x[1], fw * l[i].y),
+                                    fmaf(fb, x[2], fw * l[i].z), fmaf(fb, x[3], fw * l[i].w));
             }
-            const float4 other = *reinterpret_cast<const float4*>(&half[group][i][lane * 4]);
-            x[0] += other.x; x[1] += other.y; x[2] += other.z; x[3] += other.w;
-            if (in && t0 + i < cnt) {
-                float* to = a.out + ((size_t)(row0 + t0 + i) * H + head) * E + e;
-                const float4 l = *reinterpret_cast<const float4*>(to);
-                *reinterpret_cast<float4*>(to) = make_float4(fmaf(fb, x[0], fw * l.x), fmaf(fb, x[1], fw * l.y),
-                                                             fmaf(fb, x[2], fw * l.z), fmaf(fb, x[3], fw * l.w));
-            }
-        }
+        };
+        if (upper) close(std::integral_constant<int, 8>{});
+        else close(std::integral_constant<int, 0>{});
     }
 }
 
@@ -827,25 +846,32 @@ private:
     int share;
 };
 
+// The operands come by TMA, a box of 32 rows each, that a warp of its own asks for: as asynchronous copies of 16 bytes by
+// the threads that compute they were 1,000 to 1,600 of a chunk's 4,650 cycles; by two more warps the pipe that
+// serves shared memory was still theirs (237 -> 251 us), and a bulk copy a row costs that warp 60 cycles (401 us).
+struct WalkMaps { CUtensorMap q, w, k, u, s; };          // wq, ww, the keys, wu, ws
 template <int DP, int RULE, int ET>
-__global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
+__global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int CG = ET / 4, PS = DP + 32 / CG;
     constexpr bool VECTOR = VECTOR_DECAY<RULE>;
     // 16 columns: the queries' rows beside the state's sums, by the other half of the warps; 8: with W's rows before them
     constexpr bool BESIDE = ET == 16;
-    constexpr int STAGE = 3 * CT * DP + CT * ET;         // the queries' rows and W's over S, keys, u
+    // the queries' rows and W's over S, keys, u, the chunk's decays per channel, the tokens' numbers
+    constexpr int STAGE = 3 * CT * DP + CT * ET + DP + 4 * CT;
+    static_assert(STAGE % 32 == 0 && (2 * ET * PS + CT * ET) % 32 == 0, "boxes begin on 128-byte boundaries");
     // the second product: shares of the chunk's tokens, in lanes MS * CG apart; a thread has two pieces of four
     // channels, DP / 2 apart, and four columns; four warps
     constexpr int TS = 4096 / (DP * ET), MS = 32 / (TS * CG), TOKENS = CT / TS;
     static_assert(TS >= 2 && TS <= 8 && DP / 8 == 4 * MS, "four warps cover the state");
-    extern __shared__ __align__(16) float smem[];
-    float* states = smem;                                // [2][ET][PS]: as the chunk begins, and as it ends
+    // (no shared variable beside this one: it would come first, and a box's place is a 128-byte boundary)
+    extern __shared__ __align__(1024) float walk_smem[];
+    float* states = walk_smem;                           // [2][ET][PS]: as the chunk begins, and as it ends
     float* su = states + 2 * ET * PS;                    // [CT][ET]: u as it joins the state
-    float* sg = su + CT * ET;                            // [DP]: the chunk's decays per channel
-    float4* sc = reinterpret_cast<float4*>(sg + DP);     // [2][CT] the tokens' numbers
-    float* stage = reinterpret_cast<float*>(sc + 2 * CT);
+    float* stage = su + CT * ET;                         // [2][STAGE]
+    uint64_t* full = reinterpret_cast<uint64_t*>(stage + 2 * STAGE);      // [2]: a stage's copies have landed
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(full + 2);
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * ET;
     const int tid = threadIdx.x;
     const int D = a.D, E = a.E, H = a.H;
@@ -856,69 +882,83 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
     const int slot = a.req_state_slot[r];
     float* state = state_at(a.state, a.slot_stride, slot, a.s_off) + (size_t)head * D * E;
     auto place_of = [](int c) { return (c & 3) * CG + (c >> 2); };
-    for (int i = tid; i < DP * ET; i += THREADS) {
+    for (int i = tid; i < DP * ET; i += blockDim.x) {
         const int d = i / ET, c = i - d * ET;
         states[place_of(c) * PS + d] = d < D && col0 + c < E ? state[(size_t)d * E + col0 + c] : 0.f;
     }
-    for (int d = tid; d < DP; d += THREADS) sg[d] = 0.f;
-    for (int i = tid; i < 2 * STAGE; i += THREADS) stage[i] = 0.f;      // the rows' and columns' padding
+    for (int d = D + tid; d < DP; d += blockDim.x) {     // (the boxes bring zeros beyond the sizes; these decays are no box)
+        float* sg = stage + 3 * CT * DP + CT * ET;
+        sg[d] = sg[STAGE + d] = 0.f;
+    }
+    if (tid == 0) {
+        tc::mbar_init(&full[0], 1);
+        tc::mbar_init(&full[1], 1);
+        *abort_flag = 0;
+        tc::fence_barrier_init();
+    }
     __syncthreads();
 
-    // a thread copies the same 16-byte piece of every row that is its own
-    constexpr int PIECES = DP / 4, STEP = THREADS / PIECES;
-    const int ft = tid / PIECES, fd = (tid % PIECES) * 4;
-    auto fetch = [&](int base, int buf) {
-        float* rows = stage + buf * STAGE;
-        float* keys = rows + 2 * CT * DP;
-        float* u = keys + CT * DP;
-        const int cnt = min(CT, row1 - base);
-        if (fd < D) {
-#pragma unroll
-            for (int t = ft; t < CT; t += STEP) {
-                if (t < cnt) {
-                    const size_t at = ((size_t)(base - shift + t) * H + head) * D + fd;
-                    const float* src = a.qkv + (size_t)(base + t) * a.C + (size_t)g * D + fd;
-                    cp16(rows + t * DP + fd, a.wq + at);
-                    cp16(rows + (CT + t) * DP + fd, a.ww + at);
-                    cp16(keys + t * DP + fd, VECTOR ? a.wk + at : src + a.k_off);
-                } else {                                 // a portion's last chunk: rows of an earlier one are there
-                    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                    *reinterpret_cast<float4*>(rows + t * DP + fd) = zero;
-                    *reinterpret_cast<float4*>(rows + (CT + t) * DP + fd) = zero;
-                    *reinterpret_cast<float4*>(keys + t * DP + fd) = zero;
-                }
+    if (tid >= THREADS) {
+        // ---- the loader --------------------------------------------------------------------------------
+        const int lane = tid & 31;
+        auto landed = [&](int i) {                       // the copies of chunk i
+            bool got = false;
+            for (uint32_t n = 0; n < tc::WAIT_LIMIT && !got; ++n) got = tc::mbar_try_wait(&full[i & 1], (i >> 1) & 1);
+            return got;
+        };
+        auto fetch = [&](int base, int i) {
+            float* rows = stage + (i & 1) * STAGE;
+            float* keys = rows + 2 * CT * DP;
+            float* u = keys + CT * DP;
+            float* gs = u + CT * ET;
+            const int cnt = min(CT, row1 - base);
+            uint64_t* bar = &full[i & 1];
+            if (tc::elect_one()) {
+                tc::mbar_expect_tx(bar, 4 * (3 * CT * DP + CT * ET + (VECTOR ? D : 4 * CT)));
+                tc::tma_load_3d(rows + CT * DP, &maps.w, bar, 0, head, base - shift);
+                tc::tma_load_3d(u, &maps.u, bar, col0, head, base - shift);
+                tc::tma_load_3d(keys, &maps.k, bar, 0, VECTOR ? head : g, VECTOR ? base - shift : base);
+                tc::tma_load_3d(rows, &maps.q, bar, 0, head, base - shift);
+                if (!VECTOR) tc::tma_load_3d(gs + DP, &maps.s, bar, 0, head, base - shift);
+                else asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                  ::"r"(tc::smem_u32(gs)), "l"(a.wg + (chunk_place(base - shift, r) * H + head) * D), "r"(4 * D),
+                                  "r"(tc::smem_u32(bar)) : "memory");
             }
-        }
-        if (tid < CT * CG) {
-            const int t = tid / CG, c = (tid % CG) * 4;
-            if (t < cnt && col0 + c < E) {
-                cp16(u + t * ET + c, a.wu + ((size_t)(base - shift + t) * H + head) * E + col0 + c);
-            } else {
-                *reinterpret_cast<float4*>(u + t * ET + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();
+            if (cnt < CT) {
+                // a portion's last chunk: what lies behind its rows is another's, or nothing, and must not count
+                landed(i);
+                for (int x = cnt * DP + lane; x < CT * DP; x += 32) rows[x] = rows[CT * DP + x] = keys[x] = 0.f;
+                for (int x = cnt * ET + lane; x < CT * ET; x += 32) u[x] = 0.f;
+                if (!VECTOR && lane >= cnt) *reinterpret_cast<float4*>(gs + DP + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
+        };
+        fetch(row0, 0);
+        int sent = 1;
+        for (int base = row0; base < row1; base += CT) {
+            __syncthreads();                             // the chunk's first barrier: the other stage is free
+            if (base + CT < row1) fetch(base + CT, sent), ++sent;
         }
-        if (!VECTOR && tid >= THREADS - CT) {
-            const int t = tid - (THREADS - CT);
-            if (t < cnt) cp16(reinterpret_cast<float*>(sc + buf * CT + t),
-                              reinterpret_cast<const float*>(a.ws + (size_t)(base - shift + t) * H + head));
-            else sc[buf * CT + t] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+        if (*abort_flag)                                 // no copy is left in flight
+            for (int i = max(0, sent - 2); i < sent; ++i) landed(i);
+        __syncthreads();
+        return;
+    }
     RowsOverState<DP, ET, BESIDE ? CT : 2 * CT, THREADS> first(tid);
     RowsOverState<DP, ET, CT, THREADS / 2> queries(tid % (THREADS / 2));
     // the state's part: a share of the tokens, channels ud + DP / 2 i, columns 4 uc + c
     const int lane = tid & 31, uc = lane % CG, part = lane / (CG * MS);
     const int ud = (tid / 32 % 4 * MS + lane / CG % MS) * 4;
-    fetch(row0, 0);
     int buf = 0;
-    for (int base = row0; base < row1; base += CT, buf ^= 1) {
+    uint32_t phase = 0;
+    for (int base = row0; base < row1; base += CT, phase ^= buf, buf ^= 1) {
         const int cnt = min(CT, row1 - base);
         const float* rows = stage + buf * STAGE;
         const float* keys = rows + 2 * CT * DP;
         const float* u = keys + CT * DP;
+        const float* sg = u + CT * ET;
         const float* S = states + buf * ET * PS;
-        const float4* nums = sc + buf * CT;
+        const float4* nums = reinterpret_cast<const float4*>(sg + DP);
         // what a token has within the chunk, and with the state's share added
         auto out_at = [&](int t, int c) { return a.out + ((size_t)(base + t) * H + head) * E + col0 + c; };
         auto within = [&](bool has, int t, int c, float* to, int n) {
@@ -936,11 +976,10 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
         float local[4];
         const bool first_out = !BESIDE && first.row < cnt && col0 + first.col < E;
         if (!BESIDE) within(first_out, first.row, first.col, local, first.LEFT);
-        // the chunk's operands are there, the state is, and the other stage is free
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // the state is there, and the other stage is free; the chunk's operands are there
         __syncthreads();
-        if (base + CT < row1) fetch(base + CT, buf ^ 1);
-        if (VECTOR && tid < D) sg[tid] = a.wg[(chunk_place(base - shift, r) * H + head) * D + tid];
+        if (!tc::mbar_wait(&full[buf], phase, abort_flag) && !*abort_flag)
+            tc::give_up(abort_flag, a.status, tc::ST_EPILOGUE_TIMEOUT);      // (the rest is computed from what there is)
         {
             float sum[first.SUMS];
             first.take(rows + (BESIDE ? CT * DP : 0), S, sum);
@@ -957,7 +996,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const Args a) {
                 put(first.row, first.col, local, sum, first.LEFT);
             }
         }
-        __syncthreads();
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");      // (the loader is at its copies)
         if (tid >= THREADS / 2) {
             if (BESIDE) {
                 const bool has = queries.row < cnt && col0 + queries.col < E;
@@ -1027,19 +1066,28 @@ int allow_smem(K kernel, size_t smem, bool& configured) {
 
 template <int DP, int RULE, int ET>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
-    constexpr size_t bytes = sizeof(float) * (2 * ET * (DP + 128 / ET) + CT * ET + DP + 8 * CT + 2 * (3 * CT * DP + CT * ET));
-    static_assert(bytes <= 227 * 1024, "a block's shared memory");
+    constexpr size_t bytes = sizeof(float) * (2 * ET * (DP + 128 / ET) + CT * ET + 2 * (3 * CT * DP + CT * ET + DP + 4 * CT)) + 32;
+    static_assert(bytes <= 226 * 1024, "a block's shared memory");
     static bool configured = false;
     const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes, configured);
     if (rc) return rc;
+    WalkMaps maps;
+    const uint64_t width = (uint64_t)a.H * a.D;
+    if (!tc::make_map_heads_f32(&maps.q, a.wq, a.piece_rows, a.H, a.D, width, DP, CT) ||
+        !tc::make_map_heads_f32(&maps.w, a.ww, a.piece_rows, a.H, a.D, width, DP, CT) ||
+        !(VECTOR_DECAY<RULE> ? tc::make_map_heads_f32(&maps.k, a.wk, a.piece_rows, a.H, a.D, width, DP, CT)
+                             : tc::make_map_heads_f32(&maps.k, a.qkv + a.k_off, a.rows, a.G, a.D, a.C, DP, CT)) ||
+        !tc::make_map_heads_f32(&maps.u, a.wu, a.piece_rows, a.H, a.E, (uint64_t)a.H * a.E, ET, CT) ||
+        !tc::make_map_heads_f32(&maps.s, a.ws, a.piece_rows, a.H, 4, (uint64_t)a.H * 4, 4, CT))
+        return CB_ERR_UNSUPPORTED;
     const dim3 grid(n_requests, a.H, (a.E + ET - 1) / ET);
-    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS), bytes, s, a);
+    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS + 32), bytes, s, maps, a);
     return cb_last_error();
 }
 
 template <int DP, int RULE>
 int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
-    constexpr int P = DP + 4;
+    constexpr int P = DP + PAD<RULE>;
     // the shares of the dots, then the values (rules without a sum)
     constexpr int part = VECTOR_DECAY<RULE> ? (DP / 16) * (IS_DELTA<RULE> ? 2 : 1) * CT * CT : 0;
     constexpr int values = IS_DELTA<RULE> ? 0 : CT * P;
@@ -1083,7 +1131,8 @@ CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_o
                                       long n_off, long m_off, float* out, int n_requests, int max_new, int n_heads,
                                       int n_qk_heads, int key_dim, int value_dim, int w_off, const float* per_head,
                                       const float* kept, int limit, float* kept_room, float* wq, float* ww, float* wk, float* wu, float* ws,
-                                      float* wg, float* wl, float* wn, float* wm, void* stream) {
+                                      float* wg, float* wl, float* wn, float* wm, int rows, int piece_rows, int* status,
+                                      void* stream) {
     if (n_requests <= 0 || max_new <= 0) return 0;
     const bool vector = rule == RULE_WKV || rule == RULE_CHANNEL;
     if (n_heads % n_qk_heads != 0 || key_dim > 128 || n_requests > 65535 || n_heads > 65535
@@ -1102,6 +1151,8 @@ CB_EXPORT int cb_matrix_memory_chunks(int rule, const float* qkv, int C, int q_o
     a.wq = wq; a.ww = ww; a.wk = wk; a.wu = wu; a.wg = wg; a.wl = wl; a.wn = wn; a.wm = wm; a.ws = reinterpret_cast<float4*>(ws);
     cudaStream_t s = (cudaStream_t)stream;
     a.limit = limit;
+    a.rows = rows; a.piece_rows = piece_rows;
+    a.status = status;
     const size_t kept_size = (size_t)n_requests * n_heads * (key_dim + 1);
     for (int skip = 0, slice = 0; skip < max_new; skip += limit, ++slice) {
         a.skip = skip;

@@ -510,6 +510,35 @@ inline bool make_map_heads(CUtensorMap* out, const void* base, uint64_t rows, ui
     return true;
 }
 
+// The same of fp32 elements, [rows][heads][inner] with `ld` elements between rows, in boxes of `box_inner`
+// elements of one head of `box_rows` rows that lie unswizzled in shared memory, row after row.
+inline bool make_map_heads_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t heads, uint32_t inner,
+                               uint64_t ld, uint32_t box_inner, uint32_t box_rows) {
+    typedef std::tuple<const void*, uint64_t, uint64_t, uint32_t, uint64_t, uint32_t, uint32_t> Key;
+    static std::map<Key, CUtensorMap> cache;
+    static std::mutex mu;
+    Key key(base, rows, heads, inner, ld, box_inner, box_rows);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) {
+        *out = it->second;
+        return true;
+    }
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {inner, heads, rows};
+    cuuint64_t strides[2] = {(cuuint64_t)inner * 4, ld * 4};
+    cuuint32_t box[3] = {box_inner, 1, box_rows};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides,
+                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return false;
+    if (cache.size() > 8192) cache.clear();
+    cache[key] = *out;
+    return true;
+}
+
 // An output matrix [rows, cols] (bf16 or fp32) with `ld` elements between rows,
 // written in boxes of [box_rows, 128 bytes] with the 128-byte swizzle.
 inline bool make_out_map_2d(CUtensorMap* out, const void* base, bool f32, uint64_t rows,

@@ -49,7 +49,7 @@ MODULES: Dict[str, List[str]] = {
     "streams": ["common.cuh"],
     "sink_attention": ["common.cuh"],
     "recurrent": ["common.cuh"],
-    "recurrent_chunks": ["common.cuh"],
+    "recurrent_chunks": ["common.cuh", "tc_common.cuh"],
     "polynorm": ["common.cuh"],
     "hashed_embedding": ["common.cuh"],
     "activations": ["common.cuh"],

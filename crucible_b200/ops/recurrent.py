@@ -7,7 +7,7 @@ import functools
 
 import torch
 
-from . import LAUNCHES, KernelError, _check, _code, _need_cuda, _ptr, _stream, build
+from . import LAUNCHES, KernelError, _check, _code, _need_cuda, _ptr, _stream, build, tensor_core
 
 DELTA, MLSTM, WKV, SSD, CHANNEL = 0, 1, 2, 3, 4
 GATE_SILU, GATE_SIGMOID = 0, 1
@@ -255,7 +255,8 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
             longest, n_heads, n_qk_heads, key_dim, value_dim,
             w_off, _ptr(per_head),
             kept_at + 4 * walked * n_heads * (key_dim + 1) if kept is not None else 0,
-            limit, kept_room, wq, ww, wk, wu, ws, wg, wl, wn, wm, _stream())
+            limit, kept_room, wq, ww, wk, wu, ws, wg, wl, wn, wm,
+            qkv.shape[0], rows, tensor_core.status_word(qkv.device).data_ptr(), _stream())
         if code == build.UNSUPPORTED:            # the walk's
             walked = n
         else:

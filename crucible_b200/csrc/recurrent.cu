@@ -507,6 +507,34 @@ __global__ void retention_prepare_kernel(const T* __restrict__ proj, int proj_st
     }
 }
 
+// NC neighbouring columns of a row, 4, 8 or 16 bytes at once
+template <int NC>
+__device__ __forceinline__ void load_columns(float (&x)[NC], const float* at, bool in) {
+    if constexpr (NC == 4) {
+        const float4 v = in ? *reinterpret_cast<const float4*>(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else if constexpr (NC == 2) {
+        const float2 v = in ? *reinterpret_cast<const float2*>(at) : make_float2(0.f, 0.f);
+        x[0] = v.x; x[1] = v.y;
+    } else {
+        x[0] = in ? *at : 0.f;
+    }
+}
+template <int NC>
+__device__ __forceinline__ void store_columns(float* at, const float (&x)[NC]) {
+    if constexpr (NC == 4) *reinterpret_cast<float4*>(at) = make_float4(x[0], x[1], x[2], x[3]);
+    else if constexpr (NC == 2) *reinterpret_cast<float2*>(at) = make_float2(x[0], x[1]);
+    else *at = x[0];
+}
+// N numbers, each summed over LANES neighbouring lanes
+template <int LANES, int N>
+__device__ __forceinline__ void lanes_summed(float (&x)[N]) {
+#pragma unroll
+    for (int d = 1; d < LANES; d <<= 1)
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], d);
+}
+
 // ---- the recurrence ----------------------------------------------------------------------
 // qkv: fp32 [rows][C] with q heads at q_off, k heads at k_off (both n_qk_heads of D), v heads at
 // v_off (n_heads of E).  sc0, sc1: fp32 [rows][H]: (decay, beta) or (log keep, log in).
@@ -515,7 +543,7 @@ __global__ void retention_prepare_kernel(const T* __restrict__ proj, int proj_st
 // A block: COLS columns x LANES lanes; lane `part` of a column owns entries part * P .. part * P + P - 1
 // of it.  The staged k and q rows are padded by four floats per part, so that the parts'
 // 16-byte reads fall on different banks.
-template <int P, int LANES, int RULE>
+template <int P, int LANES, int NC, int RULE>
 __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     const float* __restrict__ qkv, int C, int q_off, int k_off, int v_off,
     const float* __restrict__ sc0, const float* __restrict__ sc1,
@@ -527,7 +555,7 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     // u [H][D], the state-space rule's skip [H]
     cb_pdl_trigger();
     cb_pdl_wait();
-    constexpr int COLS = THREADS / LANES;
+    constexpr int COLS = THREADS / LANES * NC;
     constexpr int PAD = P == 4 ? 8 : 4;       // the parts' 16-byte reads then fall on different banks
     constexpr int PITCH = LANES * (P + PAD);
     constexpr bool VECTOR = VECTOR_DECAY<RULE>;
@@ -537,7 +565,7 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS;
     const int g = head / (n_heads / n_qk_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int col = col0 + warp * (32 / LANES) + lane / LANES, part = lane % LANES;
+    const int mine = (warp * (32 / LANES) + lane / LANES) * NC, col = col0 + mine, part = lane % LANES;
     const bool live = col < E;
     const int row0 = req_row_start[r], row1 = req_row_start[r + 1];
     const int slot = req_state_slot[r];
@@ -547,12 +575,12 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     const float* kept_n = RULE == RULE_MLSTM ? kept + (size_t)r * (n_heads * D + n_heads) : nullptr;
     // the padding of the staged rows and the columns beyond E stay zero
     for (int i = threadIdx.x; i < 2 * BUF; i += blockDim.x) stage[i] = 0.f;
-    float s[P], n[P];
+    float s[P][NC], n[P];
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < P; ++i) {
         const int d = part * P + i;
-        s[i] = (live && d < D) ? S[(size_t)d * E + col] : 0.f;
+        load_columns<NC>(s[i], S + (size_t)d * E + col, live && d < D);
         n[i] = (RULE == RULE_MLSTM && d < D) ? kept_n[(size_t)head * D + d] : 0.f;
         if (RULE == RULE_WKV) n[i] = d < D ? per_head[(size_t)head * D + d] : 0.f;      // the bonus u
     }
@@ -591,10 +619,11 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 if (VECTOR) cp_async<4>(sw + at, src + w_off + (size_t)(head - g) * D);
             }
         }
-        for (int i = threadIdx.x; i < cnt * COLS; i += blockDim.x) {
-            const int tt = i / COLS, c = i - tt * COLS;
+        constexpr int VEC_V = NC > 1 ? 4 : 1;            // (several columns a lane: sizes in fours)
+        for (int i = threadIdx.x; i < cnt * (COLS / VEC_V); i += blockDim.x) {
+            const int tt = i / (COLS / VEC_V), c = (i - tt * (COLS / VEC_V)) * VEC_V;
             if (col0 + c < E)
-                cp_async<4>(sv + i, qkv + (size_t)(base + tt) * C + v_off + (size_t)head * E + col0 + c);
+                cp_async<4 * VEC_V>(sv + tt * COLS + c, qkv + (size_t)(base + tt) * C + v_off + (size_t)head * E + col0 + c);
         }
         if (RULE != RULE_WKV && threadIdx.x < cnt) {
             if (RULE != RULE_CHANNEL)
@@ -605,12 +634,23 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     };
     if (row0 < row1) fetch(row0, 0);
     // delta rule: the pending write of the token before; mLSTM: the sums of the token before
-    float k_prev[P], g_prev = 1.f, u_prev = 0.f;
+    float k_prev[P], g_prev = 1.f, u_prev[NC];
 #pragma unroll
     for (int i = 0; i < P; ++i) k_prev[i] = 0.f;
-    float p_o = 0.f, p_n = 0.f, p_m = 0.f;
+    float p_o[NC], p_v[NC], p_n = 0.f, p_m = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) u_prev[c] = p_o[c] = p_v[c] = 0.f;
     size_t p_at = 0;
     bool pending = false;
+    auto close_mlstm = [&]() {                // the token before: its sums, divided and stored
+        float one[1] = {p_n};
+        lanes_summed<LANES>(p_o);
+        lanes_summed<LANES>(one);
+        const float low = fmaxf(fabsf(one[0]), expf(-p_m)) + 1e-6f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) p_o[c] /= low;
+        if (live && part == 0) store_columns<NC>(out + p_at, p_o);
+    };
     int buf = 0;
     for (int base = row0; base < row1; base += CHUNK, buf ^= 1) {
         const int cnt = min(CHUNK, row1 - base);
@@ -638,7 +678,8 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 kk[4 * j] = a.x; kk[4 * j + 1] = a.y; kk[4 * j + 2] = a.z; kk[4 * j + 3] = a.w;
                 qq[4 * j] = b.x; qq[4 * j + 1] = b.y; qq[4 * j + 2] = b.z; qq[4 * j + 3] = b.w;
             }
-            const float v = sv[tt * COLS + (col - col0)];
+            float v[NC];
+            load_columns<NC>(v, sv + tt * COLS + mine, true);
             const size_t out_at = (size_t)(base + tt) * n_heads * E + (size_t)head * E + col;
             if (RULE == RULE_DELTA) {
                 // One pass per token.  The write of the token before (S <- g S + k u^T) is still
@@ -646,36 +687,42 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 // result.  With r = S^T k and w = S^T q over S as that write leaves it:
                 //   u = beta (v - g r),   o = g w + u (k . q)       [= (g S + k u^T)^T q]
                 const float decay = s0[tt], beta = s1[tt];
-                float rk[4] = {0.f, 0.f, 0.f, 0.f}, rq[4] = {0.f, 0.f, 0.f, 0.f}, kq[4] = {0.f, 0.f, 0.f, 0.f};
+                float rk[NC][4] = {}, rq[NC][4] = {}, kq[4] = {};
 #pragma unroll
                 for (int i = 0; i < P; ++i) {
-                    s[i] = fmaf(k_prev[i], u_prev, g_prev * s[i]);
-                    rk[i & 3] = fmaf(s[i], kk[i], rk[i & 3]);
-                    rq[i & 3] = fmaf(s[i], qq[i], rq[i & 3]);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        s[i][c] = fmaf(k_prev[i], u_prev[c], g_prev * s[i][c]);
+                        rk[c][i & 3] = fmaf(s[i][c], kk[i], rk[c][i & 3]);
+                        rq[c][i & 3] = fmaf(s[i][c], qq[i], rq[c][i & 3]);
+                    }
                     kq[i & 3] = fmaf(kk[i], qq[i], kq[i & 3]);
                 }
-                float r = (rk[0] + rk[1]) + (rk[2] + rk[3]);
-                float w = (rq[0] + rq[1]) + (rq[2] + rq[3]);
-                float c = (kq[0] + kq[1]) + (kq[2] + kq[3]);
+                float sums[2 * NC + 1];
 #pragma unroll
-                for (int x = 1; x < LANES; x <<= 1) {
-                    r += __shfl_xor_sync(0xffffffffu, r, x);
-                    w += __shfl_xor_sync(0xffffffffu, w, x);
-                    c += __shfl_xor_sync(0xffffffffu, c, x);
+                for (int c = 0; c < NC; ++c) {
+                    sums[2 * c] = (rk[c][0] + rk[c][1]) + (rk[c][2] + rk[c][3]);
+                    sums[2 * c + 1] = (rq[c][0] + rq[c][1]) + (rq[c][2] + rq[c][3]);
                 }
-                const float u = beta * (v - decay * r);
-                if (live && part == 0) out[out_at] = fmaf(u, c, decay * w);
+                sums[2 * NC] = (kq[0] + kq[1]) + (kq[2] + kq[3]);
+                lanes_summed<LANES>(sums);
+                float o[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    u_prev[c] = beta * (v[c] - decay * sums[2 * c]);
+                    o[c] = fmaf(u_prev[c], sums[2 * NC], decay * sums[2 * c + 1]);
+                }
+                if (live && part == 0) store_columns<NC>(out + out_at, o);
 #pragma unroll
                 for (int i = 0; i < P; ++i) k_prev[i] = kk[i];
                 g_prev = decay;
-                u_prev = u;
             } else if (RULE == RULE_CHANNEL) {
                 // As the delta rule: the write of the token before is applied on the way, then this
                 // token's decays; with r = S^T k and w = S^T q over what that leaves:
                 //   u = beta (v - r),   o = w + u (k . q)       [= (S + k u^T)^T q]
                 const float beta = s1[tt];
                 const float4* w4 = reinterpret_cast<const float4*>(sw + tt * PITCH + part * (P + PAD));
-                float rk[4] = {0.f, 0.f, 0.f, 0.f}, rq[4] = {0.f, 0.f, 0.f, 0.f}, kq[4] = {0.f, 0.f, 0.f, 0.f};
+                float rk[NC][4] = {}, rq[NC][4] = {}, kq[4] = {};
 #pragma unroll
                 for (int j = 0; j < P / 4; ++j) {
                     const float4 a = w4[j];
@@ -683,30 +730,36 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int i = 4 * j + e;
-                        s[i] = __fmul_rn(ww[e], fmaf(k_prev[i], u_prev, s[i]));
-                        rk[e] = fmaf(s[i], kk[i], rk[e]);
-                        rq[e] = fmaf(s[i], qq[i], rq[e]);
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            s[i][c] = __fmul_rn(ww[e], fmaf(k_prev[i], u_prev[c], s[i][c]));
+                            rk[c][e] = fmaf(s[i][c], kk[i], rk[c][e]);
+                            rq[c][e] = fmaf(s[i][c], qq[i], rq[c][e]);
+                        }
                         kq[e] = fmaf(kk[i], qq[i], kq[e]);
                     }
                 }
-                float r = (rk[0] + rk[1]) + (rk[2] + rk[3]);
-                float w = (rq[0] + rq[1]) + (rq[2] + rq[3]);
-                float c = (kq[0] + kq[1]) + (kq[2] + kq[3]);
+                float sums[2 * NC + 1];
 #pragma unroll
-                for (int x = 1; x < LANES; x <<= 1) {
-                    r += __shfl_xor_sync(0xffffffffu, r, x);
-                    w += __shfl_xor_sync(0xffffffffu, w, x);
-                    c += __shfl_xor_sync(0xffffffffu, c, x);
+                for (int c = 0; c < NC; ++c) {
+                    sums[2 * c] = (rk[c][0] + rk[c][1]) + (rk[c][2] + rk[c][3]);
+                    sums[2 * c + 1] = (rq[c][0] + rq[c][1]) + (rq[c][2] + rq[c][3]);
                 }
-                const float u = beta * (v - r);
-                if (live && part == 0) out[out_at] = fmaf(u, c, w);
+                sums[2 * NC] = (kq[0] + kq[1]) + (kq[2] + kq[3]);
+                lanes_summed<LANES>(sums);
+                float o[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    u_prev[c] = beta * (v[c] - sums[2 * c]);
+                    o[c] = fmaf(u_prev[c], sums[2 * NC], sums[2 * c + 1]);
+                }
+                if (live && part == 0) store_columns<NC>(out + out_at, o);
 #pragma unroll
                 for (int i = 0; i < P; ++i) k_prev[i] = kk[i];
-                u_prev = u;
             } else if (RULE == RULE_WKV || RULE == RULE_SSD) {
                 // As below: the update needs no sum over a column; a token's sum is reduced and
                 // stored under the next token's pass.
-                float oc[4] = {0.f, 0.f, 0.f, 0.f};
+                float oc[NC][4] = {};
                 if (RULE == RULE_WKV) {
                     const float4* w4 = reinterpret_cast<const float4*>(sw + tt * PITCH + part * (P + PAD));
                     float ww[P];
@@ -716,26 +769,37 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                         ww[4 * j] = a.x; ww[4 * j + 1] = a.y; ww[4 * j + 2] = a.z; ww[4 * j + 3] = a.w;
                     }
 #pragma unroll
-                    for (int i = 0; i < P; ++i) {
-                        const float kv = __fmul_rn(kk[i], v);
-                        oc[i & 3] = fmaf(fmaf(n[i], kv, s[i]), qq[i], oc[i & 3]);
-                        s[i] = fmaf(ww[i], s[i], kv);
-                    }
-                } else {
-                    const float a = s0[tt], dv = __fmul_rn(s1[tt], v);
+                    for (int i = 0; i < P; ++i)
 #pragma unroll
-                    for (int i = 0; i < P; ++i) {
-                        s[i] = fmaf(kk[i], dv, __fmul_rn(a, s[i]));
-                        oc[i & 3] = fmaf(s[i], qq[i], oc[i & 3]);
-                    }
+                        for (int c = 0; c < NC; ++c) {
+                            const float kv = __fmul_rn(kk[i], v[c]);
+                            oc[c][i & 3] = fmaf(fmaf(n[i], kv, s[i][c]), qq[i], oc[c][i & 3]);
+                            s[i][c] = fmaf(ww[i], s[i][c], kv);
+                        }
+                } else {
+                    const float a = s0[tt], step = s1[tt];
+                    float dv[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) dv[c] = __fmul_rn(step, v[c]);
+#pragma unroll
+                    for (int i = 0; i < P; ++i)
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            s[i][c] = fmaf(kk[i], dv[c], __fmul_rn(a, s[i][c]));
+                            oc[c][i & 3] = fmaf(s[i][c], qq[i], oc[c][i & 3]);
+                        }
                 }
                 if (pending) {
+                    lanes_summed<LANES>(p_o);
 #pragma unroll
-                    for (int x = 1; x < LANES; x <<= 1) p_o += __shfl_xor_sync(0xffffffffu, p_o, x);
-                    if (live && part == 0) out[p_at] = __fadd_rn(p_o, p_n);
+                    for (int c = 0; c < NC; ++c) p_o[c] = __fadd_rn(p_o[c], p_v[c]);
+                    if (live && part == 0) store_columns<NC>(out + p_at, p_o);
                 }
-                p_o = (oc[0] + oc[1]) + (oc[2] + oc[3]);
-                p_n = __fmul_rn(skip, v);      // never fused with the sum: every token rounds alike
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    p_o[c] = (oc[c][0] + oc[c][1]) + (oc[c][2] + oc[c][3]);
+                    p_v[c] = __fmul_rn(skip, v[c]);      // never fused with the sum: every token rounds alike
+                }
                 p_at = out_at;
                 pending = true;
             } else {
@@ -746,24 +810,22 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 const float m_new = fmaxf(f + m, in);
                 const float a = expf(f + m - m_new), b = expf(in - m_new);
                 m = m_new;
-                const float bv = b * v;
-                float oc[4] = {0.f, 0.f, 0.f, 0.f}, nc[4] = {0.f, 0.f, 0.f, 0.f};
+                float oc[NC][4] = {}, nc[4] = {}, bv[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) bv[c] = b * v[c];
 #pragma unroll
                 for (int i = 0; i < P; ++i) {
-                    s[i] = fmaf(kk[i], bv, a * s[i]);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        s[i][c] = fmaf(kk[i], bv[c], a * s[i][c]);
+                        oc[c][i & 3] = fmaf(s[i][c], qq[i], oc[c][i & 3]);
+                    }
                     n[i] = fmaf(b, kk[i], a * n[i]);
-                    oc[i & 3] = fmaf(s[i], qq[i], oc[i & 3]);
                     nc[i & 3] = fmaf(n[i], qq[i], nc[i & 3]);
                 }
-                if (pending) {
+                if (pending) close_mlstm();
 #pragma unroll
-                    for (int x = 1; x < LANES; x <<= 1) {
-                        p_o += __shfl_xor_sync(0xffffffffu, p_o, x);
-                        p_n += __shfl_xor_sync(0xffffffffu, p_n, x);
-                    }
-                    if (live && part == 0) out[p_at] = p_o / (fmaxf(fabsf(p_n), expf(-p_m)) + 1e-6f);
-                }
-                p_o = (oc[0] + oc[1]) + (oc[2] + oc[3]);
+                for (int c = 0; c < NC; ++c) p_o[c] = (oc[c][0] + oc[c][1]) + (oc[c][2] + oc[c][3]);
                 p_n = (nc[0] + nc[1]) + (nc[2] + nc[3]);
                 p_m = m;
                 p_at = out_at;
@@ -774,26 +836,26 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     }
     if (RULE == RULE_DELTA) {
 #pragma unroll
-        for (int i = 0; i < P; ++i) s[i] = fmaf(k_prev[i], u_prev, g_prev * s[i]);      // the last token's write
+        for (int i = 0; i < P; ++i)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[i][c] = fmaf(k_prev[i], u_prev[c], g_prev * s[i][c]);      // the last token's write
     } else if (RULE == RULE_CHANNEL) {
 #pragma unroll
-        for (int i = 0; i < P; ++i) s[i] = fmaf(k_prev[i], u_prev, s[i]);
+        for (int i = 0; i < P; ++i)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[i][c] = fmaf(k_prev[i], u_prev[c], s[i][c]);
     } else if ((RULE == RULE_WKV || RULE == RULE_SSD) && pending) {
+        lanes_summed<LANES>(p_o);
 #pragma unroll
-        for (int x = 1; x < LANES; x <<= 1) p_o += __shfl_xor_sync(0xffffffffu, p_o, x);
-        if (live && part == 0) out[p_at] = __fadd_rn(p_o, p_n);
+        for (int c = 0; c < NC; ++c) p_o[c] = __fadd_rn(p_o[c], p_v[c]);
+        if (live && part == 0) store_columns<NC>(out + p_at, p_o);
     } else if (pending) {
-#pragma unroll
-        for (int x = 1; x < LANES; x <<= 1) {
-            p_o += __shfl_xor_sync(0xffffffffu, p_o, x);
-            p_n += __shfl_xor_sync(0xffffffffu, p_n, x);
-        }
-        if (live && part == 0) out[p_at] = p_o / (fmaxf(fabsf(p_n), expf(-p_m)) + 1e-6f);
+        close_mlstm();
     }
 #pragma unroll
     for (int i = 0; i < P; ++i) {
         const int d = part * P + i;
-        if (live && d < D) S[(size_t)d * E + col] = s[i];
+        if (live && d < D) store_columns<NC>(S + (size_t)d * E + col, s[i]);
         if (RULE == RULE_MLSTM && blockIdx.z == 0 && col == 0 && d < D) N[d] = n[i];
     }
     if (RULE == RULE_MLSTM && blockIdx.z == 0 && threadIdx.x == 0) *M = m;
@@ -1183,25 +1245,25 @@ __global__ void __launch_bounds__(256) gate_group_norm_quad_kernel(
     }
 }
 
-template <int P, int LANES, int RULE>
+template <int P, int LANES, int NC, int RULE>
 int launch_memory_as(const float* qkv, int C, int q_off, int k_off, int v_off, const float* sc0,
                      const float* sc1, const int* req_row_start, const int* req_state_slot,
                      unsigned char* state, long slot_stride, long s_off, long n_off, long m_off, float* out,
                      int n_requests, int n_heads, int n_qk_heads, int D, int E, int w_off,
                      const float* per_head, const float* kept, cudaStream_t s) {
-    constexpr int COLS = THREADS / LANES, PAD = P == 4 ? 8 : 4, NVEC = VECTOR_DECAY<RULE> ? 3 : 2;
+    constexpr int COLS = THREADS / LANES * NC, PAD = P == 4 ? 8 : 4, NVEC = VECTOR_DECAY<RULE> ? 3 : 2;
     const dim3 grid(n_requests, n_heads, (E + COLS - 1) / COLS), block(THREADS);
     const size_t smem = 2 * (size_t)(CHUNK * (NVEC * LANES * (P + PAD) + COLS) + 2 * CHUNK) * sizeof(float);
     if (smem > 48 * 1024) {
         static bool configured = false;
         if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(matrix_memory_kernel<P, LANES, RULE>,
+            cudaError_t e = cudaFuncSetAttribute(matrix_memory_kernel<P, LANES, NC, RULE>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return (int)e;
             configured = true;
         }
     }
-    cb_launch(matrix_memory_kernel<P, LANES, RULE>, grid, block, smem, s, qkv, C, q_off, k_off, v_off, sc0,
+    cb_launch(matrix_memory_kernel<P, LANES, NC, RULE>, grid, block, smem, s, qkv, C, q_off, k_off, v_off, sc0,
               sc1, req_row_start, req_state_slot, state, slot_stride, s_off, n_off, m_off, out, n_heads,
               n_qk_heads, D, E, w_off, per_head, kept);
     return cb_last_error();
@@ -1216,16 +1278,28 @@ int launch_memory(const float* qkv, int C, int q_off, int k_off, int v_off, cons
                   const float* sc1, const int* req_row_start, const int* req_state_slot,
                   unsigned char* state, long slot_stride, long s_off, long n_off, long m_off, float* out,
                   int n_requests, int n_heads, int n_qk_heads, int D, int E, int w_off,
-                  const float* per_head, const float* kept, cudaStream_t s) {
-#define CB_MEM(PP, LL)                                                                              \
-    return launch_memory_as<PP, LL, RULE>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start,     \
+                  const float* per_head, const float* kept, int columns, cudaStream_t s) {
+#define CB_MEM(PP, LL, NN)                                                                          \
+    return launch_memory_as<PP, LL, NN, RULE>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start,     \
                                           req_state_slot, state, slot_stride, s_off, n_off, m_off,  \
                                           out, n_requests, n_heads, n_qk_heads, D, E, w_off,        \
                                           per_head, kept, s)
-    if (D <= 32) CB_MEM(4, 8);
-    if (D <= 64) CB_MEM(8, 8);
-    if (D <= 128) CB_MEM(16, 8);
-    if (D <= 256) CB_MEM(32, 8);
+    // several columns a lane: 16-byte pieces of v, of the state's rows and of the results
+    if (((C | v_off | E) & 3) != 0 || ((s_off | slot_stride) & 15) != 0 ||
+        (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)out) & 15) != 0)
+        columns = 1;
+    if (D <= 32) CB_MEM(4, 8, 1);
+    if (D <= 64) {
+        if (columns == 4) CB_MEM(8, 8, 4);
+        if (columns == 2) CB_MEM(8, 8, 2);
+        CB_MEM(8, 8, 1);
+    }
+    if (D <= 128) {
+        if (columns == 4) CB_MEM(16, 8, 4);
+        if (columns == 2) CB_MEM(16, 8, 2);
+        CB_MEM(16, 8, 1);
+    }
+    if (D <= 256) CB_MEM(32, 8, 1);
 #undef CB_MEM
     return CB_ERR_UNSUPPORTED;
 }
@@ -1406,12 +1480,14 @@ CB_EXPORT int cb_retention_prepare(const void* proj, int proj_stride, int dtype,
 // rule 2: wkv (decay vectors at w_off in the rows, per_head the bonus [H][D]);
 // rule 3: state space (sc0 decay, sc1 step size, per_head the skip [H]);
 // rule 4: channel delta (decay vectors at w_off, one of D per head; sc1 beta).
+// columns: of S that a lane takes, 1, 2 or 4 (key sizes up to 32 and beyond 128, and rows off 16-byte boundaries:
+// 1); the same bits whatever it is.
 CB_EXPORT int cb_matrix_memory(int rule, const float* qkv, int C, int q_off, int k_off, int v_off,
                                const float* sc0, const float* sc1, const int* req_row_start,
                                const int* req_state_slot, void* state, long slot_stride, long s_off,
                                long n_off, long m_off, float* out, int n_requests, int n_heads,
                                int n_qk_heads, int key_dim, int value_dim, int w_off,
-                               const float* per_head, const float* kept, void* stream) {
+                               const float* per_head, const float* kept, int columns, void* stream) {
     if (n_requests <= 0) return 0;
     if (n_heads % n_qk_heads != 0) return CB_ERR_UNSUPPORTED;
     if ((rule == RULE_WKV || rule == RULE_SSD) && per_head == nullptr) return CB_ERR_UNSUPPORTED;
@@ -1422,7 +1498,7 @@ CB_EXPORT int cb_matrix_memory(int rule, const float* qkv, int C, int q_off, int
         return launch_memory<RR>(qkv, C, q_off, k_off, v_off, sc0, sc1, req_row_start,               \
                                  req_state_slot, (unsigned char*)state, slot_stride, s_off, n_off,   \
                                  m_off, out, n_requests, n_heads, n_qk_heads, key_dim, value_dim,    \
-                                 w_off, per_head, kept, s)
+                                 w_off, per_head, kept, columns, s)
     CB_RULE(RULE_DELTA);
     CB_RULE(RULE_MLSTM);
     CB_RULE(RULE_WKV);

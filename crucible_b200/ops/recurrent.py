@@ -15,13 +15,34 @@ CHUNKS = True                # tests switch it off to reach the token-by-token w
 STEP = True                  # likewise, for the form of a token each
 
 
-# us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128, a portion and head) and of
-# the chunks (their launches, a token of the longest portion, a chunk and head of 128), fitted to both forms over 4 to 32
-# heads of 64 and 128 and 1 to 24 uneven portions of up to 40 to 500 tokens; the delta rules' chunks are walked in
-# order, the others' are not
-_DELTA_COSTS = ((1.8, 0.172, 0.0052, 0.0525), (13.3, 0.024, 0.217))
-COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS, MLSTM: ((1.8, 0.216, 0.0057, 0.0597), (23.1, 0.0, 0.137)),
-         WKV: ((2.0, 0.142, 0.0049, 0.0501), (20.5, 0.0, 0.129)), SSD: ((2.6, 0.140, 0.0037, 0.040), (20.7, 0.0, 0.1275))}
+# us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128, a portion and head) with
+# 1, 2 and 4 columns of a matrix a lane, and of the chunks (their launches, a chunk and head of 128), fitted to
+# all of them over 4 to 32 heads of 64 and 128 and 1 to 48 uneven portions of up to 4 to 490 tokens
+_DELTA_COSTS = ({1: (3.43, 0.183, 0.0060, 0.0553), 2: (3.49, 0.227, 0.0037, 0.0460), 4: (4.55, 0.337, 0.0032, 0.0383)},
+                (15.7, 0.2576))
+COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS,
+         MLSTM: ({1: (3.49, 0.192, 0.0072, 0.0613), 2: (4.35, 0.240, 0.0046, 0.0430), 4: (5.75, 0.350, 0.0036, 0.0361)},
+                 (25.8, 0.162)),
+         WKV: ({1: (3.28, 0.148, 0.0068, 0.0647), 2: (3.55, 0.172, 0.0037, 0.0515), 4: (3.50, 0.296, 0.0035, 0.0419)},
+               (19.7, 0.1485)),
+         SSD: ({1: (3.60, 0.127, 0.0038, 0.0635), 2: (4.41, 0.142, 0.0026, 0.0446), 4: (5.84, 0.181, 0.0027, 0.0341)},
+               (21.7, 0.1307))}
+
+
+@functools.lru_cache(maxsize=4096)
+def walk_columns(rule, requests: int, rows: int, longest: int, n_heads: int, key_dim: int, value_dim: int):
+    """How many columns of its matrix a lane of the walk takes, and the walk's us.  Every lane of a column's eight reads
+    the token's k and q out of shared memory, which is what many portions wait for: with 2 or 4 columns a
+    lane half or a quarter of it, and the state's rows come in 8 or 16 bytes; but fewer blocks, and a token of a
+    lone portion takes longer.  32 portions of up to 24 tokens, 16 heads of 128, with 1, 2 and 4: delta rule 78, 61
+    and 57 us, state space 67, 50 and 48; one of 90 27, 28 and 41, 21, 23 and 33.  Up to a block an SM one is
+    taken, else what costs least: of 347 steps measured 1.4 % from the quickest on average."""
+    heads = n_heads * key_dim / 128
+    cost = {c: start + token * longest + (work * rows + portion * requests) * heads
+            for c, (start, token, work, portion) in COSTS[rule][0].items()}
+    if requests * n_heads * -(-value_dim // 16) <= 148:
+        return 1, cost[1]
+    return min((us, c) for c, us in cost.items())[::-1]
 
 
 def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bool:
@@ -43,9 +64,10 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
             return False
     elif longest < 160 and (longest < 48 or rows < 24 * requests or rows * heads < 4096):
         return False
-    (start, token, work, portion), (first, step, chunk) = COSTS[rule]
-    walk = start + token * longest + (work * rows + portion * requests) * heads
-    return walk > 0.95 * (first + step * longest + chunk * (rows / 32 + requests / 2) * heads)
+    first, chunk = COSTS[rule][1]
+    walk = min(start + token * longest + (work * rows + portion * requests) * heads
+               for start, token, work, portion in COSTS[rule][0].values())
+    return walk > 0.95 * (first + chunk * (rows / 32 + requests / 2) * heads)
 
 
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces
@@ -274,7 +296,11 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
             n_heads, n_qk_heads, key_dim, value_dim, w_off,
             _ptr(per_head), kept_at, _stream())
     code = lib.cb_matrix_memory_step(*args) if step else build.UNSUPPORTED
-    _check(lib.cb_matrix_memory(*args) if code == build.UNSUPPORTED else code, "matrix_memory")
+    if code == build.UNSUPPORTED:
+        longest = 1 if host is None or walked < n else host.max_new_tokens
+        columns = walk_columns(rule, walked, walked if walked < n else qkv.shape[0], longest, n_heads, key_dim, value_dim)[0]
+        code = lib.cb_matrix_memory(*args[:-1], columns, args[-1])
+    _check(code, "matrix_memory")
 
 
 def head_norm_gate(o, gain, gain_per_head, gate, out, gate_kind, n_heads, value_dim, eps,

@@ -14,11 +14,15 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
+import platform
 import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -35,12 +39,18 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", 
 
 # Host-only sources (C++, no device code): compiled by the same nvcc call, which hands them
 # to the host compiler.
-HOST_SOURCES = {"host_step": "host_step.cpp", "host_cache": "host_cache.cpp"}
+HOST_SOURCES = {"host_step": "host_step.cpp", "host_cache": "host_cache.cpp", "host_call": "host_call.cpp"}
+# `host_call` is an extension of the interpreter: without its headers (or on another machine than
+# x86-64 Linux) the kernels' entry points are called through ctypes alone.
+PYTHON_INCLUDE = sysconfig.get_paths()["include"]
+NATIVE_CALLS = (platform.machine() == "x86_64" and sys.platform.startswith("linux") and sys.implementation.name == "cpython"
+                and os.path.exists(os.path.join(PYTHON_INCLUDE, "Python.h")))
 
 # source file -> extra headers whose change must trigger a rebuild
 MODULES: Dict[str, List[str]] = {
     "host_step": [],
     "host_cache": [],
+    **({"host_call": []} if NATIVE_CALLS else {}),
     "elementwise": ["common.cuh"],
     "gemm_simt": ["common.cuh"],
     "attention_generic": ["common.cuh"],
@@ -83,6 +93,8 @@ def _nvcc() -> str:
 def _digest(name: str) -> str:
     h = hashlib.sha256()
     h.update(" ".join(NVCC_FLAGS).encode())
+    if name == "host_call":
+        h.update(sys.implementation.cache_tag.encode())
     for fn in [_source(name)] + MODULES[name]:
         with open(os.path.join(CSRC, fn), "rb") as f:
             h.update(fn.encode())
@@ -128,6 +140,8 @@ def library_path(name: str) -> str:
                 pass
     tmp = os.path.join(out_dir, f".{fname}.{os.getpid()}.tmp")
     cmd = [_nvcc()] + NVCC_FLAGS + ["-I", CSRC, "-o", tmp, os.path.join(CSRC, _source(name))]
+    if name == "host_call":
+        cmd += ["-I", PYTHON_INCLUDE]
     print(f"[crucible_b200] compiling {_source(name)} for sm_100a (first use) ...",
           file=sys.stderr, flush=True)
     t0 = time.time()
@@ -182,10 +196,26 @@ def signatures(text: str) -> Dict[str, tuple]:
     return out
 
 
+_KINDS = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_long: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
+
+
+def _native_calls():
+    """The extension module that calls entry points (`csrc/host_call.cpp`), or None."""
+    if not NATIVE_CALLS:
+        return None
+    module = _loaded.get("host_call")
+    if module is None:
+        loader = importlib.machinery.ExtensionFileLoader("cb_host_call", library_path("host_call"))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("cb_host_call", loader))
+        loader.exec_module(module)
+        _loaded["host_call"] = module
+    return module
+
+
 def load(name: str) -> ctypes.CDLL:
     """The library of module `name`.  A kernel source's entry points know their parameters' types, read off
-    the source's own declarations, so that the wrappers pass plain numbers and addresses: a launch
-    passes some twenty, and an object made for each cost the host 2 to 3 us."""
+    the source's own declarations, so that the wrappers pass plain numbers and addresses, and those that
+    return a status are called without ctypes (`_native_calls`)."""
     lib = _loaded.get(name)
     if lib is not None:
         return lib
@@ -194,10 +224,15 @@ def load(name: str) -> ctypes.CDLL:
         if lib is None:
             lib = ctypes.CDLL(library_path(name))
             if name not in HOST_SOURCES:
+                native = _native_calls()
                 with open(os.path.join(CSRC, _source(name))) as f:
                     for entry, (result, kinds) in signatures(f.read()).items():
                         fn = getattr(lib, entry)
                         fn.restype, fn.argtypes = result, kinds
+                        if native is not None and result is ctypes.c_int:
+                            direct = native.wrap(ctypes.cast(fn, ctypes.c_void_p).value, "".join(_KINDS[k] for k in kinds), fn)
+                            if direct is not None:
+                                setattr(lib, entry, direct)
             _loaded[name] = lib
         return lib
 

@@ -1,11 +1,11 @@
 // Paged attention of the 32-bit path over tiles of keys, all in fp32 on CUDA cores.
 //
-// A block takes 64 (or 16) packed rows of one request and one key/value head, rows being (position, head
+// A block takes 32 (or 16) packed rows of one request and one key/value head, rows being (position, head
 // of the group) pairs, and walks the keys in tiles: scores as a product of row and key tiles, a running
 // maximum and sum a row, probabilities through shared memory, then the product with the values.  A key
 // read from memory serves all the block's rows; the one-warp-a-row kernels (attention_generic.cu,
 // sink_attention.cu) read it once a row and reduce every score over a warp, which bounds them: 700 tokens
-// of 12 heads of 64: 909 us there, 89 here; a token each of 24 requests behind 3,800 keys, 8 heads of 128:
+// of 12 heads of 64: 909 us there, 71 here; a token each of 24 requests behind 3,800 keys, 8 heads of 128:
 // 7.7 ms a layer there, 0.63 here.
 //
 // A row's result is a function of its own query and keys: tiles begin at multiples of the tile's size
@@ -22,8 +22,6 @@
 #include "common.cuh"
 
 namespace {
-
-constexpr int THREADS = 256;
 
 struct Params {
     const float* q;
@@ -68,20 +66,21 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // keys of a tile: a function of the row sizes alone (see above)
 template <int DP> constexpr int TILE = DP <= 128 ? 64 : 32;
 template <int DP, int QR> constexpr size_t SMEM_FLOATS =
-    (size_t)QR * (DP + 4) + 2 * (size_t)TILE<DP> * (DP + 4) + (size_t)QR * (TILE<DP> + 4);
+    (size_t)QR * (DP + 4) + 2 * (size_t)TILE<DP> * (DP + 4) + (size_t)QR * (TILE<DP> + 4) + 2 * (size_t)TILE<DP>;
 
-// DP: both sizes padded; QR: packed rows of a block, 16 or 64.  Thread (ty, tx) of 16 x 16 has the rows
-// ty + 16 i; of the scores the keys tx + 16 j, of the output the features 4 tx + 64 c ...
-template <int DP, int QR>
-__global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kernel(const Params p) {
+// DP: both sizes padded; QR: packed rows of a block, 16 or 32.  Thread (ty, tx) of TY x 16 has the rows
+// ty + TY i; of the scores the keys tx + 16 j, of the output the features 4 tx + 64 c ...
+template <int DP, int QR, int THREADS>
+__global__ void __launch_bounds__(THREADS, (DP <= 64 ? 512 : 256) / THREADS) attention_f32_kernel(const Params p) {
     cb_pdl_trigger();
     cb_pdl_wait();
-    constexpr int P = DP + 4, KT = TILE<DP>, PP = KT + 4, NR = QR / 16, NK = KT / 16, NC = DP / 64;
+    constexpr int P = DP + 4, KT = TILE<DP>, PP = KT + 4, TY = THREADS / 16, NR = QR / TY, NK = KT / 16, NC = DP / 64;
     extern __shared__ __align__(16) float smem[];
     float* sq = smem;                  // [QR][P]
     float* sk = sq + QR * P;           // [KT][P]
     float* sv = sk + KT * P;           // [KT][P]
     float* sp = sv + KT * P;           // [QR][PP] probabilities, -1 for a key the row does not see
+    int* srow = reinterpret_cast<int*>(sp + QR * PP);      // [2][KT] where a tile's keys lie
     const int req = blockIdx.z, kvh = blockIdx.y;
     const int row_base = p.req_row_start[req];
     const int n_rows = (p.req_row_start[req + 1] - row_base) * p.n_rep;
@@ -108,7 +107,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     bool real[NR];
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-        const int row = r0 + ty + 16 * i;
+        const int row = r0 + ty + TY * i;
         real[i] = row < n_rows;
         pos[i] = first_pos + min(row, n_rows - 1) / p.n_rep;
         lo[i] = low(pos[i]);
@@ -120,26 +119,28 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     const int kept_tiles = p.window > 0 ? min((p.keep_first + KT - 1) / KT, key_lo / KT) : 0;
     const int n_tiles = kept_tiles + (last_pos - key_lo) / KT + 1;
     auto tile_key0 = [&](int j) { return j < kept_tiles ? j * KT : key_lo + (j - kept_tiles) * KT; };
-    // a tile's rows of K or V; keys that none of the block's rows sees (behind its last position, ahead of
-    // its windows) are zeros and not read: their page may have been given back
-    auto fetch_keys = [&](int key0, const float* cache, int n, float* to, auto all_seen) {
+    // Where a tile's keys lie: the row of the pool's rows of this head, a key a thread, looked up a tile ahead (by every
+    // piece of 16 bytes for itself, behind a division and a dependent load each, the two fetches of a tile took
+    // a third of its time).  Keys that none of the block's rows sees (behind its last position, ahead of its windows)
+    // have none: they are zeros and not read, their page may have been given back.
+    auto place = [&](int j) {
+        const int key = tile_key0(j) + tid;
+        if (key > last_pos || (key < first_key && key >= p.keep_first)) return -1;
+        const int page = table[key / p.page_tokens];
+        return (page * p.n_kv_heads + kvh) * p.page_tokens + key % p.page_tokens;
+    };
+    auto fetch = [&](int j, const float* cache, int n, float* to) {
+        const int* rows = srow + (j & 1) * KT;
+#pragma unroll 4
         for (int i = tid; i < KT * (DP / 4); i += THREADS) {
-            const int t = i / (DP / 4), d = (i % (DP / 4)) * 4, key = key0 + t;
-            if (key <= last_pos && d < n && (decltype(all_seen)::value || key >= first_key || key < p.keep_first)) {
-                const int page = table[key / p.page_tokens];
-                cp16(to + t * P + d,
-                     cache + (((size_t)page * p.n_kv_heads + kvh) * p.page_tokens + key % p.page_tokens) * n + d);
-            } else {
-                *reinterpret_cast<float4*>(to + t * P + d) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            const int t = i / (DP / 4), d = (i % (DP / 4)) * 4, row = rows[t];
+            if (row >= 0 && d < n) cp16(to + t * P + d, cache + (size_t)row * n + d);
+            else *reinterpret_cast<float4*>(to + t * P + d) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         cp_commit();
     };
-    auto fetch = [&](int j, const float* cache, int n, float* to) {
-        const int key0 = tile_key0(j);
-        if (key0 >= first_key) fetch_keys(key0, cache, n, to, std::true_type{});
-        else fetch_keys(key0, cache, n, to, std::false_type{});
-    };
+    if (tid < KT) srow[tid] = place(0);
+    __syncthreads();
     float m[NR], l[NR];
     pair_t acc[NR][2 * NC];
 #pragma unroll
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     fetch(0, p.v_cache, E, sv);
     for (int j = 0; j < n_tiles; ++j) {
         const int key0 = tile_key0(j);
+        const int ahead = tid < KT && j + 1 < n_tiles ? place(j + 1) : -1;
         cp_wait<1>();                  // the tile's keys
         __syncthreads();
         pair_t s[NR][NK];
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
         for (int d = 0; d < DP; d += 4) {
             ulonglong2 x[NR], y[NK];
 #pragma unroll
-            for (int i = 0; i < NR; ++i) x[i] = pairs_at(sq + (ty + 16 * i) * P + d);
+            for (int i = 0; i < NR; ++i) x[i] = pairs_at(sq + (ty + TY * i) * P + d);
 #pragma unroll
             for (int k = 0; k < NK; ++k) y[k] = pairs_at(sk + (tx + 16 * k) * P + d);
 #pragma unroll
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
             for (int k = 0; k < NK; ++k) {
                 const float e = seen[k] ? expf(v[k] - m_new) : 0.f;
                 sum += e;
-                sp[(ty + 16 * i) * PP + tx + 16 * k] = seen[k] ? e : -1.f;
+                sp[(ty + TY * i) * PP + tx + 16 * k] = seen[k] ? e : -1.f;
             }
 #pragma unroll
             for (int x = 1; x < 16; x <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
@@ -208,6 +210,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
 #pragma unroll
             for (int c = 0; c < 2 * NC; ++c) acc[i][c] = fma_pair(acc[i][c], f, 0);
         }
+        if (tid < KT) srow[((j + 1) & 1) * KT + tid] = ahead;
         whole = __syncthreads_and(whole);        // the keys have been read, the probabilities are written
         if (j + 1 < n_tiles) fetch(j + 1, p.k_cache, D, sk);
         else cp_commit();
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
             for (int k = 0; k < KT; k += 4) {
                 float4 w[NR];
 #pragma unroll
-                for (int i = 0; i < NR; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (ty + 16 * i) * PP + k);
+                for (int i = 0; i < NR; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (ty + TY * i) * PP + k);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     ulonglong2 v[NC];
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
                 for (int c = 0; c < NC; ++c) v[c] = pairs_at(sv + k * P + 4 * tx + 64 * c);
 #pragma unroll
                 for (int i = 0; i < NR; ++i) {
-                    const float w = sp[(ty + 16 * i) * PP + k];
+                    const float w = sp[(ty + TY * i) * PP + k];
                     if (w < 0.f) continue;                      // not seen (a NaN is)
                     const pair_t f = both(w);
 #pragma unroll
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         if (!real[i]) continue;
-        const int row = r0 + ty + 16 * i;
+        const int row = r0 + ty + TY * i;
         const int t = row_base + row / p.n_rep, h = kvh * p.n_rep + row % p.n_rep;
         float corr = 1.f, sum = l[i];
         if (p.sinks != nullptr) {
@@ -289,19 +292,19 @@ __global__ void __launch_bounds__(THREADS, DP <= 64 ? 2 : 1) attention_f32_kerne
     }
 }
 
-template <int DP, int QR>
+template <int DP, int QR, int THREADS>
 int launch(const Params& p, int n_requests, int max_new, cudaStream_t s) {
     constexpr size_t bytes = SMEM_FLOATS<DP, QR> * sizeof(float);
     static_assert(bytes <= 227 * 1024, "a block's shared memory");
     static bool configured = false;
     if (!configured && bytes > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<DP, QR>,
+        const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<DP, QR, THREADS>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     const dim3 grid((max_new * p.n_rep + QR - 1) / QR, p.n_kv_heads, n_requests);
-    cb_launch(attention_f32_kernel<DP, QR>, grid, dim3(THREADS), bytes, s, p);
+    cb_launch(attention_f32_kernel<DP, QR, THREADS>, grid, dim3(THREADS), bytes, s, p);
     return cb_last_error();
 }
 
@@ -329,7 +332,16 @@ CB_EXPORT int cb_attention_f32(const float* q, int q_stride, const float* gate, 
     p.out_scale = out_scale; p.gate_per_head = gate_per_head;
     cudaStream_t s = (cudaStream_t)stream;
     const bool few = max_new * p.n_rep <= 16;
-#define CB_F32_ATTENTION(DD) return few ? launch<DD, 16>(p, n_requests, max_new, s) : launch<DD, 64>(p, n_requests, max_new, s)
+    // Blocks of 32 rows: two or more to an SM, so that one's barriers and exponentials run beside another's products,
+    // and twice as many to deal out where the longest walks eleven tiles and the average six.  Few blocks have an SM
+    // to themselves and take eight warps.  us with 64 rows and eight warps / 32 and four / 32 and eight: 700 tokens of 12
+    // heads of 64 75 / 71 / 78, of 8 heads of 128 116 / 97 / 89, 2,000 of 16 heads of 64 406 / 346 / 408, of 128 595 /
+    // 595 / 850, 300 of 8 heads of 128 58 / 45 / 44.
+    const long blocks = (long)((max_new * p.n_rep + 31) / 32) * n_kv_heads * n_requests;
+#define CB_F32_ATTENTION(DD)                                           \
+    return few ? launch<DD, 16, 256>(p, n_requests, max_new, s)        \
+           : blocks <= 200 ? launch<DD, 32, 256>(p, n_requests, max_new, s) \
+                           : launch<DD, 32, 128>(p, n_requests, max_new, s)
     if (most <= 64) CB_F32_ATTENTION(64);
     if (most <= 128) CB_F32_ATTENTION(128);
     CB_F32_ATTENTION(256);

@@ -46,3 +46,16 @@ def test_a_shared_expert_is_held_once(shared, slices, copies, dtype):
     assert part.slices == (slices if dtype == torch.bfloat16 else 0)
     more = 3 * width * (part.slices * ff - shared if part.slices and copies == 1 else part.slices * ff)
     assert sum(held.values()) == (matrices + more + given["router"].numel()) * size + 4 * (experts + part.slices)
+
+
+@pytest.mark.parametrize("width,ff,shared,tokens,rides", [
+    (2048, 2816, 2816, 128, True), (2048, 2816, 2816, 129, False), (2048, 2816, 2816, 319, False), (2048, 2816, 2816, 320, True),
+    (2048, 2816, 2816, 2048, True), (2048, 2816, 2816, 2049, False), (1024, 1408, 1408, 129, True), (1024, 1408, 1408, 2048, True),
+    (1024, 1408, 2816, 128, True), (1024, 1408, 2816, 129, False), (1024, 1408, 0, 64, False)])
+def test_where_a_plain_shared_expert_rides(width, ff, shared, tokens, rides):
+    from crucible_b200.config.model_config import FeedForwardSpec
+    from crucible_b200.parts import FEED_FORWARDS
+    options = (("experts", 8), ("top", 2)) + ((("shared_intermediate", shared),) if shared else ())
+    part = FEED_FORWARDS.build("moe", FeedForwardSpec("moe", width, ff, options))
+    part.dtype = torch.bfloat16
+    assert part._rides(tokens) == rides

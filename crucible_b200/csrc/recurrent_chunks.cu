@@ -850,21 +850,25 @@ private:
 // the threads that compute they were 1,000 to 1,600 of a chunk's 4,650 cycles; by two more warps the pipe that
 // serves shared memory was still theirs (237 -> 251 us), and a bulk copy a row costs that warp 60 cycles (401 us).
 struct WalkMaps { CUtensorMap q, w, k, u, s; };          // wq, ww, the keys, wu, ws
+// 16 columns: the queries' rows over S by four warps of their own, beside both products of the chain, the second of
+// which has all eight warps (against four that left the second product for them: 32 x 64 heads, 700 tokens 72.5 ->
+// 67.3 us, 16 x 128 heads, 2,048 tokens 200 -> 196, per channel 251 -> 247.7).  8: with W's rows, before them.
+template <int ET> constexpr int QUERY_THREADS = ET == 16 ? 128 : 0;
 template <int DP, int RULE, int ET>
-__global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
+__global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int CG = ET / 4, PS = DP + 32 / CG;
     constexpr bool VECTOR = VECTOR_DECAY<RULE>;
-    // 16 columns: the queries' rows beside the state's sums, by the other half of the warps; 8: with W's rows before them
-    constexpr bool BESIDE = ET == 16;
+    constexpr bool BESIDE = QUERY_THREADS<ET> > 0;
     // the queries' rows and W's over S, keys, u, the chunk's decays per channel, the tokens' numbers
     constexpr int STAGE = 3 * CT * DP + CT * ET + DP + 4 * CT;
     static_assert(STAGE % 32 == 0 && (2 * ET * PS + CT * ET) % 32 == 0, "boxes begin on 128-byte boundaries");
-    // the second product: shares of the chunk's tokens, in lanes MS * CG apart; a thread has two pieces of four
-    // channels, DP / 2 apart, and four columns; four warps
+    // the second product: shares of the chunk's tokens, in lanes MS * CG apart; a thread has four columns and a piece of four
+    // channels, of eight warps, or two pieces, DP / 2 apart, of four (8 columns)
+    constexpr int PIECES = BESIDE ? 1 : 2;
     constexpr int TS = 4096 / (DP * ET), MS = 32 / (TS * CG), TOKENS = CT / TS;
-    static_assert(TS >= 2 && TS <= 8 && DP / 8 == 4 * MS, "four warps cover the state");
+    static_assert(TS >= 2 && TS <= 8 && DP / 8 == 4 * MS, "the warps cover the state");
     // (no shared variable beside this one: it would come first, and a box's place is a 128-byte boundary)
     extern __shared__ __align__(1024) float walk_smem[];
     float* states = walk_smem;                           // [2][ET][PS]: as the chunk begins, and as it ends
@@ -898,7 +902,7 @@ __global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_c
     }
     __syncthreads();
 
-    if (tid >= THREADS) {
+    if (tid >= THREADS + QUERY_THREADS<ET>) {
         // ---- the loader --------------------------------------------------------------------------------
         const int lane = tid & 31;
         auto landed = [&](int i) {                       // the copies of chunk i
@@ -948,7 +952,7 @@ __global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_c
     RowsOverState<DP, ET, CT, THREADS / 2> queries(tid % (THREADS / 2));
     // the state's part: a share of the tokens, channels ud + DP / 2 i, columns 4 uc + c
     const int lane = tid & 31, uc = lane % CG, part = lane / (CG * MS);
-    const int ud = (tid / 32 % 4 * MS + lane / CG % MS) * 4;
+    const int ud = (tid / 32 % (BESIDE ? 8 : 4) * MS + lane / CG % MS) * 4;
     int buf = 0;
     uint32_t phase = 0;
     for (int base = row0; base < row1; base += CT, phase ^= buf, buf ^= 1) {
@@ -980,6 +984,14 @@ __global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_c
         __syncthreads();
         if (!tc::mbar_wait(&full[buf], phase, abort_flag) && !*abort_flag)
             tc::give_up(abort_flag, a.status, tc::ST_EPILOGUE_TIMEOUT);      // (the rest is computed from what there is)
+        if (BESIDE && tid >= THREADS) {
+            const bool has = queries.row < cnt && col0 + queries.col < E;
+            within(has, queries.row, queries.col, local, queries.LEFT);
+            float sum[queries.SUMS];
+            queries.take(rows, S, sum);
+            if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
+            continue;
+        }
         {
             float sum[first.SUMS];
             first.take(rows + (BESIDE ? CT * DP : 0), S, sum);
@@ -997,42 +1009,36 @@ __global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_c
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");      // (the loader is at its copies)
-        if (tid >= THREADS / 2) {
-            if (BESIDE) {
-                const bool has = queries.row < cnt && col0 + queries.col < E;
-                within(has, queries.row, queries.col, local, queries.LEFT);
-                float sum[queries.SUMS];
-                queries.take(rows, S, sum);
-                if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
-            }
-        } else {
-            pair_t x[2][4][2];
+        if (BESIDE || tid < THREADS / 2) {
+            pair_t x[PIECES][4][2];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) x[c / 4][c % 4][0] = x[c / 4][c % 4][1] = 0;
+            for (int c = 0; c < 4 * PIECES; ++c) x[c / 4][c % 4][0] = x[c / 4][c % 4][1] = 0;
 #pragma unroll
             for (int i = 0; i < TOKENS; ++i) {
                 const int t = part * TOKENS + i;
-                const ulonglong2 k0 = pairs_at(keys + t * DP + ud), k1 = pairs_at(keys + t * DP + DP / 2 + ud);
+                const ulonglong2 k0 = pairs_at(keys + t * DP + ud), k1 = pairs_at(keys + t * DP + (PIECES - 1) * (DP / 2) + ud);
                 const float4 v = *reinterpret_cast<const float4*>(su + t * ET + uc * 4);
                 const pair_t f[4] = {make_pair_of(v.x, v.x), make_pair_of(v.y, v.y), make_pair_of(v.z, v.z), make_pair_of(v.w, v.w)};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     x[0][c][0] = fma_pair(k0.x, f[c], x[0][c][0]);
                     x[0][c][1] = fma_pair(k0.y, f[c], x[0][c][1]);
-                    x[1][c][0] = fma_pair(k1.x, f[c], x[1][c][0]);
-                    x[1][c][1] = fma_pair(k1.y, f[c], x[1][c][1]);
+                    if constexpr (!BESIDE) {
+                        x[1][c][0] = fma_pair(k1.x, f[c], x[1][c][0]);
+                        x[1][c][1] = fma_pair(k1.y, f[c], x[1][c][1]);
+                    }
                 }
             }
-            // the tokens' shares: a piece of the channels to each half of the lanes, then half of its columns
-            float sum[32];
+            // the tokens' shares: a piece of the channels to each half of the lanes (two pieces), then half of its columns
+            float sum[16 * PIECES];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < 8 * PIECES; ++i) {
                 const float2 v = split_pair(x[i / 8][i / 2 % 4][i % 2]);
                 sum[2 * i] = v.x; sum[2 * i + 1] = v.y;
             }
-            shares_summed<32, TS>(sum, part, CG * MS);
-            constexpr int COLS = 8 / TS;
-            const int d = ud + (part / (TS / 2)) * (DP / 2), c0 = uc * 4 + part % (TS / 2) * COLS;
+            shares_summed<16 * PIECES, TS>(sum, part, CG * MS);
+            constexpr int COLS = 4 * PIECES / TS, SPLIT = TS / PIECES;          // lanes that share a piece's columns
+            const int d = ud + (part / SPLIT) * (DP / 2), c0 = uc * 4 + part % SPLIT * COLS;
             const float g_end = VECTOR ? 1.f : nums[cnt - 1].x;
             const float4 own = *reinterpret_cast<const float4*>(sg + d);
             float* next = states + (buf ^ 1) * ET * PS;
@@ -1049,6 +1055,7 @@ __global__ void __launch_bounds__(THREADS + 32) chunk_walk_kernel(const __grid_c
         }
     }
     __syncthreads();
+    if (BESIDE && tid >= THREADS) return;
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
         if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = states[buf * ET * PS + place_of(c) * PS + d];
@@ -1081,7 +1088,7 @@ int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
         !tc::make_map_heads_f32(&maps.s, a.ws, a.piece_rows, a.H, 4, (uint64_t)a.H * 4, 4, CT))
         return CB_ERR_UNSUPPORTED;
     const dim3 grid(n_requests, a.H, (a.E + ET - 1) / ET);
-    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS + 32), bytes, s, maps, a);
+    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS + QUERY_THREADS<ET> + 32), bytes, s, maps, a);
     return cb_last_error();
 }
 

@@ -157,6 +157,21 @@ def _tile_width(m: int, n_cols: int, epi: int = 1, multiple_of: int = 1):
     return best, 1
 
 
+@functools.lru_cache(maxsize=4096)
+def _tile_and_shares(m: int, n_cols: int, k: int, epi: int):
+    """`_tile_width` for float32 results, with the shares of K where the narrowest tiles leave no room for two and
+    wider ones do: a chain over a long K is longer than what a wider tile costs.  75 to 148 tiles of 64 columns ->
+    two shares of 96 or 128, us: 330 x 2,048 by K = 4,096 / 5,632 / 8,192 13.3 / 17.2 / 24.9 -> 11.8 / 13.9 / 18.2 (96),
+    512 rows 13.1 / 17.1 / 25.1 -> 13.0 / 15.9 / 21.4 (128), 640 x 1,024 by 4,096 13.2 -> 11.9 (96); at K = 3,072
+    10.7 and 10.4, at 2,048 8.0 and 8.3.  Tiles wider than 128 columns leave the next norm's input to another launch."""
+    bn, per_sm = _tile_width(m, n_cols, epi)
+    if bn == 64 and epi != STORE_BF16 and k_splits(m, n_cols, k, bn) == 1:
+        for wide, least in ((96, 3584), (128, 5120)):
+            if k >= least and 2 * -(-m // 128) * -(-n_cols // wide) <= K_SPLIT_BLOCK_LIMIT[2]:
+                return wide, 1, 2
+    return bn, per_sm
+
+
 TALL_MIN_ROWS = 1024        # two accumulators per block (256 x 256 of output) ...
 TALL_MIN_K = 512            # ... pay where many rows meet enough 256 x 256 tiles to fill the SMs: at
 TALL_MIN_FILL = 0.8         # long K they halve the operand bytes per flop, at short K the blocks' starts and ends
@@ -418,7 +433,7 @@ def linear(a, w, out, *, accumulate=False, tile=None, emit=None, pre=None, act=0
         if waves and _gemm_waves(a, w, out, n, epi, waves, act=act):
             return True
         tile = (256, 0) if tall else None
-    bn, per_sm, *splits = _tile_of(tile) if tile else _tile_width(m, n, epi)
+    bn, per_sm, *splits = _tile_of(tile) if tile else _tile_and_shares(m, n, k, epi)
     return _gemm(a, w, out, n, epi, bn, per_sm, splits[0] if splits else None, emit, pre, None, act)
 
 

@@ -85,10 +85,17 @@ PyObject* getattro(PyObject* self, PyObject* name) {         // argtypes, restyp
     return PyObject_GetAttr(reinterpret_cast<Call*>(self)->general, name);
 }
 
+// what is set is the ctypes function's, too (another result type, other parameters), and calls are then left to it
+int setattro(PyObject* self, PyObject* name, PyObject* value) {
+    Call* c = reinterpret_cast<Call*>(self);
+    c->count = -1;
+    return PyObject_SetAttr(c->general, name, value);
+}
+
 PyMemberDef members[] = {{"__vectorcalloffset__", T_PYSSIZET, offsetof(Call, vectorcall), READONLY, nullptr},
                          {nullptr, 0, 0, 0, nullptr}};
 PyType_Slot slots[] = {{Py_tp_dealloc, (void*)dealloc}, {Py_tp_call, (void*)PyVectorcall_Call},
-                       {Py_tp_getattro, (void*)getattro}, {Py_tp_members, members}, {0, nullptr}};
+                       {Py_tp_getattro, (void*)getattro}, {Py_tp_setattro, (void*)setattro}, {Py_tp_members, members}, {0, nullptr}};
 PyType_Spec spec = {"cb_host_call.Call", sizeof(Call), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL, slots};
 PyObject* call_type = nullptr;
 

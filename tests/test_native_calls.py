@@ -51,6 +51,18 @@ def test_other_types_and_counts_are_ctypes_own():
     assert call.argtypes == (P, I, F) or list(call.argtypes) == [P, I, F]
 
 
+def test_what_is_set_is_the_ctypes_functions():
+    seen = []
+    call, general = _direct([P, I, F], seen, result=-1)
+    assert call(None, 3, 2.0) == -1
+    call.restype = ctypes.c_uint8
+    call.argtypes = [P, I, ctypes.c_float]
+    assert general.restype is ctypes.c_uint8 and call(None, 3, 2.0) == 255
+    assert seen[0] == seen[1] == (None, 3, 2.0)
+    with pytest.raises((AttributeError, TypeError)):
+        call.argtypes = 5
+
+
 def test_threads_call_side_by_side():
     seen = []
     call, _ = _direct([I, F, P], seen)

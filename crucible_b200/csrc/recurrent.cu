@@ -565,7 +565,10 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
     const int r = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS;
     const int g = head / (n_heads / n_qk_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int mine = (warp * (32 / LANES) + lane / LANES) * NC, col = col0 + mine, part = lane % LANES;
+    // (How this sum and the state's loads are written decides how far ahead the compiler takes the tokens' operands with
+    // one column: 300 tokens of 16 heads of 128 by wkv 71.5 us so and 79.8 as col0 + mine, by the delta rule 77.3 and 82.6)
+    const int mine = (warp * (32 / LANES) + lane / LANES) * NC, part = lane % LANES;
+    const int col = NC == 1 ? col0 + warp * (32 / LANES) + lane / LANES : col0 + mine;
     const bool live = col < E;
     const int row0 = req_row_start[r], row1 = req_row_start[r + 1];
     const int slot = req_state_slot[r];
@@ -580,7 +583,8 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
 #pragma unroll
     for (int i = 0; i < P; ++i) {
         const int d = part * P + i;
-        load_columns<NC>(s[i], S + (size_t)d * E + col, live && d < D);
+        if constexpr (NC == 1) s[i][0] = (live && d < D) ? S[(size_t)d * E + col] : 0.f;
+        else load_columns<NC>(s[i], S + (size_t)d * E + col, live && d < D);
         n[i] = (RULE == RULE_MLSTM && d < D) ? kept_n[(size_t)head * D + d] : 0.f;
         if (RULE == RULE_WKV) n[i] = d < D ? per_head[(size_t)head * D + d] : 0.f;      // the bonus u
     }
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 qq[4 * j] = b.x; qq[4 * j + 1] = b.y; qq[4 * j + 2] = b.z; qq[4 * j + 3] = b.w;
             }
             float v[NC];
-            load_columns<NC>(v, sv + tt * COLS + mine, true);
+            load_columns<NC>(v, sv + tt * COLS + (NC == 1 ? col - col0 : mine), true);
             const size_t out_at = (size_t)(base + tt) * n_heads * E + (size_t)head * E + col;
             if (RULE == RULE_DELTA) {
                 // One pass per token.  The write of the token before (S <- g S + k u^T) is still
@@ -791,9 +795,11 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 }
                 if (pending) {
                     lanes_summed<LANES>(p_o);
+                    if (live && part == 0) {
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) p_o[c] = __fadd_rn(p_o[c], p_v[c]);
-                    if (live && part == 0) store_columns<NC>(out + p_at, p_o);
+                        for (int c = 0; c < NC; ++c) p_o[c] = __fadd_rn(p_o[c], p_v[c]);
+                        store_columns<NC>(out + p_at, p_o);
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {

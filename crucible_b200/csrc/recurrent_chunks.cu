@@ -780,11 +780,11 @@ __global__ void __launch_bounds__(OUT_THREADS, 4) chunk_out_kernel(const Args a)
 // the chain's latencies.  So a thread's piece of a product is up to 8 x 4 numbers (12 reads of 16 bytes for 128
 // products), what is left of a sum lies in neighbouring lanes, which halve it among themselves by exchanges (no shares
 // in shared memory), S lies there twice, as the chunk begins and as it ends, and a chunk has two barriers: u is
-// there; the state is there.  2,048 tokens of 16 heads of 128 with the chunks' numbers, against pieces of 4 x 4, shares in shared memory and
-// four barriers: delta 240 -> 233 us, channel delta 328 -> 280; 8 heads 166 -> 143, 214 -> 170; 300 tokens of 16 heads
-// 46.4 -> 44.4, 61.1 -> 54.4.  The queries' rows beside the state's sums: 45.8 -> 44.4 with 16 columns a block, but
-// 34.3 -> 35.1 (333 tokens of 8 heads of 128) and 25.7 -> 28.3 (300 of 64) with 8, where W's rows alone leave a thread a
-// piece of 2 x 4; k^T over u by all eight warps: 233 -> 245.
+// there; the state is there.  2,048 tokens of 16 heads of 128 with the chunks' numbers, against pieces of 4 x 4, shares
+// in shared memory and four barriers: delta 240 -> 233 us, channel delta 328 -> 280; 8 heads 166 -> 143, 214 -> 170.
+// The queries' rows beside the chain with 8 columns a block, too: 34.3 -> 35.1 (333 tokens of 8 heads of 128) and
+// 25.7 -> 28.3 (300 of 64), where W's rows alone leave a thread a piece of 2 x 4.  What a token has within the chunk, asked
+// for before the chunk's barrier: 196 -> 202.
 // S's columns lie in shared memory as rows [ET][PS], so that sums over D run over neighbouring pairs; column
 // 4 j + i is row i * (ET / 4) + j, and the pitch puts the rows that neighbouring lanes write 128 / ET banks apart.
 

@@ -853,20 +853,25 @@ struct WalkMaps { CUtensorMap q, w, k, u, s; };          // wq, ww, the keys, wu
 // 16 columns: the queries' rows over S by four warps of their own, beside both products of the chain, the second of
 // which has all eight warps (against four that left the second product for them: 32 x 64 heads, 700 tokens 72.5 ->
 // 67.3 us, 16 x 128 heads, 2,048 tokens 200 -> 196, per channel 251 -> 247.7).  8: with W's rows, before them.
-template <int ET> constexpr int QUERY_THREADS = ET == 16 ? 128 : 0;
-template <int DP, int RULE, int ET>
-__global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
+// CROWDED: more blocks of heads of 64 than SMs, two to an SM: they hide one another's latencies, and four warps leave the
+// second product for the queries' rows.  (The nine warps of a block are three on one of the SM's four quarters, so
+// two blocks need at most 96 registers a thread.)  32 heads, 20 portions of 100: the walk 182 us with 104 registers, 168
+// with the queries' warps apart, 145 with three blocks and spills, 120 so; 8 portions of 130 75.5, 71.3, 77.7 and 56.0.
+template <int ET, bool CROWDED> constexpr int QUERY_THREADS = ET == 16 && !CROWDED ? 128 : 0;
+template <int DP, int RULE, int ET, bool CROWDED>
+__global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET, CROWDED> + 32, CROWDED ? 2 : 1)
+chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
     cb_pdl_trigger();
     cb_pdl_wait();
     constexpr int CG = ET / 4, PS = DP + 32 / CG;
     constexpr bool VECTOR = VECTOR_DECAY<RULE>;
-    constexpr bool BESIDE = QUERY_THREADS<ET> > 0;
+    constexpr bool BESIDE = ET == 16, APART = QUERY_THREADS<ET, CROWDED> > 0;
     // the queries' rows and W's over S, keys, u, the chunk's decays per channel, the tokens' numbers
     constexpr int STAGE = 3 * CT * DP + CT * ET + DP + 4 * CT;
     static_assert(STAGE % 32 == 0 && (2 * ET * PS + CT * ET) % 32 == 0, "boxes begin on 128-byte boundaries");
     // the second product: shares of the chunk's tokens, in lanes MS * CG apart; a thread has four columns and a piece of four
-    // channels, of eight warps, or two pieces, DP / 2 apart, of four (8 columns)
-    constexpr int PIECES = BESIDE ? 1 : 2;
+    // channels, of eight warps, or two pieces, DP / 2 apart, of four
+    constexpr int PIECES = APART ? 1 : 2;
     constexpr int TS = 4096 / (DP * ET), MS = 32 / (TS * CG), TOKENS = CT / TS;
     static_assert(TS >= 2 && TS <= 8 && DP / 8 == 4 * MS, "the warps cover the state");
     // (no shared variable beside this one: it would come first, and a box's place is a 128-byte boundary)
@@ -902,7 +907,7 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
     }
     __syncthreads();
 
-    if (tid >= THREADS + QUERY_THREADS<ET>) {
+    if (tid >= THREADS + QUERY_THREADS<ET, CROWDED>) {
         // ---- the loader --------------------------------------------------------------------------------
         const int lane = tid & 31;
         auto landed = [&](int i) {                       // the copies of chunk i
@@ -952,7 +957,7 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
     RowsOverState<DP, ET, CT, THREADS / 2> queries(tid % (THREADS / 2));
     // the state's part: a share of the tokens, channels ud + DP / 2 i, columns 4 uc + c
     const int lane = tid & 31, uc = lane % CG, part = lane / (CG * MS);
-    const int ud = (tid / 32 % (BESIDE ? 8 : 4) * MS + lane / CG % MS) * 4;
+    const int ud = (tid / 32 % (APART ? 8 : 4) * MS + lane / CG % MS) * 4;
     int buf = 0;
     uint32_t phase = 0;
     for (int base = row0; base < row1; base += CT, phase ^= buf, buf ^= 1) {
@@ -984,12 +989,15 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
         __syncthreads();
         if (!tc::mbar_wait(&full[buf], phase, abort_flag) && !*abort_flag)
             tc::give_up(abort_flag, a.status, tc::ST_EPILOGUE_TIMEOUT);      // (the rest is computed from what there is)
-        if (BESIDE && tid >= THREADS) {
+        auto take_queries = [&]() {
             const bool has = queries.row < cnt && col0 + queries.col < E;
             within(has, queries.row, queries.col, local, queries.LEFT);
             float sum[queries.SUMS];
             queries.take(rows, S, sum);
             if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
+        };
+        if (APART && tid >= THREADS) {
+            take_queries();
             continue;
         }
         {
@@ -1009,7 +1017,9 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");      // (the loader is at its copies)
-        if (BESIDE || tid < THREADS / 2) {
+        if (!APART && tid >= THREADS / 2) {
+            if (BESIDE) take_queries();
+        } else {
             pair_t x[PIECES][4][2];
 #pragma unroll
             for (int c = 0; c < 4 * PIECES; ++c) x[c / 4][c % 4][0] = x[c / 4][c % 4][1] = 0;
@@ -1023,7 +1033,7 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
                 for (int c = 0; c < 4; ++c) {
                     x[0][c][0] = fma_pair(k0.x, f[c], x[0][c][0]);
                     x[0][c][1] = fma_pair(k0.y, f[c], x[0][c][1]);
-                    if constexpr (!BESIDE) {
+                    if constexpr (!APART) {
                         x[1][c][0] = fma_pair(k1.x, f[c], x[1][c][0]);
                         x[1][c][1] = fma_pair(k1.y, f[c], x[1][c][1]);
                     }
@@ -1055,7 +1065,7 @@ __global__ void __launch_bounds__(THREADS + QUERY_THREADS<ET> + 32) chunk_walk_k
         }
     }
     __syncthreads();
-    if (BESIDE && tid >= THREADS) return;
+    if (APART && tid >= THREADS) return;
     for (int i = tid; i < DP * ET; i += THREADS) {
         const int d = i / ET, c = i - d * ET;
         if (d < D && col0 + c < E) state[(size_t)d * E + col0 + c] = states[buf * ET * PS + place_of(c) * PS + d];
@@ -1071,12 +1081,12 @@ int allow_smem(K kernel, size_t smem, bool& configured) {
     return (int)e;
 }
 
-template <int DP, int RULE, int ET>
+template <int DP, int RULE, int ET, bool CROWDED = false>
 int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
     constexpr size_t bytes = sizeof(float) * (2 * ET * (DP + 128 / ET) + CT * ET + 2 * (3 * CT * DP + CT * ET + DP + 4 * CT)) + 32;
     static_assert(bytes <= 226 * 1024, "a block's shared memory");
     static bool configured = false;
-    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET>, bytes, configured);
+    const int rc = allow_smem(chunk_walk_kernel<DP, RULE, ET, CROWDED>, bytes, configured);
     if (rc) return rc;
     WalkMaps maps;
     const uint64_t width = (uint64_t)a.H * a.D;
@@ -1088,9 +1098,11 @@ int launch_walk(const Args& a, int n_requests, cudaStream_t s) {
         !tc::make_map_heads_f32(&maps.s, a.ws, a.piece_rows, a.H, 4, (uint64_t)a.H * 4, 4, CT))
         return CB_ERR_UNSUPPORTED;
     const dim3 grid(n_requests, a.H, (a.E + ET - 1) / ET);
-    cb_launch(chunk_walk_kernel<DP, RULE, ET>, grid, dim3(THREADS + QUERY_THREADS<ET> + 32), bytes, s, maps, a);
+    cb_launch(chunk_walk_kernel<DP, RULE, ET, CROWDED>, grid, dim3(THREADS + QUERY_THREADS<ET, CROWDED> + 32), bytes, s, maps, a);
     return cb_last_error();
 }
+
+constexpr long CROWD = 148;          // blocks of the walk's 16 columns: beyond one an SM two share it
 
 template <int DP, int RULE>
 int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
@@ -1110,8 +1122,11 @@ int launch_chunks(const Args& a, int n_requests, int max_new, cudaStream_t s) {
     if (rc) return rc;
     if constexpr (IS_DELTA<RULE>) {
         // few heads: half the columns a block, so that twice as many SMs have one (8 heads of 128 x 128)
-        return n_requests * a.H * ((a.E + 15) / 16) <= 74 ? launch_walk<DP, RULE, 8>(a, n_requests, s)
-                                                          : launch_walk<DP, RULE, 16>(a, n_requests, s);
+        const long blocks = (long)n_requests * a.H * ((a.E + 15) / 16);
+        if (blocks <= 74) return launch_walk<DP, RULE, 8>(a, n_requests, s);
+        if constexpr (DP == 64)
+            if (blocks > CROWD) return launch_walk<DP, RULE, 16, true>(a, n_requests, s);
+        return launch_walk<DP, RULE, 16>(a, n_requests, s);
     } else {
         cb_launch(chunk_scan_kernel<RULE>, dim3((a.D * a.E / 4 + THREADS - 1) / THREADS, a.H, n_requests), dim3(THREADS), 0,
                   s, a);

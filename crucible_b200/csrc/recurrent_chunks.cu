@@ -989,15 +989,12 @@ chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
         __syncthreads();
         if (!tc::mbar_wait(&full[buf], phase, abort_flag) && !*abort_flag)
             tc::give_up(abort_flag, a.status, tc::ST_EPILOGUE_TIMEOUT);      // (the rest is computed from what there is)
-        auto take_queries = [&]() {
+        if (APART && tid >= THREADS) {
             const bool has = queries.row < cnt && col0 + queries.col < E;
             within(has, queries.row, queries.col, local, queries.LEFT);
             float sum[queries.SUMS];
             queries.take(rows, S, sum);
             if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
-        };
-        if (APART && tid >= THREADS) {
-            take_queries();
             continue;
         }
         {
@@ -1018,7 +1015,13 @@ chunk_walk_kernel(const __grid_constant__ WalkMaps maps, const Args a) {
         }
         asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");      // (the loader is at its copies)
         if (!APART && tid >= THREADS / 2) {
-            if (BESIDE) take_queries();
+            if (BESIDE) {
+                const bool has = queries.row < cnt && col0 + queries.col < E;
+                within(has, queries.row, queries.col, local, queries.LEFT);
+                float sum[queries.SUMS];
+                queries.take(rows, S, sum);
+                if (has) put(queries.row, queries.col, local, sum, queries.LEFT);
+            }
         } else {
             pair_t x[PIECES][4][2];
 #pragma unroll

@@ -28,7 +28,7 @@
 // exponentials: set half a tile apart the groups were no faster (17.9 and 17.9), in turns slower (18.5), and a quarter
 // of the exponentials on the FMA pipe gave 2 %, 7 % less where most blocks are short.
 // Measured on one B200, replayed, a 2,048-token prompt: 12 heads of 64 on 4 17.8 us a layer (27 with P in shared
-// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 25.8 (58), 16
+// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 26.3 (58), 16
 // heads of 256 on 1 30.8 (76).
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
@@ -181,37 +181,13 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return d;
 }
 
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t both_of(float v) { return pair_of(v, v); }
-
-// (a, b) times 1 / (1 + e^-x) of their logits: 16,384 of them a tile with a logit a result, when nothing else
-// is left to do, so that their instructions count: 18 a pair, where expf and the IEEE division took a hundred dependent
-// cycles an element.  e^-x = 2^n 2^f: n is -x log2(e) rounded (Cody and Waite's reduction; adding 1.5 * 2^23 leaves n in
-// the sum's low bits), f the rest with log2(e) in two parts.  The reciprocal is within one unit in the last place,
-// 2^-15 of what the bf16 result keeps; beyond +-88 the results are those at 88, 1 and (flushed) 0.
-__device__ __forceinline__ void gate_pair(float& a, float& b, float x0, float x1) {
-    constexpr float LOG2E_LOW = 1.925963033500988e-8f;            // log2(e) - LOG2E
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-88.5f));
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-88.5f));
-    asm("min.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(87.f));
-    asm("min.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(87.f));
-    const uint64_t x = pair_of(x0, x1), r = fma2(x, both_of(-LOG2E), both_of(12582912.f));
-    const uint64_t minus_n = fma2(r, both_of(-1.f), both_of(12582912.f));
-    const uint64_t f = fma2(x, both_of(-LOG2E_LOW), fma2(x, both_of(-LOG2E), minus_n));
-    float f0, f1, r0, r1;
-    pair_to(f, f0, f1);
-    pair_to(r, r0, r1);
-    const float s0 = __uint_as_float((__float_as_uint(r0) << 23) + 0x3f800000u);
-    const float s1 = __uint_as_float((__float_as_uint(r1) << 23) + 0x3f800000u);
-    float d0, d1, y0, y1;
-    pair_to(fma2(pair_of(ex2_fast(f0), ex2_fast(f1)), pair_of(s0, s1), both_of(1.f)), d0, d1);
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d0));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(d1));
-    pair_to(mul2(pair_of(a, b), pair_of(y0, y1)), a, b);
+// a times sigmoid(x) = 1 / (1 + e^-x), by t = e^-|x|: 1 / (1 + t), or t / (1 + t) for x < 0.  So the denominator is 1 to
+// 2, where the approximate division has its two units in the last place (its IEEE form, inlined 32 times, is what a block
+// would wait for at its end: 16 heads of 128, a window of 1,024, 2,048 tokens 32.9 us a layer with it, 26.3 so), and
+// a logit far below zero keeps its digits: all 65,536 logits give the bf16 nearest to the true value.
+__device__ __forceinline__ float gated(float a, float x) {
+    const float t = expf(-fabsf(x));
+    return __fdividef(x < 0.f ? a * t : a, 1.f + t);
 }
 
 // the low n bits
@@ -576,11 +552,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             if (p.sinks != nullptr) sink = p.sinks[head] * LOG2E;
             dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
             if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
-            if (GATE == GATE_HEAD) {
-                float none = 1.f;
-                const float x = __bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]);
-                gate_pair(gate_f, none, x, x);
-            }
+            if (GATE == GATE_HEAD)
+                gate_f = gated(1.f, __bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]));
         }
         if (!p.q_boxes && n_tiles > 0) {
             // group sizes whose tiles would leave much of the 128 rows empty: the rows by hand,
@@ -745,8 +718,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     const uint4 raw = *reinterpret_cast<const uint4*>(from);
                     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
 #pragma unroll
-                    for (int i = 0; i < 8; i += 2)
-                        gate_pair(o[8 * q4 + i], o[8 * q4 + i + 1], __bfloat162float(g[i]), __bfloat162float(g[i + 1]));
+                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] = gated(o[8 * q4 + i], __bfloat162float(g[i]));
                 }
                 if (GATE == GATE_HEAD) {
 #pragma unroll

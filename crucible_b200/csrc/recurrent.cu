@@ -710,13 +710,20 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 }
                 sums[2 * NC] = (kq[0] + kq[1]) + (kq[2] + kq[3]);
                 lanes_summed<LANES>(sums);
-                float o[NC];
+                // (where the results are summed up changes what the compiler takes ahead: with one column here 300 tokens of 8
+                // heads of 128 77.5 us, in the branch 76.4; with two in the branch 1 % slower)
+                if constexpr (NC == 1) {
+                    u_prev[0] = beta * (v[0] - decay * sums[0]);
+                    if (live && part == 0) out[out_at] = fmaf(u_prev[0], sums[2], decay * sums[1]);
+                } else {
+                    float o[NC];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    u_prev[c] = beta * (v[c] - decay * sums[2 * c]);
-                    o[c] = fmaf(u_prev[c], sums[2 * NC], decay * sums[2 * c + 1]);
+                    for (int c = 0; c < NC; ++c) {
+                        u_prev[c] = beta * (v[c] - decay * sums[2 * c]);
+                        o[c] = fmaf(u_prev[c], sums[2 * NC], decay * sums[2 * c + 1]);
+                    }
+                    if (live && part == 0) store_columns<NC>(out + out_at, o);
                 }
-                if (live && part == 0) store_columns<NC>(out + out_at, o);
 #pragma unroll
                 for (int i = 0; i < P; ++i) k_prev[i] = kk[i];
                 g_prev = decay;
@@ -751,13 +758,14 @@ __global__ void __launch_bounds__(THREADS) matrix_memory_kernel(
                 }
                 sums[2 * NC] = (kq[0] + kq[1]) + (kq[2] + kq[3]);
                 lanes_summed<LANES>(sums);
-                float o[NC];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    u_prev[c] = beta * (v[c] - sums[2 * c]);
-                    o[c] = fmaf(u_prev[c], sums[2 * NC], sums[2 * c + 1]);
+                for (int c = 0; c < NC; ++c) u_prev[c] = beta * (v[c] - sums[2 * c]);
+                if (live && part == 0) {
+                    float o[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) o[c] = fmaf(u_prev[c], sums[2 * NC], sums[2 * c + 1]);
+                    store_columns<NC>(out + out_at, o);
                 }
-                if (live && part == 0) store_columns<NC>(out + out_at, o);
 #pragma unroll
                 for (int i = 0; i < P; ++i) k_prev[i] = kk[i];
             } else if (RULE == RULE_WKV || RULE == RULE_SSD) {

@@ -35,12 +35,13 @@ def walk_columns(rule, requests: int, rows: int, longest: int, n_heads: int, key
     the token's k and q out of shared memory, which is what many portions wait for: with 2 or 4 columns a
     lane half or a quarter of it, and the state's rows come in 8 or 16 bytes; but fewer blocks, and a token of a
     lone portion takes longer.  32 portions of up to 24 tokens, 16 heads of 128, with 1, 2 and 4: delta rule 78, 61
-    and 57 us, state space 67, 50 and 48; one of 90 27, 28 and 41, 21, 23 and 33.  Up to a block an SM one is
-    taken, else what costs least: of 347 steps measured 1.4 % from the quickest on average."""
+    and 57 us, state space 67, 50 and 48; one of 90 27, 28 and 41, 21, 23 and 33.  Up to a block an SM, and where
+    nobody knows the longest portion (0), one is taken, else what costs least: of 347 steps measured 1.4 % from the
+    quickest on average."""
     heads = n_heads * key_dim / 128
     cost = {c: start + token * longest + (work * rows + portion * requests) * heads
             for c, (start, token, work, portion) in COSTS[rule][0].items()}
-    if requests * n_heads * -(-value_dim // 16) <= 148:
+    if longest <= 0 or requests * n_heads * -(-value_dim // 16) <= 148:
         return 1, cost[1]
     return min((us, c) for c, us in cost.items())[::-1]
 
@@ -254,7 +255,8 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
     sp, stride = _state_args(state)
     n, walked = ctx.n_requests, ctx.n_requests
     # (without the host's counts of the step, or in 32 bits: the walk alone)
-    host = getattr(ctx, "host", None) if getattr(ctx, "dtype", None) == torch.bfloat16 else None
+    counts = getattr(ctx, "host", None)
+    host = counts if getattr(ctx, "dtype", None) == torch.bfloat16 else None
     starts, slots, kept_at = (t.data_ptr() if t is not None else 0 for t in (ctx.req_row_start, ctx.req_state_slot, kept))
     w_off_read = w_off if rule in (WKV, CHANNEL) else 0
     if (CHUNKS and host is not None and chunks_pay(
@@ -297,8 +299,8 @@ def matrix_memory(rule, qkv, q_off, k_off, v_off, sc0, sc1, ctx, state, s_off, n
             _ptr(per_head), kept_at, _stream())
     code = lib.cb_matrix_memory_step(*args) if step else build.UNSUPPORTED
     if code == build.UNSUPPORTED:
-        longest = 1 if host is None or walked < n else host.max_new_tokens
-        columns = walk_columns(rule, walked, walked if walked < n else qkv.shape[0], longest, n_heads, key_dim, value_dim)[0]
+        rows, longest = ((walked, 1) if walked < n else (qkv.shape[0], counts.max_new_tokens if counts is not None else 0))
+        columns = walk_columns(rule, walked, rows, longest, n_heads, key_dim, value_dim)[0]
         code = lib.cb_matrix_memory(*args[:-1], columns, args[-1])
     _check(code, "matrix_memory")
 

@@ -1,0 +1,55 @@
+"""Which form of the walk over tokens a step is given (no GPU: the entry points are stand-ins)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+STEPS = [([700, 123, 246], 8, 128), ([700, 123], 16, 128), ([300, 300], 16, 128), ([450] * 4, 8, 128), ([600, 410, 520], 16, 64),
+         ([300, 700, 410, 520, 333], 8, 128), ([300, 700, 410, 520, 333], 16, 128), ([600] + [1] * 12, 16, 128),
+         ([24] * 32, 16, 128), ([1] * 32, 8, 128)]
+
+
+def _columns(rule, lengths, H, D, dtype, counts, monkeypatch):
+    """What `matrix_memory` asks of the walk for portions of `lengths`."""
+    from crucible_b200.engine.context import HostStep
+    from crucible_b200.ops import build, recurrent as k
+    seen = []
+    lib = SimpleNamespace(cb_matrix_memory=lambda *a: seen.append(a[-2]) or 0,
+                          cb_matrix_memory_step=lambda *a: build.UNSUPPORTED)
+    monkeypatch.setattr(k.build, "load", lambda name: lib)
+    monkeypatch.setattr(k, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(k, "_stream", lambda: 0)
+    monkeypatch.setattr(k, "CHUNKS", False)
+    R, T = len(lengths), sum(lengths)
+    vector = rule in (k.WKV, k.CHANNEL)
+    numbers = torch.zeros(T, H)
+    starts = torch.zeros(R + 1, dtype=torch.int32)
+    held = [5] * R
+    ctx = SimpleNamespace(n_requests=R, n_tokens=T, req_row_start=starts, req_state_slot=starts, dtype=dtype,
+                          host=HostStep(list(range(R)), lengths, held, [5 + n for n in lengths], held) if counts else None)
+    k.matrix_memory(rule, torch.zeros(T, 3 * H * D + H * D * vector), 0, H * D, 2 * H * D, numbers, numbers, ctx,
+                    torch.zeros((R, 4 * (H * D * D + H * D + H)), dtype=torch.uint8), 0, 4 * H * D * D, 4 * H * D * (D + 1),
+                    torch.empty(T, H * D), H, H, D, D, w_off=3 * H * D, kept=torch.zeros(R, H * (D + 1)))
+    return seen
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
+@pytest.mark.parametrize("lengths,H,D", STEPS)
+def test_a_step_is_walked_in_the_form_its_lengths_ask_for(rule, lengths, H, D, dtype, monkeypatch):
+    """In 32 bits (which always walk) as in 16: by the portions' number, tokens and longest."""
+    from crucible_b200.ops import recurrent as k
+    code = getattr(k, rule)
+    got = _columns(code, lengths, H, D, dtype, True, monkeypatch)
+    assert got == [k.walk_columns(code, len(lengths), sum(lengths), max(lengths), H, D, D)[0]]
+    if len(lengths) * H * (D // 16) <= 148:
+        assert got == [1]                              # up to a block an SM
+    elif max(lengths) >= 300 and sum(lengths) < 2 * max(lengths) and rule in ("DELTA", "MLSTM", "CHANNEL"):
+        assert got[0] < 4                              # (four take half as long again over a long portion)
+
+
+@pytest.mark.parametrize("rule", ["DELTA", "MLSTM", "WKV", "SSD", "CHANNEL"])
+def test_portions_of_unknown_length_have_a_column_a_lane(rule, monkeypatch):
+    from crucible_b200.ops import recurrent as k
+    for dtype in (torch.float32, torch.bfloat16):
+        assert _columns(getattr(k, rule), [700, 123, 246], 8, 128, dtype, False, monkeypatch) == [1]

@@ -36,14 +36,20 @@ def walk_columns(rule, requests: int, rows: int, longest: int, n_heads: int, key
     lane half or a quarter of it, and the state's rows come in 8 or 16 bytes; but fewer blocks, and a token of a
     lone portion takes longer.  32 portions of up to 24 tokens, 16 heads of 128, with 1, 2 and 4: delta rule 78, 61
     and 57 us, state space 67, 50 and 48; one of 90 27, 28 and 41, 21, 23 and 33.  Up to a block an SM, and where
-    nobody knows the longest portion (0), one is taken, else what costs least: of 347 steps measured 1.4 % from the
-    quickest on average."""
+    nobody knows the longest portion (0), one is taken, else what costs least, if that is clearly less than one costs:
+    by a twentieth; by more than a fifth where one portion is over a third of the rows, whose blocks, dealt out between
+    the others', come to lie on a few of the SMs (portions of 180, 130, 75, 40, 9 and 1, 16 heads of 128 by the delta rule,
+    1 and 2: reckoned 83 and 75 us, measured 86 and 98).  The mLSTM's one column has three blocks of 128 channels an SM, not
+    four: an eighth (330 and 290, 32 heads: 218 and 149).  Of 500 steps measured 4 are more than 1.5 % behind one
+    column as it was before there were more (up to 4 %), the mean 11 % ahead."""
     heads = n_heads * key_dim / 128
     cost = {c: start + token * longest + (work * rows + portion * requests) * heads
             for c, (start, token, work, portion) in COSTS[rule][0].items()}
-    if longest <= 0 or requests * n_heads * -(-value_dim // 16) <= 148:
+    us, columns = min((us, c) for c, us in cost.items())
+    clearly = 0.95 if rows >= 3 * longest else 0.87 if rule == MLSTM else 0.78
+    if longest <= 0 or requests * n_heads * -(-value_dim // 16) <= 148 or us > clearly * cost[1]:
         return 1, cost[1]
-    return min((us, c) for c, us in cost.items())[::-1]
+    return columns, us
 
 
 def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bool:

@@ -53,3 +53,14 @@ def test_portions_of_unknown_length_have_a_column_a_lane(rule, monkeypatch):
     from crucible_b200.ops import recurrent as k
     for dtype in (torch.float32, torch.bfloat16):
         assert _columns(getattr(k, rule), [700, 123, 246], 8, 128, dtype, False, monkeypatch) == [1]
+
+
+@pytest.mark.parametrize("rule,lengths,H,D,columns", [
+    # (measured: the quickest of one, two and four)
+    ("DELTA", [180, 1, 75, 40, 9, 130], 16, 128, 1), ("SSD", [180, 1, 75, 40, 9, 130], 16, 128, 1), ("DELTA", [900, 300, 300, 300], 32, 128, 1),
+    ("WKV", [600] + [1] * 12, 16, 64, 1), ("WKV", [400, 1, 1, 1], 32, 128, 1), ("DELTA", [300, 700, 410, 520, 333], 16, 64, 1),
+    ("DELTA", [300, 700, 410, 520, 333], 8, 128, 1), ("MLSTM", [330, 290], 32, 128, 2), ("DELTA", [450] * 4, 16, 128, 2),
+    ("MLSTM", [450] * 4, 16, 128, 2), ("SSD", [24] * 32, 16, 128, 4)])
+def test_more_columns_only_where_they_are_clearly_quicker(rule, lengths, H, D, columns):
+    from crucible_b200.ops import recurrent as k
+    assert k.walk_columns(getattr(k, rule), len(lengths), sum(lengths), max(lengths), H, D, D)[0] == columns

@@ -30,7 +30,7 @@ COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS,
 
 
 @functools.lru_cache(maxsize=4096)
-def walk_columns(rule, requests: int, rows: int, longest: int, n_heads: int, key_dim: int, value_dim: int):
+def walk_columns(rule, requests: int, rows: int, longest: int, n_heads: float, key_dim: int, value_dim: int):
     """How many columns of its matrix a lane of the walk takes, and the walk's us.  Every lane of a column's eight reads
     the token's k and q out of shared memory, which is what many portions wait for: with 2 or 4 columns a
     lane half or a quarter of it, and the state's rows come in 8 or 16 bytes; but fewer blocks, and a token of a
@@ -72,8 +72,7 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
     elif longest < 160 and (longest < 48 or rows < 24 * requests or rows * heads < 4096):
         return False
     first, chunk = COSTS[rule][1]
-    walk = min(start + token * longest + (work * rows + portion * requests) * heads
-               for start, token, work, portion in COSTS[rule][0].values())
+    walk = walk_columns(rule, requests, rows, longest, heads, 128, 128)[1]      # of the form that would be launched
     return walk > 0.95 * (first + chunk * (rows / 32 + requests / 2) * heads)
 
 

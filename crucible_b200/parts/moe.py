@@ -32,7 +32,7 @@ import torch
 
 from .. import ops
 from ..config.model_config import FeedForwardSpec
-from ..ops import moe as kernels
+from ..ops import moe as kernels, tensor_core
 from ..ops.layer_close import OpenSum
 from .base import FEED_FORWARDS, FeedForward, TensorDecl
 from .swiglu import SwiGLU
@@ -111,11 +111,8 @@ class MixtureOfExperts(FeedForward):
     RIDE_GROUPED_ROWS = 32       # the same where the experts run as grouped products (a decode step of 16 rows,
                                  # 4 layers of width 1024: 0.379 -> 0.347 ms; at 64 rows of width 2048 no gain)
     RIDE_PLAIN_ROWS = 128        # ... and one that does not join them otherwise (width 2,048, layer apart and riding: 8 rows
-                                 # 87 and 78 us, 32 93 and 81, 128 96 and 84, 192 99 and 105)
-    # Of one slice it rides on, two launches less and no second last wave: with experts of less than 16 MB at once (1,408 x
-    # 1,024, 8 of top 2: 200 rows 47 and 42 us, 650 65 and 56, 1,900 95 and 93), of more from 320 rows on (2,816 x 2,048: 230
-    # rows 96 and 98, 360 107 and 93, 1,150 167 and 156, 1,500 185 and 194, 2,048 223 and 218).
-    RIDE_LARGE_FROM, RIDE_LONG_ROWS = 320, 2048
+                                 # 87 and 78 us, 32 93 and 81, 128 96 and 84, 192 99 and 105); of one slice beyond them, too,
+                                 # where the products' waves say so (`tensor_core.riding_pays`)
     RIDE_MAX_ROWS = 2            # up to this many bfloat16 rows a joining shared expert rides with the routed ones
 
     def __init__(self, spec: FeedForwardSpec):
@@ -239,14 +236,14 @@ class MixtureOfExperts(FeedForward):
 
     def _rides(self, t: int) -> bool:
         """Whether a shared expert that does not join the others' sum rides with them all the same: in grouped
-        products of up to `RIDE_PLAIN_ROWS` rows, beyond them if it is one slice (`RIDE_LARGE_FROM`), or beside a
-        token or two."""
+        products of up to `RIDE_PLAIN_ROWS` rows, beyond them if it is one slice and its tiles fill waves that are there
+        (`riding_pays`), or beside a token or two."""
         if self.shared is None or self.slices == 0:
             return False
         if not self._grouped(t):
             return t <= self.RIDE_MAX_ROWS
-        return t <= self.RIDE_PLAIN_ROWS or (self.slices == 1 and t <= self.RIDE_LONG_ROWS and (
-            t >= self.RIDE_LARGE_FROM or 6 * self.spec.width * self.ff < 16 << 20))
+        return t <= self.RIDE_PLAIN_ROWS or (
+            self.slices == 1 and tensor_core.riding_pays(t, self.spec.width, self.ff, self.n, self.top))
 
     @functools.cached_property
     def _least_pairs(self) -> int:

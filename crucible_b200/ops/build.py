@@ -2,7 +2,8 @@
 each at its first use.
 
 `nvcc -gencode arch=compute_100a,code=sm_100a -shared` straight to a `.so` that
-is loaded with ctypes; there is no framework header in the kernels, so a file
+is loaded with ctypes, whose functions a small extension module then calls (`csrc/host_call.cpp`; ctypes itself
+where that module cannot be had); there is no framework header in the kernels, so a file
 compiles in seconds.  The library is kept beside the package (`lib/`) under a
 name that carries a hash of its sources and flags, so a changed source is
 rebuilt and a fresh checkout compiles only what the model at hand needs.  If
@@ -40,9 +41,11 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", 
 # Host-only sources (C++, no device code): compiled by the same nvcc call, which hands them
 # to the host compiler.
 HOST_SOURCES = {"host_step": "host_step.cpp", "host_cache": "host_cache.cpp", "host_call": "host_call.cpp"}
-# `host_call` is an extension of the interpreter: without its headers (or on another machine than
-# x86-64 Linux) the kernels' entry points are called through ctypes alone.
+# `host_call` is an extension of the interpreter: without its headers, where it cannot be built or loaded, or on
+# another machine than x86-64 Linux, the kernels' entry points are called through ctypes alone.  Its file carries the
+# interpreter's own tag (a debug or free-threaded one lays its objects out differently).
 PYTHON_INCLUDE = sysconfig.get_paths()["include"]
+PYTHON_TAG = sysconfig.get_config_var("SOABI") or sys.implementation.cache_tag or "python"
 NATIVE_CALLS = (platform.machine() == "x86_64" and sys.platform.startswith("linux") and sys.implementation.name == "cpython"
                 and os.path.exists(os.path.join(PYTHON_INCLUDE, "Python.h")))
 
@@ -94,7 +97,7 @@ def _digest(name: str) -> str:
     h = hashlib.sha256()
     h.update(" ".join(NVCC_FLAGS).encode())
     if name == "host_call":
-        h.update(sys.implementation.cache_tag.encode())
+        h.update(PYTHON_TAG.encode())
     for fn in [_source(name)] + MODULES[name]:
         with open(os.path.join(CSRC, fn), "rb") as f:
             h.update(fn.encode())
@@ -124,7 +127,8 @@ def library_path(name: str) -> str:
     """Path of the built library of module `name`, building it if needed."""
     if name not in MODULES:
         raise BuildError(f"no CUDA module named {name!r}; known: {sorted(MODULES)}")
-    fname = f"cb_{name}-{_digest(name)}.so"
+    stem = f"cb_{name}.{PYTHON_TAG}-" if name == "host_call" else f"cb_{name}-"
+    fname = f"{stem}{_digest(name)}.so"
     in_tree = os.path.join(_LIB_DIR, fname)
     if os.path.exists(in_tree):
         return in_tree
@@ -133,7 +137,7 @@ def library_path(name: str) -> str:
     if os.path.exists(target):
         return target
     for old in os.listdir(out_dir):
-        if old.startswith(f"cb_{name}-") and old.endswith(".so"):
+        if old.startswith(stem) and old.endswith(".so"):
             try:
                 os.remove(os.path.join(out_dir, old))
             except OSError:
@@ -199,17 +203,24 @@ def signatures(text: str) -> Dict[str, tuple]:
 _KINDS = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_long: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
 
 
+_calls: List[object] = []       # the extension module, or None where it cannot be had; empty: not asked for yet
+
+
 def _native_calls():
     """The extension module that calls entry points (`csrc/host_call.cpp`), or None."""
     if not NATIVE_CALLS:
         return None
-    module = _loaded.get("host_call")
-    if module is None:
-        loader = importlib.machinery.ExtensionFileLoader("cb_host_call", library_path("host_call"))
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("cb_host_call", loader))
-        loader.exec_module(module)
-        _loaded["host_call"] = module
-    return module
+    if not _calls:
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("cb_host_call", library_path("host_call"))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("cb_host_call", loader))
+            loader.exec_module(module)
+        except (BuildError, ImportError, OSError) as e:
+            print(f"[crucible_b200] host_call is not to be had, entry points go through ctypes: {e}",
+                  file=sys.stderr, flush=True)
+            module = None
+        _calls.append(module)
+    return _calls[0]
 
 
 def load(name: str) -> ctypes.CDLL:
@@ -238,4 +249,5 @@ def load(name: str) -> ctypes.CDLL:
 
 
 def build_all() -> List[str]:
-    return [library_path(name) for name in sorted(MODULES)]
+    """Builds every module; `host_call`, which the others do without, where it can be had."""
+    return [library_path(name) for name in sorted(MODULES) if name != "host_call" or _native_calls() is not None]

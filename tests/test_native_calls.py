@@ -72,3 +72,39 @@ def test_threads_call_side_by_side():
     for t in threads:
         t.join()
     assert sorted(seen, key=lambda a: a[0]) == [(i, 0.5 * i, None) for i in range(6) for _ in range(200)]
+
+
+@pytest.mark.parametrize("fails", ["build", "load", "file"])
+def test_without_the_module_entry_points_go_through_ctypes(fails, monkeypatch, tmp_path, capfd):
+    """Headers that are there and do not compile, a module that does not load, a folder that cannot be read: kernels load
+    all the same, and one line says so."""
+    real = build.library_path
+
+    def library_path(name):
+        if name != "host_call":
+            return real(name)
+        if fails == "build":
+            raise build.BuildError("nvcc failed on host_call.cpp")
+        if fails == "file":
+            raise PermissionError(13, "no")
+        (tmp_path / "cb_host_call.so").write_bytes(b"no library")
+        return str(tmp_path / "cb_host_call.so")
+    monkeypatch.setattr(build, "library_path", library_path)
+    monkeypatch.setattr(build, "_calls", [])
+    monkeypatch.setattr(build, "_loaded", {})
+    lib = build.load("recurrent")
+    assert isinstance(lib.cb_matrix_memory, ctypes._CFuncPtr) and lib.cb_matrix_memory.argtypes
+    build.load("streams")
+    assert capfd.readouterr().err.count("entry points go through ctypes") == 1
+    assert all("host_call" not in path for path in build.build_all())
+
+
+def test_the_module_is_this_interpreters(monkeypatch):
+    """Another interpreter's build lies beside this one's, under a name and digest of its own."""
+    import os
+    mine = build.library_path("host_call")
+    assert f"cb_host_call.{build.PYTHON_TAG}-" in os.path.basename(mine)
+    digest = build._digest("host_call")
+    monkeypatch.setattr(build, "PYTHON_TAG", "cpython-399td-x86_64-linux-gnu")
+    assert build._digest("host_call") != digest
+    assert "host_call" not in build._loaded or isinstance(build._loaded["host_call"], ctypes.CDLL)

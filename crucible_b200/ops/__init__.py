@@ -502,11 +502,12 @@ F32_TILES = True          # tests switch it off to reach the one-warp-a-row kern
 def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                   chunked, keep_first, out_scale, ctx, page_tokens, table, gate_per_head=False) -> bool:
     """The 32-bit attention over tiles of keys (`csrc/attention_f32.cu`): float32 rows of sizes up to 256
-    that are multiples of 4.  A rule of the sizes alone, so that a row's bits never depend on the
-    step.  False: not taken."""
+    that are multiples of 4, from a pool whose rows an int counts (the kernel keeps where a key lies as one).  A rule of
+    the sizes alone, so that a row's bits never depend on the step.  False: not taken."""
     host = getattr(ctx, "host", None)
     tensors = (q, out, k_cache, v_cache)
     if (not F32_TILES or host is None or any(t.dtype != torch.float32 for t in tensors)
+            or max(k_cache.shape[0], v_cache.shape[0]) * n_kv_heads * page_tokens >= 1 << 31
             or max(key_dim, value_dim) > 256 or (key_dim | value_dim | q.stride(0) | out.stride(0)) % 4
             or any(t.data_ptr() % 16 for t in tensors) or (gate is not None and gate.dtype != torch.float32)):
         return False

@@ -53,3 +53,23 @@ def test_a_steps_key_tells_short_contexts_apart():
     assert step([1, 1, 500], [100, 128, 0]).shape_key() == (500, 2, 0, 256)
     prompts = step([70], [0])
     assert prompts.lead_context_reach == 0 and prompts.shape_key() == (70, 0, 0, 0)
+
+
+@pytest.mark.parametrize("pages,heads,page,taken", [
+    (64, 4, 16, True), ((1 << 31) // 64 - 1, 4, 16, True), ((1 << 31) // 64, 4, 16, False), (1 << 25, 16, 32, False)])
+def test_32_bit_tiles_take_pools_whose_rows_an_int_counts(pages, heads, page, taken, monkeypatch):
+    """Where a key lies is kept as an int, the row of the pool; a pool with more rows than that (heads of 4: from 34 GB on)
+    goes by the kernels that reckon in 64 bits."""
+    from types import SimpleNamespace
+    import torch
+    from crucible_b200 import ops
+    calls = []
+    monkeypatch.setattr(ops.build, "load", lambda name: SimpleNamespace(cb_attention_f32=lambda *a: calls.append(a) or 0))
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "_ptr", lambda t: 0)
+    pool = torch.zeros(4).expand(pages, heads, page, 4)              # (its size alone is real)
+    rows, numbers = torch.zeros(3, 4 * heads), torch.zeros(4, dtype=torch.int32)
+    ctx = SimpleNamespace(host=SimpleNamespace(max_new_tokens=3), req_row_start=numbers, req_first_pos=numbers, n_requests=1)
+    got = ops.attention_f32(rows, None, torch.zeros(3, 4 * heads), pool, pool, None, heads, heads, 4, 4, 0.5, None, False, 0, 1.0,
+                            ctx, page, torch.zeros((1, 4), dtype=torch.int32))
+    assert got == taken and len(calls) == taken

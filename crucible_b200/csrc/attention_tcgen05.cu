@@ -28,7 +28,7 @@
 // exponentials: set half a tile apart the groups were no faster (17.9 and 17.9), in turns slower (18.5), and a quarter
 // of the exponentials on the FMA pipe gave 2 %, 7 % less where most blocks are short.
 // Measured on one B200, replayed, a 2,048-token prompt: 12 heads of 64 on 4 17.8 us a layer (27 with P in shared
-// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 26.3 (58), 16
+// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 26.5 (58), 16
 // heads of 256 on 1 30.8 (76).
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
@@ -181,13 +181,14 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return d;
 }
 
-// a times sigmoid(x) = 1 / (1 + e^-x), by t = e^-|x|: 1 / (1 + t), or t / (1 + t) for x < 0.  So the denominator is 1 to
-// 2, where the approximate division has its two units in the last place (its IEEE form, inlined 32 times, is what a block
-// would wait for at its end: 16 heads of 128, a window of 1,024, 2,048 tokens 32.9 us a layer with it, 26.3 so), and
-// a logit far below zero keeps its digits: all 65,536 logits give the bf16 nearest to the true value.
-__device__ __forceinline__ float gated(float a, float x) {
+// 1 / (1 + e^-x), by t = e^-|x|: 1 / (1 + t), or t / (1 + t) for x < 0.  So the denominator is 1 to 2, where
+// the approximate division has its two units in the last place (its IEEE form, inlined 32 times, is what a block would wait
+// for at its end: 16 heads of 128, a window of 1,024, 2,048 tokens 32.9 us a layer with it, 26.5 so), and a logit
+// far below zero keeps its digits: all 65,536 logits give the bf16 nearest to the true value.  A factor of its own, so
+// that a logit a head and the same logit at each of its features give the same bits.
+__device__ __forceinline__ float sigmoid(float x) {
     const float t = expf(-fabsf(x));
-    return __fdividef(x < 0.f ? a * t : a, 1.f + t);
+    return __fdividef(x < 0.f ? t : 1.f, 1.f + t);
 }
 
 // the low n bits
@@ -553,7 +554,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             dst = p.out + (size_t)tok * p.out_stride + (size_t)head * HD;
             if (GATE == GATE_RESULT) gate = p.gate + (size_t)tok * p.gate_stride + (size_t)head * HD;
             if (GATE == GATE_HEAD)
-                gate_f = gated(1.f, __bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]));
+                gate_f = sigmoid(__bfloat162float(p.gate[(size_t)tok * p.gate_stride + head]));
         }
         if (!p.q_boxes && n_tiles > 0) {
             // group sizes whose tiles would leave much of the 128 rows empty: the rows by hand,
@@ -718,7 +719,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                     const uint4 raw = *reinterpret_cast<const uint4*>(from);
                     const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(&raw);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] = gated(o[8 * q4 + i], __bfloat162float(g[i]));
+                    for (int i = 0; i < 8; ++i) o[8 * q4 + i] *= sigmoid(__bfloat162float(g[i]));
                 }
                 if (GATE == GATE_HEAD) {
 #pragma unroll

@@ -387,16 +387,14 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 pg0 = pg1, pg1 = pg2, pg2 = lookup(j + 3);
             }
         } else if (ok) {
-            int pg3 = S_BUFS > 2 ? lookup(3) : 0;
+            int pg3 = lookup(3);
             ok = send(pg0, false, 0);
             if (ok && n_tiles > 1) ok = send(pg1, false, 0);
-            if (S_BUFS > 2 && ok && n_tiles > 2) ok = send(pg2, false, 0);
+            if (ok && n_tiles > 2) ok = send(pg2, false, 0);
             for (int j = 0; j < n_tiles && ok; ++j) {
                 ok = send(pg0, true, 0);
-                if (ok && j + S_BUFS < n_tiles) ok = send(S_BUFS > 2 ? pg3 : pg2, false, 0);
-                pg0 = pg1, pg1 = pg2;
-                if (S_BUFS > 2) pg2 = pg3, pg3 = lookup(j + 4);
-                else pg2 = lookup(j + 3);
+                if (ok && j + S_BUFS < n_tiles) ok = send(pg3, false, 0);
+                pg0 = pg1, pg1 = pg2, pg2 = pg3, pg3 = lookup(j + 4);
             }
         }
         bool gate_sent = false;
@@ -478,8 +476,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 if (sender) {
                     tc::umma_commit(&s.s_full[to]);
                     if (NARROW) tc::umma_commit(&s.empty[3]);
-                    // pairs: K0 and K1; with two buffers V_(j-2) and K_j, with three K_(t+2) and V_t
-                    if (!BOTH && (S_BUFS == 2 ? j > 0 : j == 1)) tc::umma_commit(&s.empty[(j - 1) % Store::RELEASES]);
+                    if (!BOTH && j == 1) tc::umma_commit(&s.empty[0]);      // the pairs: K0 and K1, then K_(t+2) and V_t
                 }
                 if (++to == S_BUFS) to = 0;
                 return true;
@@ -515,7 +512,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                 if (sender) {
                     if (BOTH) tc::umma_commit(&s.pv_done[t & 1]);
                     // (not after the last tile: the loader may still be about to ask for this barrier's phase before)
-                    if (S_BUFS == 3 && t + 1 < n_tiles) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
+                    if (!BOTH && t + 1 < n_tiles) tc::umma_commit(&s.empty[(t + 1) % Store::RELEASES]);
                     if (t == n_tiles - 1) tc::umma_commit(&s.o_done);
                 }
                 return true;

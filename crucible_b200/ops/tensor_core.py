@@ -12,7 +12,6 @@ from __future__ import annotations
 import ctypes
 import functools
 import math
-import os
 
 import torch
 
@@ -684,11 +683,6 @@ def linear_rope_append(h, wqkv, qkv, n_heads, n_kv_heads, head_dim, cos, sin, ro
         raise RuntimeError(f"tensor-core q/k/v product failed to launch (CUDA error {code})")
     _count(1)
     return True
-
-
-# The prompt attention had a second form of head size 64, which callers could fix here; it has one now, and
-# the value is taken and not read.
-ATTENTION_LEAN = -1
 
 
 class _Requests:

@@ -692,13 +692,11 @@ def test_attention_tensor_core_tiles_and_split(case):
     (4, 4, 64, 32, [(0, 700)], None),
     (6, 1, 64, 8, [(513, 300), (0, 129)], None),
     (8, 2, 64, 128, [(100, 260)], 200),
-    (4, 2, 128, 16, [(0, 600), (40, 70)], None),            # head size 128: two stages, one P buffer
+    (4, 2, 128, 16, [(0, 600), (40, 70)], None),            # head size 128: one accumulator for both groups
     (2, 1, 128, 64, [(300, 420)], 256),
 ])
-@pytest.mark.parametrize("lean", [0, 1])
-def test_attention_tcgen05_matches_reference_and_mma(case, lean):
-    """Prompt portions with head size 64 or 128: S and O in tensor memory, K and V by TMA; for
-    head size 64 both forms of the kernel (an SM to a block, or two lean blocks to an SM)."""
+def test_attention_tcgen05_matches_reference_and_mma(case):
+    """Prompt portions with head size 64 or 128: S, P and O in tensor memory, queries, K and V by TMA."""
     from crucible_b200.ops import tensor_core
     n_heads, n_kv, hd, page, requests, window = case
     qkv, ctx, cache, binding, ref = _paged_case(torch.bfloat16, n_heads, n_kv, hd, page, requests,
@@ -707,14 +705,10 @@ def test_attention_tcgen05_matches_reference_and_mma(case, lean):
     cache.n_pages = k_cache.shape[0]
     out = torch.zeros(qkv.shape[0], n_heads * hd, device=DEV, dtype=torch.bfloat16)
     assert tensor_core.USE_TCGEN05_ATTENTION
-    try:
-        tensor_core.ATTENTION_LEAN = lean
-        whole = tensor_core._Requests(ctx, ctx.block_table(0), 0, ctx.n_requests,
-                                      ctx.host.max_new_tokens, ctx.host.context_bucket, ctx.n_tokens)
-        assert tensor_core._attention_tcgen05(qkv, out, k_cache, cache.values(0), whole, n_heads, n_kv,
-                                              hd, 1 / math.sqrt(hd), window, cache)
-    finally:
-        tensor_core.ATTENTION_LEAN = -1
+    whole = tensor_core._Requests(ctx, ctx.block_table(0), 0, ctx.n_requests,
+                                  ctx.host.max_new_tokens, ctx.host.context_bucket, ctx.n_tokens)
+    assert tensor_core._attention_tcgen05(qkv, out, k_cache, cache.values(0), whole, n_heads, n_kv,
+                                          hd, 1 / math.sqrt(hd), window, cache)
     torch.cuda.synchronize()
     tensor_core.check_status(DEV)
     assert rel(out, ref) < 1.5e-2

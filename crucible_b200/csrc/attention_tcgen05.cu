@@ -27,9 +27,10 @@
 // maxima 400, the way to and from the barriers 400), at which the other group is not always busy with its
 // exponentials: set half a tile apart the groups were no faster (17.9 and 17.9), in turns slower (18.5), and a quarter
 // of the exponentials on the FMA pipe gave 2 %, 7 % less where most blocks are short.
-// Measured on one B200, replayed, a 2,048-token prompt: 12 heads of 64 on 4 17.8 us a layer (27 with P in shared
-// memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a gate 26.5 (58), 16
-// heads of 256 on 1 30.8 (76).
+// Measured on one B200, a captured chain of this launch by itself, a 2,048-token prompt: 12 heads of 64 on 4 17.7 us a
+// layer (27 with P in shared memory and the rows fetched by hand), 16 heads of 128 on 4, a window of 1,024 and a
+// gate 26.5 (58), 16 heads of 256 on 1 30.8 (76), of which 192 features are values 28.5.  (A launch that begins cold, with
+// nothing ahead of it, takes 21 of the first.)
 //
 // Running maximum: a row keeps a reference maximum that is only raised when the
 // tile's maximum exceeds it by more than 2^8 (in the base-2 exponent), so P

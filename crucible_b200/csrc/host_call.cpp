@@ -1,5 +1,5 @@
-// Calls of the kernels' entry points from Python.  ctypes makes an object for every argument: a launch of 25 cost
-// the host 4.2 us that way, 0.3 here, and an eager layer is ten launches.  A `Call` keeps an entry point's address and
+// Calls of the kernels' entry points from Python.  ctypes makes an object for every argument: a launch of 26 cost
+// the host 3.3 us that way, 0.34 here, and an eager layer is ten launches.  A `Call` keeps an entry point's address and
 // the kinds of its parameters, reads plain numbers and None straight from the interpreter's argument vector, and
 // leaves everything else (other types, a wrong number of arguments, and with it the errors) to the ctypes
 // function that it was made from.

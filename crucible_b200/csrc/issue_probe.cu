@@ -1,6 +1,7 @@
 // What it costs one thread to send work to the tensor cores and to the TMA unit on this GPU:
-// two probes whose figures the tensor-core kernels' loops were shaped by (a narrow tile's step
-// of K is what its MMA thread can send, not what the tensor cores or the memory can do).
+// two probes whose figures the tensor-core kernels' loops were shaped by, for a sender picked by its number (a narrow
+// tile's step of K is then much of what its MMA thread can send).  The kernels have since elected their senders
+// (`elect_one`, tc_common.cuh), which keeps descriptors in uniform registers and takes less; the loops stayed.
 //
 //   cb_probe_mma_send: one thread sends `count` tcgen05.mma of M x N x 16 (bf16, operands
 //     resident in shared memory, one accumulator) back to back, commits and waits; returns
@@ -9,7 +10,7 @@
 //   cb_probe_tma_send: one thread sends `count` 2-D boxes of `rows` x 128 bytes (128-byte
 //     swizzle) from a matrix in global memory to shared memory, one barrier armed once for
 //     all bytes; returns cycles per box for the sending loop and until all have landed.
-//   Measured on B200: 54 cycles per MMA for tiles up to 64 columns (64 at 128, 128 at 256: there
+//   Measured on B200, `tid == 0` sending: 54 cycles per MMA for tiles up to 64 columns (64 at 128, 128 at 256: there
 //   the tensor cores' own time), 60 cycles per box of up to 64 rows, 97 for 128 rows.
 //
 // One block, a few microseconds; every wait is bounded and tensor memory is freed on all

@@ -1,7 +1,7 @@
 """The operations the parts are written in, each a hand-written CUDA kernel.
 
 Every function here launches on the current CUDA stream of torch and returns at
-once.  Tensors are passed as raw device pointers through ctypes; shapes, dtypes
+once.  Tensors are passed as raw device pointers (`build.load` says through what); shapes, dtypes
 and contiguity are checked here, on the host, before anything is launched.
 There is no CPU path: a tensor that is not on a CUDA device is an error, and so
 is a kernel library that cannot be built or loaded.

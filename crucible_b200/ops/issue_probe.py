@@ -4,8 +4,8 @@
 
 prints cycles per `tcgen05.mma` sent by one thread (by tile width, with a loop as tight as the
 kernels' and with a straightforward one) and cycles per TMA box sent by one thread (by the
-box's height).  The tensor-core kernels' loops are shaped by these figures: for tiles up to
-128 columns wide a step of K costs what its MMA thread's own instructions cost.
+box's height), for a sender picked by its number.  The tensor-core kernels' loops were shaped by these figures; an
+elected sender, as they have it now, takes less.
 """
 from __future__ import annotations
 

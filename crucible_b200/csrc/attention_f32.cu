@@ -310,12 +310,13 @@ int launch(const Params& p, int n_requests, int max_new, cudaStream_t s) {
 
 }  // namespace
 
+// warps: of a block of 32 rows, 8 or 4; the same bits either way.
 CB_EXPORT int cb_attention_f32(const float* q, int q_stride, const float* gate, int gate_stride, float* out,
                                int out_stride, const float* k_cache, const float* v_cache, const float* sinks,
                                const int* req_row_start, const int* req_first_pos, const int* block_table,
                                int table_stride, int n_requests, int max_new, int n_heads, int n_kv_heads,
                                int key_dim, int value_dim, int page_tokens, float scale, int window, int chunked,
-                               int keep_first, float out_scale, int gate_per_head, void* stream) {
+                               int keep_first, float out_scale, int gate_per_head, int warps, void* stream) {
     if (n_requests <= 0 || max_new <= 0) return 0;
     const int most = key_dim > value_dim ? key_dim : value_dim;
     if (n_heads % n_kv_heads != 0 || most > 256 || ((key_dim | value_dim | q_stride | out_stride) & 3) != 0 ||
@@ -333,14 +334,12 @@ CB_EXPORT int cb_attention_f32(const float* q, int q_stride, const float* gate, 
     cudaStream_t s = (cudaStream_t)stream;
     const bool few = max_new * p.n_rep <= 16;
     // Blocks of 32 rows: two or more to an SM, so that one's barriers and exponentials run beside another's products,
-    // and twice as many to deal out where the longest walks eleven tiles and the average six.  Few blocks have an SM
-    // to themselves and take eight warps.  us with 64 rows and eight warps / 32 and four / 32 and eight: 700 tokens of 12
-    // heads of 64 75 / 71 / 78, of 8 heads of 128 116 / 97 / 89, 2,000 of 16 heads of 64 406 / 346 / 408, of 128 595 /
-    // 595 / 850, 300 of 8 heads of 128 58 / 45 / 44.
-    const long blocks = (long)((max_new * p.n_rep + 31) / 32) * n_kv_heads * n_requests;
+    // and twice as many to deal out where the longest walks eleven tiles and the average six.  us with 64 rows and eight
+    // warps / 32 and four / 32 and eight: 700 tokens of 12 heads of 64 (264 blocks of 32) 76 / 71 / 78, 2,000 of 8 heads of 64
+    // (504) 293 / 242 / 277, of 128 on 2 (500) 314 / 310 / 443; 300 of 8 heads of 128 on 2 (76) 58 / 45 / 44.
 #define CB_F32_ATTENTION(DD)                                           \
     return few ? launch<DD, 16, 256>(p, n_requests, max_new, s)        \
-           : blocks <= 200 ? launch<DD, 32, 256>(p, n_requests, max_new, s) \
+           : warps == 8 ? launch<DD, 32, 256>(p, n_requests, max_new, s) \
                            : launch<DD, 32, 128>(p, n_requests, max_new, s)
     if (most <= 64) CB_F32_ATTENTION(64);
     if (most <= 128) CB_F32_ATTENTION(128);

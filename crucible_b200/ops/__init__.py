@@ -499,6 +499,16 @@ def rope_kv_append(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: i
 F32_TILES = True          # tests switch it off to reach the one-warp-a-row kernels with the same inputs
 
 
+def f32_attention_warps(blocks: int, max_new: int, max_context: int) -> int:
+    """Warps of a block of 32 rows of the 32-bit attention, by how many blocks there are.  Alone on its SM a block has eight;
+    with more blocks than SMs four, so that two find room.  But while a portion's first rows have few keys, the blocks
+    beyond one an SM are short ones that begin early, and eight warps stay ahead a while longer; where most keys lie ahead of
+    the portion all blocks take as long, and a second wave of them as long again.  us with 8 and 4: 700 tokens of 8 heads
+    of 128 on 2 (176 blocks) 90 and 97, of 9 heads of 64 on 1 (197) 61 and 65; 130 behind 1,500, 40 heads of 128 on 1
+    (163) 368 and 257, 48 of 64 (195) 179 and 160.  (`max_context` 0: not known.)"""
+    return 8 if blocks <= (148 if max_context >= 2 * max_new else 200) else 4
+
+
 def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, key_dim, value_dim, scale, window,
                   chunked, keep_first, out_scale, ctx, page_tokens, table, gate_per_head=False) -> bool:
     """The 32-bit attention over tiles of keys (`csrc/attention_f32.cu`): float32 rows of sizes up to 256
@@ -518,7 +528,9 @@ def attention_f32(q, gate, out, k_cache, v_cache, sinks, n_heads, n_kv_heads, ke
         _ptr(ctx.req_first_pos), _ptr(table), table.shape[1], ctx.n_requests,
         host.max_new_tokens, n_heads, n_kv_heads, key_dim, value_dim,
         page_tokens, scale, window or 0, 1 if chunked else 0, keep_first,
-        out_scale, 1 if gate_per_head else 0, _stream())
+        out_scale, 1 if gate_per_head else 0,
+        f32_attention_warps(-(-host.max_new_tokens * (n_heads // n_kv_heads) // 32) * n_kv_heads * ctx.n_requests,
+                            host.max_new_tokens, getattr(host, "max_context_len", 0)), _stream())
     if code == build.UNSUPPORTED:
         return False
     _check(code, "attention (32-bit tiles)")

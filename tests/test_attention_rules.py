@@ -73,3 +73,12 @@ def test_32_bit_tiles_take_pools_whose_rows_an_int_counts(pages, heads, page, ta
     got = ops.attention_f32(rows, None, torch.zeros(3, 4 * heads), pool, pool, None, heads, heads, 4, 4, 0.5, None, False, 0, 1.0,
                             ctx, page, torch.zeros((1, 4), dtype=torch.int32))
     assert got == taken and len(calls) == taken
+
+
+@pytest.mark.parametrize("blocks,new,context,warps", [
+    # (measured: 8 and 4 warps, us: 48 and 49, 90 and 97, 61 and 65; 202 and 197, 368 and 257, 179 and 160; 78 and 71)
+    (172, 450, 450, 8), (176, 700, 700, 8), (197, 700, 700, 8), (136, 130, 1630, 8), (163, 130, 1630, 4), (195, 130, 1630, 4),
+    (264, 700, 700, 4), (148, 90, 690, 8), (149, 90, 180, 4), (200, 90, 179, 8), (201, 90, 90, 4)])
+def test_warps_of_a_32_bit_attention_block(blocks, new, context, warps):
+    from crucible_b200 import ops
+    assert ops.f32_attention_warps(blocks, new, context) == warps

@@ -16,17 +16,17 @@ STEP = True                  # likewise, for the form of a token each
 
 
 # us of the walk over tokens (a launch, a token of the longest portion, a token and head of 128, a portion and head) with
-# 1, 2 and 4 columns of a matrix a lane, and of the chunks (their launches, a chunk and head of 128), fitted to
-# all of them over 4 to 32 heads of 64 and 128 and 1 to 48 uneven portions of up to 4 to 490 tokens
-_DELTA_COSTS = ({1: (3.43, 0.183, 0.0060, 0.0553), 2: (3.49, 0.227, 0.0037, 0.0460), 4: (4.55, 0.337, 0.0032, 0.0383)},
-                (15.7, 0.2576))
-COSTS = {DELTA: _DELTA_COSTS, CHANNEL: _DELTA_COSTS,
+# 1, 2 and 4 columns of a matrix a lane, fitted over 4 to 32 heads of 64 and 128 and 1 to 48 uneven portions of up to 4
+# to 490 tokens, and of the chunks (their launches, a chunk and head of 128), fitted over 4 to 32 heads and 1 to 12 portions of
+# 24 to 900 tokens on average
+_DELTA_WALK = {1: (3.43, 0.183, 0.0060, 0.0553), 2: (3.49, 0.227, 0.0037, 0.0460), 4: (4.55, 0.337, 0.0032, 0.0383)}
+COSTS = {DELTA: (_DELTA_WALK, (14.0, 0.188)), CHANNEL: (_DELTA_WALK, (14.5, 0.236)),
          MLSTM: ({1: (3.49, 0.192, 0.0072, 0.0613), 2: (4.35, 0.240, 0.0046, 0.0430), 4: (5.75, 0.350, 0.0036, 0.0361)},
-                 (25.8, 0.162)),
+                 (21.5, 0.124)),
          WKV: ({1: (3.28, 0.148, 0.0068, 0.0647), 2: (3.55, 0.172, 0.0037, 0.0515), 4: (3.50, 0.296, 0.0035, 0.0419)},
-               (19.7, 0.1485)),
+               (19.5, 0.120)),
          SSD: ({1: (3.60, 0.127, 0.0038, 0.0635), 2: (4.41, 0.142, 0.0026, 0.0446), 4: (5.84, 0.181, 0.0027, 0.0341)},
-               (21.7, 0.1307))}
+               (18.0, 0.112))}
 
 
 @functools.lru_cache(maxsize=4096)
@@ -62,8 +62,9 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
     The chunks' launches and workspaces are some 30 us of host work, which a step that runs eagerly pays and whose
     host time covers either form of little work (wkv, a portion of 150: 37 and 36 us on the device, the layer
     eagerly 275 and 242): less than 96 tokens a request of the delta rules, or less than 160 of a few of the others,
-    are walked, and more where the costs say that the walk is ahead.  Of 760 steps measured that is
-    3.5 % from the quicker form on average, those walked for the host's sake among them."""
+    are walked, and more where the costs say that the walk is ahead.  Of 532 steps
+    measured that are enough work for that, the choice is 0.7 % from the quicker form on average (46 % at worst), and none
+    is slower than by one column or by the chunks as they were before there were more."""
     if requests <= 0:
         return False
     if rule in (DELTA, CHANNEL):
@@ -73,7 +74,7 @@ def chunks_pay(rule, rows: int, requests: int, longest: int, heads: float) -> bo
         return False
     first, chunk = COSTS[rule][1]
     walk = walk_columns(rule, requests, rows, longest, heads, 128, 128)[1]      # of the form that would be launched
-    return walk > 0.95 * (first + chunk * (rows / 32 + requests / 2) * heads)
+    return walk > first + chunk * (rows / 32 + requests / 2) * heads
 
 
 CHUNK_SPACE = 256 << 20      # bytes of the chunks' workspaces

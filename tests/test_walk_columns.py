@@ -67,7 +67,9 @@ def test_more_columns_only_where_they_are_clearly_quicker(rule, lengths, H, D, c
 
 
 @pytest.mark.parametrize("rule,lengths,heads", [
-    # (measured, chunks and walk, us: 222 and 316, 212 and 313, 268 and 352, 178 and 274, 41 and 51, 64 and 87)
+    # (measured, chunks and walk, us: 239 and 342, 300 and 373, 222 and 316, 212 and 313, 268 and 352, 178 and 274, 41 and
+    # 51, 64 and 87)
+    ("DELTA", [300, 700, 410, 520, 333], 16), ("CHANNEL", [300, 700, 410, 520, 333], 16),
     ("DELTA", [500, 250, 125, 60, 30], 32), ("DELTA", [64, 128, 256, 512], 32), ("DELTA", [513, 511, 300], 32),
     ("CHANNEL", [330, 290], 32), ("SSD", [150, 100, 120], 16), ("SSD", [150, 100, 120], 32)])
 def test_the_walk_that_chunks_are_weighed_against_is_the_one_launched(rule, lengths, heads):
@@ -76,4 +78,4 @@ def test_the_walk_that_chunks_are_weighed_against_is_the_one_launched(rule, leng
     assert k.chunks_pay(code, *shape, float(heads))
     first, chunk = k.COSTS[code][1]
     walk = k.walk_columns(code, len(lengths), sum(lengths), max(lengths), heads, 128, 128)[1]
-    assert walk > 0.95 * (first + chunk * (sum(lengths) / 32 + len(lengths) / 2) * heads)
+    assert walk > first + chunk * (sum(lengths) / 32 + len(lengths) / 2) * heads

@@ -514,21 +514,16 @@ def tiles_by_chance(pairs: int, n_experts: int) -> float:
                            for j in range(int((mean + 4 * math.sqrt(mean)) / 128) + 1))
 
 
-WAVES_START = 64            # what the kernel of several tiles a block takes before its first product, beside a block a tile
-
-
 def _grouped_cost(pairs: int, n_experts: int, tiles: float, n_cols: int, gated: bool) -> int:
     """What a grouped product over `tiles` tiles costs in the unit of `_tile_width`: its waves, each the tile's
-    width and a fixed part."""
-    waves = grouped_waves(pairs, n_experts, n_cols)
-    bn, fixed = (256, 128) if waves else (grouped_tile(pairs, n_experts, n_cols, gated)[0], 160)
-    return -(-math.ceil(tiles * -(-n_cols // bn)) // N_SMS) * (bn + fixed) + WAVES_START * waves
+    width and a fixed part, less of it where a block takes several tiles and hides a tile's end behind the next."""
+    bn, fixed = (256, 64) if grouped_waves(pairs, n_experts, n_cols) else (grouped_tile(pairs, n_experts, n_cols, gated)[0], 112)
+    return -(-math.ceil(tiles * -(-n_cols // bn)) // N_SMS) * (bn + fixed)
 
 
 def _dense_cost(m: int, n_cols: int, k: int, epi: int) -> int:
     bn = _waves_width(m, n_cols, k, epi)
-    return (-(--(-m // 128) * -(-n_cols // bn) // N_SMS) * (bn + 128) + WAVES_START if bn
-            else _product_cost(m, n_cols, k)[0])
+    return -(--(-m // 128) * -(-n_cols // bn) // N_SMS) * (bn + 64) if bn else _product_cost(m, n_cols, k)[0]
 
 
 @functools.lru_cache(maxsize=4096)
@@ -536,11 +531,13 @@ def riding_pays(rows: int, width: int, ff: int, n_experts: int, top: int) -> boo
     """Whether one more expert of the same size that all `rows` rows choose goes with the grouped products of the
     others, `top` of `n_experts` a row, instead of by two products of its own: by the waves that the four products
     take and the two would.  Its rows fill tiles of their own, which may cost a wave more than the dense products do.
-    20 sizes (4 to 128 experts of 512 x 768 to 4,096 x 2,816, top 1 to 8) at 136 to 4,096 rows, 430 measured: where the
-    reckoned waves are 8 % less, no layer was slower by more than 0.7 %, and the mean over all is 3.5 % quicker
-    (riding always 3.4 %, 13 % slower at worst).  us apart and riding: 8 of 2,048 x 2,816, top 2, 320 rows 100 and
-    100, 600 135 and 121, 1,600 192 and 195 (apart), 2,048 223 and 217; 32 of 2,048 x 1,408, top 4, 450 rows 150 and 134,
-    900 162 and 166 (apart).  Of 5,000 to 8,192 rows neither is ahead (the mean of 18: 0.2 % behind)."""
+    Riding saves two launches (100,000 of the unit times K).  16 sizes (4 to 64 experts of 512 x 768 to 4,096 x 1,536, top 1
+    to 8) at 136 to 4,096 rows, 512 measured both replayed and eagerly, against apart: where the reckoned cost is 7 % less,
+    0.955 and 0.936 on average, 10 of them more than 1.5 % slower (3.9 % at worst).  Riding
+    always is 0.958 and 0.937, 13 % slower at worst, by two limits on the rows as before 0.965 and 0.946.  us apart and
+    riding: 8 of 2,048 x 2,816, top 2, 320 rows 100 and 100, 600 135 and 121, 2,048 223 and 217, 4,096 381 and 394; 32 of
+    2,048 x 1,408, top 4, 450 rows 150 and 134; 8 of 4,096 x 1,536, top 1, 384 rows 107 and 121.  Of 5,000 to 8,192 rows
+    neither is ahead (the mean of 18: 0.2 % behind)."""
     if rows > 4096:
         return False
     pairs = rows * top
@@ -550,7 +547,7 @@ def riding_pays(rows: int, width: int, ff: int, n_experts: int, top: int) -> boo
              + ff * (_grouped_cost(pairs, n_experts, tiles, width, False) + _dense_cost(rows, width, ff, ACCUM_F32)))
     riding = (width * _grouped_cost(pairs + rows, n_experts + 1, more, 2 * ff, True)
               + ff * _grouped_cost(pairs + rows, n_experts + 1, more, width, False))
-    return riding <= 0.92 * apart
+    return riding <= 0.93 * (apart + 100_000)
 
 
 def grouped_linear(a, w, out, plan, n_experts: int, tiles: int, gated: bool, pair=None, tile=None) -> bool:

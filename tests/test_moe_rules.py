@@ -52,7 +52,7 @@ def test_a_shared_expert_is_held_once(shared, slices, copies, dtype):
     (2048, 2816, 2816, 8, 2, 128, True), (1024, 1408, 2816, 8, 2, 128, True), (1024, 1408, 2816, 8, 2, 129, False),
     (1024, 1408, 0, 8, 2, 64, False),
     # (of one slice beyond 128 rows: layers measured to be quicker so by 2 to 18 %, or slower by 2 to 13 %)
-    (2048, 2816, 2816, 8, 2, 256, False), (2048, 2816, 2816, 8, 2, 384, True), (2048, 2816, 2816, 8, 2, 600, True),
+    (2048, 2816, 2816, 8, 2, 136, False), (1024, 1408, 1408, 8, 2, 1706, True), (2048, 2816, 2816, 8, 2, 384, True), (2048, 2816, 2816, 8, 2, 600, True),
     (2048, 2816, 2816, 8, 2, 1600, False), (2048, 2816, 2816, 8, 2, 2048, True), (2048, 2816, 2816, 8, 2, 4096, False),
     (1024, 1408, 1408, 8, 2, 136, True), (1024, 1408, 1408, 8, 2, 600, True), (2048, 1408, 1408, 32, 4, 450, True),
     (2048, 1408, 1408, 32, 4, 900, False), (1024, 1024, 1024, 16, 2, 256, True), (1024, 1024, 1024, 16, 2, 512, False),
